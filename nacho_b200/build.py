@@ -1,4 +1,5 @@
-"""Builds ``libnacho_b200.so`` (CUDA kernels + C ABI) for sm_100a with nvcc, in-tree.
+"""Builds ``libnacho_b200.so`` (CUDA kernels + C ABI) for sm_100a with nvcc and ``_native.so`` (the
+Python operators over it) with g++, in-tree.
 
 Run as ``python -m nacho_b200.build``. Objects are cached under ``nacho_b200/csrc/build/``
 and rebuilt when a source or header is newer.
@@ -11,12 +12,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libnacho_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -67,12 +70,35 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed for {cmd[-3]}")
     if jobs or _stale(LIB, objs):
-        cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
+        cmd = [nvcc, "-shared", "-o", LIB, "-Xlinker", "-soname=libnacho_b200.so"] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libnacho_b200.so failed")
+    build_native(nvcc, verbose)
     return LIB
+
+
+def build_native(nvcc: str, verbose: bool = False) -> str:
+    """``_native.so`` against the torch of this interpreter; it finds ``libnacho_b200.so`` beside itself."""
+    src = os.path.join(CSRC, "native.cpp")
+    if not _stale(NATIVE, [src, os.path.join(ROOT, "include", "nacho_b200.h"), os.path.abspath(__file__)]):
+        return NATIVE
+    import torch
+    torch_dir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in (os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
+        cmd += ["-isystem", inc]
+    cmd += ["-I", os.path.join(ROOT, "include"), src, "-o", NATIVE, "-L", os.path.join(torch_dir, "lib"), "-L", HERE, "-lnacho_b200",
+            "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode != 0:
+        raise RuntimeError("build of _native.so failed")
+    return NATIVE
 
 
 if __name__ == "__main__":
