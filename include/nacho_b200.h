@@ -159,7 +159,7 @@ int nb200_csr_add_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *z,
  * a pool that grows on demand. The call makes no cudaMalloc / cudaFree / cudaHostAlloc and
  * calls no allocating library routine; the caller provides every operand and result array.
  * Limits and rules:
- *   - nnz(A) + nnz(B) may not exceed 32768 tiles' worth of entries (about 159 million);
+ *   - nnz(A) + nnz(B) may not exceed 159350784 entries;
  *     larger inputs return NB200_E_UNSUPPORTED and nothing is launched.
  *   - `capacity` (entries in z->col / z->val) must be at least nnz(A) + nnz(B); otherwise
  *     NB200_E_CAPACITY. z->row_ptr holds rows + 1 entries.
@@ -294,8 +294,8 @@ int nb200_csf_add_f32_into(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 
  *                        min(n_i(A), n_i(B)) for the product; `capacity` as for CSR. The product
  *                        keeps every row that BOTH operands store, with an empty column range where
  *                        their columns do not meet, as nacho's level-by-level intersection does.
- * These run the CSR merge kernels on the operands' own column / value arrays after rebuilding the
- * row offsets, so they need scratch of a few int32 per matrix ROW (not per stored row). */
+ * These run the CSR merge kernels on the operands' own column / value arrays. Scratch: a few int32 per
+ * matrix row for the coordinate lists (their row offsets are rebuilt), per STORED row for DCSR. */
 int nb200_coo_add_f32_into(const nb200_coo *a, const nb200_coo *b, nb200_coo *z, int64_t capacity, void *stream);
 int nb200_coo_mul_f32_into(const nb200_coo *a, const nb200_coo *b, nb200_coo *z, int64_t capacity, void *stream);
 int nb200_coo_csr_add_f32_into(const nb200_csr *a, const nb200_coo *b, nb200_csr *z, int64_t capacity, void *stream);

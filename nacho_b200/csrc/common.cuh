@@ -34,7 +34,7 @@ int note_timeout(int site, int tile, const char *where);
 struct Workspace {
     void *dev = nullptr;
     size_t dev_bytes = 0;
-    int64_t *host = nullptr;  // pinned, 64 int64 slots
+    int64_t *host = nullptr;  // pinned, device-visible: 32 int64 slots for copies, then 32 result words that kernels write
     uint64_t generation = 0;  // bumped by every acquire: a holder can tell whether the block was handed out again
 };
 
@@ -45,6 +45,28 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
 // Counts the calls of nb200_release_workspaces(): a Workspace pointer obtained under an earlier
 // value is dangling.
 uint64_t workspace_epoch();
+
+// ---- result words ---------------------------------------------------------------------
+
+// How an operator learns a result length without a copy queued behind its kernels: the last tile
+// stores one 8-byte word {valid, status, value} straight into pinned host memory and the host polls
+// it. A copy plus a stream synchronisation costs 10 us more on a call that computes for 6.
+// The value is complete when the word arrives; the arrays it describes are complete in stream order.
+constexpr unsigned long long RW_VALID = 1ull << 63;
+constexpr int RW_STATUS_SHIFT = 56;
+constexpr unsigned long long RW_VALUE_MASK = (1ull << RW_STATUS_SHIFT) - 1;
+constexpr int RW_SLOTS = 32;
+
+// Clears result word `k` (0 .. RW_SLOTS - 1) of a workspace; to be called before the launch that writes it.
+inline unsigned long long *result_word(Workspace *ws, int k) {
+    volatile unsigned long long *w = reinterpret_cast<volatile unsigned long long *>(ws->host) + 32 + k;
+    *w = 0;
+    return const_cast<unsigned long long *>(w);
+}
+
+// Polls a result word until a kernel of `stream` has written it. Returns NB200_OK with the value and
+// the kernel's status, or an error if the stream failed or ran dry without writing the word.
+int wait_result_word(const unsigned long long *word, cudaStream_t stream, int64_t *value, int *device_status);
 
 // Carves 256-byte-aligned sub-blocks out of a Workspace.
 class Carver {
@@ -92,6 +114,12 @@ struct DeviceStatus {
 #ifdef __CUDACC__
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
+
+// Publishes a result word (see above). The store is a single 8-byte one, so it needs no fence.
+__device__ __forceinline__ void publish_result_word(unsigned long long *word, int status, long long value) {
+    if (word) *reinterpret_cast<volatile unsigned long long *>(word) = RW_VALID | ((unsigned long long)status << RW_STATUS_SHIFT) |
+                                                                       ((unsigned long long)value & RW_VALUE_MASK);
+}
 
 template <typename T>
 __device__ __forceinline__ T ld_nc(const T *p) {

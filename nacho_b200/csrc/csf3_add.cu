@@ -4,8 +4,9 @@
 // src/backend/partition.cpp:286-328, 586-811): merge the i lists, under equal i merge the j
 // fibres, under equal (i, j) merge k, otherwise copy the subtree. The result is the unique
 // canonical tree of the union of the coordinate sets, so it is produced here from flat merges, by
-// one of two routes (two_level_pays chooses; NACHO_B200_CSF_TWO_LEVEL=0 / 1 forces one).
-// Route over expanded coordinates (fibres of about one entry):
+// one of two routes (levels_pay chooses; NACHO_B200_CSF_TWO_LEVEL=0 / 1 forces one).
+// Route over expanded coordinates (an operand that stores empty slices or fibres, capacities below the worst
+// case):
 //   1. k_csf_expand    every stored entry gets its (i, j) written out next to its k: one warp
 //                      per 32 (i, j) fibres finds their i by binary search and fills their ranges;
 //   2. coo3_add_run    the sorted-union merge of the two coordinate lists (coo3_merge.cu); k and
@@ -16,15 +17,14 @@
 //                      the merged (i, j) columns: head flags for new i and new (i, j), a packed
 //                      two-counter scan across tiles by bounded look-back, and the scatter of
 //                      i_idx / j_ptr / j_idx / k_ptr.
-// Two-level route (fibres of several entries; described above csf_add_two_level): the fibre lists
-// are merged by the route above, which yields the upper levels and tells which operand holds which
-// fibre; the entries then go through the CSR union with one row per result fibre, so that no
-// per-entry (i, j) is ever written.
+// Level-by-level route (described above csf_add_levels): one merge per
+// level, each of which tells the next where the ranges of A and B begin, so that no per-entry (i, j) is
+// ever written.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
-#include "merge_common.cuh"
+#include "csr_common.cuh"
 
 namespace nb200 {
 
@@ -193,55 +193,12 @@ __global__ void __launch_bounds__(NT) k_csf_compress(int32_t nnz, const int32_t 
     }
 }
 
-constexpr int FS_VT = 8;  // fibres per thread in k_fibre_slices
-
-// i of every fibre. A CTA takes NT * FS_VT consecutive fibres; they lie in at most that many + 1
-// consecutive stored slices (a stored slice has at least one fibre), so warp 0 finds the slice of the
-// first fibre with a 32-ary search, the CTA copies that window of j_ptr / i_idx to shared memory and
-// every thread finds its fibres' slices there.
-__global__ void __launch_bounds__(NT) k_fibre_slices(int32_t n_i, int32_t n_j, const int32_t *__restrict__ i_idx,
-                                                    const int32_t *__restrict__ j_ptr, int32_t *__restrict__ out_i) {
-    constexpr int SPAN = NT * FS_VT;
-    __shared__ int32_t s_start[SPAN + 1], s_i[SPAN + 1];
-    __shared__ int s_first;
-    const int tid = threadIdx.x;
-    const int64_t q0 = (int64_t)blockIdx.x * SPAN;
-    if (tid < 32) {
-        const int64_t r = warp_last_true(0, (int64_t)n_i - 1, [&](int64_t x) { return ld_nc(j_ptr + x) <= q0; });
-        if (tid == 0) s_first = (int)r;
-    }
-    __syncthreads();
-    const int first = s_first;
-    const int need = (int)min((int64_t)SPAN, (int64_t)n_j - q0);  // fibres of this CTA: slices first .. first + need at most
-    for (int w = tid; w <= need; w += NT) {
-        const bool live = first + w < n_i;
-        s_start[w] = live ? ld_nc(j_ptr + first + w) : INT32_MAX;
-        s_i[w] = live ? ld_nc(i_idx + first + w) : 0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < FS_VT; ++v) {
-        const int64_t q = q0 + tid + v * NT;
-        if (q >= n_j) return;
-        int lo = 0, hi = need;  // largest w with s_start[w] <= q
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_start[mid] <= q) lo = mid; else hi = mid - 1;
-        }
-        out_i[q] = s_i[lo];
-    }
-}
-
 // The route over expanded coordinates: steps 1-3 of the file comment. `z`'s arrays exist and hold
 // cap_i / cap_j / cap_k entries (cap_k >= n_k(A) + n_k(B)); nothing is freed here on failure.
-// `unit_fibres`: every fibre of the operands holds exactly one entry (n_k == n_j) and their k_ptr
-// arrays are not read: the j column of the entries is j_idx itself and only i is written out.
-int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, int64_t cap_i, int64_t cap_j, int64_t cap_k,
-                     cudaStream_t stream, int slot, bool unit_fibres = false) {
+int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, int64_t cap_i, int64_t cap_j, cudaStream_t stream) {
     const int64_t total = (int64_t)a->n_k + b->n_k;
     cudaError_t e;
     int st;
-    (void)cap_k;
     // one pool block: expanded (i, j) of A, of B and of the merged list, the merge's own scratch
     // and the compress pass's control block and tile words
     const int64_t compress_tiles = std::max<int64_t>((total + NT * CVT - 1) / (NT * CVT), coo3_add_tiles(total));
@@ -255,7 +212,7 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
     sizes.take<uint64_t>((size_t)compress_tiles + 8);
     const size_t own = sizes.used();
     Workspace *ws = nullptr;
-    if ((st = acquire_workspace(stream, own + coo3_add_scratch_bytes(total) + 256, &ws, slot))) return (st);
+    if ((st = acquire_workspace(stream, own + coo3_add_scratch_bytes(total) + 256, &ws))) return (st);
     Carver carve(ws->dev);
     int32_t *ai = carve.take<int32_t>((size_t)a->n_k), *aj = carve.take<int32_t>((size_t)a->n_k);
     int32_t *bi = carve.take<int32_t>((size_t)b->n_k), *bj = carve.take<int32_t>((size_t)b->n_k);
@@ -263,26 +220,13 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
     uint64_t *compress_block = carve.take<uint64_t>((size_t)compress_tiles + 8);
     void *merge_scratch = static_cast<unsigned char *>(ws->dev) + own;
 
-    if (unit_fibres) {
-        aj = a->j_idx;
-        bj = b->j_idx;
-        if (a->n_j > 0) {
-            LaunchScope scope("csf_fibre_slices", stream);
-            k_fibre_slices<<<(int)(((int64_t)a->n_j + NT * FS_VT - 1) / (NT * FS_VT)), NT, 0, stream>>>(a->n_i, a->n_j, a->i_idx, a->j_ptr, ai);
-        }
-        if (b->n_j > 0) {
-            LaunchScope scope("csf_fibre_slices", stream);
-            k_fibre_slices<<<(int)(((int64_t)b->n_j + NT * FS_VT - 1) / (NT * FS_VT)), NT, 0, stream>>>(b->n_i, b->n_j, b->i_idx, b->j_ptr, bi);
-        }
-    } else {
-        if (a->n_j > 0) {
-            LaunchScope scope("csf_expand", stream);
-            k_csf_expand<<<(int)(((int64_t)a->n_j + 31) / 32 * 32 + NT - 1) / NT, NT, 0, stream>>>(a->n_i, a->n_j, a->i_idx, a->j_ptr, a->j_idx, a->k_ptr, ai, aj);
-        }
-        if (b->n_j > 0) {
-            LaunchScope scope("csf_expand", stream);
-            k_csf_expand<<<(int)(((int64_t)b->n_j + 31) / 32 * 32 + NT - 1) / NT, NT, 0, stream>>>(b->n_i, b->n_j, b->i_idx, b->j_ptr, b->j_idx, b->k_ptr, bi, bj);
-        }
+    if (a->n_j > 0) {
+        LaunchScope scope("csf_expand", stream);
+        k_csf_expand<<<(int)(((int64_t)a->n_j + 31) / 32 * 32 + NT - 1) / NT, NT, 0, stream>>>(a->n_i, a->n_j, a->i_idx, a->j_ptr, a->j_idx, a->k_ptr, ai, aj);
+    }
+    if (b->n_j > 0) {
+        LaunchScope scope("csf_expand", stream);
+        k_csf_expand<<<(int)(((int64_t)b->n_j + 31) / 32 * 32 + NT - 1) / NT, NT, 0, stream>>>(b->n_i, b->n_j, b->i_idx, b->j_ptr, b->j_idx, b->k_ptr, bi, bj);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return (note_cuda_error(e, "k_csf_expand"));
@@ -339,183 +283,77 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
     return NB200_OK;
 }
 
-// ------------------------------------------------------------------ the two-level route ----
+// -------------------------------------------------------------- the level-by-level route ----
 //
-// When the fibres hold several entries each, expanding (i, j) for every entry moves more bytes
-// than the tensor has. The same union then comes from two smaller merges:
-//   1. the fibre lists of A and B -- every (i, j) fibre as one entry of a tensor whose third level
-//      is a single position -- go through the expanded route above with the values 1 (A) and 2 (B):
-//      the result is Z's i_idx / j_ptr / j_idx, and per fibre of Z the sum 1, 2 or 3 says which
-//      operands hold it;
-//   2. an exclusive count of the A flags (and of the B flags) is the fibre of A (of B) that a
-//      fibre of Z corresponds to, or the next one if the operand lacks it: k_ptr[that fibre] is a
-//      row-offset array over Z's fibres in which a missing fibre is an empty row;
-//   3. with those offsets A's and B's (k_idx, val) arrays are CSR matrices with one row per fibre
-//      of Z, and the CSR union (csr_merge.cu) writes Z's k_ptr, k_idx and val in one pass.
+// Expanding (i, j) for every entry moves more bytes than the tensor has. The same union comes from one merge
+// per level, none of which waits for the host:
+//   1. the slice lists of A and B, as matrices of one row whose columns are the slice numbers, in the
+//      offsets mode of the CSR tile kernel: Z's i_idx, and over Z's slices a row-offset array into the
+//      fibres of A (of B) in which a slice the operand lacks is an empty row;
+//   2. with those, the fibre lists are CSR matrices with one row per slice of Z: the offsets mode again
+//      gives Z's j_ptr and j_idx and, over Z's fibres, offsets into the entries of A and of B;
+//   3. with those, A's and B's (k_idx, val) arrays are CSR matrices with one row per fibre of Z, and the
+//      CSR union writes Z's k_ptr, k_idx and val.
+// Steps 2 and 3 read their row count from device memory.
 
-__global__ void __launch_bounds__(NT) k_fill_float(float *__restrict__ p, int32_t n, float v) {
-    const int64_t i = (int64_t)blockIdx.x * NT + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
-constexpr int OVT = 16;  // fibres per thread in the offsets pass
-constexpr int32_t DCSR_FIBRE_ROWS = 1 << 24;  // first extent up to which the fibre lists go through the DCSR union
-
-// flags[u] in {1, 2, 3} for the n fibres of Z: which operand holds fibre u. Writes, for u = 0 .. n,
-// off_a[u] = a_kptr[fibres of A before u] and off_b[u] likewise: one pass, the two running counts
-// packed into one word and carried across tiles by bounded look-back.
-__global__ void __launch_bounds__(NT) k_fibre_offsets(const float *__restrict__ flags, int32_t n, const int32_t *__restrict__ a_kptr,
-                                                     const int32_t *__restrict__ b_kptr, int32_t *__restrict__ off_a,
-                                                     int32_t *__restrict__ off_b, uint64_t *state_raw, FusedCtl *ctl) {
-    __shared__ int scan_tmp[72];
-    __shared__ long long s_base;
-    volatile uint64_t *state = state_raw;
-    const int tid = threadIdx.x, t = blockIdx.x;  // CTAs are dispatched in index order; waits on earlier tiles are bounded
-    const int64_t p0 = ((int64_t)t * NT + tid) * OVT;
-    int f[OVT], mine_a = 0, mine_b = 0;
-    if (p0 + OVT <= n) {  // 16-byte loads: a thread's fibres are consecutive
-#pragma unroll
-        for (int q = 0; q < OVT; q += 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(flags + p0 + q));
-            f[q] = (int)v.x, f[q + 1] = (int)v.y, f[q + 2] = (int)v.z, f[q + 3] = (int)v.w;
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < OVT; ++q) f[q] = p0 + q < n ? (int)ld_nc(flags + p0 + q) : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < OVT; ++q) {
-        mine_a += f[q] & 1;
-        mine_b += f[q] >> 1;
-    }
-    int before_a, before_b, tot_a, tot_b;
-    block_excl_sum2<NT>(mine_a, mine_b, scan_tmp, before_a, before_b, tot_a, tot_b);
-    if (warp_id() == 0) {
-        const int64_t b = lookback_exclusive(state, t, ((int64_t)tot_a << 31) | (int64_t)tot_b, &ctl->status);
-        if (lane_id() == 0) s_base = b;
-    }
-    __syncthreads();
-    const long long base = s_base;
-    if (base < 0) return;
-    int ca = (int)(base >> 31) + before_a, cb = (int)(base & 0x7fffffff) + before_b;
-    int32_t va[OVT], vb[OVT];
-#pragma unroll
-    for (int q = 0; q < OVT; ++q) {
-        const bool live = p0 + q <= n;
-        va[q] = live ? ld_nc(a_kptr + ca) : 0;
-        vb[q] = live ? ld_nc(b_kptr + cb) : 0;
-        ca += f[q] & 1;
-        cb += f[q] >> 1;
-    }
-    if (p0 + OVT <= (int64_t)n + 1) {
-#pragma unroll
-        for (int q = 0; q < OVT; q += 4) {
-            *reinterpret_cast<int4 *>(off_a + p0 + q) = make_int4(va[q], va[q + 1], va[q + 2], va[q + 3]);
-            *reinterpret_cast<int4 *>(off_b + p0 + q) = make_int4(vb[q], vb[q + 1], vb[q + 2], vb[q + 3]);
-        }
-    } else {
-#pragma unroll
-        for (int q = 0; q < OVT; ++q)
-            if (p0 + q <= n) off_a[p0 + q] = va[q], off_b[p0 + q] = vb[q];
-    }
-}
-
-// The expanded route moves 8 bytes of (i, j) per entry out and back in; the two-level route moves
-// about as much per FIBRE. It pays once fibres hold a few entries on average.
-bool two_level_pays(const nb200_csf3 *a, const nb200_csf3 *b) {
+// Measured against the expanded route: 25 M entries per operand in fibres of 7, 558 us against 821; 5 M in
+// fibres of 4, 230 against 258; 5000 in fibres of 1.1, 54 against 66. So it is taken wherever it applies.
+bool levels_pay(const nb200_csf3 *a, const nb200_csf3 *b) {
     if (a->n_j == 0 || b->n_j == 0) return false;
     if (const char *e = std::getenv("NACHO_B200_CSF_TWO_LEVEL")) return e[0] != '0';  // read per call: tests take both routes
-    return 3 * ((int64_t)a->n_j + b->n_j) <= (int64_t)a->n_k + b->n_k;
+    return true;
 }
 
-int csf_add_two_level(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, int64_t cap_i, int64_t cap_j, int64_t cap_k,
-                      cudaStream_t stream) {
-    const int32_t nja = a->n_j, njb = b->n_j;
-    const int64_t bound_j = (int64_t)nja + njb;
+// `done` tells whether the result is in place; it is not where an operand stores empty slices or fibres, which
+// the canonical tree does not have (the caller then takes the other route).
+int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cudaStream_t stream, bool *done) {
+    *done = false;
+    const int64_t bound_i = (int64_t)a->n_i + b->n_i, bound_j = (int64_t)a->n_j + b->n_j, total = (int64_t)a->n_k + b->n_k;
     if (bound_j > INT32_MAX - 1) return NB200_E_OVERFLOW;
-    const int32_t most = std::max(nja, njb);
-    const int tiles_cap = (int)((bound_j + 1 + NT * OVT - 1) / (NT * OVT));
     Carver sizes;
-    sizes.take<int32_t>((size_t)most);          // k_idx of the fibre tensors: zeros
-    sizes.take<float>((size_t)nja);             // 1 per fibre of A
-    sizes.take<float>((size_t)njb);             // 2 per fibre of B
-    sizes.take<int32_t>((size_t)bound_j + 1);   // fibre tensor of Z: k_ptr
-    sizes.take<int32_t>((size_t)bound_j);       //                     k_idx
-    sizes.take<float>((size_t)bound_j);         //                     flags
-    sizes.take<int32_t>((size_t)bound_j + 1);   // offsets of A's entries over Z's fibres
-    sizes.take<int32_t>((size_t)bound_j + 1);   // the same for B
-    sizes.take<uint64_t>((size_t)tiles_cap + 8);
+    sizes.take<int32_t>((size_t)bound_i + 1);
+    sizes.take<int32_t>((size_t)bound_i + 1);
+    sizes.take<int32_t>((size_t)bound_j + 1);
+    sizes.take<int32_t>((size_t)bound_j + 1);
+    const size_t own = sizes.used(), list_bytes = csr2_scratch_bytes(bound_i), fibre_bytes = csr2_scratch_bytes(bound_j);
     Workspace *ws = nullptr;
     int st;
-    if ((st = acquire_workspace(stream, sizes.used(), &ws, 3))) return st;
+    if ((st = acquire_workspace(stream, own + list_bytes + fibre_bytes + csr2_scratch_bytes(total), &ws, 3))) return st;
     Carver carve(ws->dev);
-    int32_t *zeros = carve.take<int32_t>((size_t)most);
-    float *ones = carve.take<float>((size_t)nja), *twos = carve.take<float>((size_t)njb);
-    int32_t *zf_kptr = carve.take<int32_t>((size_t)bound_j + 1), *zf_kidx = carve.take<int32_t>((size_t)bound_j);
-    float *flags = carve.take<float>((size_t)bound_j);
-    int32_t *off_a = carve.take<int32_t>((size_t)bound_j + 1), *off_b = carve.take<int32_t>((size_t)bound_j + 1);
-    uint64_t *scan_block = carve.take<uint64_t>((size_t)tiles_cap + 8);
-    auto grid = [](int64_t n) { return (int)((n + NT - 1) / NT); };
+    int32_t *ja = carve.take<int32_t>((size_t)bound_i + 1), *jb = carve.take<int32_t>((size_t)bound_i + 1);
+    int32_t *ka = carve.take<int32_t>((size_t)bound_j + 1), *kb = carve.take<int32_t>((size_t)bound_j + 1);
+    unsigned char *scratch_i = static_cast<unsigned char *>(ws->dev) + own, *scratch_j = scratch_i + list_bytes, *scratch_k = scratch_j + fibre_bytes;
+    unsigned long long *word[3] = {result_word(ws, 0), result_word(ws, 1), result_word(ws, 2)};
+    FusedCtl *ctl[3] = {};
 
-    NB200_CUDA(cudaMemsetAsync(zeros, 0, sizeof(int32_t) * (size_t)most, stream));
-    {
-        LaunchScope scope("csf_fibre_setup", stream);
-        k_fill_float<<<grid(nja), NT, 0, stream>>>(ones, nja, 1.0f);
+    const LevelOffsets slices{a->j_ptr, b->j_ptr, ja, jb}, fibres{a->k_ptr, b->k_ptr, ka, kb};
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{nullptr, a->i_idx, nullptr, a->n_i}, CsrIn{nullptr, b->i_idx, nullptr, b->n_i}, RowCount{1}, a->dims[0],
+                           CsrOut{nullptr, z->i_idx, nullptr, nullptr, word[0]}, &slices, scratch_i, stream, &ctl[0])))
+        return st;
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{0, &ctl[0]->total}, a->dims[1],
+                           CsrOut{z->j_ptr, z->j_idx, nullptr, nullptr, word[1], ctl[0]}, &fibres, scratch_j, stream, &ctl[1])))
+        return st;
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total}, a->dims[2],
+                           CsrOut{z->k_ptr, z->k_idx, z->val, nullptr, word[2], ctl[1]}, nullptr, scratch_k, stream, &ctl[2])))
+        return st;
+    int64_t length[3];
+    for (int q = 0; q < 3; ++q) {
+        int device_status;
+        if ((st = wait_result_word(word[q], stream, &length[q], &device_status))) return st;
+        if (device_status != 0) {
+            NB200_CUDA(cudaMemcpyAsync(ws->host, ctl[q], sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
+            NB200_CUDA(cudaStreamSynchronize(stream));
+            FusedCtl h;
+            std::memcpy(&h, ws->host, sizeof(h));
+            return note_timeout(h.status.error, h.status.detail, "csf3 levels");
+        }
     }
-    {
-        LaunchScope scope("csf_fibre_setup", stream);
-        k_fill_float<<<grid(njb), NT, 0, stream>>>(twos, njb, 2.0f);
-    }
-    NB200_CUDA(cudaGetLastError());
-
-    // ---- 1. union of the fibre lists. They are DCSR matrices as they lie (slices x j): where the
-    // first extent allows scratch per slice number and the caller's i capacity covers the one-pass
-    // worst case, the DCSR union (CSR merge kernels, formats2d.cu) takes them; otherwise the route
-    // over expanded coordinates does, with every fibre as one entry.
-    const int64_t bound_i = std::min<int64_t>((int64_t)a->n_i + b->n_i, a->dims[0]);
-    nb200_csf3 fz = *z;
-    if (a->dims[0] <= DCSR_FIBRE_ROWS && cap_i >= bound_i) {
-        const nb200_dcsr da{a->dims[0], a->dims[1], a->n_i, nja, a->i_idx, a->j_ptr, a->j_idx, ones};
-        const nb200_dcsr db{b->dims[0], b->dims[1], b->n_i, njb, b->i_idx, b->j_ptr, b->j_idx, twos};
-        nb200_dcsr dz{0, 0, 0, 0, z->i_idx, z->j_ptr, z->j_idx, flags};
-        st = nb200_dcsr_add_f32_into(&da, &db, &dz, cap_i, std::min<int64_t>(cap_j, bound_j), stream);
-        fz.n_i = dz.n_i;
-        fz.n_j = dz.nnz;
-    } else {
-        nb200_csf3 fa = *a, fb = *b;
-        fa.n_k = nja, fa.k_ptr = nullptr, fa.k_idx = zeros, fa.val = ones;
-        fb.n_k = njb, fb.k_ptr = nullptr, fb.k_idx = zeros, fb.val = twos;
-        fz.k_ptr = zf_kptr, fz.k_idx = zf_kidx, fz.val = flags;
-        st = csf_add_expanded(&fa, &fb, &fz, cap_i, std::min<int64_t>(cap_j, bound_j), bound_j, stream, 0, true);
-    }
-    z->n_i = fz.n_i;
-    z->n_j = fz.n_j;
-    if (st != NB200_OK) return st;
-    const int32_t nz = fz.n_j;  // fibres of Z
-
-    // ---- 2. offsets of A's and B's entries over Z's fibres
-    NB200_CUDA(cudaMemsetAsync(scan_block, 0, sizeof(uint64_t) * ((size_t)tiles_cap + 8), stream));
-    {
-        LaunchScope scope("csf_fibre_offsets", stream);
-        k_fibre_offsets<<<(int)(((int64_t)nz + 1 + NT * OVT - 1) / (NT * OVT)), NT, 0, stream>>>(
-            flags, nz, a->k_ptr, b->k_ptr, off_a, off_b, scan_block + 4, reinterpret_cast<FusedCtl *>(scan_block));
-    }
-    NB200_CUDA(cudaGetLastError());
-    {   // a look-back of the offsets pass that gave up leaves offsets unwritten: they must not be used
-        NB200_CUDA(cudaMemcpyAsync(ws->host, scan_block, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-        NB200_CUDA(cudaStreamSynchronize(stream));
-        FusedCtl h;
-        std::memcpy(&h, ws->host, sizeof(h));
-        if (h.status.error != 0) return note_timeout(h.status.error, h.status.detail, "csf3 fibre offsets");
-    }
-
-    // ---- 3. the entries: a CSR union with one row per fibre of Z
-    const nb200_csr ma{nz, a->dims[2], a->n_k, off_a, a->k_idx, a->val};
-    const nb200_csr mb{nz, b->dims[2], b->n_k, off_b, b->k_idx, b->val};
-    nb200_csr mz{0, 0, 0, z->k_ptr, z->k_idx, z->val};
-    st = nb200_csr_add_f32_into(&ma, &mb, &mz, cap_k, stream);
-    z->n_k = mz.nnz;
-    return st;
+    if (length[2] & RW_HOLLOW) return NB200_OK;
+    z->n_i = (int32_t)(length[0] & (RW_HOLLOW - 1));
+    z->n_j = (int32_t)(length[1] & (RW_HOLLOW - 1));
+    z->n_k = (int32_t)length[2];
+    *done = true;
+    return NB200_OK;
 }
 
 int check_csf3(const nb200_csf3 *t) {
@@ -581,7 +419,11 @@ int csf_add_run(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, bool al
         return NB200_OK;
     }
 
-    st = two_level_pays(a, b) ? csf_add_two_level(a, b, z, cap_i, cap_j, cap_k, stream) : csf_add_expanded(a, b, z, cap_i, cap_j, cap_k, stream, 0);
+    // (the levels are written in one pass each: room for the worst case, or the other route)
+    bool done = false;
+    st = NB200_OK;
+    if (levels_pay(a, b) && cap_i >= bound_i && cap_j >= bound_j) st = csf_add_levels(a, b, z, stream, &done);
+    if (st == NB200_OK && !done) st = csf_add_expanded(a, b, z, cap_i, cap_j, stream);
     return st == NB200_OK ? NB200_OK : fail(st);
 }
 

@@ -14,7 +14,7 @@ namespace nb200 {
 constexpr int CSR_NT = 256;  // worker threads of a CSR tile CTA (one more warp scans)
 
 struct CsrIn {
-    const int32_t *rp;
+    const int32_t *rp;  // null: a single row that holds all entries
     const int32_t *col;
     const float *val;
     int32_t nnz;
@@ -28,7 +28,24 @@ struct CsrOut {
     // themselves. The partition kernel writes rows and a status of 0, the last tile the length, and
     // any tile whose bounded wait gives up (or a length beyond int32) raises the status.
     long long *result = nullptr;
+    // Calls that wait for their length: the result word in pinned host memory that the last tile writes.
+    unsigned long long *host = nullptr;
+    // ... and a control block of an earlier launch whose status and hollow flag the word reports too.
+    const FusedCtl *earlier = nullptr;
 };
+
+// What a merge of positions carries instead of values (offsets mode of the tile kernel): the operands'
+// entries stand for ranges of a lower level, entry p of A for [a[p], a[p + 1]). For every result entry u,
+// off_a[u] is the start of A's range where A holds the entry, else the start of its next one (the end of
+// the last range behind the last entry), so that off_a is a row-offset array over the result entries in
+// which an entry that A lacks is an empty row; off_b likewise. keep[u], when asked for, says that both hold
+// u with a range that is not empty. *hollow is raised if a result entry stands for no range but empty ones.
+struct LevelOffsets {
+    const int32_t *a = nullptr, *b = nullptr;
+    int32_t *off_a = nullptr, *off_b = nullptr, *keep = nullptr;
+};
+
+__device__ __forceinline__ int32_t row_offset(const CsrIn &m, int64_t r) { return m.rp ? ld_nc(m.rp + r) : r > 0 ? m.nnz : 0; }
 
 // Hardware barriers of the tile kernels: 0 = the whole CTA (__syncthreads), 1 = the worker
 // threads, 2 = workers arrive / the scan warp waits ("the tile's count is known").
@@ -55,6 +72,22 @@ inline int check_csr(const nb200_csr *m, bool need_arrays) {
     if (need_arrays && (!m->row_ptr || (m->nnz > 0 && (!m->col || !m->val)))) return NB200_E_BADARG;
     return NB200_OK;
 }
+
+// A row count that a call knows (`dev` null) or that an earlier launch on the stream leaves in device memory.
+struct RowCount {
+    int32_t value = 0;
+    const long long *dev = nullptr;
+    __device__ __forceinline__ int32_t get() const { return dev ? (int32_t)*dev : value; }
+};
+
+constexpr long long RW_HOLLOW = 1ll << 48;  // beside the length in a result word: the hollow flag of this or an earlier launch
+
+// One single-pass merge as part of a longer call: the partition and the tile kernel are queued and nothing
+// is waited for. `scratch` holds csr2_scratch_bytes(entries) bytes; the control block (length, status) that
+// *ctl then points to lies in it. With `levels` the offsets mode runs (values are not read).
+size_t csr2_scratch_bytes(int64_t entries);
+int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
+                 void *scratch, cudaStream_t stream, FusedCtl **ctl);
 
 // Two chained two-operand unions (A + B) + C through a pool intermediate: the route of callers
 // whose capacity is below the worst case, and of inputs the fused kernel does not take.

@@ -2,15 +2,15 @@
 // operands, as flat merge-path over the (row, column) order.
 //
 // The merged sequence of all stored entries of A and B, ordered by (row, column) with A first
-// on ties, is cut into tiles of TILE_STEP entries. A partition kernel finds every cut with
-// warp-wide 32-ary searches (rows on the summed row offsets, then the merge-path diagonal
-// inside the row). One CTA then owns one tile: the copy engine stages the tile's column indices
-// and values in shared memory, the columns are turned into composite (row-in-tile, column) keys
-// so that row boundaries need no special casing, the tile is split among the threads with an
-// in-shared-memory merge-path search, every thread merges its entries in registers (a bitonic
-// network), and the survivors are compacted through shared memory and written back coalesced.
-// Row offsets of the result are produced by the same pass: a tile owns the offsets of the rows
-// that begin inside it.
+// on ties, is cut into tiles of a few thousand entries. A partition kernel finds every cut with
+// k-ary searches (rows on the summed row offsets, then the merge-path diagonal inside the row).
+// One CTA then owns one tile: the copy engine stages the tile's column indices and values in shared
+// memory, every row that begins in the tile adds one to the upper bits of its first column (so a
+// key of the next entry is "row of the entry before it + this word"), every thread finds where its
+// share of the merged sequence begins with two searches in shared memory, and merges its entries
+// one result after the other, values included. The results are compacted through shared memory and
+// written back coalesced. Row offsets of the result are produced by the same pass: a tile owns the
+// offsets of the rows that begin inside it.
 //
 // Reference behaviour restated (not its code): partition src/backend/partition.cpp:813-993
 // (equal columns never split, :964-983), count src/backend/compute.cpp:152-271, fill
@@ -20,40 +20,24 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "csr_common.cuh"
-#include "warp_merge.cuh"
 
 namespace nb200 {
 
 namespace {
 
-// Tuning knobs (compile-time): merged entries per worker thread, and the number of CTAs per SM the
-// register allocator is asked to leave room for. The CTA always has 256 worker threads and one
-// scan warp.
-#ifndef CSR2_V
-#define CSR2_V 19            // merged entries per worker thread; (V + 1) rounded up to 4 must be an odd multiple of 4
-#endif
-#ifndef CSR2_LB_DEPTH
-#define CSR2_LB_DEPTH 1      // predecessors read per round of the look-back, in units of 32
-#endif
-#ifndef CSR2_LB_HURRY
-#define CSR2_LB_HURRY 1000  // ns between polls of the look-back once the tile itself waits for the result (faster polling
-                            // was measured: 64 ns costs 5 %, the poll traffic slows the workers of the other tiles)
-#endif
-#ifndef CSR2_LB_SLEEP
-#define CSR2_LB_SLEEP 2000  // nanoseconds between polls of the predecessors' tile words (shorter polls measurably slow the workers)
-#endif
-#ifndef CSR2_MIN_CTAS
-#define CSR2_MIN_CTAS 3
-#endif
 constexpr int NT = CSR_NT;
 
-// Tile cuts: for cut t, the row it falls in and the absolute positions in A and B.
-struct Cuts {
-    int32_t *row;
-    int32_t *a;
-    int32_t *b;
+// Tile cuts: for cut t, {the row it falls in, the absolute positions in A and B, unused}. A null
+// pointer stands for the two cuts of a single tile, which need no search.
+using Cuts = int4 *;
+
+// One tile: rows i0 (where it begins) .. i1 (where the next one begins), its entries in A and B.
+struct TileRange {
+    int32_t i0, i1, a0, b0;
+    int na, nb;
 };
 
 // Result words of an asynchronous call (CsrOut::result), written from inside the tile kernel.
@@ -66,342 +50,191 @@ __device__ __forceinline__ void publish_timeout(long long *result) {
     if (result) atomicMax(result + 1, (long long)NB200_E_TIMEOUT);
 }
 
+// All counts are in: the result length (negative after a give-up) goes to the control block and to
+// whoever waits for it. A tile that gave up wrote the error word before the count that let its
+// successors through, so the status read here covers every tile.
+__device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, long long total) {
+    __threadfence();
+    int status = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK;
+    if (total >= 0) {
+        ctl->total = total;
+        publish_length(Z.result, total);
+    } else {
+        publish_timeout(Z.result);
+    }
+    long long value = total < 0 ? 0 : total;
+    if (Z.earlier) {  // complete since before this launch; handed on, so that the last launch of a chain reports all of it
+        if (Z.earlier->status.error != 0) {
+            status = NB200_E_TIMEOUT;
+            ctl->status = Z.earlier->status;
+        }
+        if (Z.earlier->hollow) {
+            ctl->hollow = 1;
+            value |= RW_HOLLOW;
+        }
+    }
+    publish_result_word(Z.host, status, value);
+}
+
 // ------------------------------------------------------------------------- partition ----
 
-// One warp per cut. Cut t sits at merged position min(t * tile_step, total).
-__global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, int32_t rows, int64_t total,
+// Number of leading true values of a monotone pred over [lo, hi), returned as lo + count; G
+// neighbouring lanes search together, each group of a warp on its own range. All 32 lanes call this
+// together; a group that is done idles until the warp's last one is.
+template <int G, typename Pred>
+__device__ __forceinline__ uint32_t group_count_true(uint32_t lo, uint32_t hi, Pred pred) {
+    const int in_group = lane_id() & (G - 1), shift = lane_id() & ~(G - 1);
+    while (__any_sync(FULL_MASK, lo < hi)) {
+        const uint32_t step = lo < hi ? (hi - lo + G - 1) / G : 0u;
+        const uint32_t p = lo + (in_group + 1) * step - 1;
+        const bool ok = step > 0 && p < hi && pred(p);
+        const unsigned votes = __ballot_sync(FULL_MASK, ok);
+        const int c = __popc(G == 32 ? votes : (votes >> shift) & ((1u << (G & 31)) - 1u));
+        if (step > 0) {
+            lo += c * step;
+            hi = min(hi, lo + step - 1);
+        }
+    }
+    return lo;
+}
+
+// G lanes per cut. Cut t sits at merged position min(t * tile_step, total).
+template <int G>
+__global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count, uint32_t total,
                                                        int32_t tile_step, int32_t num_tiles, Cuts cuts, long long *result,
                                                        uint64_t *zero_block, int zero_words) {
-    if (result && blockIdx.x == 0 && threadIdx.x == 0) {  // the tile kernel that follows fills in the rest
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the tile kernel may take its places; it waits for the cuts
+    const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
+    const int32_t rows = row_count.get();
+    if (result && gid == 0) {  // the tile kernel that follows fills in the rest
         result[1] = NB200_OK;
         result[2] = rows;
     }
     // the control block and the tile words of the kernel that follows start from zero (the grid has at
-    // least 32 threads per tile word, so one word per thread covers them)
-    if (blockIdx.x * NT + threadIdx.x < zero_words) zero_block[blockIdx.x * NT + threadIdx.x] = 0;
-    const int t = (blockIdx.x * NT + threadIdx.x) >> 5;
-    if (t > num_tiles) return;
-    const int32_t a_base = ld_nc(A.rp), b_base = ld_nc(B.rp);
-    int64_t d = (int64_t)t * tile_step;
-    int32_t row, pa, pb;
-    if (t == 0) {
-        row = 0;
-        pa = a_base;
-        pb = b_base;
-    } else if (t == num_tiles || d >= total) {
-        row = rows;
-        pa = a_base + A.nnz;
-        pb = b_base + B.nnz;
-    } else {
-        // Row holding merged position d: the largest i with work(i) <= d, where work(i) is the
-        // number of entries of A and B in rows before i.
-        auto work = [&](int64_t i) -> int64_t {
-            return (int64_t)(ld_nc(A.rp + i) - a_base) + (int64_t)(ld_nc(B.rp + i) - b_base);
-        };
-        row = (int32_t)warp_last_true(0, (int64_t)rows - 1, [&](int64_t i) { return work(i) <= d; });
-        const int32_t a_lo = ld_nc(A.rp + row), a_hi = ld_nc(A.rp + row + 1);
-        const int32_t b_lo = ld_nc(B.rp + row), b_hi = ld_nc(B.rp + row + 1);
-        const int64_t dd = d - ((int64_t)(a_lo - a_base) + (int64_t)(b_lo - b_base));
-        const int64_t len_a = a_hi - a_lo, len_b = b_hi - b_lo;
-        // Merge-path diagonal dd inside the row: x entries of A and dd - x of B come first.
-        const int64_t x_lo = dd - len_b > 0 ? dd - len_b : 0;
-        const int64_t x_hi = dd < len_a ? dd : len_a;
-        const int64_t x = warp_count_true(x_lo, x_hi, [&](int64_t m) {
-            return ld_nc(A.col + a_lo + m) <= ld_nc(B.col + b_lo + (dd - 1 - m));
-        });
-        int64_t y = dd - x;
+    // least G >= 8 threads per tile word, so one word per thread covers them)
+    if (gid < zero_words) zero_block[gid] = 0;
+    const int t = (int)min(gid / G, (int64_t)num_tiles);  // spare groups repeat the last cut
+    const int32_t a_base = row_offset(A, 0), b_base = row_offset(B, 0);
+    const uint32_t d = (uint32_t)min((int64_t)t * tile_step, (int64_t)total);
+    const bool inner = t > 0 && t < num_tiles;
+    // Row holding merged position d: the largest i with work(i) <= d, where work(i) is the number of
+    // entries of A and B in rows before i; work(0) = 0, so it is the number of rows i >= 1 that satisfy it.
+    const int32_t row = (int32_t)group_count_true<G>(1, inner ? (uint32_t)rows : 1u, [&](uint32_t i) {
+        return (uint32_t)(row_offset(A, i) - a_base) + (uint32_t)(row_offset(B, i) - b_base) <= d;
+    }) - 1;
+    const int32_t a_lo = row_offset(A, row), a_hi = row_offset(A, row + 1);
+    const int32_t b_lo = row_offset(B, row), b_hi = row_offset(B, row + 1);
+    const int64_t dd = (int64_t)d - ((int64_t)(a_lo - a_base) + (int64_t)(b_lo - b_base));
+    const int64_t len_a = a_hi - a_lo, len_b = b_hi - b_lo;
+    // Merge-path diagonal dd inside the row: x entries of A and dd - x of B come first.
+    const uint32_t x_lo = (uint32_t)max((int64_t)0, dd - len_b), x_hi = (uint32_t)min(dd, len_a);
+    const uint32_t x = group_count_true<G>(x_lo, inner ? x_hi : x_lo, [&](uint32_t m) {
+        return ld_nc(A.col + a_lo + m) <= ld_nc(B.col + b_lo + (dd - 1 - m));
+    });
+    int64_t y = dd - x;
+    if (inner) {
         // Keep a column present in both operands on one side of the cut.
         if (x > 0 && y < len_b && ld_nc(A.col + a_lo + x - 1) == ld_nc(B.col + b_lo + y)) ++y;
-        pa = a_lo + (int32_t)x;
-        pb = b_lo + (int32_t)y;
     }
-    if (lane_id() == 0) {
-        cuts.row[t] = row;
-        cuts.a[t] = pa;
-        cuts.b[t] = pb;
+    if ((threadIdx.x & (G - 1)) == 0 && gid / G <= num_tiles) {
+        cuts[t] = inner ? make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0)
+                        : t == 0 ? make_int4(0, a_base, b_base, 0) : make_int4(rows, a_base + A.nnz, b_base + B.nnz, 0);
     }
 }
 
 // ------------------------------------------------------------------------ tile kernel ----
 
 
-// Tiles whose rows do not fit a 32-bit composite key (long runs of empty rows) take this body:
-// 64-bit keys (row in tile, column), plain loads, a sequential merge of VT entries per thread,
-// values fetched from global memory. It is rarely taken and kept simple; the common case is
-// csr2_tile_blocked below.
-template <int VT, int OP, int MODE>
-// (Not inlined, so the structs are taken by address: the kernel declares them __grid_constant__,
-// which lets that address point at the parameter space instead of a per-thread stack copy.)
-__device__ __noinline__ void csr2_tile_wide(const CsrIn &A, const CsrIn &B, const Cuts &cuts, const int t, int32_t *tile_count,
-                                            volatile uint64_t *tile_state, FusedCtl *ctl, const CsrOut &Z, unsigned char *smem_raw,
-                                            const int num_tiles, const int poll_limit) {
-    constexpr uint64_t INF = ~0ull;
-    __shared__ int scan_tmp[72];
-    __shared__ int thread_rank[NT];
-    __shared__ unsigned thread_emit[NT];
-    __shared__ long long s_base;
-    const int tid = threadIdx.x;
-    const int32_t i0 = cuts.row[t], i1 = cuts.row[t + 1];
-    const int32_t a0 = cuts.a[t], b0 = cuts.b[t];
-    const int na = cuts.a[t + 1] - a0, nb = cuts.b[t + 1] - b0;
-    const int n = na + nb;
+// Shared-memory plan of the tile body. The column words of both operands lie in one array: A's entry e at
+// word oa + e, B's at word ob + e, where oa and ob are chosen so that a global address on a 16-byte
+// boundary lands on a 16-byte boundary in shared memory too (what a bulk copy needs). Behind them, one
+// 16-bit word per result entry says where it comes from (offsets mode: two, for both operands).
+template <int VT, bool LEVELS>
+struct TilePlan {
+    static constexpr int CAP = NT * VT;         // most merged entries of one tile
+    static constexpr int SLOTS = CAP + 16;      // + alignment words of both operands and their sentinels
+    static constexpr size_t BYTES = (LEVELS ? 8 : 6) * (size_t)SLOTS;
+    static_assert(VT <= 31, "a thread's twins are kept in the lower 31 bits of a word");
+    static_assert(4 * SLOTS < 32768, "byte offsets of entries are kept in 15 bits");
+};
+constexpr uint32_t ROW_FAR = 0xffffu;
+constexpr int ROWS_CAP = 1024;  // row starts kept in shared memory; tiles with more rows search the offsets in global memory
+constexpr int GATHER = 8;       // result entries a thread fetches together
 
-    // Shared layout: keys of A, a sentinel, keys of B, a sentinel, then VT words of slack so
-    // that the merge may read a little past the end.
-    constexpr int KEY_SLOTS = NT * VT + 2 + VT;
-    uint64_t *kx = reinterpret_cast<uint64_t *>(smem_raw);
-    uint64_t *ky = kx + na + 1;
-    unsigned *kx_hi = reinterpret_cast<unsigned *>(kx) + 1, *ky_hi = reinterpret_cast<unsigned *>(ky) + 1;
-
-    for (int i = tid; i < na; i += NT) kx[i] = (uint64_t)(uint32_t)ld_nc(A.col + a0 + i);
-    for (int i = tid; i < nb; i += NT) ky[i] = (uint64_t)(uint32_t)ld_nc(B.col + b0 + i);
-    WorkerBar::sync();
-
-    // ---- mark the first entry of every row that starts inside the tile with its row number
-    // relative to i0 in the key's upper word (max wins where empty rows share a start), then spread
-    // it forward with a running maximum so that every entry carries its row.
-    for (int64_t r = (int64_t)i0 + 1 + tid; r <= i1; r += NT) {
-        const uint32_t rr = (uint32_t)(r - i0);
-        const int sa = ld_nc(A.rp + r) - a0, sb = ld_nc(B.rp + r) - b0;
-        if (sa < na) atomicMax(kx_hi + 2 * sa, rr);
-        if (sb < nb) atomicMax(ky_hi + 2 * sb, rr);
-    }
-    WorkerBar::sync();
-    {
-        // thread tid owns merged-array slots [tid*VT, tid*VT+VT): first the A part, then B
-        const int lo = tid * VT, hi = min(lo + VT, n);
-        unsigned ma = 0, mb = 0;
-        for (int i = lo; i < hi; ++i) {
-            if (i < na) ma = max(ma, kx_hi[2 * i]); else mb = max(mb, ky_hi[2 * (i - na)]);
-        }
-        unsigned ea, eb;
-        block_excl_max2<NT, WorkerBar>(ma, mb, reinterpret_cast<unsigned *>(scan_tmp), ea, eb);
-        for (int i = lo; i < hi; ++i) {
-            if (i < na) {
-                ea = max(ea, kx_hi[2 * i]);
-                kx_hi[2 * i] = ea;
-            } else {
-                eb = max(eb, ky_hi[2 * (i - na)]);
-                ky_hi[2 * (i - na)] = eb;
-            }
-        }
-        if (tid < VT + 1) ky[nb + tid] = INF;
-        if (tid == 0) kx[na] = INF;
-    }
-    WorkerBar::sync();
-
-    // ---- split the tile among threads: merge-path diagonal tid * VT, ties take A first
-    const int diag = min(tid * VT, n);
-    int x, y;
-    {
-        int lo = max(0, diag - nb), hi = min(diag, na);
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (kx[mid] <= ky[diag - 1 - mid]) lo = mid + 1; else hi = mid;
-        }
-        x = lo;
-        y = diag - lo;
-    }
-    const int x0 = x, y0 = y;
-
-    // ---- merge VT entries. Bit i of `from_a` says entry i came from A, of `twin` that the same
-    // column is in B too, of `emit` that the entry goes to the result.
-    uint32_t col[VT];
-    unsigned from_a = 0, twin = 0, emit = 0;
-    {
-        const int valid = min(VT, n - diag);
-        uint64_t hx = kx[x], hy = ky[y];
-        uint64_t last_x = x > 0 ? kx[x - 1] : INF;
-#pragma unroll
-        for (int i = 0; i < VT; ++i) {
-            const bool ok = i < valid;
-            const bool tx = hx <= hy;
-            const bool both = hx == hy;
-            col[i] = (uint32_t)(tx ? hx : hy);
-            const bool out = OP == OP_UNION ? (tx || hy != last_x) : (tx && both);
-            from_a |= (unsigned)tx << i;
-            twin |= (unsigned)(tx && both) << i;
-            emit |= (unsigned)(ok && out) << i;
-            last_x = tx ? hx : last_x;
-            x += tx;
-            y += !tx;
-            hx = kx[x];
-            hy = ky[y];
-        }
-    }
-
-    // ---- rank the survivors inside the tile
-    int total;
-    const int mine = __popc(emit);
-    const int rank = block_excl_sum<NT, WorkerBar>(mine, scan_tmp, total);  // syncs: key reads are done
-    if (MODE == MODE_COUNT) {
-        if (tid == 0) tile_count[t] = total;
-        return;
-    }
-
-    // ---- output base of the tile
-    long long base;
-    if (MODE == MODE_FILL) {
-        base = tile_count[t];  // exclusive prefix over tiles, made between the two passes
-    } else {
-        if (warp_id() == 0) {
-            if (lane_id() == 0) st_relaxed_gpu(tile_state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)total);
-            int64_t b = 0;
-            if (t > 0) {
-                b = lookback_predecessors(tile_state, t, &ctl->status, 32, nullptr, 64, poll_limit);
-                if (lane_id() == 0) st_relaxed_gpu(tile_state + t, LB_PREFIX | (uint64_t)(b < 0 ? 0 : b + total));
-            }
-            if (lane_id() == 0) s_base = b;
-        }
-    }
-    thread_rank[tid] = rank;
-    thread_emit[tid] = emit;
-    WorkerBar::sync();
-    if (MODE == MODE_FUSED) {
-        base = s_base;
-        if (base < 0) {  // a bounded wait gave up; the host reports it
-            if (tid == 0) publish_timeout(Z.result);
-            return;
-        }
-        if (t == num_tiles - 1 && tid == 0) {
-            ctl->total = base + total;
-            publish_length(Z.result, base + total);
-        }
-    }
-
-    // ---- row offsets. Result row r starts after every result entry of rows < r; inside this
-    // tile those are the survivors among the first d = (A entries before row r) + (B entries
-    // before row r) merged entries, read off the per-thread ranks. The tile owns rows
-    // i0+1 .. i1 (the next tile's first row).
-    for (int64_t r = (int64_t)i0 + 1 + tid; r <= i1; r += NT) {
-        const int d = (ld_nc(A.rp + r) - a0) + (ld_nc(B.rp + r) - b0);
-        const int owner = d / VT, off = d - owner * VT;
-        const int before = owner >= NT ? total : thread_rank[owner] + __popc(thread_emit[owner] & ((1u << off) - 1u));
-        Z.rp[r] = (int32_t)(base + before);
-    }
-    if (t == 0 && tid == 0) Z.rp[0] = 0;
-
-    // ---- fetch values, compact through shared memory (the staging arrays reuse the key words:
-    // the barriers above separate the last key read from the first write), store coalesced
-    int32_t *out_col = reinterpret_cast<int32_t *>(smem_raw);
-    float *out_val = reinterpret_cast<float *>(smem_raw) + KEY_SLOTS;
-    {
-        int r = rank, xi = x0, yi = y0;
-#pragma unroll
-        for (int i = 0; i < VT; ++i) {
-            const bool tx = (from_a >> i) & 1u;
-            const bool both = (twin >> i) & 1u;
-            if ((emit >> i) & 1u) {
-                float v;
-                if (OP == OP_UNION) {
-                    v = tx ? ld_nc(A.val + a0 + xi) : ld_nc(B.val + b0 + yi);
-                    if (both) v = v + ld_nc(B.val + b0 + yi);
-                } else {
-                    v = ld_nc(A.val + a0 + xi) * ld_nc(B.val + b0 + yi);
-                }
-                out_col[r] = (int32_t)col[i];
-                out_val[r] = v;
-                ++r;
-            }
-            xi += tx;
-            yi += !tx;
-        }
-    }
-    WorkerBar::sync();
-    for (int i = tid; i < total; i += NT) {
-        Z.col[base + i] = out_col[i];
-        Z.val[base + i] = out_val[i];
-    }
-}
-
-// Shared-memory plan of the thread-blocked tile body, in 4-byte words. Keys and values use the
-// same word positions: A's entry e sits at word oa + e and B's at word obv + e, where oa and obv
-// are chosen so that a global address on a 16-byte boundary lands on a 16-byte boundary in
-// shared memory too (what a bulk copy needs). The (column, value) staging pairs of the result reuse
-// the key words (the keys live in registers by then) and run on into extra words.
-template <int VT>
-struct BlockedPlan {
-    static constexpr int CAP = NT * VT;
-    static constexpr int NETV = VT + 1;                          // merge-network slots in use
-    static constexpr int CH = (VT + 1 + 3) & ~3;                 // words each thread scans
-    static constexpr int SLOTS = NT * CH + ((NETV + 4 + 3) & ~3);  // key words = value words
-    static constexpr int OUT = CAP + 8;                          // staging words per array
-    static constexpr size_t BYTES = 4 * (size_t)(2 * SLOTS + OUT);
-    // A thread's CH-word chunk is read and written as 16-byte vectors; an odd number of
-    // vectors per chunk keeps those accesses free of shared-memory bank conflicts.
-    static_assert((CH / 4) % 2 == 1, "choose VT so that (VT + 1) rounded up to 4 is an odd multiple of 4");
-    static_assert(NT * CH >= CAP + 12, "scan range must cover the padded tile");
-    static_assert(OUT <= SLOTS, "column staging must fit the key words it reuses");
+// Fixed shared memory of a tile (one block for both key widths).
+struct TileShared {
+    uint64_t mbar;
+    long long base;                 // output base of the tile
+    uint32_t rows[ROWS_CAP + 2];    // start of row r in the tile: A's in the lower half, B's in the upper
+    int trow[NT], wrow[NT / 32];    // the last row that starts at or before a thread's / between two warps' diagonals
+    int rank[NT];
+    unsigned twin[NT];
+    int wtotal[NT / 32];            // survivors of each warp
 };
 
-// The common tile body, thread-blocked form. Keys are 32-bit composites (row in tile, column, operand bit):
-//     key = ((row << cbits | column) << 1) | (0 for A, 1 for B)
-// so that one unsigned compare orders entries by (row, column) with A first on ties, and
-// two entries are the same position exactly when their keys differ in the last bit only.
+// The tile body. Keys order entries by (row in tile, column):
+//   narrow  32 bits, (row << cbits) | column. A staged word is a column; the first entry of a row also
+//           carries, above the column bits, how many rows begin there, so that the key after key k of the
+//           same operand is (k & row bits) + next word. That is all the row handling there is: no key array
+//           is ever written.
+//   WIDE    64 bits, row and column, for tiles that span too many rows for that (rows of an entry or two,
+//           long runs of empty rows): the row of an entry that begins one comes from its row mark.
+// A row mark is 16 bits per staged word, in the place of the source indices that come later: the last row
+// that begins at the entry (ROW_FAR: beyond 16 bits, looked up in the row offsets).
 //
-// The CTA has NT worker threads and one more warp, the scan warp. Workers stage the operands
-// with bulk copies, build keys (row marks, then a running maximum that every warp runs over its
-// own words), split the tile by merge-path, merge VT entries each in registers with a bitonic
-// network, rank the survivors (warp scans, one barrier) and compact them into shared memory. In
-// the single-pass mode the scan warp meanwhile turns the tile's count into its output base by
-// look-back over earlier tiles, so that this wait overlaps the workers' compaction. Six CTA-wide
-// barriers per tile.
-template <int VT, int OP, int MODE>
-__device__ __forceinline__ void csr2_tile_blocked(const CsrIn &A, const CsrIn &B, const Cuts &cuts, const int cbits, const int t,
-                                                  const int num_tiles, int32_t *tile_count, volatile uint64_t *tile_state,
-                                                  FusedCtl *ctl, const CsrOut &Z, unsigned char *smem_raw, uint64_t *mbar,
-                                                  const int poll_limit) {
-    using P = BlockedPlan<VT>;
+// What bounds this kernel is instruction issue and, for a tile, latency: the wait for its columns and the
+// wait for the counts of all earlier tiles, together half of its lifetime. So
+//   - the merge is sequential and moves columns only: one compare and at most two loads per result entry
+//     (a key-building pass, a register merge network and a per-entry value gather took four times the
+//     instructions), and it leaves a 16-bit source index per result entry;
+//   - the tile's count goes out right after it, and the values are fetched (from L2, where a prefetch has
+//     brought them meanwhile) while the count travels;
+//   - a tile needs 6 bytes of shared memory per entry instead of 16, so five CTAs share an SM.
+template <int VT, int OP, int MODE, bool LEVELS, bool WIDE>
+__device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const TileRange &tile, const int cbits, const int t,
+                                          const int num_tiles, int32_t *tile_count, const TileWords &words, FusedCtl *ctl,
+                                          const CsrOut &Z, const LevelOffsets &L, unsigned char *smem_raw, TileShared &sh,
+                                          const int poll_limit) {
+    using P = TilePlan<VT, LEVELS>;
+    using Key = typename std::conditional<WIDE, uint64_t, uint32_t>::type;
     constexpr int W = NT / 32;
-    __shared__ int thread_rank[NT];
-    __shared__ unsigned thread_emit[NT];
-    __shared__ int s_wtotal[W];  // survivors of each warp
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    constexpr int NETV = P::NETV;
+    constexpr Key END = WIDE ? (Key)~0ull : (Key)0x80000000u;  // after every key (narrow: keys are below 2^31), also with row bits added
     constexpr bool WRITES = MODE != MODE_COUNT;
-    constexpr uint32_t INF = 0xffffffffu;
-    __shared__ long long s_base;
-    __shared__ int s_total;
-    __shared__ int s_hurry;  // set once the tile's count is out: from then on the tile waits for its base
-    const int tid = threadIdx.x;
-    const bool scan_warp = tid >= NT;
-    const int32_t i0 = cuts.row[t], i1 = cuts.row[t + 1];
-    const int32_t a0 = cuts.a[t], b0 = cuts.b[t];
-    const int na = cuts.a[t + 1] - a0, nb = cuts.b[t + 1] - b0;
-    const int n = na + nb;
-    const uint32_t cmask = (1u << cbits) - 1u;
+    uint32_t *s_rows = sh.rows;
+    int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.rank, *s_wtotal = sh.wtotal;
+    unsigned *s_twin = sh.twin;
+    long long &s_base = sh.base;
+    uint64_t *mbar = &sh.mbar;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int na = tile.na, nb = tile.nb, n = na + nb;
+    const int nr = tile.i1 - tile.i0;  // rows 1 .. nr (relative) begin in this tile
+    const bool rows_fit = nr <= ROWS_CAP;
+    const uint32_t cmask = WIDE ? 0xffffffffu : (1u << cbits) - 1u;
+    uint32_t *keys = reinterpret_cast<uint32_t *>(smem_raw);
+    using Src = typename std::conditional<LEVELS, uint32_t, uint16_t>::type;
+    Src *src_of = reinterpret_cast<Src *>(smem_raw + 4 * P::SLOTS);
+    uint16_t *row_mark = reinterpret_cast<uint16_t *>(smem_raw + 4 * P::SLOTS);
+    auto word_at = [&](uint32_t byte) -> uint32_t & { return *reinterpret_cast<uint32_t *>(smem_raw + byte); };
 
-    // layout: values | keys | extra words. The (column, value) staging pairs of the result
-    // reuse the keys (in registers by then) and run on into the extra words.
-    float *vals = reinterpret_cast<float *>(smem_raw);
-    uint32_t *keys = reinterpret_cast<uint32_t *>(smem_raw) + P::SLOTS;
-    uint2 *out_pair = reinterpret_cast<uint2 *>(keys);
-    static_assert(P::SLOTS % 2 == 0 && P::SLOTS + P::OUT >= 2 * P::OUT, "staging pairs must fit keys + extra words, 8-byte aligned");
-
-    const int32_t *ga_col = A.col + a0, *gb_col = B.col + b0;
-    const float *ga_val = A.val + a0, *gb_val = B.val + b0;
+    const int32_t *ga_col = A.col + tile.a0, *gb_col = B.col + tile.b0;
+    const float *ga_val = A.val + tile.a0, *gb_val = B.val + tile.b0;
     const int ha = head_elems(ga_col), hb = head_elems(gb_col);
-    const int oa = (4 - ha) & 3;                 // word of A's entry 0
-    const int ob = (oa + na + 1 + 3) & ~3;       // first word of B's region (A's sentinel before it)
-    const int obv = ob + ((4 - hb) & 3);         // word of B's entry 0
-    const int scan_end = (obv + nb + 3) & ~3;
-    uint32_t *kx = keys + oa, *ky = keys + obv;
+    const int oa = (4 - ha) & 3;
+    const int ob = ((oa + na + 1 + 3) & ~3) + ((4 - hb) & 3);  // A's sentinel lies before it
 
-    // ---- stage the tile. One thread hands the 16-byte-aligned interior of each array to the
-    // copy engine; a few other threads load the ragged ends (at most 3 entries each side).
-    // Value arrays whose alignment differs from their column arrays' take plain loads.
-    const bool va_bulk = !WRITES || head_elems(ga_val) == ha, vb_bulk = !WRITES || head_elems(gb_val) == hb;
+    // ---- stage the columns. One thread hands the 16-byte-aligned interior of each array to the copy
+    // engine (and asks for the values' lines in L2); a few others load the ragged ends (at most 3 entries
+    // each side).
     const int head_a = min(na, ha), head_b = min(nb, hb);
     const int nva = (na - head_a) >> 2, nvb = (nb - head_b) >> 2;  // 16-byte vectors in the interior
     if (tid == 0) {
-        s_hurry = 0;
-        uint32_t bytes = 16u * (uint32_t)(nva + nvb);
-        if (WRITES) bytes += (va_bulk ? 16u * nva : 0u) + (vb_bulk ? 16u * nvb : 0u);
-        mbar_arrive_expect_tx(mbar, bytes);
-        if (nva) bulk_load(kx + head_a, ga_col + head_a, 16u * nva, mbar);
-        if (nvb) bulk_load(ky + head_b, gb_col + head_b, 16u * nvb, mbar);
-        if (WRITES && va_bulk && nva) bulk_load(vals + oa + head_a, ga_val + head_a, 16u * nva, mbar);
-        if (WRITES && vb_bulk && nvb) bulk_load(vals + obv + head_b, gb_val + head_b, 16u * nvb, mbar);
+        mbar_arrive_expect_tx(mbar, 16u * (uint32_t)(nva + nvb));
+        if (nva) bulk_load(keys + oa + head_a, ga_col + head_a, 16u * nva, mbar);
+        if (nvb) bulk_load(keys + ob + head_b, gb_col + head_b, 16u * nvb, mbar);
+        if (WRITES && OP == OP_UNION && !LEVELS) {
+            prefetch_l2(ga_val, na);
+            prefetch_l2(gb_val, nb);
+        }
     }
     if (tid >= 32 && tid < 32 + 12) {  // ragged ends: 3 head + 3 tail slots for A, then for B
         const int k = tid - 32;
@@ -409,185 +242,166 @@ __device__ __forceinline__ void csr2_tile_blocked(const CsrIn &A, const CsrIn &B
         const int e = is_b ? k - 6 : k;
         const int count = is_b ? nb : na, head = is_b ? head_b : head_a, nv = is_b ? nvb : nva;
         const int idx = e < 3 ? e : head + 4 * nv + (e - 3);
-        const bool live = e < 3 ? e < head : idx < count;
-        if (live) {
-            const int w = (is_b ? obv : oa) + idx;
-            keys[w] = (uint32_t)ld_nc((is_b ? gb_col : ga_col) + idx);
-            if (WRITES && (is_b ? vb_bulk : va_bulk)) vals[w] = ld_nc((is_b ? gb_val : ga_val) + idx);
-        }
+        if (e < 3 ? e < head : idx < count) keys[(is_b ? ob : oa) + idx] = (uint32_t)ld_nc((is_b ? gb_col : ga_col) + idx);
     }
-    if (WRITES && !va_bulk && !scan_warp) for (int i = tid; i < na; i += NT) vals[oa + i] = ld_nc(ga_val + i);
-    if (WRITES && !vb_bulk && !scan_warp) for (int i = tid; i < nb; i += NT) vals[obv + i] = ld_nc(gb_val + i);
-    // padding words that precede live keys must read as "no row mark"; the end-of-list
-    // sentinels are all-ones, which the row spreading below keeps above every live key
-    if (tid >= 64 && tid < 64 + 3) { if (tid - 64 < oa) keys[tid - 64] = 0u; }
-    if (tid >= 68 && tid < 68 + 3) { if (ob + (tid - 68) < obv) keys[ob + (tid - 68)] = 0u; }
-    if (tid == 72) keys[oa + na] = INF;
-    if (tid >= 76 && tid < 76 + NETV + 1) keys[obv + nb + (tid - 76)] = INF;
-    static_assert(76 + NETV + 1 <= NT, "sentinel writers must be worker threads");
+    if (tid == 64) keys[oa + na] = (uint32_t)END;
+    if (tid == 65) keys[ob + nb] = (uint32_t)END;
+    s_trow[tid] = 0;
+    if (WIDE) for (int i = tid; i < P::SLOTS / 2; i += NT) reinterpret_cast<uint32_t *>(row_mark)[i] = 0u;
+    if (tid < W) s_wrow[tid] = 0;
 
-    // row offsets of the first row this thread looks after (rows i0+1 .. i1 are spread over the
-    // workers); kept in registers for the row-offset pass at the end
-    const int64_t my_row = (int64_t)i0 + 1 + tid;
-    int32_t my_sa = 0, my_sb = 0;
-    if (!scan_warp && my_row <= i1) {
-        my_sa = ld_nc(A.rp + my_row) - a0;
-        my_sb = ld_nc(B.rp + my_row) - b0;
+    // ---- row starts (relative to the tile), while the copies fly. Row 0 is the one the tile begins in.
+    auto global_start = [&](int r) -> uint32_t {
+        return (uint32_t)(row_offset(A, (int64_t)tile.i0 + r) - tile.a0) | (uint32_t)(row_offset(B, (int64_t)tile.i0 + r) - tile.b0) << 16;
+    };
+    if (rows_fit) {
+        for (int r = tid; r <= nr; r += NT) s_rows[r] = r == 0 ? 0u : global_start(r);
+        if (tid == 0) s_rows[nr + 1] = (uint32_t)na | (uint32_t)nb << 16;
     }
-    // ---- the row (relative to i0) that the first key word of this warp's scan region belongs to:
-    // the last row that starts at or before it. Regions that begin with an operand's first entry,
-    // or in padding before it, start from row 0 of the tile. (Found while the copies fly.)
-    const int w0 = wid * 32 * P::CH;
-    const bool region_in_a = w0 < ob;
-    unsigned carry = 0;
-    if (!scan_warp) {
-        const int pos = region_in_a ? w0 - oa : w0 - obv;
-        if (pos > 0 && i1 > i0) {
-            const int32_t *rp = region_in_a ? A.rp : B.rp;
-            const int32_t start = region_in_a ? a0 : b0;
-            carry = (unsigned)(warp_last_true(i0, i1, [&](int64_t r) { return ld_nc(rp + r) - start <= pos; }) - i0);
-        }
-    }
+    auto row_start = [&](int r) -> uint32_t {  // packed like s_rows, r in [0, nr + 1]
+        if (rows_fit) return s_rows[r];
+        return r == 0 ? 0u : r > nr ? (uint32_t)na | (uint32_t)nb << 16 : global_start(r);
+    };
     const bool landed = mbar_wait_bounded(mbar, 0, MBAR_POLL_LIMIT);
     if (!__syncthreads_and(landed)) {  // the copies did not land in time: report, touch nothing
         if (tid == 0) {
             if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
             publish_timeout(Z.result);
-            if (MODE == MODE_FUSED) tile_state[t] = LB_PREFIX;  // successors must not wait on this tile
+            __threadfence();
+            if (MODE == MODE_FUSED) {
+                publish_count(words, t, 0);  // successors must not wait on this tile
+                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+            }
             mbar_wait_bounded(mbar, 0, MBAR_POLL_LIMIT);        // second bounded wait for copies in flight
         }
         return;
     }
 
-    if (scan_warp) {
-        // ---- scan warp: the output base of the tile is the sum of the counts of all earlier
-        // tiles, which does not depend on this tile's own count. So the walk over the
-        // predecessors' words starts now, while the workers are still merging, and is usually
-        // over by the time they know their count.
-        if (MODE != MODE_FUSED) return;
-        const int64_t bse = t == 0 ? 0 : lookback_predecessors<CSR2_LB_DEPTH>(tile_state, t, &ctl->status, CSR2_LB_SLEEP, &s_hurry,
-                                                                             CSR2_LB_HURRY, poll_limit);
-        CountBar::sync();  // the workers have published the tile's count by now
-        const int total = s_total;
-        if (lane_id() == 0) {
-            if (t > 0) st_relaxed_gpu(tile_state + t, LB_PREFIX | (uint64_t)(bse < 0 ? 0 : bse + total));
-            s_base = bse;
-            if (bse < 0) publish_timeout(Z.result);
-            if (bse >= 0 && t == num_tiles - 1) {
-                ctl->total = bse + total;
-                publish_length(Z.result, bse + total);
-            }
+    // ---- every row that begins in the tile adds one above the column bits of its first entry (several
+    // where empty rows share a start), and the last row that starts at or before a thread's diagonal is
+    // noted for that thread, and for its warp
+    for (int r = 1 + tid; r <= nr; r += NT) {
+        const uint32_t w = row_start(r), w_next = row_start(r + 1);
+        const int sa = (int)(w & 0xffffu), sb = (int)(w >> 16);
+        if (!WIDE) {
+            if (sa < na) atomicAdd(keys + oa + sa, 1u << cbits);
+            if (sb < nb) atomicAdd(keys + ob + sb, 1u << cbits);
         }
-        __syncthreads();
-        return;
-    }
-
-    // ---- mark the first entry of every row that starts inside the tile with its row number
-    // relative to i0, in the bits above the column (max wins where empty rows share a start)
-    for (int64_t r = my_row; r <= i1; r += NT) {
-        const uint32_t rr = (uint32_t)(r - i0);
-        const int sa = r == my_row ? my_sa : ld_nc(A.rp + r) - a0;
-        const int sb = r == my_row ? my_sb : ld_nc(B.rp + r) - b0;
-        if (sa < na) atomicMax(kx + sa, (rr << cbits) | (kx[sa] & cmask));
-        if (sb < nb) atomicMax(ky + sb, (rr << cbits) | (ky[sb] & cmask));
-    }
-    WorkerBar::sync();
-
-    // ---- spread the marks forward (running maximum) so that every key carries its row, and
-    // append the operand bit. Each thread owns CH consecutive words, each warp 32 * CH, and a warp
-    // needs nothing from the other warps (its region's first row came from the search above); A's
-    // words and B's words run separately.
-    {
-        constexpr int NV = P::CH / 4;
-        const int w_base = tid * P::CH;
-        uint4 q[NV];
-        unsigned ma = 0, mb = 0;
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int w = w_base + 4 * j;
-            q[j] = w < scan_end ? *reinterpret_cast<const uint4 *>(keys + w) : make_uint4(0, 0, 0, 0);
-            const unsigned m = max(max(q[j].x & ~cmask, q[j].y & ~cmask), max(q[j].z & ~cmask, q[j].w & ~cmask));
-            if (w < ob) ma = max(ma, m); else mb = max(mb, m);
-        }
-        // running maximum over the lanes before this one, on top of the row the warp's region starts in
-        unsigned ea = __shfl_up_sync(FULL_MASK, warp_incl_max(ma), 1), eb = __shfl_up_sync(FULL_MASK, warp_incl_max(mb), 1);
-        if (lane == 0) ea = eb = 0u;
-        if (region_in_a) ea = max(ea, carry << cbits); else eb = max(eb, carry << cbits);
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const int w = w_base + 4 * j;
-            const bool in_a = w < ob;
-            const unsigned src = in_a ? 0u : 1u;
-            unsigned run = in_a ? ea : eb;
-            uint4 v = q[j];
-            run = max(run, v.x & ~cmask); v.x = ((run | (v.x & cmask)) << 1) | src;
-            run = max(run, v.y & ~cmask); v.y = ((run | (v.y & cmask)) << 1) | src;
-            run = max(run, v.z & ~cmask); v.z = ((run | (v.z & cmask)) << 1) | src;
-            run = max(run, v.w & ~cmask); v.w = ((run | (v.w & cmask)) << 1) | src;
-            if (in_a) ea = run; else eb = run;
-            if (w < scan_end) *reinterpret_cast<uint4 *>(keys + w) = v;
+        const uint16_t mark = (uint16_t)min((uint32_t)r, ROW_FAR);
+        if (sa < (int)(w_next & 0xffffu)) row_mark[oa + sa] = mark;  // row r holds entries of A: nothing else marks that word
+        if (sb < (int)(w_next >> 16)) row_mark[ob + sb] = mark;
+        const int q = (sa + sb + VT - 1) / VT;  // the first thread whose diagonal is not before this row
+        const int q_next = r < nr ? ((int)(w_next & 0xffffu) + (int)(w_next >> 16) + VT - 1) / VT : NT + 32;
+        if (q < NT && q_next != q) {
+            s_trow[q] = r;
+            if ((q_next >> 5) != (q >> 5)) s_wrow[q >> 5] = r;
         }
     }
-    WorkerBar::sync();
+    __syncthreads();
 
-    // ---- split the tile among threads: merge-path diagonal tid * VT (the operand bit makes
-    // an A entry smaller than the B entry at the same position, so ties take A first)
+    // ---- where this thread's share begins: the row of merged position tid * VT, then the merge-path
+    // diagonal inside that row (ties take A first; a column both operands hold stays on one side)
     const int diag = min(tid * VT, n);
-    int x0;
-    {
-        int lo = max(0, diag - nb), hi = min(diag, na);
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (kx[mid] < ky[diag - 1 - mid]) lo = mid + 1; else hi = mid;
+    int x, y, shifted = 0, row;
+    Key ka = END, kb = END;
+    int row_a = 0, row_b = 0;  // WIDE: row of each head
+    // row of the entry at staged word `at`, position `pos` of its operand, that begins one after row `from`
+    auto marked_row = [&](const int at, const int pos, const int from, const int shift) -> int {
+        const uint32_t mark = row_mark[at];
+        if (mark != ROW_FAR) return (int)mark;
+        int r = from + 1, top = nr;
+        while (r < top) {  // the last row that starts at or before pos
+            const int mid = (r + top + 1) >> 1;
+            if ((int)((row_start(mid) >> shift) & 0xffffu) <= pos) r = mid; else top = mid - 1;
         }
-        x0 = lo;
-    }
-    const int y0 = diag - x0;
-    const int cnt = min(VT, n - diag);
-    // the next thread's split: from the next lane; the warp's last lane takes the split of the
-    // warp's end diagonal, which the 32 lanes find together
-    int x1 = __shfl_down_sync(FULL_MASK, x0, 1);
+        return r;
+    };
     {
-        const int x_end = warp_count_cut(kx, na, ky, nb, min((wid + 1) * 32 * VT, n));
-        if (lane == 31) x1 = x_end;
-    }
-    const int a = min(x1, x0 + cnt) - x0, b = cnt - a;
-
-    // ---- merge in registers: A's entries ascending, the successor of the thread's range, an
-    // all-ones plateau, B's entries descending -- a bitonic sequence -- through a merge network
-    uint32_t r[NETV];
-    {
-        const uint32_t succ = min(kx[x0 + a], ky[y0 + b]);  // next merged key after this thread's range
-#pragma unroll
-        for (int i = 0; i < NETV; ++i) {
-            const bool is_a = i < a, is_b = i >= NETV - b;
-            const uint32_t *p = is_a ? kx + x0 + i : ky + y0 + (NETV - 1 - i);
-            const uint32_t v = *p;  // stays inside the slack-padded key array either way
-            r[i] = (is_a || is_b) ? v : (i == a ? succ : INF);
+        row = (int)warp_incl_max((unsigned)s_trow[tid]);
+        row = max(row, (int)__reduce_max_sync(FULL_MASK, lane < wid ? (unsigned)s_wrow[lane & (W - 1)] : 0u));
+        const uint32_t w0 = row_start(row), w1 = row_start(row + 1);
+        const int a_lo = (int)(w0 & 0xffffu), b_lo = (int)(w0 >> 16), a_hi = (int)(w1 & 0xffffu), b_hi = (int)(w1 >> 16);
+        const int dd = diag - a_lo - b_lo;
+        int lo = max(0, dd - (b_hi - b_lo)), up = min(dd, a_hi - a_lo);
+        const uint32_t *ca = keys + oa + a_lo, *cb = keys + ob + b_lo + dd - 1;
+        while (lo < up) {
+            const int mid = (lo + up) >> 1;
+            if ((ca[mid] & cmask) <= (cb[-mid] & cmask)) lo = mid + 1; else up = mid;
+        }
+        x = a_lo + lo;
+        y = b_lo + dd - lo;
+        if (lo > 0 && y < b_hi && ((keys[oa + x - 1] ^ keys[ob + y]) & cmask) == 0u) {
+            ++y;
+            shifted = 1;
+        }
+        // keys of the two heads. A head beyond this row begins a later row of its operand.
+        auto head_key = [&](const int at, const int pos, const int end, const int count, const int shift, int &head_row) -> Key {
+            head_row = row;
+            if (pos >= count) return END;
+            if (pos >= end) head_row = marked_row(at, pos, row, shift);
+            return WIDE ? (Key)((uint64_t)(uint32_t)head_row << 32 | keys[at]) : (Key)((uint32_t)head_row << cbits | (keys[at] & cmask));
+        };
+        if (diag < n) {
+            ka = head_key(oa + x, x, a_hi, na, 0, row_a);
+            kb = head_key(ob + y, y, b_hi, nb, 16, row_b);
         }
     }
-    const uint32_t prev_a = x0 > 0 ? kx[x0 - 1] : 0u;  // only an A entry can pair with a B entry
-    bitonic_merge<NETV>(r);
 
-    // Bit i of `from_a`: entry i came from A; of `same`: entries i and i+1 are one position (an A
-    // entry and its B twin); of `emit`: entry i goes to the result.
-    unsigned from_a = 0, same = 0;
+    // ---- merge, one result entry per step: take the smaller head, or both where they are equal. Offsets are
+    // in bytes from the start of the column words. src[i]: the entry step i took (A's where both), with
+    // the top bit set where it took both; in the offsets mode both heads, bit 0 of each half set where it was taken.
+    const uint32_t pa0 = 4u * (uint32_t)(oa + x), pb0 = 4u * (uint32_t)(ob + y);
+    uint32_t src[VT];
+    unsigned twin = 0;  // bit i: step i took an entry of each operand
+    int steps = 0;
+    {
+        uint32_t pa = pa0, pb = pb0;
+        const uint32_t end = 4u * (uint32_t)(oa + ob + min(tid * VT + VT, n));  // pa + pb once the share is done
 #pragma unroll
-    for (int i = 0; i < VT; ++i) {
-        from_a |= (~r[i] & 1u) << i;
-        same |= (unsigned)((r[i] ^ r[i + 1]) == 1u) << i;
+        for (int i = 0; i < VT; ++i) {
+            const bool go = pa + pb < end;
+            const bool ta = go && ka <= kb, tb = go && kb <= ka;
+            const uint32_t row_bits = (uint32_t)min(ka, kb) & ~cmask;
+            if (LEVELS) {
+                src[i] = (pa | (ta ? 1u : 0u)) | (pb | (tb ? 1u : 0u)) << 16;
+                if (ta && tb) twin |= 1u << i;
+            } else {
+                src[i] = ta ? pa : pb;
+                if (ta && tb) {
+                    twin |= 1u << i;
+                    src[i] |= 0x8000u;
+                }
+            }
+            if (ta) {
+                pa += 4;
+                if (!WIDE) {
+                    ka = (Key)(row_bits + word_at(pa));
+                } else {
+                    const int at = (int)(pa >> 2), pos = at - oa;
+                    if (pos < na && row_mark[at]) row_a = marked_row(at, pos, row_a, 0);
+                    ka = pos < na ? (Key)(((uint64_t)(uint32_t)row_a << 32) | word_at(pa)) : END;
+                }
+            }
+            if (tb) {
+                pb += 4;
+                if (!WIDE) {
+                    kb = (Key)(row_bits + word_at(pb));
+                } else {
+                    const int at = (int)(pb >> 2), pos = at - ob;
+                    if (pos < nb && row_mark[at]) row_b = marked_row(at, pos, row_b, 16);
+                    kb = pos < nb ? (Key)(((uint64_t)(uint32_t)row_b << 32) | word_at(pb)) : END;
+                }
+            }
+            if (go) ++steps;
+        }
     }
-    const unsigned live = (1u << cnt) - 1u;
-    const unsigned dup = (same << 1) | (unsigned)(x0 > 0 && (prev_a ^ r[0]) == 1u);  // B entries whose A twin precedes them
-    const unsigned twin = same & from_a & live;
-    const unsigned emit = OP == OP_UNION ? (live & ~dup) : twin;
-    static_assert(VT < 32, "entry masks are 32 bits wide");
 
     // ---- rank the survivors inside the tile
-    const int mine = __popc(emit);
+    const int mine = OP == OP_UNION ? steps : __popc(twin);
     const int incl = warp_incl_sum(mine);
     if (lane == 31) s_wtotal[wid] = incl;
-    WorkerBar::sync();  // also retires every thread's key reads: the staging pairs may overwrite the keys
+    s_twin[tid] = twin | (unsigned)shifted << 31;
+    __syncthreads();  // also retires the merge of every thread: words of consumed twins may change from here on
     int total = 0, wbase = 0;
 #pragma unroll
     for (int w = 0; w < W; ++w) {
@@ -600,122 +414,235 @@ __device__ __forceinline__ void csr2_tile_blocked(const CsrIn &A, const CsrIn &B
         if (tid == 0) tile_count[t] = total;
         return;
     }
-    thread_rank[tid] = rank;
-    thread_emit[tid] = emit;
-    if (MODE == MODE_FUSED) {
-        if (tid == 0) {
-            // successors can add this tile's count from here on
-            st_relaxed_gpu(tile_state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)total);
-            s_total = total;
-            *(volatile int *)&s_hurry = 1;
-        }
-        __threadfence_block();
-        CountBar::arrive();  // the scan warp turns the count into the tile's inclusive prefix
-    }
+    if (MODE == MODE_FUSED && tid == 0) publish_count(words, t, total);
+    s_rank[tid] = rank;
 
-    // ---- compact (column, value) pairs of the survivors into the staging array. Entry i of the
-    // thread came from A iff its key's operand bit is clear; its value sits at A's start + (A
-    // entries before it) or B's start + (B entries before it), and an A entry's twin is the
-    // next B entry.
+    // ---- compact: source of every result entry, in order. A twin's A word now points to its B word
+    // (byte offsets: step i began at pa0 + pb0 + 4 (i + twins before it)).
+    if (!LEVELS && __any_sync(FULL_MASK, twin != 0u)) {
+#pragma unroll
+        for (int i = 0; i < VT; ++i)
+            if ((twin >> i) & 1u) {
+                const uint32_t at = src[i] & 0x7fffu;
+                word_at(at) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - at;
+            }
+    }
     {
-        const float *pa = vals + oa + x0, *pb = vals + obv + y0;
-        uint2 *po = out_pair + rank;
-        int ca = 0;  // A entries among the thread's first i entries
+        Src *to = src_of + rank;
 #pragma unroll
         for (int i = 0; i < VT; ++i) {
-            const bool tx = (r[i] & 1u) == 0u;
             if (OP == OP_UNION) {
-                float v = *(tx ? pa + ca : pb + (i - ca));
-                if ((twin >> i) & 1u) v = v + pb[i - ca];  // an A entry whose twin is the next B entry
-                if ((emit >> i) & 1u) {
-                    *po = make_uint2((r[i] >> 1) & cmask, __float_as_uint(v));
-                    ++po;
-                }
-            } else if ((emit >> i) & 1u) {  // intersection: only the twins need their values
-                *po = make_uint2((r[i] >> 1) & cmask, __float_as_uint(pa[ca] * pb[i - ca]));
-                ++po;
+                if (i < steps) to[i] = (Src)src[i];
+            } else if ((twin >> i) & 1u) {
+                *to++ = (Src)src[i];
             }
-            ca += tx;
         }
     }
+    __syncthreads();
+
+    // ---- fetch columns and values, result entries q * NT + tid; the first batch before the output base is
+    // asked for
+    const char *va = reinterpret_cast<const char *>(ga_val) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(gb_val) - 4 * (int64_t)ob;
+    const uint32_t first_b = 4u * (uint32_t)ob;
+    uint32_t col[GATHER];
+    float val[GATHER];
+    auto gather = [&](const int q0) {
+        uint32_t s[GATHER];
+        uint32_t any = 0;
+#pragma unroll
+        for (int g = 0; g < GATHER; ++g) {
+            const int o = (q0 + g) * NT + tid;
+            s[g] = q0 + g < VT && o < total ? (uint32_t)src_of[o] : 4u * (uint32_t)oa;  // spare slots read A's first word (or its sentinel)
+            any |= s[g];
+        }
+        if (OP == OP_INTERSECT || __any_sync(FULL_MASK, (any & 0x8000u) != 0u)) {
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                const bool both = (s[g] & 0x8000u) != 0u;
+                const uint32_t at = s[g] & 0x7fffu;
+                const uint32_t w = word_at(at);
+                const uint32_t other = both ? w : at;
+                col[g] = word_at(other) & cmask;
+                const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
+                float v = 0.0f;
+                if (ok) v = __ldg(reinterpret_cast<const float *>((at >= first_b ? vb : va) + at));
+                if (both) {
+                    const float u = __ldg(reinterpret_cast<const float *>(vb + other));
+                    v = OP == OP_UNION ? v + u : v * u;
+                }
+                val[g] = v;
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
+                col[g] = word_at(s[g]) & cmask;
+                val[g] = ok ? __ldg(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
+            }
+        }
+    };
+    if (!LEVELS) gather(0);
 
     // ---- output base of the tile
-    if (MODE == MODE_FUSED) __syncthreads(); else WorkerBar::sync();
+    if (MODE == MODE_FUSED && wid == 0) {
+        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, poll_limit);
+        if (lane == 0) {
+            s_base = b;
+            if (b < 0) publish_timeout(Z.result);
+            if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) finish_total(ctl, Z, b < 0 ? b : b + total);
+        }
+    }
+    __syncthreads();
     const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
     if (base < 0) return;  // a bounded wait gave up; the host reports it
 
-    // ---- row offsets. Result row r starts after every result entry of rows < r; inside this
-    // tile those are the survivors among the first d = (A entries before row r) + (B entries
-    // before row r) merged entries, read off the per-thread ranks. The tile owns rows
-    // i0+1 .. i1 (the next tile's first row).
-    for (int64_t rw = my_row; rw <= i1; rw += NT) {
-        const int sa = rw == my_row ? my_sa : ld_nc(A.rp + rw) - a0;
-        const int sb = rw == my_row ? my_sb : ld_nc(B.rp + rw) - b0;
-        const int d = sa + sb;
-        const int owner = d / VT, off = d - owner * VT;
-        const int before = owner >= NT ? total : thread_rank[owner] + __popc(thread_emit[owner] & ((1u << off) - 1u));
-        Z.rp[rw] = (int32_t)(base + before);
+    if (LEVELS) {
+        // ---- offsets mode: the column and the two range starts of every result entry
+        for (int o = tid; o < total; o += NT) {
+            const uint32_t s = src_of[o];
+            const bool ta = s & 1u, tb = (s >> 16) & 1u;
+            const uint32_t pa = s & 0xfffcu, pb = (s >> 16) & 0xfffcu;
+            const int32_t *la = L.a + tile.a0 + ((int)(pa >> 2) - oa), *lb = L.b + tile.b0 + ((int)(pb >> 2) - ob);
+            const int32_t at_a = ld_nc(la), at_b = ld_nc(lb);
+            const bool full_a = ta && ld_nc(la + 1) > at_a, full_b = tb && ld_nc(lb + 1) > at_b;
+            Z.col[base + o] = (int32_t)(word_at(ta ? pa : pb) & cmask);
+            L.off_a[base + o] = at_a;
+            L.off_b[base + o] = at_b;
+            if (L.keep) L.keep[base + o] = full_a && full_b;
+            if (!full_a && !full_b) ctl->hollow = 1;
+        }
+        if (t == num_tiles - 1 && tid == 0) {
+            L.off_a[base + total] = ld_nc(L.a + tile.a0 + na);
+            L.off_b[base + total] = ld_nc(L.b + tile.b0 + nb);
+        }
+    } else {
+    // ---- store the tile, coalesced
+    int32_t *gz_col = Z.col + base + tid;
+    float *gz_val = Z.val + base + tid;
+#pragma unroll
+    for (int q0 = 0; q0 < VT; q0 += GATHER) {
+        if (q0 > 0) {
+            if (q0 * NT >= total) break;
+            gather(q0);
+        }
+#pragma unroll
+        for (int g = 0; g < GATHER; ++g) {
+            if (q0 + g < VT && (q0 + g) * NT + tid < total) {
+                gz_col[(q0 + g) * NT] = (int32_t)col[g];
+                gz_val[(q0 + g) * NT] = val[g];
+            }
+        }
+    }
+    }
+
+    // ---- row offsets. Result row r starts after every result entry of rows < r; inside this tile those
+    // are the survivors among the first d = (A entries before row r) + (B entries before row r) merged
+    // entries: all of them up to the thread that holds position d, then, in that thread, a step per entry
+    // except that a twin step covers two. The tile owns rows i0+1 .. i1 (the next tile's first row).
+    if (LEVELS && !Z.rp) return;
+    for (int r = 1 + tid; r <= nr; r += NT) {
+        const uint32_t w = row_start(r);
+        const int d = (int)((w & 0xffffu) + (w >> 16));
+        const int owner = d / VT;
+        int before = total;
+        if (owner < NT) {
+            const unsigned info = s_twin[owner];
+            const int m = d - owner * VT - (int)(info >> 31);  // merged entries of that thread before the row
+            unsigned left = info & 0x7fffffffu;
+            int pairs = 0;  // twins among them
+            while (left) {
+                const int at = __ffs(left) - 1;
+                if (at + pairs + 2 > m) break;
+                ++pairs;
+                left &= left - 1u;
+            }
+            before = s_rank[owner] + (OP == OP_UNION ? m - pairs : pairs);
+        }
+        Z.rp[tile.i0 + (int64_t)r] = (int32_t)(base + before);
     }
     if (t == 0 && tid == 0) Z.rp[0] = 0;
-
-    // ---- store the compacted tile, coalesced
-    int32_t *gz_col = Z.col + base;
-    float *gz_val = Z.val + base;
-    for (int i = tid; i < total; i += NT) {
-        const uint2 p = out_pair[i];
-        gz_col[i] = (int32_t)p.x;
-        gz_val[i] = __uint_as_float(p.y);
-    }
 }
 
-template <int V, int OP, int MODE>
-__global__ void __launch_bounds__(NT + 32, CSR2_MIN_CTAS) k_csr2_tile(const __grid_constant__ CsrIn A, const __grid_constant__ CsrIn B,
-                                                                         const __grid_constant__ Cuts cuts, int cbits, int32_t *tile_count,
-                                                                         uint64_t *tile_state, FusedCtl *ctl,
-                                                                         const __grid_constant__ CsrOut Z, int first_tile, int poll_limit) {
+template <int VT, int OP, int MODE, bool LEVELS>
+__device__ __noinline__ void csr2_tile_wide(const CsrIn &A, const CsrIn &B, const TileRange tile, const int cbits, const int t,
+                                            const int num_tiles, int32_t *tile_count, const TileWords &words, FusedCtl *ctl,
+                                            const CsrOut &Z, const LevelOffsets &L, unsigned char *smem_raw, TileShared &sh,
+                                          const int poll_limit) {
+    csr2_tile<VT, OP, MODE, LEVELS, true>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
+}
+
+template <int V, int OP, int MODE, bool LEVELS>
+__global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ CsrIn A, const __grid_constant__ CsrIn B,
+                                                                    const RowCount row_count, const Cuts cuts, int cbits,
+                                                                    int32_t *tile_count, const __grid_constant__ TileWords words, FusedCtl *ctl,
+                                                                    const __grid_constant__ CsrOut Z, const __grid_constant__ LevelOffsets L, int num_tiles,
+                                                                    int first_tile, int poll_limit) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t mbar;
-    // Tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
-    // only ever waits on CTAs that were dispatched before it (and every such wait is bounded).
-    // first_tile is 0 except in the self-test of the bounded waits, which leaves tile 0 out.
-    const int t = blockIdx.x + first_tile;
-    const int num_tiles = gridDim.x + first_tile;
+    __shared__ TileShared sh;
     if (threadIdx.x == 0) {
-        mbar_init(&mbar, 1);
+        mbar_init(&sh.mbar, 1);
         mbar_fence_init();
     }
     __syncthreads();
-    // 32-bit composite keys hold ((row in tile << cbits | column) << 1 | operand) when that
-    // fits; tiles that span too many rows for that (long runs of empty rows) use 64-bit keys.
-    const uint64_t nr = (uint64_t)(cuts.row[t + 1] - cuts.row[t]) + 1;
-    const bool narrow = cbits < 31 && (nr << cbits) < 0x7fffffffull;
-    if (narrow) {
-        csr2_tile_blocked<V, OP, MODE>(A, B, cuts, cbits, t, num_tiles, tile_count, tile_state, ctl, Z, smem_raw, &mbar, poll_limit);
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the cuts (no wait where no partition kernel ran)
+    const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
+    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
+        if (threadIdx.x < 32) {
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, poll_limit);
+            if (threadIdx.x == 0) finish_total(ctl, Z, total);
+        }
+        return;
+    }
+    // Tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
+    // only ever waits on CTAs that were dispatched before it (and every such wait is bounded).
+    // first_tile is 0 except in the self-test of the bounded waits, which leaves tile 0 out.
+    const int t = blockIdx.x + first_tile - (scanned ? 1 : 0);
+    TileRange tile;
+    if (cuts) {
+        const int4 c0 = cuts[t], c1 = cuts[t + 1];
+        tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
     } else {
-        if (threadIdx.x >= NT) return;  // the wide-key body works with the NT worker threads alone
-        csr2_tile_wide<V, OP, MODE>(A, B, cuts, t, tile_count, tile_state, ctl, Z, smem_raw, num_tiles, poll_limit);
+        const int32_t rows = row_count.get();
+        tile = TileRange{0, rows, row_offset(A, 0), row_offset(B, 0), A.nnz, B.nnz};
+        if (threadIdx.x == 0) {  // what the partition kernel does otherwise
+            ctl->status = DeviceStatus{0, 0};
+            ctl->hollow = 0;
+            if (Z.result) Z.result[1] = NB200_OK, Z.result[2] = rows;
+        }
+        __syncthreads();
+    }
+    // 32-bit keys hold (row in tile << cbits | column) when that fits; tiles that span too many rows for
+    // that (long runs of empty rows) use 64-bit keys.
+    const uint64_t nr = (uint64_t)(tile.i1 - tile.i0) + 1;
+    const bool narrow = cbits < 31 && (nr << cbits) <= 0x80000000ull;
+    if (narrow) {
+        csr2_tile<V, OP, MODE, LEVELS, false>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
+    } else {
+        csr2_tile_wide<V, OP, MODE, LEVELS>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
     }
 }
 
 // ------------------------------------------------------------------------ host driver ----
 
-constexpr int V_CSR2 = CSR2_V;
-constexpr int TILE_STEP = NT * V_CSR2 - 1;  // merged entries between two tile cuts
-
-// Dynamic shared memory of the tile kernel: the staging arrays of the common body, or the 64-bit
-// keys of the wide-key body, whichever is larger.
-constexpr size_t csr2_smem_bytes() {
-    return std::max<size_t>(BlockedPlan<V_CSR2>::BYTES, 8 * (size_t)(NT * V_CSR2 + 2 + V_CSR2));
-}
+// Merged entries per worker thread. Large tiles amortise what a tile costs whatever its size (searches,
+// barriers, the wait for the earlier counts): 64 M entries per operand take 471 us with 31, 477 with 27, 526
+// with 15, 638 with 11. With fewer than about 750 large tiles the chip (592 resident ones) is better filled by
+// small ones: 2 M merged entries 22.8 us with 15 against 24.9, 0.8 M 15.8 against 18.9; at 6 M the two are even.
+// Both are odd: a thread's shares of A and B then start at odd word distances from its neighbour's where
+// rows alternate evenly, and the shared-memory banks are hit evenly (16 took twice the time of 18).
+constexpr int V_LARGE = 31, V_SMALL = 15;
+constexpr int64_t LARGE_FROM = 6000000;
+constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
+constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between two tile cuts (a twin may add one)
 
 // Raises the tile kernel's dynamic shared-memory limit once per instantiation and device.
-template <int OP, int MODE>
+template <int V, int OP, int MODE, bool LEVELS = false>
 cudaError_t configure_tile_kernel() {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_csr2_tile<V_CSR2, OP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csr2_smem_bytes());
+        cudaError_t e = cudaFuncSetAttribute(k_csr2_tile<V, OP, MODE, LEVELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TilePlan<V, LEVELS>::BYTES);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
@@ -730,18 +657,49 @@ struct LaunchKnobs {
     int poll_limit = LOOKBACK_POLL_LIMIT;
 };
 
-template <int OP, int MODE>
-cudaError_t launch_tile(const CsrIn &A, const CsrIn &B, const Cuts &cuts, int cbits, int32_t *tile_count,
-                        uint64_t *tile_state, FusedCtl *ctl, const CsrOut &Z, int num_tiles, cudaStream_t stream,
-                        const LaunchKnobs &knobs = LaunchKnobs()) {
-    cudaError_t e = configure_tile_kernel<OP, MODE>();
+// Launches the tile kernel so that it may take its places while the kernel before it on the stream (the
+// partition) still runs; it waits for that kernel's results itself.
+template <int V, int OP, int MODE, bool LEVELS = false>
+cudaError_t launch_tile_v(const CsrIn &A, const CsrIn &B, const RowCount &rows, const Cuts &cuts, int cbits, int32_t *tile_count,
+                          TileWords words, FusedCtl *ctl, const CsrOut &Z, int num_tiles, cudaStream_t stream, const LaunchKnobs &knobs,
+                          const LevelOffsets &levels = LevelOffsets()) {
+    cudaError_t e = configure_tile_kernel<V, OP, MODE, LEVELS>();
     if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(num_tiles - knobs.first_tile + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = TilePlan<V, LEVELS>::BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    if (MODE == MODE_FUSED && cuts) cfg.attrs = &early, cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_csr2_tile<V, OP, MODE, LEVELS>, A, B, rows, cuts, cbits, tile_count, words, ctl, Z, levels, num_tiles, knobs.first_tile,
+                              knobs.poll_limit);
+}
+
+template <int OP, int MODE>
+cudaError_t launch_tile(const CsrIn &A, const CsrIn &B, const RowCount &rows, const Cuts &cuts, int cbits, int32_t *tile_count,
+                        TileWords words, FusedCtl *ctl, const CsrOut &Z, int num_tiles, int v, cudaStream_t stream,
+                        const LaunchKnobs &knobs = LaunchKnobs()) {
     static const char *const names[2][3] = {{"csr_add_count", "csr_add_fill", "csr_add_fused"},
                                             {"csr_mul_count", "csr_mul_fill", "csr_mul_fused"}};
     if (num_tiles - knobs.first_tile <= 0) return cudaSuccess;
     LaunchScope scope(names[OP][MODE], stream);
-    k_csr2_tile<V_CSR2, OP, MODE><<<num_tiles - knobs.first_tile, NT + 32, csr2_smem_bytes(), stream>>>(
-        A, B, cuts, cbits, tile_count, tile_state, ctl, Z, knobs.first_tile, knobs.poll_limit);
+    return v == V_LARGE ? launch_tile_v<V_LARGE, OP, MODE>(A, B, rows, cuts, cbits, tile_count, words, ctl, Z, num_tiles, stream, knobs)
+                        : launch_tile_v<V_SMALL, OP, MODE>(A, B, rows, cuts, cbits, tile_count, words, ctl, Z, num_tiles, stream, knobs);
+}
+
+// Eight lanes per cut once a full warp per cut would need more than one wave of the chip: the searches
+// then run a few dependent loads longer, but four times fewer warps issue them.
+cudaError_t launch_partition(const CsrIn &A, const CsrIn &B, const RowCount &rows, int64_t total, int num_tiles, int step, const Cuts &cuts,
+                             long long *result, uint64_t *zero_block, int zero_words, cudaStream_t stream) {
+    const int64_t lanes = num_tiles < 8192 ? 32 : 8;
+    const int blocks = (int)(((int64_t)(num_tiles + 1) * lanes + NT - 1) / NT);
+    if (lanes == 32)
+        k_csr2_partition<32><<<blocks, NT, 0, stream>>>(A, B, rows, (uint32_t)total, step, num_tiles, cuts, result, zero_block, zero_words);
+    else
+        k_csr2_partition<8><<<blocks, NT, 0, stream>>>(A, B, rows, (uint32_t)total, step, num_tiles, cuts, result, zero_block, zero_words);
     return cudaGetLastError();
 }
 
@@ -764,8 +722,10 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     if (!alloc && (!z->row_ptr || capacity < 0)) return NB200_E_BADARG;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int32_t rows = a->rows;
+    const RowCount row_count{rows};
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    const int64_t tiles64 = (total + TILE_STEP - 1) / TILE_STEP;
+    const int v = tile_v(total), step = tile_step(v);
+    const int64_t tiles64 = (total + step - 1) / step;
     if (tiles64 > INT32_MAX - 1) return NB200_E_OVERFLOW;
     const int num_tiles = (int)tiles64;
     const int64_t bound = OP == OP_UNION ? total : std::min<int64_t>(a->nnz, b->nnz);
@@ -803,25 +763,20 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     }
 
     Carver sizes;
+    sizes.take<int4>((size_t)num_tiles + 1);
     sizes.take<int32_t>((size_t)num_tiles + 1);
-    sizes.take<int32_t>((size_t)num_tiles + 1);
-    sizes.take<int32_t>((size_t)num_tiles + 1);
-    sizes.take<int32_t>((size_t)num_tiles + 1);
-    sizes.take<uint64_t>((size_t)num_tiles + 8);
+    sizes.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     Workspace *ws = nullptr;
     if ((st = acquire_workspace(stream, sizes.used(), &ws))) return fail(st);
     Carver carve(ws->dev);
-    Cuts cuts;
-    cuts.row = carve.take<int32_t>((size_t)num_tiles + 1);
-    cuts.a = carve.take<int32_t>((size_t)num_tiles + 1);
-    cuts.b = carve.take<int32_t>((size_t)num_tiles + 1);
+    Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
     // control block (status word, result length) and the tile words of the single-pass kernel,
     // contiguous for one memset; the two-pass route uses the control block alone
-    uint64_t *fused_block = carve.take<uint64_t>((size_t)num_tiles + 8);
+    uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     static_assert(sizeof(FusedCtl) <= 4 * sizeof(uint64_t), "control block must fit its slot");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    uint64_t *tile_state = fused_block + 4;
+    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};
     const int cbits = col_bits(a->cols);
@@ -839,13 +794,12 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
         if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&z->val), sizeof(float) * (size_t)bound, stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
     }
-    {
+    if (num_tiles == 1) {
+        cuts = nullptr;  // one tile: no cut to search, and the tile kernel clears the control block itself
+    } else {
         LaunchScope scope("csr2_partition", stream);
-        const int warps = num_tiles + 1;
-        const int blocks = (warps * 32 + NT - 1) / NT;
-        k_csr2_partition<<<blocks, NT, 0, stream>>>(A, B, rows, total, TILE_STEP, num_tiles, cuts, reinterpret_cast<long long *>(device_result),
-                                                    fused_block, fused ? num_tiles + 4 : 4);
-        e = cudaGetLastError();
+        e = launch_partition(A, B, row_count, total, num_tiles, step, cuts, reinterpret_cast<long long *>(device_result), fused_block,
+                             fused ? (int)TileWords::needed(num_tiles) + 4 : 4, stream);
     }
     if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_partition"));
 
@@ -860,12 +814,20 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
 
     FusedCtl h;
     if (fused) {
-        e = launch_tile<OP, MODE_FUSED>(A, B, cuts, cbits, nullptr, tile_state, ctl,
-                                        CsrOut{z->row_ptr, z->col, z->val, reinterpret_cast<long long *>(device_result)}, num_tiles, stream, knobs);
+        unsigned long long *word = device_result ? nullptr : result_word(ws, 0);
+        e = launch_tile<OP, MODE_FUSED>(A, B, row_count, cuts, cbits, nullptr, words, ctl,
+                                        CsrOut{z->row_ptr, z->col, z->val, reinterpret_cast<long long *>(device_result), word}, num_tiles, v, stream,
+                                        knobs);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_tile<fused>"));
         if (device_result) return NB200_OK;  // length, status and rows arrive in the caller's device words, written by the kernels
-        if ((st = read_ctl(h))) return fail(st);
-        if (h.status.error != 0) return fail(note_timeout(h.status.error, h.status.detail, "csr merge"));
+        int64_t length;
+        int device_status;
+        if ((st = wait_result_word(word, stream, &length, &device_status))) return fail(st);
+        if (device_status != 0) {
+            if ((st = read_ctl(h))) return fail(st);
+            return fail(note_timeout(h.status.error, h.status.detail, "csr merge"));
+        }
+        h.total = length;
         if (h.total > INT32_MAX) return fail(NB200_E_OVERFLOW);
         z->nnz = (int32_t)h.total;
         if (alloc && h.total == 0) {  // zero-length arrays are handed over as NULL
@@ -879,7 +841,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
 
     // count -> scan -> fill. The scan leaves the result length in the control block, whose status
     // word also collects a give-up of either tile launch (a bulk copy that did not land in time).
-    e = launch_tile<OP, MODE_COUNT>(A, B, cuts, cbits, tile_count, nullptr, ctl, CsrOut{nullptr, nullptr, nullptr}, num_tiles, stream);
+    e = launch_tile<OP, MODE_COUNT>(A, B, row_count, cuts, cbits, tile_count, TileWords{}, ctl, CsrOut{nullptr, nullptr, nullptr}, num_tiles, v, stream);
     if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_tile<count>"));
     {
         LaunchScope scope("scan_tiles", stream);
@@ -900,7 +862,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     } else if (h.total > capacity) {
         return NB200_E_CAPACITY;
     }
-    e = launch_tile<OP, MODE_FILL>(A, B, cuts, cbits, tile_count, nullptr, ctl, CsrOut{z->row_ptr, z->col, z->val}, num_tiles, stream);
+    e = launch_tile<OP, MODE_FILL>(A, B, row_count, cuts, cbits, tile_count, TileWords{}, ctl, CsrOut{z->row_ptr, z->col, z->val}, num_tiles, v, stream);
     if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_tile<fill>"));
     if ((st = read_ctl(h))) return fail(st);
     if (h.status.error != 0) return fail(note_timeout(h.status.error, h.status.detail, "csr merge"));
@@ -944,7 +906,9 @@ int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb2
 // Scratch of nb200_csr_add_f32_noalloc: tile cuts, the single-pass control block and one
 // 8-byte word per tile, carved out of one fixed array that lives in the library's device image
 // (so every GPU that loads the library holds these bytes until the process exits).
-constexpr int NOALLOC_MAX_TILES = 32768;
+constexpr int64_t NOALLOC_MAX_ENTRIES = 159350784;
+constexpr int NOALLOC_MAX_TILES = (int)(NOALLOC_MAX_ENTRIES / tile_step(V_LARGE)) + 1;
+static_assert(LARGE_FROM / tile_step(V_SMALL) + 1 <= NOALLOC_MAX_TILES, "small tiles must fit the scratch too");
 constexpr size_t NOALLOC_SCRATCH_BYTES = 1u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
@@ -963,8 +927,8 @@ int noalloc_scratch_address(void **out) {
         NB200_CUDA(cudaGetSymbolAddress(&p, g_noalloc_scratch));
         // the tile kernel needs more dynamic shared memory than the default limit; set that
         // here too so that later calls are launches and nothing else
-        NB200_CUDA(cudaFuncSetAttribute(k_csr2_tile<V_CSR2, OP_UNION, MODE_FUSED>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csr2_smem_bytes()));
+        NB200_CUDA((configure_tile_kernel<V_LARGE, OP_UNION, MODE_FUSED>()));
+        NB200_CUDA((configure_tile_kernel<V_SMALL, OP_UNION, MODE_FUSED>()));
         address[dev] = p;
     }
     *out = address[dev];
@@ -977,10 +941,11 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     if (!z || !z->row_ptr || capacity < 0 || a->rows != b->rows || a->cols != b->cols) return NB200_E_BADARG;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int32_t rows = a->rows;
+    const RowCount row_count{rows};
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    constexpr int tile_step = TILE_STEP;
-    const int64_t tiles64 = (total + tile_step - 1) / tile_step;
-    if (tiles64 > NOALLOC_MAX_TILES) return NB200_E_UNSUPPORTED;
+    const int v = tile_v(total), step = tile_step(v);
+    const int64_t tiles64 = (total + step - 1) / step;
+    if (total > NOALLOC_MAX_ENTRIES) return NB200_E_UNSUPPORTED;
     if (capacity < total) return NB200_E_CAPACITY;  // this entry point has the single-pass route only
     if (total > 0 && (!z->col || !z->val)) return NB200_E_BADARG;
     const int num_tiles = (int)tiles64;
@@ -994,26 +959,20 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     void *scratch = nullptr;
     if ((st = noalloc_scratch_address(&scratch))) return st;
     Carver carve(scratch);
-    uint64_t *fused_block = carve.take<uint64_t>((size_t)NOALLOC_MAX_TILES + 8);
-    Cuts cuts;
-    cuts.row = carve.take<int32_t>((size_t)NOALLOC_MAX_TILES + 1);
-    cuts.a = carve.take<int32_t>((size_t)NOALLOC_MAX_TILES + 1);
-    cuts.b = carve.take<int32_t>((size_t)NOALLOC_MAX_TILES + 1);
-    static_assert(8 * (NOALLOC_MAX_TILES + 8 + 32) + 3 * (4 * (NOALLOC_MAX_TILES + 1) + 256) <= NOALLOC_SCRATCH_BYTES,
+    uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(NOALLOC_MAX_TILES) + 4);
+    Cuts cuts = carve.take<int4>((size_t)NOALLOC_MAX_TILES + 1);
+    static_assert(8 * (TileWords::needed(NOALLOC_MAX_TILES) + 4) + 16 * (NOALLOC_MAX_TILES + 1) + 512 <= NOALLOC_SCRATCH_BYTES,
                   "scratch layout must fit the fixed array");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    uint64_t *tile_state = fused_block + 4;
+    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
     // the array keeps the previous call's contents: the ticket, the status and every tile word
     // must start at zero (the partition kernel clears them)
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};
-    const int warps = num_tiles + 1;
-    k_csr2_partition<<<(warps * 32 + NT - 1) / NT, NT, 0, stream>>>(A, B, rows, total, tile_step, num_tiles, cuts, nullptr, fused_block,
-                                                                    num_tiles + 4);
-    NB200_CUDA(cudaGetLastError());
-    k_csr2_tile<V_CSR2, OP_UNION, MODE_FUSED><<<num_tiles, NT + 32, csr2_smem_bytes(), stream>>>(
-        A, B, cuts, col_bits(a->cols), nullptr, tile_state, ctl, CsrOut{z->row_ptr, z->col, z->val}, 0, LOOKBACK_POLL_LIMIT);
-    NB200_CUDA(cudaGetLastError());
+    NB200_CUDA(launch_partition(A, B, row_count, total, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream));
+    const CsrOut Z{z->row_ptr, z->col, z->val};
+    NB200_CUDA((v == V_LARGE ? launch_tile_v<V_LARGE, OP_UNION, MODE_FUSED>(A, B, row_count, cuts, col_bits(a->cols), nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs())
+                            : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED>(A, B, row_count, cuts, col_bits(a->cols), nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs())));
     FusedCtl h;  // read back into ordinary host memory: no pinned buffer is taken for this
     NB200_CUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, stream));
     NB200_CUDA(cudaStreamSynchronize(stream));
@@ -1023,7 +982,50 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     return NB200_OK;
 }
 
+// In the offsets mode a tile needs 8 bytes of shared memory per entry, so its large tile is smaller.
+constexpr int V_LEVELS = 23;
+
 }  // namespace
+
+size_t csr2_scratch_bytes(int64_t entries) {
+    const size_t tiles = (size_t)(entries / tile_step(V_SMALL)) + 2;  // the smallest tile, whichever will be taken
+    Carver sizes;
+    sizes.take<int4>(tiles + 1);
+    sizes.take<uint64_t>(TileWords::needed(tiles) + 4);
+    return sizes.used();
+}
+
+int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
+                 void *scratch, cudaStream_t stream, FusedCtl **ctl_out) {
+    const int64_t total = (int64_t)A.nnz + B.nnz;
+    const int v = tile_v(total) == V_LARGE ? (levels ? V_LEVELS : V_LARGE) : V_SMALL, step = tile_step(v);
+    const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
+    Carver carve(scratch);
+    Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
+    uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
+    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
+    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
+    *ctl_out = ctl;
+    cudaError_t e = cudaSuccess;
+    if (num_tiles == 1) {
+        cuts = nullptr;
+    } else {
+        LaunchScope scope("csr2_partition", stream);
+        e = launch_partition(A, B, rows, total, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream);
+    }
+    if (e != cudaSuccess) return note_cuda_error(e, "k_csr2_partition");
+    const int cbits = col_bits(cols);
+    if (levels) {
+        LaunchScope scope("csr_levels_fused", stream);
+        e = v == V_LEVELS ? launch_tile_v<V_LEVELS, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels)
+                          : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels);
+    } else if (op == OP_UNION) {
+        e = launch_tile<OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream);
+    } else {
+        e = launch_tile<OP_INTERSECT, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream);
+    }
+    return e == cudaSuccess ? NB200_OK : note_cuda_error(e, "k_csr2_tile");
+}
 
 int csr_add3_chained(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, bool alloc, int64_t capacity,
                      void *stream_v) {

@@ -3,21 +3,23 @@
 //   coo_add, coo_mul        COO  (+|.*) COO  -> COO
 //   coo_csr_add             CSR  +      COO  -> CSR
 //   dcsr_add, dcsr_mul      DCSR (+|.*) DCSR -> DCSR
-// A sorted coordinate list and a DCSR matrix are both a CSR matrix whose row offsets are not
-// stored: their column and value arrays are already in CSR order. So each kernel here builds the
-// missing row offsets (one small pass over the rows), runs the CSR merge kernels of csr_merge.cu
-// on the caller's own column / value arrays, and converts the result's row level back:
-//   COO   the row index of every result entry is written out (one warp per 32 rows);
-//   DCSR  the rows that the reference keeps are selected and compressed (scan + scatter):
-//         for the sum, the rows that hold a result entry; for the product, the rows that BOTH
-//         operands store -- also those whose columns do not meet, which the reference keeps as
-//         an empty fibre (its intersection works level by level: src/backend/compute.cpp:619-1392
-//         run on the i level first, then on j inside the matched rows).
-// Scratch: three row-offset arrays of rows + 1 entries (and one flag array for DCSR).
+// Both formats hold their columns and values in CSR order, so each kernel here runs the CSR merge kernels of
+// csr_merge.cu on the caller's own column / value arrays; what differs is the row level.
+//   COO   the missing row offsets are built (one small pass over the rows) and the row index of every
+//         result entry is written out (one warp per 32 rows).
+//   DCSR  the two row lists are merged first, as matrices of one row whose columns are the row numbers
+//         (offsets mode of the tile kernel): that yields the union of the stored rows and, over it, a row
+//         offset array for each operand in which a row it lacks is empty. With those the entries are a
+//         CSR merge whose rows are the stored ones only, however many the matrix has; its row count is
+//         read from device memory, so nothing waits in between. The sum keeps the rows that hold a result
+//         entry: all of the union, unless an operand stores empty rows. The product keeps the rows that
+//         BOTH operands store -- also those whose columns do not meet, which the reference keeps as an
+//         empty fibre (its intersection works level by level: src/backend/compute.cpp:619-1392 run on the
+//         i level first, then on j inside the matched rows). Rows are dropped by a scan and a scatter.
 #include <algorithm>
 #include <cstring>
 
-#include "merge_common.cuh"
+#include "csr_common.cuh"
 
 namespace nb200 {
 
@@ -63,33 +65,30 @@ __global__ void __launch_bounds__(NT) k_expand_rows(const int32_t *__restrict__ 
     }
 }
 
-// keep[r] = 1 for the rows the result stores. Sum: a row with a result entry. Product: a row
-// that both operands store (whatever its result holds).
-__global__ void __launch_bounds__(NT) k_dcsr_keep(const int32_t *__restrict__ rpa, const int32_t *__restrict__ rpb,
-                                                 const int32_t *__restrict__ rpz, int32_t rows, int product, int32_t *__restrict__ keep) {
-    const int64_t r = (int64_t)blockIdx.x * NT + threadIdx.x;
-    if (r >= rows) return;
-    const bool in_a = ld_nc(rpa + r + 1) > ld_nc(rpa + r), in_b = ld_nc(rpb + r + 1) > ld_nc(rpb + r);
-    keep[r] = product ? (in_a && in_b) : (ld_nc(rpz + r + 1) > ld_nc(rpz + r));
+// keep[u] = 1 for the rows of a CSR structure that hold an entry.
+__global__ void __launch_bounds__(NT) k_rows_nonempty(const int32_t *__restrict__ rp, int32_t rows, int32_t *__restrict__ keep) {
+    const int64_t u = (int64_t)blockIdx.x * NT + threadIdx.x;
+    if (u < rows) keep[u] = ld_nc(rp + u + 1) > ld_nc(rp + u);
 }
 
-// After the exclusive scan of keep[]: row r, if kept, is result row pos[r]. The flag is recomputed
-// (pos[r + 1] > pos[r], with the total after the last row).
-__global__ void __launch_bounds__(NT) k_dcsr_scatter(const int32_t *__restrict__ pos, const long long *__restrict__ total,
-                                                    const int32_t *__restrict__ rpz, int32_t rows, int32_t *__restrict__ i_idx,
-                                                    int32_t *__restrict__ j_ptr) {
-    const int64_t r = (int64_t)blockIdx.x * NT + threadIdx.x;
-    if (r > rows) return;
-    const int32_t n = (int32_t)*total;
-    if (r == rows) {
-        j_ptr[n] = ld_nc(rpz + rows);
+// After the exclusive scan of keep[]: row u, if kept, is result row pos[u]. The flag is recomputed
+// (pos[u + 1] > pos[u], with the total after the last row). The result length goes to `word`.
+__global__ void __launch_bounds__(NT) k_rows_scatter(const int32_t *__restrict__ pos, const FusedCtl *__restrict__ ctl, const int32_t *__restrict__ ids,
+                                                    const int32_t *__restrict__ rp, int32_t rows, int32_t *__restrict__ i_idx,
+                                                    int32_t *__restrict__ j_ptr, unsigned long long *word) {
+    const int64_t u = (int64_t)blockIdx.x * NT + threadIdx.x;
+    if (u > rows) return;
+    const int32_t n = (int32_t)ctl->total;
+    if (u == rows) {
+        j_ptr[n] = ld_nc(rp + rows);
+        publish_result_word(word, ctl->status.error != 0 ? NB200_E_TIMEOUT : NB200_OK, n);
         return;
     }
-    const int32_t at = ld_nc(pos + r);
-    const int32_t next = r + 1 < rows ? ld_nc(pos + r + 1) : n;
+    const int32_t at = ld_nc(pos + u);
+    const int32_t next = u + 1 < rows ? ld_nc(pos + u + 1) : n;
     if (next > at) {
-        i_idx[at] = (int32_t)r;
-        j_ptr[at] = ld_nc(rpz + r);
+        i_idx[at] = ld_nc(ids + u);
+        j_ptr[at] = ld_nc(rp + u);
     }
 }
 
@@ -113,27 +112,22 @@ cudaError_t launch_row_offsets(const int32_t *ids, const int32_t *ptr, int32_t n
 
 typedef int (*csr_into_fn)(const nb200_csr *, const nb200_csr *, nb200_csr *, int64_t, void *);
 
-// Scratch of one call: three row-offset arrays, the keep / position array and a control block
-// with the scan's tile words (DCSR only). Pool slot 1: the CSR kernels underneath use slot 0.
+// Scratch of a call on coordinate lists: row offsets of A, B and the result. Pool slot 1: the CSR kernels
+// underneath use slot 0.
 struct Scratch2d {
-    int32_t *rpa, *rpb, *rpz, *keep;
-    uint64_t *scan_block;
-    Workspace *ws;
+    int32_t *rpa, *rpb, *rpz;
 };
 
 int take_scratch(int32_t rows, cudaStream_t stream, Scratch2d *s) {
-    const size_t scan_ctas = ((size_t)rows + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT) + 1;
     Carver sizes;
-    for (int q = 0; q < 4; ++q) sizes.take<int32_t>((size_t)rows + 2);
-    sizes.take<uint64_t>(scan_ctas + 8);
+    for (int q = 0; q < 3; ++q) sizes.take<int32_t>((size_t)rows + 2);
+    Workspace *ws = nullptr;
     int st;
-    if ((st = acquire_workspace(stream, sizes.used(), &s->ws, 1))) return st;
-    Carver carve(s->ws->dev);
+    if ((st = acquire_workspace(stream, sizes.used(), &ws, 1))) return st;
+    Carver carve(ws->dev);
     s->rpa = carve.take<int32_t>((size_t)rows + 2);
     s->rpb = carve.take<int32_t>((size_t)rows + 2);
     s->rpz = carve.take<int32_t>((size_t)rows + 2);
-    s->keep = carve.take<int32_t>((size_t)rows + 2);
-    s->scan_block = carve.take<uint64_t>(scan_ctas + 8);
     return NB200_OK;
 }
 
@@ -168,59 +162,125 @@ int coo2_run(csr_into_fn op, bool is_union, const nb200_coo *a, const nb200_coo 
     return NB200_OK;
 }
 
+// Numbers the kept ones of `n` rows (flags in `keep`, overwritten) and writes the compressed row level of the
+// result; *count receives its length. `block` holds the scan's control block and tile words.
+int compress_rows(int32_t *keep, int32_t n, const int32_t *ids, const int32_t *rp, uint64_t *block, nb200_dcsr *z, unsigned long long *word,
+                  cudaStream_t stream) {
+    const int ctas = (int)(((int64_t)n + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT));
+    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(block);
+    NB200_CUDA(cudaMemsetAsync(block, 0, sizeof(uint64_t) * ((size_t)ctas + 4), stream));
+    {
+        LaunchScope scope("scan_lookback", stream);
+        k_scan_lookback<<<ctas, SCAN_NT, 0, stream>>>(keep, n, block + 4, ctl);
+    }
+    {
+        LaunchScope scope("dcsr_scatter", stream);
+        k_rows_scatter<<<(int)(((int64_t)n + 1 + NT - 1) / NT), NT, 0, stream>>>(keep, ctl, ids, rp, n, z->i_idx, z->j_ptr, word);
+    }
+    NB200_CUDA(cudaGetLastError());
+    int64_t kept;
+    int st, device_status;
+    if ((st = wait_result_word(word, stream, &kept, &device_status))) return st;
+    if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "dcsr row compress");
+    z->n_i = (int32_t)kept;
+    return NB200_OK;
+}
+
 int dcsr2_run(csr_into_fn op, bool is_union, const nb200_dcsr *a, const nb200_dcsr *b, nb200_dcsr *z, int64_t cap_i, int64_t capacity,
               void *stream_v) {
     int st;
     if ((st = check_dcsr(a)) || (st = check_dcsr(b))) return st;
     if (!z || a->rows != b->rows || a->cols != b->cols || capacity < 0 || cap_i < 0 || !z->j_ptr) return NB200_E_BADARG;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    const int32_t rows = a->rows;
-    z->rows = rows;
+    z->rows = a->rows;
     z->cols = a->cols;
     z->n_i = z->nnz = 0;
-    const int64_t bound_i = is_union ? std::min<int64_t>((int64_t)a->n_i + b->n_i, rows) : std::min(a->n_i, b->n_i);
+    const int64_t stored = (int64_t)a->n_i + b->n_i;  // most rows of the union
+    const int64_t bound_i = is_union ? std::min<int64_t>(stored, a->rows) : std::min(a->n_i, b->n_i);
     if (cap_i < bound_i) return NB200_E_CAPACITY;  // the row level is written in one pass: room for the worst case
     if (bound_i > 0 && !z->i_idx) return NB200_E_BADARG;
-    if (bound_i == 0) {  // no row survives: one leading zero in the offsets
+    const int64_t total = (int64_t)a->nnz + b->nnz;
+    if (bound_i == 0 || total == 0) {  // no row survives: one leading zero in the offsets
         NB200_CUDA(cudaMemsetAsync(z->j_ptr, 0, sizeof(int32_t), stream));
         return NB200_OK;
     }
     if (capacity > 0 && (!z->j_idx || !z->val)) return NB200_E_BADARG;
-    Scratch2d s;
-    if ((st = take_scratch(rows, stream, &s))) return st;
-    cudaError_t e = launch_row_offsets(a->i_idx, a->j_ptr, a->n_i, rows, s.rpa, stream);
-    if (e == cudaSuccess) e = launch_row_offsets(b->i_idx, b->j_ptr, b->n_i, rows, s.rpb, stream);
-    if (e != cudaSuccess) return note_cuda_error(e, "k_row_offsets");
-    const nb200_csr ca{rows, a->cols, a->nnz, s.rpa, a->j_idx, a->val}, cb{rows, b->cols, b->nnz, s.rpb, b->j_idx, b->val};
-    nb200_csr cz{rows, a->cols, 0, s.rpz, z->j_idx, z->val};
-    st = op(&ca, &cb, &cz, capacity, stream_v);
-    z->nnz = cz.nnz;
-    if (st != NB200_OK) return st;
-    // select the rows the result stores, number them, write the compressed row level
-    const int scan_ctas = (int)(((int64_t)rows + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT));
-    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(s.scan_block);
-    NB200_CUDA(cudaMemsetAsync(s.scan_block, 0, sizeof(uint64_t) * ((size_t)scan_ctas + 4), stream));
+    if (stored > INT32_MAX - 1) return NB200_E_OVERFLOW;
+
+    // pool slot 1: the union's rows, the offsets of both operands over it, flags, the result's offsets over it
+    const size_t scan_words = (size_t)stored / (SCAN_NT * SCAN_VT) + 8;
+    Carver sizes;
+    for (int q = 0; q < 5; ++q) sizes.take<int32_t>((size_t)stored + 2);
+    sizes.take<uint64_t>(scan_words);
+    const size_t own = sizes.used();
+    const size_t list_bytes = csr2_scratch_bytes(stored), entry_bytes = csr2_scratch_bytes(total);
+    Workspace *ws = nullptr;
+    if ((st = acquire_workspace(stream, own + list_bytes + entry_bytes, &ws, 1))) return st;
+    Carver carve(ws->dev);
+    int32_t *off_a = carve.take<int32_t>((size_t)stored + 2), *off_b = carve.take<int32_t>((size_t)stored + 2);
+    int32_t *keep = carve.take<int32_t>((size_t)stored + 2), *ids = carve.take<int32_t>((size_t)stored + 2);
+    int32_t *rpz = carve.take<int32_t>((size_t)stored + 2);
+    uint64_t *scan_block = carve.take<uint64_t>(scan_words);
+    unsigned char *list_scratch = static_cast<unsigned char *>(ws->dev) + own, *entry_scratch = list_scratch + list_bytes;
+    unsigned long long *rows_word = result_word(ws, 0), *length_word = result_word(ws, 1), *kept_word = result_word(ws, 2);
+
+    // ---- the stored rows of both operands, and where their entries begin
+    const LevelOffsets levels{a->j_ptr, b->j_ptr, off_a, off_b, is_union ? nullptr : keep};
+    FusedCtl *rows_ctl = nullptr, *ctl = nullptr;
+    int32_t *union_rows = is_union ? z->i_idx : ids;
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{nullptr, a->i_idx, nullptr, a->n_i}, CsrIn{nullptr, b->i_idx, nullptr, b->n_i}, RowCount{1}, a->rows,
+                           CsrOut{nullptr, union_rows, nullptr, nullptr, rows_word}, &levels, list_scratch, stream, &rows_ctl)))
+        return st;
+
+    // ---- the entries, on the rows of the union
+    int64_t length, n_rows;
+    int rows_status, device_status = 0;
+    int32_t *result_rp = is_union ? z->j_ptr : rpz;
+    const CsrIn A{off_a, a->j_idx, a->val, a->nnz}, B{off_b, b->j_idx, b->val, b->nnz};
+    const bool one_pass = capacity >= (is_union ? total : std::min<int64_t>(a->nnz, b->nnz));
+    bool hollow = false;
+    if (one_pass) {
+        if ((st = csr2_enqueue(is_union ? OP_UNION : OP_INTERSECT, A, B, RowCount{0, &rows_ctl->total}, a->cols,
+                               CsrOut{result_rp, z->j_idx, z->val, nullptr, length_word, rows_ctl}, nullptr, entry_scratch, stream, &ctl)))
+            return st;
+    }
+    if ((st = wait_result_word(rows_word, stream, &n_rows, &rows_status))) return st;
+    n_rows &= RW_HOLLOW - 1;
+    if (one_pass) {
+        if ((st = wait_result_word(length_word, stream, &length, &device_status))) return st;
+        hollow = (length & RW_HOLLOW) != 0;
+        length &= RW_HOLLOW - 1;
+        if (length > INT32_MAX) return NB200_E_OVERFLOW;
+        z->nnz = (int32_t)length;
+    }
+    if (rows_status != 0 || device_status != 0) {
+        NB200_CUDA(cudaMemcpyAsync(ws->host, rows_status != 0 ? rows_ctl : ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
+        NB200_CUDA(cudaStreamSynchronize(stream));
+        FusedCtl h;
+        std::memcpy(&h, ws->host, sizeof(h));
+        return note_timeout(h.status.error, h.status.detail, "dcsr merge");
+    }
+    if (!one_pass) {  // less room than the worst case: count first
+        const nb200_csr ca{(int32_t)n_rows, a->cols, a->nnz, off_a, a->j_idx, a->val}, cb{(int32_t)n_rows, b->cols, b->nnz, off_b, b->j_idx, b->val};
+        nb200_csr cz{(int32_t)n_rows, a->cols, 0, result_rp, z->j_idx, z->val};
+        st = op(&ca, &cb, &cz, capacity, stream_v);
+        z->nnz = cz.nnz;
+        if (st != NB200_OK) return st;
+        hollow = true;  // (not reported on this route: check below)
+    }
+
+    // ---- the rows the result stores
+    if (!is_union) return compress_rows(keep, (int32_t)n_rows, ids, rpz, scan_block, z, kept_word, stream);
+    z->n_i = (int32_t)n_rows;
+    if (!hollow) return NB200_OK;
+    NB200_CUDA(cudaMemcpyAsync(ids, z->i_idx, sizeof(int32_t) * (size_t)n_rows, cudaMemcpyDeviceToDevice, stream));
+    NB200_CUDA(cudaMemcpyAsync(rpz, z->j_ptr, sizeof(int32_t) * ((size_t)n_rows + 1), cudaMemcpyDeviceToDevice, stream));
     {
         LaunchScope scope("dcsr_keep", stream);
-        k_dcsr_keep<<<(int)(((int64_t)rows + NT - 1) / NT), NT, 0, stream>>>(s.rpa, s.rpb, s.rpz, rows, is_union ? 0 : 1, s.keep);
+        k_rows_nonempty<<<(int)((n_rows + NT - 1) / NT), NT, 0, stream>>>(rpz, (int32_t)n_rows, keep);
     }
-    {
-        LaunchScope scope("scan_lookback", stream);
-        k_scan_lookback<<<scan_ctas, SCAN_NT, 0, stream>>>(s.keep, rows, s.scan_block + 4, ctl);
-    }
-    {
-        LaunchScope scope("dcsr_scatter", stream);
-        k_dcsr_scatter<<<(int)(((int64_t)rows + 1 + NT - 1) / NT), NT, 0, stream>>>(s.keep, &ctl->total, s.rpz, rows, z->i_idx, z->j_ptr);
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return note_cuda_error(e, "dcsr row level");
-    NB200_CUDA(cudaMemcpyAsync(s.ws->host, ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaStreamSynchronize(stream));
-    FusedCtl h;
-    std::memcpy(&h, s.ws->host, sizeof(h));
-    if (h.status.error != 0) return note_timeout(h.status.error, h.status.detail, "dcsr row compress");
-    z->n_i = (int32_t)h.total;
-    return NB200_OK;
+    NB200_CUDA(cudaGetLastError());
+    return compress_rows(keep, (int32_t)n_rows, ids, rpz, scan_block, z, kept_word, stream);
 }
 
 }  // namespace

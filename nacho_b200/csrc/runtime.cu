@@ -97,6 +97,25 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
     return NB200_OK;
 }
 
+int wait_result_word(const unsigned long long *word, cudaStream_t stream, int64_t *value, int *device_status) {
+    const volatile unsigned long long *w = word;
+    unsigned long long v;
+    for (unsigned spins = 1; !((v = *w) & RW_VALID); ++spins) {
+#if defined(__x86_64__)
+        __builtin_ia32_pause();
+#endif
+        if (spins % 4096 != 0) continue;  // about every 100 us: has the stream failed, or ended without the word?
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess) return note_cuda_error(e, "wait for a result length");
+        if ((v = *w) & RW_VALID) break;
+        return note_cuda_error(cudaErrorUnknown, "the kernels ended without a result length");
+    }
+    *device_status = (int)((v & ~RW_VALID) >> RW_STATUS_SHIFT);
+    *value = (int64_t)(v & RW_VALUE_MASK);
+    return NB200_OK;
+}
+
 uint64_t workspace_epoch() { return g_ws_epoch.load(std::memory_order_acquire); }
 
 LaunchScope::LaunchScope(const char *name, cudaStream_t stream)
