@@ -264,6 +264,7 @@ __device__ __forceinline__ int64_t lookback_exclusive(volatile uint64_t *state, 
     if (lane_id() == 0) st_relaxed_gpu(state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)aggregate);
     if (t == 0) return 0;
     const int64_t exclusive = lookback_predecessors(state, t, status, 32);
+    if (exclusive < 0) __threadfence();  // the error word goes out before the word that lets the successors through
     if (lane_id() == 0) st_relaxed_gpu(state + t, LB_PREFIX | (uint64_t)(exclusive < 0 ? 0 : exclusive + aggregate));
     return exclusive;
 }

@@ -103,6 +103,26 @@ private:
     bool timed_;
 };
 
+// Launches `kernel` so that its CTAs may take their places while the kernel before it on the stream still
+// runs (programmatic dependent launch; that kernel says when, with trigger_dependents). A kernel that reads
+// what the one before it writes calls wait_for_previous first; one that does not calls it in its last CTA
+// before it ends (finish_after_previous), so that "this kernel is complete" still means that everything
+// before it is.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Error word shared by kernels with bounded waits: 0 = fine, otherwise a site code.
 struct DeviceStatus {
     int error;
@@ -114,6 +134,13 @@ struct DeviceStatus {
 #ifdef __CUDACC__
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
+
+// The two sides of launch_overlapped; both do nothing where a kernel was launched without it.
+__device__ __forceinline__ void trigger_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void finish_after_previous() {
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) wait_for_previous();
+}
 
 // Publishes a result word (see above). The store is a single 8-byte one, so it needs no fence.
 __device__ __forceinline__ void publish_result_word(unsigned long long *word, int status, long long value) {

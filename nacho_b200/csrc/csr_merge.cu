@@ -103,7 +103,7 @@ template <int G>
 __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count, uint32_t total,
                                                        int32_t tile_step, int32_t num_tiles, Cuts cuts, long long *result,
                                                        uint64_t *zero_block, int zero_words) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the tile kernel may take its places; it waits for the cuts
+    trigger_dependents();  // the tile kernel may take its places; it waits for the cuts
     const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
     const int32_t rows = row_count.get();
     if (result && gid == 0) {  // the tile kernel that follows fills in the rest
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
         mbar_fence_init();
     }
     __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the cuts (no wait where no partition kernel ran)
+    wait_for_previous();  // the cuts (no wait where no partition kernel ran)
     const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
     if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
         if (threadIdx.x < 32) {
@@ -665,17 +665,14 @@ cudaError_t launch_tile_v(const CsrIn &A, const CsrIn &B, const RowCount &rows, 
                           const LevelOffsets &levels = LevelOffsets()) {
     cudaError_t e = configure_tile_kernel<V, OP, MODE, LEVELS>();
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(num_tiles - knobs.first_tile + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = TilePlan<V, LEVELS>::BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    if (MODE == MODE_FUSED && cuts) cfg.attrs = &early, cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_csr2_tile<V, OP, MODE, LEVELS>, A, B, rows, cuts, cbits, tile_count, words, ctl, Z, levels, num_tiles, knobs.first_tile,
-                              knobs.poll_limit);
+    const dim3 grid(num_tiles - knobs.first_tile + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
+    constexpr size_t smem = TilePlan<V, LEVELS>::BYTES;
+    if (MODE == MODE_FUSED && cuts)
+        return launch_overlapped(k_csr2_tile<V, OP, MODE, LEVELS>, grid, dim3(NT), smem, stream, A, B, rows, cuts, cbits, tile_count, words, ctl, Z,
+                                 levels, num_tiles, knobs.first_tile, knobs.poll_limit);
+    k_csr2_tile<V, OP, MODE, LEVELS><<<grid, NT, smem, stream>>>(A, B, rows, cuts, cbits, tile_count, words, ctl, Z, levels, num_tiles,
+                                                                knobs.first_tile, knobs.poll_limit);
+    return cudaGetLastError();
 }
 
 template <int OP, int MODE>

@@ -208,4 +208,39 @@ static __global__ void __launch_bounds__(SCAN_NT) k_scan_lookback(int32_t *data,
     if (t == (int)gridDim.x - 1 && tid == SCAN_NT - 1) ctl->total = acc;
 }
 
+// The same scan out of place, for counts that turn into offsets: out[i] = sum of data[0 .. i), i = 0 .. n, and
+// the total as a result word.
+static __global__ void __launch_bounds__(SCAN_NT) k_scan_offsets(const int32_t *__restrict__ data, int32_t n, int32_t *__restrict__ out,
+                                                                uint64_t *state, FusedCtl *ctl, unsigned long long *word) {
+    __shared__ int scan_tmp[40];
+    __shared__ long long s_base;
+    const int tid = threadIdx.x, t = blockIdx.x;  // CTAs are dispatched in index order; waits on earlier tiles are bounded
+    const int64_t p0 = ((int64_t)t * SCAN_NT + tid) * SCAN_VT;
+    int v[SCAN_VT], mine = 0;
+#pragma unroll
+    for (int q = 0; q < SCAN_VT; ++q) {
+        v[q] = p0 + q < n ? ld_nc(data + p0 + q) : 0;
+        mine += v[q];
+    }
+    int total;
+    const int run = block_excl_sum<SCAN_NT>(mine, scan_tmp, total);
+    if (warp_id() == 0) {
+        const int64_t b = lookback_exclusive(state, t, total, &ctl->status);
+        if (lane_id() == 0) s_base = b;
+    }
+    __syncthreads();
+    const bool last = t == (int)gridDim.x - 1;
+    if (last && tid == 0) {
+        if (s_base >= 0) ctl->total = s_base + total;
+        publish_result_word(word, s_base < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK, s_base < 0 ? 0 : s_base + total);
+    }
+    if (s_base < 0) return;
+    long long acc = s_base + run;
+#pragma unroll
+    for (int q = 0; q < SCAN_VT; ++q) {
+        if (p0 + q <= n) out[p0 + q] = (int32_t)min(acc, (long long)INT32_MAX);
+        acc += v[q];
+    }
+}
+
 }  // namespace nb200

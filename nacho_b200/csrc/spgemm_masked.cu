@@ -19,13 +19,12 @@
 //   k_sssmm_search_*    rows with few products (one warp per row) and rows whose span exceeds the
 //                       largest bitmap (one CTA per row): binary search of the product's column in
 //                       the mask row, float atomics on the global accumulators.
-//   k_scan_lookback     exclusive scan of the "reached" flags: the result position of every mask
-//                       position.
+//   k_sssmm_scan        exclusive scan of the "reached" flags (the result position of every mask position)
+//                       and, in the same pass, the reached positions written there.
 //   k_sssmm_compact     reached positions move to their result slot (column, value); the result's
 //                       row offsets are the scanned flags at the mask's row starts.
 // The sums are float32 atomics in arrival order, as the reference's compress is for every row.
 #include <algorithm>
-#include <cstring>
 
 #include "block_utils.cuh"
 #include "merge_common.cuh"
@@ -69,6 +68,7 @@ struct SssmmCtl {
 __global__ void __launch_bounds__(256) k_sssmm_classify(CsrView A, CsrView B, CsrView C, int32_t rows, int64_t list_cap,
                                                        int2 *__restrict__ units, int32_t *__restrict__ light,
                                                        SssmmCtl *__restrict__ ctl) {
+    trigger_dependents();
     const int lane = lane_id();
     const int64_t warps = (int64_t)gridDim.x * (256 / 32);
     for (int64_t i = (int64_t)blockIdx.x * (256 / 32) + warp_id(); i < rows; i += warps) {
@@ -121,6 +121,7 @@ __device__ __forceinline__ void search_product(const CsrView &B, const CsrView &
 __global__ void __launch_bounds__(256) k_sssmm_search_warp(CsrView A, CsrView B, CsrView C, const int32_t *__restrict__ list,
                                                           SssmmCtl *__restrict__ ctl, float *__restrict__ acc,
                                                           int32_t *__restrict__ hit) {
+    trigger_dependents();
     const int lane = lane_id();
     const int32_t c0 = ld_nc(C.rp);  // the mask may be a row block of a larger matrix: positions count from its first entry
     const int count = ctl->count[LIST_LIGHT];
@@ -128,7 +129,10 @@ __global__ void __launch_bounds__(256) k_sssmm_search_warp(CsrView A, CsrView B,
         int t = 0;
         if (lane == 0) t = atomicAdd(&ctl->ticket[LIST_LIGHT], 1);
         t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= count) return;
+        if (t >= count) {
+            finish_after_previous();
+            return;
+        }
         const int64_t i = ld_nc(list + t);
         const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
         for (int32_t p = ld_nc(A.rp + i), a_hi = ld_nc(A.rp + i + 1); p < a_hi; ++p) {
@@ -140,7 +144,8 @@ __global__ void __launch_bounds__(256) k_sssmm_search_warp(CsrView A, CsrView B,
     }
 }
 
-constexpr int CHUNK = 128;  // products one warp takes at a time: four loads per lane in flight
+constexpr int PER_LANE = 8;           // products of a chunk per lane: that many loads in flight
+constexpr int CHUNK = 32 * PER_LANE;  // products one warp takes at a time
 
 // Shared memory of unit_products: for every entry of the unit, the bounds of its row of B, its
 // value, and the number of chunks in front of it.
@@ -156,11 +161,15 @@ struct UnitRows {
 // the rows of B the entries select are cut into chunks of CHUNK products, the chunks are numbered
 // through (an exclusive sum over the entries) and warp w takes chunks w, w + warps, ...; a chunk
 // finds its entry by binary search in the shared-memory sums. The columns of a warp's next chunk
-// are requested before the current one is worked. The CTA must be in step on entry; `product(q, k,
-// a)` receives the position in B, the column and A's value.
-template <int NT, typename Product>
+// are requested before the current one is worked. The CTA must be in step on entry. `reaches(k)` says
+// whether the mask may hold column k; `product(q, k, a)` receives the position in B, the column and A's
+// value of those products that pass. The two are apart because few pass (one in sixteen on R-MAT graphs) and
+// a lane that does makes its whole warp walk the long way: the tests of a chunk are done first, then every
+// lane works off its own hits, so the long way is walked as often as the luckiest lane has hits (under 3
+// times per 8 products) and not once per product.
+template <int NT, typename Reaches, typename Product>
 __device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B, int32_t p_begin, int32_t p_end, UnitRows<NT> &rows,
-                                              Product product) {
+                                              Reaches reaches, Product product) {
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x, lane = lane_id(), n_e = p_end - p_begin;
     int chunks = 0;
@@ -178,7 +187,7 @@ __device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B
     __syncthreads();
 
     struct Fetched {
-        int32_t k[4], q;
+        int32_t k[PER_LANE], q, live;  // live: products of this lane's warp in steps of 32
         float a;
     };
     auto fetch = [&](int c, Fetched &f) {
@@ -190,17 +199,26 @@ __device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B
         const int32_t hi = rows.hi[e];
         f.q = rows.lo[e] + (c - rows.first[e]) * CHUNK + lane;
         f.a = rows.av[e];
+        f.live = min(PER_LANE, (hi - (f.q - lane) + 31) >> 5);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) f.k[u] = f.q + 32 * u < hi ? ld_nc(B.col + f.q + 32 * u) : -1;
+        for (int u = 0; u < PER_LANE; ++u) f.k[u] = f.q + 32 * u < hi ? ld_nc(B.col + f.q + 32 * u) : -1;
     };
     Fetched cur, next;
     int c = warp_id();
     if (c < total) fetch(c, cur);
     for (; c < total; c += NW) {
         if (c + NW < total) fetch(c + NW, next);
+        unsigned hits = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (cur.k[u] >= 0) product(cur.q + 32 * u, cur.k[u], cur.a);
+        for (int u = 0; u < PER_LANE; ++u) {
+            if (u >= cur.live) break;  // uniform
+            if (cur.k[u] >= 0 && reaches(cur.k[u])) hits |= 1u << u;
+        }
+        while (hits) {
+            const int32_t q = cur.q + 32 * (__ffs((int)hits) - 1);
+            product(q, ld_nc(B.col + q), cur.a);  // the column again, from cache: an index into registers would cost more
+            hits &= hits - 1u;
+        }
         cur = next;
     }
 }
@@ -208,6 +226,7 @@ __device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B
 __global__ void __launch_bounds__(SEARCH_NT) k_sssmm_search_cta(CsrView A, CsrView B, CsrView C, const int2 *__restrict__ units,
                                                                SssmmCtl *__restrict__ ctl, float *__restrict__ acc,
                                                                int32_t *__restrict__ hit) {
+    trigger_dependents();
     __shared__ UnitRows<SEARCH_NT> s_rows;
     const int32_t c0 = ld_nc(C.rp);
     const int count = ctl->count[LIST_WIDE];
@@ -216,9 +235,10 @@ __global__ void __launch_bounds__(SEARCH_NT) k_sssmm_search_cta(CsrView A, CsrVi
         const int64_t i = unit.x;
         const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
         unit_products<SEARCH_NT>(A, B, unit.y, min(unit.y + CLASS[LIST_WIDE].unit(), ld_nc(A.rp + i + 1)), s_rows,
-                                 [&](int32_t q, int32_t k, float av) { search_product(B, C, q, k, av, c_lo, c_hi, c0, acc, hit); });
+                                 [](int32_t) { return true; }, [&](int32_t q, int32_t k, float av) { search_product(B, C, q, k, av, c_lo, c_hi, c0, acc, hit); });
         __syncthreads();
     }
+    finish_after_previous();
 }
 
 template <int NT, bool SHARED_ACC>
@@ -233,6 +253,10 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
     unsigned char *flag_s = reinterpret_cast<unsigned char *>(acc_s + entries_cap);
     __shared__ int2 s_unit;
     __shared__ UnitRows<NT> s_rows;
+    // The list kernels run side by side. Only the first (which == 2) waits for the lists, and lets the next
+    // one start after that; each of the others lets its successor start at once.
+    if (which == 2) wait_for_previous();
+    trigger_dependents();
     const int tid = threadIdx.x;
     const int32_t c0 = ld_nc(C.rp);
     const int count = ctl->count[which];
@@ -244,7 +268,10 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
         __syncthreads();
         const int2 unit = s_unit;
         const int64_t i = unit.x;
-        if (i < 0) return;
+        if (i < 0) {
+            finish_after_previous();
+            return;
+        }
         const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
         const int32_t w0 = ld_nc(C.col + c_lo) >> 6;
         const int32_t words = (ld_nc(C.col + c_hi - 1) >> 6) - w0 + 1, entries = c_hi - c_lo;
@@ -274,9 +301,11 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
         __syncthreads();
         const int32_t col0 = w0 << 6;
         const uint32_t span = (uint32_t)words << 6;
-        unit_products<NT>(A, B, unit.y, min(unit.y + WARP_ENTRIES * (NT / 32), ld_nc(A.rp + i + 1)), s_rows, [&](int32_t q, int32_t k, float av) {
+        unit_products<NT>(A, B, unit.y, min(unit.y + WARP_ENTRIES * (NT / 32), ld_nc(A.rp + i + 1)), s_rows, [&](int32_t k) {
             const uint32_t bit = (uint32_t)(k - col0);
-            if (bit >= span || !((bm32[bit >> 5] >> (bit & 31)) & 1)) return;  // most products end here
+            return bit < span && ((bm32[bit >> 5] >> (bit & 31)) & 1u) != 0u;  // most products end here
+        }, [&](int32_t q, int32_t k, float av) {
+            const uint32_t bit = (uint32_t)(k - col0);
             const uint32_t w = bit >> 6, sh = bit & 63;
             const int32_t pos = (int32_t)rank[w] + __popcll(bm[w] & ((1ull << sh) - 1));
             const float v = (av * ld_nc(B.val + q)) * ld_nc(C.val + c_lo + pos);
@@ -300,8 +329,59 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
     }
 }
 
-// `pos` holds the exclusive scan of the flags over nnz + 1 entries (the last flag is 0, so
-// pos[nnz] is the total).
+// Exclusive scan of the flags over nnz + 1 entries, in place (the last flag is 0, so pos[nnz] is the total, which
+// also goes to `word`), and, where the caller's arrays hold every mask position (`z_col` set), the reached
+// positions written to their places in the same pass.
+__global__ void __launch_bounds__(SCAN_NT) k_sssmm_scan(int32_t *__restrict__ pos, const float *__restrict__ acc, const int32_t *__restrict__ c_rp,
+                                                       const int32_t *__restrict__ c_col, int32_t nnz, uint64_t *state, FusedCtl *ctl,
+                                                       int32_t *__restrict__ z_col, float *__restrict__ z_val, unsigned long long *word) {
+    __shared__ int scan_tmp[40];
+    __shared__ long long s_base;
+    trigger_dependents();
+    wait_for_previous();
+    const int tid = threadIdx.x, t = blockIdx.x;  // CTAs are dispatched in index order; waits on earlier tiles are bounded
+    const int64_t n = (int64_t)nnz + 1, p0 = ((int64_t)t * SCAN_NT + tid) * SCAN_VT;
+    int v[SCAN_VT], mine = 0;
+#pragma unroll
+    for (int q = 0; q < SCAN_VT; ++q) {
+        v[q] = p0 + q < n ? pos[p0 + q] : 0;
+        mine += v[q];
+    }
+    int total;
+    const int run = block_excl_sum<SCAN_NT>(mine, scan_tmp, total);
+    if (warp_id() == 0) {
+        const int64_t b = lookback_exclusive(state, t, total, &ctl->status);
+        if (lane_id() == 0) s_base = b;
+    }
+    __syncthreads();
+    if (t == (int)gridDim.x - 1 && tid == 0)
+        publish_result_word(word, s_base < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK, s_base < 0 ? 0 : s_base + total);
+    if (s_base < 0) return;
+    int32_t at = (int32_t)s_base + run;  // at most nnz
+    const int32_t *mask_col = c_col + ld_nc(c_rp);
+#pragma unroll
+    for (int q = 0; q < SCAN_VT; ++q) {
+        if (p0 + q >= n) break;
+        pos[p0 + q] = at;
+        if (v[q]) {
+            if (z_col) {
+                z_col[at] = ld_nc(mask_col + p0 + q);
+                z_val[at] = acc[p0 + q];
+            }
+            ++at;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sssmm_row_offsets(const int32_t *__restrict__ pos, const int32_t *__restrict__ c_rp,
+                                                          int32_t rows, int32_t *__restrict__ z_rp) {
+    wait_for_previous();
+    const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (r > rows) return;
+    z_rp[r] = pos[ld_nc(c_rp + r) - ld_nc(c_rp)];
+}
+
+// Writes the reached positions after the scan, for callers with less room than the mask has entries.
 __global__ void __launch_bounds__(256) k_sssmm_compact(const int32_t *__restrict__ pos, const float *__restrict__ acc,
                                                       const int32_t *__restrict__ c_rp, const int32_t *__restrict__ c_col, int32_t nnz,
                                                       int32_t *__restrict__ z_col, float *__restrict__ z_val) {
@@ -312,13 +392,6 @@ __global__ void __launch_bounds__(256) k_sssmm_compact(const int32_t *__restrict
         z_col[at] = ld_nc(c_col + ld_nc(c_rp) + p);
         z_val[at] = ld_nc(acc + p);
     }
-}
-
-__global__ void __launch_bounds__(256) k_sssmm_row_offsets(const int32_t *__restrict__ pos, const int32_t *__restrict__ c_rp,
-                                                          int32_t rows, int32_t *__restrict__ z_rp) {
-    const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (r > rows) return;
-    z_rp[r] = ld_nc(pos + (ld_nc(c_rp + r) - ld_nc(c_rp)));
 }
 
 int check(const nb200_csr *m) {
@@ -366,10 +439,9 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     int2 *units = carve.take<int2>((size_t)4 * list_cap);
     int32_t *light = carve.take<int32_t>((size_t)rows);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(scan_block);
-    NB200_CUDA(cudaMemsetAsync(acc, 0, sizeof(float) * (size_t)nnz, stream));
-    NB200_CUDA(cudaMemsetAsync(hit, 0, sizeof(int32_t) * ((size_t)nnz + 1), stream));
-    NB200_CUDA(cudaMemsetAsync(scan_block, 0, sizeof(uint64_t) * ((size_t)scan_ctas + 4), stream));
-    NB200_CUDA(cudaMemsetAsync(sctl, 0, sizeof(SssmmCtl), stream));
+    // sums, flags and control blocks lie next to one another: one fill clears them all
+    NB200_CUDA(cudaMemsetAsync(acc, 0, (size_t)(reinterpret_cast<unsigned char *>(units) - reinterpret_cast<unsigned char *>(acc)), stream));
+    unsigned long long *word = result_word(ws, 0);
     const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val}, C{c->row_ptr, c->col, c->val};
     const int row_warps_grid = (int)std::min<int64_t>(((int64_t)rows + 7) / 8, (int64_t)sms * 8);
     const int most = (int)std::min<int64_t>(list_cap, 1 << 30);
@@ -381,44 +453,46 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     // the device, so an empty list costs one launch of CTAs that leave at once.
     {
         LaunchScope scope("sssmm_bitmap_wide", stream);
-        k_sssmm_bitmap<1024, false><<<std::min(sms, most), 1024, CLASS[2].smem(), stream>>>(A, B, C, units + 2 * list_cap, sctl, 2,
-                                                                                           CLASS[2].words, 0, acc, hit);
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<1024, false>, dim3(std::min(sms, most)), dim3(1024), CLASS[2].smem(), stream, A, B, C,
+                                     units + 2 * list_cap, sctl, 2, CLASS[2].words, 0, acc, hit));
     }
     {
         LaunchScope scope("sssmm_bitmap_medium", stream);
-        k_sssmm_bitmap<1024, true><<<std::min(2 * sms, most), 1024, CLASS[1].smem(), stream>>>(A, B, C, units + list_cap, sctl, 1,
-                                                                                              CLASS[1].words, CLASS[1].entries, acc, hit);
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<1024, true>, dim3(std::min(2 * sms, most)), dim3(1024), CLASS[1].smem(), stream, A, B, C,
+                                     units + list_cap, sctl, 1, CLASS[1].words, CLASS[1].entries, acc, hit));
     }
     {
         LaunchScope scope("sssmm_bitmap_narrow", stream);
-        k_sssmm_bitmap<256, true><<<std::min(8 * sms, most), 256, CLASS[0].smem(), stream>>>(A, B, C, units, sctl, 0, CLASS[0].words,
-                                                                                            CLASS[0].entries, acc, hit);
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<256, true>, dim3(std::min(8 * sms, most)), dim3(256), CLASS[0].smem(), stream, A, B, C, units, sctl, 0,
+                                     CLASS[0].words, CLASS[0].entries, acc, hit));
     }
     {
         LaunchScope scope("sssmm_search_wide", stream);
-        k_sssmm_search_cta<<<std::min(16 * sms, most), SEARCH_NT, 0, stream>>>(A, B, C, units + (size_t)LIST_WIDE * list_cap, sctl, acc, hit);
+        NB200_CUDA(launch_overlapped(k_sssmm_search_cta, dim3(std::min(16 * sms, most)), dim3(SEARCH_NT), 0, stream, A, B, C,
+                                     units + (size_t)LIST_WIDE * list_cap, sctl, acc, hit));
     }
     {
         LaunchScope scope("sssmm_search_light", stream);
-        k_sssmm_search_warp<<<row_warps_grid, 256, 0, stream>>>(A, B, C, light, sctl, acc, hit);
+        NB200_CUDA(launch_overlapped(k_sssmm_search_warp, dim3(row_warps_grid), dim3(256), 0, stream, A, B, C, light, sctl, acc, hit));
     }
+    const bool room = capacity >= nnz && z->col && z->val;  // then every reached position has its place already
     {
-        LaunchScope scope("scan_lookback", stream);
-        k_scan_lookback<<<scan_ctas, SCAN_NT, 0, stream>>>(hit, nnz + 1, scan_block + 4, ctl);
+        LaunchScope scope("sssmm_scan", stream);
+        NB200_CUDA(launch_overlapped(k_sssmm_scan, dim3(scan_ctas), dim3(SCAN_NT), 0, stream, hit, acc, c->row_ptr, c->col, nnz, scan_block + 4, ctl,
+                                     room ? z->col : nullptr, z->val, word));
     }
     {
         LaunchScope scope("sssmm_row_offsets", stream);
-        k_sssmm_row_offsets<<<(int)(((int64_t)rows + 1 + 255) / 256), 256, 0, stream>>>(hit, c->row_ptr, rows, z->row_ptr);
+        NB200_CUDA(launch_overlapped(k_sssmm_row_offsets, dim3((int)(((int64_t)rows + 1 + 255) / 256)), dim3(256), 0, stream, hit, c->row_ptr, rows, z->row_ptr));
     }
-    NB200_CUDA(cudaGetLastError());
-    NB200_CUDA(cudaMemcpyAsync(ws->host, ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaStreamSynchronize(stream));
-    FusedCtl h;
-    std::memcpy(&h, ws->host, sizeof(h));
-    if (h.status.error != 0) return note_timeout(h.status.error, h.status.detail, "sssmm scan");
-    z->nnz = (int32_t)h.total;
-    if (h.total > capacity) return NB200_E_CAPACITY;
-    if (h.total > 0) {
+    int64_t length;
+    int device_status;
+    if ((st = wait_result_word(word, stream, &length, &device_status))) return st;
+    if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "sssmm scan");
+    z->nnz = (int32_t)length;
+    if (room) return NB200_OK;
+    if (length > capacity) return NB200_E_CAPACITY;
+    if (length > 0) {
         if (!z->col || !z->val) return NB200_E_BADARG;
         LaunchScope scope("sssmm_compact", stream);
         k_sssmm_compact<<<(int)(((int64_t)nnz + 255) / 256), 256, 0, stream>>>(hit, acc, c->row_ptr, c->col, nnz, z->col, z->val);
