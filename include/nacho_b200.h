@@ -246,6 +246,14 @@ int nb200_spgemm_f32_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr 
 int nb200_spgemm_f32_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c,
                              void *stream);
 
+/* One-call form for caller-owned memory. _bound bins the rows and sets *capacity to the number of entries of
+ * col / val with which _into runs in one pass, or to 0 where it has to count first (any but matrices of
+ * short rows: at most 8 entries in a row of A and 32 products). _into takes any capacity that holds the
+ * result (less returns NB200_E_CAPACITY with c->nnz filled in); right after _bound on the same arrays and
+ * stream it, or a _symbolic call, does not bin the rows again. */
+int nb200_spgemm_f32_bound(const nb200_csr *a, const nb200_csr *b, int64_t *capacity, void *stream);
+int nb200_spgemm_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t capacity, void *stream);
+
 /* Masked SpGEMM: Z_ik = sum_j a_ij * b_jk * c_ik on the positions the mask C stores and at least
  * one product reaches (explicit zeros kept, columns in C's order). Replaces
  * sssmm::sssmm_gpu_i32_f32 (compiler.cpp:150-153). The mask drives the accumulation: every product

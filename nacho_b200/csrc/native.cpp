@@ -255,7 +255,15 @@ PyObject *spgemm(PyObject *const *args) {
     at::Tensor rp = int_array((int64_t)a.rows + 1, va.device), col, val;
     nb200_csr c{a.rows, b.cols, 0, ints(rp), nullptr, nullptr};
     launch(va, where, [&](void *stream) {
-        const int st = nb200_spgemm_f32_symbolic(&a, &b, &c, nullptr, stream);
+        int64_t capacity;
+        int st = nb200_spgemm_f32_bound(&a, &b, &capacity, stream);
+        if (st != NB200_OK) return st;
+        if (capacity > 0) {  // short rows: one pass, no count first
+            col = int_array(capacity, va.device), val = float_array(capacity, va.device);
+            c.col = ints(col), c.val = floats(val);
+            return nb200_spgemm_f32_into(&a, &b, &c, capacity, stream);
+        }
+        st = nb200_spgemm_f32_symbolic(&a, &b, &c, nullptr, stream);
         if (st != NB200_OK) return st;
         col = int_array(c.nnz, va.device), val = float_array(c.nnz, va.device);
         if (c.nnz > 0) c.col = ints(col), c.val = floats(val);

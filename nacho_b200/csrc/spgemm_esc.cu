@@ -51,8 +51,29 @@ struct EscCtl {
     unsigned long long products;
     int n_small, n_medium, n_ranked;
     int n_giant, n_heavy;  // heavy rows with more / at most GIANT_P products
-    int pad;
+    int max_entries;       // longest row of A
+    int arrived;           // CTAs of the binning kernel that are done
 };
+
+// Result words of the binning kernel, in this order.
+enum { W_PRODUCTS, W_SMALL, W_MEDIUM, W_RANKED, W_GIANT, W_HEAVY, W_ENTRIES, W_NNZ, W_COUNT };
+
+// The last CTA of the binning kernel to get here tells the host the counters. `prefix` may be null.
+__device__ __forceinline__ void publish_counters(EscCtl *ctl, const FusedCtl *prefix, unsigned long long *words) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&ctl->arrived, 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    const volatile EscCtl *c = ctl;
+    publish_result_word(words + W_SMALL, 0, c->n_small);
+    publish_result_word(words + W_MEDIUM, 0, c->n_medium);
+    publish_result_word(words + W_RANKED, 0, c->n_ranked);
+    publish_result_word(words + W_GIANT, 0, c->n_giant);
+    publish_result_word(words + W_HEAVY, 0, c->n_heavy);
+    publish_result_word(words + W_ENTRIES, 0, c->max_entries);
+    publish_result_word(words + W_PRODUCTS, prefix && prefix->status.error != 0 ? NB200_E_TIMEOUT : NB200_OK, (long long)c->products);
+}
 
 // heavy_rows holds the giant rows from its front and the other heavy rows from its back, so
 // that the heaviest rows are handed out first.
@@ -65,6 +86,7 @@ struct RowLists {
 // in one pass, 2048 entries per CTA, CTA totals chained by bounded look-back.
 __global__ void __launch_bounds__(256) k_esc_product_prefix(CsrView A, CsrView B, int32_t nnz_a, unsigned long long *__restrict__ P,
                                                              uint64_t *state_raw, FusedCtl *ctl) {
+    trigger_dependents();
     constexpr int VT = 8;
     __shared__ unsigned long long warp_sums[9];
     __shared__ long long s_base;
@@ -119,7 +141,9 @@ __global__ void __launch_bounds__(256) k_esc_product_prefix(CsrView A, CsrView B
 // Rows without products get their count (0) written here. The counts come from the prefix P of
 // B's row lengths over A's entries (k_esc_product_prefix): a hub row costs one subtraction.
 __global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned long long *__restrict__ P, int32_t rows,
-                                                     int32_t *__restrict__ row_count, RowLists lists, EscCtl *ctl) {
+                                                     int32_t *__restrict__ row_count, RowLists lists, EscCtl *ctl,
+                                                     const FusedCtl *prefix, unsigned long long *words) {
+    wait_for_previous();
     __shared__ unsigned long long warp_p[8];
     const int i = blockIdx.x * 256 + threadIdx.x;  // one lane per row: its products are a difference of the prefix
     unsigned long long p = 0;
@@ -152,13 +176,14 @@ __global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned l
         for (int v = 0; v < 8; ++v) sum += warp_p[v];
         if (sum) atomicAdd(&ctl->products, sum);
     }
+    publish_counters(ctl, prefix, words);
 }
 
 // The same with the product counts taken row by row: one lane per row walks its entries (the warp
 // shares the work of its longer rows). For matrices of short rows, where a prefix pass over A's
 // entries costs more than it saves.
 __global__ void __launch_bounds__(256) k_esc_rowwork_walk(CsrView A, CsrView B, int32_t rows, int32_t *__restrict__ row_count,
-                                                     RowLists lists, EscCtl *ctl) {
+                                                     RowLists lists, EscCtl *ctl, unsigned long long *words) {
     __shared__ unsigned long long warp_p[8];
     const int i = blockIdx.x * 256 + threadIdx.x;  // one lane per row; the warp shares the work of its longer rows
     int32_t lo = 0, hi = 0;
@@ -211,6 +236,9 @@ __global__ void __launch_bounds__(256) k_esc_rowwork_walk(CsrView A, CsrView B, 
         for (int v = 0; v < 8; ++v) sum += warp_p[v];
         if (sum) atomicAdd(&ctl->products, sum);
     }
+    const int longest = __reduce_max_sync(FULL_MASK, hi - lo);
+    if (lane_id() == 0 && longest > 0) atomicMax(&ctl->max_entries, longest);
+    publish_counters(ctl, nullptr, words);
 }
 
 // ------------------------------------------------------------------------- small rows ----
@@ -260,6 +288,7 @@ template <bool NUMERIC, bool NARROW>
 __global__ void __launch_bounds__(256) k_esc_small(CsrView A, CsrView B, const int32_t *__restrict__ row_list, int n_rows,
                                                    int32_t *__restrict__ row_count, const int32_t *__restrict__ c_rp,
                                                    int32_t *__restrict__ c_col, float *__restrict__ c_val) {
+    trigger_dependents();
     constexpr int R = ESC_SMALL_ROWS;
     const int w = ((blockIdx.x * 256 + threadIdx.x) >> 5) * R;
     if (w >= n_rows) return;
@@ -389,6 +418,7 @@ __global__ void __launch_bounds__(256) k_esc_small(CsrView A, CsrView B, const i
             c_val[pos] = acc;
         }
     }
+    finish_after_previous();
 }
 
 // ------------------------------------------------------------------------ medium rows ----
@@ -402,6 +432,7 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
     __shared__ uint64_t keys[MEDIUM_P];
     __shared__ float vals[NUMERIC ? MEDIUM_P : 1];
     __shared__ int scan_tmp[40];
+    trigger_dependents();
     const int tid = threadIdx.x;
     const int32_t i = ld_nc(row_list + blockIdx.x);
     const int32_t lo = ld_nc(A.rp + i), hi = ld_nc(A.rp + i + 1);
@@ -453,12 +484,9 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
     for (int p = p_lo; p < p_hi; ++p) heads += p == 0 || (uint32_t)(keys[p] >> 32) != (uint32_t)(keys[p - 1] >> 32);
     int unique;
     int rank = block_excl_sum<MED_NT>(heads, scan_tmp, unique);
-    if (!NUMERIC) {
-        if (tid == 0) row_count[i] = unique;
-        return;
-    }
-    const int32_t out = ld_nc(c_rp + i);
-    for (int p = p_lo; p < p_hi; ++p) {
+    if (!NUMERIC && tid == 0) row_count[i] = unique;
+    const int32_t out = NUMERIC ? ld_nc(c_rp + i) : 0;
+    for (int p = p_lo; NUMERIC && p < p_hi; ++p) {
         const uint32_t col = (uint32_t)(keys[p] >> 32);
         if (p == 0 || col != (uint32_t)(keys[p - 1] >> 32)) {
             float acc = vals[(uint32_t)keys[p]];
@@ -468,6 +496,7 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
             ++rank;
         }
     }
+    finish_after_previous();
 }
 
 // ----------------------------------------------------------------- product walk ----
@@ -636,6 +665,7 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
     __shared__ float seg_a[NUMERIC ? NT : 1];
     __shared__ int scan_tmp[72];
     __shared__ int warp_base[NT / 32];
+    trigger_dependents();
     const int tid = threadIdx.x;
     const int r = blockIdx.x;
     const int32_t i = ld_nc(row_list + (r < n_front ? r : list_len - 1 - (r - n_front)));
@@ -784,14 +814,107 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
         out += cnt;
     }
     if (!NUMERIC && tid == 0) row_count[i] = (int32_t)out;
+    finish_after_previous();
 }
 
-// Turns the exclusive prefix of the per-row counts into row offsets (rows + 1 entries).
-__global__ void __launch_bounds__(256) k_esc_row_offsets(const int32_t *__restrict__ excl, const long long *__restrict__ total,
-                                                         int32_t rows, int32_t *__restrict__ c_rp) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < rows) c_rp[i] = excl[i];
-    if (i == rows) c_rp[rows] = (int32_t)min(*total, (long long)INT32_MAX);
+// ------------------------------------------------------------- matrices of short rows ----
+
+constexpr int SHORT_NT = 128, SHORT_ENTRIES = 8;
+
+// The whole product in one pass, for matrices whose rows of A hold at most K <= 8 entries and reach at
+// most SMALL_P products (meshes, bands). One THREAD merges one row: the K rows of B are sorted lists whose
+// heads it keeps in registers; a step takes the smallest head and adds up the lists that hold it, in the
+// order of A's entries (ascending j, the same sum as the other kernels form). A row is staged in shared memory
+// at the offset of its product count, the CTA's result count goes through the cross-tile scan of the merge
+// kernels, and the rows are copied out eight lanes to a row. 512 x 512 5-point mesh squared: a warp per row with
+// a 32-wide bitonic sort, counting first, took 240 instructions a row and 156 us in two kernels.
+template <int K>
+__global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, int32_t rows, TileWords words, FusedCtl *ctl, int num_tiles,
+                                                       int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col, float *__restrict__ c_val,
+                                                       unsigned long long *word) {
+    constexpr uint32_t END = 0xffffffffu;
+    __shared__ uint32_t s_col[SHORT_NT * SMALL_P];
+    __shared__ float s_val[SHORT_NT * SMALL_P];
+    __shared__ int scan_tmp[40];
+    __shared__ long long s_base;
+    auto finish = [&](long long total) {
+        __threadfence();
+        const bool bad = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0;
+        publish_result_word(word, bad ? NB200_E_TIMEOUT : NB200_OK, bad ? 0 : total);
+    };
+    const bool scanned = num_tiles > DIRECT_TILES;
+    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no rows
+        if (threadIdx.x < 32) {
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+            if (threadIdx.x == 0) finish(total);
+        }
+        return;
+    }
+    const int t = blockIdx.x - (scanned ? 1 : 0), tid = threadIdx.x, lane = lane_id();
+    const int64_t i = (int64_t)t * SHORT_NT + tid;
+    const int32_t lo = i < rows ? ld_nc(A.rp + i) : 0, hi = i < rows ? ld_nc(A.rp + i + 1) : 0;
+    int32_t pos[K], end[K];
+    uint32_t head[K];
+    float a[K];
+    int products = 0;
+#pragma unroll
+    for (int e = 0; e < K; ++e) {
+        const int32_t j = lo + e < hi ? ld_nc(A.col + lo + e) : -1;
+        a[e] = j >= 0 ? ld_nc(A.val + lo + e) : 0.f;
+        pos[e] = j >= 0 ? ld_nc(B.rp + j) : 0;
+        end[e] = j >= 0 ? ld_nc(B.rp + j + 1) : 0;
+        products += end[e] - pos[e];
+    }
+#pragma unroll
+    for (int e = 0; e < K; ++e) head[e] = pos[e] < end[e] ? (uint32_t)ld_nc(B.col + pos[e]) : END;
+    int tile_products;
+    const int staged = block_excl_sum<SHORT_NT>(products, scan_tmp, tile_products);
+    int count = 0;
+    for (;;) {
+        uint32_t m = head[0];
+#pragma unroll
+        for (int e = 1; e < K; ++e) m = min(m, head[e]);
+        if (m == END) break;
+        float acc = 0.f;
+        bool first = true;
+#pragma unroll
+        for (int e = 0; e < K; ++e) {
+            if (head[e] == m) {
+                const float v = a[e] * ld_nc(B.val + pos[e]);
+                acc = first ? v : acc + v;
+                first = false;
+                ++pos[e];
+                head[e] = pos[e] < end[e] ? (uint32_t)ld_nc(B.col + pos[e]) : END;
+            }
+        }
+        s_col[staged + count] = m;
+        s_val[staged + count] = acc;
+        ++count;
+    }
+    int total;
+    const int rank = block_excl_sum<SHORT_NT>(count, scan_tmp, total);
+    if (tid == 0) publish_count(words, t, total);
+    if (warp_id() == 0) {
+        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+        if (lane == 0) {
+            s_base = b;
+            if (t == num_tiles - 1 && !scanned) finish(b < 0 ? b : b + total);
+        }
+    }
+    __syncthreads();
+    const long long base = s_base;
+    if (base < 0) return;  // a bounded wait gave up; the host reports it
+    if (i < rows) c_rp[i] = (int32_t)(base + rank);
+    if (t == num_tiles - 1 && tid == 0) c_rp[rows] = (int32_t)(base + total);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const int r = 4 * s + (lane >> 3);
+        const int n = __shfl_sync(FULL_MASK, count, r), from = __shfl_sync(FULL_MASK, staged, r), to = __shfl_sync(FULL_MASK, rank, r);
+        for (int q = lane & 7; q < n; q += 8) {
+            c_col[base + to + q] = (int32_t)s_col[from + q];
+            c_val[base + to + q] = s_val[from + q];
+        }
+    }
 }
 
 // ------------------------------------------------------------------------ host driver ----
@@ -824,7 +947,10 @@ struct EscPlan {
     int32_t *win_ptr;      // window pointer table (null: one window, or beyond its budget)
     uint32_t *cache_ranked, *cache_heavy;  // bitmaps carried from the symbolic to the numeric pass (or null)
     Workspace *cache_ws;   // pool block of the bitmaps (null without them)
-    EscCtl host;           // counters read back after the row-work kernel
+    EscCtl host;           // counters reported by the binning kernel
+    uint64_t *short_block; // FusedCtl + tile words of the short-row kernel
+    int short_tiles;
+    unsigned long long *words;
 };
 
 // Bins the rows (kernel + one read-back) and carves the scratch of a symbolic pass, a numeric
@@ -837,16 +963,19 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     const int64_t n_win = std::max<int64_t>(1, ((int64_t)b->cols + RK_WINDOW_COLS - 1) / RK_WINDOW_COLS);
     const size_t ptr_entries = n_win > 1 ? (size_t)b->rows * (size_t)(n_win + 1) : 0;
     const bool with_table = ptr_entries > 0 && ptr_entries * 4 <= RK_PTR_BUDGET;
-    const int scan_ctas = (rows + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT);
+    const int scan_ctas = (int)(((int64_t)rows + 1 + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT));
     Carver sizes;
     for (int q = 0; q < 4; ++q) sizes.take<int32_t>((size_t)rows);
     sizes.take<int32_t>((size_t)rows + 1);
-    sizes.take<uint64_t>((size_t)scan_ctas + 8);
-    sizes.take<EscCtl>(1);
     if (with_table) sizes.take<int32_t>(ptr_entries);
     const int prefix_ctas = (int)(((int64_t)a->nnz + 1 + 2047) / 2048);
+    const int short_tiles = (int)(((int64_t)rows + SHORT_NT - 1) / SHORT_NT);
     sizes.take<unsigned long long>((size_t)a->nnz + 1);
+    const size_t clear_from = sizes.used();
+    sizes.take<uint64_t>((size_t)scan_ctas + 8);
+    sizes.take<EscCtl>(1);
     sizes.take<uint64_t>((size_t)prefix_ctas + 8);
+    sizes.take<uint64_t>(TileWords::needed(short_tiles) + 4);
     int st;
     if ((st = acquire_workspace(stream, sizes.used(), &plan->ws))) return st;
     Carver carve(plan->ws->dev);
@@ -855,21 +984,26 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     plan->lists.ranked_rows = carve.take<int32_t>((size_t)rows);
     plan->lists.heavy_rows = carve.take<int32_t>((size_t)rows);
     plan->row_count = carve.take<int32_t>((size_t)rows + 1);
-    plan->scan_block = carve.take<uint64_t>((size_t)scan_ctas + 8);
-    plan->scan_ctas = scan_ctas;
-    plan->ctl = carve.take<EscCtl>(1);
     plan->n_win = (int)n_win;
     plan->win_ptr = with_table ? carve.take<int32_t>(ptr_entries) : nullptr;
     unsigned long long *prefix = carve.take<unsigned long long>((size_t)a->nnz + 1);
+    plan->scan_block = carve.take<uint64_t>((size_t)scan_ctas + 8);
+    plan->scan_ctas = scan_ctas;
+    plan->ctl = carve.take<EscCtl>(1);
     uint64_t *prefix_block = carve.take<uint64_t>((size_t)prefix_ctas + 8);
+    plan->short_block = carve.take<uint64_t>(TileWords::needed(short_tiles) + 4);
+    plan->short_tiles = short_tiles;
+    plan->words = result_word(plan->ws, 0);
+    for (int k = 1; k < W_COUNT; ++k) result_word(plan->ws, k);
 
-    NB200_CUDA(cudaMemsetAsync(plan->ctl, 0, sizeof(EscCtl), stream));
-    NB200_CUDA(cudaMemsetAsync(prefix_block, 0, sizeof(uint64_t) * ((size_t)prefix_ctas + 8), stream));
+    // every control block and tile word of the call lies in one piece: one fill clears them all
+    NB200_CUDA(cudaMemsetAsync(static_cast<unsigned char *>(plan->ws->dev) + clear_from, 0, carve.used() - clear_from, stream));
+    plan->host = EscCtl{};
     const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
     const bool short_rows = (int64_t)a->nnz <= 8 * (int64_t)rows;  // then a lane walks its row faster than a prefix pass pays
     if (rows > 0 && short_rows) {
         LaunchScope scope("esc_rowwork", stream);
-        k_esc_rowwork_walk<<<(rows + 255) / 256, 256, 0, stream>>>(A, B, rows, counts ? plan->row_count : nullptr, plan->lists, plan->ctl);
+        k_esc_rowwork_walk<<<(rows + 255) / 256, 256, 0, stream>>>(A, B, rows, counts ? plan->row_count : nullptr, plan->lists, plan->ctl, plan->words);
         NB200_CUDA(cudaGetLastError());
     } else if (rows > 0) {
         {
@@ -877,17 +1011,22 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
             k_esc_product_prefix<<<prefix_ctas, 256, 0, stream>>>(A, B, a->nnz, prefix, prefix_block + 4, reinterpret_cast<FusedCtl *>(prefix_block));
         }
         LaunchScope scope("esc_rowwork", stream);
-        k_esc_rowwork<<<(rows + 255) / 256, 256, 0, stream>>>(A, prefix, rows, counts ? plan->row_count : nullptr, plan->lists, plan->ctl);
-        NB200_CUDA(cudaGetLastError());
+        NB200_CUDA(launch_overlapped(k_esc_rowwork, dim3((rows + 255) / 256), dim3(256), 0, stream, A, prefix, rows, counts ? plan->row_count : nullptr,
+                                     plan->lists, plan->ctl, reinterpret_cast<const FusedCtl *>(prefix_block), plan->words));
     }
-    NB200_CUDA(cudaMemcpyAsync(plan->ws->host, plan->ctl, sizeof(EscCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaMemcpyAsync(plan->ws->host + 16, prefix_block, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaStreamSynchronize(stream));
-    std::memcpy(&plan->host, plan->ws->host, sizeof(EscCtl));
-    {   // a prefix whose look-back gave up leaves rows with wrong product counts: nothing may be built on them
-        FusedCtl hp;
-        std::memcpy(&hp, plan->ws->host + 16, sizeof(hp));
-        if (hp.status.error != 0) return note_timeout(hp.status.error, hp.status.detail, "spgemm product prefix");
+    if (rows > 0) {
+        int64_t v[W_NNZ];
+        int device_status = 0, failed = 0;
+        for (int k = 0; k < W_NNZ; ++k) {
+            if ((st = wait_result_word(plan->words + k, stream, &v[k], &device_status))) return st;
+            failed |= device_status;
+        }
+        // a prefix whose look-back gave up leaves rows with wrong product counts: nothing may be built on them
+        if (failed) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm product prefix");
+        plan->host.products = (unsigned long long)v[W_PRODUCTS];
+        plan->host.n_small = (int)v[W_SMALL], plan->host.n_medium = (int)v[W_MEDIUM], plan->host.n_ranked = (int)v[W_RANKED];
+        plan->host.n_giant = (int)v[W_GIANT], plan->host.n_heavy = (int)v[W_HEAVY];
+        plan->host.max_entries = short_rows ? (int)v[W_ENTRIES] : INT_MAX;
     }
     if (with_table && plan->host.n_ranked + plan->host.n_giant + plan->host.n_heavy > 0) {
         LaunchScope scope("esc_window_ptr", stream);
@@ -919,10 +1058,24 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     return NB200_OK;
 }
 
+// The bins of a pass touch different rows, so each kernel after the first starts beside the one before it
+// (a few hub rows on as many CTAs would otherwise leave the rest of the chip idle: 16 of them took 150 us of
+// 780 on a graph of 24405 vertices).
+template <typename... P, typename... V>
+int launch_bin(bool beside, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, V... args) {
+    if (beside) {
+        NB200_CUDA(launch_overlapped(kernel, dim3(grid), dim3(block), smem, stream, args...));
+    } else {
+        kernel<<<grid, block, smem, stream>>>(args...);
+        NB200_CUDA(cudaGetLastError());
+    }
+    return NB200_OK;
+}
+
 template <bool NUMERIC, int NT>
 int launch_ranked(const CsrView &A, const CsrView &B, const EscPlan &plan, int32_t b_cols, const int32_t *list, int32_t list_len,
                   int n_front, int n_rows, uint32_t *cache, int32_t *count, const int32_t *c_rp, int32_t *c_col, float *c_val,
-                  cudaStream_t stream) {
+                  cudaStream_t stream, bool beside) {
     int wshift = 5;
     const int words = ranked_words(NT, b_cols, &wshift);
     // numeric: whatever the bitmap and the ranks leave of the CTA's shared memory accumulates sums
@@ -934,10 +1087,8 @@ int launch_ranked(const CsrView &A, const CsrView &B, const EscPlan &plan, int32
     const size_t smem = NUMERIC ? (size_t)words * 5 + (size_t)acc_slots * 4 : (size_t)words * 4;
     NB200_CUDA(cudaFuncSetAttribute(k_esc_ranked<NUMERIC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(NUMERIC ? budget : (size_t)RK_WORDS * 4)));
-    k_esc_ranked<NUMERIC, NT><<<n_rows, NT, smem, stream>>>(A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift,
-                                                          acc_slots, cache, count, c_rp, c_col, c_val);
-    NB200_CUDA(cudaGetLastError());
-    return NB200_OK;
+    return launch_bin(beside, k_esc_ranked<NUMERIC, NT>, n_rows, NT, smem, stream, A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift,
+                      acc_slots, cache, count, c_rp, c_col, c_val);
 }
 
 template <bool NUMERIC>
@@ -949,32 +1100,33 @@ int esc_run_bins(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, co
     float *c_val = NUMERIC ? c->val : nullptr;
     int st;
     const int n_heavy = plan.host.n_giant + plan.host.n_heavy;
+    bool beside = false;
     if (n_heavy > 0) {  // first: the heaviest rows take longest
         LaunchScope scope(NUMERIC ? "esc_heavy_numeric" : "esc_heavy_symbolic", stream);
         if ((st = launch_ranked<NUMERIC, HEAVY_NT>(A, B, plan, b->cols, plan.lists.heavy_rows, a->rows, plan.host.n_giant, n_heavy,
-                                                             plan.cache_heavy, count, c_rp, c_col, c_val, stream)))
+                                                             plan.cache_heavy, count, c_rp, c_col, c_val, stream, false)))
             return st;
+        beside = true;
     }
     if (plan.host.n_ranked > 0) {
         LaunchScope scope(NUMERIC ? "esc_ranked_numeric" : "esc_ranked_symbolic", stream);
         if ((st = launch_ranked<NUMERIC, RK_NT>(A, B, plan, b->cols, plan.lists.ranked_rows, a->rows, plan.host.n_ranked,
-                                                          plan.host.n_ranked, plan.cache_ranked, count, c_rp, c_col, c_val, stream)))
+                                                          plan.host.n_ranked, plan.cache_ranked, count, c_rp, c_col, c_val, stream, beside)))
             return st;
+        beside = true;
     }
     if (plan.host.n_medium > 0) {
         LaunchScope scope(NUMERIC ? "esc_medium_numeric" : "esc_medium_symbolic", stream);
-        k_esc_medium<NUMERIC><<<plan.host.n_medium, MED_NT, 0, stream>>>(A, B, plan.lists.medium_rows, count, c_rp, c_col, c_val);
-        NB200_CUDA(cudaGetLastError());
+        if ((st = launch_bin(beside, k_esc_medium<NUMERIC>, plan.host.n_medium, MED_NT, 0, stream, A, B, plan.lists.medium_rows, count, c_rp, c_col, c_val)))
+            return st;
+        beside = true;
     }
     if (plan.host.n_small > 0) {
         LaunchScope scope(NUMERIC ? "esc_small_numeric" : "esc_small_symbolic", stream);
         const int warps = plan.host.n_small;  // rows on the list
         const int small_warps = (warps + ESC_SMALL_ROWS - 1) / ESC_SMALL_ROWS;
-        if (b->cols < (1 << 27))
-            k_esc_small<NUMERIC, true><<<(small_warps + 7) / 8, 256, 0, stream>>>(A, B, plan.lists.small_rows, warps, count, c_rp, c_col, c_val);
-        else
-            k_esc_small<NUMERIC, false><<<(small_warps + 7) / 8, 256, 0, stream>>>(A, B, plan.lists.small_rows, warps, count, c_rp, c_col, c_val);
-        NB200_CUDA(cudaGetLastError());
+        auto kernel = b->cols < (1 << 27) ? k_esc_small<NUMERIC, true> : k_esc_small<NUMERIC, false>;
+        if ((st = launch_bin(beside, kernel, (small_warps + 7) / 8, 256, 0, stream, A, B, plan.lists.small_rows, warps, count, c_rp, c_col, c_val))) return st;
     }
     return NB200_OK;
 }
@@ -995,14 +1147,15 @@ struct SavedPlan {
     uint64_t gen_main = 0, gen_cache = 0, epoch = 0;
 };
 std::mutex g_saved_mutex;
-SavedPlan g_saved;
+SavedPlan g_after_symbolic;  // for a numeric pass
+SavedPlan g_after_bound;     // rows are binned and the control blocks clear: for the one symbolic or one-pass call that follows
 
-void save_plan(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, const EscPlan &plan, cudaStream_t stream) {
+void save_plan(SavedPlan &g_saved, const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, const EscPlan &plan, cudaStream_t stream) {
     std::lock_guard<std::mutex> g(g_saved_mutex);
     g_saved.valid = cudaGetDevice(&g_saved.device) == cudaSuccess;
     g_saved.plan = plan;
     g_saved.a_rp = a->row_ptr, g_saved.a_col = a->col, g_saved.b_rp = b->row_ptr, g_saved.b_col = b->col;
-    g_saved.c_rp = c->row_ptr, g_saved.c_nnz = c->nnz;
+    g_saved.c_rp = c ? c->row_ptr : nullptr, g_saved.c_nnz = c ? c->nnz : 0;
     g_saved.a_rows = a->rows, g_saved.a_nnz = a->nnz, g_saved.b_rows = b->rows, g_saved.b_cols = b->cols, g_saved.b_nnz = b->nnz;
     g_saved.stream = stream;
     g_saved.epoch = workspace_epoch();
@@ -1010,19 +1163,20 @@ void save_plan(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, const
     g_saved.gen_cache = plan.cache_ws ? plan.cache_ws->generation : 0;
 }
 
-bool take_saved_plan(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, cudaStream_t stream, EscPlan *out) {
+bool take_saved_plan(SavedPlan &g_saved, const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, cudaStream_t stream, EscPlan *out) {
     std::lock_guard<std::mutex> g(g_saved_mutex);
     int dev = -1;
     if (!g_saved.valid || g_saved.epoch != workspace_epoch()) return false;  // the pool blocks may be gone
     if (cudaGetDevice(&dev) != cudaSuccess || dev != g_saved.device || stream != g_saved.stream) return false;
     if (a->row_ptr != g_saved.a_rp || a->col != g_saved.a_col || b->row_ptr != g_saved.b_rp || b->col != g_saved.b_col) return false;
-    if (c->row_ptr != g_saved.c_rp || c->nnz != g_saved.c_nnz) return false;  // row offsets obtained elsewhere: recompute
+    if (c && (c->row_ptr != g_saved.c_rp || c->nnz != g_saved.c_nnz)) return false;  // row offsets obtained elsewhere: recompute
     if (a->rows != g_saved.a_rows || a->nnz != g_saved.a_nnz || b->rows != g_saved.b_rows || b->cols != g_saved.b_cols ||
         b->nnz != g_saved.b_nnz)
         return false;
     if (g_saved.plan.ws->generation != g_saved.gen_main) return false;
     if (g_saved.plan.cache_ws && g_saved.plan.cache_ws->generation != g_saved.gen_cache) return false;
     *out = g_saved.plan;
+    if (!c) g_saved.valid = false;  // its cleared control blocks serve one call
     return true;
 }
 
@@ -1042,31 +1196,23 @@ int spgemm_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_
         return NB200_OK;
     }
     EscPlan plan{};
-    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+    if (!take_saved_plan(g_after_bound, a, b, nullptr, stream, &plan) && (st = esc_prepare(a, b, true, true, stream, &plan))) return st;
     if (keep) *keep = plan;
     if (products) *products = (int64_t)plan.host.products;
     if ((st = esc_run_bins<false>(a, b, plan, nullptr, stream))) return st;
-    FusedCtl *scan_ctl = reinterpret_cast<FusedCtl *>(plan.scan_block);
-    NB200_CUDA(cudaMemsetAsync(plan.scan_block, 0, sizeof(uint64_t) * ((size_t)plan.scan_ctas + 4), stream));
     {
-        LaunchScope scope("scan_lookback", stream);
-        k_scan_lookback<<<plan.scan_ctas, SCAN_NT, 0, stream>>>(plan.row_count, a->rows, plan.scan_block + 4, scan_ctl);
+        LaunchScope scope("esc_scan_offsets", stream);
+        k_scan_offsets<<<plan.scan_ctas, SCAN_NT, 0, stream>>>(plan.row_count, a->rows, c->row_ptr, plan.scan_block + 4,
+                                                              reinterpret_cast<FusedCtl *>(plan.scan_block), plan.words + W_NNZ);
         NB200_CUDA(cudaGetLastError());
     }
-    {
-        LaunchScope scope("esc_row_offsets", stream);
-        k_esc_row_offsets<<<(a->rows + 256) / 256, 256, 0, stream>>>(plan.row_count, &scan_ctl->total, a->rows, c->row_ptr);
-        NB200_CUDA(cudaGetLastError());
-    }
-    NB200_CUDA(cudaMemcpyAsync(plan.ws->host, scan_ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaStreamSynchronize(stream));
-    FusedCtl h;
-    std::memcpy(&h, plan.ws->host, sizeof(h));
-    if (h.status.error != 0) return note_timeout(h.status.error, h.status.detail, "spgemm row scan");
-    const int64_t nnz = h.total;
+    int64_t nnz;
+    int device_status;
+    if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
+    if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm row scan");
     if (nnz > INT32_MAX) return NB200_E_OVERFLOW;
     c->nnz = (int32_t)nnz;
-    save_plan(a, b, c, plan, stream);
+    save_plan(g_after_symbolic, a, b, c, plan, stream);
     return NB200_OK;
 }
 
@@ -1079,9 +1225,64 @@ int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *s
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     if (kept) return esc_run_bins<true>(a, b, *kept, c, stream);
     EscPlan plan{};
-    if (take_saved_plan(a, b, c, stream, &plan)) return esc_run_bins<true>(a, b, plan, c, stream);
+    if (take_saved_plan(g_after_symbolic, a, b, c, stream, &plan)) return esc_run_bins<true>(a, b, plan, c, stream);
     if ((st = esc_prepare(a, b, false, false, stream, &plan))) return st;
     return esc_run_bins<true>(a, b, plan, c, stream);
+}
+
+bool is_short(const EscPlan &plan) {
+    return plan.host.n_medium + plan.host.n_ranked + plan.host.n_giant + plan.host.n_heavy == 0 && plan.host.max_entries <= SHORT_ENTRIES &&
+           plan.host.products > 0 && plan.host.products <= INT32_MAX;
+}
+
+// Bins the rows; *capacity receives the number of entries with which spgemm_into runs in one pass (the number
+// of products, an upper bound of nnz(C)) if the matrices are of the kind it can do that for, else 0.
+int spgemm_bound(const nb200_csr *a, const nb200_csr *b, int64_t *capacity, void *stream_v) {
+    int st;
+    if ((st = check_operand(a)) || (st = check_operand(b))) return st;
+    if (!capacity || a->cols != b->rows) return NB200_E_BADARG;
+    *capacity = 0;
+    if (a->rows == 0) return NB200_OK;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    EscPlan plan{};
+    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+    save_plan(g_after_bound, a, b, nullptr, plan, stream);
+    if (is_short(plan)) *capacity = (int64_t)plan.host.products;
+    return NB200_OK;
+}
+
+int spgemm_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t capacity, void *stream_v) {
+    int st;
+    if ((st = check_operand(a)) || (st = check_operand(b))) return st;
+    if (!c || !c->row_ptr || a->cols != b->rows || capacity < 0 || (capacity > 0 && (!c->col || !c->val))) return NB200_E_BADARG;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    EscPlan plan{};
+    if (a->rows > 0) {
+        if (!take_saved_plan(g_after_bound, a, b, nullptr, stream, &plan) && (st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+        if (is_short(plan) && capacity >= (int64_t)plan.host.products) {
+            c->rows = a->rows, c->cols = b->cols, c->nnz = 0;
+            const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
+            FusedCtl *ctl = reinterpret_cast<FusedCtl *>(plan.short_block);
+            const TileWords words = TileWords::at(plan.short_block + 4, plan.short_tiles);
+            auto kernel = plan.host.max_entries <= 4 ? k_esc_short<4> : plan.host.max_entries <= 6 ? k_esc_short<6> : k_esc_short<8>;
+            {
+                LaunchScope scope("esc_short", stream);
+                kernel<<<plan.short_tiles + (plan.short_tiles > DIRECT_TILES ? 1 : 0), SHORT_NT, 0, stream>>>(
+                    A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.words + W_NNZ);
+                NB200_CUDA(cudaGetLastError());
+            }
+            int64_t nnz;
+            int device_status;
+            if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
+            if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm of short rows");
+            c->nnz = (int32_t)nnz;
+            return NB200_OK;
+        }
+        save_plan(g_after_bound, a, b, nullptr, plan, stream);
+    }
+    if ((st = spgemm_symbolic(a, b, c, nullptr, stream_v))) return st;
+    if (c->nnz > capacity) return NB200_E_CAPACITY;
+    return spgemm_numeric(a, b, c, stream_v);
 }
 
 }  // namespace
@@ -1091,6 +1292,14 @@ int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *s
 using namespace nb200;
 
 extern "C" {
+
+int nb200_spgemm_f32_bound(const nb200_csr *a, const nb200_csr *b, int64_t *capacity, void *stream) {
+    return spgemm_bound(a, b, capacity, stream);
+}
+
+int nb200_spgemm_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t capacity, void *stream) {
+    return spgemm_into(a, b, c, capacity, stream);
+}
 
 int nb200_spgemm_f32_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t *products, void *stream) {
     return spgemm_symbolic(a, b, c, products, stream);
