@@ -6,17 +6,18 @@
 // merge-path with the rule that equal coordinates are never split
 // (src/backend/partition.cpp:813-993, :964-983). Here each coordinate is packed into one
 // 64-bit key, i in the top bits, then j, then k, using just enough bits for each extent, so
-// that tuple order is integer order. Tensors whose three extents need more than 63 bits in
-// total take a second, simpler tile kernel that compares (i, j) and k as a 64-bit and a 32-bit
-// word, i.e. the full three-int32 tuple compare of the reference for any extents.
+// that tuple order is integer order; inside a tile the keys are counted from its smallest and then nearly
+// always fit 32 bits. Tensors whose three extents need more than 63 bits in total take a second, simpler
+// tile kernel that compares (i, j) and k as a 64-bit and a 32-bit word, i.e. the full three-int32 tuple
+// compare of the reference for any extents.
 //
-// Kernels: k_coo3_partition (one warp per tile cut, 32-ary diagonal search) and k_coo3_tile
-// (one CTA per tile: pack keys into shared memory, split by merge-path, merge VT entries per
-// thread, rank survivors, obtain the output base -- single pass with bounded look-back, or
-// from the scanned counts of a first pass -- compact through shared memory, store coalesced).
+// Kernels: k_coo3_partition (tile cuts) and k_coo3_tile (one CTA per tile: stage and pack the coordinates,
+// split by merge-path, merge VT entries per thread, rank survivors, obtain the output base -- single pass
+// with the cross-tile scan, or from the scanned counts of a first pass -- fetch values, store coalesced).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "merge_common.cuh"
 #include "tma.cuh"
@@ -25,20 +26,7 @@ namespace nb200 {
 
 namespace {
 
-#ifndef COO3_NT
-#define COO3_NT 256
-#endif
-#ifndef COO3_VT
-#define COO3_VT 11
-#endif
-#ifndef COO3_MIN_CTAS
-#define COO3_MIN_CTAS 4
-#endif
-constexpr int NT = COO3_NT;
-constexpr int VT = COO3_VT;
-constexpr int CAP = NT * VT;
-constexpr int KEY_SLOTS = CAP + 2 + VT;
-constexpr uint64_t INF = ~0ull;
+constexpr int NT = 256;
 
 struct Coo3In {
     const int32_t *i, *j, *k;
@@ -49,6 +37,8 @@ struct Coo3In {
 struct Coo3Out {
     int32_t *i, *j, *k;
     float *val;
+    unsigned long long *host = nullptr;  // result word: the length, or for a reduction that it is done
+    float *scalar = nullptr;             // result of a reduction
 };
 
 struct Packing {
@@ -87,80 +77,56 @@ __device__ __forceinline__ typename PK::Key key_at(const Coo3In &T, const PK &pk
     return pk.pack(ld_nc(T.i + p), ld_nc(T.j + p), ld_nc(T.k + p));
 }
 
-// Tile cuts, found in two levels so that the searches read little: every COARSE-th cut by one
-// warp with a 32-ary search over the whole diagonal (few cuts, many probes each), then every
-// other cut by one thread with a binary search between its two coarse neighbours (many cuts,
-// few probes each). Cut t sits at merged position min(t * tile_step, total); equal coordinates
-// stay on one side of a cut.
-constexpr int COARSE = 32;
-
-template <typename PK>
-__device__ __forceinline__ void finish_cut(const Coo3In &A, const Coo3In &B, const PK &pk, int64_t d, int64_t x,
-                                           int32_t *pa, int32_t *pb) {
-    int64_t y = d - x;
-    if (x > 0 && y < B.nnz && key_at(A, pk, x - 1) == key_at(B, pk, y)) ++y;
-    *pa = (int32_t)x;
-    *pb = (int32_t)y;
+// Whether A's entry m orders before B's entry p or is the same position, by tuple order; j and k are read only
+// where i (and j) do not decide: most probes of a search end after two loads instead of six.
+__device__ __forceinline__ bool at_or_before(const Coo3In &A, int64_t m, const Coo3In &B, int64_t p) {
+    const int32_t ia = ld_nc(A.i + m), ib = ld_nc(B.i + p);
+    if (ia != ib) return ia < ib;
+    const int32_t ja = ld_nc(A.j + m), jb = ld_nc(B.j + p);
+    if (ja != jb) return ja < jb;
+    return ld_nc(A.k + m) <= ld_nc(B.k + p);
 }
 
-template <typename PK>
-__global__ void __launch_bounds__(NT) k_coo3_partition_coarse(Coo3In A, Coo3In B, PK pk, int64_t total, int32_t tile_step,
-                                                              int32_t num_tiles, Cuts2 cuts) {
-    const int c = (blockIdx.x * NT + threadIdx.x) >> 5;
-    const int64_t t64 = (int64_t)c * COARSE;
-    if (t64 > num_tiles + COARSE - 1) return;
-    const int t = (int)min(t64, (int64_t)num_tiles);  // the last coarse cut is the end of the data
-    const int64_t d = (int64_t)t * tile_step;
-    int32_t pa, pb;
-    if (t == 0) {
-        pa = pb = 0;
-    } else if (t == num_tiles || d >= total) {
+// Tile cuts, G lanes per cut. Cut t sits at merged position min(t * tile_step, total); equal coordinates stay on one
+// side of a cut. `stride` > 1: only every stride-th cut (and the last) is made. `between` > 0: only the cuts that
+// a launch with that stride left out, each searched between its two neighbours among those. The control block and
+// the tile words of the tile kernel are cleared on the way.
+template <int G>
+__global__ void __launch_bounds__(NT) k_coo3_partition(Coo3In A, Coo3In B, int64_t total, int32_t tile_step, int32_t num_tiles, int stride, int between,
+                                                       Cuts2 cuts, uint64_t *zero_block, int zero_words) {
+    trigger_dependents();
+    const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
+    for (int64_t z = gid; z < zero_words; z += (int64_t)gridDim.x * NT) zero_block[z] = 0;
+    if (between) wait_for_previous();           // the cuts made so far
+    const int64_t t64 = gid / G * stride;
+    const int t = (int)min(t64, (int64_t)num_tiles);  // spare groups repeat the last cut
+    const bool mine = t64 < num_tiles + stride && !(between && (t % between == 0 || t == num_tiles));
+    const int64_t d = min((int64_t)t * tile_step, total);
+    const bool inner = t > 0 && t < num_tiles;
+    int64_t x_lo = max((int64_t)0, d - B.nnz), x_hi = min(d, (int64_t)A.nnz);
+    if (between && mine) {
+        const int before = t / between * between;
+        x_lo = max(x_lo, (int64_t)cuts.a[before]);
+        x_hi = min(x_hi, (int64_t)cuts.a[min(before + between, num_tiles)]);
+    }
+    const int64_t x = group_count_true<G>((uint32_t)x_lo, (uint32_t)(inner && mine ? x_hi : x_lo), [&](uint32_t m) { return at_or_before(A, m, B, d - 1 - m); });
+    int32_t pa = 0, pb = 0;
+    if (inner) {
+        int64_t y = d - x;
+        if (mine && x > 0 && y < B.nnz && ld_nc(A.i + x - 1) == ld_nc(B.i + y) && ld_nc(A.j + x - 1) == ld_nc(B.j + y) && ld_nc(A.k + x - 1) == ld_nc(B.k + y)) ++y;
+        pa = (int32_t)x;
+        pb = (int32_t)y;
+    } else if (t == num_tiles) {
         pa = A.nnz;
         pb = B.nnz;
-    } else {
-        const int64_t x_lo = d - B.nnz > 0 ? d - B.nnz : 0;
-        const int64_t x_hi = d < A.nnz ? d : A.nnz;
-        const int64_t x = warp_count_true(x_lo, x_hi, [&](int64_t m) { return key_at(A, pk, m) <= key_at(B, pk, d - 1 - m); });
-        finish_cut(A, B, pk, d, x, &pa, &pb);
     }
-    if (lane_id() == 0) {
+    if ((threadIdx.x & (G - 1)) == 0 && mine) {
         cuts.a[t] = pa;
         cuts.b[t] = pb;
     }
 }
 
-template <typename PK>
-__global__ void __launch_bounds__(NT) k_coo3_partition_fine(Coo3In A, Coo3In B, PK pk, int64_t total, int32_t tile_step,
-                                                            int32_t num_tiles, Cuts2 cuts) {
-    const int t = blockIdx.x * NT + threadIdx.x;
-    if (t >= num_tiles || t % COARSE == 0) return;
-    const int64_t d = (int64_t)t * tile_step;
-    int32_t pa, pb;
-    if (d >= total) {
-        pa = A.nnz;
-        pb = B.nnz;
-    } else {
-        const int c0 = t / COARSE * COARSE, c1 = min(c0 + COARSE, num_tiles);
-        int64_t lo = max((int64_t)cuts.a[c0], d - B.nnz > 0 ? d - B.nnz : 0);
-        int64_t hi = min((int64_t)cuts.a[c1], d < A.nnz ? d : (int64_t)A.nnz);
-        while (lo < hi) {  // first m with key_A(m) > key_B(d - 1 - m)
-            const int64_t mid = (lo + hi) >> 1;
-            if (key_at(A, pk, mid) <= key_at(B, pk, d - 1 - mid)) lo = mid + 1; else hi = mid;
-        }
-        finish_cut(A, B, pk, d, lo, &pa, &pb);
-    }
-    cuts.a[t] = pa;
-    cuts.b[t] = pb;
-}
-
-// Hardware barriers of the tile kernel: 0 = whole CTA, 1 = the NT worker threads, 2 = workers
-// arrive / the scan warp waits ("the tile's count is known").
-using WorkerBar = NamedBarrier<1, NT>;
-using CountBar = NamedBarrier<2, NT + 32>;
-using LevelBar = NamedBarrier<3, NT + 32>;  // second hand-over to the scan warp (CSF3 levels)
-
-constexpr int RAW_SLOTS = CAP + 16;  // words per staged raw array (i, j, k, value)
-static_assert(RAW_SLOTS >= KEY_SLOTS, "packed keys reuse the raw i and j arrays");
+constexpr int RW_COO3 = 8;  // index of the result word (the callers that lend their workspace use lower ones)
 constexpr int MBAR_POLL_LIMIT = 1 << 24;
 constexpr int ERR_COPY_TIMEOUT = 2;
 
@@ -169,354 +135,369 @@ __device__ __forceinline__ int head_elems(const void *p) {
     return (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) >> 2);
 }
 
-template <int MODE, bool CSF_OUT>
-__global__ void __launch_bounds__(NT + 32, COO3_MIN_CTAS) k_coo3_tile(Coo3In A, Coo3In B, Packing pk, Cuts2 cuts, int32_t *tile_count,
-                                                                 uint64_t *tile_state_raw, FusedCtl *ctl, Coo3Out Z,
-                                                                 CsfLevelsOut csf) {
-    static_assert(!CSF_OUT || MODE == MODE_FUSED, "the CSF3 levels are written by the single-pass launch only");
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ int scan_tmp[72];
-    __shared__ long long s_base, s_base_levels, s_levels;
-    __shared__ int s_hurry, s_hurry_levels;  // set once the tile's count / packed level count is out
-    __shared__ unsigned long long s_prev_key;
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ int s_total;
-    constexpr bool WRITES = MODE != MODE_COUNT;
-    volatile uint64_t *tile_state = tile_state_raw;
-    const int tid = threadIdx.x;
-    const bool scan_warp = tid >= NT;  // one extra warp: it only turns counts into output bases
-    int t = blockIdx.x;
-    if (tid == 0) {
-        mbar_init(&mbar, 1);
-        mbar_fence_init();
-        s_hurry = 0;
-        s_hurry_levels = 0;
+// All counts are in: the result length (negative after a give-up) goes to the control block and the host.
+__device__ __forceinline__ void coo3_finish(FusedCtl *ctl, const Coo3Out &Z, long long total) {
+    __threadfence();
+    const int status = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK;
+    if (total >= 0) ctl->total = total;
+    publish_result_word(Z.host, status, total < 0 ? 0 : total);
+}
+
+// One thread per tile, after the tile's sum: the last tile to get here writes the reduction's result.
+__device__ __forceinline__ void coo3_reduce_done(FusedCtl *ctl, const Coo3Out &Z, int num_tiles) {
+    __threadfence();
+    if (atomicAdd(&ctl->hollow, 1) != num_tiles - 1) return;
+    __threadfence();
+    *Z.scalar = (float)__longlong_as_double(*(volatile long long *)&ctl->total);
+    publish_result_word(Z.host, ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK, 0);
+}
+
+// Shared-memory plan of the tile body, in 4-byte words: three raw arrays (i, j, k), in which A's entry e sits
+// at word oa + e and B's at word ob + e, chosen so that 16-byte boundaries of global memory fall on 16-byte
+// boundaries here (what a bulk copy needs). Every entry's coordinates are packed in place: the key takes the
+// place of i (and, for 64-bit keys, of j), and the 16-bit source indices of the result take the place of an
+// array that is no longer needed.
+template <int VT>
+struct Coo3Plan {
+    static constexpr int CAP = NT * VT;
+    static constexpr int SLOTS = CAP + 16;
+    static constexpr size_t BYTES = 12 * (size_t)SLOTS;
+    static_assert(4 * SLOTS < 32768, "byte offsets of entries are kept in 15 bits");
+};
+constexpr int GATHER = 8;  // result entries a thread fetches together
+
+struct Coo3Shared {
+    uint64_t mbar;
+    long long base;  // output base of the tile
+    int wtotal[NT / 32];
+    double partial[NT / 32];
+};
+
+// One tile. NARROW: the keys of the tile, counted from its smallest, fit 32 bits (true of nearly every tile of
+// a tensor of millions of entries); otherwise they are kept as a low and a high word.
+//
+// The structure is that of the CSR tile kernel (csr_merge.cu), without rows: coordinates alone are staged and
+// merged, one result entry per step; a 16-bit source index per result entry is compacted; the count goes out
+// before the values are fetched from L2, where a prefetch has brought them. REDUCE (inner product): only
+// the coordinates both operands hold are kept, and their products summed.
+//
+// Bound by instruction issue and the latency of a tile's barrier-separated phases, at a bit over half of the copy
+// rate; 100 M entries per operand: 1550 us with staged values, 64-bit keys in a serial merge of 11 entries per
+// thread and a look-back per tile, 1195 us in this form.
+template <int VT, int MODE, bool NARROW>
+__device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, const Packing &pk, const int32_t a0, const int32_t b0, const int na,
+                                          const int nb, const int oa, const int ob, const uint64_t key0, const int t, const int num_tiles,
+                                          int32_t *tile_count, const TileWords &words, FusedCtl *ctl, const Coo3Out &Z,
+                                          unsigned char *smem_raw, Coo3Shared &sh) {
+    using P = Coo3Plan<VT>;
+    using Key = typename std::conditional<NARROW, uint32_t, uint64_t>::type;
+    constexpr Key END = (Key)~(Key)0;
+    constexpr bool REDUCE = MODE == MODE_REDUCE;
+    constexpr uint32_t HIGH = 4 * P::SLOTS;  // byte distance from a key's low to its high word
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = na + nb;
+    uint32_t *raw = reinterpret_cast<uint32_t *>(smem_raw);
+    uint16_t *src_of = reinterpret_cast<uint16_t *>(raw + (NARROW ? 1 : 2) * P::SLOTS);
+    auto word_at = [&](uint32_t byte) -> uint32_t & { return *reinterpret_cast<uint32_t *>(smem_raw + byte); };
+    auto key_at_byte = [&](uint32_t byte) -> Key {
+        return NARROW ? (Key)word_at(byte) : (Key)((uint64_t)word_at(byte + HIGH) << 32 | word_at(byte));
+    };
+
+    // ---- pack
+#pragma unroll
+    for (int q = 0; q < VT; ++q) {
+        const int e = tid + q * NT;  // A's entries first, then B's
+        const int w = e < na ? oa + e : ob + (e - na);
+        if (e < n) {
+            const uint64_t key = pk.pack((int32_t)raw[w], (int32_t)raw[P::SLOTS + w], (int32_t)raw[2 * P::SLOTS + w]) - key0;
+            raw[w] = (uint32_t)key;
+            if (!NARROW) raw[P::SLOTS + w] = (uint32_t)(key >> 32);
+        }
+    }
+    if (tid < 2) {
+        const int w = tid == 0 ? oa + na : ob + nb;
+        raw[w] = 0xffffffffu;
+        if (!NARROW) raw[P::SLOTS + w] = 0xffffffffu;
     }
     __syncthreads();
-    // tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
-    // only waits on CTAs dispatched before it (and every such wait is bounded)
-    const int32_t a0 = cuts.a[t], b0 = cuts.b[t];
-    const int na = cuts.a[t + 1] - a0, nb = cuts.b[t + 1] - b0;
-    const int n = na + nb;
-    if (CSF_OUT && tid == NT - 1) {
-        // the coordinate that precedes the tile's first result entry: the larger of the last
-        // entries before the cut (a cut never separates equal coordinates); all-ones if none
-        uint64_t prev = INF;
-        if (a0 > 0) prev = key_at(A, pk, (int64_t)a0 - 1);
-        if (b0 > 0) {
-            const uint64_t pb = key_at(B, pk, (int64_t)b0 - 1);
-            prev = prev == INF ? pb : max(prev, pb);
-        }
-        s_prev_key = prev;
-    }
 
-    // Shared layout, in 4-byte words: four raw arrays of RAW_SLOTS words each (i, j, k, value),
-    // where A's entry e sits at word oa + e and B's at word ob + e, chosen so that 16-byte
-    // boundaries of global memory fall on 16-byte boundaries here (what a bulk copy needs).
-    // Once the coordinates are packed, the 64-bit keys take the place of the raw i and j arrays,
-    // and the value staging array of the result takes the place of the raw k array.
-    uint32_t *raw = reinterpret_cast<uint32_t *>(smem_raw);
-    uint64_t *kx = reinterpret_cast<uint64_t *>(smem_raw);
-    uint64_t *ky = kx + na + 1;
-    float *out_val = reinterpret_cast<float *>(raw + 2 * RAW_SLOTS);
-    uint64_t *out_key = kx;
-    const int ha = head_elems(A.i + a0), hb = head_elems(B.i + b0);
-    const int oa = (4 - ha) & 3;
-    const int ob = ((oa + na + 3) & ~3) + ((4 - hb) & 3);
-    const float *vx = reinterpret_cast<const float *>(raw + 3 * RAW_SLOTS) + oa;
-    const float *vy = reinterpret_cast<const float *>(raw + 3 * RAW_SLOTS) + ob;
-
-    // ---- stage the eight operand arrays: aligned interiors by bulk copy, ragged ends (at most
-    // three entries each side) and arrays whose alignment differs from their i array's by
-    // plain loads
-    {
-        const void *src[8] = {A.i + a0, A.j + a0, A.k + a0, A.val + a0, B.i + b0, B.j + b0, B.k + b0, B.val + b0};
-        const int head_a = min(na, ha), head_b = min(nb, hb);
-        const int nva = (na - head_a) >> 2, nvb = (nb - head_b) >> 2;
-        bool bulk[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) bulk[q] = head_elems(src[q]) == (q < 4 ? ha : hb) && (WRITES || (q & 3) != 3);
-        if (tid == 0) {
-            uint32_t bytes = 0;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) bytes += bulk[q] ? 16u * (q < 4 ? nva : nvb) : 0u;
-            mbar_arrive_expect_tx(&mbar, bytes);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int nv = q < 4 ? nva : nvb, head = q < 4 ? head_a : head_b;
-                if (bulk[q] && nv)
-                    bulk_load(raw + (q & 3) * RAW_SLOTS + (q < 4 ? oa : ob) + head,
-                              static_cast<const uint32_t *>(src[q]) + head, 16u * nv, &mbar);
-            }
-        }
-        if (tid >= 32 && tid < 32 + 48) {  // ragged ends: 8 arrays x (3 head + 3 tail)
-            const int q = (tid - 32) / 6, e = (tid - 32) % 6;
-            const int count = q < 4 ? na : nb, head = q < 4 ? head_a : head_b, nv = q < 4 ? nva : nvb;
-            const int idx = e < 3 ? e : head + 4 * nv + (e - 3);
-            const bool live = (e < 3 ? e < head : idx < count) && (WRITES || (q & 3) != 3);
-            bool is_bulk = false;
-#pragma unroll
-            for (int qq = 0; qq < 8; ++qq) is_bulk = qq == q ? bulk[qq] : is_bulk;
-            if (live && is_bulk) {
-                const uint32_t *g = nullptr;
-#pragma unroll
-                for (int qq = 0; qq < 8; ++qq) g = qq == q ? static_cast<const uint32_t *>(src[qq]) : g;
-                raw[(q & 3) * RAW_SLOTS + (q < 4 ? oa : ob) + idx] = ld_nc(g + idx);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (!bulk[q] && (WRITES || (q & 3) != 3)) {
-                const int count = q < 4 ? na : nb;
-                for (int e = tid; e < count && !scan_warp; e += NT)
-                    raw[(q & 3) * RAW_SLOTS + (q < 4 ? oa : ob) + e] = ld_nc(static_cast<const uint32_t *>(src[q]) + e);
-            }
-        }
-    }
-    const bool landed = mbar_wait_bounded(&mbar, 0, MBAR_POLL_LIMIT);
-    if (!__syncthreads_and(landed)) {  // the copies did not land in time: report, touch nothing
-        if (tid == 0) {
-            if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
-            if (MODE == MODE_FUSED) tile_state[t] = LB_PREFIX;
-            mbar_wait_bounded(&mbar, 0, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
-        }
-        return;
-    }
-
-    if (scan_warp) {
-        // the output base is the sum of the counts of all earlier tiles and does not depend on
-        // this tile's count: walk the predecessors' words while the workers merge
-        if (MODE != MODE_FUSED) return;
-        const int64_t bse = t == 0 ? 0 : lookback_predecessors(tile_state, t, &ctl->status, 1000, &s_hurry, 1000);
-        CountBar::sync();  // the workers have published the tile's count by now
-        const int total = s_total;
-        if (lane_id() == 0) {
-            if (t > 0) st_relaxed_gpu(tile_state + t, LB_PREFIX | (uint64_t)(bse < 0 ? 0 : bse + total));
-            s_base = bse;
-            if (bse >= 0 && t == (int)gridDim.x - 1) ctl->total = bse + total;
-        }
-        __syncthreads();
-        if (CSF_OUT) {
-            // second walk: slices and fibres of all earlier tiles (packed), while the workers store
-            volatile uint64_t *level_state = csf.tile_state;
-            const int64_t lv = t == 0 ? 0 : lookback_predecessors(level_state, t, &ctl->status, 1000, &s_hurry_levels, 1000);
-            LevelBar::sync();  // the workers have published the tile's packed count by now
-            const long long packed = s_levels;
-            if (lane_id() == 0) {
-                if (t > 0) st_relaxed_gpu(level_state + t, LB_PREFIX | (uint64_t)(lv < 0 ? 0 : lv + packed));
-                s_base_levels = lv;
-            }
-            __syncthreads();
-        }
-        return;
-    }
-
-    // ---- pack the coordinates into 64-bit keys (registers first: the keys overwrite the raw
-    // i and j arrays)
-    {
-        uint64_t packed[VT];
-#pragma unroll
-        for (int q = 0; q < VT; ++q) {
-            const int e = tid + q * NT;  // merged staging slot: A's entries first, then B's
-            const int w = e < na ? oa + e : ob + (e - na);
-            packed[q] = e < n ? pk.pack((int32_t)raw[w], (int32_t)raw[RAW_SLOTS + w], (int32_t)raw[2 * RAW_SLOTS + w]) : INF;
-        }
-        WorkerBar::sync();
-#pragma unroll
-        for (int q = 0; q < VT; ++q) {
-            const int e = tid + q * NT;
-            if (e < na) kx[e] = packed[q];
-            else if (e < n) ky[e - na] = packed[q];
-        }
-        if (tid < VT + 1) ky[nb + tid] = INF;
-        if (tid == 0) kx[na] = INF;
-    }
-    WorkerBar::sync();
-
-    // ---- split the tile among threads: merge-path diagonal tid * VT, ties take A first
+    // ---- where this thread's share begins: merge-path diagonal tid * VT (ties take A first; a coordinate that
+    // both operands hold stays on one side)
     const int diag = min(tid * VT, n);
     int x, y;
     {
-        int lo = max(0, diag - nb), hi = min(diag, na);
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (kx[mid] <= ky[diag - 1 - mid]) lo = mid + 1; else hi = mid;
+        int lo = max(0, diag - nb), up = min(diag, na);
+        const uint32_t ca = 4u * (uint32_t)oa, cb = 4u * (uint32_t)(ob + diag - 1);
+        while (lo < up) {
+            const int mid = (lo + up) >> 1;
+            if (key_at_byte(ca + 4u * mid) <= key_at_byte(cb - 4u * mid)) lo = mid + 1; else up = mid;
         }
         x = lo;
         y = diag - lo;
+        if (x > 0 && y < nb && key_at_byte(4u * (uint32_t)(oa + x - 1)) == key_at_byte(4u * (uint32_t)(ob + y))) ++y;
     }
-    const int x0 = x, y0 = y;
 
-    // ---- merge VT entries, straight-line. Bit i of `from_a`: entry i came from A; of `twin`:
-    // the same coordinate is in B too; of `emit`: the entry goes to the result (B's copy of a
-    // shared coordinate does not).
-    uint64_t key[VT];
-    unsigned from_a = 0, twin = 0, emit = 0;
+    // ---- merge, one result entry per step; src[i]: the entry step i took (A's where both), top bit set where both
+    const uint32_t pa0 = 4u * (uint32_t)(oa + x), pb0 = 4u * (uint32_t)(ob + y);
+    uint32_t src[VT];
+    unsigned twin = 0;
+    int steps = 0;
     {
-        const int valid = min(VT, n - diag);
-        uint64_t hx = kx[x], hy = ky[y];
-        uint64_t last_x = x > 0 ? kx[x - 1] : INF;
+        uint32_t pa = pa0, pb = pb0;
+        const uint32_t end = 4u * (uint32_t)(oa + ob + min(tid * VT + VT, n));
+        Key ka = diag < n ? key_at_byte(pa) : END, kb = diag < n ? key_at_byte(pb) : END;
 #pragma unroll
         for (int i = 0; i < VT; ++i) {
-            const bool tx = hx <= hy;
-            const bool both = hx == hy;
-            key[i] = tx ? hx : hy;
-            from_a |= (unsigned)tx << i;
-            twin |= (unsigned)(tx && both) << i;
-            emit |= (unsigned)(i < valid && (tx || hy != last_x)) << i;
-            last_x = tx ? hx : last_x;
-            x += tx;
-            y += !tx;
-            hx = kx[x];
-            hy = ky[y];
+            const bool go = pa + pb < end;
+            const bool ta = go && ka <= kb, tb = go && kb <= ka;
+            src[i] = ta ? pa : pb;
+            if (ta && tb) {
+                twin |= 1u << i;
+                src[i] |= 0x8000u;
+            }
+            if (ta) {
+                pa += 4;
+                ka = key_at_byte(pa);
+            }
+            if (tb) {
+                pb += 4;
+                kb = key_at_byte(pb);
+            }
+            if (go) ++steps;
         }
-    }
-
-    if (MODE == MODE_REDUCE) {
-        // ---- inner product: sum a * b over the coordinates both operands hold, in double; one
-        // atomic per tile into the control block (the order of the tiles' sums is not fixed, as
-        // with the reference's atomic accumulation, src/backend/compute.cpp:498-525)
-        double sum = 0.0;
-        int xi = x0, yi = y0;
-#pragma unroll
-        for (int i = 0; i < VT; ++i) {
-            const bool tx = (from_a >> i) & 1u;
-            if ((twin >> i) & 1u && i < min(VT, n - diag)) sum += (double)(vx[xi] * vy[yi]);
-            xi += tx;
-            yi += !tx;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL_MASK, sum, o);
-        double *partial = reinterpret_cast<double *>(scan_tmp);  // 72 ints = room for 8 doubles and more
-        WorkerBar::sync();
-        if (lane_id() == 0) partial[warp_id()] = sum;
-        WorkerBar::sync();
-        if (tid == 0) {
-            double s = 0.0;
-            for (int w = 0; w < NT / 32; ++w) s += partial[w];
-            atomicAdd(reinterpret_cast<double *>(&ctl->total), s);
-        }
-        return;
     }
 
     // ---- rank the survivors inside the tile
-    int total;
-    const int mine = __popc(emit);
-    const int rank = block_excl_sum<NT, WorkerBar>(mine, scan_tmp, total);  // syncs: key reads are done
+    const int mine = REDUCE ? __popc(twin) : steps;
+    const int incl = warp_incl_sum(mine);
+    if (lane == 31) sh.wtotal[wid] = incl;
+    __syncthreads();  // also retires the merge of every thread: words of consumed twins may change from here on
+    int total = 0, wbase = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+        const int c = sh.wtotal[w];
+        wbase += w < wid ? c : 0;
+        total += c;
+    }
+    const int rank = wbase + incl - mine;
     if (MODE == MODE_COUNT) {
         if (tid == 0) tile_count[t] = total;
         return;
     }
-    if (MODE == MODE_FUSED) {
-        if (tid == 0) {
-            // successors can add this tile's count from here on
-            st_relaxed_gpu(tile_state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)total);
-            s_total = total;
-            *(volatile int *)&s_hurry = 1;
-        }
-        __threadfence_block();
-        CountBar::arrive();  // the scan warp turns the count into the tile's inclusive prefix
-    }
+    if (MODE == MODE_FUSED && tid == 0) publish_count(words, t, total);
 
-    // ---- compact through shared memory, then unpack and store coalesced
+    // ---- compact. A twin's A word now points to its B word (step i began at pa0 + pb0 + 4 (i + twins before it)).
+    if (__any_sync(FULL_MASK, twin != 0u)) {
+#pragma unroll
+        for (int i = 0; i < VT; ++i)
+            if ((twin >> i) & 1u) {
+                const uint32_t at = src[i] & 0x7fffu;
+                word_at(at) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - at;
+            }
+    }
     {
-        int r = rank, xi = x0, yi = y0;
+        uint16_t *to = src_of + rank;
 #pragma unroll
         for (int i = 0; i < VT; ++i) {
-            const bool tx = (from_a >> i) & 1u;
-            const bool both = (twin >> i) & 1u;
-            const bool out = (emit >> i) & 1u;
-            float v = tx ? vx[xi] : vy[yi];
-            if (both) v = v + vy[yi];
-            if (out) {
-                out_key[r] = key[i];
-                out_val[r] = v;
-            }
-            r += out;
-            xi += tx;
-            yi += !tx;
-        }
-    }
-    // ---- CSF3 levels above k, first half: thread t looks after the staged result entries
-    // [t VT, t VT + VT); bit q of `new_i` / `new_ij`: entry q opens a new i slice / a new (i, j)
-    // fibre. The tile's packed count goes out before the tile waits for anything.
-    const int e0 = tid * VT;
-    unsigned new_i = 0, new_ij = 0;
-    int rank_i = 0, rank_ij = 0;
-    if (CSF_OUT) {
-        WorkerBar::sync();  // the staged entries of the other workers are in place
-        const int mine_n = max(0, min(VT, total - e0));
-        const int sh_ij = pk.bk, sh_i = pk.bj + pk.bk;
-        uint64_t prev = e0 == 0 ? (uint64_t)s_prev_key : (mine_n > 0 ? out_key[e0 - 1] : 0ull);
-#pragma unroll
-        for (int q = 0; q < VT; ++q) {
-            if (q < mine_n) {
-                const uint64_t cur = out_key[e0 + q];
-                new_i |= (unsigned)((cur >> sh_i) != (prev >> sh_i)) << q;
-                new_ij |= (unsigned)((cur >> sh_ij) != (prev >> sh_ij)) << q;
-                prev = cur;
+            if (!REDUCE) {
+                if (i < steps) to[i] = (uint16_t)src[i];
+            } else if ((twin >> i) & 1u) {
+                *to++ = (uint16_t)src[i];
             }
         }
-        int tot_i, tot_ij;
-        block_excl_sum2<NT, WorkerBar>(__popc(new_i), __popc(new_ij), scan_tmp, rank_i, rank_ij, tot_i, tot_ij);
-        if (tid == 0) {
-            const long long packed = ((long long)tot_i << 31) | (long long)tot_ij;
-            st_relaxed_gpu(csf.tile_state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)packed);
-            s_levels = packed;
-            *(volatile int *)&s_hurry_levels = 1;
-        }
-        __threadfence_block();
-        LevelBar::arrive();  // the scan warp turns the packed count into the tile's inclusive prefix
     }
+    __syncthreads();
 
-    // ---- output base of the tile (from the scan warp, or from the scanned counts)
-    if (MODE == MODE_FUSED) __syncthreads(); else WorkerBar::sync();
-    const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
-    if (base < 0) {  // a bounded wait gave up; the host reports it
-        if (CSF_OUT) __syncthreads();  // the scan warp still waits at the levels barrier
+    const char *va = reinterpret_cast<const char *>(A.val + a0) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(B.val + b0) - 4 * (int64_t)ob;
+    if (REDUCE) {
+        // ---- inner product: products in float32 as the reference's, summed in double; one atomic per tile into
+        // the control block (the order of the tiles' sums is not fixed, as with the reference's atomic
+        // accumulation, src/backend/compute.cpp:498-525)
+        double sum = 0.0;
+        for (int o = tid; o < total; o += NT) {
+            const uint32_t at = src_of[o] & 0x7fffu;
+            sum += (double)(__ldg(reinterpret_cast<const float *>(va + at)) * __ldg(reinterpret_cast<const float *>(vb + word_at(at))));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL_MASK, sum, o);
+        if (lane == 0) sh.partial[wid] = sum;
+        __syncthreads();
+        if (tid == 0) {
+            double s = 0.0;
+            for (int w = 0; w < NT / 32; ++w) s += sh.partial[w];
+            if (s != 0.0) atomicAdd(reinterpret_cast<double *>(&ctl->total), s);
+        }
         return;
     }
-    for (int i = tid; i < total; i += NT) {
-        const uint64_t kq = out_key[i];
-        if (!CSF_OUT) {
-            Z.i[base + i] = pk.i_of(kq);
-            Z.j[base + i] = pk.j_of(kq);
-        }
-        Z.k[base + i] = pk.k_of(kq);
-        Z.val[base + i] = out_val[i];
-    }
-    if (!CSF_OUT) return;
 
-    // ---- CSF3 levels above k, second half: slices / fibres of the earlier tiles, then the scatter
-    __syncthreads();
-    const long long levels_base = s_base_levels;
-    if (levels_base < 0) return;
-    int r = (int)(levels_base >> 31) + rank_i;
-    int f = (int)(levels_base & 0x7fffffff) + rank_ij;
+    // ---- fetch coordinates and values, result entries q * NT + tid; the first batch before the output base is asked for
+    const uint32_t first_b = 4u * (uint32_t)ob;
+    Key key[GATHER];
+    float val[GATHER];
+    auto live = [&](int q) { return q < VT && q * NT + tid < total; };
+    auto gather = [&](const int q0) {
+        uint32_t s[GATHER], any = 0;
 #pragma unroll
-    for (int q = 0; q < VT; ++q) {
-        if ((new_ij >> q) & 1u) {
-            const uint64_t cur = out_key[e0 + q];
-            if (f < csf.cap_j) {
-                csf.j_idx[f] = pk.j_of(cur);
-                csf.k_ptr[f] = (int32_t)(base + e0 + q);
+        for (int g = 0; g < GATHER; ++g) {
+            s[g] = live(q0 + g) ? (uint32_t)src_of[(q0 + g) * NT + tid] : 4u * (uint32_t)oa;
+            any |= s[g];
+        }
+        if (__any_sync(FULL_MASK, (any & 0x8000u) != 0u)) {
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                const bool both = (s[g] & 0x8000u) != 0u;
+                const uint32_t at = s[g] & 0x7fffu, other = both ? word_at(at) : at;
+                key[g] = key_at_byte(other);
+                float v = 0.0f;
+                if (live(q0 + g)) v = __ldg(reinterpret_cast<const float *>((at >= first_b ? vb : va) + at));
+                if (both) v = v + __ldg(reinterpret_cast<const float *>(vb + other));
+                val[g] = v;
             }
-            if ((new_i >> q) & 1u) {
-                if (r < csf.cap_i) {
-                    csf.i_idx[r] = pk.i_of(cur);
-                    csf.j_ptr[r] = f;
-                }
-                ++r;
+        } else {
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                key[g] = key_at_byte(s[g]);
+                val[g] = live(q0 + g) ? __ldg(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
             }
-            ++f;
+        }
+    };
+    gather(0);
+
+    // ---- output base of the tile
+    if (MODE == MODE_FUSED && wid == 0) {
+        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+        if (lane == 0) {
+            sh.base = b;
+            if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) coo3_finish(ctl, Z, b < 0 ? b : b + total);
         }
     }
-    if (t == (int)gridDim.x - 1 && tid == NT - 1) {  // the last worker of the last tile holds the totals
-        csf.totals->n_i = r;
-        csf.totals->n_j = f;
-        if (f <= csf.cap_j) csf.k_ptr[f] = (int32_t)(base + total);
-        if (r <= csf.cap_i) csf.j_ptr[r] = f;
+    __syncthreads();
+    const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : sh.base;
+    if (base < 0) return;  // a bounded wait gave up; the host reports it
+
+    // ---- unpack and store, coalesced
+#pragma unroll
+    for (int q0 = 0; q0 < VT; q0 += GATHER) {
+        if (q0 > 0) {
+            if (q0 * NT >= total) break;
+            gather(q0);
+        }
+#pragma unroll
+        for (int g = 0; g < GATHER; ++g) {
+            if (live(q0 + g)) {
+                const long long o = base + (q0 + g) * NT + tid;
+                const uint64_t full = key0 + key[g];
+                Z.i[o] = pk.i_of(full);
+                Z.j[o] = pk.j_of(full);
+                Z.k[o] = pk.k_of(full);
+                Z.val[o] = val[g];
+            }
+        }
     }
+}
+
+template <int VT, int MODE>
+__global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo3In A, const __grid_constant__ Coo3In B, const Packing pk,
+                                                     const Cuts2 cuts, int32_t *tile_count, const __grid_constant__ TileWords words, FusedCtl *ctl,
+                                                     const __grid_constant__ Coo3Out Z, int num_tiles) {
+    using P = Coo3Plan<VT>;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ Coo3Shared sh;
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        mbar_init(&sh.mbar, 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    wait_for_previous();  // the cuts
+    const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
+    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
+        if (tid < 32) {
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+            if (tid == 0) coo3_finish(ctl, Z, total);
+        }
+        return;
+    }
+    // tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
+    // only waits on CTAs dispatched before it (and every such wait is bounded)
+    const int t = blockIdx.x - (scanned ? 1 : 0);
+    int32_t a0 = 0, b0 = 0;
+    int na = A.nnz, nb = B.nnz;
+    if (cuts.a) {
+        a0 = cuts.a[t], b0 = cuts.b[t];
+        na = cuts.a[t + 1] - a0, nb = cuts.b[t + 1] - b0;
+    } else if (tid == 0) {  // a single tile: no partition kernel ran, so this clears the control block
+        *ctl = FusedCtl{};
+    }
+
+    // ---- stage the six coordinate arrays: aligned interiors by bulk copy, ragged ends (at most three entries
+    // each side) and arrays whose alignment differs from their i array's by plain loads
+    uint32_t *raw = reinterpret_cast<uint32_t *>(smem_raw);
+    const int ha = head_elems(A.i + a0), hb = head_elems(B.i + b0);
+    const int oa = (4 - ha) & 3;
+    const int ob = ((oa + na + 1 + 3) & ~3) + ((4 - hb) & 3);  // A's sentinel lies before it
+    {
+        const int32_t *src[6] = {A.i + a0, A.j + a0, A.k + a0, B.i + b0, B.j + b0, B.k + b0};
+        const int head_a = min(na, ha), head_b = min(nb, hb);
+        const int nva = (na - head_a) >> 2, nvb = (nb - head_b) >> 2;
+        bool bulk[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) bulk[q] = head_elems(src[q]) == (q < 3 ? ha : hb);
+        if (tid == 0) {
+            uint32_t bytes = 0;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) bytes += bulk[q] ? 16u * (q < 3 ? nva : nvb) : 0u;
+            mbar_arrive_expect_tx(&sh.mbar, bytes);
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const int nv = q < 3 ? nva : nvb, head = q < 3 ? head_a : head_b;
+                if (bulk[q] && nv) bulk_load(raw + (q % 3) * P::SLOTS + (q < 3 ? oa : ob) + head, src[q] + head, 16u * nv, &sh.mbar);
+            }
+            if (MODE == MODE_FUSED || MODE == MODE_FILL) {
+                prefetch_l2(A.val + a0, na);
+                prefetch_l2(B.val + b0, nb);
+            }
+        }
+        if (tid >= 32 && tid < 32 + 36) {  // ragged ends: 6 arrays x (3 head + 3 tail)
+            const int q = (tid - 32) / 6, e = (tid - 32) % 6;
+            const int count = q < 3 ? na : nb, head = q < 3 ? head_a : head_b, nv = q < 3 ? nva : nvb;
+            const int idx = e < 3 ? e : head + 4 * nv + (e - 3);
+            bool is_bulk = false;
+            const int32_t *g = nullptr;
+#pragma unroll
+            for (int qq = 0; qq < 6; ++qq)
+                if (qq == q) is_bulk = bulk[qq], g = src[qq];
+            if (is_bulk && (e < 3 ? e < head : idx < count)) raw[(q % 3) * P::SLOTS + (q < 3 ? oa : ob) + idx] = (uint32_t)ld_nc(g + idx);
+        }
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            if (!bulk[q])
+                for (int e = tid; e < (q < 3 ? na : nb); e += NT) raw[(q % 3) * P::SLOTS + (q < 3 ? oa : ob) + e] = (uint32_t)ld_nc(src[q] + e);
+    }
+    const bool landed = mbar_wait_bounded(&sh.mbar, 0, MBAR_POLL_LIMIT);
+    if (!__syncthreads_and(landed)) {  // the copies did not land in time: report, touch nothing
+        if (tid == 0) {
+            if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
+            __threadfence();
+            if (MODE == MODE_FUSED) {
+                publish_count(words, t, 0);  // successors must not wait on this tile
+                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+            }
+            if (MODE == MODE_REDUCE) coo3_reduce_done(ctl, Z, num_tiles);
+            mbar_wait_bounded(&sh.mbar, 0, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
+        }
+        return;
+    }
+    // ---- smallest and largest key of the tile
+    auto staged_key = [&](int w) { return pk.pack((int32_t)raw[w], (int32_t)raw[P::SLOTS + w], (int32_t)raw[2 * P::SLOTS + w]); };
+    uint64_t key0 = ~0ull, key1 = 0;
+    if (na > 0) key0 = staged_key(oa), key1 = staged_key(oa + na - 1);
+    if (nb > 0) key0 = min(key0, staged_key(ob)), key1 = max(key1, staged_key(ob + nb - 1));
+    __syncthreads();  // everybody has read them: packing overwrites them
+    if (key1 - key0 < 0xffffffffull)
+        coo3_tile<VT, MODE, true>(A, B, pk, a0, b0, na, nb, oa, ob, key0, t, num_tiles, tile_count, words, ctl, Z, smem_raw, sh);
+    else
+        coo3_tile<VT, MODE, false>(A, B, pk, a0, b0, na, nb, oa, ob, key0, t, num_tiles, tile_count, words, ctl, Z, smem_raw, sh);
+    if (MODE == MODE_REDUCE && tid == 0) coo3_reduce_done(ctl, Z, num_tiles);
 }
 
 // ---------------------------------------------------------------- wide coordinates ----
@@ -651,7 +632,6 @@ cudaError_t launch_coo3_tile_wide(const Coo3In &A, const Coo3In &B, const Cuts2 
     return cudaGetLastError();
 }
 
-constexpr size_t coo3_smem_bytes() { return 16 * (size_t)RAW_SLOTS; }
 static_assert(coo3_wide_smem_bytes() <= 48 * 1024, "the wide tile kernel stays within the default shared-memory limit");
 
 
@@ -661,23 +641,62 @@ int bits_for(int32_t extent) {
     return b;
 }
 
-template <int MODE, bool CSF_OUT = false>
-cudaError_t launch_coo3_tile(const Coo3In &A, const Coo3In &B, const Packing &pk, const Cuts2 &cuts, int32_t *tile_count,
-                             uint64_t *tile_state, FusedCtl *ctl, const Coo3Out &Z, int num_tiles, cudaStream_t stream,
-                             const CsfLevelsOut &csf = CsfLevelsOut{}) {
-    auto kernel = k_coo3_tile<MODE, CSF_OUT>;
+// Merged entries per worker thread: large tiles amortise the searches and the wait for the earlier counts, small
+// ones fill the chip when there are few entries. 100 M entries per operand, tile kernel: 1257 us with 13, 1195
+// with 17 (52 KB of shared memory: the most of which four CTAs fit an SM), 1331 with 19.
+constexpr int V_LARGE = 17, V_SMALL = 7;
+constexpr int64_t LARGE_FROM = 3000000;
+constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
+constexpr int tile_step_of(int v) { return NT * v - 1; }  // a twin may add one entry
+
+template <int VT, int MODE>
+cudaError_t launch_coo3_tile_v(const Coo3In &A, const Coo3In &B, const Packing &pk, const Cuts2 &cuts, int32_t *tile_count, const TileWords &words,
+                               FusedCtl *ctl, const Coo3Out &Z, int num_tiles, cudaStream_t stream) {
+    auto kernel = k_coo3_tile<VT, MODE>;
+    constexpr size_t smem = Coo3Plan<VT>::BYTES;
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coo3_smem_bytes());
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    static const char *const names[4] = {"coo3_add_count", "coo3_add_fill", "coo3_add_fused", "coo3_inner_prod"};
-    LaunchScope scope(CSF_OUT ? "coo3_add_fused_csf" : names[MODE], stream);
-    kernel<<<num_tiles, NT + 32, coo3_smem_bytes(), stream>>>(A, B, pk, cuts, tile_count, tile_state, ctl, Z, csf);
+    const dim3 grid(num_tiles + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
+    if ((MODE == MODE_FUSED || MODE == MODE_REDUCE) && cuts.a)
+        return launch_overlapped(kernel, grid, dim3(NT), smem, stream, A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles);
+    kernel<<<grid, NT, smem, stream>>>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles);
     return cudaGetLastError();
+}
+
+template <int MODE>
+cudaError_t launch_coo3_tile(const Coo3In &A, const Coo3In &B, const Packing &pk, const Cuts2 &cuts, int32_t *tile_count, const TileWords &words,
+                             FusedCtl *ctl, const Coo3Out &Z, int num_tiles, int v, cudaStream_t stream) {
+    static const char *const names[4] = {"coo3_add_count", "coo3_add_fill", "coo3_add_fused", "coo3_inner_prod"};
+    LaunchScope scope(names[MODE], stream);
+    return v == V_LARGE ? launch_coo3_tile_v<V_LARGE, MODE>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles, stream)
+                        : launch_coo3_tile_v<V_SMALL, MODE>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles, stream);
+}
+
+// Queues the cuts; `zero_words` words of control block and tile words are cleared on the way. Up to about a wave of
+// warps, a warp per cut. Beyond that the bytes that the probes touch count (a sector each, far apart): a warp for
+// every 32nd cut, then four lanes for every other one between its two neighbours. 46 000 cuts (100 M entries per
+// operand): 87 us so, 104 with eight lanes, 83 with two, 166 with eight lanes over the whole range; 5500 cuts: 33
+// with four lanes, 44 with two, a chain of dependent loads by then.
+cudaError_t launch_coo3_partition(const Coo3In &A, const Coo3In &B, int64_t total, int32_t step, int num_tiles, const Cuts2 &cuts, uint64_t *zero_block,
+                                  int zero_words, cudaStream_t stream) {
+    constexpr int COARSE = 32, FINE = 4;
+    LaunchScope scope("coo3_partition", stream);
+    auto ctas = [&](int64_t groups, int lanes) { return (unsigned)((groups * lanes + NT - 1) / NT); };
+    if (num_tiles <= 4096) {
+        k_coo3_partition<32><<<ctas(num_tiles + 1, 32), NT, 0, stream>>>(A, B, total, step, num_tiles, 1, 0, cuts, zero_block, zero_words);
+        return cudaGetLastError();
+    }
+    k_coo3_partition<32><<<ctas(num_tiles / COARSE + 2, 32), NT, 0, stream>>>(A, B, total, step, num_tiles, COARSE, 0, cuts, nullptr, 0);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    return launch_overlapped(k_coo3_partition<FINE>, dim3(ctas(num_tiles + 1, FINE)), dim3(NT), 0, stream, A, B, total, step, num_tiles, 1, COARSE, cuts,
+                             zero_block, zero_words);
 }
 
 int check_coo3(const nb200_coo3 *t) {
@@ -692,14 +711,11 @@ int check_coo3(const nb200_coo3 *t) {
 // When `alloc` is set the four result arrays are allocated here (one cudaMallocAsync each, at
 // the worst-case length nnz(A) + nnz(B)); otherwise they are the caller's, `capacity` entries.
 //
-// `scratch` / `host_slot`, when given, replace the library's pooled workspace (the caller then
-// owns a block of coo3_add_scratch_bytes() bytes and a pinned int64[8]); the CSF3 add uses this
-// to keep its own temporaries and this function's in one pool block.
-//
-// `csf`, when given, asks the single-pass launch to write the CSF3 levels above k instead of the
-// merged i and j columns (z->i and z->j may then be null); `*csf_done` tells whether that
-// happened (the count -> scan -> fill route does not do it).
-// (Both sized for the smaller tile of the wide-coordinate kernel, an upper bound for the other.)
+// `scratch` / `ws`, when given, replace the library's pooled workspace (the caller then owns a block of
+// coo3_add_scratch_bytes() bytes; result words and copies go to the pinned slots of `ws`); the CSF3 kernels use
+// this to keep their own temporaries and this function's in one pool block.
+// (Both sized for the smallest tile of the kernels here, an upper bound for the others.)
+static_assert(WCAP - 1 <= tile_step_of(V_SMALL), "scratch is sized for the smallest tile");
 int64_t coo3_add_tiles(int64_t total_entries) { return (total_entries + (WCAP - 1) - 1) / (WCAP - 1); }
 
 size_t coo3_add_scratch_bytes(int64_t total_entries) {
@@ -708,15 +724,13 @@ size_t coo3_add_scratch_bytes(int64_t total_entries) {
     sizes.take<int32_t>((size_t)tiles + 1);
     sizes.take<int32_t>((size_t)tiles + 1);
     sizes.take<int32_t>((size_t)tiles + 1);
-    sizes.take<int64_t>(1);
-    sizes.take<uint64_t>((size_t)tiles + 8);
+    sizes.take<uint64_t>(TileWords::needed((size_t)tiles) + 8);
     return sizes.used();
 }
 
 int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool alloc, int64_t capacity, void *stream_v,
-                 void *scratch, int64_t *host_slot, const CsfLevelsOut *csf, bool *csf_done) {
+                 void *scratch, Workspace *ws) {
     int st;
-    if (csf_done) *csf_done = false;
     if ((st = check_coo3(a)) || (st = check_coo3(b))) return st;
     if (!z || a->dims[0] != b->dims[0] || a->dims[1] != b->dims[1] || a->dims[2] != b->dims[2]) return NB200_E_BADARG;
     if (!alloc && capacity < 0) return NB200_E_BADARG;
@@ -724,7 +738,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     const bool wide = bi + bj + bk > 63;  // the coordinates do not pack into one 64-bit key
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    const int tile_step = wide ? WCAP - 1 : CAP - 1;
+    const int v = tile_v(total), tile_step = wide ? WCAP - 1 : tile_step_of(v);
     const int64_t tiles64 = (total + tile_step - 1) / tile_step;
     if (tiles64 > INT32_MAX - 1) return NB200_E_OVERFLOW;
     const int num_tiles = (int)tiles64;
@@ -732,7 +746,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     z->nnz = 0;
     if (alloc) z->i = z->j = z->k = nullptr, z->val = nullptr;
     if (num_tiles == 0) return NB200_OK;
-    if (!alloc && capacity > 0 && (!z->k || !z->val)) return NB200_E_BADARG;
+    if (!alloc && capacity > 0 && (!z->i || !z->j || !z->k || !z->val)) return NB200_E_BADARG;
 
     auto fail = [&](int code) {
         if (alloc) {
@@ -747,75 +761,40 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     };
 
     if (!scratch) {
-        Workspace *ws = nullptr;
         if ((st = acquire_workspace(stream, coo3_add_scratch_bytes(total), &ws))) return st;
         scratch = ws->dev;
-        host_slot = ws->host;
     }
+    int64_t *host_slot = ws->host;
     Carver carve(scratch);
     Cuts2 cuts;
     cuts.a = carve.take<int32_t>((size_t)num_tiles + 1);
     cuts.b = carve.take<int32_t>((size_t)num_tiles + 1);
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
-    carve.take<int64_t>(1);
-    uint64_t *fused_block = carve.take<uint64_t>((size_t)num_tiles + 8);
+    uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed((size_t)num_tiles) + 4);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    uint64_t *tile_state = fused_block + 4;
+    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
 
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     const Packing pk{bj, bk};
     static const bool force_two_pass = [] { const char *e = std::getenv("NACHO_B200_TWO_PASS"); return e && e[0] == '1'; }();
     const bool fused = alloc || (capacity >= total && !force_two_pass);
-    const bool levels = fused && csf != nullptr && !alloc && !wide;  // the wide kernel writes coordinates only
-    if (!levels && !alloc && capacity > 0 && (!z->i || !z->j)) return NB200_E_BADARG;
-    cudaError_t e = cudaMemsetAsync(fused_block, 0, sizeof(uint64_t) * (fused ? (size_t)num_tiles + 4 : 4), stream);
-    if (e != cudaSuccess) return note_cuda_error(e, "cudaMemsetAsync");
-    if (fused) {
-        if (alloc) {
-            void **arrays[4] = {reinterpret_cast<void **>(&z->i), reinterpret_cast<void **>(&z->j),
-                                reinterpret_cast<void **>(&z->k), reinterpret_cast<void **>(&z->val)};
-            for (auto p : arrays) {
-                e = cudaMallocAsync(p, 4 * (size_t)total, stream);
-                if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
-            }
+    cudaError_t e = cudaSuccess;
+    if (fused && alloc) {
+        void **arrays[4] = {reinterpret_cast<void **>(&z->i), reinterpret_cast<void **>(&z->j),
+                            reinterpret_cast<void **>(&z->k), reinterpret_cast<void **>(&z->val)};
+        for (auto p : arrays) {
+            e = cudaMallocAsync(p, 4 * (size_t)total, stream);
+            if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
         }
     }
-    {
-        LaunchScope scope("coo3_partition", stream);
-        const int warps = num_tiles / COARSE + 2;
-        if (wide) {
-            k_coo3_partition_coarse<<<(warps * 32 + NT - 1) / NT, NT, 0, stream>>>(A, B, WidePacking{}, total, tile_step, num_tiles, cuts);
-            k_coo3_partition_fine<<<(num_tiles + NT - 1) / NT, NT, 0, stream>>>(A, B, WidePacking{}, total, tile_step, num_tiles, cuts);
-        } else {
-            k_coo3_partition_coarse<<<(warps * 32 + NT - 1) / NT, NT, 0, stream>>>(A, B, pk, total, tile_step, num_tiles, cuts);
-            k_coo3_partition_fine<<<(num_tiles + NT - 1) / NT, NT, 0, stream>>>(A, B, pk, total, tile_step, num_tiles, cuts);
-        }
-        e = cudaGetLastError();
+    if (num_tiles == 1 && fused && !wide) {
+        cuts = Cuts2{nullptr, nullptr};  // one tile: no cut to search, and the tile kernel clears the control block itself
+    } else {
+        e = launch_coo3_partition(A, B, total, tile_step, num_tiles, cuts, fused_block, fused ? (int)TileWords::needed((size_t)num_tiles) + 4 : 4, stream);
     }
     if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_partition"));
-    const Coo3Out Z{z->i, z->j, z->k, z->val};
-    if (fused) {
-        if (wide) {
-            e = launch_coo3_tile_wide<MODE_FUSED>(A, B, cuts, nullptr, tile_state, ctl, Z, num_tiles, stream);
-        } else if (levels) {
-            e = launch_coo3_tile<MODE_FUSED, true>(A, B, pk, cuts, nullptr, tile_state, ctl, Z, num_tiles, stream, *csf);
-            if (csf_done) *csf_done = true;
-        } else {
-            e = launch_coo3_tile<MODE_FUSED>(A, B, pk, cuts, nullptr, tile_state, ctl, Z, num_tiles, stream);
-        }
-        if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_tile<fused>"));
-        e = cudaMemcpyAsync(host_slot, ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) return fail(note_cuda_error(e, "read result length"));
-        FusedCtl h;
-        std::memcpy(&h, host_slot, sizeof(h));
-        if (h.status.error != 0) return fail(note_timeout(h.status.error, h.status.detail, "coo3 merge"));
-        if (h.total > INT32_MAX) return fail(NB200_E_OVERFLOW);
-        z->nnz = (int32_t)h.total;
-        return NB200_OK;
-    }
-    // count -> scan -> fill. The scan leaves the result length in the control block, whose status
-    // word also collects a give-up of either tile launch (a bulk copy that did not land in time).
+    const Coo3Out Z{z->i, z->j, z->k, z->val, result_word(ws, RW_COO3)};
+    // Reads the control block back (one small copy and a wait for the GPU).
     auto read_ctl = [&](FusedCtl &h) -> int {
         cudaError_t c = cudaMemcpyAsync(host_slot, ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream);
         if (c == cudaSuccess) c = cudaStreamSynchronize(stream);
@@ -824,8 +803,33 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
         return NB200_OK;
     };
     FusedCtl h;
+    if (fused && !wide) {
+        e = launch_coo3_tile<MODE_FUSED>(A, B, pk, cuts, nullptr, words, ctl, Z, num_tiles, v, stream);
+        if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_tile<fused>"));
+        int64_t length;
+        int device_status;
+        if ((st = wait_result_word(Z.host, stream, &length, &device_status))) return fail(st);
+        if (device_status != 0) {
+            if ((st = read_ctl(h))) return fail(st);
+            return fail(note_timeout(h.status.error, h.status.detail, "coo3 merge"));
+        }
+        if (length > INT32_MAX) return fail(NB200_E_OVERFLOW);
+        z->nnz = (int32_t)length;
+        return NB200_OK;
+    }
+    if (fused) {
+        e = launch_coo3_tile_wide<MODE_FUSED>(A, B, cuts, nullptr, words.count, ctl, Z, num_tiles, stream);
+        if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_tile_wide<fused>"));
+        if ((st = read_ctl(h))) return fail(st);
+        if (h.status.error != 0) return fail(note_timeout(h.status.error, h.status.detail, "coo3 merge"));
+        if (h.total > INT32_MAX) return fail(NB200_E_OVERFLOW);
+        z->nnz = (int32_t)h.total;
+        return NB200_OK;
+    }
+    // count -> scan -> fill. The scan leaves the result length in the control block, whose status
+    // word also collects a give-up of either tile launch (a bulk copy that did not land in time).
     e = wide ? launch_coo3_tile_wide<MODE_COUNT>(A, B, cuts, tile_count, nullptr, ctl, Coo3Out{}, num_tiles, stream)
-             : launch_coo3_tile<MODE_COUNT>(A, B, pk, cuts, tile_count, nullptr, ctl, Coo3Out{}, num_tiles, stream);
+             : launch_coo3_tile<MODE_COUNT>(A, B, pk, cuts, tile_count, TileWords{}, ctl, Coo3Out{}, num_tiles, v, stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_tile<count>");
     {
         LaunchScope scope("scan_tiles", stream);
@@ -839,15 +843,11 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     z->nnz = (int32_t)h.total;
     if (h.total > capacity) return NB200_E_CAPACITY;
     e = wide ? launch_coo3_tile_wide<MODE_FILL>(A, B, cuts, tile_count, nullptr, ctl, Z, num_tiles, stream)
-             : launch_coo3_tile<MODE_FILL>(A, B, pk, cuts, tile_count, nullptr, ctl, Z, num_tiles, stream);
+             : launch_coo3_tile<MODE_FILL>(A, B, pk, cuts, tile_count, TileWords{}, ctl, Z, num_tiles, v, stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_tile<fill>");
     if ((st = read_ctl(h))) return st;
     if (h.status.error != 0) return note_timeout(h.status.error, h.status.detail, "coo3 merge");
     return NB200_OK;
-}
-
-__global__ void k_store_scalar(const FusedCtl *ctl, float *out) {
-    out[0] = (float)__longlong_as_double(ctl->total);
 }
 
 // Inner product of two COO3 tensors: sum over the coordinates both hold of a * b, written as one
@@ -855,8 +855,8 @@ __global__ void k_store_scalar(const FusedCtl *ctl, float *out) {
 // append-reduction src/backend/compute.cpp:498-525). The same partition and tile kernel as the add,
 // in a mode that writes no tensor. Products are float32 (as the reference's), their sum is kept in
 // double until the end. Extents that do not pack into 64 bits are not supported here.
-// `scratch` / `host_slot` as for coo3_add_run.
-int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *stream_v, void *scratch, int64_t *host_slot) {
+// `scratch` / `ws` as for coo3_add_run.
+int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *stream_v, void *scratch, Workspace *ws) {
     int st;
     if ((st = check_coo3(a)) || (st = check_coo3(b))) return st;
     if (!z || a->dims[0] != b->dims[0] || a->dims[1] != b->dims[1] || a->dims[2] != b->dims[2]) return NB200_E_BADARG;
@@ -864,7 +864,7 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
     if (bi + bj + bk > 63) return NB200_E_UNSUPPORTED;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    constexpr int tile_step = CAP - 1;
+    const int v = tile_v(total), tile_step = tile_step_of(v);
     const int64_t tiles64 = (total + tile_step - 1) / tile_step;
     if (tiles64 > INT32_MAX - 1) return NB200_E_OVERFLOW;
     const int num_tiles = (int)tiles64;
@@ -873,37 +873,29 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
         return NB200_OK;
     }
     if (!scratch) {
-        Workspace *ws = nullptr;
         if ((st = acquire_workspace(stream, coo3_add_scratch_bytes(total), &ws))) return st;
         scratch = ws->dev;
-        host_slot = ws->host;
     }
     Carver carve(scratch);
     Cuts2 cuts;
     cuts.a = carve.take<int32_t>((size_t)num_tiles + 1);
     cuts.b = carve.take<int32_t>((size_t)num_tiles + 1);
-    carve.take<int32_t>((size_t)num_tiles + 1);
-    carve.take<int64_t>(1);
-    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(carve.take<uint64_t>((size_t)num_tiles + 8));
+    uint64_t *block = carve.take<uint64_t>(4);
+    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(block);
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
-    const Packing pk{bj, bk};
-    NB200_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(uint64_t), stream));
-    {
-        LaunchScope scope("coo3_partition", stream);
-        const int warps = num_tiles / COARSE + 2;
-        k_coo3_partition_coarse<<<(warps * 32 + NT - 1) / NT, NT, 0, stream>>>(A, B, pk, total, tile_step, num_tiles, cuts);
-        k_coo3_partition_fine<<<(num_tiles + NT - 1) / NT, NT, 0, stream>>>(A, B, pk, total, tile_step, num_tiles, cuts);
-        NB200_CUDA(cudaGetLastError());
-    }
-    cudaError_t e = launch_coo3_tile<MODE_REDUCE>(A, B, pk, cuts, nullptr, nullptr, ctl, Coo3Out{}, num_tiles, stream);
+    cudaError_t e = cudaSuccess;
+    if (num_tiles == 1) cuts = Cuts2{nullptr, nullptr};
+    else e = launch_coo3_partition(A, B, total, tile_step, num_tiles, cuts, block, 4, stream);
+    if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_partition");
+    Coo3Out Z{};
+    Z.host = result_word(ws, RW_COO3);
+    Z.scalar = z;
+    e = launch_coo3_tile<MODE_REDUCE>(A, B, Packing{bj, bk}, cuts, nullptr, TileWords{}, ctl, Z, num_tiles, v, stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_tile<reduce>");
-    k_store_scalar<<<1, 1, 0, stream>>>(ctl, z);
-    NB200_CUDA(cudaGetLastError());
-    NB200_CUDA(cudaMemcpyAsync(host_slot, ctl, sizeof(FusedCtl), cudaMemcpyDeviceToHost, stream));
-    NB200_CUDA(cudaStreamSynchronize(stream));
-    FusedCtl h;
-    std::memcpy(&h, host_slot, sizeof(h));
-    return h.status.error != 0 ? note_timeout(h.status.error, h.status.detail, "coo3 inner product") : NB200_OK;
+    int64_t done;
+    int device_status;
+    if ((st = wait_result_word(Z.host, stream, &done, &device_status))) return st;
+    return device_status != 0 ? note_timeout(ERR_COPY_TIMEOUT, 0, "coo3 inner product") : NB200_OK;
 }
 
 }  // namespace nb200
@@ -913,11 +905,11 @@ using namespace nb200;
 extern "C" {
 
 int nb200_coo3d_add_f32(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, int32_t, int32_t, void *stream) {
-    return coo3_add_run(a, b, z, true, 0, stream, nullptr, nullptr, nullptr, nullptr);
+    return coo3_add_run(a, b, z, true, 0, stream, nullptr, nullptr);
 }
 
 int nb200_coo3d_add_f32_into(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, int64_t capacity, void *stream) {
-    return coo3_add_run(a, b, z, false, capacity, stream, nullptr, nullptr, nullptr, nullptr);
+    return coo3_add_run(a, b, z, false, capacity, stream, nullptr, nullptr);
 }
 
 int nb200_inner_prod_coo_f32(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *stream) {

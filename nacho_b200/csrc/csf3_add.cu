@@ -10,13 +10,10 @@
 //   1. k_csf_expand    every stored entry gets its (i, j) written out next to its k: one warp
 //                      per 32 (i, j) fibres finds their i by binary search and fills their ranges;
 //   2. coo3_add_run    the sorted-union merge of the two coordinate lists (coo3_merge.cu); k and
-//                      the values go straight into the result's k_idx / val arrays. On its
-//                      single-pass route the merge also writes i_idx / j_ptr / j_idx / k_ptr
-//                      itself (CsfLevelsOut) and nothing else is left to do;
-//   3. k_csf_compress  only after the count -> scan -> fill route of the merge: one pass over
-//                      the merged (i, j) columns: head flags for new i and new (i, j), a packed
-//                      two-counter scan across tiles by bounded look-back, and the scatter of
-//                      i_idx / j_ptr / j_idx / k_ptr.
+//                      the values go straight into the result's k_idx / val arrays;
+//   3. k_csf_compress  one pass over the merged (i, j) columns: head flags for new i and new
+//                      (i, j), a packed two-counter scan across tiles by bounded look-back, and
+//                      the scatter of i_idx / j_ptr / j_idx / k_ptr.
 // Level-by-level route (described above csf_add_levels): one merge per
 // level, each of which tells the next where the ranges of A and B begin, so that no per-entry (i, j) is
 // ever written.
@@ -29,8 +26,8 @@
 namespace nb200 {
 
 int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool alloc, int64_t capacity, void *stream_v,
-                 void *scratch, int64_t *host_slot, const CsfLevelsOut *csf, bool *csf_done);
-int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *stream_v, void *scratch, int64_t *host_slot);
+                 void *scratch, Workspace *ws);
+int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *stream_v, void *scratch, Workspace *ws);
 size_t coo3_add_scratch_bytes(int64_t total_entries);
 int64_t coo3_add_tiles(int64_t total_entries);
 
@@ -201,7 +198,7 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
     int st;
     // one pool block: expanded (i, j) of A, of B and of the merged list, the merge's own scratch
     // and the compress pass's control block and tile words
-    const int64_t compress_tiles = std::max<int64_t>((total + NT * CVT - 1) / (NT * CVT), coo3_add_tiles(total));
+    const int64_t compress_tiles = (total + NT * CVT - 1) / (NT * CVT);
     Carver sizes;
     sizes.take<int32_t>((size_t)a->n_k);
     sizes.take<int32_t>((size_t)a->n_k);
@@ -238,28 +235,9 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
     static_assert(sizeof(CompressCtl) <= 4 * sizeof(uint64_t), "control block must fit its slot");
     uint64_t *tile_state = compress_block + 4;
 
-    // single-pass route: the merge writes the levels above k itself (no merged i / j columns, no
-    // compress pass); its second look-back runs over `tile_state`, its totals land in ctl
-    e = cudaMemsetAsync(compress_block, 0, sizeof(uint64_t) * ((size_t)coo3_add_tiles(total) + 4), stream);
-    if (e != cudaSuccess) return (note_cuda_error(e, "cudaMemsetAsync"));
-    const CsfLevelsOut levels{z->i_idx, z->j_ptr, z->j_idx, z->k_ptr, (int32_t)std::min<int64_t>(cap_i, INT32_MAX),
-                              (int32_t)std::min<int64_t>(cap_j, INT32_MAX), tile_state, reinterpret_cast<CsfTotals *>(&ctl->n_i)};
-    bool levels_done = false;
-    if ((st = coo3_add_run(&ca, &cb, &cz, false, total, stream, merge_scratch, ws->host, &levels, &levels_done))) return (st);
+    if ((st = coo3_add_run(&ca, &cb, &cz, false, total, stream, merge_scratch, ws))) return (st);
     const int32_t nnz = cz.nnz;
     z->n_k = nnz;
-    if (levels_done) {
-        e = cudaMemcpyAsync(ws->host, ctl, sizeof(CompressCtl), cudaMemcpyDeviceToHost, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e != cudaSuccess) return (note_cuda_error(e, "read result lengths"));
-        CompressCtl h;
-        std::memcpy(&h, ws->host, sizeof(h));
-        z->n_i = h.n_i;
-        z->n_j = h.n_j;
-        if (h.n_i > cap_i || h.n_j > cap_j) return (NB200_E_CAPACITY);
-        return NB200_OK;
-    }
-
     const int tiles = (int)(((int64_t)nnz + NT * CVT - 1) / (NT * CVT));
     e = cudaMemsetAsync(compress_block, 0, sizeof(uint64_t) * ((size_t)tiles + 4), stream);
     if (e != cudaSuccess) return (note_cuda_error(e, "cudaMemsetAsync"));
@@ -464,7 +442,7 @@ int csf_inner_run(const nb200_csf3 *a, const nb200_csf3 *b, float *z, void *stre
     NB200_CUDA(cudaGetLastError());
     nb200_coo3 ca{{a->dims[0], a->dims[1], a->dims[2]}, a->n_k, ai, aj, a->k_idx, a->val};
     nb200_coo3 cb{{b->dims[0], b->dims[1], b->dims[2]}, b->n_k, bi, bj, b->k_idx, b->val};
-    return coo3_inner_run(&ca, &cb, z, stream_v, merge_scratch, ws->host);
+    return coo3_inner_run(&ca, &cb, z, stream_v, merge_scratch, ws);
 }
 
 }  // namespace

@@ -78,26 +78,6 @@ __device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, lon
 
 // ------------------------------------------------------------------------- partition ----
 
-// Number of leading true values of a monotone pred over [lo, hi), returned as lo + count; G
-// neighbouring lanes search together, each group of a warp on its own range. All 32 lanes call this
-// together; a group that is done idles until the warp's last one is.
-template <int G, typename Pred>
-__device__ __forceinline__ uint32_t group_count_true(uint32_t lo, uint32_t hi, Pred pred) {
-    const int in_group = lane_id() & (G - 1), shift = lane_id() & ~(G - 1);
-    while (__any_sync(FULL_MASK, lo < hi)) {
-        const uint32_t step = lo < hi ? (hi - lo + G - 1) / G : 0u;
-        const uint32_t p = lo + (in_group + 1) * step - 1;
-        const bool ok = step > 0 && p < hi && pred(p);
-        const unsigned votes = __ballot_sync(FULL_MASK, ok);
-        const int c = __popc(G == 32 ? votes : (votes >> shift) & ((1u << (G & 31)) - 1u));
-        if (step > 0) {
-            lo += c * step;
-            hi = min(hi, lo + step - 1);
-        }
-    }
-    return lo;
-}
-
 // G lanes per cut. Cut t sits at merged position min(t * tile_step, total).
 template <int G>
 __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count, uint32_t total,

@@ -25,22 +25,6 @@ struct FusedCtl {
     long long total;      // result entries, written by the last tile (MODE_REDUCE: the bits of a double, the running sum)
 };
 
-// Optional second result form of the coordinate merge: the CSF3 levels above k. When a fused
-// launch of the COO3 tile kernel is given one of these, it does not write the merged i and j
-// columns; instead every tile flags the result entries that open a new i slice or a new (i, j)
-// fibre, obtains the number of slices / fibres of all earlier tiles by a second bounded look-back
-// (packed as slices << 31 | fibres in `tile_state`, one zeroed word per tile), and writes
-// i_idx / j_ptr / j_idx / k_ptr directly. The last tile leaves the totals in `totals`.
-struct CsfTotals {
-    int n_i, n_j;
-};
-struct CsfLevelsOut {
-    int32_t *i_idx, *j_ptr, *j_idx, *k_ptr;
-    int32_t cap_i, cap_j;  // entries the arrays can hold (offset arrays: one more)
-    uint64_t *tile_state;
-    CsfTotals *totals;
-};
-
 // ------------------------------------------------------------------- output bases ----
 //
 // The output base of a tile is the number of results of all earlier tiles, some 600 of which may still be
