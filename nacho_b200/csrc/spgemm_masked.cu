@@ -5,9 +5,8 @@
 // that survive the three-way intersection.
 //
 // Here the mask drives the accumulation, so nothing outside it is ever formed, sorted or written:
-//   k_sssmm_classify    one warp per row: does the row have fewer than LIGHT_P products (counted
-//                       only until that is known), and how wide (first to last column) and how
-//                       long is its mask row? The row goes on one of five lists.
+//   k_sssmm_classify    one warp per row: how many products does the row have, and how wide (first to
+//                       last column) and how long is its mask row? The row goes on one of six lists.
 //   k_sssmm_bitmap      rows with many products, one CTA per row taken from a ticket: the mask row
 //                       becomes a bitmap over its column span in shared memory plus, per 64-bit
 //                       word, the count of set bits before it. A product tests one bit; a hit finds
@@ -16,6 +15,8 @@
 //                       shared-memory accumulator (rows whose mask row is too long for that, or
 //                       whose span needs the whole shared memory, accumulate in global memory).
 //                       Three list classes, by the shared memory a row needs.
+//   k_sssmm_look_up     rows with a mask row of some dozens of positions, one warp per row: the other way round,
+//                       the mask's columns are searched in the rows of B, sums in registers.
 //   k_sssmm_search_*    rows with few products (one warp per row) and rows whose span exceeds the
 //                       largest bitmap (one CTA per row): binary search of the product's column in
 //                       the mask row, float atomics on the global accumulators.
@@ -35,8 +36,11 @@ namespace {
 
 constexpr int LIGHT_P = 256;    // rows with fewer products than this are searched by one warp
 constexpr int SEARCH_NT = 128;  // threads of a searching CTA
-// lists: bitmap classes 0..2, wide rows (searched by a CTA), light rows (searched by a warp)
-constexpr int LIST_WIDE = 3, LIST_LIGHT = 4;
+// lists: bitmap classes 0..2, wide rows (searched by a CTA), light rows (searched by a warp), rows whose mask
+// positions are looked up in B
+constexpr int LIST_WIDE = 3, LIST_LIGHT = 4, LIST_MASK = 5;
+constexpr int MASK_UNIT = 8;    // entries of A's row that one warp looks the mask row up for: its searches are a chain of loads
+                                // (R-MAT 15021 vertices: 83 us with 8, 89 with 16, 134 with 64)
 constexpr int WARP_ENTRIES = 8; // entries of A's row one warp of a unit takes
 
 // Work classes. A unit of work is a run of `unit` consecutive entries of one row of A (a row with
@@ -75,31 +79,38 @@ __global__ void __launch_bounds__(256) k_sssmm_classify(CsrView A, CsrView B, Cs
         const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
         const int32_t a_lo = ld_nc(A.rp + i), a_hi = ld_nc(A.rp + i + 1);
         if (c_lo == c_hi || a_lo == a_hi) continue;
-        unsigned products = 0;  // exact below LIGHT_P, a lower bound beyond
-        for (int32_t p0 = a_lo; p0 < a_hi && products < LIGHT_P; p0 += 32) {
-            unsigned mine = 0;
-            if (p0 + lane < a_hi) {
-                const int32_t j = ld_nc(A.col + p0 + lane);
-                mine = min((unsigned)(ld_nc(B.rp + j + 1) - ld_nc(B.rp + j)), (unsigned)LIGHT_P);
-            }
-            products += __reduce_add_sync(0xffffffffu, mine);
+        float mine = 0.f;  // rounding does not matter: the count only chooses a list
+        for (int32_t p = a_lo + lane; p < a_hi; p += 32) {
+            const int32_t j = ld_nc(A.col + p);
+            mine += (float)(ld_nc(B.rp + j + 1) - ld_nc(B.rp + j));
         }
-        if (products == 0) continue;
-        if (products < LIGHT_P) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+        const float products = mine;
+        if (products == 0.f) continue;
+        if (products < (float)LIGHT_P) {
             if (lane == 0) light[atomicAdd(&ctl->count[LIST_LIGHT], 1)] = (int32_t)i;
             continue;
         }
         const int32_t words = (ld_nc(C.col + c_hi - 1) >> 6) - (ld_nc(C.col + c_lo) >> 6) + 1, entries = c_hi - c_lo;
+        // Warp instructions of the two ways, roughly: looking the mask row up in every selected row of B costs
+        // 150 per entry and 32 mask positions; walking the products costs 4000 for the bitmap of the mask row,
+        // 200 per entry and 0.7 per product. R-MAT rows of a few dozen entries are an order of magnitude cheaper
+        // to look up, hub rows are not. (50021 vertices, 800003 edges: 506 us with 150, 534 with 300, 693 without
+        // the look-up.)
+        const float entries_a = (float)(a_hi - a_lo);
+        const bool by_mask = 150.f * entries_a * (float)((entries + 31) / 32) <= 4000.f + 200.f * entries_a + 0.7f * products;
         int list = LIST_WIDE;
-        if (words <= CLASS[0].words && entries <= CLASS[0].entries) list = 0;
+        if (by_mask) list = LIST_MASK;
+        else if (words <= CLASS[0].words && entries <= CLASS[0].entries) list = 0;
         else if (words <= CLASS[1].words && entries <= CLASS[1].entries) list = 1;
         else if (words <= CLASS[2].words) list = 2;
-        const int unit = list == 0 ? CLASS[0].unit() : list == LIST_WIDE ? CLASS[LIST_WIDE].unit() : CLASS[1].unit();
+        const int unit = list == LIST_MASK ? MASK_UNIT : list == 0 ? CLASS[0].unit() : list == LIST_WIDE ? CLASS[LIST_WIDE].unit() : CLASS[1].unit();
         const int n_units = (a_hi - a_lo + unit - 1) / unit;
         int base = 0;
         if (lane == 0) base = atomicAdd(&ctl->count[list], n_units);
         base = __shfl_sync(0xffffffffu, base, 0);
-        for (int u = lane; u < n_units; u += 32) units[list * list_cap + base + u] = make_int2((int)i, a_lo + u * unit);
+        for (int u = lane; u < n_units; u += 32) units[(list == LIST_MASK ? 4 : list) * list_cap + base + u] = make_int2((int)i, a_lo + u * unit);
     }
 }
 
@@ -142,6 +153,107 @@ __global__ void __launch_bounds__(256) k_sssmm_search_warp(CsrView A, CsrView B,
                 search_product(B, C, q, ld_nc(B.col + q), av, c_lo, c_hi, c0, acc, hit);
         }
     }
+}
+
+// The mask positions of one row, tile by tile of 32 NR, looked up in the rows of B that the entries
+// [p_begin, p_end) of A's row select, NE entries at a time: a lane keeps the sums of its NR positions in
+// registers and searches NE * NR rows side by side, so that the dependent loads of one search hide the others'.
+// The number of steps depends on the row of B alone, so the warp stays together. Terms are added in the order of
+// A's entries.
+template <int NE, int NR>
+__device__ __forceinline__ void look_up_tile(const CsrView &A, const CsrView &B, int32_t p_begin, int32_t p_end, const int32_t (&k)[4],
+                                             const float (&cv)[4], float (&sum)[4], unsigned &found) {
+    const int lane = lane_id();
+    for (int32_t p0 = p_begin; p0 < p_end; p0 += 32) {
+        int32_t my_lo = 0, my_len = 0;
+        float my_a = 0.f;
+        if (p0 + lane < p_end) {
+            const int32_t j = ld_nc(A.col + p0 + lane);
+            my_lo = ld_nc(B.rp + j);
+            my_len = ld_nc(B.rp + j + 1) - my_lo;
+            my_a = ld_nc(A.val + p0 + lane);
+        }
+        const int n_here = min(32, p_end - p0);
+        for (int e0 = 0; e0 < n_here; e0 += NE) {
+            int32_t at[NE][NR];
+            int n[NE], len[NE], longest = 0;
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                const int32_t lo = __shfl_sync(FULL_MASK, my_lo, (e0 + e) & 31);
+                const int32_t l = __shfl_sync(FULL_MASK, my_len, (e0 + e) & 31);
+                len[e] = n[e] = e0 + e < n_here ? l : 0;
+                longest = max(longest, n[e]);
+#pragma unroll
+                for (int r = 0; r < NR; ++r) at[e][r] = lo;
+            }
+            for (; longest > 1; longest -= longest >> 1) {  // the last position of the row whose column is <= k, or its first
+#pragma unroll
+                for (int e = 0; e < NE; ++e) {
+                    if (n[e] > 1) {  // uniform
+                        const int half = n[e] >> 1;
+#pragma unroll
+                        for (int r = 0; r < NR; ++r) at[e][r] += ld_nc(B.col + at[e][r] + half) <= k[r] ? half : 0;
+                        n[e] -= half;
+                    }
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < NE; ++e) {
+                const float a = __shfl_sync(FULL_MASK, my_a, (e0 + e) & 31);
+                if (len[e] > 0) {  // uniform
+#pragma unroll
+                    for (int r = 0; r < NR; ++r) {
+                        if (ld_nc(B.col + at[e][r]) == k[r]) {
+                            sum[r] += (a * ld_nc(B.val + at[e][r])) * cv[r];
+                            found |= 1u << r;
+                        }
+                    }
+                }
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sssmm_look_up(CsrView A, CsrView B, CsrView C, const int2 *__restrict__ units,
+                                                      SssmmCtl *__restrict__ ctl, float *__restrict__ acc, int32_t *__restrict__ hit) {
+    trigger_dependents();
+    const int lane = lane_id();
+    const int32_t c0 = ld_nc(C.rp);
+    const int count = ctl->count[LIST_MASK];
+    for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(&ctl->ticket[LIST_MASK], 1);
+        t = __shfl_sync(FULL_MASK, t, 0);
+        if (t >= count) break;
+        const int2 unit = units[t];
+        const int64_t i = unit.x;
+        const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1), a_lo = ld_nc(A.rp + i), a_hi = ld_nc(A.rp + i + 1);
+        const int32_t p_end = min(unit.y + MASK_UNIT, a_hi);
+        const bool alone = a_hi - a_lo <= MASK_UNIT;  // no other unit adds to this row's sums
+        for (int32_t m0 = c_lo; m0 < c_hi; m0 += 128) {
+            int32_t k[4];
+            float cv[4], sum[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned found = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int32_t m = m0 + 32 * r + lane;
+                k[r] = m < c_hi ? ld_nc(C.col + m) : -1;
+                cv[r] = m < c_hi ? ld_nc(C.val + m) : 0.f;
+            }
+            const int left = c_hi - m0;
+            if (left <= 32) look_up_tile<8, 1>(A, B, unit.y, p_end, k, cv, sum, found);
+            else if (left <= 64) look_up_tile<4, 2>(A, B, unit.y, p_end, k, cv, sum, found);
+            else look_up_tile<2, 4>(A, B, unit.y, p_end, k, cv, sum, found);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (!((found >> r) & 1u)) continue;
+                const int32_t at = m0 + 32 * r + lane - c0;
+                if (alone) acc[at] = sum[r]; else atomicAdd(acc + at, sum[r]);
+                hit[at] = 1;
+            }
+        }
+    }
+    finish_after_previous();
 }
 
 constexpr int PER_LANE = 8;           // products of a chunk per lane: that many loads in flight
@@ -421,13 +533,14 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     NB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
 
     const int scan_ctas = (int)(((int64_t)nnz + 1 + SCAN_NT * SCAN_VT - 1) / (SCAN_NT * SCAN_VT));
-    const int64_t list_cap = (int64_t)rows + a->nnz / CLASS[LIST_WIDE].unit() + 1;  // the smallest unit bounds every list
+    const int64_t list_cap = (int64_t)rows + a->nnz / CLASS[LIST_WIDE].unit() + 1;  // the smallest unit of those classes bounds every list
+    const int64_t mask_cap = (int64_t)rows + a->nnz / MASK_UNIT + 1;
     Carver sizes;
     sizes.take<float>((size_t)nnz);
     sizes.take<int32_t>((size_t)nnz + 1);
     sizes.take<uint64_t>((size_t)scan_ctas + 8);
     sizes.take<SssmmCtl>(1);
-    sizes.take<int2>((size_t)4 * list_cap);
+    sizes.take<int2>((size_t)4 * list_cap + mask_cap);
     sizes.take<int32_t>((size_t)rows);
     Workspace *ws = nullptr;
     if ((st = acquire_workspace(stream, sizes.used(), &ws, 1))) return st;
@@ -436,7 +549,7 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     int32_t *hit = carve.take<int32_t>((size_t)nnz + 1);
     uint64_t *scan_block = carve.take<uint64_t>((size_t)scan_ctas + 8);
     SssmmCtl *sctl = carve.take<SssmmCtl>(1);
-    int2 *units = carve.take<int2>((size_t)4 * list_cap);
+    int2 *units = carve.take<int2>((size_t)4 * list_cap + mask_cap);
     int32_t *light = carve.take<int32_t>((size_t)rows);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(scan_block);
     // sums, flags and control blocks lie next to one another: one fill clears them all
@@ -465,6 +578,10 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
         LaunchScope scope("sssmm_bitmap_narrow", stream);
         NB200_CUDA(launch_overlapped(k_sssmm_bitmap<256, true>, dim3(std::min(8 * sms, most)), dim3(256), CLASS[0].smem(), stream, A, B, C, units, sctl, 0,
                                      CLASS[0].words, CLASS[0].entries, acc, hit));
+    }
+    {
+        LaunchScope scope("sssmm_look_up", stream);
+        NB200_CUDA(launch_overlapped(k_sssmm_look_up, dim3(row_warps_grid), dim3(256), 0, stream, A, B, C, units + (size_t)4 * list_cap, sctl, acc, hit));
     }
     {
         LaunchScope scope("sssmm_search_wide", stream);
