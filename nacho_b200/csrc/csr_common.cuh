@@ -1,5 +1,5 @@
-// Types and small helpers shared by the CSR element-wise kernels (two-operand kernels in
-// csr_merge.cu, the fused three-operand add in csr_add3.cu).
+// Types and small helpers shared by the CSR element-wise kernels (csr_merge.cu) and by the formats that run on
+// them (formats2d.cu, csf3_add.cu).
 #pragma once
 
 #include <stdint.h>
@@ -11,13 +11,15 @@
 
 namespace nb200 {
 
-constexpr int CSR_NT = 256;  // worker threads of a CSR tile CTA (one more warp scans)
+constexpr int CSR_NT = 256;  // threads of a CSR tile CTA
 
 struct CsrIn {
     const int32_t *rp;  // null: a single row that holds all entries
     const int32_t *col;
     const float *val;
-    int32_t nnz;
+    int32_t nnz;                         // stored entries, or the most there can be where
+    const long long *nnz_dev = nullptr;  // an earlier launch on the stream leaves their number in device memory
+    __device__ __forceinline__ int32_t entries() const { return nnz_dev ? (int32_t)*nnz_dev : nnz; }
 };
 
 struct CsrOut {
@@ -45,16 +47,10 @@ struct LevelOffsets {
     int32_t *off_a = nullptr, *off_b = nullptr, *keep = nullptr;
 };
 
-__device__ __forceinline__ int32_t row_offset(const CsrIn &m, int64_t r) { return m.rp ? ld_nc(m.rp + r) : r > 0 ? m.nnz : 0; }
-
-// Hardware barriers of the tile kernels: 0 = the whole CTA (__syncthreads), 1 = the worker
-// threads, 2 = workers arrive / the scan warp waits ("the tile's count is known").
-using WorkerBar = NamedBarrier<1, CSR_NT>;
-using CountBar = NamedBarrier<2, CSR_NT + 32>;
+__device__ __forceinline__ int32_t row_offset(const CsrIn &m, int64_t r) { return m.rp ? ld_nc(m.rp + r) : r > 0 ? m.entries() : 0; }
 
 constexpr int MBAR_POLL_LIMIT = 1 << 24;
 constexpr int ERR_COPY_TIMEOUT = 2;
-constexpr int ERR_WIDE_TILE = 3;  // a tile's rows do not fit the 32-bit composite key of a kernel without a wide-key body
 
 // Number of 4-byte elements from `p` up to the next 16-byte boundary (0..3).
 __device__ __forceinline__ int head_elems(const void *p) {
@@ -88,10 +84,5 @@ constexpr long long RW_HOLLOW = 1ll << 48;  // beside the length in a result wor
 size_t csr2_scratch_bytes(int64_t entries);
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl);
-
-// Two chained two-operand unions (A + B) + C through a pool intermediate: the route of callers
-// whose capacity is below the worst case, and of inputs the fused kernel does not take.
-int csr_add3_chained(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, bool alloc, int64_t capacity,
-                     void *stream_v);
 
 }  // namespace nb200

@@ -70,8 +70,8 @@ int note_cuda_error(cudaError_t e, const char *what) {
 }
 
 int note_timeout(int site, int tile, const char *where) {
-    static const char *const names[] = {"?", "look-back over earlier tiles", "bulk copy into shared memory", "tile wider than its key"};
-    std::snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s gave up at tile %d", where, names[site >= 1 && site <= 3 ? site : 0], tile);
+    static const char *const names[] = {"?", "look-back over earlier tiles", "bulk copy into shared memory"};
+    std::snprintf(g_cuda_error, sizeof(g_cuda_error), "%s: %s gave up at tile %d", where, names[site >= 1 && site <= 2 ? site : 0], tile);
     return NB200_E_TIMEOUT;
 }
 
