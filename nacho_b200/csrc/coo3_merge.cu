@@ -236,34 +236,45 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         if (x > 0 && y < nb && key_at_byte(4u * (uint32_t)(oa + x - 1)) == key_at_byte(4u * (uint32_t)(ob + y))) ++y;
     }
 
-    // ---- merge, one result entry per step; src[i]: the entry step i took (A's where both), top bit set where both
+    // ---- merge, one result entry per step; src[i]: the entry step i took (A's where both)
     const uint32_t pa0 = 4u * (uint32_t)(oa + x), pb0 = 4u * (uint32_t)(ob + y);
     uint32_t src[VT];
     unsigned twin = 0;
-    int steps = 0;
+    int steps;
     {
+        // (as in the CSR tile kernel: VT steps for everybody, cut to the thread's share afterwards, and the key behind each
+        // head a step ahead. Past its end a list reads other words of the tile's shared memory.)
         uint32_t pa = pa0, pb = pb0;
-        const uint32_t end = 4u * (uint32_t)(oa + ob + min(tid * VT + VT, n));
-        Key ka = diag < n ? key_at_byte(pa) : END, kb = diag < n ? key_at_byte(pb) : END;
+        Key ka = key_at_byte(pa), kb = key_at_byte(pb);
+        Key next_a = key_at_byte(pa + 4), next_b = key_at_byte(pb + 4);
 #pragma unroll
         for (int i = 0; i < VT; ++i) {
-            const bool go = pa + pb < end;
-            const bool ta = go && ka <= kb, tb = go && kb <= ka;
+            const bool ta = ka <= kb, tb = kb <= ka;
             src[i] = ta ? pa : pb;
-            if (ta && tb) {
-                twin |= 1u << i;
-                src[i] |= 0x8000u;
-            }
+            if (ta && tb) twin |= 1u << i;
             if (ta) {
                 pa += 4;
-                ka = key_at_byte(pa);
+                ka = next_a;
+                next_a = key_at_byte(pa + 4);
             }
             if (tb) {
                 pb += 4;
-                kb = key_at_byte(pb);
+                kb = next_b;
+                next_b = key_at_byte(pb + 4);
             }
-            if (go) ++steps;
         }
+        // step i is the thread's where the entries taken before it, i + (twins before it), are fewer than its share
+        const int share = min(tid * VT + VT, n) - (x + y);
+        steps = share;
+        if (__any_sync(FULL_MASK, twin != 0u)) {
+            int lo = 0, hi = max(share, 0);
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (mid + __popc(twin & ((1u << mid) - 1u)) >= share) hi = mid; else lo = mid + 1;
+            }
+            steps = lo;
+        }
+        twin &= (1u << steps) - 1u;
     }
 
     // ---- rank the survivors inside the tile
@@ -290,8 +301,8 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) {
-                const uint32_t at = src[i] & 0x7fffu;
-                word_at(at) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - at;
+                word_at(src[i]) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - src[i];
+                src[i] |= 0x8000u;
             }
     }
     {

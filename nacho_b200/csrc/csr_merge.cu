@@ -139,7 +139,8 @@ struct TilePlan {
     static_assert(4 * SLOTS < 32768, "byte offsets of entries are kept in 15 bits");
 };
 constexpr uint32_t ROW_FAR = 0xffffu;
-constexpr int ROWS_CAP = 1024;  // row starts kept in shared memory; tiles with more rows search the offsets in global memory
+constexpr int ROWS_CAP = 1856;  // row starts kept in shared memory (the most of which four CTAs fit an SM); tiles with more rows search the
+                                // offsets in global memory
 constexpr int GATHER = 8;       // result entries a thread fetches together
 
 // Fixed shared memory of a tile (one block for both key widths).
@@ -147,8 +148,8 @@ struct TileShared {
     uint64_t mbar;
     long long base;                 // output base of the tile
     uint32_t rows[ROWS_CAP + 2];    // start of row r in the tile: A's in the lower half, B's in the upper
-    int trow[NT], wrow[NT / 32];    // the last row that starts at or before a thread's / between two warps' diagonals
-    int rank[NT];
+    int trow[NT], wrow[NT / 32];    // the last row that starts at or before a thread's / between two warps' diagonals;
+                                    // once every thread has its row, trow holds the threads' first results instead
     unsigned twin[NT];
     int wtotal[NT / 32];            // survivors of each warp
 };
@@ -182,7 +183,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     constexpr Key END = WIDE ? (Key)~0ull : (Key)0x80000000u;  // after every key (narrow: keys are below 2^31), also with row bits added
     constexpr bool WRITES = MODE != MODE_COUNT;
     uint32_t *s_rows = sh.rows;
-    int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.rank, *s_wtotal = sh.wtotal;
+    int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.trow, *s_wtotal = sh.wtotal;
     unsigned *s_twin = sh.twin;
     long long &s_base = sh.base;
     uint64_t *mbar = &sh.mbar;
@@ -334,29 +335,28 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     const uint32_t pa0 = 4u * (uint32_t)(oa + x), pb0 = 4u * (uint32_t)(ob + y);
     uint32_t src[VT];
     unsigned twin = 0;  // bit i: step i took an entry of each operand
-    int steps = 0;
+    int steps;
     {
+        // Every thread takes VT steps, whatever its share: what runs over the end (into the next thread's share, or past
+        // a sentinel into other words of the tile's shared memory) is cut off afterwards, which is cheaper than a test
+        // per step. The word behind each head is loaded a step ahead, so that a step waits for no load of its own.
         uint32_t pa = pa0, pb = pb0;
-        const uint32_t end = 4u * (uint32_t)(oa + ob + min(tid * VT + VT, n));  // pa + pb once the share is done
+        uint32_t next_a = word_at(pa + 4), next_b = word_at(pb + 4);
 #pragma unroll
         for (int i = 0; i < VT; ++i) {
-            const bool go = pa + pb < end;
-            const bool ta = go && ka <= kb, tb = go && kb <= ka;
+            const bool ta = ka <= kb, tb = kb <= ka;
             const uint32_t row_bits = (uint32_t)min(ka, kb) & ~cmask;
             if (LEVELS) {
                 src[i] = (pa | (ta ? 1u : 0u)) | (pb | (tb ? 1u : 0u)) << 16;
-                if (ta && tb) twin |= 1u << i;
             } else {
                 src[i] = ta ? pa : pb;
-                if (ta && tb) {
-                    twin |= 1u << i;
-                    src[i] |= 0x8000u;
-                }
             }
+            if (ta && tb) twin |= 1u << i;
             if (ta) {
                 pa += 4;
                 if (!WIDE) {
-                    ka = (Key)(row_bits + word_at(pa));
+                    ka = (Key)(row_bits + next_a);
+                    next_a = word_at(pa + 4);
                 } else {
                     const int at = (int)(pa >> 2), pos = at - oa;
                     if (pos < na && row_mark[at]) row_a = marked_row(at, pos, row_a, 0);
@@ -366,15 +366,27 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             if (tb) {
                 pb += 4;
                 if (!WIDE) {
-                    kb = (Key)(row_bits + word_at(pb));
+                    kb = (Key)(row_bits + next_b);
+                    next_b = word_at(pb + 4);
                 } else {
                     const int at = (int)(pb >> 2), pos = at - ob;
                     if (pos < nb && row_mark[at]) row_b = marked_row(at, pos, row_b, 16);
                     kb = pos < nb ? (Key)(((uint64_t)(uint32_t)row_b << 32) | word_at(pb)) : END;
                 }
             }
-            if (go) ++steps;
         }
+        // step i is the thread's where the entries taken before it, i + (twins before it), are fewer than its share
+        const int share = min(tid * VT + VT, n) - diag - shifted;
+        steps = share;
+        if (__any_sync(FULL_MASK, twin != 0u)) {
+            int lo = 0, hi = share;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (mid + __popc(twin & ((1u << mid) - 1u)) >= share) hi = mid; else lo = mid + 1;
+            }
+            steps = lo;
+        }
+        twin &= (1u << steps) - 1u;
     }
 
     // ---- rank the survivors inside the tile
@@ -404,8 +416,8 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) {
-                const uint32_t at = src[i] & 0x7fffu;
-                word_at(at) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - at;
+                word_at(src[i]) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - src[i];
+                src[i] |= 0x8000u;
             }
     }
     {
