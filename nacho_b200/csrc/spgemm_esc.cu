@@ -431,13 +431,15 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
                                                        int32_t *__restrict__ c_col, float *__restrict__ c_val) {
     __shared__ uint64_t keys[MEDIUM_P];
     __shared__ float vals[NUMERIC ? MEDIUM_P : 1];
-    __shared__ int scan_tmp[40];
+    __shared__ int seg_off[MED_NT], seg_start[MED_NT];
+    __shared__ float seg_a[NUMERIC ? MED_NT : 1];
+    __shared__ int scan_tmp[72];
     trigger_dependents();
     const int tid = threadIdx.x;
     const int32_t i = ld_nc(row_list + blockIdx.x);
     const int32_t lo = ld_nc(A.rp + i), hi = ld_nc(A.rp + i + 1);
 
-    int p_total = 0;
+    int p_total = 0, rows_of_b = 0;
     for (int32_t chunk = lo; chunk < hi; chunk += MED_NT) {  // expand phase 2, MED_NT entries of A at a time
         const int32_t e = chunk + tid;
         int32_t b_lo = 0, len = 0;
@@ -448,21 +450,35 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
             len = ld_nc(B.rp + j + 1) - b_lo;
             if (NUMERIC) a = ld_nc(A.val + e);
         }
-        int chunk_total;
-        const int off = block_excl_sum<MED_NT>(len, scan_tmp, chunk_total);
-        for (int q = 0; q < len; ++q) {
-            const int idx = p_total + off + q;
-            keys[idx] = ((uint64_t)(uint32_t)ld_nc(B.col + b_lo + q) << 32) | (uint32_t)idx;
-            if (NUMERIC) vals[idx] = a * ld_nc(B.val + b_lo + q);
+        int k, off, n, chunk_total;
+        block_excl_sum2<MED_NT>(len > 0 ? 1 : 0, len, scan_tmp, k, off, n, chunk_total);
+        if (len > 0) {
+            seg_off[k] = off;
+            seg_start[k] = b_lo;
+            if (NUMERIC) seg_a[k] = a;
+        }
+        __syncthreads();
+        for (int p = tid; p < chunk_total; p += MED_NT) {  // thread = product: a long row of B is not one thread's work
+            int seg = 0, above = n;
+            while (above - seg > 1) {
+                const int mid = (seg + above) >> 1;
+                if (seg_off[mid] <= p) seg = mid; else above = mid;
+            }
+            const int32_t q = seg_start[seg] + (p - seg_off[seg]);
+            const int idx = p_total + p;
+            keys[idx] = ((uint64_t)(uint32_t)ld_nc(B.col + q) << 32) | (uint32_t)idx;
+            if (NUMERIC) vals[idx] = seg_a[seg] * ld_nc(B.val + q);
         }
         p_total += chunk_total;
+        rows_of_b += n;
+        __syncthreads();
     }
     int n2 = 2;
     while (n2 < p_total) n2 <<= 1;
     for (int p = p_total + tid; p < n2; p += MED_NT) keys[p] = ~0ull;
     __syncthreads();
 
-    for (int k = 2; k <= n2; k <<= 1) {  // sort
+    for (int k = rows_of_b > 1 ? 2 : n2 + 1; k <= n2; k <<= 1) {  // sort (one row of B is in order)
         for (int j = k >> 1; j > 0; j >>= 1) {
             for (int p = tid; p < (n2 >> 1); p += MED_NT) {
                 const int i1 = 2 * j * (p / j) + (p % j), i2 = i1 + j;
@@ -501,97 +517,78 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
 
 // ----------------------------------------------------------------- product walk ----
 
-#ifndef ESC_WIN_ITEMS
-#define ESC_WIN_ITEMS 4  // 32-product blocks a warp keeps in flight
-#endif
+constexpr int CHUNK = 32;           // products a warp takes with one instruction; a chunk lies in one row of B
+constexpr int FLIGHT = 4;  // chunks whose loads a warp keeps in flight (8 measured slower: registers; 2: 2616 against 2579 us)
 
-// Walks a flat product range cut into segments: segment k covers the products
-// [seg_off[k], seg_off[k + 1]) and they are the entries seg_start[k] ... of B, each multiplied
-// by seg_a[k]; every segment is non-empty and seg_off[n_seg] == total. Called by all NT threads
-// of the CTA. Every warp takes one contiguous share of the range (a multiple of 32 products) and
-// moves through it 32 products at a time, lane = product, so the loads from B coalesce; the
-// segment of the current block is warp-uniform state that only moves forward, and a block that
-// lies inside one segment (the common case for long rows of B) needs no per-lane search.
-// ESC_WIN_ITEMS blocks have their loads in flight together. f(column, value) gets every product.
-template <int NT, bool WITH_VALUES, typename F>
-__device__ __forceinline__ void walk_segments(const int *seg_off, const int *seg_start, const float *seg_a, int n_seg, int total,
-                                              const CsrView &B, F f) {
-    constexpr int NW = NT / 32;
-    const int share = ((total + NW * 32 - 1) / (NW * 32)) * 32;
-    int pb = warp_id() * share;
-    const int pe = min(pb + share, total);
-    if (pb >= pe) return;
-    int k = 0;
-    {  // largest k with seg_off[k] <= pb
-        int h = n_seg - 1;
-        while (k < h) {
-            const int mid = (k + h + 1) >> 1;
-            if (seg_off[mid] <= pb)
-                k = mid;
-            else
-                h = mid - 1;
-        }
+// The rows of B that a chunk of A's row selects, as segments: segment k covers the chunks [first[k], first[k + 1]) of
+// the flat chunk sequence, and its products are the entries start[k] .. start[k] + len[k] - 1 of B, each multiplied by
+// a[k]. Only non-empty segments.
+template <int NT>
+struct Segments {
+    int first[NT], start[NT], len[NT];
+    float a[NT];
+    int n, chunks;
+};
+
+// Lists the segments of the CTA's threads ({start, len, a} of the thread's entry of A; len 0: none). All NT threads; ends
+// with a barrier. `tmp`: 72 ints.
+template <int NT>
+__device__ __forceinline__ void list_segments(Segments<NT> &seg, int *tmp, int32_t start, int len, float a) {
+    int k, off, n, chunks;
+    block_excl_sum2<NT>(len > 0 ? 1 : 0, (len + CHUNK - 1) / CHUNK, tmp, k, off, n, chunks);
+    if (len > 0) {
+        seg.first[k] = off;
+        seg.start[k] = start;
+        seg.len[k] = len;
+        seg.a[k] = a;
     }
-    int k_end = seg_off[k + 1];
-    int delta = seg_start[k] - seg_off[k];  // position in B = delta + product index
-    float k_a = WITH_VALUES ? seg_a[k] : 0.f;
-    for (; pb < pe; pb += 32 * ESC_WIN_ITEMS) {
-        while (pb >= k_end) {
-            ++k;
-            k_end = seg_off[k + 1];
-            delta = seg_start[k] - seg_off[k];
-            if (WITH_VALUES) k_a = seg_a[k];
+    if (threadIdx.x == 0) {
+        seg.n = n;
+        seg.chunks = chunks;
+    }
+    __syncthreads();
+}
+
+// Walks all products of the segments: f(column, value). Every warp takes one contiguous share of the chunks. For 32 chunks
+// at a time every lane finds the segment of one of them by binary search; then the chunks go by one after the other, what
+// their lane knows broadcast, lane = product, so that the loads from B coalesce, nothing diverges, and FLIGHT chunks
+// have their loads in flight. (Products dealt out in a flat sequence, blocks of 128, took 44 instructions per 32 products
+// where the rows of B hold a hundred entries: the blocks cross rows, and every lane then searches its own. The symbolic
+// pass of 65536 vertices' heavy rows 375 -> 293 us, of 24405 vertices' 94 -> 63.)
+template <int NT, bool WITH_VALUES, typename F>
+__device__ __forceinline__ void walk_segments(const Segments<NT> &seg, const CsrView &B, F f) {
+    constexpr int NW = NT / 32;
+    const int lane = lane_id(), n_seg = seg.n, share = (seg.chunks + NW - 1) / NW;
+    const int c_end = min((warp_id() + 1) * share, seg.chunks);
+    for (int c = warp_id() * share; c < c_end; c += 32) {
+        const int mine = min(c + lane, c_end - 1);
+        int k = 0, above = n_seg;  // the last segment that begins at or before this lane's chunk
+        while (above - k > 1) {
+            const int mid = (k + above) >> 1;
+            if (seg.first[mid] <= mine) k = mid; else above = mid;
         }
-        if (pb + 32 * ESC_WIN_ITEMS <= min(k_end, pe)) {  // uniform: all the blocks lie inside segment k
-            const int32_t *bc = B.col + (delta + pb + lane_id());
-            const float *bvp = B.val + (delta + pb + lane_id());
-            int32_t c[ESC_WIN_ITEMS];
-            float bv[ESC_WIN_ITEMS];
+        const int at = (mine - seg.first[k]) * CHUNK;
+        const int my_q = seg.start[k] + at, my_n = c + lane < c_end ? seg.len[k] - at : 0;
+        const float my_a = WITH_VALUES ? seg.a[k] : 0.f;
+        const int here = min(32, c_end - c);
+        for (int u = 0; u < here; u += FLIGHT) {
+            int32_t col[FLIGHT];
+            float val[FLIGHT];
+            unsigned live = 0;
 #pragma unroll
-            for (int it = 0; it < ESC_WIN_ITEMS; ++it) {
-                c[it] = ld_nc(bc + 32 * it);
-                bv[it] = WITH_VALUES ? ld_nc(bvp + 32 * it) : 0.f;
+            for (int j = 0; j < FLIGHT; ++j) {
+                const int q = __shfl_sync(FULL_MASK, my_q, u + j), n = __shfl_sync(FULL_MASK, my_n, u + j);
+                const bool ok = lane < n;  // chunks past the share have n = 0 (u + j stays below 32: FLIGHT divides it)
+                live |= (unsigned)ok << j;
+                col[j] = ok ? ld_nc(B.col + q + lane) : 0;
+                if (WITH_VALUES) val[j] = ok ? ld_nc(B.val + q + lane) : 0.f;
             }
 #pragma unroll
-            for (int it = 0; it < ESC_WIN_ITEMS; ++it) f(c[it], k_a * bv[it]);
-            continue;
-        }
-        int32_t q[ESC_WIN_ITEMS];
-        float av[ESC_WIN_ITEMS];
-#pragma unroll
-        for (int it = 0; it < ESC_WIN_ITEMS; ++it) {
-            const int b = pb + 32 * it;
-            q[it] = -1;
-            av[it] = 0.f;
-            if (b < pe) {
-                while (b >= k_end) {
-                    ++k;
-                    k_end = seg_off[k + 1];
-                    delta = seg_start[k] - seg_off[k];
-                    if (WITH_VALUES) k_a = seg_a[k];
-                }
-                const int p = b + lane_id();
-                if (b + 32 <= k_end) {
-                    q[it] = delta + p;
-                    av[it] = k_a;
-                } else if (p < pe) {
-                    int kk = k;
-                    while (seg_off[kk + 1] <= p) ++kk;  // ends: seg_off[n_seg] == total > p
-                    q[it] = seg_start[kk] + (p - seg_off[kk]);
-                    if (WITH_VALUES) av[it] = seg_a[kk];
-                }
+            for (int j = 0; j < FLIGHT; ++j) {
+                const float a = WITH_VALUES ? __shfl_sync(FULL_MASK, my_a, u + j) : 0.f;
+                if ((live >> j) & 1u) f(col[j], WITH_VALUES ? a * val[j] : 0.f);
             }
         }
-        int32_t c[ESC_WIN_ITEMS];
-        float bv[ESC_WIN_ITEMS];
-#pragma unroll
-        for (int it = 0; it < ESC_WIN_ITEMS; ++it) {
-            c[it] = q[it] >= 0 ? ld_nc(B.col + q[it]) : 0;
-            bv[it] = WITH_VALUES && q[it] >= 0 ? ld_nc(B.val + q[it]) : 0.f;
-        }
-#pragma unroll
-        for (int it = 0; it < ESC_WIN_ITEMS; ++it)
-            if (q[it] >= 0) f(c[it], av[it] * bv[it]);
     }
 }
 
@@ -602,9 +599,8 @@ constexpr int RK_WINDOW_COLS = RK_WORDS * 32;      // 262144 columns per window
 constexpr size_t RK_PTR_BUDGET = size_t(1) << 30;  // bytes of the window pointer table; beyond it windows are searched on the fly
 constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a CTA for rows up to / above RANKED_P products
 constexpr size_t HEAVY_SMEM_NUMERIC = 104 * 1024;  // dynamic shared memory of a numeric heavy-row CTA: two per SM
-#ifndef ESC_RANKED_SMEM_KB
-#define ESC_RANKED_SMEM_KB 0                       // of a numeric ranked-row CTA; 0: bitmap and ranks only, four per SM
-#endif
+constexpr int RK_MANY_ROWS = 8192;                 // from this many ranked rows on, their CTAs hold sums in shared memory too
+constexpr size_t RK_SMEM_NUMERIC = 32 * 1024;      // dynamic shared memory of such a CTA: bitmap, ranks, then sums
 
 // First index in [lo, hi) whose column is >= key (hi if none).
 __device__ __forceinline__ int32_t first_col_at_least(const int32_t *__restrict__ col, int32_t lo, int32_t hi, int64_t key) {
@@ -660,9 +656,7 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
     const uint64_t *bitmap64 = reinterpret_cast<const uint64_t *>(rk_smem);  // the same bits, 64 columns per element
     uint16_t *rank16 = reinterpret_cast<uint16_t *>(rk_smem + (size_t)words * 4);  // one rank per 64 columns
     float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * 5);
-    __shared__ int seg_off[NT + 1];
-    __shared__ int seg_start[NT];
-    __shared__ float seg_a[NUMERIC ? NT : 1];
+    __shared__ Segments<NT> seg;
     __shared__ int scan_tmp[72];
     __shared__ int warp_base[NT / 32];
     trigger_dependents();
@@ -688,7 +682,6 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
         auto pass = [&](bool build, auto f) -> bool {
             bool any = false;
             for (int32_t chunk = lo; chunk < hi; chunk += NT) {
-                int n_seg, total;
                 if (build) {
                     int32_t j = my_j;
                     float a = my_a;
@@ -713,24 +706,10 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
                             len = (w == n_win - 1 ? b_hi : first_col_at_least(B.col, s, b_hi, (int64_t)c_first + RK_WINDOW_COLS)) - s;
                         }
                     }
-                    int k_idx, off;
-                    block_excl_sum2<NT>(len > 0 ? 1 : 0, len, scan_tmp, k_idx, off, n_seg, total);
-                    if (len > 0) {
-                        seg_off[k_idx] = off;
-                        seg_start[k_idx] = s;
-                        if (NUMERIC) seg_a[k_idx] = a;
-                    }
-                    if (tid == 0) {
-                        seg_off[n_seg] = total;
-                        scan_tmp[70] = n_seg;
-                    }
-                    __syncthreads();
-                } else {
-                    n_seg = scan_tmp[70];
-                    total = seg_off[n_seg];
+                    list_segments<NT>(seg, scan_tmp, s, len, a);
                 }
-                any |= total > 0;
-                walk_segments<NT, NUMERIC>(seg_off, seg_start, seg_a, n_seg, total, B, f);
+                any |= seg.n > 0;
+                walk_segments<NT, NUMERIC>(seg, B, f);
                 __syncthreads();  // the segment arrays are rewritten by the next chunk
             }
             return any;
@@ -1079,14 +1058,17 @@ int launch_ranked(const CsrView &A, const CsrView &B, const EscPlan &plan, int32
     int wshift = 5;
     const int words = ranked_words(NT, b_cols, &wshift);
     // numeric: whatever the bitmap and the ranks leave of the CTA's shared memory accumulates sums
-    // The lighter rows do better without a shared accumulator: their CTAs are bound by the latency of
-    // a row's short phases, and four CTAs per SM hide more of it than three with an accumulator
-    // (7.7 against 9.2 ms on configuration 4a); the heavy rows gain (10.7 -> 7.5 ms).
-    const size_t budget = std::max(NT == HEAVY_NT ? HEAVY_SMEM_NUMERIC : (size_t)ESC_RANKED_SMEM_KB * 1024, (size_t)words * 5);
+    // Heavy rows always have some. The lighter ones only where there are many: a few thousand CTAs are bound by
+    // the latency of a row's short phases, and without a shared accumulator one more fits on an SM (a graph of 2698
+    // vertices 111 against 117 us, of 9000 vertices 198 against 209); tens of thousands are bound by the
+    // reductions that go to L2 instead (24405 vertices 434 -> 430 us, 65536 vertices 2579 -> 2436).
+    const size_t rows_budget = NT == HEAVY_NT ? HEAVY_SMEM_NUMERIC : n_rows >= RK_MANY_ROWS ? RK_SMEM_NUMERIC : 0;
+    const size_t budget = std::max(rows_budget, (size_t)words * 5);
     const int acc_slots = NUMERIC ? (int)((budget - (size_t)words * 5) / 4 / NT) * NT : 0;
     const size_t smem = NUMERIC ? (size_t)words * 5 + (size_t)acc_slots * 4 : (size_t)words * 4;
+    // the most that any call asks for: several threads may be here with different sizes
     NB200_CUDA(cudaFuncSetAttribute(k_esc_ranked<NUMERIC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(NUMERIC ? budget : (size_t)RK_WORDS * 4)));
+                                    (int)(NUMERIC ? std::max(HEAVY_SMEM_NUMERIC, (size_t)RK_WORDS * 5) : (size_t)RK_WORDS * 4)));
     return launch_bin(beside, k_esc_ranked<NUMERIC, NT>, n_rows, NT, smem, stream, A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift,
                       acc_slots, cache, count, c_rp, c_col, c_val);
 }
