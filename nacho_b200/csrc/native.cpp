@@ -8,12 +8,14 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "nacho_b200.h"
 
@@ -44,7 +46,7 @@ const at::Tensor &tensor_of(PyObject *obj, Name slot) {
         PyErr_SetString(PyExc_TypeError, "operand slot does not hold a tensor");
         throw PyFailure();
     }
-    return THPVariable_Unpack(t.p);  // the operand object keeps it alive
+    return THPVariable_Unpack(t.p);  // the operand object keeps it alive while the interpreter lock is held
 }
 
 template <int N>
@@ -72,51 +74,59 @@ void need_kind(PyObject *obj, Kind kind, const char *where, const char *what) {
 int32_t *ints(const at::Tensor &t) { return static_cast<int32_t *>(t.data_ptr()); }
 float *floats(const at::Tensor &t) { return static_cast<float *>(t.data_ptr()); }
 
-struct View {  // device of the operand, for the checks that all kinds share
+struct View {  // device and arrays of one operand, for what all kinds share
     c10::Device device = c10::Device(c10::kCPU);
+    at::Tensor arrays[6];  // references of their own: another thread may give the operand new arrays meanwhile
+    int n = 0;
+
+    const at::Tensor &array(PyObject *o, Name slot) {
+        arrays[n] = tensor_of(o, slot);
+        return arrays[n++];
+    }
+    int32_t *index(PyObject *o, Name slot) { return ints(array(o, slot)); }
 };
 
 nb200_csr view_csr(PyObject *o, View &v) {
-    const at::Tensor &val = tensor_of(o, N_values);
+    const at::Tensor &val = v.array(o, N_values);
     int32_t d[2];
     dims_of<2>(o, d);
     v.device = val.device();
-    return nb200_csr{d[0], d[1], (int32_t)val.numel(), ints(tensor_of(o, N_offsets)), ints(tensor_of(o, N_indices)), floats(val)};
+    return nb200_csr{d[0], d[1], (int32_t)val.numel(), v.index(o, N_offsets), v.index(o, N_indices), floats(val)};
 }
 
 nb200_coo view_coo(PyObject *o, View &v) {
-    const at::Tensor &val = tensor_of(o, N_values);
+    const at::Tensor &val = v.array(o, N_values);
     int32_t d[2];
     dims_of<2>(o, d);
     v.device = val.device();
-    return nb200_coo{d[0], d[1], (int32_t)val.numel(), ints(tensor_of(o, N_i)), ints(tensor_of(o, N_j)), floats(val)};
+    return nb200_coo{d[0], d[1], (int32_t)val.numel(), v.index(o, N_i), v.index(o, N_j), floats(val)};
 }
 
 nb200_dcsr view_dcsr(PyObject *o, View &v) {
-    const at::Tensor &val = tensor_of(o, N_values), &i = tensor_of(o, N_i);
+    const at::Tensor &val = v.array(o, N_values), &i = v.array(o, N_i);
     int32_t d[2];
     dims_of<2>(o, d);
     v.device = val.device();
-    return nb200_dcsr{d[0], d[1], (int32_t)i.numel(), (int32_t)val.numel(), ints(i), ints(tensor_of(o, N_jp)), ints(tensor_of(o, N_j)), floats(val)};
+    return nb200_dcsr{d[0], d[1], (int32_t)i.numel(), (int32_t)val.numel(), ints(i), v.index(o, N_jp), v.index(o, N_j), floats(val)};
 }
 
 nb200_coo3 view_coo3(PyObject *o, View &v) {
-    const at::Tensor &val = tensor_of(o, N_values);
+    const at::Tensor &val = v.array(o, N_values);
     nb200_coo3 s{};
     dims_of<3>(o, s.dims);
     v.device = val.device();
     s.nnz = (int32_t)val.numel();
-    s.i = ints(tensor_of(o, N_i)), s.j = ints(tensor_of(o, N_j)), s.k = ints(tensor_of(o, N_k)), s.val = floats(val);
+    s.i = v.index(o, N_i), s.j = v.index(o, N_j), s.k = v.index(o, N_k), s.val = floats(val);
     return s;
 }
 
 nb200_csf3 view_csf3(PyObject *o, View &v) {
-    const at::Tensor &val = tensor_of(o, N_values), &i = tensor_of(o, N_i), &j = tensor_of(o, N_j), &k = tensor_of(o, N_k);
+    const at::Tensor &val = v.array(o, N_values), &i = v.array(o, N_i), &j = v.array(o, N_j), &k = v.array(o, N_k);
     nb200_csf3 s{};
     dims_of<3>(o, s.dims);
     v.device = val.device();
     s.n_i = (int32_t)i.numel(), s.n_j = (int32_t)j.numel(), s.n_k = (int32_t)k.numel();
-    s.i_idx = ints(i), s.j_ptr = ints(tensor_of(o, N_jp)), s.j_idx = ints(j), s.k_ptr = ints(tensor_of(o, N_kp)), s.k_idx = ints(k), s.val = floats(val);
+    s.i_idx = ints(i), s.j_ptr = v.index(o, N_jp), s.j_idx = ints(j), s.k_ptr = v.index(o, N_kp), s.k_idx = ints(k), s.val = floats(val);
     return s;
 }
 
@@ -167,16 +177,30 @@ struct NoLock {  // releases the interpreter lock
     ~NoLock() { PyEval_RestoreThread(state); }
 };
 
-// Runs a C-ABI call on the operands' device and the current stream of the caller, without the interpreter lock.
-template <typename F>
-void launch(const View &v, const char *where, F call) {
-    c10::cuda::CUDAGuard guard(v.device);
-    void *stream = c10::cuda::getCurrentCUDAStream(v.device.index()).stream();
+// Calls of several host threads on one stream take turns at issuing their kernels: they share the stream's scratch
+// arrays and result words. A few locks serve all streams.
+std::mutex &stream_lock(void *stream) {
+    static std::mutex locks[61];
+    return locks[(reinterpret_cast<uintptr_t>(stream) >> 4) % 61];
+}
+
+// Runs a C-ABI call on the operands' device and the current stream of the caller, without the interpreter lock. A call
+// returns when the result's length is known, with kernels still running: the allocator is told that the
+// operands' arrays are in use on this stream, which matters when they came from another one.
+template <size_t N, typename F>
+void launch(const View *const (&operands)[N], const char *where, F call) {
+    const c10::Device device = operands[0]->device;
+    c10::cuda::CUDAGuard guard(device);
+    const c10::cuda::CUDAStream current = c10::cuda::getCurrentCUDAStream(device.index());
+    void *stream = current.stream();
     int status;
     {
         NoLock unlocked;
+        std::lock_guard<std::mutex> turn(stream_lock(stream));
         status = call(stream);
     }
+    for (const View *operand : operands)
+        for (int k = 0; k < operand->n; ++k) c10::cuda::CUDACachingAllocator::recordStream(operand->arrays[k].storage().data_ptr(), current);
     check(status, where);
 }
 
@@ -187,11 +211,12 @@ typedef int (*coo2_fn)(const nb200_coo *, const nb200_coo *, nb200_coo *, int64_
 typedef int (*dcsr2_fn)(const nb200_dcsr *, const nb200_dcsr *, nb200_dcsr *, int64_t, int64_t, void *);
 
 // A CSR result of up to `capacity` entries, filled by `call(z, stream)`.
-template <typename F>
-PyObject *csr_result(const View &v, const char *where, int32_t rows, int32_t cols, int64_t capacity, F call) {
-    at::Tensor rp = int_array((int64_t)rows + 1, v.device), col = int_array(capacity, v.device), val = float_array(capacity, v.device);
+template <size_t N, typename F>
+PyObject *csr_result(const View *const (&operands)[N], const char *where, int32_t rows, int32_t cols, int64_t capacity, F call) {
+    const c10::Device device = operands[0]->device;
+    at::Tensor rp = int_array((int64_t)rows + 1, device), col = int_array(capacity, device), val = float_array(capacity, device);
     nb200_csr z{rows, cols, 0, ints(rp), ints(col), floats(val)};
-    launch(v, where, [&](void *stream) { return call(&z, stream); });
+    launch(operands, where, [&](void *stream) { return call(&z, stream); });
     used(col, z.nnz);
     used(val, z.nnz);
     Result r(CSR);
@@ -207,7 +232,7 @@ PyObject *csr_binary(csr2_fn fn, bool is_union, const char *where, PyObject *con
     const nb200_csr a = view_csr(args[0], va), b = view_csr(args[1], vb);
     same_device(va, vb);
     const int64_t capacity = is_union ? (int64_t)a.nnz + b.nnz : std::min(a.nnz, b.nnz);
-    return csr_result(va, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return fn(&a, &b, z, capacity, stream); });
+    return csr_result({&va, &vb}, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return fn(&a, &b, z, capacity, stream); });
 }
 
 PyObject *csr_add(PyObject *const *args) { return csr_binary(nb200_csr_add_f32_into, true, "gpu_csr_add_f32", args); }
@@ -221,7 +246,7 @@ PyObject *csr_add_3(PyObject *const *args) {
     same_device(va, vb);
     same_device(va, vc);
     const int64_t capacity = (int64_t)a.nnz + b.nnz + c.nnz;
-    return csr_result(va, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_into(&a, &b, &c, z, capacity, stream); });
+    return csr_result({&va, &vb, &vc}, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_into(&a, &b, &c, z, capacity, stream); });
 }
 
 PyObject *sssmm(PyObject *const *args) {
@@ -231,7 +256,7 @@ PyObject *sssmm(PyObject *const *args) {
     const nb200_csr a = view_csr(args[0], va), b = view_csr(args[1], vb), c = view_csr(args[2], vc);
     same_device(va, vb);
     same_device(va, vc);
-    return csr_result(va, where, a.rows, b.cols, c.nnz, [&](nb200_csr *z, void *stream) { return nb200_sssmm_f32_into(&a, &b, &c, z, c.nnz, stream); });
+    return csr_result({&va, &vb, &vc}, where, a.rows, b.cols, c.nnz, [&](nb200_csr *z, void *stream) { return nb200_sssmm_f32_into(&a, &b, &c, z, c.nnz, stream); });
 }
 
 PyObject *coo_csr_add(PyObject *const *args) {
@@ -243,7 +268,7 @@ PyObject *coo_csr_add(PyObject *const *args) {
     const nb200_coo b = view_coo(args[1], vb);
     same_device(va, vb);
     const int64_t capacity = (int64_t)a.nnz + b.nnz;
-    return csr_result(va, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return nb200_coo_csr_add_f32_into(&a, &b, z, capacity, stream); });
+    return csr_result({&va, &vb}, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return nb200_coo_csr_add_f32_into(&a, &b, z, capacity, stream); });
 }
 
 PyObject *spgemm(PyObject *const *args) {
@@ -254,7 +279,7 @@ PyObject *spgemm(PyObject *const *args) {
     same_device(va, vb);
     at::Tensor rp = int_array((int64_t)a.rows + 1, va.device), col, val;
     nb200_csr c{a.rows, b.cols, 0, ints(rp), nullptr, nullptr};
-    launch(va, where, [&](void *stream) {
+    launch({&va, &vb}, where, [&](void *stream) {
         int64_t capacity;
         int st = nb200_spgemm_f32_bound(&a, &b, &capacity, stream);
         if (st != NB200_OK) return st;
@@ -286,7 +311,7 @@ PyObject *coo_binary(coo2_fn fn, bool is_union, const char *where, PyObject *con
     const int64_t capacity = is_union ? (int64_t)a.nnz + b.nnz : std::min(a.nnz, b.nnz);
     at::Tensor i = int_array(capacity, va.device), j = int_array(capacity, va.device), val = float_array(capacity, va.device);
     nb200_coo z{a.rows, a.cols, 0, ints(i), ints(j), floats(val)};
-    launch(va, where, [&](void *stream) { return fn(&a, &b, &z, capacity, stream); });
+    launch({&va, &vb}, where, [&](void *stream) { return fn(&a, &b, &z, capacity, stream); });
     used(i, z.nnz), used(j, z.nnz), used(val, z.nnz);
     Result r(COO);
     r.set(N_i, i), r.set(N_j, j), r.set(N_values, val);
@@ -307,7 +332,7 @@ PyObject *dcsr_binary(dcsr2_fn fn, bool is_union, const char *where, PyObject *c
     const int64_t capacity = is_union ? (int64_t)a.nnz + b.nnz : std::min(a.nnz, b.nnz);
     at::Tensor i = int_array(cap_i, va.device), jp = int_array(cap_i + 1, va.device), j = int_array(capacity, va.device), val = float_array(capacity, va.device);
     nb200_dcsr z{a.rows, a.cols, 0, 0, ints(i), ints(jp), ints(j), floats(val)};
-    launch(va, where, [&](void *stream) { return fn(&a, &b, &z, cap_i, capacity, stream); });
+    launch({&va, &vb}, where, [&](void *stream) { return fn(&a, &b, &z, cap_i, capacity, stream); });
     used(i, z.n_i), used(jp, (int64_t)z.n_i + 1), used(j, z.nnz), used(val, z.nnz);
     Result r(DCSR);
     r.set(N_i, i), r.set(N_jp, jp), r.set(N_j, j), r.set(N_values, val);
@@ -329,7 +354,7 @@ PyObject *coo3d_add(PyObject *const *args) {
     at::Tensor i = int_array(capacity, va.device), j = int_array(capacity, va.device), k = int_array(capacity, va.device), val = float_array(capacity, va.device);
     nb200_coo3 z{};
     z.i = ints(i), z.j = ints(j), z.k = ints(k), z.val = floats(val);
-    launch(va, where, [&](void *stream) { return nb200_coo3d_add_f32_into(&a, &b, &z, capacity, stream); });
+    launch({&va, &vb}, where, [&](void *stream) { return nb200_coo3d_add_f32_into(&a, &b, &z, capacity, stream); });
     used(i, z.nnz), used(j, z.nnz), used(k, z.nnz), used(val, z.nnz);
     Result r(COO3);
     r.set(N_i, i), r.set(N_j, j), r.set(N_k, k), r.set(N_values, val);
@@ -348,7 +373,7 @@ PyObject *csf_add(PyObject *const *args) {
     at::Tensor kp = int_array(cap_j + 1, va.device), k = int_array(cap_k, va.device), val = float_array(cap_k, va.device);
     nb200_csf3 z{};
     z.i_idx = ints(i), z.j_ptr = ints(jp), z.j_idx = ints(j), z.k_ptr = ints(kp), z.k_idx = ints(k), z.val = floats(val);
-    launch(va, where, [&](void *stream) { return nb200_csf_add_f32_into(&a, &b, &z, cap_i, cap_j, cap_k, stream); });
+    launch({&va, &vb}, where, [&](void *stream) { return nb200_csf_add_f32_into(&a, &b, &z, cap_i, cap_j, cap_k, stream); });
     used(i, z.n_i), used(jp, (int64_t)z.n_i + 1), used(j, z.n_j), used(kp, (int64_t)z.n_j + 1), used(k, z.n_k), used(val, z.n_k);
     Result r(CSF3);
     r.set(N_i, i), r.set(N_jp, jp), r.set(N_j, j), r.set(N_kp, kp), r.set(N_k, k), r.set(N_values, val);
@@ -363,7 +388,7 @@ PyObject *inner(Kind kind, const char *what, const char *where, PyObject *const 
     const S a = view(args[0], va), b = view(args[1], vb);
     same_device(va, vb);
     at::Tensor z = float_array(1, va.device);
-    launch(va, where, [&](void *stream) { return fn(&a, &b, floats(z), stream); });
+    launch({&va, &vb}, where, [&](void *stream) { return fn(&a, &b, floats(z), stream); });
     Result r(SCALAR);
     r.set(N_values, z);
     return r.obj.release();

@@ -1,0 +1,203 @@
+"""GPU suite: the sizes at which the merge tiles, the row classes and the routes of a call change, held to the
+CPU oracle. Merged values are one float32 addition or product, so everything there is compared bit for bit;
+sums of products are held to a bound in the magnitude that was summed."""
+import threading
+
+import numpy as np
+import pytest
+
+from helpers import assert_same, csf3_levels, csr_from_gpu, csr_to_gpu
+from oracle.cpu_oracle import COO3, CSF3, CSR, DCSR
+
+pytestmark = pytest.mark.gpu
+
+SMALL_STEP = 256 * 15 - 1  # entries of a CSR tile below LARGE_FROM entries
+LARGE_FROM = 6_000_000     # a tile holds 256 * 31 from here
+COO_STEP = 256 * 7 - 1     # entries of a coordinate tile below 3 M
+DIRECT_TILES = 128         # beyond it one CTA sums the tiles' lengths
+
+
+@pytest.fixture(scope="module")
+def nacho():
+    import torch
+    assert torch.cuda.is_available(), "GPU suite needs a CUDA device"
+    from nacho_b200 import nacho as mod
+    return mod
+
+
+def csr_of_keys(key, rows, cols, rng):
+    row = key // cols
+    val = rng.uniform(-1, 1, len(key)).astype(np.float32)
+    val[rng.random(len(key)) < 0.01] = -0.0
+    return CSR(rows, cols, np.searchsorted(row, np.arange(rows + 1)).astype(np.int32), (key % cols).astype(np.int32), val)
+
+
+def key_pair(total, space, shared, rng):
+    """Two sorted lists of distinct keys below `space`, exactly `total` keys together, `shared` of the second in both."""
+    n_a, n_b = total - total // 2, total // 2
+    both = int(n_b * shared)
+    n = total - both
+    every = np.cumsum(1 + rng.integers(0, max((space - n) // n, 1), n)) - 1
+    in_a = rng.permutation(n) < n_a
+    in_b = ~in_a
+    in_b[rng.permutation(np.flatnonzero(in_a))[:both]] = True
+    assert in_a.sum() + in_b.sum() == total and every[-1] < space
+    return every[in_a], every[in_b]
+
+
+EDGES = [1, SMALL_STEP - 1, SMALL_STEP, SMALL_STEP + 1, 2 * SMALL_STEP, 2 * SMALL_STEP + 1, DIRECT_TILES * SMALL_STEP,
+         DIRECT_TILES * SMALL_STEP + 1, (DIRECT_TILES + 1) * SMALL_STEP + 7]
+
+
+@pytest.mark.parametrize("shape", ["one row", "rows of an entry", "rows of ten", "wide rows", "equal operands"])
+@pytest.mark.parametrize("total", EDGES + [LARGE_FROM - 1, LARGE_FROM + 2])
+def test_csr_tiles(nacho, oracle, total, shape):
+    """Tiles of one entry more or less, more row starts than a tile keeps, columns too wide for keys of 32 bits,
+    and operands with equal columns only, so that twins fall on every share and tile boundary."""
+    rows, cols = {"one row": (1, 1 << 28), "rows of an entry": (total + 1, 300), "rows of ten": (total // 10 + 1, 4000),
+                  "wide rows": (1 << 12, (1 << 31) - 1), "equal operands": (total // 30 + 1, 1 << 16)}[shape]
+    rng = np.random.default_rng(total)
+    ka, kb = key_pair(total, rows * cols, 1.0 if shape == "equal operands" else 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+    c = csr_of_keys(np.union1d(ka[::2], kb[1::3]), rows, cols, rng)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, csr_to_gpu(c))), oracle.csr_add_3(a, b, c, 8), "add_3")
+
+
+@pytest.mark.parametrize("dims", [(3, 4, 1 << 28), (1 << 26, 9, 5), (1 << 20, 1 << 21, 1 << 22)])
+@pytest.mark.parametrize("total", [1, COO_STEP, COO_STEP + 1, DIRECT_TILES * COO_STEP + 1, 3_000_000, 4096 * (256 * 17 - 1) + 1])
+def test_coordinate_tiles(nacho, oracle, total, dims):
+    """Coordinates whose differences within a tile fit 32 bits, and such that do not; the cuts of few and of many tiles."""
+    from test_tensor3_gpu import coo3_from_gpu, coo3_to_gpu
+    space = min(dims[0] * dims[1] * dims[2], 1 << 62)
+    rng = np.random.default_rng(total)
+    ka, kb = key_pair(total, space, 0.3, rng)
+
+    def tensor(key):
+        ij, k = np.divmod(key, dims[2])
+        i, j = np.divmod(ij, dims[1])
+        return COO3(dims, i.astype(np.int32), j.astype(np.int32), k.astype(np.int32), rng.uniform(-1, 1, len(key)).astype(np.float32))
+
+    a, b = tensor(ka), tensor(kb)
+    ga, gb = coo3_to_gpu(nacho, a), coo3_to_gpu(nacho, b)
+    assert_same(coo3_from_gpu(nacho.gpu_coo3d_add_f32(ga, gb)), oracle.coo3_add(a, b, 8), "coo3 add")
+    _, at_a, at_b = np.intersect1d(ka, kb, assume_unique=True, return_indices=True)
+    terms = a.val[at_a].astype(np.float64) * b.val[at_b]
+    got = float(nacho.gpu_inner_prod_coo_f32(ga, gb).values.cpu()[0])
+    assert abs(got - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30  # float32 products, 2^-24 each, summed wider
+
+
+def test_stored_empty_rows_and_fibres(nacho, oracle):
+    """Row lists that hold rows without entries, and trees that hold slices and fibres without any, come out without them."""
+    from test_family_gpu import dcsr_from_gpu, dcsr_to_gpu
+    from test_tensor3_gpu import _seeded, csf3_from_gpu
+    import torch
+    rng = np.random.default_rng(7)
+    rows, cols = 5000, 800
+    ops = []
+    for _ in range(2):
+        stored = np.sort(rng.choice(rows, 3000, replace=False))
+        length = np.zeros(rows, np.int64)
+        length[stored] = rng.integers(0, 9, len(stored))
+        m = csr_of_keys(np.concatenate([r * cols + np.sort(rng.choice(cols, n, replace=False)) for r, n in enumerate(length)]).astype(np.int64), rows, cols, rng)
+        ops.append((m, DCSR(rows, cols, stored.astype(np.int32), np.append(m.row_ptr[stored], m.row_ptr[-1]).astype(np.int32), m.col, m.val)))
+    (a, da), (b, db) = ops
+    z = oracle.csr_add(a, b)
+    held = np.flatnonzero(np.diff(z.row_ptr)).astype(np.int32)
+    want = DCSR(rows, cols, held, np.append(z.row_ptr[held], z.row_ptr[-1]).astype(np.int32), z.col, z.val)
+    assert_same(dcsr_from_gpu(nacho.gpu_dcsr_add_f32(dcsr_to_gpu(nacho, da), dcsr_to_gpu(nacho, db))), want, "dcsr")
+
+    dims = (40, 50, 60)
+    (ca, va), (cb, vb) = _seeded(dims, 3000, 8)
+    fa, fb = CSF3(dims, *csf3_levels(ca), va), CSF3(dims, *csf3_levels(cb), vb)
+    j = np.setdiff1d(np.arange(dims[1]), fa.j_idx[:fa.j_ptr[1]])[:1]  # a fibre that slice 0 of A lacks, now stored without entries
+    at = int(np.searchsorted(fa.j_idx[:fa.j_ptr[1]], j[0]))
+    j_ptr = fa.j_ptr.copy()
+    j_ptr[1:] += 1
+    k_ptr = np.insert(fa.k_ptr, at, fa.k_ptr[at])
+    to = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    plain = nacho.to_csf3(ca, va, dims, "cuda")
+    hollow = type(plain)(to(fa.i_idx), to(j_ptr), to(np.insert(fa.j_idx, at, j[0]).astype(np.int32)), to(k_ptr.astype(np.int32)),
+                         to(fa.k_idx), to(fa.val), torch.tensor(dims, dtype=torch.int32))
+    gb = nacho.to_csf3(cb, vb, dims, "cuda")
+    assert_same(csf3_from_gpu(nacho.gpu_csf_add_f32(hollow, gb)), oracle.csf3_add(fa, fb), "csf3")
+
+
+@pytest.mark.parametrize("entries,length", [(1, 32), (4, 8), (6, 5), (8, 4), (9, 3), (4, 9), (1, 33), (3, 85), (2, 128), (1, 256), (64, 4), (300, 40)])
+def test_product_rows(nacho, oracle, entries, length):
+    """Rows of A of `entries` entries that select rows of B of `length`: up to 8 and 32 products in one pass, up to
+    256 sorted, more ranked; at the tile of 128 rows and beyond 128 such tiles."""
+    from test_spgemm_gpu import check
+    rng = np.random.default_rng(entries * 1000 + length)
+    inner, cols = 400, 5000
+    rows = 128 * DIRECT_TILES + 1 if entries * length <= 33 else 129
+    keys = lambda r, c, n: (np.arange(r)[:, None] * c + np.sort(np.argsort(rng.random((r, c)), axis=1)[:, :n], axis=1)).ravel()
+    a = csr_of_keys(keys(rows, inner, entries), rows, inner, rng)
+    b = csr_of_keys(keys(inner, cols, length), inner, cols, rng)
+    check(nacho, oracle, a, b)
+
+
+def test_many_ranked_rows(nacho, oracle):
+    """8192 rows of 300 products and more: their CTAs hold sums in shared memory, and some rows more than those hold."""
+    from test_spgemm_gpu import check
+    rng = np.random.default_rng(3)
+    rows, inner, cols = 8192 + 40, 600, 20000
+    keys = lambda r, c, n: np.unique(np.repeat(np.arange(r), n) * c + rng.integers(0, c, r * n))
+    length = np.full(inner, 110)
+    length[:20] = 3000
+    b_key = np.unique(np.concatenate([r * cols + rng.integers(0, cols, n) for r, n in enumerate(length)]))
+    check(nacho, oracle, csr_of_keys(keys(rows, inner, 5), rows, inner, rng), csr_of_keys(b_key, inner, cols, rng))
+
+
+@pytest.mark.parametrize("mask", [1, 31, 32, 33, 64, 65, 128, 129, 500])
+def test_masked_rows_looked_up(nacho, oracle, mask):
+    """Mask rows at the lengths where their look-up changes, under rows of A around its units of 8 entries."""
+    rng = np.random.default_rng(mask)
+    rows, inner, cols = 40, 3000, 100000
+    per_row = np.array([1, 7, 8, 9, 64, 65, 300, 0] * 5)
+    a = csr_of_keys(np.concatenate([r * inner + np.sort(rng.choice(inner, n, replace=False)) for r, n in enumerate(per_row)]).astype(np.int64), rows, inner, rng)
+    b = csr_of_keys(np.unique(rng.integers(0, inner * cols, inner * 400)), inner, cols, rng)
+    full, v64, abs64, _ = oracle.spgemm(a, b, 8, extras=True)
+    key = lambda m: np.repeat(np.arange(m.rows, dtype=np.int64), np.diff(m.row_ptr)) * m.cols + m.col
+    reached = [np.flatnonzero(key(full) // cols == r) for r in range(rows)]
+    picks = [key(full)[rng.permutation(q)[:mask - mask // 3]] for q in reached]
+    c = csr_of_keys(np.unique(np.concatenate(picks + [r * cols + rng.choice(cols, mask // 3, replace=False) for r in range(rows)])).astype(np.int64), rows, cols, rng)
+    z = csr_from_gpu(nacho.gpu_sssmm_f32(csr_to_gpu(a), csr_to_gpu(b), csr_to_gpu(c)))
+    common, i_f, i_c = np.intersect1d(key(full), key(c), return_indices=True)
+    assert np.array_equal(key(z), common)
+    bound = 1e-5 * abs64[i_f] * np.abs(c.val[i_c]) + 1e-30
+    assert np.all(np.abs(z.val.astype(np.float64) - v64[i_f] * c.val[i_c].astype(np.float64)) <= bound)
+
+
+def test_threads_share_a_stream(nacho, oracle):
+    """Calls of several host threads on one stream, and on streams of their own with operands of another, as if alone."""
+    import torch
+    rng = np.random.default_rng(11)
+    jobs = []
+    for total in (200, 4000, 50_000, 700_000):
+        ka, kb = key_pair(total, 3000 * 5000, 0.3, rng)
+        a, b = csr_of_keys(ka, 3000, 5000, rng), csr_of_keys(kb, 3000, 5000, rng)
+        jobs.append((csr_to_gpu(a), csr_to_gpu(b), oracle.csr_add(a, b, 8), oracle.csr_mul(a, b, 8)))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(job, stream):
+        ga, gb, add, mul = job
+        try:
+            with torch.cuda.stream(stream):
+                for _ in range(20):
+                    z, p = nacho.gpu_csr_add_f32(ga, gb), nacho.gpu_csr_mul_f32(ga, gb)
+                    assert_same(csr_from_gpu(z), add, "add")
+                    assert_same(csr_from_gpu(p), mul, "mul")
+        except BaseException as e:  # reported by the main thread
+            wrong.append(e)
+
+    for streams in ([torch.cuda.current_stream()] * 4, [torch.cuda.Stream() for _ in range(4)]):
+        threads = [threading.Thread(target=work, args=(j, s)) for j, s in zip(jobs, streams)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong, wrong[0]
