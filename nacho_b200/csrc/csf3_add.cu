@@ -274,7 +274,7 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
 //      CSR union writes Z's k_ptr, k_idx and val.
 // Steps 2 and 3 read their row count from device memory.
 
-// Measured against the expanded route: 25 M entries per operand in fibres of 7, 558 us against 821; 5 M in
+// Measured against the expanded route: 25 M entries per operand in fibres of 7, 445 us against 821; 5 M in
 // fibres of 4, 230 against 258; 5000 in fibres of 1.1, 54 against 66. So it is taken wherever it applies.
 bool levels_pay(const nb200_csf3 *a, const nb200_csf3 *b) {
     if (a->n_j == 0 || b->n_j == 0) return false;
@@ -311,7 +311,7 @@ int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cuda
     if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{0, &ctl[0]->total}, a->dims[1],
                            CsrOut{z->j_ptr, z->j_idx, nullptr, nullptr, word[1], ctl[0]}, &fibres, scratch_j, stream, &ctl[1])))
         return st;
-    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total}, a->dims[2],
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total, true}, a->dims[2],
                            CsrOut{z->k_ptr, z->k_idx, z->val, nullptr, word[2], ctl[1]}, nullptr, scratch_k, stream, &ctl[2])))
         return st;
     int64_t length[3];

@@ -139,8 +139,8 @@ struct TilePlan {
     static constexpr int CAP = NT * VT;         // most merged entries of one tile
     static constexpr int SLOTS = CAP + 16;      // + alignment words of both operands and their sentinels
     // Row starts kept in shared memory; tiles with more rows search the offsets in global memory. The most of which four CTAs
-    // fit an SM; the small tile has room for a row per entry.
-    static constexpr int ROWS = VT > 15 ? 1856 : 4096;
+    // fit an SM; the small tile and that for fibres have room for a row per entry.
+    static constexpr int ROWS = VT > 21 ? 1856 : VT > 15 ? CAP : 4096;
     static constexpr size_t ROWS_AT = (LEVELS ? 8 : 6) * (size_t)SLOTS;
     static constexpr size_t BYTES = ROWS_AT + 4 * (size_t)(ROWS + 2);
     static_assert(VT <= 31, "a thread's twins are kept in the lower 31 bits of a word");
@@ -222,6 +222,10 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             prefetch_l2(ga_val, na);
             prefetch_l2(gb_val, nb);
         }
+        if (!rows_fit) {  // read three times
+            if (A.rp) prefetch_l2(A.rp + tile.i0 + 1, nr);
+            if (B.rp) prefetch_l2(B.rp + tile.i0 + 1, nr);
+        }
     }
     if (tid >= 32 && tid < 32 + 12) {  // ragged ends: 3 head + 3 tail slots for A, then for B
         const int k = tid - 32;
@@ -241,9 +245,27 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     auto global_start = [&](int r) -> uint32_t {
         return (uint32_t)(row_offset(A, (int64_t)tile.i0 + r) - tile.a0) | (uint32_t)(row_offset(B, (int64_t)tile.i0 + r) - tile.b0) << 16;
     };
-    if (rows_fit) {
-        for (int r = tid; r <= nr; r += NT) s_rows[r] = r == 0 ? 0u : global_start(r);
-        if (tid == 0) s_rows[nr + 1] = (uint32_t)na | (uint32_t)nb << 16;
+    constexpr int RB = 4;  // rows a thread fetches together
+    if (nr <= NT) {
+        if (tid < nr) s_rows[1 + tid] = global_start(1 + tid);
+    } else if (rows_fit) {
+        for (int r0 = 1; r0 <= nr; r0 += RB * NT) {
+            uint32_t w[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+                const int r = r0 + u * NT + tid;
+                w[u] = r <= nr ? global_start(r) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+                const int r = r0 + u * NT + tid;
+                if (r <= nr) s_rows[r] = w[u];
+            }
+        }
+    }
+    if (rows_fit && tid == 0) {
+        s_rows[0] = 0u;
+        s_rows[nr + 1] = (uint32_t)na | (uint32_t)nb << 16;
     }
     auto row_start = [&](int r) -> uint32_t {  // packed like s_rows, r in [0, nr + 1]
         if (rows_fit) return s_rows[r];
@@ -267,8 +289,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     // ---- every row that begins in the tile adds one above the column bits of its first entry (several
     // where empty rows share a start), and the last row that starts at or before a thread's diagonal is
     // noted for that thread, and for its warp
-    for (int r = 1 + tid; r <= nr; r += NT) {
-        const uint32_t w = row_start(r), w_next = row_start(r + 1);
+    auto begin_row = [&](const int r, const uint32_t w, const uint32_t w_next) {
         const int sa = (int)(w & 0xffffu), sb = (int)(w >> 16);
         if (!WIDE) {
             if (sa < na) atomicAdd(keys + oa + sa, 1u << cbits);
@@ -283,6 +304,11 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             s_trow[q] = r;
             if ((q_next >> 5) != (q >> 5)) s_wrow[q >> 5] = r;
         }
+    };
+    if (rows_fit) {
+        for (int r = 1 + tid; r <= nr; r += NT) begin_row(r, s_rows[r], s_rows[r + 1]);
+    } else {
+        for (int r = 1 + tid; r <= nr; r += NT) begin_row(r, global_start(r), row_start(r + 1));
     }
     __syncthreads();
 
@@ -430,11 +456,13 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     // ---- compact: source of every result entry, in order. A twin's A word now points to its B word
     // (byte offsets: step i began at pa0 + pb0 + 4 (i + twins before it)).
     if (!LEVELS && __any_sync(FULL_MASK, twin != 0u)) {
+        uint32_t begun = pa0 + pb0;  // where step i began, less 4 i
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) {
-                word_at(src[i]) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - src[i];
+                word_at(src[i]) = begun + 4u * (uint32_t)i - src[i];
                 src[i] |= 0x8000u;
+                begun += 4u;
             }
     }
     {
@@ -543,25 +571,31 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     // entries: all of them up to the thread that holds position d, then, in that thread, a step per entry
     // except that a twin step covers two. The tile owns rows i0+1 .. i1 (the next tile's first row).
     if (LEVELS && !Z.rp) return;
-    for (int r = 1 + tid; r <= nr; r += NT) {
-        const uint32_t w = row_start(r);
+    auto end_row = [&](const int r, const uint32_t w) {
         const int d = (int)((w & 0xffffu) + (w >> 16));
         const int owner = d / VT;
         int before = total;
         if (owner < NT) {
             const unsigned info = s_twin[owner];
             const int m = d - owner * VT - (int)(info >> 31);  // merged entries of that thread before the row
-            unsigned left = info & 0x7fffffffu;
-            int pairs = 0;  // twins among them
-            while (left) {
-                const int at = __ffs(left) - 1;
-                if (at + pairs + 2 > m) break;
-                ++pairs;
-                left &= left - 1u;
+            const unsigned twins = info & 0x7fffffffu;
+            int steps_before = m;
+            if (twins) {  // the steps that take m entries: s + (twins among the first s) grows with s
+                int lo = m >> 1, hi = m;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (mid + __popc(twins & ((1u << mid) - 1u)) >= m) hi = mid; else lo = mid + 1;
+                }
+                steps_before = lo;
             }
-            before = s_rank[owner] + (OP == OP_UNION ? m - pairs : pairs);
+            before = s_rank[owner] + (OP == OP_UNION ? steps_before : m - steps_before);
         }
         Z.rp[tile.i0 + (int64_t)r] = (int32_t)(base + before);
+    };
+    if (rows_fit) {
+        for (int r = 1 + tid; r <= nr; r += NT) end_row(r, s_rows[r]);
+    } else {
+        for (int r = 1 + tid; r <= nr; r += NT) end_row(r, global_start(r));
     }
     if (t == 0 && tid == 0) Z.rp[0] = 0;
 }
@@ -946,6 +980,11 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
 
 // In the offsets mode a tile needs 8 bytes of shared memory per entry, so its large tile is smaller.
 constexpr int V_LEVELS = 23;
+// Large tile where the caller says that many rows hold an entry or two (the fibres of a tree): a tile of 31 with more
+// rows than fit takes twice the time of the others and holds up their output bases. 25 M entries per operand in 6 M
+// fibres take 450 us with 17, 443 with 21, 463 with 23, 484 with 31. The stored rows of a doubly compressed
+// matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
+constexpr int V_FIBRES = 21;
 
 }  // namespace
 
@@ -960,7 +999,7 @@ size_t csr2_scratch_bytes(int64_t entries) {
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl_out) {
     const int64_t total = (int64_t)A.nnz + B.nnz;
-    const int v = tile_v(total) == V_LARGE ? (levels ? V_LEVELS : V_LARGE) : V_SMALL, step = tile_step(v);
+    const int v = tile_v(total) == V_SMALL ? V_SMALL : levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE, step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
     Carver carve(scratch);
     Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
@@ -981,6 +1020,9 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
         LaunchScope scope("csr_levels_fused", stream);
         e = v == V_LEVELS ? launch_tile_v<V_LEVELS, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels)
                           : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels);
+    } else if (v == V_FIBRES) {
+        LaunchScope scope("csr_add_fused", stream);
+        e = launch_tile_v<V_FIBRES, OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs());
     } else if (op == OP_UNION) {
         e = launch_tile<OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream);
     } else {
