@@ -1,8 +1,8 @@
 // Thin wrappers over the sm_90+/sm_100a asynchronous-copy PTX used by the tile kernels:
-// one-dimensional bulk copies between global and shared memory (the TMA engine's untiled
-// form, cp.async.bulk), the shared-memory mbarrier they complete on, and the proxy fence that
-// orders ordinary shared-memory writes before an engine read. No multicast form is used
-// anywhere: every copy has exactly one destination CTA, the one that issued it.
+// one-dimensional bulk copies from global to shared memory (the TMA engine's untiled form,
+// cp.async.bulk), the shared-memory mbarrier they complete on, and prefetches into L2. No
+// multicast form is used anywhere: every copy has exactly one destination CTA, the one that
+// issued it.
 //
 // Both addresses of a bulk copy must be 16-byte aligned and the size a multiple of 16 bytes.
 #pragma once
@@ -65,21 +65,5 @@ __device__ __forceinline__ void prefetch_l2(const void *p, int count) {
     if (to > from)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"((uint32_t)(to - from)) : "memory");
 }
-
-// shared -> global, tracked by the issuing thread's bulk group.
-__device__ __forceinline__ void bulk_store(void *gmem_dst, const void *smem_src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)),
-                 "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-
-// Blocks the issuing thread until the engine has finished READING shared memory for all of
-// its committed bulk stores (the data may still be on its way to global memory).
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-
-// Orders this thread's earlier ordinary shared-memory writes before later copy-engine reads.
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 }  // namespace nb200
