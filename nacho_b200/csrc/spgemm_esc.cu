@@ -596,6 +596,7 @@ __device__ __forceinline__ void walk_segments(const Segments<NT> &seg, const Csr
 
 constexpr int RK_WORDS = 8192;                     // bitmap words of one column window in shared memory
 constexpr int RK_WINDOW_COLS = RK_WORDS * 32;      // 262144 columns per window
+constexpr size_t RK_WORD_BYTES = 6;                // shared memory per bitmap word of a numeric launch: the word and its rank
 constexpr size_t RK_PTR_BUDGET = size_t(1) << 30;  // bytes of the window pointer table; beyond it windows are searched on the fly
 constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a CTA for rows up to / above RANKED_P products
 constexpr size_t HEAVY_SMEM_NUMERIC = 104 * 1024;  // dynamic shared memory of a numeric heavy-row CTA: two per SM
@@ -636,8 +637,11 @@ __global__ void __launch_bounds__(256) k_esc_window_ptr(CsrView B, int32_t b_row
 // with coalesced writes at the end, the positions beyond them take a float32 reduction in L2 on
 // the row's own output range, which this CTA zeroed first. Symbolic: pass 1 and the count only.
 //
-// Ranks are kept per 64 columns, in 16 bits relative to the first word of the warp that scanned
-// them (a warp scans `1 << wshift` consecutive words, at most 32768 columns), plus one base per warp.
+// Ranks are kept in 16 bits per bitmap word. Positions fit them in rows of at most 65535 products and in windows of at
+// most 65536 columns; otherwise (FAR) a rank counts from the first word of the warp that scanned it (a warp scans
+// `1 << wshift` consecutive words, at most 32768 columns), and there is one base per warp. The walk of pass 2 is bound
+// by the instructions it issues per product, so a look-up is two loads and a popcount of one word (a rank per 64
+// columns and a base per warp for every row took three loads and twice the instructions).
 //
 // `row_list` is read from the front for the first n_front CTAs and from the back (list_len - 1
 // downwards) for the others. `words`: bitmap words in use, (NT / 32) << wshift, covering a window.
@@ -645,7 +649,7 @@ __global__ void __launch_bounds__(256) k_esc_window_ptr(CsrView B, int32_t b_row
 // `cache` (one window only), when given, carries the bitmaps from the symbolic launch to the
 // numeric launch of one call, `words` per CTA: the symbolic launch stores them, the numeric
 // launch loads them instead of walking the products a first time.
-template <bool NUMERIC, int NT>
+template <bool NUMERIC, int NT, bool FAR>
 __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const int32_t *__restrict__ win_ptr, int n_win,
                                                    const int32_t *__restrict__ row_list, int32_t list_len, int n_front, int words,
                                                    int wshift, int acc_slots, uint32_t *cache, int32_t *__restrict__ row_count,
@@ -654,8 +658,8 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
     extern __shared__ __align__(16) unsigned char rk_smem[];
     uint32_t *bitmap = reinterpret_cast<uint32_t *>(rk_smem);
     const uint64_t *bitmap64 = reinterpret_cast<const uint64_t *>(rk_smem);  // the same bits, 64 columns per element
-    uint16_t *rank16 = reinterpret_cast<uint16_t *>(rk_smem + (size_t)words * 4);  // one rank per 64 columns
-    float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * 5);
+    uint16_t *rank16 = reinterpret_cast<uint16_t *>(rk_smem + (size_t)words * 4);  // one rank per 32 columns
+    float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * RK_WORD_BYTES);
     __shared__ Segments<NT> seg;
     __shared__ int scan_tmp[72];
     __shared__ int warp_base[NT / 32];
@@ -745,7 +749,7 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
             continue;
         }
         const int my_base = __shfl_sync(FULL_MASK, excl, 0);  // columns of the window before this warp's words
-        if (lane_id() == 0) warp_base[warp_id()] = my_base;
+        if (FAR && lane_id() == 0) warp_base[warp_id()] = my_base;
         int running = 0;
 #pragma unroll 2
         for (int g = 0; g < groups; ++g) {
@@ -754,7 +758,8 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
             const int c = __popcll(bits);
             const int incl = warp_incl_sum(c);
             const int first = running + incl - c;
-            rank16[idx] = (uint16_t)first;
+            const uint32_t rank = (uint32_t)(FAR ? first : my_base + first);
+            reinterpret_cast<uint32_t *>(rank16)[idx] = (rank & 0xffffu) | (rank + __popc((uint32_t)bits)) << 16;
             // the lane's columns, in 32-bit halves and 32-bit positions (the loop is the hot part of
             // the scan: one trip per result entry)
             int32_t *gcol = c_col + (out + my_base);
@@ -780,13 +785,14 @@ __global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const i
         __syncthreads();  // ranks complete, output zeroed (the reductions below come from this CTA only)
         pass(!one_chunk || from_cache, [&](int32_t col, float v) {
             const uint32_t cw = (uint32_t)(col - c_first);
-            const uint32_t dw = cw >> 6;
-            const uint64_t bits = bitmap64[dw];
-            const uint32_t pos = (uint32_t)warp_base[dw >> (wshift - 1)] + rank16[dw] + __popcll(bits & ((1ull << (cw & 63u)) - 1ull));
-            if (pos < (uint32_t)acc_slots)
-                atomicAdd(acc + pos, v);      // shared memory
+            const uint32_t word = cw >> 5;
+            // columns of the word up to and with this one, whose bit is set: the position plus one
+            uint32_t next = (uint32_t)rank16[word] + __popc(bitmap[word] << (~cw & 31u));
+            if (FAR) next += (uint32_t)warp_base[word >> wshift];
+            if (next <= (uint32_t)acc_slots)
+                atomicAdd(acc - 1 + next, v);      // shared memory
             else
-                atomicAdd(row_val + pos, v);  // reduction in L2
+                atomicAdd(row_val - 1 + next, v);  // reduction in L2
         });
         // the pass ends with a barrier: every sum is in place
         for (int k = tid; k < in_acc; k += NT) row_val[k] = acc[k];
@@ -1063,14 +1069,16 @@ int launch_ranked(const CsrView &A, const CsrView &B, const EscPlan &plan, int32
     // vertices 111 against 117 us, of 9000 vertices 198 against 209); tens of thousands are bound by the
     // reductions that go to L2 instead (24405 vertices 434 -> 430 us, 65536 vertices 2579 -> 2436).
     const size_t rows_budget = NT == HEAVY_NT ? HEAVY_SMEM_NUMERIC : n_rows >= RK_MANY_ROWS ? RK_SMEM_NUMERIC : 0;
-    const size_t budget = std::max(rows_budget, (size_t)words * 5);
-    const int acc_slots = NUMERIC ? (int)((budget - (size_t)words * 5) / 4 / NT) * NT : 0;
-    const size_t smem = NUMERIC ? (size_t)words * 5 + (size_t)acc_slots * 4 : (size_t)words * 4;
+    const size_t table = (size_t)words * RK_WORD_BYTES;
+    const int acc_slots = NUMERIC ? (int)((std::max(rows_budget, table) - table) / 4 / NT) * NT : 0;
+    const size_t smem = NUMERIC ? table + (size_t)acc_slots * 4 : (size_t)words * 4;
+    const bool far = NUMERIC && NT == HEAVY_NT && words * 32 > 65536;
+    auto kernel = far ? k_esc_ranked<NUMERIC, NT, NUMERIC && NT == HEAVY_NT> : k_esc_ranked<NUMERIC, NT, false>;
     // the most that any call asks for: several threads may be here with different sizes
-    NB200_CUDA(cudaFuncSetAttribute(k_esc_ranked<NUMERIC, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(NUMERIC ? std::max(HEAVY_SMEM_NUMERIC, (size_t)RK_WORDS * 5) : (size_t)RK_WORDS * 4)));
-    return launch_bin(beside, k_esc_ranked<NUMERIC, NT>, n_rows, NT, smem, stream, A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift,
-                      acc_slots, cache, count, c_rp, c_col, c_val);
+    NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(NUMERIC ? std::max(HEAVY_SMEM_NUMERIC, RK_WORDS * RK_WORD_BYTES) : (size_t)RK_WORDS * 4)));
+    return launch_bin(beside, kernel, n_rows, NT, smem, stream, A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift, acc_slots, cache,
+                      count, c_rp, c_col, c_val);
 }
 
 template <bool NUMERIC>

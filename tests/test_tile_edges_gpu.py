@@ -151,6 +151,17 @@ def test_many_ranked_rows(nacho, oracle):
     check(nacho, oracle, csr_of_keys(keys(rows, inner, 5), rows, inner, rng), csr_of_keys(b_key, inner, cols, rng))
 
 
+@pytest.mark.parametrize("cols", [65535, 65536, 65537])
+def test_full_heavy_row(nacho, oracle, cols):
+    """A row of more than 65535 products that reaches every column, at the width up to which positions fit 16 bits."""
+    from test_spgemm_gpu import check
+    rng = np.random.default_rng(cols)
+    every = np.arange(cols)
+    b_key = np.unique(np.concatenate([(every % 40) * cols + every, rng.integers(0, 40 * cols, 30000)]))  # 40 rows that cover all columns
+    a_key = np.concatenate([np.arange(40), [40 + 3, 40 + 7], 80 + np.arange(40)])
+    check(nacho, oracle, csr_of_keys(a_key, 3, 40, rng), csr_of_keys(b_key, 40, cols, rng))
+
+
 @pytest.mark.parametrize("mask", [1, 31, 32, 33, 64, 65, 128, 129, 500])
 def test_masked_rows_looked_up(nacho, oracle, mask):
     """Mask rows at the lengths where their look-up changes, under rows of A around its units of 8 entries."""
