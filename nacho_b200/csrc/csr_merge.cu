@@ -130,6 +130,12 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
 // ------------------------------------------------------------------------ tile kernel ----
 
 
+// Large tile where the caller says that many rows hold an entry or two (the fibres of a tree): a tile of 31 with more
+// rows than fit takes twice the time of the others and holds up their output bases. 25 M entries per operand in 6 M
+// fibres take 450 us with 17, 443 with 21, 463 with 23, 484 with 31. The stored rows of a doubly compressed
+// matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
+constexpr int V_FIBRES = 21;
+
 // Shared-memory plan of the tile body. The column words of both operands lie in one array: A's entry e at
 // word oa + e, B's at word ob + e, where oa and ob are chosen so that a global address on a 16-byte
 // boundary lands on a 16-byte boundary in shared memory too (what a bulk copy needs). Behind them, one
@@ -187,6 +193,9 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     constexpr int W = NT / 32;
     constexpr Key END = WIDE ? (Key)~0ull : (Key)0x80000000u;  // after every key (narrow: keys are below 2^31), also with row bits added
     constexpr bool WRITES = MODE != MODE_COUNT;
+    // Rows of an entry or two: a mask by entries instead of steps spares every row offset a search of it (25 M entries per
+    // operand in 6 M rows: 440 -> 432 us). With fewer rows the mask costs more than the searches (67 M entries 1 %).
+    constexpr bool MANY_ROWS = VT == V_FIBRES;
     uint32_t *s_rows = reinterpret_cast<uint32_t *>(smem_raw + P::ROWS_AT);  // start of row r in the tile: A's in the lower half, B's in the upper
     int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.trow, *s_wtotal = sh.wtotal;
     unsigned *s_twin = sh.twin;
@@ -424,7 +433,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     const int mine = OP == OP_UNION ? steps : __popc(twin);
     const int incl = warp_incl_sum(mine);
     if (lane == 31) s_wtotal[wid] = incl;
-    s_twin[tid] = twin | (unsigned)shifted << 31;
+    if (!MANY_ROWS) s_twin[tid] = twin | (unsigned)shifted << 31;  // bit i: step i took an entry of each operand
     __syncthreads();  // also retires the merge of every thread: words of consumed twins may change from here on
     int total = 0, wbase = 0;
 #pragma unroll
@@ -464,6 +473,12 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
                 src[i] |= 0x8000u;
                 begun += 4u;
             }
+    }
+    if (MANY_ROWS) {
+        // The row offsets ask how many of a thread's first m entries are a twin's second: bit e for its entry e
+        unsigned second = 0;
+        for (unsigned left = twin << 1; left; left = (left & (left - 1u)) << 1) second |= left & (0u - left);
+        s_twin[tid] = (second & 0x7fffffffu) | (unsigned)shifted << 31;
     }
     {
         Src *to = src_of + rank;
@@ -577,18 +592,20 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
         int before = total;
         if (owner < NT) {
             const unsigned info = s_twin[owner];
-            const int m = d - owner * VT - (int)(info >> 31);  // merged entries of that thread before the row
-            const unsigned twins = info & 0x7fffffffu;
-            int steps_before = m;
-            if (twins) {  // the steps that take m entries: s + (twins among the first s) grows with s
+            const int m = d - owner * VT - (int)(info >> 31);  // merged entries of that thread before the row, fewer than VT
+            int twins;
+            if (MANY_ROWS) {
+                twins = __popc(info & ((1u << m) - 1u));  // no row begins between a twin's two
+            } else {  // the steps that take m entries: s + (twins among the first s) grows with s
                 int lo = m >> 1, hi = m;
+                if ((info << 1) == 0u) lo = m;
                 while (lo < hi) {
                     const int mid = (lo + hi) >> 1;
-                    if (mid + __popc(twins & ((1u << mid) - 1u)) >= m) hi = mid; else lo = mid + 1;
+                    if (mid + __popc(info & ((1u << mid) - 1u)) >= m) hi = mid; else lo = mid + 1;
                 }
-                steps_before = lo;
+                twins = m - lo;
             }
-            before = s_rank[owner] + (OP == OP_UNION ? steps_before : m - steps_before);
+            before = s_rank[owner] + (OP == OP_UNION ? m - twins : twins);
         }
         Z.rp[tile.i0 + (int64_t)r] = (int32_t)(base + before);
     };
@@ -980,11 +997,6 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
 
 // In the offsets mode a tile needs 8 bytes of shared memory per entry, so its large tile is smaller.
 constexpr int V_LEVELS = 23;
-// Large tile where the caller says that many rows hold an entry or two (the fibres of a tree): a tile of 31 with more
-// rows than fit takes twice the time of the others and holds up their output bases. 25 M entries per operand in 6 M
-// fibres take 450 us with 17, 443 with 21, 463 with 23, 484 with 31. The stored rows of a doubly compressed
-// matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
-constexpr int V_FIBRES = 21;
 
 }  // namespace
 
