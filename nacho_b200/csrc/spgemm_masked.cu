@@ -5,8 +5,8 @@
 // that survive the three-way intersection.
 //
 // Here the mask drives the accumulation, so nothing outside it is ever formed, sorted or written:
-//   k_sssmm_classify    one warp per row: how many products does the row have, and how wide (first to
-//                       last column) and how long is its mask row? The row goes on one of six lists.
+//   k_sssmm_classify    how many products does a row have, and how wide (first to last column) and
+//                       how long is its mask row? The row goes on one of six lists.
 //   k_sssmm_bitmap      rows with many products, one CTA per row taken from a ticket: the mask row
 //                       becomes a bitmap over its column span in shared memory plus, per 64-bit
 //                       word, the count of set bits before it. A product tests one bit; a hit finds
@@ -59,6 +59,11 @@ constexpr WorkClass CLASS[4] = {
     {0, 0, SEARCH_NT},    // wider still: no bitmap, binary search
 };
 
+// Entries of A's row in a unit of a list (LIST_LIGHT has whole rows).
+__device__ __forceinline__ int unit_of(int list) {
+    return list == LIST_MASK ? MASK_UNIT : list == 0 ? CLASS[0].unit() : list == LIST_WIDE ? CLASS[LIST_WIDE].unit() : CLASS[1].unit();
+}
+
 struct CsrView {
     const int32_t *rp, *col;
     const float *val;
@@ -69,48 +74,119 @@ struct SssmmCtl {
     int ticket[8];  // next list position to hand out
 };
 
+// Rows of one CTA of the classification. A warp has the dependent loads of eight rows (A's columns, then B's offsets)
+// in flight together, rows of more than LONG_ROW entries are left to the whole CTA, and a list's length is
+// advanced once per CTA: with a warp per row, one row after the other, the chains of loads and 50021 atomics on
+// six words took 39 us on a graph of 50021 vertices. A CTA's rows lie far apart: the hubs of a graph are often
+// neighbours.
+constexpr int ROWS_PER_WARP = 8, ROWS_PER_CTA = 8 * ROWS_PER_WARP, LONG_ROW = 128;
+
 __global__ void __launch_bounds__(256) k_sssmm_classify(CsrView A, CsrView B, CsrView C, int32_t rows, int64_t list_cap,
                                                        int2 *__restrict__ units, int32_t *__restrict__ light,
                                                        SssmmCtl *__restrict__ ctl) {
+    __shared__ int s_lo[ROWS_PER_CTA], s_hi[ROWS_PER_CTA], s_list[ROWS_PER_CTA], s_units[ROWS_PER_CTA], s_at[ROWS_PER_CTA];
+    __shared__ float s_products[ROWS_PER_CTA];
+    __shared__ int s_long[ROWS_PER_CTA], s_n_long, s_count[LIST_MASK + 1];
     trigger_dependents();
-    const int lane = lane_id();
-    const int64_t warps = (int64_t)gridDim.x * (256 / 32);
-    for (int64_t i = (int64_t)blockIdx.x * (256 / 32) + warp_id(); i < rows; i += warps) {
-        const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
-        const int32_t a_lo = ld_nc(A.rp + i), a_hi = ld_nc(A.rp + i + 1);
-        if (c_lo == c_hi || a_lo == a_hi) continue;
-        float mine = 0.f;  // rounding does not matter: the count only chooses a list
-        for (int32_t p = a_lo + lane; p < a_hi; p += 32) {
+    const int tid = threadIdx.x, lane = lane_id(), first = warp_id() * ROWS_PER_WARP;
+    auto row_of = [&](int r) -> int64_t { return (int64_t)r * gridDim.x + blockIdx.x; };  // neighbouring rows in different CTAs
+    if (tid <= LIST_MASK) s_count[tid] = 0;
+    if (tid == 0) s_n_long = 0;
+    __syncthreads();
+    {
+        int32_t lo = 0, hi = 0;  // lane r: A's entries of the warp's row r; none where the mask has none
+        if (lane < ROWS_PER_WARP && row_of(first + lane) < rows) {
+            const int64_t i = row_of(first + lane);
+            lo = ld_nc(A.rp + i);
+            hi = ld_nc(C.rp + i) == ld_nc(C.rp + i + 1) ? lo : ld_nc(A.rp + i + 1);
+        }
+        const bool is_long = hi - lo > LONG_ROW;
+        if (lane < ROWS_PER_WARP) {
+            s_lo[first + lane] = lo;
+            s_hi[first + lane] = hi;
+            s_products[first + lane] = 0.f;
+            if (is_long) s_long[atomicAdd(&s_n_long, 1)] = first + lane;
+        }
+        const int len = is_long ? 0 : hi - lo;
+        const int most = __reduce_max_sync(FULL_MASK, (unsigned)len);
+        float mine[ROWS_PER_WARP] = {};  // rounding does not matter: the counts only choose a list
+        for (int p = lane; p - lane < most; p += 32) {
+            int32_t j[ROWS_PER_WARP];
+#pragma unroll
+            for (int r = 0; r < ROWS_PER_WARP; ++r) {
+                const int n = __shfl_sync(FULL_MASK, len, r), from = __shfl_sync(FULL_MASK, lo, r);
+                j[r] = p < n ? ld_nc(A.col + from + p) : -1;
+            }
+#pragma unroll
+            for (int r = 0; r < ROWS_PER_WARP; ++r)
+                if (j[r] >= 0) mine[r] += (float)(ld_nc(B.rp + j[r] + 1) - ld_nc(B.rp + j[r]));
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS_PER_WARP; ++r) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mine[r] += __shfl_xor_sync(FULL_MASK, mine[r], o);
+            if (lane == r && !is_long) s_products[first + r] = mine[r];
+        }
+    }
+    __syncthreads();
+    for (int l = 0; l < s_n_long; ++l) {
+        const int row = s_long[l];
+        float mine = 0.f;
+#pragma unroll 4
+        for (int32_t p = s_lo[row] + tid; p < s_hi[row]; p += 256) {
             const int32_t j = ld_nc(A.col + p);
             mine += (float)(ld_nc(B.rp + j + 1) - ld_nc(B.rp + j));
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-        const float products = mine;
-        if (products == 0.f) continue;
-        if (products < (float)LIGHT_P) {
-            if (lane == 0) light[atomicAdd(&ctl->count[LIST_LIGHT], 1)] = (int32_t)i;
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(FULL_MASK, mine, o);
+        if (lane == 0) atomicAdd(s_products + row, mine);
+    }
+    __syncthreads();
+    if (tid < ROWS_PER_CTA) {
+        const float products = s_products[tid];
+        const int32_t a_lo = s_lo[tid], a_hi = s_hi[tid];
+        int list = -1, n_units = 0, at = 0;
+        if (products > 0.f && products < (float)LIGHT_P) {
+            list = LIST_LIGHT;
+            n_units = 1;
+        } else if (products > 0.f) {
+            const int64_t i = row_of(tid);
+            const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
+            const int32_t words = (ld_nc(C.col + c_hi - 1) >> 6) - (ld_nc(C.col + c_lo) >> 6) + 1, entries = c_hi - c_lo;
+            // Warp instructions of the two ways, roughly: looking the mask row up in every selected row of B costs
+            // 150 per entry and 32 mask positions; walking the products costs 4000 for the bitmap of the mask row,
+            // 200 per entry and 0.7 per product. R-MAT rows of a few dozen entries are an order of magnitude cheaper
+            // to look up, hub rows are not. (50021 vertices, 800003 edges: 506 us with 150, 534 with 300, 693 without
+            // the look-up.)
+            const float entries_a = (float)(a_hi - a_lo);
+            const bool by_mask = 150.f * entries_a * (float)((entries + 31) / 32) <= 4000.f + 200.f * entries_a + 0.7f * products;
+            list = LIST_WIDE;
+            if (by_mask) list = LIST_MASK;
+            else if (words <= CLASS[0].words && entries <= CLASS[0].entries) list = 0;
+            else if (words <= CLASS[1].words && entries <= CLASS[1].entries) list = 1;
+            else if (words <= CLASS[2].words) list = 2;
+            n_units = (a_hi - a_lo + unit_of(list) - 1) / unit_of(list);
+        }
+        if (list >= 0) at = atomicAdd(&s_count[list], n_units);
+        s_list[tid] = list;
+        s_units[tid] = n_units;
+        s_at[tid] = at;
+    }
+    __syncthreads();
+    if (tid <= LIST_MASK && s_count[tid] > 0) s_count[tid] = atomicAdd(&ctl->count[tid], s_count[tid]);  // from here on: where the CTA's units begin
+    __syncthreads();
+#pragma unroll
+    for (int r = first; r < first + ROWS_PER_WARP; ++r) {
+        const int list = s_list[r], n_units = s_units[r];
+        if (list < 0) continue;
+        const int64_t at = s_count[list] + s_at[r];
+        if (list == LIST_LIGHT) {
+            if (lane == 0) light[at] = (int32_t)row_of(r);
             continue;
         }
-        const int32_t words = (ld_nc(C.col + c_hi - 1) >> 6) - (ld_nc(C.col + c_lo) >> 6) + 1, entries = c_hi - c_lo;
-        // Warp instructions of the two ways, roughly: looking the mask row up in every selected row of B costs
-        // 150 per entry and 32 mask positions; walking the products costs 4000 for the bitmap of the mask row,
-        // 200 per entry and 0.7 per product. R-MAT rows of a few dozen entries are an order of magnitude cheaper
-        // to look up, hub rows are not. (50021 vertices, 800003 edges: 506 us with 150, 534 with 300, 693 without
-        // the look-up.)
-        const float entries_a = (float)(a_hi - a_lo);
-        const bool by_mask = 150.f * entries_a * (float)((entries + 31) / 32) <= 4000.f + 200.f * entries_a + 0.7f * products;
-        int list = LIST_WIDE;
-        if (by_mask) list = LIST_MASK;
-        else if (words <= CLASS[0].words && entries <= CLASS[0].entries) list = 0;
-        else if (words <= CLASS[1].words && entries <= CLASS[1].entries) list = 1;
-        else if (words <= CLASS[2].words) list = 2;
-        const int unit = list == LIST_MASK ? MASK_UNIT : list == 0 ? CLASS[0].unit() : list == LIST_WIDE ? CLASS[LIST_WIDE].unit() : CLASS[1].unit();
-        const int n_units = (a_hi - a_lo + unit - 1) / unit;
-        int base = 0;
-        if (lane == 0) base = atomicAdd(&ctl->count[list], n_units);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        for (int u = lane; u < n_units; u += 32) units[(list == LIST_MASK ? 4 : list) * list_cap + base + u] = make_int2((int)i, a_lo + u * unit);
+        const int unit = unit_of(list);
+        int2 *to = units + (list == LIST_MASK ? 4 : list) * list_cap + at;
+        for (int u = lane; u < n_units; u += 32) to[u] = make_int2((int)row_of(r), s_lo[r] + u * unit);
     }
 }
 
@@ -560,7 +636,7 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     const int most = (int)std::min<int64_t>(list_cap, 1 << 30);
     {
         LaunchScope scope("sssmm_classify", stream);
-        k_sssmm_classify<<<row_warps_grid, 256, 0, stream>>>(A, B, C, rows, list_cap, units, light, sctl);
+        k_sssmm_classify<<<(int)(((int64_t)rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, stream>>>(A, B, C, rows, list_cap, units, light, sctl);
     }
     // Every list is worked by resident CTAs that take units from a ticket; a list's length stays on
     // the device, so an empty list costs one launch of CTAs that leave at once.
