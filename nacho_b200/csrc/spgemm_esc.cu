@@ -46,11 +46,12 @@ struct CsrView {
     const float *val;
 };
 
+enum { BIN_SMALL, BIN_MEDIUM, BIN_RANKED, BIN_GIANT, BIN_HEAVY, BINS };  // heavy rows with more / at most GIANT_P products
+
 // Device-side counters of one call.
 struct EscCtl {
     unsigned long long products;
-    int n_small, n_medium, n_ranked;
-    int n_giant, n_heavy;  // heavy rows with more / at most GIANT_P products
+    int n_rows[BINS];
     int max_entries;       // longest row of A
     int arrived;           // CTAs of the binning kernel that are done
 };
@@ -66,11 +67,11 @@ __device__ __forceinline__ void publish_counters(EscCtl *ctl, const FusedCtl *pr
     if (atomicAdd(&ctl->arrived, 1) != (int)gridDim.x - 1) return;
     __threadfence();
     const volatile EscCtl *c = ctl;
-    publish_result_word(words + W_SMALL, 0, c->n_small);
-    publish_result_word(words + W_MEDIUM, 0, c->n_medium);
-    publish_result_word(words + W_RANKED, 0, c->n_ranked);
-    publish_result_word(words + W_GIANT, 0, c->n_giant);
-    publish_result_word(words + W_HEAVY, 0, c->n_heavy);
+    publish_result_word(words + W_SMALL, 0, c->n_rows[BIN_SMALL]);
+    publish_result_word(words + W_MEDIUM, 0, c->n_rows[BIN_MEDIUM]);
+    publish_result_word(words + W_RANKED, 0, c->n_rows[BIN_RANKED]);
+    publish_result_word(words + W_GIANT, 0, c->n_rows[BIN_GIANT]);
+    publish_result_word(words + W_HEAVY, 0, c->n_rows[BIN_HEAVY]);
     publish_result_word(words + W_ENTRIES, 0, c->max_entries);
     publish_result_word(words + W_PRODUCTS, prefix && prefix->status.error != 0 ? NB200_E_TIMEOUT : NB200_OK, (long long)c->products);
 }
@@ -137,6 +138,44 @@ __global__ void __launch_bounds__(256) k_esc_product_prefix(CsrView A, CsrView B
     }
 }
 
+// Puts row i (p products) of every thread of the CTA on its list, and adds the products up. A CTA advances each list
+// once: every warp's atomics on the same few words held the kernel up (262144 rows of a mesh 22.2 -> 14.6 us).
+__device__ __forceinline__ void bin_rows(const int i, const unsigned long long p, const int32_t rows, int32_t *row_count, const RowLists &lists, EscCtl *ctl) {
+    __shared__ unsigned long long s_products;
+    __shared__ int s_count[BINS];
+    if (threadIdx.x < BINS) s_count[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_products = 0;
+    __syncthreads();
+    const int bin = p == 0 ? -1 : p <= SMALL_P ? BIN_SMALL : p <= MEDIUM_P ? BIN_MEDIUM : p <= RANKED_P ? BIN_RANKED : p > GIANT_P ? BIN_GIANT : BIN_HEAVY;
+    int at = 0;
+#pragma unroll
+    for (int b = 0; b < BINS; ++b) {  // the rows of a list stay in order within a warp
+        const unsigned same = __ballot_sync(FULL_MASK, bin == b);
+        if (same == 0u) continue;
+        int first = 0;
+        if (lane_id() == 0) first = atomicAdd(&s_count[b], __popc(same));
+        first = __shfl_sync(FULL_MASK, first, 0);
+        if (bin == b) at = first + __popc(same & ((1u << lane_id()) - 1u));
+    }
+    unsigned long long sum = p;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL_MASK, sum, o);
+    if (lane_id() == 0 && sum) atomicAdd(&s_products, sum);
+    __syncthreads();
+    if (threadIdx.x < BINS && s_count[threadIdx.x] > 0) s_count[threadIdx.x] = atomicAdd(&ctl->n_rows[threadIdx.x], s_count[threadIdx.x]);  // from here on: where the CTA's rows begin
+    if (threadIdx.x == BINS && s_products) atomicAdd(&ctl->products, s_products);
+    __syncthreads();
+    if (bin >= 0) {
+        at += s_count[bin];
+        if (bin == BIN_SMALL) lists.small_rows[at] = i;
+        else if (bin == BIN_MEDIUM) lists.medium_rows[at] = i;
+        else if (bin == BIN_RANKED) lists.ranked_rows[at] = i;
+        else lists.heavy_rows[bin == BIN_GIANT ? at : rows - 1 - at] = i;
+    } else if (i < rows && row_count) {
+        row_count[i] = 0;
+    }
+}
+
 // Expand phase 1 (src/backend/compute.cpp:541-611): per-row product counts, and the bins.
 // Rows without products get their count (0) written here. The counts come from the prefix P of
 // B's row lengths over A's entries (k_esc_product_prefix): a hub row costs one subtraction.
@@ -144,38 +183,13 @@ __global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned l
                                                      int32_t *__restrict__ row_count, RowLists lists, EscCtl *ctl,
                                                      const FusedCtl *prefix, unsigned long long *words) {
     wait_for_previous();
-    __shared__ unsigned long long warp_p[8];
     const int i = blockIdx.x * 256 + threadIdx.x;  // one lane per row: its products are a difference of the prefix
     unsigned long long p = 0;
     if (i < rows) {
         const int32_t base = ld_nc(A.rp);
         p = ld_nc(P + (ld_nc(A.rp + i + 1) - base)) - ld_nc(P + (ld_nc(A.rp + i) - base));
     }
-    if (i < rows) {  // lanes of a warp that take the same branch share one atomic
-        if (p == 0) {
-            if (row_count) row_count[i] = 0;
-        } else if (p <= SMALL_P) {
-            lists.small_rows[atomicAdd(&ctl->n_small, 1)] = i;
-        } else if (p <= MEDIUM_P) {
-            lists.medium_rows[atomicAdd(&ctl->n_medium, 1)] = i;
-        } else if (p <= RANKED_P) {
-            lists.ranked_rows[atomicAdd(&ctl->n_ranked, 1)] = i;
-        } else if (p > GIANT_P) {
-            lists.heavy_rows[atomicAdd(&ctl->n_giant, 1)] = i;
-        } else {
-            lists.heavy_rows[rows - 1 - atomicAdd(&ctl->n_heavy, 1)] = i;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(FULL_MASK, p, o);
-    // one atomic per CTA for the product total
-    if (lane_id() == 0) warp_p[warp_id()] = p;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long sum = 0;
-        for (int v = 0; v < 8; ++v) sum += warp_p[v];
-        if (sum) atomicAdd(&ctl->products, sum);
-    }
+    bin_rows(i, p, rows, row_count, lists, ctl);
     publish_counters(ctl, prefix, words);
 }
 
@@ -184,7 +198,6 @@ __global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned l
 // entries costs more than it saves.
 __global__ void __launch_bounds__(256) k_esc_rowwork_walk(CsrView A, CsrView B, int32_t rows, int32_t *__restrict__ row_count,
                                                      RowLists lists, EscCtl *ctl, unsigned long long *words) {
-    __shared__ unsigned long long warp_p[8];
     const int i = blockIdx.x * 256 + threadIdx.x;  // one lane per row; the warp shares the work of its longer rows
     int32_t lo = 0, hi = 0;
     if (i < rows) {
@@ -194,50 +207,38 @@ __global__ void __launch_bounds__(256) k_esc_rowwork_walk(CsrView A, CsrView B, 
     unsigned long long p = 0;
     const bool together = hi - lo > 32;
     if (!together) {
-        for (int32_t e = lo; e < hi; ++e) {
-            const int32_t j = ld_nc(A.col + e);
-            p += (unsigned long long)(ld_nc(B.rp + j + 1) - ld_nc(B.rp + j));
+        for (int32_t e = lo; e < hi; e += 4) {  // four entries' loads in flight
+            int32_t j[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) j[q] = e + q < hi ? ld_nc(A.col + e + q) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (j[q] >= 0) p += (unsigned long long)(ld_nc(B.rp + j[q] + 1) - ld_nc(B.rp + j[q]));
         }
     }
     for (unsigned todo = __ballot_sync(FULL_MASK, together); todo; todo &= todo - 1) {
         const int r = __ffs(todo) - 1;
         const int32_t l = __shfl_sync(FULL_MASK, lo, r), h = __shfl_sync(FULL_MASK, hi, r);
         unsigned long long q = 0;
-        for (int32_t e = l + lane_id(); e < h; e += 32) {
-            const int32_t j = ld_nc(A.col + e);
-            q += (unsigned long long)(ld_nc(B.rp + j + 1) - ld_nc(B.rp + j));
+        for (int32_t e = l + lane_id(); e < h; e += 128) {  // a hub row is a chain of these: four entries' loads in flight
+            int32_t j[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) j[u] = e + 32 * u < h ? ld_nc(A.col + e + 32 * u) : -1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j[u] >= 0) q += (unsigned long long)(ld_nc(B.rp + j[u] + 1) - ld_nc(B.rp + j[u]));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(FULL_MASK, q, o);
         if (lane_id() == r) p = q;
     }
-    if (i < rows) {  // lanes of a warp that take the same branch share one atomic
-        if (p == 0) {
-            if (row_count) row_count[i] = 0;
-        } else if (p <= SMALL_P) {
-            lists.small_rows[atomicAdd(&ctl->n_small, 1)] = i;
-        } else if (p <= MEDIUM_P) {
-            lists.medium_rows[atomicAdd(&ctl->n_medium, 1)] = i;
-        } else if (p <= RANKED_P) {
-            lists.ranked_rows[atomicAdd(&ctl->n_ranked, 1)] = i;
-        } else if (p > GIANT_P) {
-            lists.heavy_rows[atomicAdd(&ctl->n_giant, 1)] = i;
-        } else {
-            lists.heavy_rows[rows - 1 - atomicAdd(&ctl->n_heavy, 1)] = i;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(FULL_MASK, p, o);
-    // one atomic per CTA for the product total
-    if (lane_id() == 0) warp_p[warp_id()] = p;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long sum = 0;
-        for (int v = 0; v < 8; ++v) sum += warp_p[v];
-        if (sum) atomicAdd(&ctl->products, sum);
-    }
+    __shared__ int s_longest;
+    if (threadIdx.x == 0) s_longest = 0;
+    bin_rows(i, p, rows, row_count, lists, ctl);
     const int longest = __reduce_max_sync(FULL_MASK, hi - lo);
-    if (lane_id() == 0 && longest > 0) atomicMax(&ctl->max_entries, longest);
+    if (lane_id() == 0) atomicMax(&s_longest, longest);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_longest > 0) atomicMax(&ctl->max_entries, s_longest);
     publish_counters(ctl, nullptr, words);
 }
 
@@ -1009,11 +1010,11 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
         // a prefix whose look-back gave up leaves rows with wrong product counts: nothing may be built on them
         if (failed) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm product prefix");
         plan->host.products = (unsigned long long)v[W_PRODUCTS];
-        plan->host.n_small = (int)v[W_SMALL], plan->host.n_medium = (int)v[W_MEDIUM], plan->host.n_ranked = (int)v[W_RANKED];
-        plan->host.n_giant = (int)v[W_GIANT], plan->host.n_heavy = (int)v[W_HEAVY];
+        plan->host.n_rows[BIN_SMALL] = (int)v[W_SMALL], plan->host.n_rows[BIN_MEDIUM] = (int)v[W_MEDIUM], plan->host.n_rows[BIN_RANKED] = (int)v[W_RANKED];
+        plan->host.n_rows[BIN_GIANT] = (int)v[W_GIANT], plan->host.n_rows[BIN_HEAVY] = (int)v[W_HEAVY];
         plan->host.max_entries = short_rows ? (int)v[W_ENTRIES] : INT_MAX;
     }
-    if (with_table && plan->host.n_ranked + plan->host.n_giant + plan->host.n_heavy > 0) {
+    if (with_table && plan->host.n_rows[BIN_RANKED] + plan->host.n_rows[BIN_GIANT] + plan->host.n_rows[BIN_HEAVY] > 0) {
         LaunchScope scope("esc_window_ptr", stream);
         k_esc_window_ptr<<<(unsigned)((ptr_entries + 255) / 256), 256, 0, stream>>>(B, b->rows, plan->n_win, plan->win_ptr);
         NB200_CUDA(cudaGetLastError());
@@ -1022,8 +1023,8 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     plan->cache_ws = nullptr;
     if (carry_bitmaps && plan->n_win == 1) {
         // a second pool block: its size is only known now, and the first must not move
-        const size_t ranked_bytes = (size_t)plan->host.n_ranked * ranked_words(RK_NT, b->cols) * 4;
-        const size_t heavy_bytes = ((size_t)plan->host.n_giant + plan->host.n_heavy) * ranked_words(HEAVY_NT, b->cols) * 4;
+        const size_t ranked_bytes = (size_t)plan->host.n_rows[BIN_RANKED] * ranked_words(RK_NT, b->cols) * 4;
+        const size_t heavy_bytes = ((size_t)plan->host.n_rows[BIN_GIANT] + plan->host.n_rows[BIN_HEAVY]) * ranked_words(HEAVY_NT, b->cols) * 4;
         if (ranked_bytes + heavy_bytes > 0 && ranked_bytes + heavy_bytes <= BITMAP_CACHE_BUDGET) {
             Carver cache_sizes;
             cache_sizes.take<uint32_t>(ranked_bytes / 4);
@@ -1089,31 +1090,31 @@ int esc_run_bins(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, co
     int32_t *c_col = NUMERIC ? c->col : nullptr;
     float *c_val = NUMERIC ? c->val : nullptr;
     int st;
-    const int n_heavy = plan.host.n_giant + plan.host.n_heavy;
+    const int n_heavy = plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY];
     bool beside = false;
     if (n_heavy > 0) {  // first: the heaviest rows take longest
         LaunchScope scope(NUMERIC ? "esc_heavy_numeric" : "esc_heavy_symbolic", stream);
-        if ((st = launch_ranked<NUMERIC, HEAVY_NT>(A, B, plan, b->cols, plan.lists.heavy_rows, a->rows, plan.host.n_giant, n_heavy,
+        if ((st = launch_ranked<NUMERIC, HEAVY_NT>(A, B, plan, b->cols, plan.lists.heavy_rows, a->rows, plan.host.n_rows[BIN_GIANT], n_heavy,
                                                              plan.cache_heavy, count, c_rp, c_col, c_val, stream, false)))
             return st;
         beside = true;
     }
-    if (plan.host.n_ranked > 0) {
+    if (plan.host.n_rows[BIN_RANKED] > 0) {
         LaunchScope scope(NUMERIC ? "esc_ranked_numeric" : "esc_ranked_symbolic", stream);
-        if ((st = launch_ranked<NUMERIC, RK_NT>(A, B, plan, b->cols, plan.lists.ranked_rows, a->rows, plan.host.n_ranked,
-                                                          plan.host.n_ranked, plan.cache_ranked, count, c_rp, c_col, c_val, stream, beside)))
+        if ((st = launch_ranked<NUMERIC, RK_NT>(A, B, plan, b->cols, plan.lists.ranked_rows, a->rows, plan.host.n_rows[BIN_RANKED],
+                                                          plan.host.n_rows[BIN_RANKED], plan.cache_ranked, count, c_rp, c_col, c_val, stream, beside)))
             return st;
         beside = true;
     }
-    if (plan.host.n_medium > 0) {
+    if (plan.host.n_rows[BIN_MEDIUM] > 0) {
         LaunchScope scope(NUMERIC ? "esc_medium_numeric" : "esc_medium_symbolic", stream);
-        if ((st = launch_bin(beside, k_esc_medium<NUMERIC>, plan.host.n_medium, MED_NT, 0, stream, A, B, plan.lists.medium_rows, count, c_rp, c_col, c_val)))
+        if ((st = launch_bin(beside, k_esc_medium<NUMERIC>, plan.host.n_rows[BIN_MEDIUM], MED_NT, 0, stream, A, B, plan.lists.medium_rows, count, c_rp, c_col, c_val)))
             return st;
         beside = true;
     }
-    if (plan.host.n_small > 0) {
+    if (plan.host.n_rows[BIN_SMALL] > 0) {
         LaunchScope scope(NUMERIC ? "esc_small_numeric" : "esc_small_symbolic", stream);
-        const int warps = plan.host.n_small;  // rows on the list
+        const int warps = plan.host.n_rows[BIN_SMALL];  // rows on the list
         const int small_warps = (warps + ESC_SMALL_ROWS - 1) / ESC_SMALL_ROWS;
         auto kernel = b->cols < (1 << 27) ? k_esc_small<NUMERIC, true> : k_esc_small<NUMERIC, false>;
         if ((st = launch_bin(beside, kernel, (small_warps + 7) / 8, 256, 0, stream, A, B, plan.lists.small_rows, warps, count, c_rp, c_col, c_val))) return st;
@@ -1221,7 +1222,7 @@ int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *s
 }
 
 bool is_short(const EscPlan &plan) {
-    return plan.host.n_medium + plan.host.n_ranked + plan.host.n_giant + plan.host.n_heavy == 0 && plan.host.max_entries <= SHORT_ENTRIES &&
+    return plan.host.n_rows[BIN_MEDIUM] + plan.host.n_rows[BIN_RANKED] + plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY] == 0 && plan.host.max_entries <= SHORT_ENTRIES &&
            plan.host.products > 0 && plan.host.products <= INT32_MAX;
 }
 
