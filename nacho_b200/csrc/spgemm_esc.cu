@@ -809,11 +809,13 @@ constexpr int SHORT_NT = 128, SHORT_ENTRIES = 8;
 
 // The whole product in one pass, for matrices whose rows of A hold at most K <= 8 entries and reach at
 // most SMALL_P products (meshes, bands). One THREAD merges one row: the K rows of B are sorted lists whose
-// heads it keeps in registers; a step takes the smallest head and adds up the lists that hold it, in the
+// heads it keeps in registers, with the entry behind each (the steps are bound by the latency of these loads, at the
+// 24 warps per SM that the staging leaves); a step takes the smallest head and adds up the lists that hold it, in the
 // order of A's entries (ascending j, the same sum as the other kernels form). A row is staged in shared memory
 // at the offset of its product count, the CTA's result count goes through the cross-tile scan of the merge
 // kernels, and the rows are copied out eight lanes to a row. 512 x 512 5-point mesh squared: a warp per row with
-// a 32-wide bitonic sort, counting first, took 240 instructions a row and 156 us in two kernels.
+// a 32-wide bitonic sort, counting first, took 240 instructions a row and 156 us in two kernels; without the entry
+// behind each head this one took 49 us, with it 44.
 template <int K>
 __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, int32_t rows, TileWords words, FusedCtl *ctl, int num_tiles,
                                                        int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col, float *__restrict__ c_val,
@@ -839,9 +841,9 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
     const int t = blockIdx.x - (scanned ? 1 : 0), tid = threadIdx.x, lane = lane_id();
     const int64_t i = (int64_t)t * SHORT_NT + tid;
     const int32_t lo = i < rows ? ld_nc(A.rp + i) : 0, hi = i < rows ? ld_nc(A.rp + i + 1) : 0;
-    int32_t pos[K], end[K];
-    uint32_t head[K];
-    float a[K];
+    uint32_t pos[K], end[K];  // one past the last entry of 2^31 - 1 is still a position
+    uint32_t head[K], next[K];
+    float a[K], head_val[K], next_val[K];
     int products = 0;
 #pragma unroll
     for (int e = 0; e < K; ++e) {
@@ -852,7 +854,14 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
         products += end[e] - pos[e];
     }
 #pragma unroll
-    for (int e = 0; e < K; ++e) head[e] = pos[e] < end[e] ? (uint32_t)ld_nc(B.col + pos[e]) : END;
+    for (int e = 0; e < K; ++e) {
+        auto fetch = [&](uint32_t q, uint32_t &col, float &val) {
+            col = q < end[e] ? (uint32_t)ld_nc(B.col + q) : END;
+            val = q < end[e] ? ld_nc(B.val + q) : 0.f;
+        };
+        fetch(pos[e], head[e], head_val[e]);
+        fetch(++pos[e], next[e], next_val[e]);  // from here on pos is that of `next`
+    }
     int tile_products;
     const int staged = block_excl_sum<SHORT_NT>(products, scan_tmp, tile_products);
     int count = 0;
@@ -866,11 +875,17 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
 #pragma unroll
         for (int e = 0; e < K; ++e) {
             if (head[e] == m) {
-                const float v = a[e] * ld_nc(B.val + pos[e]);
+                const float v = a[e] * head_val[e];
                 acc = first ? v : acc + v;
                 first = false;
-                ++pos[e];
-                head[e] = pos[e] < end[e] ? (uint32_t)ld_nc(B.col + pos[e]) : END;
+                head[e] = next[e];
+                head_val[e] = next_val[e];
+                if (++pos[e] < end[e]) {
+                    next[e] = (uint32_t)ld_nc(B.col + pos[e]);
+                    next_val[e] = ld_nc(B.val + pos[e]);
+                } else {
+                    next[e] = END;
+                }
             }
         }
         s_col[staged + count] = m;
