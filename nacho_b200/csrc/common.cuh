@@ -148,9 +148,19 @@ __device__ __forceinline__ void publish_result_word(unsigned long long *word, in
                                                                        ((unsigned long long)value & RW_VALUE_MASK);
 }
 
+// For memory that nothing writes while the kernel runs: from the moment it could start, that is, which for a kernel
+// of launch_overlapped lies before the end of the kernel in front of it.
 template <typename T>
 __device__ __forceinline__ T ld_nc(const T *p) {
     return __ldg(p);
+}
+
+// For what a kernel of launch_overlapped reads of the work in front of it, operands that an earlier call may still be
+// writing among it: a plain load, which the compiler keeps behind wait_for_previous. (ld_nc tells it that the memory never
+// changes, and it may then ask for it before the wait; so does a const __restrict__ parameter.)
+template <typename T>
+__device__ __forceinline__ T ld_late(const T *p) {
+    return *p;
 }
 #endif
 

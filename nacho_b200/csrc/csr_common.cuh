@@ -47,7 +47,7 @@ struct LevelOffsets {
     int32_t *off_a = nullptr, *off_b = nullptr, *keep = nullptr;
 };
 
-__device__ __forceinline__ int32_t row_offset(const CsrIn &m, int64_t r) { return m.rp ? ld_nc(m.rp + r) : r > 0 ? m.entries() : 0; }
+__device__ __forceinline__ int32_t row_offset(const CsrIn &m, int64_t r) { return m.rp ? ld_late(m.rp + r) : r > 0 ? m.entries() : 0; }
 
 constexpr int MBAR_POLL_LIMIT = 1 << 24;
 constexpr int ERR_COPY_TIMEOUT = 2;

@@ -114,12 +114,12 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
     // Merge-path diagonal dd inside the row: x entries of A and dd - x of B come first.
     const uint32_t x_lo = (uint32_t)max((int64_t)0, dd - len_b), x_hi = (uint32_t)min(dd, len_a);
     const uint32_t x = group_count_true<G>(x_lo, inner ? x_hi : x_lo, [&](uint32_t m) {
-        return ld_nc(A.col + a_lo + m) <= ld_nc(B.col + b_lo + (dd - 1 - m));
+        return ld_late(A.col + a_lo + m) <= ld_late(B.col + b_lo + (dd - 1 - m));
     });
     int64_t y = dd - x;
     if (inner) {
         // Keep a column present in both operands on one side of the cut.
-        if (x > 0 && y < len_b && ld_nc(A.col + a_lo + x - 1) == ld_nc(B.col + b_lo + y)) ++y;
+        if (x > 0 && y < len_b && ld_late(A.col + a_lo + x - 1) == ld_late(B.col + b_lo + y)) ++y;
     }
     if ((threadIdx.x & (G - 1)) == 0 && gid / G <= num_tiles) {
         cuts[t] = inner ? make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0)
@@ -242,7 +242,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
         const int e = is_b ? k - 6 : k;
         const int count = is_b ? nb : na, head = is_b ? head_b : head_a, nv = is_b ? nvb : nva;
         const int idx = e < 3 ? e : head + 4 * nv + (e - 3);
-        if (e < 3 ? e < head : idx < count) keys[(is_b ? ob : oa) + idx] = (uint32_t)ld_nc((is_b ? gb_col : ga_col) + idx);
+        if (e < 3 ? e < head : idx < count) keys[(is_b ? ob : oa) + idx] = (uint32_t)ld_late((is_b ? gb_col : ga_col) + idx);
     }
     if (tid == 64) keys[oa + na] = (uint32_t)END;
     if (tid == 65) keys[ob + nb] = (uint32_t)END;
@@ -317,7 +317,18 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     if (rows_fit) {
         for (int r = 1 + tid; r <= nr; r += NT) begin_row(r, s_rows[r], s_rows[r + 1]);
     } else {
-        for (int r = 1 + tid; r <= nr; r += NT) begin_row(r, global_start(r), row_start(r + 1));
+        for (int r0 = 1; r0 <= nr; r0 += RB * NT) {
+            uint32_t w[RB], w_next[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u) {
+                const int r = r0 + u * NT + tid;
+                w[u] = r <= nr ? global_start(r) : 0u;
+                w_next[u] = r <= nr ? row_start(r + 1) : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+                if (r0 + u * NT + tid <= nr) begin_row(r0 + u * NT + tid, w[u], w_next[u]);
+        }
     }
     __syncthreads();
 
@@ -518,9 +529,9 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
                 col[g] = word_at(other) & cmask;
                 const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
                 float v = 0.0f;
-                if (ok) v = __ldg(reinterpret_cast<const float *>((at >= first_b ? vb : va) + at));
+                if (ok) v = ld_late(reinterpret_cast<const float *>((at >= first_b ? vb : va) + at));
                 if (both) {
-                    const float u = __ldg(reinterpret_cast<const float *>(vb + other));
+                    const float u = ld_late(reinterpret_cast<const float *>(vb + other));
                     v = OP == OP_UNION ? v + u : v * u;
                 }
                 val[g] = v;
@@ -530,7 +541,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             for (int g = 0; g < GATHER; ++g) {
                 const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
                 col[g] = word_at(s[g]) & cmask;
-                val[g] = ok ? __ldg(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
+                val[g] = ok ? ld_late(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
             }
         }
     };
@@ -544,22 +555,33 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
 
     if (LEVELS) {
         // ---- offsets mode: the column and the two range starts of every result entry
-        for (int o = tid; o < total; o += NT) {
-            const uint32_t s = src_of[o];
-            const bool ta = s & 1u, tb = (s >> 16) & 1u;
-            const uint32_t pa = s & 0xfffcu, pb = (s >> 16) & 0xfffcu;
-            const int32_t *la = L.a + tile.a0 + ((int)(pa >> 2) - oa), *lb = L.b + tile.b0 + ((int)(pb >> 2) - ob);
-            const int32_t at_a = ld_nc(la), at_b = ld_nc(lb);
-            const bool full_a = ta && ld_nc(la + 1) > at_a, full_b = tb && ld_nc(lb + 1) > at_b;
-            Z.col[base + o] = (int32_t)(word_at(ta ? pa : pb) & cmask);
-            L.off_a[base + o] = at_a;
-            L.off_b[base + o] = at_b;
-            if (L.keep) L.keep[base + o] = full_a && full_b;
-            if (!full_a && !full_b) ctl->hollow = 1;
+        constexpr int LB = 4;  // result entries a thread fetches together
+        const int32_t *from_a = L.a + (tile.a0 - oa), *from_b = L.b + (tile.b0 - ob);
+        for (int o0 = tid; o0 < total; o0 += LB * NT) {
+            int32_t at_a[LB], at_b[LB], end_a[LB], end_b[LB], col[LB];
+#pragma unroll
+            for (int u = 0; u < LB; ++u) {
+                const uint32_t s = src_of[min(o0 + u * NT, total - 1)], pa = s & 0xfffcu, pb = (s >> 16) & 0xfffcu;
+                const int32_t *la = from_a + (pa >> 2), *lb = from_b + (pb >> 2);
+                at_a[u] = ld_late(la), end_a[u] = ld_late(la + (s & 1u));
+                at_b[u] = ld_late(lb), end_b[u] = ld_late(lb + ((s >> 16) & 1u));
+                col[u] = (int32_t)(word_at(s & 1u ? pa : pb) & cmask);
+            }
+#pragma unroll
+            for (int u = 0; u < LB; ++u) {
+                if (o0 + u * NT >= total) break;
+                const long long o = base + o0 + u * NT;
+                const bool full_a = end_a[u] > at_a[u], full_b = end_b[u] > at_b[u];
+                Z.col[o] = col[u];
+                L.off_a[o] = at_a[u];
+                L.off_b[o] = at_b[u];
+                if (L.keep) L.keep[o] = full_a && full_b;
+                if (!full_a && !full_b) ctl->hollow = 1;
+            }
         }
         if (t == num_tiles - 1 && tid == 0) {
-            L.off_a[base + total] = ld_nc(L.a + tile.a0 + na);
-            L.off_b[base + total] = ld_nc(L.b + tile.b0 + nb);
+            L.off_a[base + total] = ld_late(L.a + tile.a0 + na);
+            L.off_b[base + total] = ld_late(L.b + tile.b0 + nb);
         }
     } else {
     // ---- store the tile, coalesced
@@ -612,7 +634,14 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     if (rows_fit) {
         for (int r = 1 + tid; r <= nr; r += NT) end_row(r, s_rows[r]);
     } else {
-        for (int r = 1 + tid; r <= nr; r += NT) end_row(r, global_start(r));
+        for (int r0 = 1; r0 <= nr; r0 += RB * NT) {
+            uint32_t w[RB];
+#pragma unroll
+            for (int u = 0; u < RB; ++u) w[u] = r0 + u * NT + tid <= nr ? global_start(r0 + u * NT + tid) : 0u;
+#pragma unroll
+            for (int u = 0; u < RB; ++u)
+                if (r0 + u * NT + tid <= nr) end_row(r0 + u * NT + tid, w[u]);
+        }
     }
     if (t == 0 && tid == 0) Z.rp[0] = 0;
 }

@@ -179,7 +179,7 @@ __device__ __forceinline__ void bin_rows(const int i, const unsigned long long p
 // Expand phase 1 (src/backend/compute.cpp:541-611): per-row product counts, and the bins.
 // Rows without products get their count (0) written here. The counts come from the prefix P of
 // B's row lengths over A's entries (k_esc_product_prefix): a hub row costs one subtraction.
-__global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned long long *__restrict__ P, int32_t rows,
+__global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned long long *P, int32_t rows,
                                                      int32_t *__restrict__ row_count, RowLists lists, EscCtl *ctl,
                                                      const FusedCtl *prefix, unsigned long long *words) {
     wait_for_previous();
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) k_esc_rowwork(CsrView A, const unsigned l
     unsigned long long p = 0;
     if (i < rows) {
         const int32_t base = ld_nc(A.rp);
-        p = ld_nc(P + (ld_nc(A.rp + i + 1) - base)) - ld_nc(P + (ld_nc(A.rp + i) - base));
+        p = ld_late(P + (ld_nc(A.rp + i + 1) - base)) - ld_late(P + (ld_nc(A.rp + i) - base));  // (A lay ready before the prefix pass began)
     }
     bin_rows(i, p, rows, row_count, lists, ctl);
     publish_counters(ctl, prefix, words);

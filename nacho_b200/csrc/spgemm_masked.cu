@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(SEARCH_NT) k_sssmm_search_cta(CsrView A, CsrVi
 }
 
 template <int NT, bool SHARED_ACC>
-__global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrView C, const int2 *__restrict__ units,
-                                                    SssmmCtl *__restrict__ ctl, int which, int words_cap, int entries_cap,
+__global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrView C, const int2 *units,
+                                                    SssmmCtl *ctl, int which, int words_cap, int entries_cap,
                                                     float *__restrict__ acc, int32_t *__restrict__ hit) {
     extern __shared__ uint64_t sm_words[];
     uint64_t *bm = sm_words;                                         // bit (k - 64 * w0) set: the mask row stores column k
@@ -520,9 +520,9 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
 // Exclusive scan of the flags over nnz + 1 entries, in place (the last flag is 0, so pos[nnz] is the total, which
 // also goes to `word`), and, where the caller's arrays hold every mask position (`z_col` set), the reached
 // positions written to their places in the same pass.
-__global__ void __launch_bounds__(SCAN_NT) k_sssmm_scan(int32_t *__restrict__ pos, const float *__restrict__ acc, const int32_t *__restrict__ c_rp,
+__global__ void __launch_bounds__(SCAN_NT) k_sssmm_scan(int32_t *pos, const float *acc, const int32_t *__restrict__ c_rp,
                                                        const int32_t *__restrict__ c_col, int32_t nnz, uint64_t *state, FusedCtl *ctl,
-                                                       int32_t *__restrict__ z_col, float *__restrict__ z_val, unsigned long long *word) {
+                                                       int32_t *z_col, float *z_val, unsigned long long *word) {
     __shared__ int scan_tmp[40];
     __shared__ long long s_base;
     trigger_dependents();
@@ -547,6 +547,9 @@ __global__ void __launch_bounds__(SCAN_NT) k_sssmm_scan(int32_t *__restrict__ po
     if (s_base < 0) return;
     int32_t at = (int32_t)s_base + run;  // at most nnz
     const int32_t *mask_col = c_col + ld_nc(c_rp);
+    float sum[SCAN_VT];  // fetched together: a plain load stays behind the stores in front of it
+#pragma unroll
+    for (int q = 0; q < SCAN_VT; ++q) sum[q] = v[q] && z_col ? ld_late(acc + p0 + q) : 0.f;
 #pragma unroll
     for (int q = 0; q < SCAN_VT; ++q) {
         if (p0 + q >= n) break;
@@ -554,19 +557,19 @@ __global__ void __launch_bounds__(SCAN_NT) k_sssmm_scan(int32_t *__restrict__ po
         if (v[q]) {
             if (z_col) {
                 z_col[at] = ld_nc(mask_col + p0 + q);
-                z_val[at] = acc[p0 + q];
+                z_val[at] = sum[q];
             }
             ++at;
         }
     }
 }
 
-__global__ void __launch_bounds__(256) k_sssmm_row_offsets(const int32_t *__restrict__ pos, const int32_t *__restrict__ c_rp,
-                                                          int32_t rows, int32_t *__restrict__ z_rp) {
+__global__ void __launch_bounds__(256) k_sssmm_row_offsets(const int32_t *pos, const int32_t *__restrict__ c_rp,
+                                                          int32_t rows, int32_t *z_rp) {
     wait_for_previous();
     const int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (r > rows) return;
-    z_rp[r] = pos[ld_nc(c_rp + r) - ld_nc(c_rp)];
+    z_rp[r] = ld_late(pos + (ld_nc(c_rp + r) - ld_nc(c_rp)));
 }
 
 // Writes the reached positions after the scan, for callers with less room than the mask has entries.

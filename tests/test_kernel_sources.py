@@ -1,0 +1,36 @@
+"""CPU suite: rules that a compiled kernel cannot show and its source can."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nacho_b200", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def parameters(text, kernel):
+    """The parameter list of a kernel's definition."""
+    return re.search(re.escape(kernel) + r"\(([^{;]*)\)\s*\{", text).group(1)
+
+
+def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():
+    """A kernel that starts beside the one in front of it must not use read-only loads (ld.global.nc, or a const
+    __restrict__ parameter that the compiler turns into one) for what that kernel writes: they may be issued before the
+    wait. All kernels of the CSR merge start like that, and their operands may be an earlier call's result."""
+    for name in ("csr_merge.cu", "csr_common.cuh"):
+        text = source(name)
+        assert not re.search(r"\bld_nc\b|\b__ldg\b|\b__ldcs\b|__restrict__", text), name
+    late = {("spgemm_esc.cu", "k_esc_rowwork"): ["P"], ("spgemm_masked.cu", "k_sssmm_bitmap"): ["units", "ctl"],
+            ("spgemm_masked.cu", "k_sssmm_scan"): ["pos", "acc"], ("spgemm_masked.cu", "k_sssmm_row_offsets"): ["pos"]}
+    for (name, kernel), arrays in late.items():
+        text = source(name)
+        given = parameters(text, kernel)
+        for a in arrays:
+            assert re.search(r"\*" + a + r"\b", given), (kernel, a)
+            assert not re.search(r"__restrict__\s+" + a + r"\b", given), (kernel, a)
+        body = text[text.index(given):]
+        body = body[:re.search(r"\n\}", body).start()]
+        for a in arrays:
+            assert not re.search(r"(ld_nc|__ldg|__ldcs)\(" + a + r"\b", body), (kernel, a)
