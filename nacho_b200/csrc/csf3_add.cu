@@ -284,7 +284,8 @@ bool levels_pay(const nb200_csf3 *a, const nb200_csf3 *b) {
 
 // `done` tells whether the result is in place; it is not where an operand stores empty slices or fibres, which
 // the canonical tree does not have (the caller then takes the other route).
-int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cudaStream_t stream, bool *done) {
+int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cudaStream_t stream, bool *done,
+                   const LaunchKnobs &first_knobs = LaunchKnobs()) {
     *done = false;
     const int64_t bound_i = (int64_t)a->n_i + b->n_i, bound_j = (int64_t)a->n_j + b->n_j, total = (int64_t)a->n_k + b->n_k;
     if (bound_j > INT32_MAX - 1) return NB200_E_OVERFLOW;
@@ -306,7 +307,7 @@ int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cuda
 
     const LevelOffsets slices{a->j_ptr, b->j_ptr, ja, jb}, fibres{a->k_ptr, b->k_ptr, ka, kb};
     if ((st = csr2_enqueue(OP_UNION, CsrIn{nullptr, a->i_idx, nullptr, a->n_i}, CsrIn{nullptr, b->i_idx, nullptr, b->n_i}, RowCount{1}, a->dims[0],
-                           CsrOut{nullptr, z->i_idx, nullptr, nullptr, word[0]}, &slices, scratch_i, stream, &ctl[0])))
+                           CsrOut{nullptr, z->i_idx, nullptr, nullptr, word[0]}, &slices, scratch_i, stream, &ctl[0], first_knobs)))
         return st;
     if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{0, &ctl[0]->total}, a->dims[1],
                            CsrOut{z->j_ptr, z->j_idx, nullptr, nullptr, word[1], ctl[0]}, &fibres, scratch_j, stream, &ctl[1])))
@@ -464,6 +465,19 @@ int nb200_csf_add_f32_into(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 
 
 int nb200_inner_prod_f32(const nb200_csf3 *a, const nb200_csf3 *b, float *z, void *stream) {
     return csf_inner_run(a, b, z, stream);
+}
+
+int nb200_selftest_levels_timeout(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, int64_t cap_i, int64_t cap_j, int64_t cap_k,
+                                  int32_t polls, void *stream) {
+    int st;
+    if ((st = check_csf3(a)) || (st = check_csf3(b))) return st;
+    if ((int64_t)a->n_i + b->n_i < SELFTEST_ENTRIES) return NB200_E_BADARG;
+    if (polls < 1 || !z || cap_i < (int64_t)a->n_i + b->n_i || cap_j < (int64_t)a->n_j + b->n_j || cap_k < (int64_t)a->n_k + b->n_k) return NB200_E_BADARG;
+    LaunchKnobs knobs;
+    knobs.first_tile = 1;
+    knobs.poll_limit = polls;
+    bool done;
+    return csf_add_levels(a, b, z, static_cast<cudaStream_t>(stream), &done, knobs);
 }
 
 }  // extern "C"

@@ -32,7 +32,8 @@ struct CsrOut {
     long long *result = nullptr;
     // Calls that wait for their length: the result word in pinned host memory that the last tile writes.
     unsigned long long *host = nullptr;
-    // ... and a control block of an earlier launch whose status and hollow flag the word reports too.
+    // ... and the control block of the earlier merge that this one builds on: the word reports its status and hollow flag
+    // too, and where it gave up nothing that it should have left is read.
     const FusedCtl *earlier = nullptr;
 };
 
@@ -79,11 +80,20 @@ struct RowCount {
 
 constexpr long long RW_HOLLOW = 1ll << 48;  // beside the length in a result word: the hollow flag of this or an earlier launch
 
+// Test knobs of a launch: the first tile to run (the self-test of the bounded waits leaves tile 0
+// out, so that every other tile waits for a count that never comes) and the number of polls after
+// which a look-back gives up.
+struct LaunchKnobs {
+    int first_tile = 0;
+    int poll_limit = LOOKBACK_POLL_LIMIT;
+};
+constexpr int64_t SELFTEST_ENTRIES = 24000;  // three tiles, of whatever size: enough for one to be left out
+
 // One single-pass merge as part of a longer call: the partition and the tile kernel are queued and nothing
 // is waited for. `scratch` holds csr2_scratch_bytes(entries) bytes; the control block (length, status) that
 // *ctl then points to lies in it. With `levels` the offsets mode runs (values are not read).
 size_t csr2_scratch_bytes(int64_t entries);
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
-                 void *scratch, cudaStream_t stream, FusedCtl **ctl);
+                 void *scratch, cudaStream_t stream, FusedCtl **ctl, const LaunchKnobs &knobs = LaunchKnobs());
 
 }  // namespace nb200

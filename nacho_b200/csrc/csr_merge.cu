@@ -50,6 +50,9 @@ __device__ __forceinline__ void publish_timeout(long long *result) {
     if (result) atomicMax(result + 1, (long long)NB200_E_TIMEOUT);
 }
 
+// Whether an earlier launch on the stream, whose results a kernel builds on, ended without them.
+__device__ __forceinline__ bool gave_up(const FusedCtl *earlier) { return earlier && earlier->status.error != 0; }
+
 // All counts are in: the result length (negative after a give-up) goes to the control block and to
 // whoever waits for it. A tile that gave up wrote the error word before the count that let its
 // successors through, so the status read here covers every tile.
@@ -67,7 +70,7 @@ __device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, lon
     }
     long long value = total < 0 ? 0 : total;
     if (Z.earlier) {  // complete since before this launch; handed on, so that the last launch of a chain reports all of it
-        if (Z.earlier->status.error != 0) {
+        if (gave_up(Z.earlier)) {
             status = NB200_E_TIMEOUT;
             ctl->status = Z.earlier->status;
         }
@@ -85,11 +88,14 @@ __device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, lon
 template <int G>
 __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count,
                                                        int32_t tile_step, int32_t num_tiles, Cuts cuts, long long *result,
-                                                       uint64_t *zero_block, int zero_words) {
+                                                       uint64_t *zero_block, int zero_words, const FusedCtl *earlier) {
     wait_for_previous();   // the scratch that is cleared below may still be in use
     trigger_dependents();  // the tile kernel may take its places; it waits for the cuts
     const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
     const int32_t rows = row_count.get();
+    // The merge in front of this one gave up: its offsets and columns are whatever the scratch held. No offset is
+    // followed, and every tile is empty; the tile kernel hands the status on.
+    const bool failed = gave_up(earlier);
     const uint32_t total = (uint32_t)A.entries() + (uint32_t)B.entries();  // may be less than the tiles cover
     if (result && gid == 0) {  // the tile kernel that follows fills in the rest
         result[1] = NB200_OK;
@@ -101,7 +107,7 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
     const int t = (int)min(gid / G, (int64_t)num_tiles);  // spare groups repeat the last cut
     const int32_t a_base = row_offset(A, 0), b_base = row_offset(B, 0);
     const uint32_t d = (uint32_t)min((int64_t)t * tile_step, (int64_t)total);
-    const bool inner = t > 0 && t < num_tiles && d < total;
+    const bool inner = t > 0 && t < num_tiles && d < total && !failed;
     // Row holding merged position d: the largest i with work(i) <= d, where work(i) is the number of
     // entries of A and B in rows before i; work(0) = 0, so it is the number of rows i >= 1 that satisfy it.
     const int32_t row = (int32_t)group_count_true<G>(1, inner ? (uint32_t)rows : 1u, [&](uint32_t i) {
@@ -122,7 +128,8 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
         if (x > 0 && y < len_b && ld_late(A.col + a_lo + x - 1) == ld_late(B.col + b_lo + y)) ++y;
     }
     if ((threadIdx.x & (G - 1)) == 0 && gid / G <= num_tiles) {
-        cuts[t] = inner ? make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0)
+        cuts[t] = failed ? make_int4(0, 0, 0, 0)
+                : inner ? make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0)
                         : t == 0 ? make_int4(0, a_base, b_base, 0) : make_int4(rows, a_base + A.entries(), b_base + B.entries(), 0);
     }
 }
@@ -688,9 +695,9 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     } else {
         const int32_t rows = row_count.get();
         tile = TileRange{0, rows, row_offset(A, 0), row_offset(B, 0), A.entries(), B.entries()};
+        if (gave_up(Z.earlier)) tile = TileRange{0, 0, 0, 0, 0, 0};
         if (threadIdx.x == 0) {  // what the partition kernel does otherwise
-            ctl->status = DeviceStatus{0, 0};
-            ctl->hollow = 0;
+            *ctl = FusedCtl{};
             if (Z.result) Z.result[1] = NB200_OK, Z.result[2] = rows;
         }
         __syncthreads();
@@ -733,14 +740,6 @@ cudaError_t configure_tile_kernel() {
     return cudaSuccess;
 }
 
-// Test knobs of a launch: the first tile to run (the self-test of the bounded waits leaves tile 0
-// out, so that every other tile waits for a count that never comes) and the number of polls after
-// which a look-back gives up.
-struct LaunchKnobs {
-    int first_tile = 0;
-    int poll_limit = LOOKBACK_POLL_LIMIT;
-};
-
 // Launches the tile kernel so that it may take its places while the kernel before it on the stream (the
 // partition) still runs; it waits for that kernel's results itself.
 template <int V, int OP, int MODE, bool LEVELS = false>
@@ -770,11 +769,11 @@ cudaError_t launch_tile(const CsrIn &A, const CsrIn &B, const RowCount &rows, co
 // Eight lanes per cut once a full warp per cut would need more than one wave of the chip: the searches
 // then run a few dependent loads longer, but four times fewer warps issue them.
 cudaError_t launch_partition(const CsrIn &A, const CsrIn &B, const RowCount &rows, int num_tiles, int step, const Cuts &cuts,
-                             long long *result, uint64_t *zero_block, int zero_words, cudaStream_t stream) {
+                             long long *result, uint64_t *zero_block, int zero_words, cudaStream_t stream, const FusedCtl *earlier = nullptr) {
     const int64_t lanes = num_tiles < 8192 ? 32 : 8;
     const int blocks = (int)(((int64_t)(num_tiles + 1) * lanes + NT - 1) / NT);
     return launch_overlapped(lanes == 32 ? k_csr2_partition<32> : k_csr2_partition<8>, dim3(blocks), dim3(NT), 0, stream, A, B, rows, step, num_tiles, cuts,
-                             result, zero_block, zero_words);
+                             result, zero_block, zero_words, earlier);
 }
 
 // Shared driver of add and multiply. When `alloc` is set the result arrays are allocated
@@ -1038,7 +1037,7 @@ size_t csr2_scratch_bytes(int64_t entries) {
 }
 
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
-                 void *scratch, cudaStream_t stream, FusedCtl **ctl_out) {
+                 void *scratch, cudaStream_t stream, FusedCtl **ctl_out, const LaunchKnobs &knobs) {
     const int64_t total = (int64_t)A.nnz + B.nnz;
     const int v = tile_v(total) == V_SMALL ? V_SMALL : levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE, step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
@@ -1053,21 +1052,21 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
         cuts = nullptr;
     } else {
         LaunchScope scope("csr2_partition", stream);
-        e = launch_partition(A, B, rows, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream);
+        e = launch_partition(A, B, rows, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream, Z.earlier);
     }
     if (e != cudaSuccess) return note_cuda_error(e, "k_csr2_partition");
     const int cbits = col_bits(cols);
     if (levels) {
         LaunchScope scope("csr_levels_fused", stream);
-        e = v == V_LEVELS ? launch_tile_v<V_LEVELS, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels)
-                          : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs(), *levels);
+        e = v == V_LEVELS ? launch_tile_v<V_LEVELS, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, knobs, *levels)
+                          : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED, true>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, knobs, *levels);
     } else if (v == V_FIBRES) {
         LaunchScope scope("csr_add_fused", stream);
-        e = launch_tile_v<V_FIBRES, OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs());
+        e = launch_tile_v<V_FIBRES, OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, stream, knobs);
     } else if (op == OP_UNION) {
-        e = launch_tile<OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream);
+        e = launch_tile<OP_UNION, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream, knobs);
     } else {
-        e = launch_tile<OP_INTERSECT, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream);
+        e = launch_tile<OP_INTERSECT, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream, knobs);
     }
     return e == cudaSuccess ? NB200_OK : note_cuda_error(e, "k_csr2_tile");
 }
@@ -1083,7 +1082,7 @@ namespace {
 // waits in between. A kernel that merged three operands in one pass, in two stages per tile, took 2.0 ms where
 // this takes 1.17 (three times 67 M entries), although it moves 1.6 GB less.
 int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, bool alloc,
-                 int64_t capacity, void *stream_v) {
+                 int64_t capacity, void *stream_v, const LaunchKnobs &first_knobs = LaunchKnobs()) {
     int st;
     if ((st = check_csr(a, true)) || (st = check_csr(b, true)) || (st = check_csr(c, true))) return st;
     if (!z || a->rows != b->rows || a->cols != b->cols || a->rows != c->rows || a->cols != c->cols) return NB200_E_BADARG;
@@ -1113,7 +1112,7 @@ int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb2
     unsigned long long *word = result_word(ws, 0);
     FusedCtl *first = nullptr, *second = nullptr;
     if ((st = csr2_enqueue(OP_UNION, CsrIn{a->row_ptr, a->col, a->val, a->nnz}, CsrIn{b->row_ptr, b->col, b->val, b->nnz}, RowCount{a->rows}, a->cols,
-                           CsrOut{t.row_ptr, t.col, t.val}, nullptr, scratch, stream, &first)))
+                           CsrOut{t.row_ptr, t.col, t.val}, nullptr, scratch, stream, &first, first_knobs)))
         return st;
     if ((st = csr2_enqueue(OP_UNION, CsrIn{t.row_ptr, t.col, t.val, (int32_t)bound, &first->total}, CsrIn{c->row_ptr, c->col, c->val, c->nnz},
                            RowCount{a->rows}, a->cols, CsrOut{z->row_ptr, z->col, z->val, nullptr, word, first}, nullptr, scratch + first_bytes, stream,
@@ -1192,6 +1191,15 @@ int nb200_selftest_lookback_timeout(const nb200_csr *a, const nb200_csr *b, nb20
     knobs.first_tile = 1;
     knobs.poll_limit = polls;
     return csr2_run<OP_UNION>(a, b, z, false, capacity, stream, nullptr, knobs);
+}
+
+int nb200_selftest_chain_timeout(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, int64_t capacity, int32_t polls,
+                                 void *stream) {
+    if (polls < 1 || !a || !b || !c || capacity < (int64_t)a->nnz + b->nnz + c->nnz || (int64_t)a->nnz + b->nnz < SELFTEST_ENTRIES) return NB200_E_BADARG;
+    LaunchKnobs knobs;
+    knobs.first_tile = 1;
+    knobs.poll_limit = polls;
+    return csr_add3_run(a, b, c, z, false, capacity, stream, knobs);
 }
 
 }  // extern "C"

@@ -48,3 +48,63 @@ def test_product_of_a_fresh_sum(nacho, oracle):
         z = csr_from_gpu(m)
         assert np.array_equal(key(z), common)
         assert np.all(np.abs(z.val - v64[i_f] * s.val[i_s].astype(np.float64)) <= 1e-5 * abs64[i_f] * np.abs(s.val[i_s]) + 1e-30)
+
+
+@pytest.mark.parametrize("total", [24_000, 700_000, 6_100_000])
+def test_a_merge_that_gives_up_ends_its_chain(nacho, oracle, total):
+    """A three-operand add whose first union runs without its first tile, with few and with many tiles: the second
+    union follows none of its offsets, which are what the scratch held, and so writes no row; the call reports the wait,
+    and the same call works afterwards."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import CsrStruct, lib
+    rng = np.random.default_rng(total)
+    rows, cols = total // 9, 30000
+    ka, kb = key_pair(total, rows * cols, 0.2, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    cap = 2 * len(a.col) + len(b.col)
+    want = oracle.csr_add_3(a, b, a, 8)
+    for _ in range(2):
+        assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, ga)), want, "add_3")
+        rp = torch.full((rows + 1,), -1, dtype=torch.int32, device="cuda")
+        col = torch.empty(cap, dtype=torch.int32, device="cuda")
+        val = torch.empty(cap, dtype=torch.float32, device="cuda")
+        z = CsrStruct(rows, cols, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr())
+        sa, sb = ga._struct(), gb._struct()
+        status = lib.nb200_selftest_chain_timeout(C.byref(sa), C.byref(sb), C.byref(sa), C.byref(z), cap, 50, None)
+        torch.cuda.synchronize()
+        assert status == _capi.E_TIMEOUT and "look-back" in lib.nb200_last_cuda_error().decode()
+        assert bool((rp[1:] == -1).all())
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, ga)), want, "add_3 after a give-up")
+    sa.nnz = 10
+    assert lib.nb200_selftest_chain_timeout(C.byref(sa), C.byref(sa), C.byref(sa), C.byref(z), cap, 50, None) == _capi.E_BADARG
+
+
+def test_levels_behind_one_that_gave_up(nacho, oracle):
+    """A CSF3 add whose slice lists give up: neither the fibres nor the entries are merged, and the call says why."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import Csf3Struct, lib
+    from helpers import csf3_levels
+    from oracle.cpu_oracle import CSF3
+    from test_tensor3_gpu import _seeded, csf3_from_gpu
+    dims = (60_000, 500, 400)
+    (ca, va), (cb, vb) = _seeded(dims, 90_000, 5)
+    ga, gb = nacho.to_csf3(ca, va, dims, "cuda"), nacho.to_csf3(cb, vb, dims, "cuda")
+    want = oracle.csf3_add(CSF3(dims, *csf3_levels(ca), va), CSF3(dims, *csf3_levels(cb), vb))
+    n_i, n_j, n_k = (len(getattr(ga, f)) + len(getattr(gb, f)) for f in ("dim_i_indices", "dim_j_indices", "dim_k_indices"))
+    assert n_i >= 24_000
+    for _ in range(2):
+        assert_same(csf3_from_gpu(nacho.gpu_csf_add_f32(ga, gb)), want, "csf3")
+        i, jp, j, kp, k = (torch.full((n,), -1, dtype=torch.int32, device="cuda") for n in (n_i, n_i + 1, n_j, n_j + 1, n_k))
+        v = torch.empty(n_k, dtype=torch.float32, device="cuda")
+        z = Csf3Struct((C.c_int32 * 3)(), 0, 0, 0, *(t.data_ptr() for t in (i, jp, j, kp, k, v)))
+        sa, sb = ga._struct(), gb._struct()
+        status = lib.nb200_selftest_levels_timeout(C.byref(sa), C.byref(sb), C.byref(z), n_i, n_j, n_k, 50, None)
+        torch.cuda.synchronize()
+        assert status == _capi.E_TIMEOUT and "look-back" in lib.nb200_last_cuda_error().decode()
+        assert bool((jp[1:] == -1).all()) and bool((kp[1:] == -1).all()) and bool((k == -1).all())
+    assert_same(csf3_from_gpu(nacho.gpu_csf_add_f32(ga, gb)), want, "csf3 after a give-up")
