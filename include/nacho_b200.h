@@ -333,7 +333,12 @@ int nb200_inner_prod_coo_f32(const nb200_coo3 *a, const nb200_coo3 *b, float *z,
 int nb200_selftest_lookback_timeout(const nb200_csr *a, const nb200_csr *b, nb200_csr *z,
                                     int64_t capacity, int32_t polls, void *stream);
 
-/* The same for calls that queue several merges, each of which reads the one before it on the device: the FIRST merge
+/* A give-up that comes late: all tiles run, but a tile waits for its output base for `polls` polls only, while the
+ * counts it depends on do arrive. Returns NB200_E_TIMEOUT, or NB200_OK with a result that is whole. */
+int nb200_selftest_late_give_up(const nb200_csr *a, const nb200_csr *b, nb200_csr *z,
+                                int64_t capacity, int32_t polls, void *stream);
+
+/* For calls that queue several merges, each of which reads the one before it on the device: the FIRST merge
  * of a three-operand add, and of a CSF3 add level by level, runs without its first tile and gives up. The merges behind
  * it must read none of its results and the call must return NB200_E_TIMEOUT. Needs 24000 entries in A and B (of
  * the CSF3 tensors: slices); capacities of the worst case. */

@@ -68,6 +68,7 @@ PROTOTYPES = {
     "nb200_csr_add_f32_async": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64, C.c_void_p, C.c_void_p]),
     "nb200_csr_mul_f32_async": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64, C.c_void_p, C.c_void_p]),
     "nb200_selftest_lookback_timeout": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64, C.c_int32, C.c_void_p]),
+    "nb200_selftest_late_give_up": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64, C.c_int32, C.c_void_p]),
     "nb200_selftest_chain_timeout": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_int32, C.c_void_p]),
     "nb200_selftest_levels_timeout": (C.c_int, [_P(Csf3Struct)] * 3 + [C.c_int64] * 3 + [C.c_int32, C.c_void_p]),
     "nb200_csr_mul_f32": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int32, C.c_int32, C.c_void_p]),

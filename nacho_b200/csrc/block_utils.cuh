@@ -111,11 +111,14 @@ __device__ __forceinline__ uint32_t group_count_true(uint32_t lo, uint32_t hi, P
 // an order in which their CTAs start: the CTA index (the hardware hands CTAs out in index
 // order, the numbering the kernels here use) or an atomic ticket taken at CTA start.
 //
-// Every wait is bounded: after LOOKBACK_POLL_LIMIT polls of one word the walk gives up,
-// records the tile in `status` and returns -1; the caller then skips its writes. The tile
-// still publishes a prefix so that its successors do not wait on it in turn.
+// Every wait is bounded: after LOOKBACK_POLL_LIMIT polls the walk gives up, records the tile in `status` and
+// returns -1; the caller then skips its writes. A give-up is never lost, however late it comes: the waiter puts
+// LB_FAILED in the place of the word it misses (unless that word has come after all), a word is first published only
+// in the place of zero, and so no tile behind the missing word gets a base, the last one among them, which is the
+// one that publishes the total.
 constexpr uint64_t LB_AGGREGATE = 1ull << 62;
 constexpr uint64_t LB_PREFIX = 2ull << 62;
+constexpr uint64_t LB_FAILED = 3ull << 62;
 constexpr uint64_t LB_VALUE_MASK = (1ull << 62) - 1;
 constexpr int LOOKBACK_POLL_LIMIT = 1 << 22;
 constexpr int ERR_LOOKBACK_TIMEOUT = 1;
@@ -136,10 +139,15 @@ __device__ __forceinline__ int ld_relaxed_gpu_i32(const int *p) {
     return v;
 }
 
+// Writes `v` into a word that is still zero; returns what the word held.
+__device__ __forceinline__ uint64_t set_if_zero(volatile uint64_t *word, uint64_t v) {
+    return atomicCAS(reinterpret_cast<unsigned long long *>(const_cast<uint64_t *>(word)), 0ull, (unsigned long long)v);
+}
+
 // Sum of the counts of tiles [0, t), read off the tile words of the predecessors, 32 at a time
 // from the nearest one backwards; publishes nothing. A round is complete once every word up to
 // the nearest tile that already knows its prefix is published (the words beyond it are not
-// needed). Returns -1 (and records the tile in `status`) if a bounded wait gives up. Called by
+// needed). Returns -1 (and records the tile in `status`) if a bounded wait gives up, here or on the way. Called by
 // all 32 lanes of one warp, t > 0.
 __device__ __forceinline__ int64_t lookback_predecessors(volatile uint64_t *state, int t, DeviceStatus *status) {
     int64_t exclusive = 0;
@@ -154,10 +162,19 @@ __device__ __forceinline__ int64_t lookback_predecessors(volatile uint64_t *stat
             need = prefixes ? FULL_MASK >> (32 - __ffs(prefixes)) : FULL_MASK;
             if ((published & need) == need) break;
             if (polls >= LOOKBACK_POLL_LIMIT) {
-                if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
-                return -1;
+                if (s == 0 && ((need >> lane_id()) & 1u)) {
+                    s = set_if_zero(state + idx, LB_FAILED);
+                    if (s == 0) s = LB_FAILED;
+                }
+                prefixes = __ballot_sync(FULL_MASK, (s >> 62) == 2);
+                need = prefixes ? FULL_MASK >> (32 - __ffs(prefixes)) : FULL_MASK;
+                break;
             }
             __nanosleep(32);
+        }
+        if (__ballot_sync(FULL_MASK, s >= LB_FAILED) & need) {
+            if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
+            return -1;
         }
         long long v = (need >> lane_id()) & 1u ? (long long)(s & LB_VALUE_MASK) : 0;
 #pragma unroll
@@ -168,15 +185,15 @@ __device__ __forceinline__ int64_t lookback_predecessors(volatile uint64_t *stat
 }
 
 // Publishes the tile's count, walks back, publishes the inclusive prefix. Returns the sum of the
-// counts of tiles [0, t), or -1 after a give-up (the tile then still publishes a prefix so that
-// its successors do not wait on it). Called by all 32 lanes of one warp.
+// counts of tiles [0, t), or -1 after a give-up. Called by all 32 lanes of one warp.
 __device__ __forceinline__ int64_t lookback_exclusive(volatile uint64_t *state, int t, int64_t aggregate,
                                                       DeviceStatus *status) {
-    if (lane_id() == 0) st_relaxed_gpu(state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)aggregate);
+    uint64_t before = 0;  // not zero: some tile has given up on this one
+    if (lane_id() == 0) before = set_if_zero(state + t, (t == 0 ? LB_PREFIX : LB_AGGREGATE) | (uint64_t)aggregate);
     if (t == 0) return 0;
     const int64_t exclusive = lookback_predecessors(state, t, status);
-    if (exclusive < 0) __threadfence();  // the error word goes out before the word that lets the successors through
-    if (lane_id() == 0) st_relaxed_gpu(state + t, LB_PREFIX | (uint64_t)(exclusive < 0 ? 0 : exclusive + aggregate));
+    if (exclusive < 0) __threadfence();  // the error word goes out before the word that tells the successors
+    if (lane_id() == 0 && before == 0) st_relaxed_gpu(state + t, exclusive < 0 ? LB_FAILED : LB_PREFIX | (uint64_t)(exclusive + aggregate));
     return exclusive;
 }
 

@@ -80,9 +80,9 @@ struct RowCount {
 
 constexpr long long RW_HOLLOW = 1ll << 48;  // beside the length in a result word: the hollow flag of this or an earlier launch
 
-// Test knobs of a launch: the first tile to run (the self-test of the bounded waits leaves tile 0
+// Test knobs of a launch: the first tile to run (a self-test of the bounded waits leaves tile 0
 // out, so that every other tile waits for a count that never comes) and the number of polls after
-// which a look-back gives up.
+// which a tile gives up on its output base; where tile 0 is left out, the CTA that hands out the bases too.
 struct LaunchKnobs {
     int first_tile = 0;
     int poll_limit = LOOKBACK_POLL_LIMIT;

@@ -54,8 +54,8 @@ __device__ __forceinline__ void publish_timeout(long long *result) {
 __device__ __forceinline__ bool gave_up(const FusedCtl *earlier) { return earlier && earlier->status.error != 0; }
 
 // All counts are in: the result length (negative after a give-up) goes to the control block and to
-// whoever waits for it. A tile that gave up wrote the error word before the count that let its
-// successors through, so the status read here covers every tile.
+// whoever waits for it. The status read here covers every tile: one whose columns did not land wrote it before its
+// count, and one that gives up on its base later than this finds that base there after all (merge_common.cuh).
 __device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, long long total, bool alone = false) {
     int status = NB200_OK;
     if (!alone) {  // a single tile has nobody's status to look at
@@ -679,14 +679,14 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
     if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
         if (threadIdx.x < 32) {
-            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, poll_limit);
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, first_tile ? poll_limit : LOOKBACK_POLL_LIMIT);
             if (threadIdx.x == 0) finish_total(ctl, Z, total);
         }
         return;
     }
     // Tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
     // only ever waits on CTAs that were dispatched before it (and every such wait is bounded).
-    // first_tile is 0 except in the self-test of the bounded waits, which leaves tile 0 out.
+    // first_tile is 0 except in the self-tests that leave tile 0 out; poll_limit is smaller in all self-tests.
     const int t = blockIdx.x + first_tile - (scanned ? 1 : 0);
     TileRange tile;
     if (cuts) {
@@ -1200,6 +1200,13 @@ int nb200_selftest_chain_timeout(const nb200_csr *a, const nb200_csr *b, const n
     knobs.first_tile = 1;
     knobs.poll_limit = polls;
     return csr_add3_run(a, b, c, z, false, capacity, stream, knobs);
+}
+
+int nb200_selftest_late_give_up(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_t capacity, int32_t polls, void *stream) {
+    if (polls < 1 || !a || !b || capacity < (int64_t)a->nnz + b->nnz) return NB200_E_BADARG;
+    LaunchKnobs knobs;
+    knobs.poll_limit = polls;
+    return csr2_run<OP_UNION>(a, b, z, false, capacity, stream, nullptr, knobs);
 }
 
 }  // extern "C"

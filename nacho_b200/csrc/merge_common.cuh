@@ -35,8 +35,12 @@ struct FusedCtl {
 // counts back 32 at a time 609 us, per-group sums that every tile reads in one round 519 us, this 470 us.
 // Up to DIRECT_TILES tiles, when everything is resident and little is polled, a tile adds up the counts
 // before it itself, one hop less.
+//
+// Whoever publishes the length (CTA 0, or the last tile) has read every count, and reads the status behind a fence
+// after that. A tile that gives up writes the status, and behind a fence looks at the word it misses once more: it is
+// still missing only if the publisher's look at the status is yet to come. So a length goes out as good only if
+// every tile has, or will find, its base.
 constexpr int DIRECT_TILES = 128;
-constexpr uint64_t LB_FAILED = 3ull << 62;
 
 // Words of one launch, zero at the start: a count and a base per tile.
 struct TileWords {
@@ -68,7 +72,10 @@ __device__ __forceinline__ int64_t scan_tile_counts(const TileWords &words, cons
             if (lane < n) st_relaxed_gpu(words.base + pos + lane, LB_PREFIX | (uint64_t)(run + incl - v));
             run += __shfl_sync(FULL_MASK, incl, 31);
             idle = 0;
-            if (next >= num_tiles) return run;
+            if (next >= num_tiles) {
+                __syncwarp();  // the bases of all lanes lie before the fence of the one that publishes the length
+                return run;
+            }
         } else if (++idle > poll_limit) {
             if (lane == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = pos;
             __threadfence();
@@ -83,6 +90,11 @@ __device__ __forceinline__ int64_t scan_tile_counts(const TileWords &words, cons
 // Output base of tile t, or -1 after a give-up. Called by all 32 lanes of one warp.
 __device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t, const int num_tiles, DeviceStatus *status, const int poll_limit) {
     if (t == 0) return 0;
+    auto record = [&]() {
+        if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
+        __syncwarp();
+        __threadfence();
+    };
     uint64_t w = LB_AGGREGATE;  // lanes past the last predecessor add nothing
     if (num_tiles <= DIRECT_TILES) {
         int sum = 0;
@@ -93,25 +105,30 @@ __device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t
                 if (at < t) w = ld_relaxed_gpu(words.count + at);
                 if (__all_sync(FULL_MASK, (w >> 62) != 0)) break;
                 if (polls >= poll_limit) {
-                    if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
-                    __threadfence();
+                    record();
+                    if (at < t) w = ld_relaxed_gpu(words.count + at);
+                    if (__all_sync(FULL_MASK, (w >> 62) != 0)) break;
                     return -1;
                 }
             }
             sum += (int)(w & LB_VALUE_MASK);
         }
+        __syncwarp();  // every lane's look at the counts lies before the fence of the one that publishes the length
         return __reduce_add_sync(FULL_MASK, sum);
     }
-    for (int polls = 0; polls <= poll_limit; ++polls) {
+    for (int polls = 0;; ++polls) {
         if (lane_id() == 0) w = ld_relaxed_gpu(words.base + t);
         w = __shfl_sync(FULL_MASK, w, 0);
         if (w >> 62) break;
+        if (polls >= poll_limit) {
+            record();
+            if (lane_id() == 0) w = ld_relaxed_gpu(words.base + t);
+            w = __shfl_sync(FULL_MASK, w, 0);
+            break;
+        }
         __nanosleep(64);
     }
-    if ((w >> 62) == 2) return (int64_t)(w & LB_VALUE_MASK);
-    if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
-    __threadfence();
-    return -1;
+    return (w >> 62) == 2 ? (int64_t)(w & LB_VALUE_MASK) : -1;
 }
 
 // Exclusive prefix of the per-tile counts, in place, by one CTA; the grand total goes to

@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 from helpers import assert_same, csr_from_gpu, csr_to_gpu
+from oracle.cpu_oracle import CSR
 from test_tile_edges_gpu import csr_of_keys, key_pair, nacho  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -108,3 +109,36 @@ def test_levels_behind_one_that_gave_up(nacho, oracle):
         assert status == _capi.E_TIMEOUT and "look-back" in lib.nb200_last_cuda_error().decode()
         assert bool((jp[1:] == -1).all()) and bool((kp[1:] == -1).all()) and bool((k == -1).all())
     assert_same(csf3_from_gpu(nacho.gpu_csf_add_f32(ga, gb)), want, "csf3 after a give-up")
+
+
+@pytest.mark.parametrize("total", [24_000, 400_000, 1_500_000, 6_100_000])
+def test_a_late_give_up_is_reported(nacho, oracle, total):
+    """A first tile that takes a millisecond, for the two million empty rows it begins with, and others that wait for its
+    count for some polls only: a call either says that they gave up or its result is whole. Few tiles that add up the
+    counts themselves, many that are handed their base."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import CsrStruct, lib
+    rng = np.random.default_rng(total)
+    empty, cols = 2_000_000, 30000
+    rows = empty + total // 9
+    ka, kb = key_pair(total, (total // 9) * cols, 0.2, rng)
+    a, b = csr_of_keys(ka + empty * cols, rows, cols, rng), csr_of_keys(kb + empty * cols, rows, cols, rng)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    want = oracle.csr_add(a, b, 8)
+    seen = []
+    for polls in [1, 8, 64, 200, 500, 1000, 1500, 2000, 1 << 20]:
+        rp = torch.full((rows + 1,), -1, dtype=torch.int32, device="cuda")
+        col = torch.full((total,), -1, dtype=torch.int32, device="cuda")
+        val = torch.full((total,), float("nan"), dtype=torch.float32, device="cuda")
+        z = CsrStruct(rows, cols, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr())
+        sa, sb = ga._struct(), gb._struct()
+        status = lib.nb200_selftest_late_give_up(C.byref(sa), C.byref(sb), C.byref(z), total, polls, None)
+        torch.cuda.synchronize()
+        assert status in (_capi.OK, _capi.E_TIMEOUT)
+        seen.append(status)
+        if status == _capi.OK:
+            assert_same(CSR(rows, cols, rp.cpu().numpy(), col[:z.nnz].cpu().numpy(), val[:z.nnz].cpu().numpy()), want, f"{polls} polls")
+    assert seen[0] == _capi.E_TIMEOUT and seen[-1] == _capi.OK, seen
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), want, "add after a give-up")
