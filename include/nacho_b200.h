@@ -246,11 +246,19 @@ int nb200_spgemm_f32_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr 
 int nb200_spgemm_f32_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c,
                              void *stream);
 
-/* One-call form for caller-owned memory. _bound bins the rows and sets *capacity to the number of entries of
- * col / val with which _into runs in one pass, or to 0 where it has to count first (any but matrices of
- * short rows: at most 8 entries in a row of A and 32 products). _into takes any capacity that holds the
- * result (less returns NB200_E_CAPACITY with c->nnz filled in); right after _bound on the same arrays and
- * stream it, or a _symbolic call, does not bin the rows again. */
+/* One-call forms for caller-owned memory.
+ *
+ * _with asks for the result's arrays when it knows how many entries they need: `take(ctx, entries, &col, &val)` is called
+ * once (not at all for an empty result) on the calling thread, hands out two arrays of that many entries that
+ * may be used on `stream`, and returns NB200_OK, or a status with which the call then ends. It must not throw, nor call
+ * this library on `stream`. c->row_ptr is the caller's; c->col / c->val are set to the arrays taken, of which the
+ * first c->nnz entries are in use. Matrices of short rows (at most 8 entries in a row of A and 32 products) are
+ * multiplied in one pass into an entry per product, any other into nnz(C) entries.
+ *
+ * _into takes any capacity that holds the result (less returns NB200_E_CAPACITY with c->nnz filled in). _bound sets
+ * *capacity to the number of entries with which _into runs in one pass, or to 0 where it has to count first. */
+typedef int (*nb200_take_fn)(void *ctx, int64_t entries, int32_t **col, float **val);
+int nb200_spgemm_f32_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take_fn take, void *ctx, void *stream);
 int nb200_spgemm_f32_bound(const nb200_csr *a, const nb200_csr *b, int64_t *capacity, void *stream);
 int nb200_spgemm_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t capacity, void *stream);
 

@@ -51,6 +51,9 @@ OK, E_BADARG, E_CUDA, E_OVERFLOW, E_CAPACITY, E_TIMEOUT, E_NOMEM, E_UNSUPPORTED 
 
 # name -> (restype, argtypes); every symbol include/nacho_b200.h declares.
 _P = C.POINTER
+# nb200_take_fn: (ctx, entries, &col, &val) -> status
+TakeFn = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_int64, _P(C.c_void_p), _P(C.c_void_p))
+
 PROTOTYPES = {
     "nb200_version": (C.c_int, []),
     "nb200_strerror": (C.c_char_p, [C.c_int]),
@@ -79,6 +82,7 @@ PROTOTYPES = {
     "nb200_csr_add_3_f32_into": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_void_p]),
     "nb200_spgemm_f32": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int32, C.c_int32, C.c_void_p]),
     "nb200_sssmm_f32_into": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_void_p]),
+    "nb200_spgemm_f32_with": (C.c_int, [_P(CsrStruct)] * 3 + [TakeFn, C.c_void_p, C.c_void_p]),
     "nb200_spgemm_f32_bound": (C.c_int, [_P(CsrStruct)] * 2 + [_P(C.c_int64), C.c_void_p]),
     "nb200_spgemm_f32_into": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64, C.c_void_p]),
     "nb200_spgemm_f32_symbolic": (C.c_int, [_P(CsrStruct)] * 3 + [_P(C.c_int64), C.c_void_p]),

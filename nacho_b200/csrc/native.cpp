@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <exception>
 #include <mutex>
 
 #include "nacho_b200.h"
@@ -188,7 +189,7 @@ std::mutex &stream_lock(void *stream) {
 // returns when the result's length is known, with kernels still running: the allocator is told that the
 // operands' arrays are in use on this stream, which matters when they came from another one.
 template <size_t N, typename F>
-void launch(const View *const (&operands)[N], const char *where, F call) {
+int run(const View *const (&operands)[N], F call) {
     const c10::Device device = operands[0]->device;
     c10::cuda::CUDAGuard guard(device);
     const c10::cuda::CUDAStream current = c10::cuda::getCurrentCUDAStream(device.index());
@@ -201,7 +202,12 @@ void launch(const View *const (&operands)[N], const char *where, F call) {
     }
     for (const View *operand : operands)
         for (int k = 0; k < operand->n; ++k) c10::cuda::CUDACachingAllocator::recordStream(operand->arrays[k].storage().data_ptr(), current);
-    check(status, where);
+    return status;
+}
+
+template <size_t N, typename F>
+void launch(const View *const (&operands)[N], const char *where, F call) {
+    check(run(operands, call), where);
 }
 
 // ---- operators -----------------------------------------------------------------------------
@@ -277,23 +283,29 @@ PyObject *spgemm(PyObject *const *args) {
     View va, vb;
     const nb200_csr a = view_csr(args[0], va), b = view_csr(args[1], vb);
     same_device(va, vb);
-    at::Tensor rp = int_array((int64_t)a.rows + 1, va.device), col, val;
+    at::Tensor rp = int_array((int64_t)a.rows + 1, va.device);
     nb200_csr c{a.rows, b.cols, 0, ints(rp), nullptr, nullptr};
-    launch({&va, &vb}, where, [&](void *stream) {
-        int64_t capacity;
-        int st = nb200_spgemm_f32_bound(&a, &b, &capacity, stream);
-        if (st != NB200_OK) return st;
-        if (capacity > 0) {  // short rows: one pass, no count first
-            col = int_array(capacity, va.device), val = float_array(capacity, va.device);
-            c.col = ints(col), c.val = floats(val);
-            return nb200_spgemm_f32_into(&a, &b, &c, capacity, stream);
+    struct Taken {  // the result's arrays, taken when their length is known
+        c10::Device device;
+        at::Tensor col, val;
+        std::exception_ptr failure;
+    } taken{va.device};
+    auto take = [](void *ctx, int64_t entries, int32_t **col, float **val) noexcept -> int {
+        Taken &t = *static_cast<Taken *>(ctx);
+        try {
+            t.col = int_array(entries, t.device), t.val = float_array(entries, t.device);
+            *col = ints(t.col), *val = floats(t.val);
+            return NB200_OK;
+        } catch (...) {
+            t.failure = std::current_exception();
+            return NB200_E_NOMEM;
         }
-        st = nb200_spgemm_f32_symbolic(&a, &b, &c, nullptr, stream);
-        if (st != NB200_OK) return st;
-        col = int_array(c.nnz, va.device), val = float_array(c.nnz, va.device);
-        if (c.nnz > 0) c.col = ints(col), c.val = floats(val);
-        return nb200_spgemm_f32_numeric(&a, &b, &c, stream);
-    });
+    };
+    const int status = run({&va, &vb}, [&](void *stream) { return nb200_spgemm_f32_with(&a, &b, &c, take, &taken, stream); });
+    if (status == NB200_E_NOMEM && taken.failure) std::rethrow_exception(taken.failure);
+    check(status, where);
+    at::Tensor &col = taken.col, &val = taken.val;
+    if (!col.defined()) col = int_array(0, va.device), val = float_array(0, va.device);
     used(col, c.nnz);
     used(val, c.nnz);
     Result r(CSR);

@@ -1153,15 +1153,14 @@ struct SavedPlan {
     uint64_t gen_main = 0, gen_cache = 0, epoch = 0;
 };
 std::mutex g_saved_mutex;
-SavedPlan g_after_symbolic;  // for a numeric pass
-SavedPlan g_after_bound;     // rows are binned and the control blocks clear: for the one symbolic or one-pass call that follows
+SavedPlan g_saved;
 
-void save_plan(SavedPlan &g_saved, const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, const EscPlan &plan, cudaStream_t stream) {
+void save_plan(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, const EscPlan &plan, cudaStream_t stream) {
     std::lock_guard<std::mutex> g(g_saved_mutex);
     g_saved.valid = cudaGetDevice(&g_saved.device) == cudaSuccess;
     g_saved.plan = plan;
     g_saved.a_rp = a->row_ptr, g_saved.a_col = a->col, g_saved.b_rp = b->row_ptr, g_saved.b_col = b->col;
-    g_saved.c_rp = c ? c->row_ptr : nullptr, g_saved.c_nnz = c ? c->nnz : 0;
+    g_saved.c_rp = c->row_ptr, g_saved.c_nnz = c->nnz;
     g_saved.a_rows = a->rows, g_saved.a_nnz = a->nnz, g_saved.b_rows = b->rows, g_saved.b_cols = b->cols, g_saved.b_nnz = b->nnz;
     g_saved.stream = stream;
     g_saved.epoch = workspace_epoch();
@@ -1169,42 +1168,38 @@ void save_plan(SavedPlan &g_saved, const nb200_csr *a, const nb200_csr *b, const
     g_saved.gen_cache = plan.cache_ws ? plan.cache_ws->generation : 0;
 }
 
-bool take_saved_plan(SavedPlan &g_saved, const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, cudaStream_t stream, EscPlan *out) {
+bool take_saved_plan(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, cudaStream_t stream, EscPlan *out) {
     std::lock_guard<std::mutex> g(g_saved_mutex);
     int dev = -1;
     if (!g_saved.valid || g_saved.epoch != workspace_epoch()) return false;  // the pool blocks may be gone
     if (cudaGetDevice(&dev) != cudaSuccess || dev != g_saved.device || stream != g_saved.stream) return false;
     if (a->row_ptr != g_saved.a_rp || a->col != g_saved.a_col || b->row_ptr != g_saved.b_rp || b->col != g_saved.b_col) return false;
-    if (c && (c->row_ptr != g_saved.c_rp || c->nnz != g_saved.c_nnz)) return false;  // row offsets obtained elsewhere: recompute
+    if (c->row_ptr != g_saved.c_rp || c->nnz != g_saved.c_nnz) return false;  // row offsets obtained elsewhere: recompute
     if (a->rows != g_saved.a_rows || a->nnz != g_saved.a_nnz || b->rows != g_saved.b_rows || b->cols != g_saved.b_cols ||
         b->nnz != g_saved.b_nnz)
         return false;
     if (g_saved.plan.ws->generation != g_saved.gen_main) return false;
     if (g_saved.plan.cache_ws && g_saved.plan.cache_ws->generation != g_saved.gen_cache) return false;
     *out = g_saved.plan;
-    if (!c) g_saved.valid = false;  // its cleared control blocks serve one call
     return true;
 }
 
-// `keep`: if given, the plan is handed back, so that a numeric pass that follows at once
-// (nothing else touching the stream's scratch in between) skips the binning.
-int spgemm_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t *products, void *stream_v, EscPlan *keep = nullptr) {
+// What every form of the call checks first. *done is set where the product has no rows.
+int spgemm_begin(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStream_t stream, bool *done) {
     int st;
     if ((st = check_operand(a)) || (st = check_operand(b))) return st;
     if (!c || !c->row_ptr || a->cols != b->rows) return NB200_E_BADARG;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     c->rows = a->rows;
     c->cols = b->cols;
     c->nnz = 0;
-    if (products) *products = 0;
-    if (a->rows == 0) {
-        NB200_CUDA(cudaMemsetAsync(c->row_ptr, 0, sizeof(int32_t), stream));
-        return NB200_OK;
-    }
-    EscPlan plan{};
-    if (!take_saved_plan(g_after_bound, a, b, nullptr, stream, &plan) && (st = esc_prepare(a, b, true, true, stream, &plan))) return st;
-    if (keep) *keep = plan;
-    if (products) *products = (int64_t)plan.host.products;
+    *done = a->rows == 0;
+    if (*done) NB200_CUDA(cudaMemsetAsync(c->row_ptr, 0, sizeof(int32_t), stream));
+    return NB200_OK;
+}
+
+// The symbolic pass on rows that `plan` has just binned (its control blocks serve one call).
+int symbolic_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStream_t stream) {
+    int st;
     if ((st = esc_run_bins<false>(a, b, plan, nullptr, stream))) return st;
     {
         LaunchScope scope("esc_scan_offsets", stream);
@@ -1218,77 +1213,105 @@ int spgemm_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_
     if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm row scan");
     if (nnz > INT32_MAX) return NB200_E_OVERFLOW;
     c->nnz = (int32_t)nnz;
-    save_plan(g_after_symbolic, a, b, c, plan, stream);
     return NB200_OK;
 }
 
-int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *stream_v, const EscPlan *kept = nullptr) {
+int spgemm_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t *products, void *stream_v) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    bool done;
+    int st;
+    if (products) *products = 0;
+    if ((st = spgemm_begin(a, b, c, stream, &done)) || done) return st;
+    EscPlan plan{};
+    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+    if (products) *products = (int64_t)plan.host.products;
+    if ((st = symbolic_on(plan, a, b, c, stream))) return st;
+    save_plan(a, b, c, plan, stream);
+    return NB200_OK;
+}
+
+int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *stream_v) {
     int st;
     if ((st = check_operand(a)) || (st = check_operand(b))) return st;
     if (!c || !c->row_ptr || a->cols != b->rows || c->nnz < 0) return NB200_E_BADARG;
     if (c->nnz > 0 && (!c->col || !c->val)) return NB200_E_BADARG;
     if (a->rows == 0 || c->nnz == 0) return NB200_OK;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-    if (kept) return esc_run_bins<true>(a, b, *kept, c, stream);
     EscPlan plan{};
-    if (take_saved_plan(g_after_symbolic, a, b, c, stream, &plan)) return esc_run_bins<true>(a, b, plan, c, stream);
-    if ((st = esc_prepare(a, b, false, false, stream, &plan))) return st;
+    if (!take_saved_plan(a, b, c, stream, &plan) && (st = esc_prepare(a, b, false, false, stream, &plan))) return st;
     return esc_run_bins<true>(a, b, plan, c, stream);
 }
 
+// Whether the one-pass kernel can do the product. It wants room for as many entries as there are products, an upper bound of nnz(C).
 bool is_short(const EscPlan &plan) {
     return plan.host.n_rows[BIN_MEDIUM] + plan.host.n_rows[BIN_RANKED] + plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY] == 0 && plan.host.max_entries <= SHORT_ENTRIES &&
            plan.host.products > 0 && plan.host.products <= INT32_MAX;
 }
 
-// Bins the rows; *capacity receives the number of entries with which spgemm_into runs in one pass (the number
-// of products, an upper bound of nnz(C)) if the matrices are of the kind it can do that for, else 0.
+int short_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStream_t stream) {
+    const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
+    FusedCtl *ctl = reinterpret_cast<FusedCtl *>(plan.short_block);
+    const TileWords words = TileWords::at(plan.short_block + 4, plan.short_tiles);
+    auto kernel = plan.host.max_entries <= 4 ? k_esc_short<4> : plan.host.max_entries <= 6 ? k_esc_short<6> : k_esc_short<8>;
+    {
+        LaunchScope scope("esc_short", stream);
+        kernel<<<plan.short_tiles + (plan.short_tiles > DIRECT_TILES ? 1 : 0), SHORT_NT, 0, stream>>>(
+            A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.words + W_NNZ);
+        NB200_CUDA(cudaGetLastError());
+    }
+    int st;
+    int64_t nnz;
+    int device_status;
+    if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
+    if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm of short rows");
+    c->nnz = (int32_t)nnz;
+    return NB200_OK;
+}
+
 int spgemm_bound(const nb200_csr *a, const nb200_csr *b, int64_t *capacity, void *stream_v) {
     int st;
     if ((st = check_operand(a)) || (st = check_operand(b))) return st;
     if (!capacity || a->cols != b->rows) return NB200_E_BADARG;
     *capacity = 0;
     if (a->rows == 0) return NB200_OK;
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     EscPlan plan{};
-    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
-    save_plan(g_after_bound, a, b, nullptr, plan, stream);
+    if ((st = esc_prepare(a, b, false, false, static_cast<cudaStream_t>(stream_v), &plan))) return st;
     if (is_short(plan)) *capacity = (int64_t)plan.host.products;
     return NB200_OK;
 }
 
 int spgemm_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t capacity, void *stream_v) {
-    int st;
-    if ((st = check_operand(a)) || (st = check_operand(b))) return st;
-    if (!c || !c->row_ptr || a->cols != b->rows || capacity < 0 || (capacity > 0 && (!c->col || !c->val))) return NB200_E_BADARG;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    bool done;
+    int st;
+    if (!c || capacity < 0 || (capacity > 0 && (!c->col || !c->val))) return NB200_E_BADARG;
+    if ((st = spgemm_begin(a, b, c, stream, &done)) || done) return st;
     EscPlan plan{};
-    if (a->rows > 0) {
-        if (!take_saved_plan(g_after_bound, a, b, nullptr, stream, &plan) && (st = esc_prepare(a, b, true, true, stream, &plan))) return st;
-        if (is_short(plan) && capacity >= (int64_t)plan.host.products) {
-            c->rows = a->rows, c->cols = b->cols, c->nnz = 0;
-            const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
-            FusedCtl *ctl = reinterpret_cast<FusedCtl *>(plan.short_block);
-            const TileWords words = TileWords::at(plan.short_block + 4, plan.short_tiles);
-            auto kernel = plan.host.max_entries <= 4 ? k_esc_short<4> : plan.host.max_entries <= 6 ? k_esc_short<6> : k_esc_short<8>;
-            {
-                LaunchScope scope("esc_short", stream);
-                kernel<<<plan.short_tiles + (plan.short_tiles > DIRECT_TILES ? 1 : 0), SHORT_NT, 0, stream>>>(
-                    A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.words + W_NNZ);
-                NB200_CUDA(cudaGetLastError());
-            }
-            int64_t nnz;
-            int device_status;
-            if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
-            if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm of short rows");
-            c->nnz = (int32_t)nnz;
-            return NB200_OK;
-        }
-        save_plan(g_after_bound, a, b, nullptr, plan, stream);
-    }
-    if ((st = spgemm_symbolic(a, b, c, nullptr, stream_v))) return st;
+    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+    if (is_short(plan) && capacity >= (int64_t)plan.host.products) return short_on(plan, a, b, c, stream);
+    if ((st = symbolic_on(plan, a, b, c, stream))) return st;
     if (c->nnz > capacity) return NB200_E_CAPACITY;
-    return spgemm_numeric(a, b, c, stream_v);
+    return c->nnz > 0 ? esc_run_bins<true>(a, b, plan, c, stream) : NB200_OK;
+}
+
+// The whole product into arrays that the caller hands out once their length is known: no plan outlives the call.
+int spgemm_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take_fn take, void *ctx, bool one_pass, void *stream_v) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    bool done;
+    int st;
+    if (!c || !take) return NB200_E_BADARG;
+    c->col = nullptr;
+    c->val = nullptr;
+    if ((st = spgemm_begin(a, b, c, stream, &done)) || done) return st;
+    EscPlan plan{};
+    if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
+    if (one_pass && is_short(plan)) {
+        if ((st = take(ctx, (int64_t)plan.host.products, &c->col, &c->val))) return st;
+        return short_on(plan, a, b, c, stream);
+    }
+    if ((st = symbolic_on(plan, a, b, c, stream)) || c->nnz == 0) return st;
+    if ((st = take(ctx, c->nnz, &c->col, &c->val))) return st;
+    return esc_run_bins<true>(a, b, plan, c, stream);
 }
 
 }  // namespace
@@ -1307,6 +1330,10 @@ int nb200_spgemm_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, 
     return spgemm_into(a, b, c, capacity, stream);
 }
 
+int nb200_spgemm_f32_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take_fn take, void *ctx, void *stream) {
+    return spgemm_with(a, b, c, take, ctx, true, stream);
+}
+
 int nb200_spgemm_f32_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t *products, void *stream) {
     return spgemm_symbolic(a, b, c, products, stream);
 }
@@ -1322,14 +1349,13 @@ int nb200_spgemm_f32(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int32
     c->col = nullptr;
     c->val = nullptr;
     NB200_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&c->row_ptr), sizeof(int32_t) * ((size_t)std::max(a->rows, 0) + 1), stream));
-    EscPlan plan{};
-    int st = spgemm_symbolic(a, b, c, nullptr, stream_v, &plan);
-    if (st == NB200_OK && c->nnz > 0) {
-        cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&c->col), sizeof(int32_t) * (size_t)c->nnz, stream);
-        if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&c->val), sizeof(float) * (size_t)c->nnz, stream);
-        if (e != cudaSuccess) st = note_cuda_error(e, "cudaMallocAsync");
-        else st = spgemm_numeric(a, b, c, stream_v, &plan);
-    }
+    auto take = [](void *ctx, int64_t entries, int32_t **col, float **val) -> int {
+        cudaStream_t on = static_cast<cudaStream_t>(ctx);
+        NB200_CUDA(cudaMallocAsync(reinterpret_cast<void **>(col), sizeof(int32_t) * (size_t)entries, on));
+        NB200_CUDA(cudaMallocAsync(reinterpret_cast<void **>(val), sizeof(float) * (size_t)entries, on));
+        return NB200_OK;
+    };
+    const int st = spgemm_with(a, b, c, take, stream_v, false, stream_v);  // arrays of nnz(C) entries, so the rows are counted first
     if (st != NB200_OK) {
         if (c->row_ptr) cudaFreeAsync(c->row_ptr, stream);
         if (c->col) cudaFreeAsync(c->col, stream);

@@ -289,3 +289,87 @@ def test_numeric_after_other_work_on_the_stream(nacho, oracle):
     torch.cuda.synchronize()
     assert np.array_equal(col.cpu().numpy(), want.col)
     assert np.all(np.abs(val.cpu().numpy().astype(np.float64) - 2.0 * v64) <= 2.0 * REL_TOL * abs64 + 1e-30)
+
+
+def test_no_plan_outlives_a_call(nacho, oracle):
+    """A's pattern is rewritten in place after a _bound call, to the same lengths at the same addresses: every form of the
+    product that follows is that of the new pattern. The first one has rows of 5 entries, the second rows of up to 800."""
+    import ctypes as C
+    import torch
+    from nacho_b200._capi import CsrStruct, OK, TakeFn, check as ck, lib
+    rng = np.random.default_rng(12)
+    n = 800
+
+    def with_lengths(length):
+        col = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for k in length]).astype(np.int32)
+        return CSR(n, n, np.append(0, np.cumsum(length)).astype(np.int32), col, rng.uniform(-1, 1, len(col)).astype(np.float32))
+
+    flat = with_lengths(np.full(n, 5))
+    skewed = np.zeros(n, np.int64)
+    skewed[:3], skewed[3:11], skewed[11:331] = 800, 160, 1
+    skew = with_lengths(skewed)
+    assert len(flat.col) == len(skew.col)
+    b = with_lengths(np.full(n, 6))
+    ga, gb = csr_to_gpu(flat), csr_to_gpu(b)
+    sa, sb = ga._struct(), gb._struct()
+    want, v64, abs64, _ = oracle.spgemm(skew, b, 4, extras=True)
+    nnz = len(want.col)
+    rp = torch.empty(n + 1, dtype=torch.int32, device="cuda")
+    col, val = torch.empty(nnz, dtype=torch.int32, device="cuda"), torch.empty(nnz, dtype=torch.float32, device="cuda")
+
+    def put(m):
+        for t, x in ((ga.dim_j_offsets, m.row_ptr), (ga.dim_j_indices, m.col), (ga.values, m.val)):
+            t.copy_(torch.from_numpy(x))
+
+    def take(ctx, entries, p_col, p_val):
+        assert entries == nnz
+        p_col[0], p_val[0] = col.data_ptr(), val.data_ptr()
+        return OK
+
+    taker, capacity = TakeFn(take), C.c_int64(0)
+    for form in ("into", "with", "symbolic", "allocating"):
+        put(flat)
+        ck(lib.nb200_spgemm_f32_bound(C.byref(sa), C.byref(sb), C.byref(capacity), None), "bound")
+        assert capacity.value == 30 * n  # rows of 5 entries that reach 30 products
+        put(skew)
+        for t in (rp, col, val):
+            t.fill_(-1)
+        c = CsrStruct(0, 0, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr())
+        if form == "into":
+            ck(lib.nb200_spgemm_f32_into(C.byref(sa), C.byref(sb), C.byref(c), nnz, None), form)
+        elif form == "with":
+            ck(lib.nb200_spgemm_f32_with(C.byref(sa), C.byref(sb), C.byref(c), taker, None, None), form)
+        elif form == "symbolic":
+            ck(lib.nb200_spgemm_f32_symbolic(C.byref(sa), C.byref(sb), C.byref(c), None, None), form)
+            c.col, c.val = col.data_ptr(), val.data_ptr()
+            ck(lib.nb200_spgemm_f32_numeric(C.byref(sa), C.byref(sb), C.byref(c), None), form)
+        else:
+            ck(lib.nb200_spgemm_f32(C.byref(sa), C.byref(sb), C.byref(c), 0, 0, None), form)
+        torch.cuda.synchronize()
+        assert c.nnz == nnz, form
+        if form == "allocating":
+            for p in (c.row_ptr, c.col, c.val):
+                ck(lib.nb200_free_async(p, None), "free")
+            continue
+        assert np.array_equal(rp.cpu().numpy(), want.row_ptr) and np.array_equal(col.cpu().numpy(), want.col), form
+        assert np.all(np.abs(val.cpu().numpy().astype(np.float64) - v64) <= REL_TOL * abs64 + 1e-30), form
+
+
+def test_arrays_handed_out_by_the_caller(nacho, oracle):
+    """nb200_spgemm_f32_with: what the callback reports ends the call, and an empty product asks for nothing."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi, synth
+    from nacho_b200._capi import CsrStruct, TakeFn, lib
+    asked = []
+    refuse = TakeFn(lambda ctx, entries, p_col, p_val: asked.append(entries) or _capi.E_NOMEM)
+    rp = torch.empty(501, dtype=torch.int32, device="cuda")
+    for density, calls in ((0.03, 1), (0.0, 0)):
+        ga, gb = synth_to_gpu(synth.random_csr(500, 400, density, 21)), synth_to_gpu(synth.random_csr(400, 300, 0.03, 22))
+        sa, sb, c = ga._struct(), gb._struct(), CsrStruct(0, 0, 0, rp.data_ptr(), None, None)
+        del asked[:]
+        status = lib.nb200_spgemm_f32_with(C.byref(sa), C.byref(sb), C.byref(c), refuse, None, None)
+        torch.cuda.synchronize()
+        assert len(asked) == calls and status == (_capi.E_NOMEM if calls else _capi.OK)
+    assert lib.nb200_spgemm_f32_with(C.byref(sa), C.byref(sb), C.byref(c), TakeFn(), None, None) == _capi.E_BADARG
+    assert not rp.any()
