@@ -249,11 +249,13 @@ int nb200_spgemm_f32_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *
 /* One-call forms for caller-owned memory.
  *
  * _with asks for the result's arrays when it knows how many entries they need: `take(ctx, entries, &col, &val)` is called
- * once (not at all for an empty result) on the calling thread, hands out two arrays of that many entries that
- * may be used on `stream`, and returns NB200_OK, or a status with which the call then ends. It must not throw, nor call
- * this library on `stream`. c->row_ptr is the caller's; c->col / c->val are set to the arrays taken, of which the
- * first c->nnz entries are in use. Matrices of short rows (at most 8 entries in a row of A and 32 products) are
- * multiplied in one pass into an entry per product, any other into nnz(C) entries.
+ * on the calling thread, hands out two arrays of that many entries that may be used on `stream`, and returns NB200_OK, or
+ * a status with which the call then ends. It must not throw, nor call this library on `stream`. c->row_ptr is the
+ * caller's; c->col / c->val are set to the arrays in use, of which the first c->nnz entries are. An empty result
+ * takes none. Matrices of short rows (at most 8 entries in a row of A and 32 products) are multiplied in one pass into an
+ * entry per product: if `take` refuses that with NB200_E_NOMEM they are counted first, like any others, and if fewer
+ * than half of the entries are in use, `take` is called again for nnz(C) entries, to which the result moves (the arrays
+ * of the first call are read until the work queued on `stream` is done; a refusal leaves the result where it is).
  *
  * _into takes any capacity that holds the result (less returns NB200_E_CAPACITY with c->nnz filled in). _bound sets
  * *capacity to the number of entries with which _into runs in one pass, or to 0 where it has to count first. */

@@ -285,15 +285,17 @@ PyObject *spgemm(PyObject *const *args) {
     same_device(va, vb);
     at::Tensor rp = int_array((int64_t)a.rows + 1, va.device);
     nb200_csr c{a.rows, b.cols, 0, ints(rp), nullptr, nullptr};
-    struct Taken {  // the result's arrays, taken when their length is known
+    struct Taken {  // the result's arrays, taken when their length is known, and those it moved out of
         c10::Device device;
-        at::Tensor col, val;
+        at::Tensor col, val, earlier_col, earlier_val;
         std::exception_ptr failure;
     } taken{va.device};
     auto take = [](void *ctx, int64_t entries, int32_t **col, float **val) noexcept -> int {
         Taken &t = *static_cast<Taken *>(ctx);
         try {
-            t.col = int_array(entries, t.device), t.val = float_array(entries, t.device);
+            at::Tensor c = int_array(entries, t.device), v = float_array(entries, t.device);
+            t.earlier_col = std::move(t.col), t.earlier_val = std::move(t.val);
+            t.col = std::move(c), t.val = std::move(v);
             *col = ints(t.col), *val = floats(t.val);
             return NB200_OK;
         } catch (...) {

@@ -1306,8 +1306,22 @@ int spgemm_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take
     EscPlan plan{};
     if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
     if (one_pass && is_short(plan)) {
-        if ((st = take(ctx, (int64_t)plan.host.products, &c->col, &c->val))) return st;
-        return short_on(plan, a, b, c, stream);
+        const int64_t products = (int64_t)plan.host.products;
+        st = take(ctx, products, &c->col, &c->val);
+        if (st == NB200_OK) {
+            if ((st = short_on(plan, a, b, c, stream))) return st;
+            // A result holds at most twice its length, as a union's does: one that has shrunk further (32 products
+            // can meet in 4 entries) moves to arrays of its own, where there is room for them.
+            int32_t *col = nullptr;
+            float *val = nullptr;
+            if (2 * (int64_t)c->nnz >= products || take(ctx, c->nnz, &col, &val) != NB200_OK) return NB200_OK;
+            NB200_CUDA(cudaMemcpyAsync(col, c->col, sizeof(int32_t) * (size_t)c->nnz, cudaMemcpyDeviceToDevice, stream));
+            NB200_CUDA(cudaMemcpyAsync(val, c->val, sizeof(float) * (size_t)c->nnz, cudaMemcpyDeviceToDevice, stream));
+            c->col = col;
+            c->val = val;
+            return NB200_OK;
+        }
+        if (st != NB200_E_NOMEM) return st;  // no room for an entry per product: count first
     }
     if ((st = symbolic_on(plan, a, b, c, stream)) || c->nnz == 0) return st;
     if ((st = take(ctx, c->nnz, &c->col, &c->val))) return st;

@@ -373,3 +373,51 @@ def test_arrays_handed_out_by_the_caller(nacho, oracle):
         assert len(asked) == calls and status == (_capi.E_NOMEM if calls else _capi.OK)
     assert lib.nb200_spgemm_f32_with(C.byref(sa), C.byref(sb), C.byref(c), TakeFn(), None, None) == _capi.E_BADARG
     assert not rp.any()
+
+
+@pytest.mark.parametrize("shared", [True, False])
+def test_short_rows_that_shrink(nacho, oracle, shared):
+    """Rows of 8 entries that select rows of 4: 32 products that meet in 4 entries leave no array of 32 behind, such as
+    stay 32 apart keep theirs. With an entry per product refused, the rows are counted first."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import CsrStruct, TakeFn, check as ck, lib
+    rng = np.random.default_rng(5)
+    rows, inner, cols = 700, 64, 400
+    a_col = np.sort(np.argsort(rng.random((rows, inner)), axis=1)[:, :8], axis=1).ravel().astype(np.int32)
+    a = CSR(rows, inner, (8 * np.arange(rows + 1)).astype(np.int32), a_col, rng.uniform(-1, 1, 8 * rows).astype(np.float32))
+    b_col = (np.tile([3, 50, 51, 399], inner) if shared else np.arange(4 * inner)).astype(np.int32)
+    b = CSR(inner, cols, (4 * np.arange(inner + 1)).astype(np.int32), b_col, rng.uniform(-1, 1, 4 * inner).astype(np.float32))
+    want, v64, abs64, products = oracle.spgemm(a, b, 4, extras=True)
+    nnz = len(want.col)
+    assert products == 32 * rows and nnz == (4 if shared else 32) * rows
+    check(nacho, oracle, a, b)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    z = nacho.gpu_spgemm_f32(ga, gb)
+    for t in (z.dim_j_indices, z.values):
+        assert t.numel() == nnz and t.untyped_storage().nbytes() == 4 * nnz
+
+    for most in sorted({products, products - 1, nnz, nnz - 1}):  # entries that there is room for
+        asked, held = [], []
+
+        def take(ctx, entries, p_col, p_val):
+            asked.append(entries)
+            if entries > most:
+                return _capi.E_NOMEM
+            held.append((torch.empty(entries, dtype=torch.int32, device="cuda"), torch.empty(entries, dtype=torch.float32, device="cuda")))
+            p_col[0], p_val[0] = held[-1][0].data_ptr(), held[-1][1].data_ptr()
+            return _capi.OK
+
+        rp = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+        sa, sb, c = ga._struct(), gb._struct(), CsrStruct(0, 0, 0, rp.data_ptr(), None, None)
+        status = lib.nb200_spgemm_f32_with(C.byref(sa), C.byref(sb), C.byref(c), TakeFn(take), None, None)
+        torch.cuda.synchronize()
+        assert asked == [products] if most >= products and not shared else asked == [products, nnz]
+        if most < nnz:
+            assert status == _capi.E_NOMEM
+            continue
+        ck(status, "with")
+        assert c.nnz == nnz and c.col == held[-1][0].data_ptr() and c.val == held[-1][1].data_ptr()
+        assert np.array_equal(rp.cpu().numpy(), want.row_ptr) and np.array_equal(held[-1][0].cpu().numpy(), want.col)
+        assert np.all(np.abs(held[-1][1].cpu().numpy().astype(np.float64) - v64) <= REL_TOL * abs64 + 1e-30)
