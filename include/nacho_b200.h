@@ -218,6 +218,13 @@ int nb200_csr_add_3_f32(const nb200_csr *a, const nb200_csr *b, const nb200_csr 
                         void *stream);
 int nb200_csr_add_3_f32_into(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c,
                              nb200_csr *z, int64_t capacity, void *stream);
+/* The sum A + B is formed on the way: 8 bytes per entry of A and of B. The forms above keep it in the library's scratch
+ * pool, where the room stays taken until nb200_release_workspaces (three times 67 million entries: 1.3 GB). _lent is
+ * _into with scratch of the caller's: at least nb200_csr_add_3_f32_scratch(a, b, c) bytes (0 for operands that the call
+ * would refuse) on a 256-byte boundary, in use until the work queued on `stream` is done. */
+int64_t nb200_csr_add_3_f32_scratch(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c);
+int nb200_csr_add_3_f32_lent(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z,
+                             int64_t capacity, void *scratch, int64_t scratch_bytes, void *stream);
 
 /* ---- SpGEMM ----------------------------------------------------------------------------- */
 

@@ -80,6 +80,8 @@ PROTOTYPES = {
     "nb200_csr_mul_f32_host": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int64]),
     "nb200_csr_add_3_f32": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int32, C.c_int32, C.c_void_p]),
     "nb200_csr_add_3_f32_into": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_void_p]),
+    "nb200_csr_add_3_f32_scratch": (C.c_int64, [_P(CsrStruct)] * 3),
+    "nb200_csr_add_3_f32_lent": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_void_p, C.c_int64, C.c_void_p]),
     "nb200_spgemm_f32": (C.c_int, [_P(CsrStruct)] * 3 + [C.c_int32, C.c_int32, C.c_void_p]),
     "nb200_sssmm_f32_into": (C.c_int, [_P(CsrStruct)] * 4 + [C.c_int64, C.c_void_p]),
     "nb200_spgemm_f32_with": (C.c_int, [_P(CsrStruct)] * 3 + [TakeFn, C.c_void_p, C.c_void_p]),

@@ -1077,29 +1077,46 @@ namespace {
 // (src/backend/compute.cpp:426-432 builds a + b first), so running the two-operand union twice
 // gives bit-identical values to the reference's fused three-way merge: positions present in A
 // and C only hold a + c, in B and C only b + c, in all three (a + b) + c, and explicit zeros
-// stay. The intermediate A + B lives in the scratch pool, and its length stays in device memory: the second
-// union is cut into the tiles that its longest possible input needs (those past its end are empty) and nothing
-// waits in between. A kernel that merged three operands in one pass, in two stages per tile, took 2.0 ms where
-// this takes 1.17 (three times 67 M entries), although it moves 1.6 GB less.
-int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, bool alloc,
-                 int64_t capacity, void *stream_v, const LaunchKnobs &first_knobs = LaunchKnobs()) {
+// stay. The intermediate A + B, eight bytes per entry of A and of B, lies in the caller's scratch or in the pool, and its
+// length stays in device memory: the second union is cut into the tiles that its longest possible input needs (those
+// past its end are empty) and nothing waits in between. A kernel that merged three operands in one pass, in two stages
+// per tile, took 2.0 ms where this takes 1.17 (three times 67 M entries), although it moves 1.6 GB less.
+struct Add3Sizes {
+    int64_t bound, total;              // most entries of the intermediate and of the result
+    size_t own, first_bytes, all;      // bytes: the intermediate, the first union's scratch, everything
+    Add3Sizes(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c) : bound((int64_t)a->nnz + b->nnz), total(bound + c->nnz) {
+        Carver sizes;
+        sizes.take<int32_t>((size_t)a->rows + 1);
+        sizes.take<int32_t>((size_t)bound);
+        sizes.take<float>((size_t)bound);
+        own = sizes.used(), first_bytes = csr2_scratch_bytes(bound);
+        all = own + first_bytes + csr2_scratch_bytes(total);
+    }
+};
+
+int check_add3(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c) {
     int st;
     if ((st = check_csr(a, true)) || (st = check_csr(b, true)) || (st = check_csr(c, true))) return st;
-    if (!z || a->rows != b->rows || a->cols != b->cols || a->rows != c->rows || a->cols != c->cols) return NB200_E_BADARG;
+    return a->rows != b->rows || a->cols != b->cols || a->rows != c->rows || a->cols != c->cols ? NB200_E_BADARG : NB200_OK;
+}
+
+// `lent`: scratch of the caller's (Add3Sizes::all bytes), or null for the pool's.
+int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, bool alloc, int64_t capacity, void *lent,
+                 void *stream_v, const LaunchKnobs &first_knobs = LaunchKnobs()) {
+    int st;
+    if ((st = check_add3(a, b, c))) return st;
+    if (!z) return NB200_E_BADARG;
     if (!alloc && (!z->row_ptr || capacity < 0)) return NB200_E_BADARG;
-    const int64_t bound = (int64_t)a->nnz + b->nnz, total = bound + c->nnz;
+    const Add3Sizes sizes(a, b, c);
+    const int64_t bound = sizes.bound, total = sizes.total;
     if (total > INT32_MAX) return NB200_E_OVERFLOW;
     if (!alloc && capacity > 0 && total > 0 && (!z->col || !z->val)) return NB200_E_BADARG;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     // pool slot 1: the calls below use slot 0
-    Carver sizes;
-    sizes.take<int32_t>((size_t)a->rows + 1);
-    sizes.take<int32_t>((size_t)bound);
-    sizes.take<float>((size_t)bound);
-    const size_t own = sizes.used(), first_bytes = csr2_scratch_bytes(bound);
     Workspace *ws = nullptr;
-    if ((st = acquire_workspace(stream, own + first_bytes + csr2_scratch_bytes(total), &ws, 1))) return st;
-    Carver carve(ws->dev);
+    if ((st = acquire_workspace(stream, lent ? 0 : sizes.all, &ws, 1))) return st;
+    unsigned char *base = static_cast<unsigned char *>(lent ? lent : ws->dev);
+    Carver carve(base);
     nb200_csr t{};
     t.row_ptr = carve.take<int32_t>((size_t)a->rows + 1);
     t.col = carve.take<int32_t>((size_t)bound);
@@ -1108,14 +1125,14 @@ int csr_add3_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb2
         if ((st = csr2_run<OP_UNION>(a, b, &t, false, bound, stream_v))) return st;
         return csr2_run<OP_UNION>(&t, c, z, alloc, capacity, stream_v);
     }
-    unsigned char *scratch = static_cast<unsigned char *>(ws->dev) + own;
+    unsigned char *scratch = base + sizes.own;
     unsigned long long *word = result_word(ws, 0);
     FusedCtl *first = nullptr, *second = nullptr;
     if ((st = csr2_enqueue(OP_UNION, CsrIn{a->row_ptr, a->col, a->val, a->nnz}, CsrIn{b->row_ptr, b->col, b->val, b->nnz}, RowCount{a->rows}, a->cols,
                            CsrOut{t.row_ptr, t.col, t.val}, nullptr, scratch, stream, &first, first_knobs)))
         return st;
     if ((st = csr2_enqueue(OP_UNION, CsrIn{t.row_ptr, t.col, t.val, (int32_t)bound, &first->total}, CsrIn{c->row_ptr, c->col, c->val, c->nnz},
-                           RowCount{a->rows}, a->cols, CsrOut{z->row_ptr, z->col, z->val, nullptr, word, first}, nullptr, scratch + first_bytes, stream,
+                           RowCount{a->rows}, a->cols, CsrOut{z->row_ptr, z->col, z->val, nullptr, word, first}, nullptr, scratch + sizes.first_bytes, stream,
                            &second)))
         return st;
     int64_t length;
@@ -1160,12 +1177,22 @@ int nb200_csr_mul_f32_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *z,
 
 int nb200_csr_add_3_f32(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, int32_t, int32_t,
                         void *stream) {
-    return csr_add3_run(a, b, c, z, true, 0, stream);
+    return csr_add3_run(a, b, c, z, true, 0, nullptr, stream);
 }
 
 int nb200_csr_add_3_f32_into(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z,
                              int64_t capacity, void *stream) {
-    return csr_add3_run(a, b, c, z, false, capacity, stream);
+    return csr_add3_run(a, b, c, z, false, capacity, nullptr, stream);
+}
+
+int64_t nb200_csr_add_3_f32_scratch(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c) {
+    return check_add3(a, b, c) == NB200_OK ? (int64_t)Add3Sizes(a, b, c).all : 0;
+}
+
+int nb200_csr_add_3_f32_lent(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_csr *z, int64_t capacity, void *scratch,
+                             int64_t scratch_bytes, void *stream) {
+    if (check_add3(a, b, c) == NB200_OK && (!scratch || scratch_bytes < (int64_t)Add3Sizes(a, b, c).all)) return NB200_E_BADARG;
+    return csr_add3_run(a, b, c, z, false, capacity, scratch, stream);
 }
 
 int nb200_csr_add_f32_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_t capacity, void *stream) {
@@ -1199,7 +1226,7 @@ int nb200_selftest_chain_timeout(const nb200_csr *a, const nb200_csr *b, const n
     LaunchKnobs knobs;
     knobs.first_tile = 1;
     knobs.poll_limit = polls;
-    return csr_add3_run(a, b, c, z, false, capacity, stream, knobs);
+    return csr_add3_run(a, b, c, z, false, capacity, nullptr, stream, knobs);
 }
 
 int nb200_selftest_late_give_up(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_t capacity, int32_t polls, void *stream) {

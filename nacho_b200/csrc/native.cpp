@@ -252,7 +252,11 @@ PyObject *csr_add_3(PyObject *const *args) {
     same_device(va, vb);
     same_device(va, vc);
     const int64_t capacity = (int64_t)a.nnz + b.nnz + c.nnz;
-    return csr_result({&va, &vb, &vc}, where, a.rows, a.cols, capacity, [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_into(&a, &b, &c, z, capacity, stream); });
+    // the intermediate sum is as large as the operands: it lies in an array of this call, not in the library's pool
+    const int64_t scratch_bytes = nb200_csr_add_3_f32_scratch(&a, &b, &c);
+    at::Tensor scratch = array(scratch_bytes, at::kByte, va.device);
+    return csr_result({&va, &vb, &vc}, where, a.rows, a.cols, capacity,
+                      [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_lent(&a, &b, &c, z, capacity, scratch.data_ptr(), scratch_bytes, stream); });
 }
 
 PyObject *sssmm(PyObject *const *args) {

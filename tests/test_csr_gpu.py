@@ -367,3 +367,32 @@ def test_host_streaming_entry_points(nacho, oracle, op):
     r = fn(pin(small), pin(small))
     w = (oracle.csr_add if op == "add" else oracle.csr_mul)(synth_csr(small), synth_csr(small), 1)
     assert_same(CSR(r[0], r[1], r[2].numpy(), r[3].numpy(), r[4].numpy()), w, f"host {op} small")
+
+
+def test_three_operand_add_gives_its_intermediate_back(nacho):
+    """The sum of the first two operands is as large as they are. Once the result is gone, so is the room it took."""
+    import torch
+    from nacho_b200._capi import check, lib
+    rows, cols, n = 1 << 16, 1 << 16, 1 << 23
+
+    def operand():
+        gap = rows * cols // n
+        key = torch.arange(n, device="cuda", dtype=torch.int64) * gap + torch.randint(0, gap, (n,), device="cuda")
+        r = key // cols
+        rp = torch.searchsorted(r, torch.arange(rows + 1, device="cuda")).to(torch.int32)
+        return nacho.CSR_gpu(rp, (key - r * cols).to(torch.int32), torch.rand(n, device="cuda"), torch.tensor([rows, cols], dtype=torch.int32))
+
+    ops = [operand() for _ in range(3)]
+    check(lib.nb200_release_workspaces(), "release")
+
+    def used():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, total = torch.cuda.mem_get_info()
+        return total - free
+
+    before = used()
+    z = nacho.gpu_csr_add_3_f32(*ops)
+    assert z.values.numel() > 2 * n
+    del z
+    assert used() - before < 8 * 2 * n // 4
