@@ -16,7 +16,9 @@
 
 #include <algorithm>
 #include <exception>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "nacho_b200.h"
 
@@ -179,10 +181,13 @@ struct NoLock {  // releases the interpreter lock
 };
 
 // Calls of several host threads on one stream take turns at issuing their kernels: they share the stream's scratch
-// arrays and result words. A few locks serve all streams.
-std::mutex &stream_lock(void *stream) {
-    static std::mutex locks[61];
-    return locks[(reinterpret_cast<uintptr_t>(stream) >> 4) % 61];
+// arrays and result words. The lock's key is the pool's, device and stream: the default stream has the same handle
+// on every device, and a lock is held while its call waits for a length. (Locks stay, as the pool's entries do.)
+std::mutex &stream_lock(int device, void *stream) {
+    static std::mutex guard;
+    static std::map<std::pair<int, void *>, std::mutex> locks;
+    std::lock_guard<std::mutex> g(guard);
+    return locks[{device, stream}];
 }
 
 // Runs a C-ABI call on the operands' device and the current stream of the caller, without the interpreter lock. A call
@@ -197,7 +202,7 @@ int run(const View *const (&operands)[N], F call) {
     int status;
     {
         NoLock unlocked;
-        std::lock_guard<std::mutex> turn(stream_lock(stream));
+        std::lock_guard<std::mutex> turn(stream_lock(device.index(), stream));
         status = call(stream);
     }
     for (const View *operand : operands)
@@ -448,13 +453,21 @@ PyObject *bind(PyObject *, PyObject *args) {
     Py_RETURN_NONE;
 }
 
+// turn_of(device, stream handle): identity of the lock by which calls there take turns (for tests)
+PyObject *turn_of(PyObject *, PyObject *args) {
+    int device;
+    unsigned long long stream;
+    if (!PyArg_ParseTuple(args, "iK", &device, &stream)) return nullptr;
+    return PyLong_FromVoidPtr(&stream_lock(device, reinterpret_cast<void *>(stream)));
+}
+
 template <PyObject *(*OP)(PyObject *const *), int ARGS>
 PyMethodDef op(const char *name) {
     return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(entry<OP, ARGS>)), METH_FASTCALL, nullptr};
 }
 
 PyMethodDef g_methods[] = {
-    {"bind", bind, METH_VARARGS, nullptr},
+    {"bind", bind, METH_VARARGS, nullptr}, {"turn_of", turn_of, METH_VARARGS, nullptr},
     op<csr_add, 2>("csr_add"), op<csr_mul, 2>("csr_mul"), op<csr_add_3, 3>("csr_add_3"), op<spgemm, 2>("spgemm"),
     op<sssmm, 3>("sssmm"), op<coo3d_add, 2>("coo3d_add"), op<csf_add, 2>("csf_add"), op<coo_add, 2>("coo_add"),
     op<coo_mul, 2>("coo_mul"), op<coo_csr_add, 2>("coo_csr_add"), op<dcsr_add, 2>("dcsr_add"), op<dcsr_mul, 2>("dcsr_mul"),

@@ -36,3 +36,13 @@ def test_mirror_surface():
     nacho_b200.install_as_nacho()
     import nacho as installed
     assert installed is nacho
+
+
+def test_calls_take_turns_by_device_and_stream():
+    """Host threads wait for one another where they share a device's stream, and nowhere else: the default stream has the
+    same handle on every device."""
+    from nacho_b200 import _native
+    places = [(device, stream) for device in range(8) for stream in (0, *range(0x55550000, 0x55550000 + 64 * 0x3d0, 0x3d0))]
+    turns = [_native.turn_of(*p) for p in places]
+    assert len(set(turns)) == len(places)
+    assert turns == [_native.turn_of(*p) for p in places]
