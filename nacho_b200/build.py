@@ -79,12 +79,17 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     return LIB
 
 
-def build_native(nvcc: str, verbose: bool = False) -> str:
-    """``_native.so`` against the torch of this interpreter; it finds ``libnacho_b200.so`` beside itself."""
+def build_native(nvcc: str, verbose: bool = False) -> str | None:
+    """``_native.so`` against the torch of this interpreter; it finds ``libnacho_b200.so`` beside itself. The C library
+    needs no torch: without one this says so and builds nothing."""
+    try:
+        import torch
+    except ImportError:
+        sys.stderr.write("torch is not installed: nacho_b200/_native.so, the Python operators, is not built\n")
+        return None
     src = os.path.join(CSRC, "native.cpp")
     if not _stale(NATIVE, [src, os.path.join(ROOT, "include", "nacho_b200.h"), os.path.abspath(__file__)]):
         return NATIVE
-    import torch
     torch_dir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
