@@ -20,6 +20,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB = os.path.join(HERE, "libnacho_b200.so")
 NATIVE = os.path.join(HERE, "_native.so")
+NATIVE_FOR = os.path.join(OBJ_DIR, "native.txt")  # the interpreter and the torch that it was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -42,6 +43,13 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _read(path: str) -> str | None:
+    if not os.path.exists(path):
+        return None
+    with open(path) as f:
+        return f.read()
 
 
 def build(verbose: bool = False, ptxas_info: bool = False) -> str:
@@ -80,15 +88,17 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
 
 
 def build_native(nvcc: str, verbose: bool = False) -> str | None:
-    """``_native.so`` against the torch of this interpreter; it finds ``libnacho_b200.so`` beside itself. The C library
-    needs no torch: without one this says so and builds nothing."""
+    """``_native.so`` against the torch of this interpreter; it finds ``libnacho_b200.so`` beside itself. Rebuilt when a source
+    is newer or it was built for another interpreter or torch. The C library needs neither: without a torch this says so
+    and builds nothing."""
     try:
         import torch
     except ImportError:
         sys.stderr.write("torch is not installed: nacho_b200/_native.so, the Python operators, is not built\n")
         return None
     src = os.path.join(CSRC, "native.cpp")
-    if not _stale(NATIVE, [src, os.path.join(ROOT, "include", "nacho_b200.h"), os.path.abspath(__file__)]):
+    built_for = f"python {sys.version}\ntorch {torch.__version__} {torch.version.git_version}\n"
+    if not _stale(NATIVE, [src, os.path.join(ROOT, "include", "nacho_b200.h"), os.path.abspath(__file__)]) and _read(NATIVE_FOR) == built_for:
         return NATIVE
     torch_dir = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
@@ -103,6 +113,8 @@ def build_native(nvcc: str, verbose: bool = False) -> str | None:
         sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
     if r.returncode != 0:
         raise RuntimeError("build of _native.so failed")
+    with open(NATIVE_FOR, "w") as f:
+        f.write(built_for)
     return NATIVE
 
 
