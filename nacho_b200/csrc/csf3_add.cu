@@ -349,6 +349,7 @@ int csf_add_run(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, bool al
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int64_t total = (int64_t)a->n_k + b->n_k;
     if (total > INT32_MAX) return NB200_E_OVERFLOW;
+    if (total > 0 && (a->dims[0] < 0 || a->dims[1] < 0 || a->dims[2] < 0)) return NB200_E_BADARG;
     const int64_t bound_i = (int64_t)a->n_i + b->n_i, bound_j = (int64_t)a->n_j + b->n_j;
     for (int d = 0; d < 3; ++d) z->dims[d] = a->dims[d];
     z->n_i = z->n_j = z->n_k = 0;

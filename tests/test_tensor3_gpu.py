@@ -247,3 +247,25 @@ def test_csf3_both_routes(nacho, oracle, monkeypatch, route, dims, n, seed):
             want = oracle.csf3_add(CSF3(dims, *csf3_levels(cl), vl), CSF3(dims, *csf3_levels(ch), vh))
             got = nacho.gpu_csf_add_f32(nacho.to_csf3(cl, vl, dims, "cuda"), nacho.to_csf3(ch, vh, dims, "cuda"))
             assert_same(csf3_from_gpu(got), want, f"csf3 route {route}, disjoint slices")
+
+
+def test_negative_extents_are_refused(nacho):
+    """Extents below zero end a CSF3 add of entries with a status, whatever its route; an empty one has nothing to refuse."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import Csf3Struct, lib
+    dims = (30, 40, 50)
+    (ca, va), (cb, vb) = _seeded(dims, 500, 3)
+    ga, gb = nacho.to_csf3(ca, va, dims, "cuda"), nacho.to_csf3(cb, vb, dims, "cuda")
+    n_i, n_j, n_k = (len(getattr(ga, f)) + len(getattr(gb, f)) for f in ("dim_i_indices", "dim_j_indices", "dim_k_indices"))
+    arrays = [torch.empty(n, dtype=torch.int32, device="cuda") for n in (n_i, n_i + 1, n_j, n_j + 1, n_k, n_k)]
+    for mode in range(3):
+        sa, sb = ga._struct(), gb._struct()
+        sa.dims[mode] = sb.dims[mode] = -5
+        z = Csf3Struct((C.c_int32 * 3)(), 0, 0, 0, *(t.data_ptr() for t in arrays))
+        assert lib.nb200_csf_add_f32_into(C.byref(sa), C.byref(sb), C.byref(z), n_i, n_j, n_k, None) == _capi.E_BADARG
+        assert lib.nb200_csf_add_f32(C.byref(sa), C.byref(sb), C.byref(z), 0, 0, None) == _capi.E_BADARG
+        sa.n_i = sa.n_j = sa.n_k = sb.n_i = sb.n_j = sb.n_k = 0
+        z = Csf3Struct((C.c_int32 * 3)(), 0, 0, 0, *(t.data_ptr() for t in arrays))
+        assert lib.nb200_csf_add_f32_into(C.byref(sa), C.byref(sb), C.byref(z), 0, 0, 0, None) == _capi.OK
