@@ -85,6 +85,7 @@ WORKLOADS = {
     "c5_csf_add": dict(op="csf_add", fmt="csf3"),
     "n1_sssmm_rmat": dict(op="sssmm", fmt="csr"),
 }
+NO_REFERENCE_CPU = ("spgemm", "sssmm")  # the reference compiles these for the GPU only
 RMAT_WORKLOADS = ("c4a_spgemm_rmat", "n1_sssmm_rmat")
 
 
@@ -222,7 +223,7 @@ def cpu_baseline(name: str, operands, steps: int = 3, warmup: int = 1):
     spec = WORKLOADS[name]
     op = spec["op"]
     cores = default_threads()
-    use_ref = Reference.available() and op not in ("spgemm", "sssmm")
+    use_ref = Reference.available() and op not in NO_REFERENCE_CPU
     if use_ref:
         impl = Reference()
         cores = impl.threads()
@@ -330,12 +331,19 @@ def default_scaling(args, spec) -> str:
 def run_reference(args):
     """`--impl reference`: the reference's CPU implementation of the path on the host cores, on
     the same workload as the other arm (the whole job: under strong scaling that is the one fixed
-    operand pair whatever N is). Rank 0 only."""
+    operand pair whatever N is). Rank 0 only. Where there is no such implementation -- its kernels were
+    not built here, or it has none for the CPU -- the line says so: the oracle is no stand-in for it."""
     if int(os.environ.get("RANK", "0")) != 0:
         return
     import torch
+    from oracle.cpu_oracle import Reference
     dev = "cuda" if torch.cuda.is_available() else "cpu"
     spec = WORKLOADS[args.workload]
+    why = (f"the reference has no CPU implementation of {spec['op']}" if spec["op"] in NO_REFERENCE_CPU else
+           None if Reference.available() else "the reference's kernels are not built here (oracle/_ref: needs its sources)")
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+        return
     scale = cpu_sample_scale(args.workload, args.cpu_scale) * args.rows_scale
     cpu_rmat = min(args.rmat_scale, 14)  # the CPU port sorts every product; keep its sample bounded
     ops = make_operands(args.workload, 0, dev, scale=scale, rmat_scale=cpu_rmat)
