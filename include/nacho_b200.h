@@ -16,8 +16,9 @@
  *   - `stream` is a cudaStream_t passed as void* (NULL = the legacy default stream, which is
  *     what nacho's drivers use, src/backend/stitch_and_generate_gpu.cpp:163-167).
  *   - Every call returns an nb200_status; 0 is success. Nothing throws and nothing aborts.
- *   - The calls block the host until the result lengths are known (one small device-to-host
- *     read), like nacho's drivers do; on return the result is complete in stream order.
+ *   - The calls block the host until the result lengths are known (a kernel writes them to pinned
+ *     host memory), like nacho's drivers do; on return kernels may still be running, and the result is
+ *     complete in stream order.
  *   - num_blocks / threads_per_block are accepted for signature compatibility
  *     (src/backend/generate_bindings.cpp:317-327); the kernels size their own grids, so the
  *     two values are ignored.

@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(NT) k_csf_expand(int32_t n_i, int32_t n_j, con
 }
 
 struct CompressCtl {
-    int ticket;
     DeviceStatus status;
     int n_i, n_j;
 };
@@ -117,7 +116,6 @@ __global__ void __launch_bounds__(NT) k_csf_compress(int32_t nnz, const int32_t 
                                                      int32_t *__restrict__ j_idx, int32_t *__restrict__ k_ptr,
                                                      uint64_t *tile_state_raw, CompressCtl *ctl) {
     __shared__ int scan_tmp[72];
-    __shared__ int s_tile;
     __shared__ long long s_base;
     volatile uint64_t *tile_state = tile_state_raw;
     const int tid = threadIdx.x;

@@ -4,13 +4,13 @@
 // The merged sequence of all stored entries of A and B, ordered by (row, column) with A first
 // on ties, is cut into tiles of a few thousand entries. A partition kernel finds every cut with
 // k-ary searches (rows on the summed row offsets, then the merge-path diagonal inside the row).
-// One CTA then owns one tile: the copy engine stages the tile's column indices and values in shared
-// memory, every row that begins in the tile adds one to the upper bits of its first column (so a
+// One CTA then owns one tile: the copy engine stages the tile's columns in shared memory (the values stay where they
+// are, prefetched into L2), every row that begins in the tile adds one to the upper bits of its first column (so a
 // key of the next entry is "row of the entry before it + this word"), every thread finds where its
-// share of the merged sequence begins with two searches in shared memory, and merges its entries
-// one result after the other, values included. The results are compacted through shared memory and
-// written back coalesced. Row offsets of the result are produced by the same pass: a tile owns the
-// offsets of the rows that begin inside it.
+// share of the merged sequence begins with two searches in shared memory, and merges the columns of its entries
+// one result after the other, noting where each comes from. The tile's count goes out; then columns and values of the
+// results are fetched by those notes, in order, and written back coalesced. Row offsets of the result are produced by
+// the same pass: a tile owns the offsets of the rows that begin inside it.
 //
 // Reference behaviour restated (not its code): partition src/backend/partition.cpp:813-993
 // (equal columns never split, :964-983), count src/backend/compute.cpp:152-271, fill
@@ -189,7 +189,7 @@ struct TileShared {
 //     instructions), and it leaves a 16-bit source index per result entry;
 //   - the tile's count goes out right after it, and the values are fetched (from L2, where a prefetch has
 //     brought them meanwhile) while the count travels;
-//   - a tile needs 6 bytes of shared memory per entry instead of 16, so five CTAs share an SM.
+//   - a tile needs 6 bytes of shared memory per entry instead of 16: 55 KB with 31 entries per thread, so four CTAs share an SM.
 template <int VT, int OP, int MODE, bool LEVELS, bool WIDE>
 __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const TileRange &tile, const int cbits, const int t,
                                           const int num_tiles, int32_t *tile_count, const TileWords &words, FusedCtl *ctl,
@@ -844,8 +844,8 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     Carver carve(ws->dev);
     Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
-    // control block (status word, result length) and the tile words of the single-pass kernel,
-    // contiguous for one memset; the two-pass route uses the control block alone
+    // control block (status word, result length) and the tile words of the single-pass kernel, contiguous for the partition
+    // kernel, which clears them; the two-pass route uses the control block alone
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     static_assert(sizeof(FusedCtl) <= 4 * sizeof(uint64_t), "control block must fit its slot");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
@@ -1006,7 +1006,7 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
                   "scratch layout must fit the fixed array");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
     const TileWords words = TileWords::at(fused_block + 4, num_tiles);
-    // the array keeps the previous call's contents: the ticket, the status and every tile word
+    // the array keeps the previous call's contents: the control block and every tile word
     // must start at zero (the partition kernel clears them)
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};

@@ -13,7 +13,7 @@ enum SetOp { OP_UNION = 0, OP_INTERSECT = 1 };
 // What one launch of the tile kernel does.
 //   MODE_COUNT  count the tile's result entries (first pass of the two-pass scheme)
 //   MODE_FILL   write the result; the tile's output base comes from the scanned counts
-//   MODE_FUSED  single pass: count, obtain the base by look-back over earlier tiles, write
+//   MODE_FUSED  single pass: count, obtain the output base (below), write
 //   MODE_REDUCE no result tensor: the products of the entries both operands hold are summed
 //               (inner product); the tile's partial sum is added to a double in the control block
 enum Mode { MODE_COUNT = 0, MODE_FILL = 1, MODE_FUSED = 2, MODE_REDUCE = 3 };
@@ -22,7 +22,7 @@ enum Mode { MODE_COUNT = 0, MODE_FILL = 1, MODE_FUSED = 2, MODE_REDUCE = 3 };
 struct FusedCtl {
     int hollow;           // offsets mode: a result entry stands for empty ranges only
     DeviceStatus status;  // bounded-wait failures
-    long long total;      // result entries, written by the last tile (MODE_REDUCE: the bits of a double, the running sum)
+    long long total;      // result entries, written by whoever has all counts: the last of few tiles, else CTA 0 (MODE_REDUCE: the bits of a double, the running sum)
 };
 
 // ------------------------------------------------------------------- output bases ----

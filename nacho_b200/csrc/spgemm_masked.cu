@@ -53,8 +53,8 @@ struct WorkClass {
     constexpr size_t smem() const { return size_t(12) * words + size_t(5) * entries + 16; }
 };
 constexpr WorkClass CLASS[4] = {
-    {1024, 2048, 256},    //  65536 columns of span, 22.5 KB: eight CTAs per SM
-    {4096, 8192, 1024},   // 262144 columns, 88 KB: two CTAs per SM
+    {1024, 2048, 256},    //  65536 columns of span, 22.5 KB: six CTAs per SM (40 registers)
+    {4096, 8192, 1024},   // 262144 columns, 88 KB: one CTA per SM (54 registers; the shared memory is there for two)
     {16384, 0, 1024},     // 2^20 columns, 192 KB, sums in global memory: one CTA per SM
     {0, 0, SEARCH_NT},    // wider still: no bitmap, binary search
 };
@@ -642,7 +642,8 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
         k_sssmm_classify<<<(int)(((int64_t)rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, stream>>>(A, B, C, rows, list_cap, units, light, sctl);
     }
     // Every list is worked by resident CTAs that take units from a ticket; a list's length stays on
-    // the device, so an empty list costs one launch of CTAs that leave at once.
+    // the device, so an empty list costs one launch of CTAs that leave at once. (The grids are those of the shared memory;
+    // where registers let fewer CTAs in, the others find the list worked off.)
     {
         LaunchScope scope("sssmm_bitmap_wide", stream);
         NB200_CUDA(launch_overlapped(k_sssmm_bitmap<1024, false>, dim3(std::min(sms, most)), dim3(1024), CLASS[2].smem(), stream, A, B, C,

@@ -16,7 +16,7 @@ import ctypes as C
 import torch
 
 from .. import _capi
-from .._capi import Coo3Struct, CooStruct, CsrStruct, Csf3Struct, DcsrStruct
+from .._capi import Coo3Struct, CsrStruct, Csf3Struct
 
 try:
     from .. import _native
@@ -233,10 +233,6 @@ class COO_gpu:
     def device(self):
         return self._values.device
 
-    def _struct(self) -> CooStruct:
-        return CooStruct(*self._dims, self._values.numel(), self._i.data_ptr(),
-                         self._j.data_ptr(), self._values.data_ptr())
-
     def __repr__(self):
         return f"COO_gpu(shape={self._dims}, nnz={self._values.numel()})"
 
@@ -268,10 +264,6 @@ class DCSR_gpu:
     @property
     def device(self):
         return self._values.device
-
-    def _struct(self) -> DcsrStruct:
-        return DcsrStruct(*self._dims, self._i.numel(), self._values.numel(),
-                          self._i.data_ptr(), self._jp.data_ptr(), self._j.data_ptr(), self._values.data_ptr())
 
     def __repr__(self):
         return f"DCSR_gpu(shape={self._dims}, rows_stored={self._i.numel()}, nnz={self._values.numel()})"

@@ -142,3 +142,54 @@ def test_a_late_give_up_is_reported(nacho, oracle, total):
             assert_same(CSR(rows, cols, rp.cpu().numpy(), col[:z.nnz].cpu().numpy(), val[:z.nnz].cpu().numpy()), want, f"{polls} polls")
     assert seen[0] == _capi.E_TIMEOUT and seen[-1] == _capi.OK, seen
     assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), want, "add after a give-up")
+
+
+@pytest.mark.parametrize("total", [2000, 200_000])
+@pytest.mark.parametrize("before", ["nothing", "kernel", "copy", "other stream"])
+def test_asynchronous_calls_in_a_graph(nacho, oracle, total, before):
+    """Two asynchronous sums captured behind nothing, a kernel, a copy or the work of another stream, and replayed."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import CsrStruct, check, lib
+    rng = np.random.default_rng(total)
+    rows, cols = total // 10, 3000
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    want = oracle.csr_add(a, b, 8)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    rp, col = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (rows + 1, total))
+    val, x, y = (torch.zeros(n, device="cuda") for n in (total, 1000, 1000))
+    res = torch.empty(3, dtype=torch.int64, device="cuda")
+    z, sa, sb = CsrStruct(rows, cols, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr()), ga._struct(), gb._struct()
+    stream, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def call():
+        check(lib.nb200_csr_add_f32_async(C.byref(sa), C.byref(sb), C.byref(z), total, res.data_ptr(), stream.cuda_stream), "async")
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()  # takes the stream's scratch before the capture begins
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        if before == "kernel":
+            x.add_(1)
+        elif before == "copy":
+            x.copy_(y)
+        elif before == "other stream":
+            side.wait_stream(stream)
+            with torch.cuda.stream(side):
+                y.add_(1)
+            stream.wait_stream(side)
+        call()
+        call()
+        x.add_(1)
+    for _ in range(3):
+        for t in (rp, col, val, res):
+            t.fill_(-1)
+        graph.replay()
+        torch.cuda.synchronize()
+        n = len(want.col)
+        assert res.tolist() == [n, _capi.OK, rows]
+        assert_same(CSR(rows, cols, rp.cpu().numpy(), col[:n].cpu().numpy(), val[:n].cpu().numpy()), want, before)

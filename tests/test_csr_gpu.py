@@ -269,8 +269,7 @@ def test_two_pass_route_with_exact_capacity(nacho, csr_golden, case):
 
 def test_env_knobs_in_a_child_process(tmp_path):
     """NACHO_B200_EXACT_ALLOC=1 (the allocating entry points count first and allocate exactly nnz, as
-    the reference's drivers do) and NACHO_B200_ADD3_CHAINED=1 (the three-operand add as two chained
-    unions): both read once per process, both must give the golden results."""
+    the reference's drivers do): read once per process, must give the golden results."""
     import os
     import subprocess
     import sys
@@ -299,10 +298,10 @@ for case in ("smoke", "medium", "all_empty", "giant_row", "cancel"):
         assert (z.nnz > 0) == bool(z.col) == bool(z.val)
         for p in (z.row_ptr, z.col, z.val):
             check(lib.nb200_free_async(p, None), "free")
-    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, gc)), golden_csr(g, case, "add3"), case + " add3 (chained)")
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, gc)), golden_csr(g, case, "add3"), case + " add3")
 print("knobs ok")
 ''')
-    env = dict(os.environ, NACHO_B200_EXACT_ALLOC="1", NACHO_B200_ADD3_CHAINED="1")
+    env = dict(os.environ, NACHO_B200_EXACT_ALLOC="1")
     r = subprocess.run([sys.executable, str(script)], env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "knobs ok" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
 
@@ -396,3 +395,45 @@ def test_three_operand_add_gives_its_intermediate_back(nacho):
     assert z.values.numel() > 2 * n
     del z
     assert used() - before < 8 * 2 * n // 4
+
+
+@pytest.mark.parametrize("n_a,n_b,n_c", [(1000, 900, 800), (30_000, 200_000, 100_000), (0, 0, 50_000), (0, 60_000, 0), (700, 0, 600_000),
+                                         (3_500_000, 2_600_000, 400_000)])
+def test_three_operand_add_by_each_route(nacho, oracle, n_a, n_b, n_c):
+    """Two unions back to back with the intermediate's length on the device (room for the worst case), or one call after the
+    other (allocating, room for the result only, A and B empty): the same bits."""
+    import torch
+    from nacho_b200._capi import CsrStruct, E_CAPACITY, check, lib
+    rng = np.random.default_rng(n_a + 3 * n_b + 7 * n_c)
+    rows, cols = 40_000, 20_000
+
+    def operand(n):
+        key = np.unique(rng.integers(0, rows * cols, n))
+        return CSR(rows, cols, np.searchsorted(key // cols, np.arange(rows + 1)).astype(np.int32), (key % cols).astype(np.int32),
+                   rng.uniform(-1, 1, len(key)).astype(np.float32))
+
+    ops = [operand(n) for n in (n_a, n_b, n_c)]
+    want = oracle.csr_add_3(*ops, 8)
+    gpu = [csr_to_gpu(m) for m in ops]
+    structs = [g._struct() for g in gpu]
+    refs = [C.byref(s) for s in structs]
+    nnz, total = len(want.col), sum(len(m.col) for m in ops)
+    rp = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+    scratch_bytes = lib.nb200_csr_add_3_f32_scratch(*refs)
+    scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device="cuda")
+    for capacity, lent in ((total, False), (nnz, False), (total, True), (nnz, True)):
+        col, val = torch.empty(capacity, dtype=torch.int32, device="cuda"), torch.empty(capacity, dtype=torch.float32, device="cuda")
+        z = CsrStruct(rows, cols, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr())
+        if lent:
+            check(lib.nb200_csr_add_3_f32_lent(*refs, C.byref(z), capacity, scratch.data_ptr(), scratch_bytes, None), "lent")
+        else:
+            check(lib.nb200_csr_add_3_f32_into(*refs, C.byref(z), capacity, None), "into")
+        torch.cuda.synchronize()
+        assert_same(CSR(rows, cols, rp.cpu().numpy(), col[:z.nnz].cpu().numpy(), val[:z.nnz].cpu().numpy()), want, f"capacity {capacity}, lent {lent}")
+    assert lib.nb200_csr_add_3_f32_into(*refs, C.byref(z), nnz - 1, None) == E_CAPACITY and z.nnz == nnz
+    z = CsrStruct()
+    check(lib.nb200_csr_add_3_f32(*refs, C.byref(z), 256, 256, None), "allocating")
+    torch.cuda.synchronize()
+    assert_same(CSR(z.rows, z.cols, _d2h(z.row_ptr, z.rows + 1, np.int32), _d2h(z.col, z.nnz, np.int32), _d2h(z.val, z.nnz, np.float32)), want, "allocating")
+    for p in (z.row_ptr, z.col, z.val):
+        check(lib.nb200_free_async(p, None), "free")
