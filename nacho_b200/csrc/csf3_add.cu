@@ -280,6 +280,11 @@ bool levels_pay(const nb200_csf3 *a, const nb200_csf3 *b) {
     return true;
 }
 
+// Up to this many entries per fibre of the operands, the tile for short rows takes the entries. 25 M entries per operand,
+// whole call, that tile against the large one: 365 us against 411 with 6 entries per fibre, 297 against 317 with 30, 291
+// against 294 with 50, 270 against 254 with 113; 5 M: 102 against 104 with 36.
+constexpr int64_t SHORT_FIBRE = 64;
+
 // `done` tells whether the result is in place; it is not where an operand stores empty slices or fibres, which
 // the canonical tree does not have (the caller then takes the other route).
 int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cudaStream_t stream, bool *done,
@@ -310,7 +315,7 @@ int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cuda
     if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{0, &ctl[0]->total}, a->dims[1],
                            CsrOut{z->j_ptr, z->j_idx, nullptr, nullptr, word[1], ctl[0]}, &fibres, scratch_j, stream, &ctl[1])))
         return st;
-    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total, true}, a->dims[2],
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total, total < SHORT_FIBRE * bound_j}, a->dims[2],
                            CsrOut{z->k_ptr, z->k_idx, z->val, nullptr, word[2], ctl[1]}, nullptr, scratch_k, stream, &ctl[2])))
         return st;
     int64_t length[3];

@@ -74,7 +74,7 @@ inline int check_csr(const nb200_csr *m, bool need_arrays) {
 struct RowCount {
     int32_t value = 0;
     const long long *dev = nullptr;
-    bool short_rows = false;  // many rows hold an entry or two (chooses the tile, nothing else)
+    bool short_rows = false;  // rows of a few dozen entries or less (chooses the tile, nothing else)
     __device__ __forceinline__ int32_t get() const { return dev ? (int32_t)*dev : value; }
 };
 

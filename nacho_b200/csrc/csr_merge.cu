@@ -137,10 +137,10 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
 // ------------------------------------------------------------------------ tile kernel ----
 
 
-// Large tile where the caller says that many rows hold an entry or two (the fibres of a tree): a tile of 31 with more
-// rows than fit takes twice the time of the others and holds up their output bases. 25 M entries per operand in 6 M
-// fibres take 450 us with 17, 443 with 21, 463 with 23, 484 with 31. The stored rows of a doubly compressed
-// matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
+// Large tile where the caller says that rows are short (the fibres of a tree): a tile of 31 with more rows than fit takes
+// twice the time of the others and holds up their output bases, and the twin mask by entries (below) pays. 25 M entries
+// per operand in 6 M fibres take 384 us with 17, 389 with 21, 426 with 23, 446 with 31; 50 M in 4 M fibres 513, 508,
+// 563, 548. The stored rows of a doubly compressed matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
 constexpr int V_FIBRES = 21;
 
 // Shared-memory plan of the tile body. The column words of both operands lie in one array: A's entry e at

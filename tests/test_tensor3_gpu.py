@@ -269,3 +269,19 @@ def test_negative_extents_are_refused(nacho):
         sa.n_i = sa.n_j = sa.n_k = sb.n_i = sb.n_j = sb.n_k = 0
         z = Csf3Struct((C.c_int32 * 3)(), 0, 0, 0, *(t.data_ptr() for t in arrays))
         assert lib.nb200_csf_add_f32_into(C.byref(sa), C.byref(sb), C.byref(z), 0, 0, 0, None) == _capi.OK
+
+
+@pytest.mark.parametrize("fibres", [90_000, 60_000, 50_000, 40_000, 700])
+def test_csf3_short_and_long_fibres(nacho, oracle, fibres):
+    """Large trees on both sides of the entries per fibre (64) up to which the tile for short rows is taken."""
+    rng = np.random.default_rng(fibres)
+    n, dims = 3_200_000, (100, fibres // 100, 1 << 14)
+    ops = []
+    for _ in range(2):
+        key = np.unique(rng.integers(0, fibres * dims[2], n))
+        ij, k = np.divmod(key, dims[2])
+        i, j = np.divmod(ij, dims[1])
+        ops.append((np.stack([i, j, k], 1).astype(np.int32), rng.uniform(-1, 1, len(key)).astype(np.float32)))
+    (ca, va), (cb, vb) = ops
+    z = nacho.gpu_csf_add_f32(nacho.to_csf3(ca, va, dims, "cuda"), nacho.to_csf3(cb, vb, dims, "cuda"))
+    assert_same(csf3_from_gpu(z), oracle.csf3_add(CSF3(dims, *csf3_levels(ca), va), CSF3(dims, *csf3_levels(cb), vb)), "csf3")
