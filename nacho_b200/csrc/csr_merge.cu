@@ -201,7 +201,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     constexpr Key END = WIDE ? (Key)~0ull : (Key)0x80000000u;  // after every key (narrow: keys are below 2^31), also with row bits added
     constexpr bool WRITES = MODE != MODE_COUNT;
     // Rows of an entry or two: a mask by entries instead of steps spares every row offset a search of it (25 M entries per
-    // operand in 6 M rows: 440 -> 432 us). With fewer rows the mask costs more than the searches (67 M entries 1 %).
+    // operand in 6 M rows: 391.5 -> 388.5 us). With fewer rows the mask costs more than the searches (67 M entries 458 -> 460.5).
     constexpr bool MANY_ROWS = VT == V_FIBRES;
     uint32_t *s_rows = reinterpret_cast<uint32_t *>(smem_raw + P::ROWS_AT);  // start of row r in the tile: A's in the lower half, B's in the upper
     int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.trow, *s_wtotal = sh.wtotal;
@@ -257,13 +257,14 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     if (WIDE) for (int i = tid; i < P::SLOTS / 2; i += NT) reinterpret_cast<uint32_t *>(row_mark)[i] = 0u;
     if (tid < W) s_wrow[tid] = 0;
 
-    // ---- row starts (relative to the tile), while the copies fly. Row 0 is the one the tile begins in.
+    // ---- row starts (relative to the tile), while the copies fly. Row 0 is the one the tile begins in. A few rows fall to
+    // the last warps, which have nothing to stage: plain loads do not pass the staging.
     auto global_start = [&](int r) -> uint32_t {
         return (uint32_t)(row_offset(A, (int64_t)tile.i0 + r) - tile.a0) | (uint32_t)(row_offset(B, (int64_t)tile.i0 + r) - tile.b0) << 16;
     };
     constexpr int RB = 4;  // rows a thread fetches together
     if (nr <= NT) {
-        if (tid < nr) s_rows[1 + tid] = global_start(1 + tid);
+        if (NT - tid <= nr) s_rows[NT - tid] = global_start(NT - tid);
     } else if (rows_fit) {
         for (int r0 = 1; r0 <= nr; r0 += RB * NT) {
             uint32_t w[RB];

@@ -186,8 +186,15 @@ struct NoLock {  // releases the interpreter lock
 std::mutex &stream_lock(int device, void *stream) {
     static std::mutex guard;
     static std::map<std::pair<int, void *>, std::mutex> locks;
-    std::lock_guard<std::mutex> g(guard);
-    return locks[{device, stream}];
+    thread_local std::pair<int, void *> last{-1, nullptr};
+    thread_local std::mutex *last_lock = nullptr;
+    const std::pair<int, void *> key{device, stream};
+    if (!last_lock || last != key) {
+        std::lock_guard<std::mutex> g(guard);
+        last_lock = &locks[key];
+        last = key;
+    }
+    return *last_lock;
 }
 
 // Runs a C-ABI call on the operands' device and the current stream of the caller, without the interpreter lock. A call
@@ -249,6 +256,8 @@ PyObject *csr_binary(csr2_fn fn, bool is_union, const char *where, PyObject *con
 PyObject *csr_add(PyObject *const *args) { return csr_binary(nb200_csr_add_f32_into, true, "gpu_csr_add_f32", args); }
 PyObject *csr_mul(PyObject *const *args) { return csr_binary(nb200_csr_mul_f32_into, false, "gpu_csr_mul_f32", args); }
 
+constexpr int64_t ADD3_POOL_BYTES = 8 << 20;
+
 PyObject *csr_add_3(PyObject *const *args) {
     const char *where = "gpu_csr_add_3_f32";
     for (int k = 0; k < 3; ++k) need_kind(args[k], CSR, where, "CSR_gpu");
@@ -257,8 +266,12 @@ PyObject *csr_add_3(PyObject *const *args) {
     same_device(va, vb);
     same_device(va, vc);
     const int64_t capacity = (int64_t)a.nnz + b.nnz + c.nnz;
-    // the intermediate sum is as large as the operands: it lies in an array of this call, not in the library's pool
+    // The intermediate sum is as large as the operands: it lies in an array of this call. Only a small one stays in the
+    // library's pool (the array costs half a microsecond).
     const int64_t scratch_bytes = nb200_csr_add_3_f32_scratch(&a, &b, &c);
+    if (scratch_bytes <= ADD3_POOL_BYTES)
+        return csr_result({&va, &vb, &vc}, where, a.rows, a.cols, capacity,
+                          [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_into(&a, &b, &c, z, capacity, stream); });
     at::Tensor scratch = array(scratch_bytes, at::kByte, va.device);
     return csr_result({&va, &vb, &vc}, where, a.rows, a.cols, capacity,
                       [&](nb200_csr *z, void *stream) { return nb200_csr_add_3_f32_lent(&a, &b, &c, z, capacity, scratch.data_ptr(), scratch_bytes, stream); });
