@@ -53,11 +53,6 @@ if ROOT not in sys.path:
 
 FALLBACK_HBM_GBS = 6650.0
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic byte of one launch
-# of a kernel, from one ncu capture of a reduced case each (profiles/*.md give the commands);
-# traffic grows in proportion to the entries, so the ratio is applied to the full launch.
-TRAFFIC_PER_ALGORITHMIC_BYTE = {"csr_add_fused": 0.816, "coo3_add_fused": 0.92}
-
 
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -708,8 +703,7 @@ def main():
             achieved = roof_bytes / (roof_ms * 1e-3) / 1e9
             roof = {"bound": "hbm", "kernel": roof_kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
                     "frac": achieved / peak, "peak_kind": f"{peak_kind} HBM copy bandwidth",
-                    "traffic": (TRAFFIC_PER_ALGORITHMIC_BYTE[top] * roof_bytes / max(kernels[top]["launches_per_step"], 1)
-                                if top in TRAFFIC_PER_ALGORITHMIC_BYTE else None),
+                    "traffic": None,  # DRAM bytes: no capture of the present kernels
                     "kernel_ms_per_step": roof_ms, "frac_of_nominal_8TBs": achieved / 8000.0,
                     "scope": "this rank's block" if world > 1 else "the whole workload"}
         base = None
