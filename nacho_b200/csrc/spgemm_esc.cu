@@ -13,9 +13,8 @@
 //   medium  P_i <= 256     one CTA per row: products in shared memory, bitonic sort there
 //   ranked  P_i <= 65535   one CTA per row: a bitmap of the produced columns in shared memory is
 //   heavy   P_i  > 65535   turned into the rank of every column within the result row, then every
-//                          product is added straight into its final position of C (float32
-//                          reductions in L2 on the row's own compact output range). Heavy rows
-//                          keep 32-bit ranks, take larger CTAs and start in order of weight.
+//                          product is added straight into its position of the row, in shared memory
+//                          where the row's result fits there. Heavy rows start in order of weight.
 // Matrices wider than the bitmap (262144 columns) are walked in column windows of that width.
 // Two passes: symbolic (unique columns per row -> row offsets by a scan) and numeric (fill).
 // Small and medium rows sum equal-column products in expansion order (ascending j), a fixed
@@ -24,8 +23,10 @@
 #include <climits>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "merge_common.cuh"
+#include "row_words.cuh"
 
 namespace nb200 {
 
@@ -38,7 +39,7 @@ constexpr int SMALL_P = 32;
 constexpr int MEDIUM_P = ESC_MEDIUM_P;
 constexpr int MED_NT = 128;
 constexpr unsigned long long RANKED_P = 65535;   // 16-bit ranks up to here
-constexpr unsigned long long GIANT_P = 1ull << 20;
+constexpr unsigned long long GIANT_P = 1ull << 18;
 
 struct CsrView {
     const int32_t *rp;
@@ -518,25 +519,30 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
 
 // ----------------------------------------------------------------- product walk ----
 
-constexpr int CHUNK = 32;           // products a warp takes with one instruction; a chunk lies in one row of B
-constexpr int FLIGHT = 4;  // chunks whose loads a warp keeps in flight (8 measured slower: registers; 2: 2616 against 2579 us)
+// A warp takes FLIGHT times 32 products at a time, in pieces that lie in one row of B each: of LONG products where there
+// are rows enough to keep the chip busy, because the broadcasts and addresses of a piece cost as much as 32 of its products
+// (pieces of 32 took 33 instructions per 32 products in the symbolic pass of 32768 vertices' heavy rows, of 128 take 23);
+// of SHORT products where there are few rows and the latency of each counts: the rows of B are then often shorter than LONG,
+// and the loads of four of them are in flight together (whole calls on graphs of 2698 / 9000 vertices 92 / 208 us, with LONG
+// pieces 105 / 235).
+constexpr int FLIGHT = 4, SHORT = 32, LONG = 32 * FLIGHT;
 
-// The rows of B that a chunk of A's row selects, as segments: segment k covers the chunks [first[k], first[k + 1]) of
-// the flat chunk sequence, and its products are the entries start[k] .. start[k] + len[k] - 1 of B, each multiplied by
+// The rows of B that a chunk of A's row selects, as segments: segment k covers the pieces [first[k], first[k + 1]) of
+// the flat sequence of pieces, and its products are the entries start[k] .. start[k] + len[k] - 1 of B, each multiplied by
 // a[k]. Only non-empty segments.
 template <int NT>
 struct Segments {
     int first[NT], start[NT], len[NT];
     float a[NT];
-    int n, chunks;
+    int n, pieces;
 };
 
 // Lists the segments of the CTA's threads ({start, len, a} of the thread's entry of A; len 0: none). All NT threads; ends
 // with a barrier. `tmp`: 72 ints.
-template <int NT>
+template <int NT, int PIECE>
 __device__ __forceinline__ void list_segments(Segments<NT> &seg, int *tmp, int32_t start, int len, float a) {
-    int k, off, n, chunks;
-    block_excl_sum2<NT>(len > 0 ? 1 : 0, (len + CHUNK - 1) / CHUNK, tmp, k, off, n, chunks);
+    int k, off, n, pieces;
+    block_excl_sum2<NT>(len > 0 ? 1 : 0, (len + PIECE - 1) / PIECE, tmp, k, off, n, pieces);
     if (len > 0) {
         seg.first[k] = off;
         seg.start[k] = start;
@@ -545,64 +551,70 @@ __device__ __forceinline__ void list_segments(Segments<NT> &seg, int *tmp, int32
     }
     if (threadIdx.x == 0) {
         seg.n = n;
-        seg.chunks = chunks;
+        seg.pieces = pieces;
     }
     __syncthreads();
 }
 
-// Walks all products of the segments: f(column, value). Every warp takes one contiguous share of the chunks. For 32 chunks
-// at a time every lane finds the segment of one of them by binary search; then the chunks go by one after the other, what
-// their lane knows broadcast, lane = product, so that the loads from B coalesce, nothing diverges, and FLIGHT chunks
-// have their loads in flight. (Products dealt out in a flat sequence, blocks of 128, took 44 instructions per 32 products
-// where the rows of B hold a hundred entries: the blocks cross rows, and every lane then searches its own. The symbolic
-// pass of 65536 vertices' heavy rows 375 -> 293 us, of 24405 vertices' 94 -> 63.)
-template <int NT, bool WITH_VALUES, typename F>
-__device__ __forceinline__ void walk_segments(const Segments<NT> &seg, const CsrView &B, F f) {
-    constexpr int NW = NT / 32;
-    const int lane = lane_id(), n_seg = seg.n, share = (seg.chunks + NW - 1) / NW;
-    const int c_end = min((warp_id() + 1) * share, seg.chunks);
-    for (int c = warp_id() * share; c < c_end; c += 32) {
-        const int mine = min(c + lane, c_end - 1);
-        int k = 0, above = n_seg;  // the last segment that begins at or before this lane's chunk
+// Walks all products of the segments: f(what load(position in B) gives, a). Every warp takes one contiguous share of the
+// pieces. For 32 pieces at a time every lane finds the segment of one of them by binary search; then the pieces go by one
+// after the other, what their lane knows broadcast, lane = product, so that the loads from B coalesce and nothing diverges.
+template <int NT, int PIECE, bool VALUES, typename Load, typename F>
+__device__ __forceinline__ void walk_segments(const Segments<NT> &seg, Load load, F f) {
+    constexpr int NW = NT / 32, TOGETHER = LONG / PIECE, EACH = PIECE / 32;  // pieces in flight, loads per lane of each
+    const int lane = lane_id(), n_seg = seg.n, share = (seg.pieces + NW - 1) / NW;
+    const int end = min((warp_id() + 1) * share, seg.pieces);
+    for (int c = warp_id() * share; c < end; c += 32) {
+        const int mine = min(c + lane, end - 1);
+        int k = 0, above = n_seg;  // the last segment that begins at or before this lane's piece
         while (above - k > 1) {
             const int mid = (k + above) >> 1;
             if (seg.first[mid] <= mine) k = mid; else above = mid;
         }
-        const int at = (mine - seg.first[k]) * CHUNK;
-        const int my_q = seg.start[k] + at, my_n = c + lane < c_end ? seg.len[k] - at : 0;
-        const float my_a = WITH_VALUES ? seg.a[k] : 0.f;
-        const int here = min(32, c_end - c);
-        for (int u = 0; u < here; u += FLIGHT) {
-            int32_t col[FLIGHT];
-            float val[FLIGHT];
+        const int at = (mine - seg.first[k]) * PIECE;
+        const int my_q = seg.start[k] + at, my_n = c + lane < end ? seg.len[k] - at : 0;
+        const float my_a = VALUES ? seg.a[k] : 0.f;
+        const int here = min(32, end - c);
+        for (int u = 0; u < here; u += TOGETHER) {  // (u + t stays below 32; pieces past the share have n = 0)
+            decltype(load(0)) x[FLIGHT];
+            float a[TOGETHER];
             unsigned live = 0;
 #pragma unroll
-            for (int j = 0; j < FLIGHT; ++j) {
-                const int q = __shfl_sync(FULL_MASK, my_q, u + j), n = __shfl_sync(FULL_MASK, my_n, u + j);
-                const bool ok = lane < n;  // chunks past the share have n = 0 (u + j stays below 32: FLIGHT divides it)
-                live |= (unsigned)ok << j;
-                col[j] = ok ? ld_nc(B.col + q + lane) : 0;
-                if (WITH_VALUES) val[j] = ok ? ld_nc(B.val + q + lane) : 0.f;
+            for (int t = 0; t < TOGETHER; ++t) {
+                const int q = __shfl_sync(FULL_MASK, my_q, u + t) + lane, n = __shfl_sync(FULL_MASK, my_n, u + t) - lane;
+                a[t] = VALUES ? __shfl_sync(FULL_MASK, my_a, u + t) : 0.f;
+#pragma unroll
+                for (int j = 0; j < EACH; ++j)
+                    if (32 * j < n) {
+                        x[t * EACH + j] = load(q + 32 * j);
+                        live |= 1u << (t * EACH + j);
+                    }
             }
 #pragma unroll
-            for (int j = 0; j < FLIGHT; ++j) {
-                const float a = WITH_VALUES ? __shfl_sync(FULL_MASK, my_a, u + j) : 0.f;
-                if ((live >> j) & 1u) f(col[j], WITH_VALUES ? a * val[j] : 0.f);
-            }
+            for (int j = 0; j < FLIGHT; ++j)
+                if ((live >> j) & 1u) f(x[j], a[j / EACH]);
         }
     }
 }
 
 // ------------------------------------------------------------- ranked and heavy rows ----
+//
+// Rows of more than MEDIUM_P products. The symbolic pass (k_esc_mark) sets a bit per produced column in a shared-memory
+// bitmap and counts; its bitmaps are kept for the numeric pass (k_esc_rank), which turns them into the rank of every
+// word's columns within the result row, writes the row's columns, walks the products and adds each one into its position.
+// Matrices wider than one bitmap are walked in column windows.
 
 constexpr int RK_WORDS = 8192;                     // bitmap words of one column window in shared memory
 constexpr int RK_WINDOW_COLS = RK_WORDS * 32;      // 262144 columns per window
-constexpr size_t RK_WORD_BYTES = 6;                // shared memory per bitmap word of a numeric launch: the word and its rank
 constexpr size_t RK_PTR_BUDGET = size_t(1) << 30;  // bytes of the window pointer table; beyond it windows are searched on the fly
-constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a CTA for rows up to / above RANKED_P products
-constexpr size_t HEAVY_SMEM_NUMERIC = 104 * 1024;  // dynamic shared memory of a numeric heavy-row CTA: two per SM
-constexpr int RK_MANY_ROWS = 8192;                 // from this many ranked rows on, their CTAs hold sums in shared memory too
-constexpr size_t RK_SMEM_NUMERIC = 32 * 1024;      // dynamic shared memory of such a CTA: bitmap, ranks, then sums
+constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a symbolic CTA for rows up to / above RANKED_P products
+constexpr int MANY_NT = 128, MANY_ROWS = 8192;     // ... and up to RANKED_P where there are many
+
+// Where the word w of a window lies in shared memory. The low bits of a graph's column numbers are far from uniform (in an
+// R-MAT graph each is 0 three times in four, so a quarter of all words would lie in one bank; random look-ups with that skew
+// take 8 cycles per warp instead of 3); folding the bits above into them spreads the banks. One to one on any power
+// of two of words.
+__device__ __forceinline__ uint32_t spread(uint32_t w) { return w ^ (w >> 4) ^ (w >> 8); }
 
 // First index in [lo, hi) whose column is >= key (hi if none).
 __device__ __forceinline__ int32_t first_col_at_least(const int32_t *__restrict__ col, int32_t lo, int32_t hi, int64_t key) {
@@ -629,177 +641,338 @@ __global__ void __launch_bounds__(256) k_esc_window_ptr(CsrView B, int32_t b_row
     ptr[t] = w == 0 ? lo : w == n_win ? hi : first_col_at_least(B.col, lo, hi, (int64_t)w * RK_WINDOW_COLS);
 }
 
-// One CTA per row, column window by column window (one window unless B is wider than
-// RK_WINDOW_COLS). Per window: pass 1 walks the row's products and sets a bit per produced column
-// in a shared-memory bitmap; a popcount scan turns the bitmap into the rank of every column within
-// the result row and the columns are written out; pass 2 walks the products again and adds each
-// one into its final position: the first `acc_slots` positions of the window accumulate in shared
-// memory (float32 atomics there run several times faster than reductions in L2) and are stored
-// with coalesced writes at the end, the positions beyond them take a float32 reduction in L2 on
-// the row's own output range, which this CTA zeroed first. Symbolic: pass 1 and the count only.
+// Column windows of B: their number, and the window pointer table (null: one window, or a table beyond its budget).
+struct Windows {
+    int n;
+    const int32_t *ptr;
+    // The entries of row j whose columns lie in window w.
+    __device__ __forceinline__ void range(const CsrView &B, int32_t j, int w, int32_t &start, int32_t &len) const {
+        if (n == 1) {
+            start = ld_nc(B.rp + j);
+            len = ld_nc(B.rp + j + 1) - start;
+        } else if (ptr) {
+            const int64_t at = (int64_t)j * (n + 1) + w;
+            start = ld_nc(ptr + at);
+            len = ld_nc(ptr + at + 1) - start;
+        } else {
+            const int32_t b_lo = ld_nc(B.rp + j), b_hi = ld_nc(B.rp + j + 1), c_first = w * RK_WINDOW_COLS;
+            start = w == 0 ? b_lo : first_col_at_least(B.col, b_lo, b_hi, c_first);
+            len = (w == n - 1 ? b_hi : first_col_at_least(B.col, start, b_hi, (int64_t)c_first + RK_WINDOW_COLS)) - start;
+        }
+    }
+};
+
+// The entries of A's row and the walks over what they select, NT entries at a time (a thread keeps its entry where one
+// chunk is all).
+template <int NT, int PIECE, bool VALUES>
+struct RowWalk {
+    int32_t lo, hi, my_j = -1;
+    float my_a = 0.f;
+    __device__ __forceinline__ RowWalk(const CsrView &A, int32_t i) : lo(ld_nc(A.rp + i)), hi(ld_nc(A.rp + i + 1)) {
+        if (one_chunk()) fetch(A, lo);
+    }
+    __device__ __forceinline__ bool one_chunk() const { return hi - lo <= NT; }
+    __device__ __forceinline__ void fetch(const CsrView &A, int32_t chunk) {
+        my_j = -1;
+        if (chunk + (int)threadIdx.x >= hi) return;
+        my_j = ld_nc(A.col + chunk + threadIdx.x);
+        if (VALUES) my_a = ld_nc(A.val + chunk + threadIdx.x);
+    }
+    // range(j, start, len) gives the segment of an entry. `build` false: the segments of a single chunk are there already.
+    // Returns whether there was any segment; ends with a barrier.
+    template <typename Range, typename Load, typename F>
+    __device__ __forceinline__ bool run(const CsrView &A, Segments<NT> &seg, int *tmp, bool build, Range range, Load load, F f) {
+        bool any = false;
+        for (int32_t chunk = lo; chunk < hi; chunk += NT) {
+            if (build) {
+                if (!one_chunk()) fetch(A, chunk);
+                int32_t start = 0, len = 0;
+                if (my_j >= 0) range(my_j, start, len);
+                list_segments<NT, PIECE>(seg, tmp, start, len, my_a);
+            }
+            any |= seg.n > 0;
+            walk_segments<NT, PIECE, VALUES>(seg, load, f);
+            __syncthreads();  // the segment arrays are rewritten by the next chunk
+        }
+        return any;
+    }
+};
+
+// Symbolic pass, one CTA per row: a bit per produced column, window by window, and their number. WORDS: the rows of B are
+// walked as bitmap words (row_words.cuh), one window only. `row_list` is read from the front for the first n_front CTAs and from the back (list_len - 1
+// downwards) for the others. `words`: bitmap words in use, a power of two of at least 128. `cache` (one window only), when
+// given, receives the bitmaps, `words` per CTA, word w at place w.
 //
-// Ranks are kept in 16 bits per bitmap word. Positions fit them in rows of at most 65535 products and in windows of at
-// most 65536 columns; otherwise (FAR) a rank counts from the first word of the warp that scanned it (a warp scans
-// `1 << wshift` consecutive words, at most 32768 columns), and there is one base per warp. The walk of pass 2 is bound
-// by the instructions it issues per product, so a look-up is two loads and a popcount of one word (a rank per 64
-// columns and a base per warp for every row took three loads and twice the instructions).
-//
-// `row_list` is read from the front for the first n_front CTAs and from the back (list_len - 1
-// downwards) for the others. `words`: bitmap words in use, (NT / 32) << wshift, covering a window.
-// `win_ptr` is the window pointer table, or null (one window, or a table beyond its budget).
-// `cache` (one window only), when given, carries the bitmaps from the symbolic launch to the
-// numeric launch of one call, `words` per CTA: the symbolic launch stores them, the numeric
-// launch loads them instead of walking the products a first time.
-template <bool NUMERIC, int NT, bool FAR>
-__global__ void __launch_bounds__(NT) k_esc_ranked(CsrView A, CsrView B, const int32_t *__restrict__ win_ptr, int n_win,
-                                                   const int32_t *__restrict__ row_list, int32_t list_len, int n_front, int words,
-                                                   int wshift, int acc_slots, uint32_t *cache, int32_t *__restrict__ row_count,
-                                                   const int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col,
-                                                   float *__restrict__ c_val) {
+// Bound by instructions and shared-memory wavefronts together; a pass over entries instead of words sets twice the bits.
+template <int NT, int PIECE, bool WORDS>
+__global__ void __launch_bounds__(NT, 1536 / NT) k_esc_mark(CsrView A, CsrView B, RowWords B_words, Windows windows, const int32_t *__restrict__ row_list,
+                                                 int32_t list_len, int n_front, int words, uint4 *cache, int32_t *__restrict__ row_count) {
     extern __shared__ __align__(16) unsigned char rk_smem[];
     uint32_t *bitmap = reinterpret_cast<uint32_t *>(rk_smem);
-    const uint64_t *bitmap64 = reinterpret_cast<const uint64_t *>(rk_smem);  // the same bits, 64 columns per element
-    uint16_t *rank16 = reinterpret_cast<uint16_t *>(rk_smem + (size_t)words * 4);  // one rank per 32 columns
-    float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * RK_WORD_BYTES);
     __shared__ Segments<NT> seg;
     __shared__ int scan_tmp[72];
-    __shared__ int warp_base[NT / 32];
+    __shared__ int s_count;
     trigger_dependents();
-    const int tid = threadIdx.x;
-    const int r = blockIdx.x;
+    const int tid = threadIdx.x, r = blockIdx.x;
     const int32_t i = ld_nc(row_list + (r < n_front ? r : list_len - 1 - (r - n_front)));
-    const int32_t lo = ld_nc(A.rp + i), hi = ld_nc(A.rp + i + 1);
-    const bool one_chunk = hi - lo <= NT;  // then a thread keeps its entry, and pass 2 reuses the segments of pass 1
-    const int per = n_win + 1;
-    int32_t my_j = -1;
-    float my_a = 0.f;
-    if (one_chunk && lo + tid < hi) {
-        my_j = ld_nc(A.col + lo + tid);
-        if (NUMERIC) my_a = ld_nc(A.val + lo + tid);
-    }
-    int64_t out = NUMERIC ? (int64_t)ld_nc(c_rp + i) : 0;  // next free position of the row (count so far, symbolic)
-
-    for (int w = 0; w < n_win; ++w) {
+    RowWalk<NT, PIECE, false> row(A, i);
+    if (tid == 0) s_count = 0;
+    int count = 0;
+    for (int w = 0; w < windows.n; ++w) {
         const int32_t c_first = w * RK_WINDOW_COLS;  // below 2^31: it is a column of B
-
-        // builds the segments of one chunk of the row's entries (their rows of B inside the window)
-        // and walks them; returns whether the window holds any product
-        auto pass = [&](bool build, auto f) -> bool {
-            bool any = false;
-            for (int32_t chunk = lo; chunk < hi; chunk += NT) {
-                if (build) {
-                    int32_t j = my_j;
-                    float a = my_a;
-                    if (!one_chunk) {
-                        j = -1;
-                        if (chunk + tid < hi) {
-                            j = ld_nc(A.col + chunk + tid);
-                            if (NUMERIC) a = ld_nc(A.val + chunk + tid);
-                        }
-                    }
-                    int32_t s = 0, len = 0;
-                    if (j >= 0) {
-                        if (n_win == 1) {
-                            s = ld_nc(B.rp + j);
-                            len = ld_nc(B.rp + j + 1) - s;
-                        } else if (win_ptr) {
-                            s = ld_nc(win_ptr + (int64_t)j * per + w);
-                            len = ld_nc(win_ptr + (int64_t)j * per + w + 1) - s;
-                        } else {
-                            const int32_t b_lo = ld_nc(B.rp + j), b_hi = ld_nc(B.rp + j + 1);
-                            s = w == 0 ? b_lo : first_col_at_least(B.col, b_lo, b_hi, c_first);
-                            len = (w == n_win - 1 ? b_hi : first_col_at_least(B.col, s, b_hi, (int64_t)c_first + RK_WINDOW_COLS)) - s;
-                        }
-                    }
-                    list_segments<NT>(seg, scan_tmp, s, len, a);
-                }
-                any |= seg.n > 0;
-                walk_segments<NT, NUMERIC>(seg, B, f);
-                __syncthreads();  // the segment arrays are rewritten by the next chunk
-            }
-            return any;
-        };
-
-        uint4 *cached = cache ? reinterpret_cast<uint4 *>(cache + (size_t)r * words) : nullptr;
-        const bool from_cache = NUMERIC && cached != nullptr;
-        if (from_cache) {
-            for (int c = tid; c < words / 4; c += NT) reinterpret_cast<uint4 *>(bitmap)[c] = __ldcs(cached + c);
-            __syncthreads();
+        for (int c = tid; c < words / 4; c += NT) reinterpret_cast<uint4 *>(bitmap)[c] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        bool any;
+        if (WORDS) {
+            any = row.run(A, seg, scan_tmp, true, [&](int32_t j, int32_t &start, int32_t &len) {
+                start = ld_nc(B_words.rp + j);
+                len = ld_nc(B_words.rp + j + 1) - start;
+            }, [&](int q) { return __ldg(B_words.items + q); }, [&](uint2 item, float) { atomicOr(bitmap + spread(item.x), item.y); });
         } else {
-            for (int c = tid; c < words / 4; c += NT) reinterpret_cast<uint4 *>(bitmap)[c] = make_uint4(0u, 0u, 0u, 0u);
-            __syncthreads();
-            const bool any = pass(true, [&](int32_t col, float) {
-                const uint32_t cw = (uint32_t)(col - c_first);
-                atomicOr(bitmap + (cw >> 5), 1u << (cw & 31u));
-            });
-            if (!any) continue;  // uniform
-            if (!NUMERIC && cached)
-                for (int c = tid; c < words / 4; c += NT) __stcs(cached + c, reinterpret_cast<const uint4 *>(bitmap)[c]);
+            any = row.run(A, seg, scan_tmp, true, [&](int32_t j, int32_t &start, int32_t &len) { windows.range(B, j, w, start, len); },
+                          [&](int q) { return ld_nc(B.col + q); }, [&](int32_t col, float) {
+                              const uint32_t cw = (uint32_t)(col - c_first);
+                              atomicOr(bitmap + spread(cw >> 5), 1u << (cw & 31u));
+                          });
         }
-
-        // warp v looks after the words [v << wshift, (v + 1) << wshift), 64 columns per lane and step
-        const int groups = 1 << (wshift - 6);
-        const int dbase = warp_id() << (wshift - 1);  // first 64-bit element of the warp
-        int mine = 0;
-#pragma unroll 4
-        for (int g = 0; g < groups; ++g) mine += __popcll(bitmap64[dbase + g * 32 + lane_id()]);
-        int cnt;
-        const int excl = block_excl_sum<NT>(mine, scan_tmp, cnt);
-        if (!NUMERIC) {
-            out += cnt;
-            continue;
+        if (!any) continue;  // uniform
+        for (int q = tid; q < words / 4; q += NT) {
+            uint4 v;
+            v.x = bitmap[spread(4 * q)], v.y = bitmap[spread(4 * q + 1)], v.z = bitmap[spread(4 * q + 2)], v.w = bitmap[spread(4 * q + 3)];
+            count += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+            if (cache) __stcs(cache + (size_t)r * (words / 4) + q, v);
         }
-        const int my_base = __shfl_sync(FULL_MASK, excl, 0);  // columns of the window before this warp's words
-        if (FAR && lane_id() == 0) warp_base[warp_id()] = my_base;
-        int running = 0;
-#pragma unroll 2
-        for (int g = 0; g < groups; ++g) {
-            const int idx = dbase + g * 32 + lane_id();
-            uint64_t bits = bitmap64[idx];
-            const int c = __popcll(bits);
-            const int incl = warp_incl_sum(c);
-            const int first = running + incl - c;
-            const uint32_t rank = (uint32_t)(FAR ? first : my_base + first);
-            reinterpret_cast<uint32_t *>(rank16)[idx] = (rank & 0xffffu) | (rank + __popc((uint32_t)bits)) << 16;
-            // the lane's columns, in 32-bit halves and 32-bit positions (the loop is the hot part of
-            // the scan: one trip per result entry)
-            int32_t *gcol = c_col + (out + my_base);
-            int pos = first;
-            uint32_t half = (uint32_t)bits;
-            int32_t col0 = c_first + idx * 64;
-            while (half) {
-                gcol[pos++] = col0 + (__ffs((int)half) - 1);
-                half &= half - 1u;
-            }
-            half = (uint32_t)(bits >> 32);
-            col0 += 32;
-            while (half) {
-                gcol[pos++] = col0 + (__ffs((int)half) - 1);
-                half &= half - 1u;
-            }
-            running += __shfl_sync(FULL_MASK, incl, 31);
-        }
-        float *row_val = c_val + out;  // the window's part of the row; its length fits 32 bits
-        const int in_acc = min(cnt, acc_slots);
-        for (int k = tid; k < in_acc; k += NT) acc[k] = 0.f;
-        for (int k = acc_slots + tid; k < cnt; k += NT) row_val[k] = 0.f;  // positions beyond the shared accumulator
-        __syncthreads();  // ranks complete, output zeroed (the reductions below come from this CTA only)
-        pass(!one_chunk || from_cache, [&](int32_t col, float v) {
-            const uint32_t cw = (uint32_t)(col - c_first);
-            const uint32_t word = cw >> 5;
-            // columns of the word up to and with this one, whose bit is set: the position plus one
-            uint32_t next = (uint32_t)rank16[word] + __popc(bitmap[word] << (~cw & 31u));
-            if (FAR) next += (uint32_t)warp_base[word >> wshift];
-            if (next <= (uint32_t)acc_slots)
-                atomicAdd(acc - 1 + next, v);      // shared memory
-            else
-                atomicAdd(row_val - 1 + next, v);  // reduction in L2
-        });
-        // the pass ends with a barrier: every sum is in place
-        for (int k = tid; k < in_acc; k += NT) row_val[k] = acc[k];
-        out += cnt;
+        __syncthreads();  // the next window clears the bitmap
     }
-    if (!NUMERIC && tid == 0) row_count[i] = (int32_t)out;
+    count = __reduce_add_sync(FULL_MASK, count);
+    if (lane_id() == 0 && count) atomicAdd(&s_count, count);
+    __syncthreads();
+    if (tid == 0) row_count[i] = s_count;
+    finish_after_previous();
+}
+
+// The rows of the heavy and the ranked list, numbered through: heavy rows first (giant ones from the front of their list,
+// the others from its back). The number is also the place of a row's bitmap.
+struct ListedRows {
+    const int32_t *heavy_rows, *ranked_rows;
+    int32_t rows;  // length of the heavy list
+    int n_giant, n_heavy, n;
+    __device__ __forceinline__ int32_t row(int t) const {
+        return t < n_giant ? ld_nc(heavy_rows + t) : t < n_heavy ? ld_nc(heavy_rows + rows - 1 - (t - n_giant)) : ld_nc(ranked_rows + (t - n_heavy));
+    }
+};
+
+// The numeric pass takes its rows by the length of their results: a row's sums, four bytes per entry, should lie in shared
+// memory (float32 atomics there run at 960 G per second, reductions in L2 at 182), and the shorter the rows the more CTAs
+// share an SM. A class holds the rows whose results fit what its CTAs have beside the table of words; what does not fit the
+// last one keeps the rest of its sums in L2.
+struct RankClass {
+    int nt, per_sm;       // threads of a CTA, CTAs of an SM
+    size_t smem;          // dynamic shared memory of a CTA
+    bool columns_walked;  // the walk of the products notes their columns, in shared memory too (below)
+    int piece;
+};
+constexpr int CLASSES = 5, FEW = 5, FEW_HEAVY = 6;  // the last two: where there are few rows they are not sorted by class
+constexpr RankClass RANK_CLASS[] = {{128, 8, 25 * 1024, true, LONG},  {256, 4, 50 * 1024, true, LONG},    {320, 3, 68 * 1024, true, LONG},   {512, 2, 104 * 1024, true, LONG},
+                                    {1024, 1, 208 * 1024, false, LONG}, {256, 6, 0, false, SHORT}, {1024, 1, 208 * 1024, false, SHORT}};
+constexpr int NARROW_WORDS = 2048;  // windows of up to 65536 columns: the table has 16 columns and their rank in 32 bits
+// Sums of a CTA of class `cls` beside a table of `words` bitmap words.
+constexpr int rank_slots(int cls, int words) {
+    const bool narrow = words <= NARROW_WORDS;
+    const size_t table = (size_t)words * 8, slot = !RANK_CLASS[cls].columns_walked ? 4 : narrow ? 6 : 8;
+    return RANK_CLASS[cls].smem < table + 1024 ? 0 : (int)((RANK_CLASS[cls].smem - table) / slot) & ~1;
+}
+
+struct ClassSlots {
+    int slots[CLASSES];
+};
+struct ClassCtl {
+    int count[CLASSES], ticket[CLASSES];
+};
+
+// Puts the listed rows on the list of their class (`stride` apart): {row, place of its bitmap}, the heaviest first as far as
+// the order of the CTAs goes.
+__global__ void __launch_bounds__(256) k_esc_classes(ListedRows listed, const int32_t *__restrict__ c_rp, const ClassSlots most, int2 *__restrict__ out,
+                                                     int64_t stride, ClassCtl *ctl) {
+    __shared__ int s_count[CLASSES];
+    if (threadIdx.x < CLASSES) s_count[threadIdx.x] = 0;
+    __syncthreads();
+    const int t = blockIdx.x * 256 + threadIdx.x;
+    int cls = -1, at = 0;
+    int32_t row = 0;
+    if (t < listed.n) {
+        row = listed.row(t);
+        const int32_t length = ld_nc(c_rp + row + 1) - ld_nc(c_rp + row);
+        cls = 0;
+#pragma unroll
+        for (int k = 0; k < CLASSES - 1; ++k) cls += length > most.slots[k] ? 1 : 0;  // slots grow with the class
+        at = atomicAdd(&s_count[cls], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < CLASSES && s_count[threadIdx.x] > 0) s_count[threadIdx.x] = atomicAdd(&ctl->count[threadIdx.x], s_count[threadIdx.x]);
+    __syncthreads();
+    if (cls >= 0) out[cls * stride + s_count[cls] + at] = make_int2(row, t);
+}
+
+// Column and value of every entry of B side by side: a product of the numeric pass is one 8-byte load.
+__global__ void __launch_bounds__(256) k_esc_pairs(const int32_t *__restrict__ rp, const int32_t *__restrict__ col, const float *__restrict__ val, int32_t nnz,
+                                                   uint2 *__restrict__ pairs) {
+    const int64_t p = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (p >= nnz) return;
+    const int64_t at = (int64_t)ld_nc(rp) + p;
+    pairs[p] = make_uint2((uint32_t)ld_nc(col + at), __float_as_uint(ld_nc(val + at)));
+}
+
+// The columns of a window and their ranks, by bitmap words. NARROW: 16 columns in the lower half of a 32-bit word, the
+// number of columns before them in the upper one (a look-up is one 4-byte load: 3 cycles of the shared-memory pipe for
+// random words against 5 for 8 bytes); otherwise 32 columns and their rank in 64 bits.
+template <bool NARROW>
+struct RankTable {
+    unsigned char *at;
+    __device__ __forceinline__ uint32_t &half(uint32_t h) const { return reinterpret_cast<uint32_t *>(at)[h ^ (h >> 5) ^ (h >> 10)]; }
+    __device__ __forceinline__ uint2 &full(uint32_t w) const { return reinterpret_cast<uint2 *>(at)[spread(w)]; }
+    __device__ __forceinline__ void mark(uint32_t cw) const {  // column cw of the window, in a table of zeros
+        if (NARROW) atomicOr(&half(cw >> 4), 1u << (cw & 15u));
+        else atomicOr(&full(cw >> 5).x, 1u << (cw & 31u));
+    }
+    __device__ __forceinline__ uint32_t marked(uint32_t w) const { return NARROW ? half(2 * w) | half(2 * w + 1) << 16 : full(w).x; }
+    __device__ __forceinline__ void put(uint32_t w, uint32_t bits, uint32_t rank) const {
+        if (NARROW) {
+            half(2 * w) = (bits & 0xffffu) | rank << 16;
+            half(2 * w + 1) = bits >> 16 | (rank + __popc(bits & 0xffffu)) << 16;
+        } else {
+            full(w) = make_uint2(bits, rank);
+        }
+    }
+    // columns up to and with cw, which is one of them: its position plus one
+    __device__ __forceinline__ uint32_t find(uint32_t cw) const {
+        if (NARROW) {
+            const uint32_t e = half(cw >> 4);
+            return (e >> 16) + __popc(e << (31u - (cw & 15u)));
+        }
+        const uint2 e = full(cw >> 5);
+        return e.y + __popc(e.x << (~cw & 31u));
+    }
+};
+
+// Numeric pass, one CTA per row: CTAs take the rows of a class from a ticket; where rows are not sorted by class, CTA t takes
+// the listed row first + t. Per window the row's bitmap, from the symbolic pass's store or from a walk of its own, becomes the table
+// of ranks; the products are walked and each one added into its position: a look-up, a popcount and an atomic. Positions beyond
+// `acc_slots` (last class; all of them where there are few rows, which the latency of shared-memory atomics would hold up) take a float32
+// reduction in L2 on the row's own output range, which this CTA zeroed first. The columns are noted by the products themselves
+// (WALKED) or written out of the bitmap into the place of the sums before the walk; both ways they are stored coalesced. (Out of the
+// bitmap every lane loops over the bits of its words, and a warp over those of its densest: rows of up to 6144 entries spent a
+// third of their instructions there. The longest rows, 7 products per entry, still do it.)
+//
+// `pairs`: B's entries as {column, value}, or null. What bounds it is the shared-memory pipe beside latency: per 32 products 3
+// cycles for the pairs, 3 for the look-up, 3 for noting the column, 10 for the atomic, of 28 to 34 that it takes at 32 to
+// 40 warps per SM. R-MAT graph of 65536 vertices times its transpose (403 M products): both passes of these rows 2.2 ms with entries
+// instead of words in the symbolic one, 5120 sums in shared memory and the others in L2, columns out of the bitmap; 1.5 ms now.
+template <int CLS, bool NARROW, bool PAIRS>
+__global__ void __launch_bounds__(RANK_CLASS[CLS].nt, RANK_CLASS[CLS].per_sm)
+    k_esc_rank(CsrView A, CsrView B, const uint2 *pairs, Windows windows, ListedRows listed, int first, int last, const int2 *list, ClassCtl *ctl, int words,
+               int acc_slots, const uint4 *cache, const int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col, float *__restrict__ c_val) {
+    constexpr RankClass K = RANK_CLASS[CLS];
+    constexpr int NT = K.nt;
+    constexpr bool WALKED = K.columns_walked, BY_CLASS = CLS < CLASSES, IN_L2 = K.smem == 0;
+    using Col = typename std::conditional<NARROW, uint16_t, uint32_t>::type;
+    extern __shared__ __align__(16) unsigned char rk_smem[];
+    const RankTable<NARROW> table{rk_smem};
+    float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * 8);
+    int32_t *stage = reinterpret_cast<int32_t *>(acc);
+    Col *noted = reinterpret_cast<Col *>(acc + acc_slots);  // WALKED
+    __shared__ Segments<NT> seg;
+    __shared__ int scan_tmp[72];
+    __shared__ int s_next;
+    trigger_dependents();
+    const int tid = threadIdx.x, count = BY_CLASS ? ctl->count[BY_CLASS ? CLS : 0] : last;
+    const int quads = words / 4, per = quads >= NT ? 4 * ((quads + NT - 1) / NT) : (words + NT - 1) / NT;  // neighbouring words fall to one thread
+    const int w_lo = min(tid * per, words), w_hi = min(w_lo + per, words);
+    const int32_t b_base = PAIRS ? ld_nc(B.rp) : 0;
+    auto load = [&](int q) -> uint2 {
+        return PAIRS ? __ldg(pairs + (q - b_base)) : make_uint2((uint32_t)ld_nc(B.col + q), __float_as_uint(ld_nc(B.val + q)));
+    };
+    if (BY_CLASS) {
+        if (tid == 0) s_next = atomicAdd(&ctl->ticket[BY_CLASS ? CLS : 0], 1);
+        __syncthreads();
+    }
+    for (;;) {
+        const int r = BY_CLASS ? s_next : first + (int)blockIdx.x;
+        if (r >= count) break;  // uniform
+        int next = count;
+        if (BY_CLASS && tid == 0) next = atomicAdd(&ctl->ticket[BY_CLASS ? CLS : 0], 1);
+        const int2 at = BY_CLASS ? list[r] : make_int2(listed.row(r), r);
+        const int32_t i = at.x;
+        RowWalk<NT, K.piece, true> row(A, i);
+        int64_t out = ld_nc(c_rp + i);  // next free position of the row
+        for (int w = 0; w < windows.n; ++w) {
+            const int32_t c_first = w * RK_WINDOW_COLS;  // below 2^31: it is a column of B
+            auto range = [&](int32_t j, int32_t &start, int32_t &len) { windows.range(B, j, w, start, len); };
+            const uint4 *from = cache ? cache + (size_t)at.y * quads : nullptr;
+            if (!cache) {
+                for (int c = tid; c < words; c += NT) reinterpret_cast<uint2 *>(rk_smem)[c] = make_uint2(0u, 0u);
+                __syncthreads();
+                const bool any = row.run(A, seg, scan_tmp, true, range, [&](int q) { return ld_nc(B.col + q); },
+                                         [&](int32_t col, float) { table.mark((uint32_t)(col - c_first)); });
+                if (!any) continue;  // uniform
+            }
+            auto each_word = [&](auto f) {  // f(word, bits) for the thread's words
+                if (!cache) {
+                    for (int c = w_lo; c < w_hi; ++c) f(c, table.marked(c));
+                } else if (quads >= NT) {
+                    for (int c = w_lo; c < w_hi; c += 4) {
+                        const uint4 v = __ldg(from + c / 4);
+                        f(c, v.x), f(c + 1, v.y), f(c + 2, v.z), f(c + 3, v.w);
+                    }
+                } else {
+                    for (int c = w_lo; c < w_hi; ++c) f(c, __ldg(reinterpret_cast<const uint32_t *>(from) + c));
+                }
+            };
+            int mine = 0;
+            each_word([&](int, uint32_t bits) { mine += __popc(bits); });
+            int cnt;
+            int rank = block_excl_sum<NT>(mine, scan_tmp, cnt);
+            const bool fits = !IN_L2 && cnt <= acc_slots;
+            each_word([&](int c, uint32_t bits) {
+                table.put(c, bits, rank);
+                if (WALKED) {
+                    rank += __popc(bits);
+                } else {
+                    const int32_t col0 = c_first + c * 32 - 1;
+                    if (fits) {
+                        for (; bits; bits &= bits - 1u) stage[rank++] = col0 + __ffs((int)bits);
+                    } else {
+                        for (; bits; bits &= bits - 1u) c_col[out + rank++] = col0 + __ffs((int)bits);
+                    }
+                }
+            });
+            if (!WALKED && !IN_L2) __syncthreads();
+            float *row_val = c_val + out;  // the window's part of the row; its length fits 32 bits
+            const int in_acc = IN_L2 ? 0 : min(cnt, acc_slots);
+            for (int k = tid; k < in_acc; k += NT) {
+                if (!WALKED && fits) c_col[out + k] = stage[k];
+                acc[k] = 0.f;
+            }
+            if (!WALKED) for (int k = (IN_L2 ? 0 : acc_slots) + tid; k < cnt; k += NT) row_val[k] = 0.f;  // positions beyond the shared sums
+            __syncthreads();  // table complete, sums zeroed (the reductions below come from this CTA only)
+            row.run(A, seg, scan_tmp, cache || !row.one_chunk(), range, load, [&](uint2 product, float a) {
+                const uint32_t cw = product.x - (uint32_t)c_first, to = table.find(cw) - 1;
+                const float v = a * __uint_as_float(product.y);
+                if (WALKED) noted[to] = (Col)cw;
+                if (WALKED || (!IN_L2 && to < (uint32_t)acc_slots)) atomicAdd(acc + to, v);
+                else atomicAdd(row_val + to, v);  // reduction in L2
+            });
+            // the pass ends with a barrier: every sum is in place
+            for (int k = tid; k < in_acc; k += NT) {
+                if (WALKED) c_col[out + k] = c_first + (int32_t)noted[k];
+                row_val[k] = acc[k];
+            }
+            out += cnt;
+        }
+        if (!BY_CLASS) break;
+        if (tid == 0) s_next = next;
+        __syncthreads();  // also: this row's sums are stored before the next row's take their place
+    }
     finish_after_previous();
 }
 
@@ -920,16 +1093,13 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
 
 // ------------------------------------------------------------------------ host driver ----
 
-// Bitmap words a ranked-row CTA keeps for B's column count (one window's worth at most): every
-// warp scans a power of two of words, at least 64. `wshift` receives log2 of that count.
-int ranked_words(int nt, int32_t b_cols, int *wshift = nullptr) {
+// Bitmap words of a row for B's column count (one window's worth at most): a power of two.
+int ranked_words(int32_t b_cols) {
     const int64_t need = (std::min<int64_t>(b_cols, RK_WINDOW_COLS) + 31) / 32;
-    int shift = 6;
-    while (((int64_t)(nt / 32) << shift) < need) ++shift;
-    if (wshift) *wshift = shift;
-    return (nt / 32) << shift;
+    int words = 128;
+    while (words < need) words *= 2;
+    return words;
 }
-
 
 int check_operand(const nb200_csr *m) {
     if (!m || m->rows < 0 || m->cols < 0 || m->nnz < 0 || !m->row_ptr) return NB200_E_BADARG;
@@ -946,17 +1116,25 @@ struct EscPlan {
     EscCtl *ctl;
     int n_win;             // column windows of RK_WINDOW_COLS
     int32_t *win_ptr;      // window pointer table (null: one window, or beyond its budget)
-    uint32_t *cache_ranked, *cache_heavy;  // bitmaps carried from the symbolic to the numeric pass (or null)
+    int words;             // bitmap words of a row in a window
+    uint4 *cache;          // bitmaps carried from the symbolic to the numeric pass, heavy rows first (or null)
+    int2 *class_rows;      // rows of every class, as many apart as there are rows above MEDIUM_P products (null: few rows, in one launch)
+    ClassCtl *classes;
+    RowWords b_words;      // rows of B as bitmap words for the symbolic pass (or null)
     Workspace *cache_ws;   // pool block of the bitmaps (null without them)
     EscCtl host;           // counters reported by the binning kernel
     uint64_t *short_block; // FusedCtl + tile words of the short-row kernel
     int short_tiles;
-    unsigned long long *words;
+    unsigned long long *result;  // result words
 };
 
 // Bins the rows (kernel + one read-back) and carves the scratch of a symbolic pass, a numeric
 // pass, or one after the other. `counts`: rows without products get their count written
 // (needed by the symbolic pass).
+// Another form of B is made for products that read every entry of it this often, and of which there are this many: its words take
+// four short launches (some 25 us with nothing beside them), its pairs one of 9. A graph of 24405 vertices, 49 M products:
+// the whole call 468 -> 357 us with both and the classes; of 9000 vertices, 7 M products, it would take 20 us more.
+constexpr unsigned long long REUSE = 16, FORMS_FROM = 32 << 20;
 constexpr size_t BITMAP_CACHE_BUDGET = size_t(8) << 30;  // bytes of bitmaps carried between the passes of one call
 
 int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_bitmaps, cudaStream_t stream, EscPlan *plan) {
@@ -968,6 +1146,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     Carver sizes;
     for (int q = 0; q < 4; ++q) sizes.take<int32_t>((size_t)rows);
     sizes.take<int32_t>((size_t)rows + 1);
+    sizes.take<ClassCtl>(1);
     if (with_table) sizes.take<int32_t>(ptr_entries);
     const int prefix_ctas = (int)(((int64_t)a->nnz + 1 + 2047) / 2048);
     const int short_tiles = (int)(((int64_t)rows + SHORT_NT - 1) / SHORT_NT);
@@ -985,7 +1164,9 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     plan->lists.ranked_rows = carve.take<int32_t>((size_t)rows);
     plan->lists.heavy_rows = carve.take<int32_t>((size_t)rows);
     plan->row_count = carve.take<int32_t>((size_t)rows + 1);
+    plan->classes = carve.take<ClassCtl>(1);
     plan->n_win = (int)n_win;
+    plan->words = ranked_words(b->cols);
     plan->win_ptr = with_table ? carve.take<int32_t>(ptr_entries) : nullptr;
     unsigned long long *prefix = carve.take<unsigned long long>((size_t)a->nnz + 1);
     plan->scan_block = carve.take<uint64_t>((size_t)scan_ctas + 8);
@@ -994,7 +1175,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     uint64_t *prefix_block = carve.take<uint64_t>((size_t)prefix_ctas + 8);
     plan->short_block = carve.take<uint64_t>(TileWords::needed(short_tiles) + 4);
     plan->short_tiles = short_tiles;
-    plan->words = result_word(plan->ws, 0);
+    plan->result = result_word(plan->ws, 0);
     for (int k = 1; k < W_COUNT; ++k) result_word(plan->ws, k);
 
     // every control block and tile word of the call lies in one piece: one fill clears them all
@@ -1004,7 +1185,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     const bool short_rows = (int64_t)a->nnz <= 8 * (int64_t)rows;  // then a lane walks its row faster than a prefix pass pays
     if (rows > 0 && short_rows) {
         LaunchScope scope("esc_rowwork", stream);
-        k_esc_rowwork_walk<<<(rows + 255) / 256, 256, 0, stream>>>(A, B, rows, counts ? plan->row_count : nullptr, plan->lists, plan->ctl, plan->words);
+        k_esc_rowwork_walk<<<(rows + 255) / 256, 256, 0, stream>>>(A, B, rows, counts ? plan->row_count : nullptr, plan->lists, plan->ctl, plan->result);
         NB200_CUDA(cudaGetLastError());
     } else if (rows > 0) {
         {
@@ -1013,13 +1194,13 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
         }
         LaunchScope scope("esc_rowwork", stream);
         NB200_CUDA(launch_overlapped(k_esc_rowwork, dim3((rows + 255) / 256), dim3(256), 0, stream, A, prefix, rows, counts ? plan->row_count : nullptr,
-                                     plan->lists, plan->ctl, reinterpret_cast<const FusedCtl *>(prefix_block), plan->words));
+                                     plan->lists, plan->ctl, reinterpret_cast<const FusedCtl *>(prefix_block), plan->result));
     }
     if (rows > 0) {
         int64_t v[W_NNZ];
         int device_status = 0, failed = 0;
         for (int k = 0; k < W_NNZ; ++k) {
-            if ((st = wait_result_word(plan->words + k, stream, &v[k], &device_status))) return st;
+            if ((st = wait_result_word(plan->result + k, stream, &v[k], &device_status))) return st;
             failed |= device_status;
         }
         // a prefix whose look-back gave up leaves rows with wrong product counts: nothing may be built on them
@@ -1034,26 +1215,46 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
         k_esc_window_ptr<<<(unsigned)((ptr_entries + 255) / 256), 256, 0, stream>>>(B, b->rows, plan->n_win, plan->win_ptr);
         NB200_CUDA(cudaGetLastError());
     }
-    plan->cache_ranked = plan->cache_heavy = nullptr;
+    plan->cache = nullptr;
     plan->cache_ws = nullptr;
-    if (carry_bitmaps && plan->n_win == 1) {
+    plan->b_words = RowWords{};
+    plan->class_rows = nullptr;
+    const int64_t listed = (int64_t)plan->host.n_rows[BIN_RANKED] + plan->host.n_rows[BIN_GIANT] + plan->host.n_rows[BIN_HEAVY];
+    if (listed > 0) {
         // a second pool block: its size is only known now, and the first must not move
-        const size_t ranked_bytes = (size_t)plan->host.n_rows[BIN_RANKED] * ranked_words(RK_NT, b->cols) * 4;
-        const size_t heavy_bytes = ((size_t)plan->host.n_rows[BIN_GIANT] + plan->host.n_rows[BIN_HEAVY]) * ranked_words(HEAVY_NT, b->cols) * 4;
-        if (ranked_bytes + heavy_bytes > 0 && ranked_bytes + heavy_bytes <= BITMAP_CACHE_BUDGET) {
-            Carver cache_sizes;
-            cache_sizes.take<uint32_t>(ranked_bytes / 4);
-            cache_sizes.take<uint32_t>(heavy_bytes / 4);
-            Workspace *cache_ws = nullptr;
-            const int cache_st = acquire_workspace(stream, cache_sizes.used(), &cache_ws, 3);
-            if (cache_st == NB200_OK) {  // without room the numeric pass walks the products twice, as it does on its own
-                Carver cache_carve(cache_ws->dev);
-                plan->cache_ranked = ranked_bytes ? cache_carve.take<uint32_t>(ranked_bytes / 4) : nullptr;
-                plan->cache_heavy = heavy_bytes ? cache_carve.take<uint32_t>(heavy_bytes / 4) : nullptr;
-                plan->cache_ws = cache_ws;
-            } else if (cache_st != NB200_E_NOMEM) {
-                return cache_st;
-            }
+        const size_t bitmap_bytes = (size_t)listed * plan->words * 4;
+        const bool many = listed >= MANY_ROWS, carry = carry_bitmaps && plan->n_win == 1 && bitmap_bytes <= BITMAP_CACHE_BUDGET;
+        auto carve_rows = [&](Carver &c) {
+            if (many) plan->class_rows = c.take<int2>((size_t)CLASSES * listed);
+            if (carry) plan->cache = c.take<uint4>(bitmap_bytes / 16);
+        };
+        Carver row_sizes;
+        carve_rows(row_sizes);
+        Workspace *row_ws = nullptr;
+        const int row_st = many || carry ? acquire_workspace(stream, row_sizes.used(), &row_ws, 3) : NB200_E_NOMEM;
+        if (row_st == NB200_OK) {
+            Carver row_carve(row_ws->dev);
+            carve_rows(row_carve);
+            plan->cache_ws = row_ws;
+        } else if (row_st != NB200_E_NOMEM) {
+            return row_st;
+        }  // without room the numeric pass walks the products twice, as it does on its own, and takes all rows in one launch
+    }
+    if (listed > 0 && counts && plan->n_win == 1 && plan->host.products >= FORMS_FROM && plan->host.products >= REUSE * (unsigned long long)b->nnz) {
+        size_t clear_from, clear_bytes;
+        Carver word_sizes;
+        RowWordsScratch::carve(word_sizes, b->rows, b->nnz, false, &clear_from, &clear_bytes);
+        Workspace *word_ws = nullptr;
+        const int word_st = acquire_workspace(stream, word_sizes.used(), &word_ws, 4);
+        if (word_st == NB200_OK) {  // without room the entries are walked
+            Carver word_carve(word_ws->dev);
+            const RowWordsScratch scratch = RowWordsScratch::carve(word_carve, b->rows, b->nnz, false, &clear_from, &clear_bytes);
+            NB200_CUDA(cudaMemsetAsync(static_cast<unsigned char *>(word_ws->dev) + clear_from, 0, clear_bytes, stream));
+            // a give-up is reported by the scan that ends the symbolic pass
+            NB200_CUDA(build_row_words(b->row_ptr, b->col, b->rows, b->nnz, scratch, reinterpret_cast<FusedCtl *>(plan->scan_block), stream));
+            plan->b_words = scratch.out;
+        } else if (word_st != NB200_E_NOMEM) {
+            return word_st;
         }
     }
     return NB200_OK;
@@ -1073,68 +1274,143 @@ int launch_bin(bool beside, void (*kernel)(P...), int grid, int block, size_t sm
     return NB200_OK;
 }
 
-template <bool NUMERIC, int NT>
-int launch_ranked(const CsrView &A, const CsrView &B, const EscPlan &plan, int32_t b_cols, const int32_t *list, int32_t list_len,
-                  int n_front, int n_rows, uint32_t *cache, int32_t *count, const int32_t *c_rp, int32_t *c_col, float *c_val,
-                  cudaStream_t stream, bool beside) {
-    int wshift = 5;
-    const int words = ranked_words(NT, b_cols, &wshift);
-    // numeric: whatever the bitmap and the ranks leave of the CTA's shared memory accumulates sums
-    // Heavy rows always have some. The lighter ones only where there are many: a few thousand CTAs are bound by
-    // the latency of a row's short phases, and without a shared accumulator one more fits on an SM (a graph of 2698
-    // vertices 111 against 117 us, of 9000 vertices 198 against 209); tens of thousands are bound by the
-    // reductions that go to L2 instead (24405 vertices 434 -> 430 us, 65536 vertices 2579 -> 2436).
-    const size_t rows_budget = NT == HEAVY_NT ? HEAVY_SMEM_NUMERIC : n_rows >= RK_MANY_ROWS ? RK_SMEM_NUMERIC : 0;
-    const size_t table = (size_t)words * RK_WORD_BYTES;
-    const int acc_slots = NUMERIC ? (int)((std::max(rows_budget, table) - table) / 4 / NT) * NT : 0;
-    const size_t smem = NUMERIC ? table + (size_t)acc_slots * 4 : (size_t)words * 4;
-    const bool far = NUMERIC && NT == HEAVY_NT && words * 32 > 65536;
-    auto kernel = far ? k_esc_ranked<NUMERIC, NT, NUMERIC && NT == HEAVY_NT> : k_esc_ranked<NUMERIC, NT, false>;
-    // the most that any call asks for: several threads may be here with different sizes
-    NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(NUMERIC ? std::max(HEAVY_SMEM_NUMERIC, RK_WORDS * RK_WORD_BYTES) : (size_t)RK_WORDS * 4)));
-    return launch_bin(beside, kernel, n_rows, NT, smem, stream, A, B, plan.win_ptr, plan.n_win, list, list_len, n_front, words, wshift, acc_slots, cache,
-                      count, c_rp, c_col, c_val);
+template <int NT, int PIECE>
+int launch_mark(const CsrView &A, const CsrView &B, const EscPlan &plan, const int32_t *list, int32_t list_len, int n_front, int n_rows, int first,
+                cudaStream_t stream, bool beside) {
+    uint4 *cache = plan.cache ? plan.cache + (size_t)first * (plan.words / 4) : nullptr;  // `first`: place of the first of these rows
+    auto kernel = plan.b_words.items ? k_esc_mark<NT, PIECE, true> : k_esc_mark<NT, PIECE, false>;
+    return launch_bin(beside, kernel, n_rows, NT, (size_t)plan.words * 4, stream, A, B, plan.b_words, Windows{plan.n_win, plan.win_ptr}, list, list_len, n_front,
+                      plan.words, cache, plan.row_count);
 }
 
-template <bool NUMERIC>
-int esc_run_bins(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const nb200_csr *c, cudaStream_t stream) {
-    const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
-    int32_t *count = NUMERIC ? nullptr : plan.row_count;
-    const int32_t *c_rp = NUMERIC ? c->row_ptr : nullptr;
-    int32_t *c_col = NUMERIC ? c->col : nullptr;
-    float *c_val = NUMERIC ? c->val : nullptr;
+int launch_sorted(bool numeric, const CsrView &A, const CsrView &B, const EscPlan &plan, int32_t b_cols, const nb200_csr *c, cudaStream_t stream, bool beside) {
+    int32_t *count = numeric ? nullptr : plan.row_count, *c_col = numeric ? c->col : nullptr;
+    const int32_t *c_rp = numeric ? c->row_ptr : nullptr;
+    float *c_val = numeric ? c->val : nullptr;
     int st;
-    const int n_heavy = plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY];
-    bool beside = false;
-    if (n_heavy > 0) {  // first: the heaviest rows take longest
-        LaunchScope scope(NUMERIC ? "esc_heavy_numeric" : "esc_heavy_symbolic", stream);
-        if ((st = launch_ranked<NUMERIC, HEAVY_NT>(A, B, plan, b->cols, plan.lists.heavy_rows, a->rows, plan.host.n_rows[BIN_GIANT], n_heavy,
-                                                             plan.cache_heavy, count, c_rp, c_col, c_val, stream, false)))
-            return st;
-        beside = true;
-    }
-    if (plan.host.n_rows[BIN_RANKED] > 0) {
-        LaunchScope scope(NUMERIC ? "esc_ranked_numeric" : "esc_ranked_symbolic", stream);
-        if ((st = launch_ranked<NUMERIC, RK_NT>(A, B, plan, b->cols, plan.lists.ranked_rows, a->rows, plan.host.n_rows[BIN_RANKED],
-                                                          plan.host.n_rows[BIN_RANKED], plan.cache_ranked, count, c_rp, c_col, c_val, stream, beside)))
-            return st;
-        beside = true;
-    }
     if (plan.host.n_rows[BIN_MEDIUM] > 0) {
-        LaunchScope scope(NUMERIC ? "esc_medium_numeric" : "esc_medium_symbolic", stream);
-        if ((st = launch_bin(beside, k_esc_medium<NUMERIC>, plan.host.n_rows[BIN_MEDIUM], MED_NT, 0, stream, A, B, plan.lists.medium_rows, count, c_rp, c_col, c_val)))
+        LaunchScope scope(numeric ? "esc_medium_numeric" : "esc_medium_symbolic", stream);
+        if ((st = launch_bin(beside, numeric ? k_esc_medium<true> : k_esc_medium<false>, plan.host.n_rows[BIN_MEDIUM], MED_NT, 0, stream, A, B,
+                             plan.lists.medium_rows, count, c_rp, c_col, c_val)))
             return st;
         beside = true;
     }
     if (plan.host.n_rows[BIN_SMALL] > 0) {
-        LaunchScope scope(NUMERIC ? "esc_small_numeric" : "esc_small_symbolic", stream);
-        const int warps = plan.host.n_rows[BIN_SMALL];  // rows on the list
-        const int small_warps = (warps + ESC_SMALL_ROWS - 1) / ESC_SMALL_ROWS;
-        auto kernel = b->cols < (1 << 27) ? k_esc_small<NUMERIC, true> : k_esc_small<NUMERIC, false>;
-        if ((st = launch_bin(beside, kernel, (small_warps + 7) / 8, 256, 0, stream, A, B, plan.lists.small_rows, warps, count, c_rp, c_col, c_val))) return st;
+        LaunchScope scope(numeric ? "esc_small_numeric" : "esc_small_symbolic", stream);
+        const int rows = plan.host.n_rows[BIN_SMALL], warps = (rows + ESC_SMALL_ROWS - 1) / ESC_SMALL_ROWS;
+        const bool narrow = b_cols < (1 << 27);
+        auto kernel = numeric ? (narrow ? k_esc_small<true, true> : k_esc_small<true, false>) : (narrow ? k_esc_small<false, true> : k_esc_small<false, false>);
+        if ((st = launch_bin(beside, kernel, (warps + 7) / 8, 256, 0, stream, A, B, plan.lists.small_rows, rows, count, c_rp, c_col, c_val))) return st;
     }
     return NB200_OK;
+}
+
+int run_symbolic(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, cudaStream_t stream) {
+    const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
+    int st;
+    const int n_heavy = plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY], n_ranked = plan.host.n_rows[BIN_RANKED];
+    const bool many = n_heavy + n_ranked >= MANY_ROWS;
+    if (n_heavy > 0) {  // first: the heaviest rows take longest
+        LaunchScope scope("esc_heavy_symbolic", stream);
+        auto launch = many ? launch_mark<HEAVY_NT, LONG> : launch_mark<HEAVY_NT, SHORT>;
+        if ((st = launch(A, B, plan, plan.lists.heavy_rows, a->rows, plan.host.n_rows[BIN_GIANT], n_heavy, 0, stream, false))) return st;
+    }
+    if (n_ranked > 0) {
+        LaunchScope scope("esc_ranked_symbolic", stream);
+        auto launch = many ? launch_mark<MANY_NT, LONG> : launch_mark<RK_NT, SHORT>;
+        if ((st = launch(A, B, plan, plan.lists.ranked_rows, a->rows, n_ranked, n_ranked, n_heavy, stream, n_heavy > 0))) return st;
+    }
+    return launch_sorted(false, A, B, plan, b->cols, nullptr, stream, n_heavy + n_ranked > 0);
+}
+
+ListedRows listed_rows(const EscPlan &plan, int32_t rows) {
+    const int n_heavy = plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY];
+    return ListedRows{plan.lists.heavy_rows, plan.lists.ranked_rows, rows, plan.host.n_rows[BIN_GIANT], n_heavy, n_heavy + plan.host.n_rows[BIN_RANKED]};
+}
+
+// What the numeric pass needs besides the result's row offsets: the rows of every class (`classes`; few rows go straight
+// to one launch), and B's entries side by side where enough products read them. Made anew for every numeric pass (the
+// values may be others than at the symbolic one).
+struct NumericPlan {
+    bool classes = false;
+    const uint2 *pairs = nullptr;
+};
+
+int prepare_numeric(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const int32_t *c_rp, NumericPlan *numeric, cudaStream_t stream) {
+    *numeric = NumericPlan{};
+    const ListedRows listed = listed_rows(plan, a->rows);
+    if (listed.n == 0) return NB200_OK;
+    numeric->classes = plan.class_rows != nullptr;
+    if (numeric->classes) {
+        NB200_CUDA(cudaMemsetAsync(plan.classes, 0, sizeof(ClassCtl), stream));
+        LaunchScope scope("esc_classes", stream);
+        ClassSlots most;
+        for (int k = 0; k < CLASSES; ++k) most.slots[k] = rank_slots(k, plan.words);
+        k_esc_classes<<<(listed.n + 255) / 256, 256, 0, stream>>>(listed, c_rp, most, plan.class_rows, listed.n, plan.classes);
+        NB200_CUDA(cudaGetLastError());
+    }
+    if (!numeric->classes || plan.host.products < FORMS_FROM || plan.host.products < REUSE * (unsigned long long)b->nnz) return NB200_OK;
+    Workspace *ws = nullptr;
+    const int st = acquire_workspace(stream, (size_t)b->nnz * sizeof(uint2), &ws, 5);
+    if (st != NB200_OK) return st == NB200_E_NOMEM ? NB200_OK : st;  // without room columns and values are loaded apart
+    LaunchScope scope("esc_pairs", stream);
+    uint2 *pairs = static_cast<uint2 *>(ws->dev);
+    k_esc_pairs<<<(unsigned)(((int64_t)b->nnz + 255) / 256), 256, 0, stream>>>(b->row_ptr, b->col, b->val, b->nnz, pairs);
+    NB200_CUDA(cudaGetLastError());
+    numeric->pairs = pairs;
+    return NB200_OK;
+}
+
+template <int CLS>
+int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const NumericPlan &numeric, int first, int last, const nb200_csr *c, cudaStream_t stream,
+                bool beside) {
+    static const char *const names[] = {"esc_rank_0", "esc_rank_1", "esc_rank_2", "esc_rank_3", "esc_rank_4", "esc_rank_few", "esc_rank_few_heavy"};
+    constexpr RankClass K = RANK_CLASS[CLS];
+    // A table that leaves no room for sums: no row is of this class, and where rows are not sorted all their sums are in L2.
+    const int slots = rank_slots(CLS, plan.words);
+    if (CLS < CLASSES && slots == 0) return NB200_OK;
+    const size_t smem = std::max(K.smem, (size_t)plan.words * 8);
+    int device = 0, ctas = last - first;
+    if (CLS < CLASSES) {
+        NB200_CUDA(cudaGetDevice(&device));
+        NB200_CUDA(cudaDeviceGetAttribute(&ctas, cudaDevAttrMultiProcessorCount, device));
+        ctas *= K.per_sm;
+    }
+    LaunchScope scope(names[CLS], stream);
+    const bool narrow = plan.words <= NARROW_WORDS;
+    auto kernel = narrow ? k_esc_rank<CLS, true, false> : k_esc_rank<CLS, false, false>;
+    if constexpr (CLS < CLASSES)
+        if (numeric.pairs) kernel = narrow ? k_esc_rank<CLS, true, true> : k_esc_rank<CLS, false, true>;
+    // the most that any call asks for: several threads may be here with different sizes
+    NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(K.smem, (size_t)RK_WORDS * 8)));
+    return launch_bin(beside, kernel, ctas, K.nt, smem, stream, CsrView{a->row_ptr, a->col, a->val},
+                      CsrView{b->row_ptr, b->col, b->val}, numeric.pairs, Windows{plan.n_win, plan.win_ptr}, listed_rows(plan, a->rows), first, last,
+                      CLS < CLASSES ? plan.class_rows + (size_t)CLS * last : nullptr, plan.classes, plan.words, slots, plan.cache, c->row_ptr, c->col, c->val);
+}
+
+// The heaviest rows first: they take longest.
+int launch_ranks(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const NumericPlan &numeric, const nb200_csr *c, cudaStream_t stream) {
+    const ListedRows listed = listed_rows(plan, a->rows);
+    int st;
+    if (numeric.classes) {
+        if ((st = launch_rank<4>(a, b, plan, numeric, 0, listed.n, c, stream, false))) return st;
+        if ((st = launch_rank<3>(a, b, plan, numeric, 0, listed.n, c, stream, true))) return st;
+        if ((st = launch_rank<2>(a, b, plan, numeric, 0, listed.n, c, stream, true))) return st;
+        if ((st = launch_rank<1>(a, b, plan, numeric, 0, listed.n, c, stream, true))) return st;
+        return launch_rank<0>(a, b, plan, numeric, 0, listed.n, c, stream, true);
+    }
+    const int n_heavy = listed.n_heavy;
+    if (n_heavy > 0 && (st = launch_rank<FEW_HEAVY>(a, b, plan, numeric, 0, n_heavy, c, stream, false))) return st;
+    return listed.n > n_heavy ? launch_rank<FEW>(a, b, plan, numeric, n_heavy, listed.n, c, stream, n_heavy > 0) : NB200_OK;
+}
+
+// The numeric pass after prepare_numeric.
+int run_numeric(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const NumericPlan &numeric, const nb200_csr *c, cudaStream_t stream) {
+    const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
+    const bool any = listed_rows(plan, a->rows).n > 0;
+    int st;
+    if (any && (st = launch_ranks(a, b, plan, numeric, c, stream))) return st;
+    return launch_sorted(true, A, B, plan, b->cols, c, stream, any);
 }
 
 // The plan of the latest symbolic pass, kept for the numeric pass that normally follows it on the
@@ -1198,18 +1474,20 @@ int spgemm_begin(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStrea
 }
 
 // The symbolic pass on rows that `plan` has just binned (its control blocks serve one call).
-int symbolic_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStream_t stream) {
+// `numeric` set: the numeric pass follows, and what it needs is queued before the host waits.
+int symbolic_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_csr *c, NumericPlan *numeric, cudaStream_t stream) {
     int st;
-    if ((st = esc_run_bins<false>(a, b, plan, nullptr, stream))) return st;
+    if ((st = run_symbolic(a, b, plan, stream))) return st;
     {
         LaunchScope scope("esc_scan_offsets", stream);
         k_scan_offsets<<<plan.scan_ctas, SCAN_NT, 0, stream>>>(plan.row_count, a->rows, c->row_ptr, plan.scan_block + 4,
-                                                              reinterpret_cast<FusedCtl *>(plan.scan_block), plan.words + W_NNZ);
+                                                              reinterpret_cast<FusedCtl *>(plan.scan_block), plan.result + W_NNZ);
         NB200_CUDA(cudaGetLastError());
     }
+    if (numeric && (st = prepare_numeric(a, b, plan, c->row_ptr, numeric, stream))) return st;
     int64_t nnz;
     int device_status;
-    if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
+    if ((st = wait_result_word(plan.result + W_NNZ, stream, &nnz, &device_status))) return st;
     if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm row scan");
     if (nnz > INT32_MAX) return NB200_E_OVERFLOW;
     c->nnz = (int32_t)nnz;
@@ -1225,7 +1503,7 @@ int spgemm_symbolic(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_
     EscPlan plan{};
     if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
     if (products) *products = (int64_t)plan.host.products;
-    if ((st = symbolic_on(plan, a, b, c, stream))) return st;
+    if ((st = symbolic_on(plan, a, b, c, nullptr, stream))) return st;
     save_plan(a, b, c, plan, stream);
     return NB200_OK;
 }
@@ -1239,7 +1517,9 @@ int spgemm_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, void *s
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     EscPlan plan{};
     if (!take_saved_plan(a, b, c, stream, &plan) && (st = esc_prepare(a, b, false, false, stream, &plan))) return st;
-    return esc_run_bins<true>(a, b, plan, c, stream);
+    NumericPlan numeric;
+    if ((st = prepare_numeric(a, b, plan, c->row_ptr, &numeric, stream))) return st;
+    return run_numeric(a, b, plan, numeric, c, stream);
 }
 
 // Whether the one-pass kernel can do the product. It wants room for as many entries as there are products, an upper bound of nnz(C).
@@ -1256,13 +1536,13 @@ int short_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_
     {
         LaunchScope scope("esc_short", stream);
         kernel<<<plan.short_tiles + (plan.short_tiles > DIRECT_TILES ? 1 : 0), SHORT_NT, 0, stream>>>(
-            A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.words + W_NNZ);
+            A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.result + W_NNZ);
         NB200_CUDA(cudaGetLastError());
     }
     int st;
     int64_t nnz;
     int device_status;
-    if ((st = wait_result_word(plan.words + W_NNZ, stream, &nnz, &device_status))) return st;
+    if ((st = wait_result_word(plan.result + W_NNZ, stream, &nnz, &device_status))) return st;
     if (device_status != 0) return note_timeout(ERR_LOOKBACK_TIMEOUT, 0, "spgemm of short rows");
     c->nnz = (int32_t)nnz;
     return NB200_OK;
@@ -1289,9 +1569,10 @@ int spgemm_into(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int64_t ca
     EscPlan plan{};
     if ((st = esc_prepare(a, b, true, true, stream, &plan))) return st;
     if (is_short(plan) && capacity >= (int64_t)plan.host.products) return short_on(plan, a, b, c, stream);
-    if ((st = symbolic_on(plan, a, b, c, stream))) return st;
+    NumericPlan numeric;
+    if ((st = symbolic_on(plan, a, b, c, &numeric, stream))) return st;
     if (c->nnz > capacity) return NB200_E_CAPACITY;
-    return c->nnz > 0 ? esc_run_bins<true>(a, b, plan, c, stream) : NB200_OK;
+    return c->nnz > 0 ? run_numeric(a, b, plan, numeric, c, stream) : NB200_OK;
 }
 
 // The whole product into arrays that the caller hands out once their length is known: no plan outlives the call.
@@ -1323,9 +1604,10 @@ int spgemm_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take
         }
         if (st != NB200_E_NOMEM) return st;  // no room for an entry per product: count first
     }
-    if ((st = symbolic_on(plan, a, b, c, stream)) || c->nnz == 0) return st;
+    NumericPlan numeric;
+    if ((st = symbolic_on(plan, a, b, c, &numeric, stream)) || c->nnz == 0) return st;
     if ((st = take(ctx, c->nnz, &c->col, &c->val))) return st;
-    return esc_run_bins<true>(a, b, plan, c, stream);
+    return run_numeric(a, b, plan, numeric, c, stream);
 }
 
 }  // namespace

@@ -151,6 +151,26 @@ def test_many_ranked_rows(nacho, oracle):
     check(nacho, oracle, csr_of_keys(keys(rows, inner, 5), rows, inner, rng), csr_of_keys(b_key, inner, cols, rng))
 
 
+@pytest.mark.parametrize("cols", [40000, 65536, 70000])
+def test_rows_by_result_length(nacho, oracle, cols):
+    """Enough rows and products for the rows of B to be walked as bitmap words and the result's rows to be sorted by length:
+    results from 300 entries to all columns, in rows of B that are scattered, solid runs, and runs that meet in one word; ranks in 16
+    and (70000 columns) 32 bits."""
+    from test_spgemm_gpu import check
+    rng = np.random.default_rng(cols)
+    inner, rows = 320, 8192 + 64
+    b_rows = [np.sort(rng.choice(cols, 2400, replace=False)) for _ in range(200)]
+    b_rows += [np.arange(q, q + n) for q, n in zip(rng.integers(0, cols - 4200, 118), rng.integers(300, 4200, 118))]
+    b_rows += [np.arange(0, 17), np.arange(19, 2100)]  # neighbouring rows that end and begin in one word
+    b_key = np.concatenate([r * cols + k for r, k in enumerate(b_rows)]).astype(np.int64)
+    per_row = np.full(rows, 2)
+    per_row[rng.integers(0, rows, 300)] = rng.integers(3, 60, 300)
+    per_row[5:9] = 120, 200, 320, 319
+    a_key = np.concatenate([r * inner + np.sort(rng.choice(inner, n, replace=False)) for r, n in enumerate(per_row)]).astype(np.int64)
+    _, products = check(nacho, oracle, csr_of_keys(a_key, rows, inner, rng), csr_of_keys(b_key, inner, cols, rng))
+    assert products >= 32 << 20
+
+
 @pytest.mark.parametrize("cols", [65535, 65536, 65537])
 def test_full_heavy_row(nacho, oracle, cols):
     """A row of more than 65535 products that reaches every column, at the width up to which positions fit 16 bits."""
