@@ -151,6 +151,33 @@ def test_many_ranked_rows(nacho, oracle):
     check(nacho, oracle, csr_of_keys(keys(rows, inner, 5), rows, inner, rng), csr_of_keys(b_key, inner, cols, rng))
 
 
+def check_masked(nacho, oracle, a, b, c):
+    """gpu_sssmm_f32 against the oracle's product on the mask's positions."""
+    full, v64, abs64, _ = oracle.spgemm(a, b, 8, extras=True)
+    key = lambda m: np.repeat(np.arange(m.rows, dtype=np.int64), np.diff(m.row_ptr)) * m.cols + m.col
+    z = csr_from_gpu(nacho.gpu_sssmm_f32(csr_to_gpu(a), csr_to_gpu(b), csr_to_gpu(c)))
+    common, i_f, i_c = np.intersect1d(key(full), key(c), return_indices=True)
+    assert np.array_equal(key(z), common)
+    bound = 1e-5 * abs64[i_f] * np.abs(c.val[i_c]) + 1e-30
+    assert np.all(np.abs(z.val.astype(np.float64) - v64[i_f] * c.val[i_c].astype(np.float64)) <= bound)
+
+
+@pytest.mark.parametrize("cols", [60000, 300000])
+def test_masked_rows_by_words(nacho, oracle, cols):
+    """A second operand of 2^18 entries and more, walked as bitmap words: mask rows up to the bitmaps' largest, products that miss, meet
+    one column of a word or all 32."""
+    rng = np.random.default_rng(cols)
+    rows, inner = 60, 1200
+    b_rows = [np.sort(rng.choice(cols, 240, replace=False)) if r % 3 else np.arange(q := int(rng.integers(0, cols - 400)), q + 250 + r % 60) for r in range(inner)]
+    b = csr_of_keys(np.concatenate([r * cols + k for r, k in enumerate(b_rows)]).astype(np.int64), inner, cols, rng)
+    assert len(b.col) >= 1 << 18
+    per_row = np.array([0, 1, 8, 63, 64, 65, 200, 400, 1000, 1200] * 6)
+    a = csr_of_keys(np.concatenate([r * inner + np.sort(rng.choice(inner, n, replace=False)) for r, n in enumerate(per_row)]).astype(np.int64), rows, inner, rng)
+    masks = [0, 1, 40, 300, 2000, 2048, 2049, 8000, 8192, 20000]
+    c = csr_of_keys(np.concatenate([r * cols + np.sort(rng.choice(cols, masks[(r + r // 10) % 10], replace=False)) for r in range(rows)]).astype(np.int64), rows, cols, rng)
+    check_masked(nacho, oracle, a, b, c)
+
+
 @pytest.mark.parametrize("cols", [40000, 65536, 70000])
 def test_rows_by_result_length(nacho, oracle, cols):
     """Enough rows and products for the rows of B to be walked as bitmap words and the result's rows to be sorted by length:
