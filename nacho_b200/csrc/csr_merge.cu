@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
 // twice the time of the others and holds up their output bases, and the twin mask by entries (below) pays. 25 M entries
 // per operand in 6 M fibres take 384 us with 17, 389 with 21, 426 with 23, 446 with 31; 50 M in 4 M fibres 513, 508,
 // 563, 548. The stored rows of a doubly compressed matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
-constexpr int V_FIBRES = 21;
+constexpr int V_FIBRES = 21, V_MOST = 31;  // V_MOST: the large tile otherwise
 
 // Shared-memory plan of the tile body. The column words of both operands lie in one array: A's entry e at
 // word oa + e, B's at word ob + e, where oa and ob are chosen so that a global address on a 16-byte
@@ -160,7 +160,11 @@ struct TilePlan {
     static_assert(4 * SLOTS < 32768, "byte offsets of entries are kept in 15 bits");
 };
 constexpr uint32_t ROW_FAR = 0xffffu;
-constexpr int GATHER = 8;       // result entries a thread fetches together
+
+// A tile of short rows asks for the row offsets of one that starts a few microseconds later, so that they wait in L2: they are
+// read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns ahead
+// as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.)
+constexpr int TILES_AHEAD = 148;
 
 // Fixed shared memory of a tile (one block for both key widths).
 struct TileShared {
@@ -516,6 +520,9 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     // asked for
     const char *va = reinterpret_cast<const char *>(ga_val) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(gb_val) - 4 * (int64_t)ob;
     const uint32_t first_b = 4u * (uint32_t)ob;
+    // Result entries a thread fetches together. A round is a trip to L2, so the smaller tiles take one or two. In the large
+    // tile, bound by throughput, 8 are better than 11 or 16 (67 M entries 449, 465, 483 us); intersections leave fewer.
+    constexpr int GATHER = OP == OP_INTERSECT || VT == V_MOST ? 8 : VT <= 16 ? VT : (VT + 1) / 2;
     uint32_t col[GATHER];
     float val[GATHER];
     auto gather = [&](const int q0) {
@@ -693,6 +700,11 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     if (cuts) {
         const int4 c0 = cuts[t], c1 = cuts[t + 1];
         tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
+        if (V != V_MOST && threadIdx.x == 96 && t + TILES_AHEAD < num_tiles) {
+            const int32_t r0 = cuts[t + TILES_AHEAD].x, n = cuts[t + TILES_AHEAD + 1].x - r0 + 1;
+            if (A.rp) prefetch_l2(A.rp + r0, n);
+            if (B.rp) prefetch_l2(B.rp + r0, n);
+        }
     } else {
         const int32_t rows = row_count.get();
         tile = TileRange{0, rows, row_offset(A, 0), row_offset(B, 0), A.entries(), B.entries()};
@@ -722,7 +734,7 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
 // small ones: 2 M merged entries 22.8 us with 15 against 24.9, 0.8 M 15.8 against 18.9; at 6 M the two are even.
 // Both are odd: a thread's shares of A and B then start at odd word distances from its neighbour's where
 // rows alternate evenly, and the shared-memory banks are hit evenly (16 took twice the time of 18).
-constexpr int V_LARGE = 31, V_SMALL = 15;
+constexpr int V_LARGE = V_MOST, V_SMALL = 15;
 constexpr int64_t LARGE_FROM = 6000000;
 constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
 constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between two tile cuts (a twin may add one)
