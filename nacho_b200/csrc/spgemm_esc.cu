@@ -613,8 +613,9 @@ constexpr int MANY_NT = 128, MANY_ROWS = 8192;     // ... and up to RANKED_P whe
 // Where the word w of a window lies in shared memory. The low bits of a graph's column numbers are far from uniform (in an
 // R-MAT graph each is 0 three times in four, so a quarter of all words would lie in one bank; random look-ups with that skew
 // take 8 cycles per warp instead of 3); folding the bits above into them spreads the banks. One to one on any power
-// of two of words.
-__device__ __forceinline__ uint32_t spread(uint32_t w) { return w ^ (w >> 4) ^ (w >> 8); }
+// of two of words. FOLD false: in order, for the kernels of few rows, which wait for loads and not for banks.
+template <bool FOLD>
+__device__ __forceinline__ uint32_t spread(uint32_t w) { return FOLD ? w ^ (w >> 4) ^ (w >> 8) : w; }
 
 // First index in [lo, hi) whose column is >= key (hi if none).
 __device__ __forceinline__ int32_t first_col_at_least(const int32_t *__restrict__ col, int32_t lo, int32_t hi, int64_t key) {
@@ -727,18 +728,18 @@ __global__ void __launch_bounds__(NT, 1536 / NT) k_esc_mark(CsrView A, CsrView B
             any = row.run(A, seg, scan_tmp, true, [&](int32_t j, int32_t &start, int32_t &len) {
                 start = ld_nc(B_words.rp + j);
                 len = ld_nc(B_words.rp + j + 1) - start;
-            }, [&](int q) { return __ldg(B_words.items + q); }, [&](uint2 item, float) { atomicOr(bitmap + spread(item.x), item.y); });
+            }, [&](int q) { return __ldg(B_words.items + q); }, [&](uint2 item, float) { atomicOr(bitmap + spread<PIECE == LONG>(item.x), item.y); });
         } else {
             any = row.run(A, seg, scan_tmp, true, [&](int32_t j, int32_t &start, int32_t &len) { windows.range(B, j, w, start, len); },
                           [&](int q) { return ld_nc(B.col + q); }, [&](int32_t col, float) {
                               const uint32_t cw = (uint32_t)(col - c_first);
-                              atomicOr(bitmap + spread(cw >> 5), 1u << (cw & 31u));
+                              atomicOr(bitmap + spread<PIECE == LONG>(cw >> 5), 1u << (cw & 31u));
                           });
         }
         if (!any) continue;  // uniform
         for (int q = tid; q < words / 4; q += NT) {
             uint4 v;
-            v.x = bitmap[spread(4 * q)], v.y = bitmap[spread(4 * q + 1)], v.z = bitmap[spread(4 * q + 2)], v.w = bitmap[spread(4 * q + 3)];
+            v.x = bitmap[spread<PIECE == LONG>(4 * q)], v.y = bitmap[spread<PIECE == LONG>(4 * q + 1)], v.z = bitmap[spread<PIECE == LONG>(4 * q + 2)], v.w = bitmap[spread<PIECE == LONG>(4 * q + 3)];
             count += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
             if (cache) __stcs(cache + (size_t)r * (words / 4) + q, v);
         }
@@ -774,7 +775,7 @@ struct RankClass {
 };
 constexpr int CLASSES = 5, FEW = 5, FEW_HEAVY = 6;  // the last two: where there are few rows they are not sorted by class
 constexpr RankClass RANK_CLASS[] = {{128, 8, 25 * 1024, true, LONG},  {256, 4, 50 * 1024, true, LONG},    {320, 3, 68 * 1024, true, LONG},   {512, 2, 104 * 1024, true, LONG},
-                                    {1024, 1, 208 * 1024, false, LONG}, {256, 6, 0, false, SHORT}, {1024, 1, 208 * 1024, false, SHORT}};
+                                    {1024, 1, 208 * 1024, false, LONG}, {256, 5, 0, false, SHORT}, {1024, 1, 208 * 1024, false, SHORT}};
 constexpr int NARROW_WORDS = 2048;  // windows of up to 65536 columns: the table has 16 columns and their rank in 32 bits
 // Sums of a CTA of class `cls` beside a table of `words` bitmap words.
 constexpr int rank_slots(int cls, int words) {
@@ -826,11 +827,11 @@ __global__ void __launch_bounds__(256) k_esc_pairs(const int32_t *__restrict__ r
 // The columns of a window and their ranks, by bitmap words. NARROW: 16 columns in the lower half of a 32-bit word, the
 // number of columns before them in the upper one (a look-up is one 4-byte load: 3 cycles of the shared-memory pipe for
 // random words against 5 for 8 bytes); otherwise 32 columns and their rank in 64 bits.
-template <bool NARROW>
+template <bool NARROW, bool FOLD>
 struct RankTable {
     unsigned char *at;
-    __device__ __forceinline__ uint32_t &half(uint32_t h) const { return reinterpret_cast<uint32_t *>(at)[h ^ (h >> 5) ^ (h >> 10)]; }
-    __device__ __forceinline__ uint2 &full(uint32_t w) const { return reinterpret_cast<uint2 *>(at)[spread(w)]; }
+    __device__ __forceinline__ uint32_t &half(uint32_t h) const { return reinterpret_cast<uint32_t *>(at)[FOLD ? h ^ (h >> 5) ^ (h >> 10) : h]; }
+    __device__ __forceinline__ uint2 &full(uint32_t w) const { return reinterpret_cast<uint2 *>(at)[spread<FOLD>(w)]; }
     __device__ __forceinline__ void mark(uint32_t cw) const {  // column cw of the window, in a table of zeros
         if (NARROW) atomicOr(&half(cw >> 4), 1u << (cw & 15u));
         else atomicOr(&full(cw >> 5).x, 1u << (cw & 31u));
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(RANK_CLASS[CLS].nt, RANK_CLASS[CLS].per_sm)
     constexpr bool WALKED = K.columns_walked, BY_CLASS = CLS < CLASSES, IN_L2 = K.smem == 0;
     using Col = typename std::conditional<NARROW, uint16_t, uint32_t>::type;
     extern __shared__ __align__(16) unsigned char rk_smem[];
-    const RankTable<NARROW> table{rk_smem};
+    const RankTable<NARROW, K.piece == LONG> table{rk_smem};
     float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * 8);
     int32_t *stage = reinterpret_cast<int32_t *>(acc);
     Col *noted = reinterpret_cast<Col *>(acc + acc_slots);  // WALKED

@@ -9,7 +9,8 @@
 //                       how long is its mask row? The row goes on one of six lists.
 //   k_sssmm_bitmap      rows with many products, one CTA per row taken from a ticket: the mask row
 //                       becomes a bitmap over its column span in shared memory plus, per 64-bit
-//                       word, the count of set bits before it. A product tests one bit; a hit finds
+//                       word, the count of set bits before it. A product tests one bit, or 32 columns of
+//                       B's row are tested at once (row_words.cuh); a hit finds
 //                       its position in the mask row as rank + popcount and adds
 //                       (a_ij * b_jk) * c_ik -- the reference's expression, left to right -- to a
 //                       shared-memory accumulator (rows whose mask row is too long for that, or
