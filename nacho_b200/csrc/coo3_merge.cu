@@ -428,7 +428,7 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
     const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
     if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
         if (tid < 32) {
-            const int64_t total = scan_tile_counts<1>(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
             if (tid == 0) coo3_finish(ctl, Z, total);
         }
         return;

@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
     if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
         if (threadIdx.x < 32) {
-            const int64_t total = scan_tile_counts<1>(words, num_tiles, &ctl->status, first_tile ? poll_limit : LOOKBACK_POLL_LIMIT);
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, first_tile ? poll_limit : LOOKBACK_POLL_LIMIT);
             if (threadIdx.x == 0) finish_total(ctl, Z, total);
         }
         return;

@@ -55,39 +55,22 @@ __device__ __forceinline__ void publish_count(const TileWords &words, const int 
 
 // Runs in one warp. Publishes the base of every tile; returns the number of results, or -1 after
 // `poll_limit` rounds without a new count (the tiles that wait are told, and the error word is set). The
-// next round's loads are on their way while a round is summed up: a round takes one trip to L2 and no more, and
-// advances by up to 32 GROUPS tiles (4 where all tiles are of a size and finish together: the short rows of a mesh squared 63.4 ->
-// 61.2 us; where they arrive one by one 1: 67 M entries 0.5 % slower with 4).
-template <int GROUPS>
+// next round's load is on its way while a round is summed up: a round takes one trip to L2 and no more.
 __device__ __forceinline__ int64_t scan_tile_counts(const TileWords &words, const int num_tiles, DeviceStatus *status, const int poll_limit) {
     const int lane = lane_id();
     int64_t run = 0;
     int idle = 0;
-    uint64_t w[GROUPS];
-    auto fetch = [&](int pos) {
-#pragma unroll
-        for (int g = 0; g < GROUPS; ++g) w[g] = pos + 32 * g + lane < num_tiles ? ld_relaxed_gpu(words.count + pos + 32 * g + lane) : 0;
-    };
-    fetch(0);
+    uint64_t w = lane < num_tiles ? ld_relaxed_gpu(words.count + lane) : 0;
     for (int pos = 0;;) {
-        int n = 0, v[GROUPS];  // counts that are there without a gap, and the lane's of every group
-#pragma unroll
-        for (int g = 0; g < GROUPS; ++g) {
-            v[g] = (int)(w[g] & LB_VALUE_MASK);
-            const unsigned missing = __ballot_sync(FULL_MASK, (w[g] >> 62) == 0);
-            if (n == 32 * g) n += missing ? __ffs(missing) - 1 : 32;
-        }
+        const unsigned missing = __ballot_sync(FULL_MASK, (w >> 62) == 0);
+        const int n = missing ? __ffs(missing) - 1 : 32;
         const int next = pos + n;
-        fetch(next);
+        const uint64_t w_next = next + lane < num_tiles ? ld_relaxed_gpu(words.count + next + lane) : 0;
         if (n > 0) {
-#pragma unroll
-            for (int g = 0; g < GROUPS; ++g) {
-                if (32 * g >= n) break;  // uniform
-                const int mine = 32 * g + lane < n ? v[g] : 0;
-                const int incl = warp_incl_sum(mine);
-                if (32 * g + lane < n) st_relaxed_gpu(words.base + pos + 32 * g + lane, LB_PREFIX | (uint64_t)(run + incl - mine));
-                run += __shfl_sync(FULL_MASK, incl, 31);
-            }
+            const int v = lane < n ? (int)(w & LB_VALUE_MASK) : 0;
+            const int incl = warp_incl_sum(v);
+            if (lane < n) st_relaxed_gpu(words.base + pos + lane, LB_PREFIX | (uint64_t)(run + incl - v));
+            run += __shfl_sync(FULL_MASK, incl, 31);
             idle = 0;
             if (next >= num_tiles) {
                 __syncwarp();  // the bases of all lanes lie before the fence of the one that publishes the length
@@ -100,6 +83,7 @@ __device__ __forceinline__ int64_t scan_tile_counts(const TileWords &words, cons
             return -1;
         }
         pos = next;
+        w = w_next;
     }
 }
 

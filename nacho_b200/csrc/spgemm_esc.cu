@@ -1007,7 +1007,7 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
     const bool scanned = num_tiles > DIRECT_TILES;
     if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no rows
         if (threadIdx.x < 32) {
-            const int64_t total = scan_tile_counts<4>(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
             if (threadIdx.x == 0) finish(total);
         }
         return;
