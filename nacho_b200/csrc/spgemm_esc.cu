@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
 // are rows enough to keep the chip busy, because the broadcasts and addresses of a piece cost as much as 32 of its products
 // (pieces of 32 took 33 instructions per 32 products in the symbolic pass of 32768 vertices' heavy rows, of 128 take 23);
 // of SHORT products where there are few rows and the latency of each counts: the rows of B are then often shorter than LONG,
-// and the loads of four of them are in flight together (whole calls on graphs of 2698 / 9000 vertices 92 / 208 us, with LONG
+// and the loads of four of them are in flight together (whole calls on graphs of 2698 / 9000 vertices, before the words lay in order, 92 / 208 us, with LONG
 // pieces 105 / 235).
 constexpr int FLIGHT = 4, SHORT = 32, LONG = 32 * FLIGHT;
 
