@@ -81,6 +81,7 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
     std::lock_guard<std::mutex> g(g_ws_mutex);
     Workspace &ws = g_workspaces[{{dev, slot}, stream}];
     if (!ws.host) NB200_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&ws.host), 64 * sizeof(int64_t), cudaHostAllocDefault));
+    ++ws.generation;  // first of all: a block that fails to grow is gone too
     if (bytes > ws.dev_bytes) {
         if (ws.dev) {
             NB200_CUDA(cudaStreamSynchronize(stream));
@@ -92,7 +93,6 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
         NB200_CUDA(cudaMalloc(&ws.dev, want));
         ws.dev_bytes = want;
     }
-    ++ws.generation;
     *out = &ws;
     return NB200_OK;
 }

@@ -291,6 +291,41 @@ def test_numeric_after_other_work_on_the_stream(nacho, oracle):
     assert np.all(np.abs(val.cpu().numpy().astype(np.float64) - 2.0 * v64) <= 2.0 * REL_TOL * abs64 + 1e-30)
 
 
+def test_numeric_after_a_call_without_room(nacho, oracle):
+    """Between the two passes another product finds no room for its scratch, for which the pool gave its block back: the
+    numeric pass uses nothing of what the symbolic one left there."""
+    import ctypes as C
+    import torch
+    from nacho_b200 import _capi, synth
+    from nacho_b200._capi import CsrStruct, check as ck, lib
+    ta = synth.rmat_csr(scale=10, seed=4110)
+    tb = synth.transpose_csr(ta)
+    want, v64, abs64, _ = oracle.spgemm(synth_csr(ta), synth_csr(tb), 8, extras=True)
+    ga, gb = synth_to_gpu(ta), synth_to_gpu(tb)
+    sa, sb = ga._struct(), gb._struct()
+    rows = 100_000_000  # 20 bytes of scratch for each
+    empty = torch.zeros(rows + 1, dtype=torch.int32, device="cuda")
+    empty_rp = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+    entry, value = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, device="cuda")
+    large = CsrStruct(rows, want.rows, 0, empty.data_ptr(), entry.data_ptr(), value.data_ptr())
+    rp = torch.empty(want.rows + 1, dtype=torch.int32, device="cuda")
+    col, val = torch.empty(len(want.col), dtype=torch.int32, device="cuda"), torch.empty(len(want.col), dtype=torch.float32, device="cuda")
+    ck(lib.nb200_release_workspaces(), "release")
+    torch.cuda.empty_cache()
+    c = CsrStruct(0, 0, 0, rp.data_ptr(), None, None)
+    ck(lib.nb200_spgemm_f32_symbolic(C.byref(sa), C.byref(sb), C.byref(c), None, None), "symbolic")
+    held = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")
+    c_large = CsrStruct(0, 0, 0, empty_rp.data_ptr(), None, None)
+    assert lib.nb200_spgemm_f32_symbolic(C.byref(large), C.byref(sb), C.byref(c_large), None, None) == _capi.E_NOMEM
+    c.col, c.val = col.data_ptr(), val.data_ptr()
+    ck(lib.nb200_spgemm_f32_numeric(C.byref(sa), C.byref(sb), C.byref(c), None), "numeric")
+    torch.cuda.synchronize()
+    del held
+    torch.cuda.empty_cache()
+    assert np.array_equal(rp.cpu().numpy(), want.row_ptr) and np.array_equal(col.cpu().numpy(), want.col)
+    assert np.all(np.abs(val.cpu().numpy().astype(np.float64) - v64) <= REL_TOL * abs64 + 1e-30)
+
+
 def test_no_plan_outlives_a_call(nacho, oracle):
     """A's pattern is rewritten in place after a _bound call, to the same lengths at the same addresses: every form of the
     product that follows is that of the new pattern. The first one has rows of 5 entries, the second rows of up to 800."""
