@@ -1,6 +1,6 @@
 // The rows of a CSR matrix as bitmap words: for every 32 neighbouring columns of which a row stores any, one item
 // {number of the word, bits of its columns}. The rows of a graph are clustered, so a product that only asks which columns
-// there are (the symbolic pass of SpGEMM, the tests of the masked product) walks half as many items as entries
+// there are (the symbolic pass of SpGEMM) walks half as many items as entries
 // (R-MAT graphs of 50000 to 65536 vertices: 2.0 entries per item, weighted by how often a row is selected), and no two
 // items of a row lie in one word.
 #pragma once
@@ -9,11 +9,10 @@
 
 namespace nb200 {
 
-// Items of row r: items[rp[r]] .. items[rp[r + 1] - 1], in the order of their columns. first[item], where asked for: the entry
-// of the matrix, counted from its first one, that the lowest bit of the item stands for; the others follow.
+// Items of row r: items[rp[r]] .. items[rp[r + 1] - 1], in the order of their columns.
 struct RowWords {
     uint2 *items = nullptr;
-    int32_t *rp = nullptr, *first = nullptr;
+    int32_t *rp = nullptr;
 };
 
 constexpr int WORDS_NT = 256, WORDS_TILE = WORDS_NT * 8;  // entries of a CTA: eight groups of 32 per warp
@@ -26,14 +25,13 @@ struct RowWordsScratch {
     uint2 *groups;      // per 32 entries: items before them, and which of them begin an item
     static int tiles(int64_t nnz) { return (int)((nnz + WORDS_TILE) / WORDS_TILE); }  // position nnz has a group too
     template <typename C>
-    static RowWordsScratch carve(C &c, int64_t rows, int64_t nnz, bool with_first, size_t *clear_from, size_t *clear_bytes) {
+    static RowWordsScratch carve(C &c, int64_t rows, int64_t nnz, size_t *clear_from, size_t *clear_bytes) {
         RowWordsScratch s;
         *clear_from = c.used();
         s.starts = c.template take<uint32_t>((size_t)tiles(nnz) * (WORDS_TILE / 32) + 1);
         s.state = c.template take<uint64_t>((size_t)tiles(nnz) + 1);
         *clear_bytes = c.used() - *clear_from;
         s.out.items = c.template take<uint2>((size_t)nnz);
-        if (with_first) s.out.first = c.template take<int32_t>((size_t)nnz);
         s.out.rp = c.template take<int32_t>((size_t)rows + 1);
         s.groups = c.template take<uint2>((size_t)tiles(nnz) * (WORDS_TILE / 32));
         return s;
@@ -53,7 +51,7 @@ static __global__ void __launch_bounds__(256) k_words_starts(const int32_t *rp, 
 // item are collected by a segmented scan within 32 entries, and what runs over into the next 32 is added there. The
 // number of items before a CTA comes from the bounded look-back.
 static __global__ void __launch_bounds__(WORDS_NT) k_words_build(const int32_t *rp, const int32_t *col, int32_t nnz, const uint32_t *starts, uint2 *groups,
-                                                                uint2 *items, int32_t *first, uint64_t *state, FusedCtl *ctl) {
+                                                                uint2 *items, uint64_t *state, FusedCtl *ctl) {
     constexpr int G = WORDS_TILE / WORDS_NT;
     __shared__ int s_warp[WORDS_NT / 32];
     __shared__ long long s_base;
@@ -111,11 +109,7 @@ static __global__ void __launch_bounds__(WORDS_NT) k_words_build(const int32_t *
         const uint32_t over = __shfl_sync(FULL_MASK, bits[g + 1], 0);  // what lies before the first head of the next group
         const bool is_last = heads[g] >> lane == 1u;
         const uint32_t v = bits[g] | (is_last && !(heads[g + 1] & 1u) ? over : 0u);
-        if ((heads[g] >> lane) & 1u) {
-            const uint32_t at = run + __popc(heads[g] & ((1u << lane) - 1u));
-            items[at] = make_uint2((uint32_t)c[g] >> 5, v);
-            if (first) first[at] = (int32_t)(p0 + 32 * g + lane);
-        }
+        if ((heads[g] >> lane) & 1u) items[run + __popc(heads[g] & ((1u << lane) - 1u))] = make_uint2((uint32_t)c[g] >> 5, v);
         if (lane == 0) groups[(p0 >> 5) + g] = make_uint2(run, heads[g]);
         run += __popc(heads[g]);
     }
@@ -140,7 +134,7 @@ inline cudaError_t build_row_words(const int32_t *rp, const int32_t *col, int32_
     }
     if (e == cudaSuccess) {
         LaunchScope scope("row_words_build", stream);
-        e = launch_overlapped(k_words_build, dim3(RowWordsScratch::tiles(nnz)), dim3(WORDS_NT), 0, stream, rp, col, nnz, s.starts, s.groups, s.out.items, s.out.first, s.state, ctl);
+        e = launch_overlapped(k_words_build, dim3(RowWordsScratch::tiles(nnz)), dim3(WORDS_NT), 0, stream, rp, col, nnz, s.starts, s.groups, s.out.items, s.state, ctl);
     }
     if (e == cudaSuccess) {
         LaunchScope scope("row_words_rp", stream);

@@ -1244,12 +1244,12 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     if (listed > 0 && counts && plan->n_win == 1 && plan->host.products >= FORMS_FROM && plan->host.products >= REUSE * (unsigned long long)b->nnz) {
         size_t clear_from, clear_bytes;
         Carver word_sizes;
-        RowWordsScratch::carve(word_sizes, b->rows, b->nnz, false, &clear_from, &clear_bytes);
+        RowWordsScratch::carve(word_sizes, b->rows, b->nnz, &clear_from, &clear_bytes);
         Workspace *word_ws = nullptr;
         const int word_st = acquire_workspace(stream, word_sizes.used(), &word_ws, 4);
         if (word_st == NB200_OK) {  // without room the entries are walked
             Carver word_carve(word_ws->dev);
-            const RowWordsScratch scratch = RowWordsScratch::carve(word_carve, b->rows, b->nnz, false, &clear_from, &clear_bytes);
+            const RowWordsScratch scratch = RowWordsScratch::carve(word_carve, b->rows, b->nnz, &clear_from, &clear_bytes);
             NB200_CUDA(cudaMemsetAsync(static_cast<unsigned char *>(word_ws->dev) + clear_from, 0, clear_bytes, stream));
             // a give-up is reported by the scan that ends the symbolic pass
             NB200_CUDA(build_row_words(b->row_ptr, b->col, b->rows, b->nnz, scratch, reinterpret_cast<FusedCtl *>(plan->scan_block), stream));

@@ -9,8 +9,7 @@
 //                       how long is its mask row? The row goes on one of six lists.
 //   k_sssmm_bitmap      rows with many products, one CTA per row taken from a ticket: the mask row
 //                       becomes a bitmap over its column span in shared memory plus, per 64-bit
-//                       word, the count of set bits before it. A product tests one bit, or 32 columns of
-//                       B's row are tested at once (row_words.cuh); a hit finds
+//                       word, the count of set bits before it. A product tests one bit; a hit finds
 //                       its position in the mask row as rank + popcount and adds
 //                       (a_ij * b_jk) * c_ik -- the reference's expression, left to right -- to a
 //                       shared-memory accumulator (rows whose mask row is too long for that, or
@@ -30,7 +29,6 @@
 
 #include "block_utils.cuh"
 #include "merge_common.cuh"
-#include "row_words.cuh"
 
 namespace nb200 {
 
@@ -55,8 +53,8 @@ struct WorkClass {
     constexpr size_t smem() const { return size_t(12) * words + size_t(5) * entries + 16; }
 };
 constexpr WorkClass CLASS[4] = {
-    {1024, 2048, 256},    //  65536 columns of span, 22.5 KB: six CTAs per SM (40 registers)
-    {4096, 8192, 1024},   // 262144 columns, 88 KB: one CTA per SM (54 registers; the shared memory is there for two)
+    {1024, 2048, 256},    //  65536 columns of span, 22.5 KB: eight CTAs per SM
+    {4096, 8192, 1024},   // 262144 columns, 88 KB: two CTAs per SM
     {16384, 0, 1024},     // 2^20 columns, 192 KB, sums in global memory: one CTA per SM
     {0, 0, SEARCH_NT},    // wider still: no bitmap, binary search
 };
@@ -190,7 +188,6 @@ __global__ void __launch_bounds__(256) k_sssmm_classify(CsrView A, CsrView B, Cs
         int2 *to = units + (list == LIST_MASK ? 4 : list) * list_cap + at;
         for (int u = lane; u < n_units; u += 32) to[u] = make_int2((int)row_of(r), s_lo[r] + u * unit);
     }
-    finish_after_previous();
 }
 
 // One product column k of the mask row [c_lo, c_hi) by binary search; on a hit the product goes to
@@ -335,11 +332,7 @@ __global__ void __launch_bounds__(256) k_sssmm_look_up(CsrView A, CsrView B, Csr
     finish_after_previous();
 }
 
-// Entries of B from which on its rows are walked as bitmap words, which three short kernels make. A graph of 24405 vertices,
-// 244 K entries: 153 us without, 169 with; of 50021 vertices, 680 K entries, 447; of 65536, 956 K entries, 764; of 262144,
-// 3.9 M entries, 4230 (as entries, and with a search for every chunk, those took 481, 848 and 5264).
-constexpr int WORDS_FROM = 1 << 18;
-// Shared memory of a unit's walk: for every entry of the unit, the bounds of its row of B, its
+// Shared memory of unit_products: for every entry of the unit, the bounds of its row of B, its
 // value, and the number of chunks in front of it.
 template <int NT>
 struct UnitRows {
@@ -349,19 +342,23 @@ struct UnitRows {
     int tmp[34];
 };
 
-// What the entries [p_begin, p_end) of A's row select of B, spread evenly over the warps of the CTA: the rows of B, ranges of
-// entries or of bitmap words by `rp`, are cut into chunks of CHUNK, the chunks are numbered through (an exclusive sum over the
-// entries) and every warp takes a contiguous share of them. For 32 chunks at a time every lane finds the entry of one of them by
-// binary search in the shared-memory sums; then the chunks go by, what their lane knows broadcast: f(position of the lane's
-// first item in B, items from there on, A's value), the lane's items 32 apart. The CTA must be in step on entry.
-template <int NT, int CHUNK, typename F>
-__device__ __forceinline__ void unit_chunks(const CsrView &A, const int32_t *rp, int32_t p_begin, int32_t p_end, UnitRows<NT> &rows, F f) {
+// The products of the entries [p_begin, p_end) of A's row, spread evenly over the warps of the CTA: the rows of B the entries
+// select are cut into chunks, the chunks are numbered through (an exclusive sum over the entries) and every warp takes a
+// contiguous share of them. For 32 chunks at a time every lane finds the entry of one of them by binary search in the
+// shared-memory sums; then the chunks go by, what their lane knows broadcast. The CTA must be in step on entry. `reaches(k)` says
+// whether the mask may hold column k; `hit(q, a)` receives the position in B and A's value of those products that
+// pass. The two are apart because few pass (one in sixteen on R-MAT graphs) and a lane that does makes its whole warp walk the
+// long way: the tests of a chunk are done first, then every lane works off its own hits, so the long way is walked as often
+// as the luckiest lane has hits (under 3 times per 8 products) and not once per product.
+template <int NT, typename Reaches, typename Hit>
+__device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B, int32_t p_begin, int32_t p_end, UnitRows<NT> &rows, Reaches reaches, Hit hit) {
     constexpr int NW = NT / 32;
+    constexpr int PER_LANE = 8, CHUNK = 32 * PER_LANE;  // products of a chunk per lane: that many loads in flight
     const int tid = threadIdx.x, lane = lane_id(), n_e = p_end - p_begin;
     int chunks = 0;
     if (tid < n_e) {
         const int32_t j = ld_nc(A.col + p_begin + tid);
-        const int32_t lo = ld_late(rp + j), hi = ld_late(rp + j + 1);
+        const int32_t lo = ld_nc(B.rp + j), hi = ld_nc(B.rp + j + 1);
         rows.av[tid] = ld_nc(A.val + p_begin + tid);
         rows.lo[tid] = lo;
         rows.hi[tid] = hi;
@@ -385,65 +382,17 @@ __device__ __forceinline__ void unit_chunks(const CsrView &A, const int32_t *rp,
         const int here = min(32, end - c0);
         for (int u = 0; u < here; ++u) {
             const int32_t q = __shfl_sync(FULL_MASK, my_q, u) + lane, n = __shfl_sync(FULL_MASK, my_hi, u) - q;
-            f(q, n, __shfl_sync(FULL_MASK, my_a, u));
+            const float a = __shfl_sync(FULL_MASK, my_a, u);
+            int32_t k[PER_LANE];
+#pragma unroll
+            for (int t = 0; t < PER_LANE; ++t) k[t] = 32 * t < n ? ld_nc(B.col + q + 32 * t) : -1;
+            unsigned hits = 0;
+#pragma unroll
+            for (int t = 0; t < PER_LANE; ++t)
+                if (k[t] >= 0 && reaches(k[t])) hits |= 1u << t;
+            for (; hits; hits &= hits - 1u) hit(q + 32 * (__ffs((int)hits) - 1), a);
         }
     }
-}
-
-// `reaches(column)` says whether the mask may hold it; `hit(q, a)` receives the products that pass. The two are apart because few
-// pass (one in sixteen on R-MAT graphs) and a lane that does makes its whole warp walk the long way: the tests of a chunk
-// are done first, then every lane works off its own hits, so the long way is walked as often as the luckiest lane has hits
-// (under 3 times per 8 products) and not once per product.
-template <int NT, typename Reaches, typename Hit>
-__device__ __forceinline__ void unit_products(const CsrView &A, const CsrView &B, int32_t p_begin, int32_t p_end, UnitRows<NT> &rows, Reaches reaches, Hit hit) {
-    constexpr int PER_LANE = 8;  // products of a chunk per lane: that many loads in flight
-    unit_chunks<NT, 32 * PER_LANE>(A, B.rp, p_begin, p_end, rows, [&](int32_t q, int32_t n, float a) {
-        int32_t k[PER_LANE];
-#pragma unroll
-        for (int u = 0; u < PER_LANE; ++u) k[u] = 32 * u < n ? ld_nc(B.col + q + 32 * u) : -1;
-        unsigned hits = 0;
-#pragma unroll
-        for (int u = 0; u < PER_LANE; ++u)
-            if (k[u] >= 0 && reaches(k[u])) hits |= 1u << u;
-        for (; hits; hits &= hits - 1u) hit(q + 32 * (__ffs((int)hits) - 1), a);
-    });
-}
-
-// The same over the bitmap words of B's rows (row_words.cuh): `common(item)` gives the columns of an item that the mask holds, and
-// hit(item number, a) receives the items that have any. A fifth of the items of an R-MAT graph's hub rows do, spread over the lanes
-// of every chunk, so they are queued, and worked off 32 at a time by a full warp: the bitmap rows of 50021 vertices' graph 261 us,
-// with every lane working off its own 399. What is left there is their shared-memory atomics (30 hits per mask position), and
-// the two trips to L2 that a batch of hits makes.
-constexpr int QUEUE = 64;  // less than 32 wait, and a step adds 32 at most
-template <int NT, typename Common, typename Hit>
-__device__ __forceinline__ void unit_words(const CsrView &A, const RowWords &B, int32_t p_begin, int32_t p_end, UnitRows<NT> &rows, uint2 *queue, Common common,
-                                           Hit hit) {
-    constexpr int PER_LANE = 4;
-    const int lane = lane_id();
-    int waiting = 0;
-    auto work_off = [&](int n) {  // the last n of those that wait
-        __syncwarp();
-        waiting -= n;
-        const uint2 e = queue[waiting + min(lane, n - 1)];
-        __syncwarp();
-        if (lane < n) hit((int32_t)e.x, __uint_as_float(e.y));
-    };
-    unit_chunks<NT, 32 * PER_LANE>(A, B.rp, p_begin, p_end, rows, [&](int32_t q, int32_t n, float a) {
-        uint2 item[PER_LANE];
-#pragma unroll
-        for (int u = 0; u < PER_LANE; ++u)
-            if (32 * u < n) item[u] = ld_late(B.items + q + 32 * u);
-#pragma unroll
-        for (int u = 0; u < PER_LANE; ++u) {
-            const bool any = 32 * u < n && common(item[u]) != 0u;
-            const unsigned lanes = __ballot_sync(FULL_MASK, any);
-            if (lanes == 0u) continue;
-            if (any) queue[waiting + __popc(lanes & ((1u << lane) - 1u))] = make_uint2((uint32_t)(q + 32 * u), __float_as_uint(a));
-            waiting += __popc(lanes);
-            if (waiting >= 32) work_off(32);
-        }
-    });
-    if (waiting > 0) work_off(waiting);
 }
 
 __global__ void __launch_bounds__(SEARCH_NT) k_sssmm_search_cta(CsrView A, CsrView B, CsrView C, const int2 *__restrict__ units,
@@ -457,15 +406,19 @@ __global__ void __launch_bounds__(SEARCH_NT) k_sssmm_search_cta(CsrView A, CsrVi
         const int2 unit = units[t];
         const int64_t i = unit.x;
         const int32_t c_lo = ld_nc(C.rp + i), c_hi = ld_nc(C.rp + i + 1);
-        unit_products<SEARCH_NT>(A, B, unit.y, min(unit.y + CLASS[LIST_WIDE].unit(), ld_nc(A.rp + i + 1)), s_rows, [](int32_t) { return true; }, [&](int32_t q, float av) { search_product(B, C, q, ld_nc(B.col + q), av, c_lo, c_hi, c0, acc, hit); });
+        unit_products<SEARCH_NT>(A, B, unit.y, min(unit.y + CLASS[LIST_WIDE].unit(), ld_nc(A.rp + i + 1)), s_rows, [](int32_t) { return true; },
+                                 [&](int32_t q, float av) { search_product(B, C, q, ld_nc(B.col + q), av, c_lo, c_hi, c0, acc, hit); });
         __syncthreads();
     }
     finish_after_previous();
 }
 
-// `B_words`, where given: the rows of B as bitmap words (row_words.cuh), whose 32 columns are tested at once.
-template <int NT, bool SHARED_ACC, bool WORDS>
-__global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrView C, RowWords B_words, const int2 *units,
+// What covers the latency of a product's loads is the number of warps, so a thread is held to 32 registers, eight and two CTAs
+// per SM instead of six and one: a graph of 50021 vertices squared on its own positions 484 -> 412 us a call, of 24405 204 -> 190, of
+// 131072 2270 -> 1555. (The rows of B as bitmap words, 32 columns to a test, need 48 and 64 registers, three kernels in front and 12
+// bytes of scratch per entry of B, and were behind at every size: 450, 204 and 1806 us.)
+template <int NT, bool SHARED_ACC>
+__global__ void __launch_bounds__(NT, 2048 / NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrView C, const int2 *units,
                                                     SssmmCtl *ctl, int which, int words_cap, int entries_cap,
                                                     float *__restrict__ acc, int32_t *__restrict__ hit) {
     extern __shared__ uint64_t sm_words[];
@@ -476,7 +429,6 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
     unsigned char *flag_s = reinterpret_cast<unsigned char *>(acc_s + entries_cap);
     __shared__ int2 s_unit;
     __shared__ UnitRows<NT> s_rows;
-    __shared__ uint2 s_queue[WORDS ? NT / 32 : 1][WORDS ? QUEUE : 1];
     // The list kernels run side by side. Only the first (which == 2) waits for the lists, and lets the next
     // one start after that; each of the others lets its successor start at once.
     if (which == 2) wait_for_previous();
@@ -525,8 +477,13 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
         __syncthreads();
         const int32_t col0 = w0 << 6;
         const uint32_t span = (uint32_t)words << 6;
-        const int32_t p_end = min(unit.y + WARP_ENTRIES * (NT / 32), ld_nc(A.rp + i + 1));
-        auto add = [&](int32_t pos, int32_t q, float av) {  // B's entry q reaches the mask row's position pos
+        unit_products<NT>(A, B, unit.y, min(unit.y + WARP_ENTRIES * (NT / 32), ld_nc(A.rp + i + 1)), s_rows, [&](int32_t k) {
+            const uint32_t bit = (uint32_t)(k - col0);
+            return bit < span && ((bm32[bit >> 5] >> (bit & 31)) & 1u) != 0u;  // most products end here
+        }, [&](int32_t q, float av) {
+            const uint32_t bit = (uint32_t)(ld_nc(B.col + q) - col0);  // the column again, from cache: an index into registers would cost more
+            const uint32_t w = bit >> 6, sh = bit & 63;
+            const int32_t pos = (int32_t)rank[w] + __popcll(bm[w] & ((1ull << sh) - 1));
             const float v = (av * ld_nc(B.val + q)) * ld_nc(C.val + c_lo + pos);
             if (SHARED_ACC) {
                 atomicAdd(acc_s + pos, v);
@@ -535,33 +492,7 @@ __global__ void __launch_bounds__(NT) k_sssmm_bitmap(CsrView A, CsrView B, CsrVi
                 atomicAdd(acc + (c_lo - c0 + pos), v);
                 hit[c_lo - c0 + pos] = 1;
             }
-        };
-        if (WORDS) {
-            const uint32_t first_word = (uint32_t)w0 << 1, n_words = (uint32_t)words << 1;
-            const int32_t b0 = ld_nc(B.rp);
-            auto common = [&](uint2 item) {
-                const uint32_t w = item.x - first_word;
-                return w < n_words ? bm32[w] & item.y : 0u;
-            };
-            unit_words<NT>(A, B_words, unit.y, p_end, s_rows, s_queue[warp_id()], common, [&](int32_t q, float av) {
-                const uint2 item = ld_late(B_words.items + q);
-                const int32_t at = b0 + ld_late(B_words.first + q);
-                const uint32_t w = item.x - first_word, mask = bm32[w];
-                const int32_t before = (int32_t)rank[w >> 1] + (w & 1u ? __popc(bm32[w - 1]) : 0);
-                for (uint32_t both = mask & item.y; both; both &= both - 1u) {
-                    const uint32_t below = (both & (0u - both)) - 1u;
-                    add(before + __popc(mask & below), at + __popc(item.y & below), av);
-                }
-            });
-        } else {
-            unit_products<NT>(A, B, unit.y, p_end, s_rows, [&](int32_t k) {
-                const uint32_t bit = (uint32_t)(k - col0);
-                return bit < span && ((bm32[bit >> 5] >> (bit & 31)) & 1u) != 0u;  // most products end here
-            }, [&](int32_t q, float av) {
-                const uint32_t bit = (uint32_t)(ld_nc(B.col + q) - col0);  // the column again, from cache: an index into registers would cost more
-                add((int32_t)rank[bit >> 6] + __popcll(bm[bit >> 6] & ((1ull << (bit & 63)) - 1)), q, av);
-            });
-        }
+        });
         __syncthreads();
         if (SHARED_ACC) {  // other units of the same row add to the same sums
             for (int p = tid; p < entries; p += NT)
@@ -662,12 +593,8 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
         return NB200_OK;
     }
     // per device, so set on every call: cheap next to the launches that follow
-    const bool with_words = b->nnz >= WORDS_FROM;
-    auto bitmap_wide = with_words ? k_sssmm_bitmap<1024, false, true> : k_sssmm_bitmap<1024, false, false>;
-    auto bitmap_medium = with_words ? k_sssmm_bitmap<1024, true, true> : k_sssmm_bitmap<1024, true, false>;
-    auto bitmap_narrow = with_words ? k_sssmm_bitmap<256, true, true> : k_sssmm_bitmap<256, true, false>;
-    NB200_CUDA(cudaFuncSetAttribute(bitmap_medium, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLASS[1].smem()));
-    NB200_CUDA(cudaFuncSetAttribute(bitmap_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLASS[2].smem()));
+    NB200_CUDA(cudaFuncSetAttribute(k_sssmm_bitmap<1024, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLASS[1].smem()));
+    NB200_CUDA(cudaFuncSetAttribute(k_sssmm_bitmap<1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CLASS[2].smem()));
     int device = 0, sms = 148;
     NB200_CUDA(cudaGetDevice(&device));
     NB200_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -680,12 +607,6 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     sizes.take<int32_t>((size_t)nnz + 1);
     sizes.take<uint64_t>((size_t)scan_ctas + 8);
     sizes.take<SssmmCtl>(1);
-    size_t clear_from, clear_bytes;
-    RowWordsScratch b_words;
-    auto carve_words = [&](Carver &c) {  // (what it clears comes first, behind the other things that are cleared)
-        if (with_words) b_words = RowWordsScratch::carve(c, b->rows, b->nnz, true, &clear_from, &clear_bytes);
-    };
-    carve_words(sizes);
     sizes.take<int2>((size_t)4 * list_cap + mask_cap);
     sizes.take<int32_t>((size_t)rows);
     Workspace *ws = nullptr;
@@ -695,44 +616,34 @@ int sssmm_run(const nb200_csr *a, const nb200_csr *b, const nb200_csr *c, nb200_
     int32_t *hit = carve.take<int32_t>((size_t)nnz + 1);
     uint64_t *scan_block = carve.take<uint64_t>((size_t)scan_ctas + 8);
     SssmmCtl *sctl = carve.take<SssmmCtl>(1);
-    carve_words(carve);
-    const size_t clear = with_words ? clear_from + clear_bytes : carve.used();
     int2 *units = carve.take<int2>((size_t)4 * list_cap + mask_cap);
     int32_t *light = carve.take<int32_t>((size_t)rows);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(scan_block);
     // sums, flags and control blocks lie next to one another: one fill clears them all
-    NB200_CUDA(cudaMemsetAsync(acc, 0, clear, stream));
+    NB200_CUDA(cudaMemsetAsync(acc, 0, (size_t)(reinterpret_cast<unsigned char *>(units) - reinterpret_cast<unsigned char *>(acc)), stream));
     unsigned long long *word = result_word(ws, 0);
     const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val}, C{c->row_ptr, c->col, c->val};
     const int row_warps_grid = (int)std::min<int64_t>(((int64_t)rows + 7) / 8, (int64_t)sms * 8);
     const int most = (int)std::min<int64_t>(list_cap, 1 << 30);
-    if (with_words) NB200_CUDA(build_row_words(b->row_ptr, b->col, b->rows, b->nnz, b_words, ctl, stream));
     {
         LaunchScope scope("sssmm_classify", stream);
-        const dim3 grid((unsigned)(((int64_t)rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA));
-        if (with_words) {  // beside the end of the kernels in front of it, which it needs nothing of
-            NB200_CUDA(launch_overlapped(k_sssmm_classify, grid, dim3(256), 0, stream, A, B, C, rows, list_cap, units, light, sctl));
-        } else {
-            k_sssmm_classify<<<grid, 256, 0, stream>>>(A, B, C, rows, list_cap, units, light, sctl);
-            NB200_CUDA(cudaGetLastError());
-        }
+        k_sssmm_classify<<<(int)(((int64_t)rows + ROWS_PER_CTA - 1) / ROWS_PER_CTA), 256, 0, stream>>>(A, B, C, rows, list_cap, units, light, sctl);
     }
     // Every list is worked by resident CTAs that take units from a ticket; a list's length stays on
-    // the device, so an empty list costs one launch of CTAs that leave at once. (The grids are those of the shared memory;
-    // where registers let fewer CTAs in, the others find the list worked off.)
+    // the device, so an empty list costs one launch of CTAs that leave at once.
     {
         LaunchScope scope("sssmm_bitmap_wide", stream);
-        NB200_CUDA(launch_overlapped(bitmap_wide, dim3(std::min(sms, most)), dim3(1024), CLASS[2].smem(), stream, A, B, C, b_words.out,
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<1024, false>, dim3(std::min(sms, most)), dim3(1024), CLASS[2].smem(), stream, A, B, C,
                                      units + 2 * list_cap, sctl, 2, CLASS[2].words, 0, acc, hit));
     }
     {
         LaunchScope scope("sssmm_bitmap_medium", stream);
-        NB200_CUDA(launch_overlapped(bitmap_medium, dim3(std::min(2 * sms, most)), dim3(1024), CLASS[1].smem(), stream, A, B, C, b_words.out,
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<1024, true>, dim3(std::min(2 * sms, most)), dim3(1024), CLASS[1].smem(), stream, A, B, C,
                                      units + list_cap, sctl, 1, CLASS[1].words, CLASS[1].entries, acc, hit));
     }
     {
         LaunchScope scope("sssmm_bitmap_narrow", stream);
-        NB200_CUDA(launch_overlapped(bitmap_narrow, dim3(std::min(8 * sms, most)), dim3(256), CLASS[0].smem(), stream, A, B, C, b_words.out, units, sctl, 0,
+        NB200_CUDA(launch_overlapped(k_sssmm_bitmap<256, true>, dim3(std::min(8 * sms, most)), dim3(256), CLASS[0].smem(), stream, A, B, C, units, sctl, 0,
                                      CLASS[0].words, CLASS[0].entries, acc, hit));
     }
     {

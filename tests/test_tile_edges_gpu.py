@@ -164,8 +164,8 @@ def check_masked(nacho, oracle, a, b, c):
 
 @pytest.mark.parametrize("cols", [60000, 300000])
 def test_masked_rows_by_words(nacho, oracle, cols):
-    """A second operand of 2^18 entries and more, walked as bitmap words: mask rows up to the bitmaps' largest, products that miss, meet
-    one column of a word or all 32."""
+    """A second operand of 2^18 entries and more: mask rows up to the bitmaps' largest, products that miss, meet one column of a
+    bitmap's word or all 32."""
     rng = np.random.default_rng(cols)
     rows, inner = 60, 1200
     b_rows = [np.sort(rng.choice(cols, 240, replace=False)) if r % 3 else np.arange(q := int(rng.integers(0, cols - 400)), q + 250 + r % 60) for r in range(inner)]
