@@ -161,10 +161,11 @@ struct TilePlan {
 };
 constexpr uint32_t ROW_FAR = 0xffffu;
 
-// A tile of short rows asks for the row offsets of one that starts a few microseconds later, so that they wait in L2: they are
-// read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns ahead
-// as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.)
-constexpr int TILES_AHEAD = 148;
+// A tile, other than the large one, asks for the row offsets of one that starts a few microseconds later, so that they wait in L2:
+// they are read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns
+// ahead as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.) Not for a tile that starts with the
+// first ones, and at most as many offsets as a tile keeps: beyond those lie runs of empty rows, which could fill the L2.
+constexpr int TILES_AHEAD = 148, RESIDENT = 592;
 
 // Fixed shared memory of a tile (one block for both key widths).
 struct TileShared {
@@ -700,8 +701,8 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     if (cuts) {
         const int4 c0 = cuts[t], c1 = cuts[t + 1];
         tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
-        if (V != V_MOST && threadIdx.x == 96 && t + TILES_AHEAD < num_tiles) {
-            const int32_t r0 = cuts[t + TILES_AHEAD].x, n = cuts[t + TILES_AHEAD + 1].x - r0 + 1;
+        if (V != V_MOST && threadIdx.x == 96 && t + TILES_AHEAD >= RESIDENT && t + TILES_AHEAD < num_tiles) {
+            const int32_t r0 = cuts[t + TILES_AHEAD].x, n = min(cuts[t + TILES_AHEAD + 1].x - r0, TilePlan<V, LEVELS>::ROWS) + 1;
             if (A.rp) prefetch_l2(A.rp + r0, n);
             if (B.rp) prefetch_l2(B.rp + r0, n);
         }

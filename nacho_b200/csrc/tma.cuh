@@ -58,10 +58,11 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gmem_src, 
                  : "memory");
 }
 
-// Asks for the L2 lines of `count` 4-byte elements at `p` (the 16-byte-aligned part of the range).
+// Asks for the L2 lines of `count` 4-byte elements at `p` (the 16-byte-aligned part of the range), 64 MB at most: what lies
+// further on would be gone from L2 again before anything reads it.
 __device__ __forceinline__ void prefetch_l2(const void *p, int count) {
     const uintptr_t from = (reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15);
-    const uintptr_t to = (reinterpret_cast<uintptr_t>(p) + 4 * (uintptr_t)count) & ~uintptr_t(15);
+    const uintptr_t to = (reinterpret_cast<uintptr_t>(p) + 4 * (uintptr_t)(count < 1 << 24 ? count : 1 << 24)) & ~uintptr_t(15);
     if (to > from)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from), "r"((uint32_t)(to - from)) : "memory");
 }

@@ -66,6 +66,23 @@ def test_csr_tiles(nacho, oracle, total, shape):
     assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, csr_to_gpu(c))), oracle.csr_add_3(a, b, c, 8), "add_3")
 
 
+@pytest.mark.parametrize("gap", [3000, 1_200_000])
+def test_runs_of_empty_rows(nacho, oracle, gap):
+    """More tiles than fit the chip at once, with more rows between two of them than a tile keeps offsets of, empty but for a few: what a tile
+    asks for ahead of time ends there."""
+    rng = np.random.default_rng(gap)
+    clusters, entries, cols = 16, 160_000, 5000
+    rows = clusters * (gap + 1000)
+    key = [np.sort(rng.choice(1000 * cols, entries, replace=False)) + c * (gap + 1000) * cols for c in range(clusters)]
+    ka = np.concatenate(key)
+    kb = np.sort(np.unique(np.concatenate([ka[::3], ka[1::4] + 1])))
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb[kb < rows * cols], rows, cols, rng)
+    assert len(a.col) + len(b.col) > 700 * SMALL_STEP
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+
+
 @pytest.mark.parametrize("dims", [(3, 4, 1 << 28), (1 << 26, 9, 5), (1 << 20, 1 << 21, 1 << 22)])
 @pytest.mark.parametrize("total", [1, COO_STEP, COO_STEP + 1, DIRECT_TILES * COO_STEP + 1, 3_000_000, 4096 * (256 * 17 - 1) + 1])
 def test_coordinate_tiles(nacho, oracle, total, dims):
