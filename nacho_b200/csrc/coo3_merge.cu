@@ -343,10 +343,10 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         return;
     }
 
-    // ---- fetch coordinates and values, result entries q * NT + tid, the first round before the output base is asked for. Every round
-    // is a trip to L2 (17 entries in rounds of 8, 9, 17: 1196, 1196, 1179 us at 100 M entries per operand); 64-bit keys would not
-    // fit the registers all at once.
-    constexpr int GATHER = NARROW ? VT : 8;
+    // ---- fetch coordinates and values, result entries q * NT + tid, the first round before the output base is asked for. Every round is a
+    // trip to L2 (17 entries in rounds of 8, 9, 17: 549, 547, 527 us at 41 M entries per operand, 1198, 1193, 1185 at 100 M); 64-bit keys
+    // would not fit the registers all at once, nor does a fill behind a count (56 bytes of spills).
+    constexpr int GATHER = NARROW && MODE != MODE_FILL ? VT : 8;
     const uint32_t first_b = 4u * (uint32_t)ob;
     Key key[GATHER];
     float val[GATHER];

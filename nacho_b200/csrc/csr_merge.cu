@@ -522,8 +522,9 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     const char *va = reinterpret_cast<const char *>(ga_val) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(gb_val) - 4 * (int64_t)ob;
     const uint32_t first_b = 4u * (uint32_t)ob;
     // Result entries a thread fetches together. A round is a trip to L2, so the smaller tiles take one or two. In the large
-    // tile, bound by throughput, 8 are better than 11 or 16 (67 M entries 449, 465, 483 us); intersections leave fewer.
-    constexpr int GATHER = OP == OP_INTERSECT || VT == V_MOST ? 8 : VT <= 16 ? VT : (VT + 1) / 2;
+    // tile, bound by throughput, 8 are better than 11 or 16 (67 M entries 449, 465, 483 us); intersections leave fewer, and a fill behind a
+    // count has no registers for more.
+    constexpr int GATHER = OP == OP_INTERSECT || VT == V_MOST || MODE == MODE_FILL ? 8 : VT <= 16 ? VT : (VT + 1) / 2;
     uint32_t col[GATHER];
     float val[GATHER];
     auto gather = [&](const int q0) {
