@@ -1362,6 +1362,13 @@ int prepare_numeric(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan,
     return NB200_OK;
 }
 
+// An SM's split between L1 and shared memory stays while CTAs are on it, and the kernel of the sorted rows, which starts beside that of
+// a few ranked rows, wants 100 KB for a full SM: a split that suits a short table alone (512 columns, 32 KB) shuts it out. (Graphs of
+// 500 / 2000 / 2700 vertices with 16 / 4 / 4 edges each: calls of 67 / 74 / 75 us, with room for both 57 / 65 / 64. All of the SM for
+// shared memory is no better, and 1 % behind where the tables are long.)
+constexpr size_t FEW_STATIC = 6 * 1024, BESIDE_SMEM = 100 * 1024, SM_SMEM = 228 * 1024;
+int shared_percent(size_t wanted) { return (int)std::min<size_t>(100, (100 * std::max(wanted, BESIDE_SMEM) + SM_SMEM - 1) / SM_SMEM); }
+
 template <int CLS>
 int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, const NumericPlan &numeric, int first, int last, const nb200_csr *c, cudaStream_t stream,
                 bool beside) {
@@ -1384,6 +1391,7 @@ int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, con
         if (numeric.pairs) kernel = narrow ? k_esc_rank<CLS, true, true> : k_esc_rank<CLS, false, true>;
     // the most that any call asks for: several threads may be here with different sizes
     NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(K.smem, (size_t)RK_WORDS * 8)));
+    if (CLS >= CLASSES) NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, shared_percent(K.per_sm * (smem + FEW_STATIC))));
     return launch_bin(beside, kernel, ctas, K.nt, smem, stream, CsrView{a->row_ptr, a->col, a->val},
                       CsrView{b->row_ptr, b->col, b->val}, numeric.pairs, Windows{plan.n_win, plan.win_ptr}, listed_rows(plan, a->rows), first, last,
                       CLS < CLASSES ? plan.class_rows + (size_t)CLS * last : nullptr, plan.classes, plan.words, slots, plan.cache, c->row_ptr, c->col, c->val);
