@@ -38,7 +38,7 @@ constexpr int SMALL_P = 32;
 #endif
 constexpr int MEDIUM_P = ESC_MEDIUM_P;
 constexpr int MED_NT = 128;
-constexpr unsigned long long RANKED_P = 65535;   // 16-bit ranks up to here
+constexpr unsigned long long RANKED_P = 65535;   // rows above are heavy: larger symbolic CTAs, first in every list
 constexpr unsigned long long GIANT_P = 1ull << 18;
 
 struct CsrView {
@@ -1129,15 +1129,18 @@ struct EscPlan {
     unsigned long long *result;  // result words
 };
 
+// Another form of B is made for products that read every entry of it this often, and of which there are this many: its words take
+// four short launches (some 25 us with nothing beside them, and 11 per million entries), its pairs one of 9. A graph of 24405 vertices, 49 M
+// products: the whole call 468 -> 357 us with both and the classes; of 9000 vertices, 7 M products, it would take 20 us more. How
+// much the words save depends on how the columns lie together, which is not known before they are made: the entries of a band,
+// read 41 times each, 2514 -> 2175 us a call; scattered ones, read 23 to 30 times, cost 4 to 5 % (9000 rows of 6000 products, 130000
+// columns: 493 us with, 470 without).
+constexpr unsigned long long PAIRS_REUSE = 16, WORDS_REUSE = 32, FORMS_FROM = 32 << 20;
+constexpr size_t BITMAP_CACHE_BUDGET = size_t(8) << 30;  // bytes of bitmaps carried between the passes of one call
+
 // Bins the rows (kernel + one read-back) and carves the scratch of a symbolic pass, a numeric
 // pass, or one after the other. `counts`: rows without products get their count written
 // (needed by the symbolic pass).
-// Another form of B is made for products that read every entry of it this often, and of which there are this many: its words take
-// four short launches (some 25 us with nothing beside them), its pairs one of 9. A graph of 24405 vertices, 49 M products:
-// the whole call 468 -> 357 us with both and the classes; of 9000 vertices, 7 M products, it would take 20 us more.
-constexpr unsigned long long REUSE = 16, FORMS_FROM = 32 << 20;
-constexpr size_t BITMAP_CACHE_BUDGET = size_t(8) << 30;  // bytes of bitmaps carried between the passes of one call
-
 int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_bitmaps, cudaStream_t stream, EscPlan *plan) {
     const int32_t rows = a->rows;
     const int64_t n_win = std::max<int64_t>(1, ((int64_t)b->cols + RK_WINDOW_COLS - 1) / RK_WINDOW_COLS);
@@ -1241,7 +1244,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
             return row_st;
         }  // without room the numeric pass walks the products twice, as it does on its own, and takes all rows in one launch
     }
-    if (listed > 0 && counts && plan->n_win == 1 && plan->host.products >= FORMS_FROM && plan->host.products >= REUSE * (unsigned long long)b->nnz) {
+    if (listed > 0 && counts && plan->n_win == 1 && plan->host.products >= FORMS_FROM && plan->host.products >= WORDS_REUSE * (unsigned long long)b->nnz) {
         size_t clear_from, clear_bytes;
         Carver word_sizes;
         RowWordsScratch::carve(word_sizes, b->rows, b->nnz, &clear_from, &clear_bytes);
@@ -1350,7 +1353,7 @@ int prepare_numeric(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan,
         k_esc_classes<<<(listed.n + 255) / 256, 256, 0, stream>>>(listed, c_rp, most, plan.class_rows, listed.n, plan.classes);
         NB200_CUDA(cudaGetLastError());
     }
-    if (!numeric->classes || plan.host.products < FORMS_FROM || plan.host.products < REUSE * (unsigned long long)b->nnz) return NB200_OK;
+    if (!numeric->classes || plan.host.products < FORMS_FROM || plan.host.products < PAIRS_REUSE * (unsigned long long)b->nnz) return NB200_OK;
     Workspace *ws = nullptr;
     const int st = acquire_workspace(stream, (size_t)b->nnz * sizeof(uint2), &ws, 5);
     if (st != NB200_OK) return st == NB200_E_NOMEM ? NB200_OK : st;  // without room columns and values are loaded apart
