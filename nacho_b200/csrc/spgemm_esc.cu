@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(MED_NT) k_esc_medium(CsrView A, CsrView B, con
 // are rows enough to keep the chip busy, because the broadcasts and addresses of a piece cost as much as 32 of its products
 // (pieces of 32 took 33 instructions per 32 products in the symbolic pass of 32768 vertices' heavy rows, of 128 take 23);
 // of SHORT products where there are few rows and the latency of each counts: the rows of B are then often shorter than LONG,
-// and the loads of four of them are in flight together (whole calls on graphs of 2698 / 9000 vertices, before the words lay in order, 92 / 208 us, with LONG
-// pieces 105 / 235).
+// and the loads of four of them are in flight together (whole calls on graphs of 2700 / 9000 vertices with SHORT pieces 98 / 229 us;
+// with LONG ones such graphs took a seventh more).
 constexpr int FLIGHT = 4, SHORT = 32, LONG = 32 * FLIGHT;
 
 // The rows of B that a chunk of A's row selects, as segments: segment k covers the pieces [first[k], first[k + 1]) of
@@ -607,8 +607,13 @@ __device__ __forceinline__ void walk_segments(const Segments<NT> &seg, Load load
 constexpr int RK_WORDS = 8192;                     // bitmap words of one column window in shared memory
 constexpr int RK_WINDOW_COLS = RK_WORDS * 32;      // 262144 columns per window
 constexpr size_t RK_PTR_BUDGET = size_t(1) << 30;  // bytes of the window pointer table; beyond it windows are searched on the fly
-constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a symbolic CTA for rows up to / above RANKED_P products
-constexpr int MANY_NT = 128, MANY_ROWS = 8192;     // ... and up to RANKED_P where there are many
+constexpr int RK_NT = 256, HEAVY_NT = 512;         // threads of a symbolic CTA for rows up to / above RANKED_P products ...
+// ... and up to RANKED_P where there are many, in windows of up to 131072 columns. A wider window's table takes 64 KB: rows of few results
+// then share an SM better without sums beside it. (Products per row, result columns: 6000, 200000 907 us with the numeric pass by classes
+// and the small symbolic CTAs, 685 without; 400, 400000 22.5 against 18.3 ms; 441 of a band, 200000 6.88 against 5.40; R-MAT graph of
+// 262144 vertices with 16 / 4 edges each 18.4 against 17.0 and 3.64 against 3.16. Up to 131072 columns the classes win: 131072
+// vertices 6.29 ms before them, 5.43.)
+constexpr int MANY_NT = 128, MANY_ROWS = 8192, MANY_WORDS = 4096;
 
 // Where the word w of a window lies in shared memory. The low bits of a graph's column numbers are far from uniform (in an
 // R-MAT graph each is 0 three times in four, so a quarter of all words would lie in one bank; random look-ups with that skew
@@ -824,33 +829,72 @@ __global__ void __launch_bounds__(256) k_esc_pairs(const int32_t *__restrict__ r
     pairs[p] = make_uint2((uint32_t)ld_nc(col + at), __float_as_uint(ld_nc(val + at)));
 }
 
-// The columns of a window and their ranks, by bitmap words. NARROW: 16 columns in the lower half of a 32-bit word, the
-// number of columns before them in the upper one (a look-up is one 4-byte load: 3 cycles of the shared-memory pipe for
-// random words against 5 for 8 bytes); otherwise 32 columns and their rank in 64 bits.
-template <bool NARROW, bool FOLD>
+// The columns of a window and their ranks, by bitmap words, in one of three forms:
+//   HALVES  16 columns in the lower half of a 32-bit word, the number of columns before them in the upper one (a look-up is one 4-byte
+//           load: 3 cycles of the shared-memory pipe for random words against 5 for 8 bytes); windows of up to 65536 columns
+//   PAIRS   32 columns and their rank in 64 bits
+//   SPLIT   the words, and behind them 16 bits of rank for each: 6 bytes where the others take 8, so that four CTAs instead of three
+//           have room for the widest window on an SM, and half as much to empty; rows of at most 65535 products
+enum Table { HALVES, PAIRS, SPLIT };
+template <Table KIND, bool FOLD>
 struct RankTable {
+    static_assert(KIND != SPLIT || !FOLD, "the words of a split table lie in order");
     unsigned char *at;
+    int words;
+    static __host__ __device__ constexpr size_t bytes(int words) { return (size_t)words * (KIND == SPLIT ? 6 : 8); }
     __device__ __forceinline__ uint32_t &half(uint32_t h) const { return reinterpret_cast<uint32_t *>(at)[FOLD ? h ^ (h >> 5) ^ (h >> 10) : h]; }
     __device__ __forceinline__ uint2 &full(uint32_t w) const { return reinterpret_cast<uint2 *>(at)[spread<FOLD>(w)]; }
-    __device__ __forceinline__ void mark(uint32_t cw) const {  // column cw of the window, in a table of zeros
-        if (NARROW) atomicOr(&half(cw >> 4), 1u << (cw & 15u));
-        else atomicOr(&full(cw >> 5).x, 1u << (cw & 31u));
+    __device__ __forceinline__ uint16_t *ranks() const { return reinterpret_cast<uint16_t *>(at + 4 * (size_t)words); }
+    // Empties what mark() writes into.
+    template <int NT>
+    __device__ __forceinline__ void clear() const {
+        for (int c = threadIdx.x; c < words / (KIND == SPLIT ? 4 : 2); c += NT) reinterpret_cast<uint4 *>(at)[c] = make_uint4(0u, 0u, 0u, 0u);
     }
-    __device__ __forceinline__ uint32_t marked(uint32_t w) const { return NARROW ? half(2 * w) | half(2 * w + 1) << 16 : full(w).x; }
+    __device__ __forceinline__ void mark(uint32_t cw) const {  // column cw of the window
+        if (KIND == HALVES) atomicOr(&half(cw >> 4), 1u << (cw & 15u));
+        else if (KIND == PAIRS) atomicOr(&full(cw >> 5).x, 1u << (cw & 31u));
+        else atomicOr(reinterpret_cast<uint32_t *>(at) + (cw >> 5), 1u << (cw & 31u));
+    }
+    // Word w of a marked table, and the same with `rank` columns before it.
+    __device__ __forceinline__ uint32_t marked(uint32_t w) const { return KIND == HALVES ? half(2 * w) | half(2 * w + 1) << 16 : full(w).x; }
     __device__ __forceinline__ void put(uint32_t w, uint32_t bits, uint32_t rank) const {
-        if (NARROW) {
+        if (KIND == HALVES) {
             half(2 * w) = (bits & 0xffffu) | rank << 16;
             half(2 * w + 1) = bits >> 16 | (rank + __popc(bits & 0xffffu)) << 16;
         } else {
             full(w) = make_uint2(bits, rank);
         }
     }
+    // The words 4 q to 4 q + 3 of a table in order, 16 bytes at a time: the lanes of a warp take neighbouring ones.
+    __device__ __forceinline__ uint4 marked4(uint32_t q) const {
+        const uint4 *from = reinterpret_cast<const uint4 *>(at);
+        if (KIND == SPLIT) return from[q];
+        const uint4 lo = from[2 * q], hi = from[2 * q + 1];
+        return KIND == HALVES ? make_uint4(lo.x | lo.y << 16, lo.z | lo.w << 16, hi.x | hi.y << 16, hi.z | hi.w << 16) : make_uint4(lo.x, lo.z, hi.x, hi.z);
+    }
+    __device__ __forceinline__ void put4(uint32_t q, uint4 v, uint32_t rank) const {
+        const uint32_t r1 = rank + __popc(v.x), r2 = r1 + __popc(v.y), r3 = r2 + __popc(v.z);
+        uint4 *to = reinterpret_cast<uint4 *>(at);
+        if (KIND == SPLIT) {
+            to[q] = v;
+            reinterpret_cast<uint2 *>(ranks())[q] = make_uint2(rank | r1 << 16, r2 | r3 << 16);
+        } else if (KIND == HALVES) {
+            auto lower = [](uint32_t bits, uint32_t r) { return (bits & 0xffffu) | r << 16; };
+            auto upper = [](uint32_t bits, uint32_t r) { return bits >> 16 | (r + __popc(bits & 0xffffu)) << 16; };
+            to[2 * q] = make_uint4(lower(v.x, rank), upper(v.x, rank), lower(v.y, r1), upper(v.y, r1));
+            to[2 * q + 1] = make_uint4(lower(v.z, r2), upper(v.z, r2), lower(v.w, r3), upper(v.w, r3));
+        } else {
+            to[2 * q] = make_uint4(v.x, rank, v.y, r1);
+            to[2 * q + 1] = make_uint4(v.z, r2, v.w, r3);
+        }
+    }
     // columns up to and with cw, which is one of them: its position plus one
     __device__ __forceinline__ uint32_t find(uint32_t cw) const {
-        if (NARROW) {
+        if (KIND == HALVES) {
             const uint32_t e = half(cw >> 4);
             return (e >> 16) + __popc(e << (31u - (cw & 15u)));
         }
+        if (KIND == SPLIT) return (uint32_t)ranks()[cw >> 5] + __popc(reinterpret_cast<const uint32_t *>(at)[cw >> 5] << (~cw & 31u));
         const uint2 e = full(cw >> 5);
         return e.y + __popc(e.x << (~cw & 31u));
     }
@@ -869,17 +913,17 @@ struct RankTable {
 // cycles for the pairs, 3 for the look-up, 3 for noting the column, 10 for the atomic, of 28 to 34 that it takes at 32 to
 // 40 warps per SM. R-MAT graph of 65536 vertices times its transpose (403 M products): both passes of these rows 2.2 ms with entries
 // instead of words in the symbolic one, 5120 sums in shared memory and the others in L2, columns out of the bitmap; 1.5 ms now.
-template <int CLS, bool NARROW, bool PAIRS>
+template <int CLS, Table KIND, bool BY_PAIR>
 __global__ void __launch_bounds__(RANK_CLASS[CLS].nt, RANK_CLASS[CLS].per_sm)
     k_esc_rank(CsrView A, CsrView B, const uint2 *pairs, Windows windows, ListedRows listed, int first, int last, const int2 *list, ClassCtl *ctl, int words,
                int acc_slots, const uint4 *cache, const int32_t *__restrict__ c_rp, int32_t *__restrict__ c_col, float *__restrict__ c_val) {
     constexpr RankClass K = RANK_CLASS[CLS];
     constexpr int NT = K.nt;
     constexpr bool WALKED = K.columns_walked, BY_CLASS = CLS < CLASSES, IN_L2 = K.smem == 0;
-    using Col = typename std::conditional<NARROW, uint16_t, uint32_t>::type;
+    using Col = typename std::conditional<KIND == HALVES, uint16_t, uint32_t>::type;
     extern __shared__ __align__(16) unsigned char rk_smem[];
-    const RankTable<NARROW, K.piece == LONG> table{rk_smem};
-    float *acc = reinterpret_cast<float *>(rk_smem + (size_t)words * 8);
+    const RankTable<KIND, K.piece == LONG> table{rk_smem, words};
+    float *acc = reinterpret_cast<float *>(rk_smem + table.bytes(words));
     int32_t *stage = reinterpret_cast<int32_t *>(acc);
     Col *noted = reinterpret_cast<Col *>(acc + acc_slots);  // WALKED
     __shared__ Segments<NT> seg;
@@ -887,11 +931,10 @@ __global__ void __launch_bounds__(RANK_CLASS[CLS].nt, RANK_CLASS[CLS].per_sm)
     __shared__ int s_next;
     trigger_dependents();
     const int tid = threadIdx.x, count = BY_CLASS ? ctl->count[BY_CLASS ? CLS : 0] : last;
-    const int quads = words / 4, per = quads >= NT ? 4 * ((quads + NT - 1) / NT) : (words + NT - 1) / NT;  // neighbouring words fall to one thread
-    const int w_lo = min(tid * per, words), w_hi = min(w_lo + per, words);
-    const int32_t b_base = PAIRS ? ld_nc(B.rp) : 0;
+    const int quads = words / 4;
+    const int32_t b_base = BY_PAIR ? ld_nc(B.rp) : 0;
     auto load = [&](int q) -> uint2 {
-        return PAIRS ? __ldg(pairs + (q - b_base)) : make_uint2((uint32_t)ld_nc(B.col + q), __float_as_uint(ld_nc(B.val + q)));
+        return BY_PAIR ? __ldg(pairs + (q - b_base)) : make_uint2((uint32_t)ld_nc(B.col + q), __float_as_uint(ld_nc(B.val + q)));
     };
     if (BY_CLASS) {
         if (tid == 0) s_next = atomicAdd(&ctl->ticket[BY_CLASS ? CLS : 0], 1);
@@ -910,43 +953,69 @@ __global__ void __launch_bounds__(RANK_CLASS[CLS].nt, RANK_CLASS[CLS].per_sm)
             const int32_t c_first = w * RK_WINDOW_COLS;  // below 2^31: it is a column of B
             auto range = [&](int32_t j, int32_t &start, int32_t &len) { windows.range(B, j, w, start, len); };
             const uint4 *from = cache ? cache + (size_t)at.y * quads : nullptr;
+            auto write_columns = [&](int c, uint32_t bits, int &rank, int cnt) {  // of word c
+                const int32_t col0 = c_first + c * 32 - 1;
+                if (!IN_L2 && cnt <= acc_slots) {
+                    for (; bits; bits &= bits - 1u) stage[rank++] = col0 + __ffs((int)bits);
+                } else {
+                    for (; bits; bits &= bits - 1u) c_col[out + rank++] = col0 + __ffs((int)bits);
+                }
+            };
             if (!cache) {
-                for (int c = tid; c < words; c += NT) reinterpret_cast<uint2 *>(rk_smem)[c] = make_uint2(0u, 0u);
+                table.template clear<NT>();
                 __syncthreads();
                 const bool any = row.run(A, seg, scan_tmp, true, range, [&](int q) { return ld_nc(B.col + q); },
                                          [&](int32_t col, float) { table.mark((uint32_t)(col - c_first)); });
                 if (!any) continue;  // uniform
             }
-            auto each_word = [&](auto f) {  // f(word, bits) for the thread's words
-                if (!cache) {
-                    for (int c = w_lo; c < w_hi; ++c) f(c, table.marked(c));
-                } else if (quads >= NT) {
-                    for (int c = w_lo; c < w_hi; c += 4) {
-                        const uint4 v = __ldg(from + c / 4);
-                        f(c, v.x), f(c + 1, v.y), f(c + 2, v.z), f(c + 3, v.w);
-                    }
-                } else {
-                    for (int c = w_lo; c < w_hi; ++c) f(c, __ldg(reinterpret_cast<const uint32_t *>(from) + c));
-                }
-            };
-            int mine = 0;
-            each_word([&](int, uint32_t bits) { mine += __popc(bits); });
             int cnt;
-            int rank = block_excl_sum<NT>(mine, scan_tmp, cnt);
-            const bool fits = !IN_L2 && cnt <= acc_slots;
-            each_word([&](int c, uint32_t bits) {
-                table.put(c, bits, rank);
-                if (WALKED) {
-                    rank += __popc(bits);
-                } else {
-                    const int32_t col0 = c_first + c * 32 - 1;
-                    if (fits) {
-                        for (; bits; bits &= bits - 1u) stage[rank++] = col0 + __ffs((int)bits);
+            if constexpr (BY_CLASS) {  // neighbouring words fall to one thread; the fold keeps them off one another's banks
+                const int per = quads >= NT ? 4 * ((quads + NT - 1) / NT) : (words + NT - 1) / NT;
+                const int w_lo = min(tid * per, words), w_hi = min(w_lo + per, words);
+                auto each_word = [&](auto f) {  // f(word, bits) for the thread's words
+                    if (!cache) {
+                        for (int c = w_lo; c < w_hi; ++c) f(c, table.marked(c));
+                    } else if (quads >= NT) {
+                        for (int c = w_lo; c < w_hi; c += 4) {
+                            const uint4 v = __ldg(from + c / 4);
+                            f(c, v.x), f(c + 1, v.y), f(c + 2, v.z), f(c + 3, v.w);
+                        }
                     } else {
-                        for (; bits; bits &= bits - 1u) c_col[out + rank++] = col0 + __ffs((int)bits);
+                        for (int c = w_lo; c < w_hi; ++c) f(c, __ldg(reinterpret_cast<const uint32_t *>(from) + c));
                     }
+                };
+                int mine = 0;
+                each_word([&](int, uint32_t bits) { mine += __popc(bits); });
+                int rank = block_excl_sum<NT>(mine, scan_tmp, cnt);
+                each_word([&](int c, uint32_t bits) {
+                    table.put(c, bits, rank);
+                    if (WALKED) rank += __popc(bits);
+                    else write_columns(c, bits, rank, cnt);
+                });
+            } else {
+                // A warp looks after a run of neighbouring words, four to a lane and step: the loads of a step are one piece of memory,
+                // and its stores meet a bank twice at most. (With a run of words to a thread, as above, those of the widest window lay
+                // 32 to a bank: 2000 rows of 20000 products in 2 M columns 1968 us a call, 1017 like this, 782 with six bytes to a word.)
+                const int share = (quads + NT - 1) / NT * 32;
+                const int q_lo = min(warp_id() * share, quads) + lane_id(), q_hi = min((warp_id() + 1) * share, quads);
+                auto fetch = [&](int q) { return q >= q_hi ? make_uint4(0u, 0u, 0u, 0u) : cache ? __ldg(from + q) : table.marked4(q); };
+                auto columns = [](uint4 v) { return __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w); };
+                const uint4 held = fetch(q_lo);  // the first step's words are not fetched again
+                int mine = columns(held);
+                for (int q = q_lo + 32; q < q_hi; q += 32) mine += columns(fetch(q));
+                int run = __shfl_sync(FULL_MASK, block_excl_sum<NT>(mine, scan_tmp, cnt), 0);  // columns before the step's
+                for (int q = q_lo; q - lane_id() < q_hi; q += 32) {
+                    const uint4 v = q == q_lo ? held : fetch(q);
+                    const int here = columns(v), incl = warp_incl_sum(here);
+                    int rank = run + incl - here;
+                    run += __shfl_sync(FULL_MASK, incl, 31);
+                    if (q >= q_hi) continue;
+                    table.put4(q, v, rank);
+                    write_columns(4 * q, v.x, rank, cnt), write_columns(4 * q + 1, v.y, rank, cnt);
+                    write_columns(4 * q + 2, v.z, rank, cnt), write_columns(4 * q + 3, v.w, rank, cnt);
                 }
-            });
+            }
+            const bool fits = !IN_L2 && cnt <= acc_slots;
             if (!WALKED && !IN_L2) __syncthreads();
             float *row_val = c_val + out;  // the window's part of the row; its length fits 32 bits
             const int in_acc = IN_L2 ? 0 : min(cnt, acc_slots);
@@ -1129,6 +1198,8 @@ struct EscPlan {
     unsigned long long *result;  // result words
 };
 
+bool many_rows(int64_t listed, int words) { return listed >= MANY_ROWS && words <= MANY_WORDS; }
+
 // Another form of B is made for products that read every entry of it this often, and of which there are this many: its words take
 // four short launches (some 25 us with nothing beside them, and 11 per million entries), its pairs one of 9. A graph of 24405 vertices, 49 M
 // products: the whole call 468 -> 357 us with both and the classes; of 9000 vertices, 7 M products, it would take 20 us more. How
@@ -1227,7 +1298,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
     if (listed > 0) {
         // a second pool block: its size is only known now, and the first must not move
         const size_t bitmap_bytes = (size_t)listed * plan->words * 4;
-        const bool many = listed >= MANY_ROWS, carry = carry_bitmaps && plan->n_win == 1 && bitmap_bytes <= BITMAP_CACHE_BUDGET;
+        const bool many = many_rows(listed, plan->words), carry = carry_bitmaps && plan->n_win == 1 && bitmap_bytes <= BITMAP_CACHE_BUDGET;
         auto carve_rows = [&](Carver &c) {
             if (many) plan->class_rows = c.take<int2>((size_t)CLASSES * listed);
             if (carry) plan->cache = c.take<uint4>(bitmap_bytes / 16);
@@ -1313,7 +1384,7 @@ int run_symbolic(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, cu
     const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
     int st;
     const int n_heavy = plan.host.n_rows[BIN_GIANT] + plan.host.n_rows[BIN_HEAVY], n_ranked = plan.host.n_rows[BIN_RANKED];
-    const bool many = n_heavy + n_ranked >= MANY_ROWS;
+    const bool many = many_rows(n_heavy + n_ranked, plan.words);
     if (n_heavy > 0) {  // first: the heaviest rows take longest
         LaunchScope scope("esc_heavy_symbolic", stream);
         auto launch = many ? launch_mark<HEAVY_NT, LONG> : launch_mark<HEAVY_NT, SHORT>;
@@ -1380,7 +1451,9 @@ int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, con
     // A table that leaves no room for sums: no row is of this class, and where rows are not sorted all their sums are in L2.
     const int slots = rank_slots(CLS, plan.words);
     if (CLS < CLASSES && slots == 0) return NB200_OK;
-    const size_t smem = std::max(K.smem, (size_t)plan.words * 8);
+    const bool halves = plan.words <= NARROW_WORDS;
+    constexpr Table WIDE = CLS == FEW ? SPLIT : PAIRS;
+    const size_t smem = std::max(K.smem, halves ? RankTable<HALVES, false>::bytes(plan.words) : RankTable<WIDE, false>::bytes(plan.words));
     int device = 0, ctas = last - first;
     if (CLS < CLASSES) {
         NB200_CUDA(cudaGetDevice(&device));
@@ -1388,10 +1461,9 @@ int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, con
         ctas *= K.per_sm;
     }
     LaunchScope scope(names[CLS], stream);
-    const bool narrow = plan.words <= NARROW_WORDS;
-    auto kernel = narrow ? k_esc_rank<CLS, true, false> : k_esc_rank<CLS, false, false>;
+    auto kernel = halves ? k_esc_rank<CLS, HALVES, false> : k_esc_rank<CLS, WIDE, false>;
     if constexpr (CLS < CLASSES)
-        if (numeric.pairs) kernel = narrow ? k_esc_rank<CLS, true, true> : k_esc_rank<CLS, false, true>;
+        if (numeric.pairs) kernel = halves ? k_esc_rank<CLS, HALVES, true> : k_esc_rank<CLS, WIDE, true>;
     // the most that any call asks for: several threads may be here with different sizes
     NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(K.smem, (size_t)RK_WORDS * 8)));
     if (CLS >= CLASSES) NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, shared_percent(K.per_sm * (smem + FEW_STATIC))));

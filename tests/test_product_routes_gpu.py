@@ -46,6 +46,86 @@ class Block:
         self.struct = CsrStruct(m.rows, m.cols, len(m.col), self.rp.data_ptr(), self.col.data_ptr(), self.val.data_ptr())
 
 
+class Result:
+    def __init__(self, rows):
+        import torch
+        from nacho_b200._capi import CsrStruct
+        self.rp = torch.empty(rows + 1, dtype=torch.int32, device="cuda")
+        self.struct = CsrStruct(0, 0, 0, self.rp.data_ptr(), None, None)
+
+    def take(self, nnz):
+        import torch
+        self.col, self.val = torch.full((nnz,), -1, dtype=torch.int32, device="cuda"), torch.full((nnz,), float("nan"), device="cuda")
+        self.struct.col, self.struct.val, self.struct.nnz = self.col.data_ptr(), self.val.data_ptr(), nnz
+
+    def holds(self, want, v64, abs64):
+        import torch
+        torch.cuda.synchronize()
+        assert np.array_equal(self.rp.cpu().numpy(), want.row_ptr), "row offsets"
+        assert np.array_equal(self.col.cpu().numpy(), want.col), "columns"
+        assert np.all(np.abs(self.val.cpu().numpy().astype(np.float64) - v64) <= REL_TOL * abs64 + 1e-30)
+
+
+def two_passes(oracle, a, b, shift):
+    """The numeric pass on offsets from elsewhere; then both passes, and the numeric one again with other values in A and B."""
+    import torch
+    from nacho_b200._capi import check, lib
+    want, v64, abs64, products = oracle.spgemm(a, b, 8, extras=True)
+    ga, gb = Block(a, shift), Block(b, shift)
+    ref = lambda x: C.byref(x.struct)
+    z = Result(a.rows)
+    z.rp.copy_(torch.from_numpy(want.row_ptr.astype(np.int32)))
+    z.struct.rows, z.struct.cols = a.rows, b.cols
+    z.take(len(want.col))
+    check(lib.nb200_release_workspaces(), "release")
+    check(lib.nb200_spgemm_f32_numeric(ref(ga), ref(gb), ref(z), None), "numeric alone")
+    z.holds(want, v64, abs64)
+    z = Result(a.rows)
+    p = C.c_int64(0)
+    check(lib.nb200_spgemm_f32_symbolic(ref(ga), ref(gb), ref(z), C.byref(p), None), "symbolic")
+    assert p.value == products and z.struct.nnz == len(want.col)
+    z.take(len(want.col))
+    check(lib.nb200_spgemm_f32_numeric(ref(ga), ref(gb), ref(z), None), "numeric")
+    z.holds(want, v64, abs64)
+    ga.val.mul_(2.0)
+    gb.val.mul_(-0.5)
+    z.take(len(want.col))
+    check(lib.nb200_spgemm_f32_numeric(ref(ga), ref(gb), ref(z), None), "numeric again")
+    z.holds(want, -v64, abs64)
+    return products
+
+
+@pytest.mark.parametrize("rows", [300, 8200])
+@pytest.mark.parametrize("cols", [131000, 131073, 262145, 600000])
+def test_wide_results(nacho, oracle, cols, rows):
+    """Windows of 4096 bitmap words and more, one and several of them, for few rows and for many; rows from 260 to 2300 entries, rows of B
+    without entries among those they select."""
+    from test_spgemm_gpu import check
+    rng = np.random.default_rng(cols + rows)
+    inner = 500
+    b = csr_of_rows([scattered(cols, n, rng) for n in rng.choice([0, 40, 130, 500], inner, p=[0.2, 0.4, 0.3, 0.1])], cols, rng)
+    lengths = np.diff(b.row_ptr)
+    long_rows = np.flatnonzero(lengths >= 130)
+    a_rows = [np.unique(np.concatenate([scattered(inner, 3, rng), rng.choice(long_rows, 3, replace=False)])) for _ in range(rows)]
+    a_rows[7] = np.arange(inner)  # every row of B
+    a = csr_of_rows(a_rows, inner, rng)
+    check(nacho, oracle, a, b)
+    two_passes(oracle, a, b, 5)
+
+
+@pytest.mark.parametrize("rows", [600, 8300])
+def test_many_products_in_two_passes(nacho, oracle, rows):
+    """More than 32 M products of a clustered B that is read often: its rows as bitmap words in the symbolic pass, as pairs in the numeric one
+    where there are many rows. B and A begin in the middle of their arrays, and some rows of B are empty."""
+    rng = np.random.default_rng(rows)
+    cols, inner = 50000, 320
+    starts = rng.integers(0, cols - 4000, inner)
+    b = csr_of_rows([np.arange(0) if r % 9 == 4 else np.sort(rng.choice(np.arange(s, s + 4000), 2400, replace=False)) for r, s in enumerate(starts)], cols, rng)
+    per_row = 2 if rows > 8192 else 40
+    a = csr_of_rows([scattered(inner, per_row + (r % 50 == 3), rng) for r in range(rows)], inner, rng)
+    assert two_passes(oracle, a, b, 5) >= 32 << 20
+
+
 def profile(run):
     """The names of the kernels that `run` launches."""
     import torch
