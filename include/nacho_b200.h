@@ -236,8 +236,11 @@ int nb200_csr_add_3_f32_lent(const nb200_csr *a, const nb200_csr *b, const nb200
  * counts are 64-bit (a product count above 2^31 is fine as long as nnz(C) fits int32) and
  * rows with at most 256 products sum equal-column products in a fixed order (ascending j);
  * longer rows accumulate with float32 atomics (as the reference does for every row). No
- * product is written to device memory; scratch is a few int32 per row, plus, for matrices wider
- * than 262144 columns, a pointer table of one int32 per row of B and 262144 columns of width. */
+ * product is written to device memory. Scratch: 24 bytes per row, 8 per entry of A, for matrices wider
+ * than 262144 columns a pointer table of one int32 per row of B and 262144 columns of width; and, where
+ * there is room, a bitmap of the result's columns for every row of more than 256 products (8 GiB at
+ * most), 40 bytes for each of them where there are 8192 and more, and, for more than 32 M products that
+ * read the entries of B 16 to 32 times, 16 bytes and more per entry of B for other forms of it. */
 int nb200_spgemm_f32(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, int32_t num_blocks,
                      int32_t threads_per_block, void *stream);
 /* Two-step form for caller-owned memory: _symbolic fills c->row_ptr (rows + 1, caller-owned)
@@ -260,7 +263,8 @@ int nb200_spgemm_f32_numeric(const nb200_csr *a, const nb200_csr *b, nb200_csr *
  * on the calling thread, hands out two arrays of that many entries that may be used on `stream`, and returns NB200_OK, or
  * a status with which the call then ends. It must not throw, nor call this library on `stream`. c->row_ptr is the
  * caller's; c->col / c->val are set to the arrays in use, of which the first c->nnz entries are. An empty result
- * takes none. Matrices of short rows (at most 8 entries in a row of A and 32 products) are multiplied in one pass into an
+ * takes none. A request refused with NB200_E_NOMEM is made once more if the call holds other forms of B, which it gives back
+ * first. Matrices of short rows (at most 8 entries in a row of A and 32 products) are multiplied in one pass into an
  * entry per product: if `take` refuses that with NB200_E_NOMEM they are counted first, like any others, and if fewer
  * than half of the entries are in use, `take` is called again for nnz(C) entries, to which the result moves (the arrays
  * of the first call are read until the work queued on `stream` is done; a refusal leaves the result where it is).

@@ -42,6 +42,9 @@ struct Workspace {
 // intermediate alive across calls into other drivers takes slot 1 for it.
 int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int slot = 0);
 
+// Gives the device memory of one block back once the work queued on `stream` is done with it. Returns whether there was any.
+bool drop_workspace(cudaStream_t stream, int slot);
+
 // Counts the calls of nb200_release_workspaces(): a Workspace pointer obtained under an earlier
 // value is dangling.
 uint64_t workspace_epoch();

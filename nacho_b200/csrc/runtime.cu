@@ -97,6 +97,20 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
     return NB200_OK;
 }
 
+bool drop_workspace(cudaStream_t stream, int slot) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> g(g_ws_mutex);
+    auto it = g_workspaces.find({{dev, slot}, stream});
+    if (it == g_workspaces.end() || !it->second.dev) return false;
+    Workspace &ws = it->second;
+    ++ws.generation;
+    if (cudaStreamSynchronize(stream) != cudaSuccess || cudaFree(ws.dev) != cudaSuccess) return false;
+    ws.dev = nullptr;
+    ws.dev_bytes = 0;
+    return true;
+}
+
 int wait_result_word(const unsigned long long *word, cudaStream_t stream, int64_t *value, int *device_status) {
     const volatile unsigned long long *w = word;
     unsigned long long v;

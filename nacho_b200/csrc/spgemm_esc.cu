@@ -778,7 +778,7 @@ struct RankClass {
     bool columns_walked;  // the walk of the products notes their columns, in shared memory too (below)
     int piece;
 };
-constexpr int CLASSES = 5, FEW = 5, FEW_HEAVY = 6;  // the last two: where there are few rows they are not sorted by class
+constexpr int CLASSES = 5, FEW = 5, FEW_HEAVY = 6;  // the last two: few rows, or windows too wide, for the rows to be sorted by class
 constexpr RankClass RANK_CLASS[] = {{128, 8, 25 * 1024, true, LONG},  {256, 4, 50 * 1024, true, LONG},    {320, 3, 68 * 1024, true, LONG},   {512, 2, 104 * 1024, true, LONG},
                                     {1024, 1, 208 * 1024, false, LONG}, {256, 5, 0, false, SHORT}, {1024, 1, 208 * 1024, false, SHORT}};
 constexpr int NARROW_WORDS = 2048;  // windows of up to 65536 columns: the table has 16 columns and their rank in 32 bits
@@ -1188,7 +1188,7 @@ struct EscPlan {
     int32_t *win_ptr;      // window pointer table (null: one window, or beyond its budget)
     int words;             // bitmap words of a row in a window
     uint4 *cache;          // bitmaps carried from the symbolic to the numeric pass, heavy rows first (or null)
-    int2 *class_rows;      // rows of every class, as many apart as there are rows above MEDIUM_P products (null: few rows, in one launch)
+    int2 *class_rows;      // rows of every class, as many apart as there are rows above MEDIUM_P products (null: not sorted by class)
     ClassCtl *classes;
     RowWords b_words;      // rows of B as bitmap words for the symbolic pass (or null)
     Workspace *cache_ws;   // pool block of the bitmaps (null without them)
@@ -1207,6 +1207,7 @@ bool many_rows(int64_t listed, int words) { return listed >= MANY_ROWS && words 
 // read 41 times each, 2514 -> 2175 us a call; scattered ones, read 23 to 30 times, cost 4 to 5 % (9000 rows of 6000 products, 130000
 // columns: 493 us with, 470 without).
 constexpr unsigned long long PAIRS_REUSE = 16, WORDS_REUSE = 32, FORMS_FROM = 32 << 20;
+constexpr int WORDS_SLOT = 4, PAIRS_SLOT = 5;  // their pool blocks
 constexpr size_t BITMAP_CACHE_BUDGET = size_t(8) << 30;  // bytes of bitmaps carried between the passes of one call
 
 // Bins the rows (kernel + one read-back) and carves the scratch of a symbolic pass, a numeric
@@ -1320,7 +1321,7 @@ int esc_prepare(const nb200_csr *a, const nb200_csr *b, bool counts, bool carry_
         Carver word_sizes;
         RowWordsScratch::carve(word_sizes, b->rows, b->nnz, &clear_from, &clear_bytes);
         Workspace *word_ws = nullptr;
-        const int word_st = acquire_workspace(stream, word_sizes.used(), &word_ws, 4);
+        const int word_st = acquire_workspace(stream, word_sizes.used(), &word_ws, WORDS_SLOT);
         if (word_st == NB200_OK) {  // without room the entries are walked
             Carver word_carve(word_ws->dev);
             const RowWordsScratch scratch = RowWordsScratch::carve(word_carve, b->rows, b->nnz, &clear_from, &clear_bytes);
@@ -1426,7 +1427,7 @@ int prepare_numeric(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan,
     }
     if (!numeric->classes || plan.host.products < FORMS_FROM || plan.host.products < PAIRS_REUSE * (unsigned long long)b->nnz) return NB200_OK;
     Workspace *ws = nullptr;
-    const int st = acquire_workspace(stream, (size_t)b->nnz * sizeof(uint2), &ws, 5);
+    const int st = acquire_workspace(stream, (size_t)b->nnz * sizeof(uint2), &ws, PAIRS_SLOT);
     if (st != NB200_OK) return st == NB200_E_NOMEM ? NB200_OK : st;  // without room columns and values are loaded apart
     LaunchScope scope("esc_pairs", stream);
     uint2 *pairs = static_cast<uint2 *>(ws->dev);
@@ -1466,7 +1467,8 @@ int launch_rank(const nb200_csr *a, const nb200_csr *b, const EscPlan &plan, con
         if (numeric.pairs) kernel = halves ? k_esc_rank<CLS, HALVES, true> : k_esc_rank<CLS, WIDE, true>;
     // the most that any call asks for: several threads may be here with different sizes
     NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(K.smem, (size_t)RK_WORDS * 8)));
-    if (CLS >= CLASSES) NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, shared_percent(K.per_sm * (smem + FEW_STATIC))));
+    if (CLS >= CLASSES)
+        NB200_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, shared_percent(K.per_sm * (smem + FEW_STATIC))));
     return launch_bin(beside, kernel, ctas, K.nt, smem, stream, CsrView{a->row_ptr, a->col, a->val},
                       CsrView{b->row_ptr, b->col, b->val}, numeric.pairs, Windows{plan.n_win, plan.win_ptr}, listed_rows(plan, a->rows), first, last,
                       CLS < CLASSES ? plan.class_rows + (size_t)CLS * last : nullptr, plan.classes, plan.words, slots, plan.cache, c->row_ptr, c->col, c->val);
@@ -1690,7 +1692,13 @@ int spgemm_with(const nb200_csr *a, const nb200_csr *b, nb200_csr *c, nb200_take
     }
     NumericPlan numeric;
     if ((st = symbolic_on(plan, a, b, c, &numeric, stream)) || c->nnz == 0) return st;
-    if ((st = take(ctx, c->nnz, &c->col, &c->val))) return st;
+    st = take(ctx, c->nnz, &c->col, &c->val);
+    if (st == NB200_E_NOMEM && (plan.b_words.items || numeric.pairs)) {  // the other forms of B are not worth a call's end
+        const bool words = drop_workspace(stream, WORDS_SLOT), pairs = drop_workspace(stream, PAIRS_SLOT);
+        numeric.pairs = nullptr;
+        if (words || pairs) st = take(ctx, c->nnz, &c->col, &c->val);
+    }
+    if (st != NB200_OK) return st;
     return run_numeric(a, b, plan, numeric, c, stream);
 }
 

@@ -126,6 +126,37 @@ def test_many_products_in_two_passes(nacho, oracle, rows):
     assert two_passes(oracle, a, b, 5) >= 32 << 20
 
 
+def test_forms_of_b_give_way_to_the_result(nacho, oracle):
+    """Where the result's arrays are refused while other forms of B are held, the call gives those back and asks again; a second refusal
+    ends it."""
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import TakeFn, lib
+    rng = np.random.default_rng(5)
+    b = csr_of_rows([np.arange(s, s + 2000) for s in rng.integers(0, 30000, 300)], 32000, rng)
+    a = csr_of_rows([scattered(300, 2, rng) for _ in range(8400)], 300, rng)
+    want, v64, abs64, products = oracle.spgemm(a, b, 8, extras=True)
+    assert products >= 32 << 20
+    ga, gb = Block(a, 0), Block(b, 0)
+    for refusals in (1, 2):
+        z, free = Result(a.rows), []
+
+        def take(ctx, entries, p_col, p_val):
+            free.append(torch.cuda.mem_get_info()[0])
+            if len(free) <= refusals:
+                return _capi.E_NOMEM
+            z.take(entries)
+            p_col[0], p_val[0] = z.col.data_ptr(), z.val.data_ptr()
+            return _capi.OK
+
+        status = lib.nb200_spgemm_f32_with(C.byref(ga.struct), C.byref(gb.struct), C.byref(z.struct), TakeFn(take), None, None)
+        torch.cuda.synchronize()
+        assert len(free) == 2 and free[1] >= free[0] + 16 * len(b.col)
+        assert status == (_capi.E_NOMEM if refusals == 2 else _capi.OK)
+        if refusals == 1:
+            z.holds(want, v64, abs64)
+
+
 def profile(run):
     """The names of the kernels that `run` launches."""
     import torch
