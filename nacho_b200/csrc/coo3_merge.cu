@@ -12,8 +12,8 @@
 // compare of the reference for any extents.
 //
 // Kernels: k_coo3_partition (tile cuts) and k_coo3_tile (one CTA per tile: stage and pack the coordinates,
-// split by merge-path, merge VT entries per thread, rank survivors, obtain the output base -- single pass
-// with the cross-tile scan, or from the scanned counts of a first pass -- fetch values, store coalesced).
+// bring the values in their place, split by merge-path, merge VT entries per thread, rank survivors, obtain the output base -- single pass
+// with the cross-tile scan, or from the scanned counts of a first pass -- store coalesced).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -155,8 +155,7 @@ __device__ __forceinline__ void coo3_reduce_done(FusedCtl *ctl, const Coo3Out &Z
 // Shared-memory plan of the tile body, in 4-byte words: three raw arrays (i, j, k), in which A's entry e sits
 // at word oa + e and B's at word ob + e, chosen so that 16-byte boundaries of global memory fall on 16-byte
 // boundaries here (what a bulk copy needs). Every entry's coordinates are packed in place: the key takes the
-// place of i (and, for 64-bit keys, of j), and the 16-bit source indices of the result take the place of an
-// array that is no longer needed.
+// place of i (and, for 64-bit keys, of j), and the 16-bit source indices of the result take the place of j (of k).
 template <int VT>
 struct Coo3Plan {
     static constexpr int CAP = NT * VT;
@@ -176,17 +175,56 @@ struct Coo3Shared {
     double partial[NT / 32];
 };
 
+// x << s, nothing where s is 32 or more.
+__device__ __forceinline__ uint32_t shl32(uint32_t x, int s) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(s));
+    return r;
+}
+
+// Brings the tile's values into shared memory, entry e of A to word oa + e of `to` and B's to ob + e: aligned interiors by bulk
+// copy on the second phase of the tile's mbarrier, ragged ends, and arrays whose alignment differs, by plain loads. Called by all threads after
+// a barrier behind the last use of the words.
+__device__ __forceinline__ void coo3_stage_values(const float *a_val, const float *b_val, const int na, const int nb, const int oa, const int ob, uint32_t *to,
+                                                  Coo3Shared &sh) {
+    const int tid = threadIdx.x;
+    const float *const src[2] = {a_val, b_val};
+    const int count[2] = {na, nb}, at[2] = {oa, ob};
+    int head[2], nv[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        head[q] = min(count[q], head_elems(src[q]));
+        nv[q] = ((at[q] + head[q]) & 3) == 0 ? (count[q] - head[q]) >> 2 : 0;
+    }
+    if (tid == 0) {
+        fence_async_shared();  // the words were read and written by the threads so far
+        mbar_arrive_expect_tx(&sh.mbar, 16u * (uint32_t)(nv[0] + nv[1]));
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (nv[q]) bulk_load(to + at[q] + head[q], src[q] + head[q], 16u * nv[q], &sh.mbar);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        // the ends of q: a warp each; nothing but ends where no vector is copied
+        if (nv[q] == 0) {
+            for (int e = tid; e < count[q]; e += NT) to[at[q] + e] = __float_as_uint(__ldg(src[q] + e));
+        } else if ((tid >> 5) == 1 + q && (tid & 31) < 6) {
+            const int e = tid & 31, idx = e < 3 ? e : head[q] + 4 * nv[q] + (e - 3);
+            if (e < 3 ? e < head[q] : idx < count[q]) to[at[q] + idx] = __float_as_uint(__ldg(src[q] + idx));
+        }
+    }
+}
+
 // One tile. NARROW: the keys of the tile, counted from its smallest, fit 32 bits (true of nearly every tile of
 // a tensor of millions of entries); otherwise they are kept as a low and a high word.
 //
-// The structure is that of the CSR tile kernel (csr_merge.cu), without rows: coordinates alone are staged and
-// merged, one result entry per step; a 16-bit source index per result entry is compacted; the count goes out
-// before the values are fetched from L2, where a prefetch has brought them. REDUCE (inner product): only
-// the coordinates both operands hold are kept, and their products summed.
+// The structure is that of the CSR tile kernel (csr_merge.cu), without rows: one result entry per step of a sequential merge; a 16-bit
+// source index per result entry is compacted. REDUCE (inner product): only the products of the coordinates that both operands hold are summed.
 //
-// Bound by instruction issue and the latency of a tile's barrier-separated phases, at a bit over half of the copy
-// rate; 100 M entries per operand: 1550 us with staged values, 64-bit keys in a serial merge of 11 entries per
-// thread and a look-back per tile, 1195 us in this form.
+// Bound by instruction issue (0.65 of the slots where this was counted) and the latency of a tile's barrier-separated phases beside HBM. 32-bit keys
+// leave the words of k free: the values are copied there during the merge, the sum of a twin is made in place by the thread that merged it, and
+// results are fetched from shared memory alone, without a test or an address per entry. 100 M entries per operand: values gathered from L2 and a
+// test for twins per result 1208 us a call, this 1098; inner product of 4 M 58.4 -> 54.8.
 template <int VT, int MODE, bool NARROW>
 __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, const Packing &pk, const int32_t a0, const int32_t b0, const int na,
                                           const int nb, const int oa, const int ob, const uint64_t key0, const int t, const int num_tiles,
@@ -196,7 +234,9 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     using Key = typename std::conditional<NARROW, uint32_t, uint64_t>::type;
     constexpr Key END = (Key)~(Key)0;
     constexpr bool REDUCE = MODE == MODE_REDUCE;
-    constexpr uint32_t HIGH = 4 * P::SLOTS;  // byte distance from a key's low to its high word
+    constexpr bool STAGED = NARROW && MODE != MODE_COUNT;  // values in shared memory (64-bit keys leave no room for them)
+    constexpr uint32_t HIGH = 4 * P::SLOTS;   // byte distance from a key's low to its high word
+    constexpr uint32_t VALUE = 8 * P::SLOTS;  // ... from a 32-bit key to its entry's value
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = na + nb;
     uint32_t *raw = reinterpret_cast<uint32_t *>(smem_raw);
     uint16_t *src_of = reinterpret_cast<uint16_t *>(raw + (NARROW ? 1 : 2) * P::SLOTS);
@@ -205,23 +245,36 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         return NARROW ? (Key)word_at(byte) : (Key)((uint64_t)word_at(byte + HIGH) << 32 | word_at(byte));
     };
 
-    // ---- pack
+    // ---- pack, four staged words at a time, whatever they hold: padding packs to something that nobody reads, and the words
+    // behind each operand become its sentinel.
+    {
+        uint4 *w4 = reinterpret_cast<uint4 *>(smem_raw);
+        constexpr int S4 = P::SLOTS / 4;
+        const int end_a = oa + na, end_b = ob + nb;
+        for (int v = tid; 4 * v <= end_b; v += NT) {
+            const uint4 i4 = w4[v], j4 = w4[S4 + v], k4 = w4[2 * S4 + v];
+            if (NARROW) {  // the low words of the packed coordinates are enough
+                auto low = [&](uint32_t i, uint32_t j, uint32_t k) { return (shl32(i, pk.bj + pk.bk) | shl32(j, pk.bk) | k) - (uint32_t)key0; };
+                w4[v] = make_uint4(low(i4.x, j4.x, k4.x), low(i4.y, j4.y, k4.y), low(i4.z, j4.z, k4.z), low(i4.w, j4.w, k4.w));
+            } else {
+                auto full = [&](uint32_t i, uint32_t j, uint32_t k) { return pk.pack((int32_t)i, (int32_t)j, (int32_t)k) - key0; };
+                const uint64_t a = full(i4.x, j4.x, k4.x), b = full(i4.y, j4.y, k4.y), c = full(i4.z, j4.z, k4.z), d = full(i4.w, j4.w, k4.w);
+                w4[v] = make_uint4((uint32_t)a, (uint32_t)b, (uint32_t)c, (uint32_t)d);
+                w4[S4 + v] = make_uint4((uint32_t)(a >> 32), (uint32_t)(b >> 32), (uint32_t)(c >> 32), (uint32_t)(d >> 32));
+            }
+            if (end_a >> 2 == v || end_b >> 2 == v) {
 #pragma unroll
-    for (int q = 0; q < VT; ++q) {
-        const int e = tid + q * NT;  // A's entries first, then B's
-        const int w = e < na ? oa + e : ob + (e - na);
-        if (e < n) {
-            const uint64_t key = pk.pack((int32_t)raw[w], (int32_t)raw[P::SLOTS + w], (int32_t)raw[2 * P::SLOTS + w]) - key0;
-            raw[w] = (uint32_t)key;
-            if (!NARROW) raw[P::SLOTS + w] = (uint32_t)(key >> 32);
+                for (int c = 0; c < 4; ++c)
+                    if (4 * v + c == end_a || 4 * v + c == end_b) {
+                        raw[4 * v + c] = 0xffffffffu;
+                        if (!NARROW) raw[P::SLOTS + 4 * v + c] = 0xffffffffu;
+                    }
+            }
         }
     }
-    if (tid < 2) {
-        const int w = tid == 0 ? oa + na : ob + nb;
-        raw[w] = 0xffffffffu;
-        if (!NARROW) raw[P::SLOTS + w] = 0xffffffffu;
-    }
     __syncthreads();
+    // ---- the values take the place of the k coordinates; they land during the merge
+    if (STAGED) coo3_stage_values(A.val + a0, B.val + b0, na, nb, oa, ob, raw + 2 * P::SLOTS, sh);
 
     // ---- where this thread's share begins: merge-path diagonal tid * VT (ties take A first; a coordinate that
     // both operands hold stays on one side)
@@ -280,56 +333,35 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         twin &= (1u << steps) - 1u;
     }
 
-    // ---- rank the survivors inside the tile
-    const int mine = REDUCE ? __popc(twin) : steps;
-    const int incl = warp_incl_sum(mine);
-    if (lane == 31) sh.wtotal[wid] = incl;
-    __syncthreads();  // also retires the merge of every thread: words of consumed twins may change from here on
-    int total = 0, wbase = 0;
-#pragma unroll
-    for (int w = 0; w < NT / 32; ++w) {
-        const int c = sh.wtotal[w];
-        wbase += w < wid ? c : 0;
-        total += c;
-    }
-    const int rank = wbase + incl - mine;
-    if (MODE == MODE_COUNT) {
-        if (tid == 0) tile_count[t] = total;
-        return;
-    }
-    if (MODE == MODE_FUSED && tid == 0) publish_count(words, t, total);
-
-    // ---- compact. A twin's A word now points to its B word (step i began at pa0 + pb0 + 4 (i + twins before it)).
-    if (__any_sync(FULL_MASK, twin != 0u)) {
-#pragma unroll
-        for (int i = 0; i < VT; ++i)
-            if ((twin >> i) & 1u) {
-                word_at(src[i]) = pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - src[i];
-                src[i] |= 0x8000u;
-            }
-    }
-    {
-        uint16_t *to = src_of + rank;
-#pragma unroll
-        for (int i = 0; i < VT; ++i) {
-            if (!REDUCE) {
-                if (i < steps) to[i] = (uint16_t)src[i];
-            } else if ((twin >> i) & 1u) {
-                *to++ = (uint16_t)src[i];
-            }
-        }
-    }
-    __syncthreads();
-
+    // byte offset of the B word of the twin at step i, whose A word is `at` (step i began at pa0 + pb0 + 4 (i + twins before it))
+    auto partner = [&](int i, uint32_t at) { return pa0 + pb0 + 4u * (uint32_t)(i + __popc(twin & ((1u << i) - 1u))) - at; };
+    auto report_copy = [&]() {
+        if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
+        __threadfence();
+    };
     const char *va = reinterpret_cast<const char *>(A.val + a0) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(B.val + b0) - 4 * (int64_t)ob;
+
     if (REDUCE) {
         // ---- inner product: products in float32 as the reference's, summed in double; one atomic per tile into
         // the control block (the order of the tiles' sums is not fixed, as with the reference's atomic
-        // accumulation, src/backend/compute.cpp:498-525)
+        // accumulation, src/backend/compute.cpp:498-525). A thread notes its twins in a part of its own of the source indices.
+        uint16_t *own = src_of + tid * VT, *to = own;
+#pragma unroll
+        for (int i = 0; i < VT; ++i)
+            if ((twin >> i) & 1u) *to++ = (uint16_t)src[i];
+        const bool landed = !STAGED || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
+        if (!__syncthreads_and(landed)) {
+            if (tid == 0) {
+                report_copy();
+                mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
+            }
+            return;
+        }
         double sum = 0.0;
-        for (int o = tid; o < total; o += NT) {
-            const uint32_t at = src_of[o] & 0x7fffu;
-            sum += (double)(__ldg(reinterpret_cast<const float *>(va + at)) * __ldg(reinterpret_cast<const float *>(vb + word_at(at))));
+        for (unsigned left = twin; left; left &= left - 1u) {
+            const uint32_t at = *own++, other = partner(__ffs(left) - 1, at);
+            if (STAGED) sum += (double)(__uint_as_float(word_at(at + VALUE)) * __uint_as_float(word_at(other + VALUE)));
+            else sum += (double)(__ldg(reinterpret_cast<const float *>(va + at)) * __ldg(reinterpret_cast<const float *>(vb + other)));
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL_MASK, sum, o);
@@ -343,24 +375,68 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         return;
     }
 
-    // ---- fetch coordinates and values, result entries q * NT + tid, the first round before the output base is asked for. Every round is a
-    // trip to L2 (17 entries in rounds of 8, 9, 17: 549, 547, 527 us at 41 M entries per operand, 1198, 1193, 1185 at 100 M); 64-bit keys
-    // would not fit the registers all at once, nor does a fill behind a count (56 bytes of spills).
-    constexpr int GATHER = NARROW && MODE != MODE_FILL ? VT : 8;
+    // ---- rank the survivors inside the tile
+    const int incl = warp_incl_sum(steps);
+    if (lane == 31) sh.wtotal[wid] = incl;
+    const bool landed = !STAGED || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
+    if (!__syncthreads_and(landed)) {  // the values did not land in time: report, touch nothing
+        if (tid == 0) {
+            report_copy();
+            if (MODE == MODE_FUSED) {
+                publish_count(words, t, 0);  // successors must not wait on this tile
+                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+            }
+            mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
+        }
+        return;
+    }
+    int total = 0, wbase = 0;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) {
+        const int c = sh.wtotal[w];
+        wbase += w < wid ? c : 0;
+        total += c;
+    }
+    const int rank = wbase + incl - steps;
+    if (MODE == MODE_COUNT) {
+        if (tid == 0) tile_count[t] = total;
+        return;
+    }
+    if (MODE == MODE_FUSED && tid == 0) publish_count(words, t, total);
+
+    // ---- compact; the value of a twin's A entry becomes the sum (64-bit keys: its A word now points to its B word)
+    {
+        uint16_t *to = src_of + rank;
+#pragma unroll
+        for (int i = 0; i < VT; ++i)
+            if (i < steps) to[i] = (uint16_t)src[i];
+        for (unsigned left = twin; left; left &= left - 1u) {
+            const int i = __ffs(left) - 1;
+            const uint32_t at = to[i], other = partner(i, at);
+            if (STAGED) {
+                word_at(at + VALUE) = __float_as_uint(__uint_as_float(word_at(at + VALUE)) + __uint_as_float(word_at(other + VALUE)));
+            } else {
+                word_at(at) = other;
+                to[i] = (uint16_t)(at | 0x8000u);
+            }
+        }
+    }
+
+    auto live = [&](int q) { return q < VT && q * NT + tid < total; };
     const uint32_t first_b = 4u * (uint32_t)ob;
+    constexpr int GATHER = STAGED ? VT : 8;
     Key key[GATHER];
     float val[GATHER];
-    auto live = [&](int q) { return q < VT && q * NT + tid < total; };
     auto gather = [&](const int q0) {
-        uint32_t s[GATHER], any = 0;
+        uint32_t s[GATHER];
+#pragma unroll
+        for (int g = 0; g < GATHER; ++g) s[g] = live(q0 + g) ? (uint32_t)src_of[(q0 + g) * NT + tid] : 4u * (uint32_t)oa;
 #pragma unroll
         for (int g = 0; g < GATHER; ++g) {
-            s[g] = live(q0 + g) ? (uint32_t)src_of[(q0 + g) * NT + tid] : 4u * (uint32_t)oa;
-            any |= s[g];
-        }
-        if (__any_sync(FULL_MASK, (any & 0x8000u) != 0u)) {
-#pragma unroll
-            for (int g = 0; g < GATHER; ++g) {
+            if (STAGED) {
+                key[g] = key_at_byte(s[g]);
+                val[g] = __uint_as_float(word_at(s[g] + VALUE));
+            } else {
                 const bool both = (s[g] & 0x8000u) != 0u;
                 const uint32_t at = s[g] & 0x7fffu, other = both ? word_at(at) : at;
                 key[g] = key_at_byte(other);
@@ -369,14 +445,9 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
                 if (both) v = v + __ldg(reinterpret_cast<const float *>(vb + other));
                 val[g] = v;
             }
-        } else {
-#pragma unroll
-            for (int g = 0; g < GATHER; ++g) {
-                key[g] = key_at_byte(s[g]);
-                val[g] = live(q0 + g) ? __ldg(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
-            }
         }
     };
+    __syncthreads();
     gather(0);
 
     // ---- output base of the tile
@@ -392,6 +463,8 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     if (base < 0) return;  // a bounded wait gave up; the host reports it
 
     // ---- unpack and store, coalesced
+    int32_t *zi = Z.i + base + tid, *zj = Z.j + base + tid, *zk = Z.k + base + tid;
+    float *zv = Z.val + base + tid;
 #pragma unroll
     for (int q0 = 0; q0 < VT; q0 += GATHER) {
         if (q0 > 0) {
@@ -401,12 +474,11 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 #pragma unroll
         for (int g = 0; g < GATHER; ++g) {
             if (live(q0 + g)) {
-                const long long o = base + (q0 + g) * NT + tid;
                 const uint64_t full = key0 + key[g];
-                Z.i[o] = pk.i_of(full);
-                Z.j[o] = pk.j_of(full);
-                Z.k[o] = pk.k_of(full);
-                Z.val[o] = val[g];
+                zi[(q0 + g) * NT] = pk.i_of(full);
+                zj[(q0 + g) * NT] = pk.j_of(full);
+                zk[(q0 + g) * NT] = pk.k_of(full);
+                zv[(q0 + g) * NT] = val[g];
             }
         }
     }
@@ -474,7 +546,7 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
                 const int nv = q < 3 ? nva : nvb, head = q < 3 ? head_a : head_b;
                 if (bulk[q] && nv) bulk_load(raw + (q % 3) * P::SLOTS + (q < 3 ? oa : ob) + head, src[q] + head, 16u * nv, &sh.mbar);
             }
-            if (MODE == MODE_FUSED || MODE == MODE_FILL) {
+            if (MODE != MODE_COUNT) {
                 prefetch_l2(A.val + a0, na);
                 prefetch_l2(B.val + b0, nb);
             }

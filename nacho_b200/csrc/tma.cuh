@@ -24,6 +24,9 @@ __device__ __forceinline__ void mbar_fence_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// Orders the shared-memory accesses of this thread, and of those it has met at a barrier, before copies that it starts from here on.
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // One arrival that also announces `bytes` of copy traffic the barrier must see before the
 // current phase completes.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t bytes) {

@@ -106,6 +106,33 @@ def test_coordinate_tiles(nacho, oracle, total, dims):
     assert abs(got - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30  # float32 products, 2^-24 each, summed wider
 
 
+@pytest.mark.parametrize("total", [9, COO_STEP - 2, 2 * COO_STEP + 5, 3_000_011])
+@pytest.mark.parametrize("shift", [(0, 1), (1, 0), (2, 3)])
+def test_coordinate_values_off_alignment(nacho, oracle, total, shift):
+    """Values whose place in memory sits differently on 16-byte boundaries than their coordinates': no bulk copy can bring them to the
+    coordinates' words."""
+    import torch
+    dims = (1000, 800, 600)
+    rng = np.random.default_rng(total)
+    ka, kb = key_pair(total, dims[0] * dims[1] * dims[2], 0.3, rng)
+
+    def moved(x, by):
+        t = torch.empty(len(x) + by, dtype=torch.from_numpy(x).dtype, device="cuda")[by:]
+        return t.copy_(torch.from_numpy(x))
+
+    def tensors(key, by):
+        t = COO3(dims, (key // 480000).astype(np.int32), (key // 600 % 800).astype(np.int32), (key % 600).astype(np.int32),
+                 rng.uniform(-1, 1, len(key)).astype(np.float32))
+        return t, nacho.COO3_gpu(*(moved(x, by[0]) for x in (t.i, t.j, t.k)), moved(t.val, by[1]), torch.tensor(dims, dtype=torch.int32))
+
+    from test_tensor3_gpu import coo3_from_gpu
+    (a, ga), (b, gb) = tensors(ka, shift), tensors(kb, shift[::-1])
+    assert_same(coo3_from_gpu(nacho.gpu_coo3d_add_f32(ga, gb)), oracle.coo3_add(a, b, 8), "coo3 add")
+    _, at_a, at_b = np.intersect1d(ka, kb, assume_unique=True, return_indices=True)
+    terms = a.val[at_a].astype(np.float64) * b.val[at_b]
+    assert abs(float(nacho.gpu_inner_prod_coo_f32(ga, gb).values.cpu()[0]) - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30
+
+
 def test_stored_empty_rows_and_fibres(nacho, oracle):
     """Row lists that hold rows without entries, and trees that hold slices and fibres without any, come out without them."""
     from test_family_gpu import dcsr_from_gpu, dcsr_to_gpu
