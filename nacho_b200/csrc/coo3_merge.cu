@@ -349,7 +349,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) *to++ = (uint16_t)src[i];
-        const bool landed = !STAGED || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
+        const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
         if (!__syncthreads_and(landed)) {
             if (tid == 0) {
                 report_copy();
@@ -378,7 +378,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     // ---- rank the survivors inside the tile
     const int incl = warp_incl_sum(steps);
     if (lane == 31) sh.wtotal[wid] = incl;
-    const bool landed = !STAGED || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
+    const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
     if (!__syncthreads_and(landed)) {  // the values did not land in time: report, touch nothing
         if (tid == 0) {
             report_copy();
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
             if (!bulk[q])
                 for (int e = tid; e < (q < 3 ? na : nb); e += NT) raw[(q % 3) * P::SLOTS + (q < 3 ? oa : ob) + e] = (uint32_t)ld_nc(src[q] + e);
     }
-    const bool landed = mbar_wait_bounded(&sh.mbar, 0, MBAR_POLL_LIMIT);
+    const bool landed = tid >= 32 || mbar_wait_bounded(&sh.mbar, 0, MBAR_POLL_LIMIT);  // one warp polls; the others' issue slots are worth more
     if (!__syncthreads_and(landed)) {  // the copies did not land in time: report, touch nothing
         if (tid == 0) {
             if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;

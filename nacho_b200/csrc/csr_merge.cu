@@ -4,12 +4,13 @@
 // The merged sequence of all stored entries of A and B, ordered by (row, column) with A first
 // on ties, is cut into tiles of a few thousand entries. A partition kernel finds every cut with
 // k-ary searches (rows on the summed row offsets, then the merge-path diagonal inside the row).
-// One CTA then owns one tile: the copy engine stages the tile's columns in shared memory (the values stay where they
-// are, prefetched into L2), every row that begins in the tile adds one to the upper bits of its first column (so a
+// One CTA then owns one tile: the copy engine stages the tile's columns in shared memory (the values are
+// prefetched into L2 meanwhile), every row that begins in the tile adds one to the upper bits of its first column (so a
 // key of the next entry is "row of the entry before it + this word"), every thread finds where its
 // share of the merged sequence begins with two searches in shared memory, and merges the columns of its entries
-// one result after the other, noting where each comes from. The tile's count goes out; then columns and values of the
-// results are fetched by those notes, in order, and written back coalesced. Row offsets of the result are produced by
+// one result after the other, noting where each comes from. The tile's count goes out; the columns of the results are taken into
+// registers by those notes, in order, and for a sum the values then take the place of the columns in shared memory; both are written
+// back coalesced. Row offsets of the result are produced by
 // the same pass: a tile owns the offsets of the rows that begin inside it.
 //
 // Reference behaviour restated (not its code): partition src/backend/partition.cpp:813-993
@@ -192,8 +193,12 @@ struct TileShared {
 //   - the merge is sequential and moves columns only: one compare and at most two loads per result entry
 //     (a key-building pass, a register merge network and a per-entry value gather took four times the
 //     instructions), and it leaves a 16-bit source index per result entry;
-//   - the tile's count goes out right after it, and the values are fetched (from L2, where a prefetch has
-//     brought them meanwhile) while the count travels;
+//   - the tile's count goes out right after it; a sum's results take their columns into registers, which frees the words for a
+//     second copy, of the values, while the count travels. One wait covers both, and no thread fetches a value from L2 with an
+//     address of its own: gathering values in four batches behind the base took 17 instructions and 2 trips to L2 more per eight results
+//     (67 M entries 446 -> 410 us a call, 16 M in rows of 16 172 -> 138, three operands of 9 M 239 -> 194, a tree of 25 M 359 -> 323);
+//   - an intersection keeps the gather: its results are few, and most values would be copied for nothing. What follows from a twin is done in a
+//     loop over a thread's twins, not as a test per step (16 M entries, half of them shared: 122 -> 114 us);
 //   - a tile needs 6 bytes of shared memory per entry instead of 16: 55 KB with 31 entries per thread, so four CTAs share an SM.
 template <int VT, int OP, int MODE, bool LEVELS, bool WIDE>
 __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const TileRange &tile, const int cbits, const int t,
@@ -293,7 +298,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
         if (rows_fit) return s_rows[r];
         return r == 0 ? 0u : r > nr ? (uint32_t)na | (uint32_t)nb << 16 : global_start(r);
     };
-    const bool landed = mbar_wait_bounded(mbar, 0, MBAR_POLL_LIMIT);
+    const bool landed = wid > 0 || mbar_wait_bounded(mbar, 0, MBAR_POLL_LIMIT);  // one warp polls; the others' issue slots are worth more
     if (!__syncthreads_and(landed)) {  // the copies did not land in time: report, touch nothing
         if (tid == 0) {
             if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
@@ -486,18 +491,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     };
     if (last && wid == 0) ask_base();
 
-    // ---- compact: source of every result entry, in order. A twin's A word now points to its B word
-    // (byte offsets: step i began at pa0 + pb0 + 4 (i + twins before it)).
-    if (!LEVELS && __any_sync(FULL_MASK, twin != 0u)) {
-        uint32_t begun = pa0 + pb0;  // where step i began, less 4 i
-#pragma unroll
-        for (int i = 0; i < VT; ++i)
-            if ((twin >> i) & 1u) {
-                word_at(src[i]) = begun + 4u * (uint32_t)i - src[i];
-                src[i] |= 0x8000u;
-                begun += 4u;
-            }
-    }
+    // ---- compact: source of every result entry, in order
     if (MANY_ROWS) {
         // The row offsets ask how many of a thread's first m entries are a twin's second: bit e for its entry e
         unsigned second = 0;
@@ -515,62 +509,17 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             }
         }
     }
-    __syncthreads();
-
-    // ---- fetch columns and values, result entries q * NT + tid; the first batch before the output base is
-    // asked for
-    const char *va = reinterpret_cast<const char *>(ga_val) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(gb_val) - 4 * (int64_t)ob;
-    const uint32_t first_b = 4u * (uint32_t)ob;
-    // Result entries a thread fetches together. A round is a trip to L2, so the smaller tiles take one or two. In the large
-    // tile, bound by throughput, 8 are better than 11 or 16 (67 M entries 449, 465, 483 us); intersections leave fewer, and a fill behind a
-    // count has no registers for more.
-    constexpr int GATHER = OP == OP_INTERSECT || VT == V_MOST || MODE == MODE_FILL ? 8 : VT <= 16 ? VT : (VT + 1) / 2;
-    uint32_t col[GATHER];
-    float val[GATHER];
-    auto gather = [&](const int q0) {
-        uint32_t s[GATHER];
-        uint32_t any = 0;
-#pragma unroll
-        for (int g = 0; g < GATHER; ++g) {
-            const int o = (q0 + g) * NT + tid;
-            s[g] = q0 + g < VT && o < total ? (uint32_t)src_of[o] : 4u * (uint32_t)oa;  // spare slots read A's first word (or its sentinel)
-            any |= s[g];
-        }
-        if (OP == OP_INTERSECT || __any_sync(FULL_MASK, (any & 0x8000u) != 0u)) {
-#pragma unroll
-            for (int g = 0; g < GATHER; ++g) {
-                const bool both = (s[g] & 0x8000u) != 0u;
-                const uint32_t at = s[g] & 0x7fffu;
-                const uint32_t w = word_at(at);
-                const uint32_t other = both ? w : at;
-                col[g] = word_at(other) & cmask;
-                const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
-                float v = 0.0f;
-                if (ok) v = ld_late(reinterpret_cast<const float *>((at >= first_b ? vb : va) + at));
-                if (both) {
-                    const float u = ld_late(reinterpret_cast<const float *>(vb + other));
-                    v = OP == OP_UNION ? v + u : v * u;
-                }
-                val[g] = v;
-            }
-        } else {
-#pragma unroll
-            for (int g = 0; g < GATHER; ++g) {
-                const bool ok = q0 + g < VT && (q0 + g) * NT + tid < total;
-                col[g] = word_at(s[g]) & cmask;
-                val[g] = ok ? ld_late(reinterpret_cast<const float *>((s[g] >= first_b ? vb : va) + s[g])) : 0.0f;
-            }
-        }
-    };
-    if (!LEVELS) gather(0);
-
-    // ---- output base of the tile
-    if (MODE == MODE_FUSED && !last && wid == 0) ask_base();
-    __syncthreads();
-    const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
-    if (base < 0) return;  // a bounded wait gave up; the host reports it
+    // Byte offset of the B word of the k-th of this thread's twins, taken by step i, whose A word is `at`: step i began at
+    // pa0 + pb0 + 4 (i + twins before it).
+    const uint32_t begun = pa0 + pb0;
+    auto partner = [&](const int i, const int k, const uint32_t at) { return begun + 4u * (uint32_t)(i + k) - at; };
 
     if (LEVELS) {
+        __syncthreads();
+        if (MODE == MODE_FUSED && !last && wid == 0) ask_base();
+        __syncthreads();
+        const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
+        if (base < 0) return;  // a bounded wait gave up; the host reports it
         // ---- offsets mode: the column and the two range starts of every result entry
         constexpr int LB = 4;  // result entries a thread fetches together
         const int32_t *from_a = L.a + (tile.a0 - oa), *from_b = L.b + (tile.b0 - ob);
@@ -600,31 +549,130 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
             L.off_a[base + total] = ld_late(L.a + tile.a0 + na);
             L.off_b[base + total] = ld_late(L.b + tile.b0 + nb);
         }
-    } else {
-    // ---- store the tile, coalesced
-    int32_t *gz_col = Z.col + base + tid;
-    float *gz_val = Z.val + base + tid;
+        if (!Z.rp) return;
+    }
+    const char *va = reinterpret_cast<const char *>(ga_val) - 4 * (int64_t)oa, *vb = reinterpret_cast<const char *>(gb_val) - 4 * (int64_t)ob;
+    auto live = [&](const int q) { return q < VT && q * NT + tid < total; };
+    if (!LEVELS && OP == OP_UNION) {
+        __syncthreads();
+        // ---- the columns of the results, q * NT + tid, into registers: then the words are free for the values
+        uint32_t col[VT];
 #pragma unroll
-    for (int q0 = 0; q0 < VT; q0 += GATHER) {
-        if (q0 > 0) {
-            if (q0 * NT >= total) break;
-            gather(q0);
+        for (int q = 0; q < VT; ++q) col[q] = live(q) ? word_at(src_of[q * NT + tid]) & cmask : 0u;
+        __syncthreads();
+        // ---- bring the values to the places of their columns, and ask for the output base meanwhile
+        const bool same_a = head_elems(ga_val) == ha, same_b = head_elems(gb_val) == hb;
+        if (tid == 0) {
+            fence_async_shared();  // the words were read and written by the threads so far
+            mbar_arrive_expect_tx(mbar, 16u * (uint32_t)((same_a ? nva : 0) + (same_b ? nvb : 0)));
+            if (same_a && nva) bulk_load(keys + oa + head_a, ga_val + head_a, 16u * nva, mbar);
+            if (same_b && nvb) bulk_load(keys + ob + head_b, gb_val + head_b, 16u * nvb, mbar);
         }
+        if (tid >= 32 && tid < 32 + 12) {  // ragged ends, as for the columns
+            const int k = tid - 32;
+            const bool is_b = k >= 6;
+            const int e = is_b ? k - 6 : k;
+            const int count = is_b ? nb : na, head = is_b ? head_b : head_a, nv = is_b ? nvb : nva;
+            const int idx = e < 3 ? e : head + 4 * nv + (e - 3);
+            if (e < 3 ? e < head : idx < count) keys[(is_b ? ob : oa) + idx] = __float_as_uint(ld_late((is_b ? gb_val : ga_val) + idx));
+        }
+        if (!same_a) for (int e = tid; e < na; e += NT) keys[oa + e] = __float_as_uint(ld_late(ga_val + e));
+        if (!same_b) for (int e = tid; e < nb; e += NT) keys[ob + e] = __float_as_uint(ld_late(gb_val + e));
+        if (MODE == MODE_FUSED && !last && wid == 0) ask_base();
+        const bool values = wid != 1 || mbar_wait_bounded(mbar, 1, MBAR_POLL_LIMIT);
+        const bool all_values = __syncthreads_and(values);
+        const long long base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
+        if (base >= 0) {
+            int32_t *gz_col = Z.col + base + tid;
+            float *gz_val = Z.val + base + tid;
 #pragma unroll
-        for (int g = 0; g < GATHER; ++g) {
-            if (q0 + g < VT && (q0 + g) * NT + tid < total) {
-                gz_col[(q0 + g) * NT] = (int32_t)col[g];
-                gz_val[(q0 + g) * NT] = val[g];
+            for (int q = 0; q < VT; ++q)
+                if (live(q)) gz_col[q * NT] = (int32_t)col[q];
+            if (all_values) {
+                if (total < n) {  // there are twins: the value of the A entry becomes the sum
+                    const Src *of = src_of + rank;
+                    int k = 0;
+                    for (unsigned left = twin; left; left &= left - 1u, ++k) {
+                        const int i = __ffs(left) - 1;
+                        const uint32_t at = of[i];
+                        word_at(at) = __float_as_uint(__uint_as_float(word_at(at)) + __uint_as_float(word_at(partner(i, k, at))));
+                    }
+                    __syncthreads();
+                }
+#pragma unroll
+                for (int q = 0; q < VT; ++q)
+                    if (live(q)) gz_val[q * NT] = __uint_as_float(word_at(src_of[q * NT + tid]));
+            } else {  // the copies did not land in time: every thread fetches the values of its own share
+                int k = 0;
+                for (int i = 0; i < steps; ++i) {
+                    const uint32_t at = src_of[rank + i];
+                    float v = ld_late(reinterpret_cast<const float *>((at >= 4u * (uint32_t)ob ? vb : va) + at));
+                    if ((twin >> i) & 1u) v = v + ld_late(reinterpret_cast<const float *>(vb + partner(i, k++, at)));
+                    Z.val[base + rank + i] = v;
+                }
+            }
+        }
+        if (!all_values) mbar_wait_bounded(mbar, 1, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
+        if (base < 0) return;  // a bounded wait gave up; the host reports it
+    }
+    long long base;
+    if (!LEVELS && OP == OP_INTERSECT) {
+        // ---- a result's A word points to its B word
+        {
+            const Src *of = src_of + rank;
+            int k = 0;
+            for (unsigned left = twin; left; left &= left - 1u, ++k) {
+                const uint32_t at = of[k];
+                word_at(at) = partner(__ffs(left) - 1, k, at);
+            }
+        }
+        __syncthreads();
+        // ---- fetch columns and values, results q * NT + tid; the first batch before the output base is asked for
+        constexpr int GATHER = 8;
+        uint32_t col[GATHER];
+        float val[GATHER];
+        auto gather = [&](const int q0) {
+            uint32_t s[GATHER];
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) s[g] = live(q0 + g) ? (uint32_t)src_of[(q0 + g) * NT + tid] : 0u;
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                val[g] = 0.0f;
+                if (live(q0 + g)) {
+                    const uint32_t other = word_at(s[g]);
+                    col[g] = word_at(other) & cmask;
+                    val[g] = ld_late(reinterpret_cast<const float *>(va + s[g])) * ld_late(reinterpret_cast<const float *>(vb + other));
+                }
+            }
+        };
+        gather(0);
+        if (MODE == MODE_FUSED && !last && wid == 0) ask_base();
+        __syncthreads();
+        base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
+        if (base < 0) return;  // a bounded wait gave up; the host reports it
+        int32_t *gz_col = Z.col + base + tid;
+        float *gz_val = Z.val + base + tid;
+#pragma unroll
+        for (int q0 = 0; q0 < VT; q0 += GATHER) {
+            if (q0 > 0) {
+                if (q0 * NT >= total) break;
+                gather(q0);
+            }
+#pragma unroll
+            for (int g = 0; g < GATHER; ++g) {
+                if (live(q0 + g)) {
+                    gz_col[(q0 + g) * NT] = (int32_t)col[g];
+                    gz_val[(q0 + g) * NT] = val[g];
+                }
             }
         }
     }
-    }
+    base = MODE == MODE_FILL ? (long long)tile_count[t] : s_base;
 
     // ---- row offsets. Result row r starts after every result entry of rows < r; inside this tile those
     // are the survivors among the first d = (A entries before row r) + (B entries before row r) merged
     // entries: all of them up to the thread that holds position d, then, in that thread, a step per entry
     // except that a twin step covers two. The tile owns rows i0+1 .. i1 (the next tile's first row).
-    if (LEVELS && !Z.rp) return;
     auto end_row = [&](const int r, const uint32_t w) {
         const int d = (int)((w & 0xffffu) + (w >> 16));
         const int owner = d / VT;

@@ -66,6 +66,29 @@ def test_csr_tiles(nacho, oracle, total, shape):
     assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, csr_to_gpu(c))), oracle.csr_add_3(a, b, c, 8), "add_3")
 
 
+@pytest.mark.parametrize("total", [9, SMALL_STEP - 2, 2 * SMALL_STEP + 5, LARGE_FROM + 3])
+@pytest.mark.parametrize("shift", [(0, 1), (1, 0), (2, 3)])
+def test_csr_values_off_alignment(nacho, oracle, total, shift):
+    """Values whose place in memory sits differently on 16-byte boundaries than their columns': no bulk copy can bring them to the
+    columns' words."""
+    import torch
+    rows, cols = total // 20 + 1, 5000
+    rng = np.random.default_rng(total)
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+
+    def moved(x, by):
+        t = torch.empty(len(x) + by, dtype=torch.from_numpy(x).dtype, device="cuda")[by:]
+        return t.copy_(torch.from_numpy(x))
+
+    def matrices(key, by):
+        m = csr_of_keys(key, rows, cols, rng)
+        return m, nacho.CSR_gpu(torch.from_numpy(m.row_ptr).cuda(), moved(m.col, by[0]), moved(m.val, by[1]), torch.tensor([rows, cols], dtype=torch.int32))
+
+    (a, ga), (b, gb) = matrices(ka, shift), matrices(kb, shift[::-1])
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+
+
 @pytest.mark.parametrize("gap", [3000, 1_200_000])
 def test_runs_of_empty_rows(nacho, oracle, gap):
     """More tiles than fit the chip at once, with more rows between two of them than a tile keeps offsets of, empty but for a few: what a tile
