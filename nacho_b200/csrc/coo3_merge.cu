@@ -135,12 +135,10 @@ __device__ __forceinline__ int head_elems(const void *p) {
     return (int)(((16u - (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u) >> 2);
 }
 
-// All counts are in: the result length (negative after a give-up) goes to the control block and the host.
+// The last tile has its base: the result length (negative after a give-up of any tile) goes to the control block and the host.
 __device__ __forceinline__ void coo3_finish(FusedCtl *ctl, const Coo3Out &Z, long long total) {
-    __threadfence();
-    const int status = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK;
     if (total >= 0) ctl->total = total;
-    publish_result_word(Z.host, status, total < 0 ? 0 : total);
+    publish_result_word(Z.host, total < 0 ? NB200_E_TIMEOUT : NB200_OK, total < 0 ? 0 : total);
 }
 
 // One thread per tile, after the tile's sum: the last tile to get here writes the reduction's result.
@@ -383,8 +381,8 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
         if (tid == 0) {
             report_copy();
             if (MODE == MODE_FUSED) {
-                publish_count(words, t, 0);  // successors must not wait on this tile
-                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+                publish_failure(words, t);
+                if (t == num_tiles - 1) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
             }
             mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
         }
@@ -452,10 +450,10 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 
     // ---- output base of the tile
     if (MODE == MODE_FUSED && wid == 0) {
-        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+        const int64_t b = tile_base(words, t, total, &ctl->status, LOOKBACK_POLL_LIMIT);
         if (lane == 0) {
             sh.base = b;
-            if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) coo3_finish(ctl, Z, b < 0 ? b : b + total);
+            if (t == num_tiles - 1) coo3_finish(ctl, Z, b < 0 ? b : b + total);
         }
     }
     __syncthreads();
@@ -498,17 +496,9 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
     }
     __syncthreads();
     wait_for_previous();  // the cuts
-    const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
-    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
-        if (tid < 32) {
-            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
-            if (tid == 0) coo3_finish(ctl, Z, total);
-        }
-        return;
-    }
     // tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
     // only waits on CTAs dispatched before it (and every such wait is bounded)
-    const int t = blockIdx.x - (scanned ? 1 : 0);
+    const int t = blockIdx.x;
     int32_t a0 = 0, b0 = 0;
     int na = A.nnz, nb = B.nnz;
     if (cuts.a) {
@@ -573,8 +563,8 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
             if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
             __threadfence();
             if (MODE == MODE_FUSED) {
-                publish_count(words, t, 0);  // successors must not wait on this tile
-                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+                publish_failure(words, t);
+                if (t == num_tiles - 1) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
             }
             if (MODE == MODE_REDUCE) coo3_reduce_done(ctl, Z, num_tiles);
             mbar_wait_bounded(&sh.mbar, 0, MBAR_POLL_LIMIT);  // second bounded wait for copies in flight
@@ -756,7 +746,7 @@ cudaError_t launch_coo3_tile_v(const Coo3In &A, const Coo3In &B, const Packing &
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    const dim3 grid(num_tiles + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
+    const dim3 grid(num_tiles);
     if ((MODE == MODE_FUSED || MODE == MODE_REDUCE) && cuts.a)
         return launch_overlapped(kernel, grid, dim3(NT), smem, stream, A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles);
     kernel<<<grid, NT, smem, stream>>>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles);
@@ -866,7 +856,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed((size_t)num_tiles) + 4);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
+    const TileWords words = TileWords::at(fused_block + 4);
 
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     const Packing pk{bj, bk};
@@ -912,7 +902,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
         return NB200_OK;
     }
     if (fused) {
-        e = launch_coo3_tile_wide<MODE_FUSED>(A, B, cuts, nullptr, words.count, ctl, Z, num_tiles, stream);
+        e = launch_coo3_tile_wide<MODE_FUSED>(A, B, cuts, nullptr, words.word, ctl, Z, num_tiles, stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_tile_wide<fused>"));
         if ((st = read_ctl(h))) return fail(st);
         if (h.status.error != 0) return fail(note_timeout(h.status.error, h.status.detail, "coo3 merge"));

@@ -54,15 +54,9 @@ __device__ __forceinline__ void publish_timeout(long long *result) {
 // Whether an earlier launch on the stream, whose results a kernel builds on, ended without them.
 __device__ __forceinline__ bool gave_up(const FusedCtl *earlier) { return earlier && earlier->status.error != 0; }
 
-// All counts are in: the result length (negative after a give-up) goes to the control block and to
-// whoever waits for it. The status read here covers every tile: one whose columns did not land wrote it before its
-// count, and one that gives up on its base later than this finds that base there after all (merge_common.cuh).
-__device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, long long total, bool alone = false) {
-    int status = NB200_OK;
-    if (!alone) {  // a single tile has nobody's status to look at
-        __threadfence();
-        status = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0 ? NB200_E_TIMEOUT : NB200_OK;
-    }
+// The last tile has its base: the result length (negative after a give-up of any tile) goes to the control block and to whoever waits for it.
+__device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, long long total) {
+    int status = total < 0 ? NB200_E_TIMEOUT : NB200_OK;
     if (total >= 0) {
         ctl->total = total;
         publish_length(Z.result, total);
@@ -303,10 +297,9 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
         if (tid == 0) {
             if (atomicCAS(&ctl->status.error, 0, ERR_COPY_TIMEOUT) == 0) ctl->status.detail = t;
             publish_timeout(Z.result);
-            __threadfence();
             if (MODE == MODE_FUSED) {
-                publish_count(words, t, 0);  // successors must not wait on this tile
-                if (t == num_tiles - 1 && num_tiles <= DIRECT_TILES) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
+                publish_failure(words, t);
+                if (t == num_tiles - 1) publish_result_word(Z.host, NB200_E_TIMEOUT, 0);
             }
             mbar_wait_bounded(mbar, 0, MBAR_POLL_LIMIT);        // second bounded wait for copies in flight
         }
@@ -478,15 +471,15 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     }
     if (MODE == MODE_FUSED && tid == 0) publish_count(words, t, total);
     s_rank[tid] = rank;
-    // The last of a few tiles has the result length as soon as it has its base: the host learns it here, and prepares what
+    // The last tile has the result length as soon as it has its base: the host learns it here, and prepares what
     // comes next while the results are still on their way (a call on 200 x 180: 2.6 us earlier).
-    const bool last = MODE == MODE_FUSED && t == num_tiles - 1 && num_tiles <= DIRECT_TILES;
+    const bool last = MODE == MODE_FUSED && t == num_tiles - 1;
     auto ask_base = [&]() {
-        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, poll_limit);
+        const int64_t b = tile_base(words, t, total, &ctl->status, poll_limit);
         if (lane == 0) {
             s_base = b;
             if (b < 0) publish_timeout(Z.result);
-            if (last) finish_total(ctl, Z, b < 0 ? b : b + total, num_tiles == 1);
+            if (last) finish_total(ctl, Z, b < 0 ? b : b + total);
         }
     };
     if (last && wid == 0) ask_base();
@@ -734,18 +727,10 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     __syncthreads();
     trigger_dependents();  // whatever follows on the stream that was launched for it may take its places, and waits
     wait_for_previous();   // the cuts (no wait where no partition kernel ran)
-    const bool scanned = MODE == MODE_FUSED && num_tiles > DIRECT_TILES;
-    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no tile
-        if (threadIdx.x < 32) {
-            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, first_tile ? poll_limit : LOOKBACK_POLL_LIMIT);
-            if (threadIdx.x == 0) finish_total(ctl, Z, total);
-        }
-        return;
-    }
     // Tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
     // only ever waits on CTAs that were dispatched before it (and every such wait is bounded).
     // first_tile is 0 except in the self-tests that leave tile 0 out; poll_limit is smaller in all self-tests.
-    const int t = blockIdx.x + first_tile - (scanned ? 1 : 0);
+    const int t = blockIdx.x + first_tile;
     TileRange tile;
     if (cuts) {
         const int4 c0 = cuts[t], c1 = cuts[t + 1];
@@ -811,7 +796,7 @@ cudaError_t launch_tile_v(const CsrIn &A, const CsrIn &B, const RowCount &rows, 
                           const LevelOffsets &levels = LevelOffsets()) {
     cudaError_t e = configure_tile_kernel<V, OP, MODE, LEVELS>();
     if (e != cudaSuccess) return e;
-    const dim3 grid(num_tiles - knobs.first_tile + (MODE == MODE_FUSED && num_tiles > DIRECT_TILES ? 1 : 0));
+    const dim3 grid(num_tiles - knobs.first_tile);
     constexpr size_t smem = TilePlan<V, LEVELS>::BYTES;
     return launch_overlapped(k_csr2_tile<V, OP, MODE, LEVELS>, grid, dim3(NT), smem, stream, A, B, rows, cuts, cbits, tile_count, words, ctl, Z,
                              levels, num_tiles, knobs.first_tile, knobs.poll_limit);
@@ -912,7 +897,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     static_assert(sizeof(FusedCtl) <= 4 * sizeof(uint64_t), "control block must fit its slot");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
+    const TileWords words = TileWords::at(fused_block + 4);
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};
     const int cbits = col_bits(a->cols);
@@ -1068,7 +1053,7 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     static_assert(8 * (TileWords::needed(NOALLOC_MAX_TILES) + 4) + 16 * (NOALLOC_MAX_TILES + 1) + 512 <= NOALLOC_SCRATCH_BYTES,
                   "scratch layout must fit the fixed array");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
+    const TileWords words = TileWords::at(fused_block + 4);
     // the array keeps the previous call's contents: the control block and every tile word
     // must start at zero (the partition kernel clears them)
 
@@ -1108,7 +1093,7 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
     Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4, num_tiles);
+    const TileWords words = TileWords::at(fused_block + 4);
     *ctl_out = ctl;
     cudaError_t e = cudaSuccess;
     if (num_tiles == 1) {

@@ -22,113 +22,91 @@ enum Mode { MODE_COUNT = 0, MODE_FILL = 1, MODE_FUSED = 2, MODE_REDUCE = 3 };
 struct FusedCtl {
     int hollow;           // offsets mode: a result entry stands for empty ranges only
     DeviceStatus status;  // bounded-wait failures
-    long long total;      // result entries, written by whoever has all counts: the last of few tiles, else CTA 0 (MODE_REDUCE: the bits of a double, the running sum)
+    long long total;      // result entries, written by the last tile (MODE_REDUCE: the bits of a double, the running sum)
 };
 
 // ------------------------------------------------------------------- output bases ----
 //
-// The output base of a tile is the number of results of all earlier tiles, some 600 of which may still be
-// at work. One warp -- CTA 0 of the launch, the first to be dispatched -- reads the counts in order and
-// hands every tile its base in a word that only this tile polls. Letting tiles read
-// their predecessors' words instead loses to the polling itself: hundreds of tiles reading the lines that
-// hundreds of others are about to write. Measured at 64 M entries per operand, whole kernel: walking the
-// counts back 32 at a time 609 us, per-group sums that every tile reads in one round 519 us, this 470 us.
-// Up to DIRECT_TILES tiles, when everything is resident and little is polled, a tile adds up the counts
-// before it itself, one hop less.
+// The output base of a tile is the number of results of all earlier tiles, some 600 of which may still be at work. Every tile
+// has a word: first its own count, then, once the tile has its base, the count of all results up to its end. A tile reads the
+// words in front of its own, 32 in a trip to L2, back to the nearest one that holds such a sum: while 40 tiles end
+// in a microsecond that is one to five trips away, and the words that are looked at first are those that come last. What this replaced,
+// one CTA that read the counts in order and handed every tile its base, was two trips one after the other for every tile and handed out no more
+// than 32 bases in one: 2.0 of the 13 us of a tile between the last count in front of it and its base (67 M entries per operand), 3.0 of
+// the 13.4 us of a merge of 521 tiles, which all count at once. 410 -> 397 us a call of the former, 23.8 -> 22.3 of the latter, 16 M
+// entries intersected 114 -> 110, 100 M coordinates per operand 1086 -> 1040. Several windows in flight (64, 96, 128 words: 397, 404, 406 us) cost more in
+// registers than they save in trips.
 //
-// Whoever publishes the length (CTA 0, or the last tile) has read every count, and reads the status behind a fence
-// after that. A tile that gives up writes the status, and behind a fence looks at the word it misses once more: it is
-// still missing only if the publisher's look at the status is yet to come. So a length goes out as good only if
-// every tile has, or will find, its base.
-constexpr int DIRECT_TILES = 128;
+// A word is {tag, 28 bits; state, 2 bits; value, 34 bits} and is only ever raised (atomicMax), so a word of an earlier call,
+// whose tag is lower, counts as unpublished and needs no clearing. Tiles are numbered by CTA index, in which order CTAs start,
+// so a tile waits only on CTAs that started before it.
+//
+// Every wait is bounded. Who gives up on a word puts "failed" in its place, by compare and swap with what it held: a count that comes
+// later does not undo it, and one that came in between is used after all. A tile without a base marks its own word the same
+// way, and so does one whose columns did not land. No tile behind a failed word gets a base, the last one among
+// them, which reports the call's length: a length goes out only if every tile has, or will find, its base.
 
-// Words of one launch, zero at the start: a count and a base per tile.
+// Words of one launch, one per tile, with its tag (shifted into place; not zero). Words of lower tags may lie there.
 struct TileWords {
-    uint64_t *count, *base;
-    __host__ __device__ static constexpr size_t needed(size_t num_tiles) { return 2 * num_tiles; }
-    __host__ __device__ static TileWords at(uint64_t *p, int num_tiles) { return TileWords{p, p + num_tiles}; }
+    uint64_t *word;
+    uint64_t tag;
+    static constexpr int TAG_SHIFT = 36;
+    __host__ __device__ static constexpr size_t needed(size_t num_tiles) { return num_tiles; }
+    // Words that are zero, or of lower tags, at the start.
+    __host__ __device__ static TileWords at(uint64_t *p, uint32_t tag = 1) { return TileWords{p, (uint64_t)tag << TAG_SHIFT}; }
 };
+constexpr uint64_t TW_COUNT = 1ull << 34, TW_SUM = 2ull << 34, TW_FAILED = 3ull << 34, TW_VALUE_MASK = (1ull << 34) - 1;
 
+__device__ __forceinline__ void raise_word(const TileWords &words, const int t, const uint64_t state_and_value) {
+    atomicMax(reinterpret_cast<unsigned long long *>(words.word + t), (unsigned long long)(words.tag | state_and_value));
+}
+
+// A tile's count, by one thread, as soon as it is known.
 __device__ __forceinline__ void publish_count(const TileWords &words, const int t, const int count) {
-    st_relaxed_gpu(words.count + t, LB_AGGREGATE | (uint64_t)count);
+    raise_word(words, t, (t == 0 ? TW_SUM : TW_COUNT) | (uint64_t)count);
 }
+// The tile has no count, and nobody behind it a base.
+__device__ __forceinline__ void publish_failure(const TileWords &words, const int t) { raise_word(words, t, TW_FAILED); }
 
-// Runs in one warp. Publishes the base of every tile; returns the number of results, or -1 after
-// `poll_limit` rounds without a new count (the tiles that wait are told, and the error word is set). The
-// next round's load is on its way while a round is summed up: a round takes one trip to L2 and no more.
-__device__ __forceinline__ int64_t scan_tile_counts(const TileWords &words, const int num_tiles, DeviceStatus *status, const int poll_limit) {
-    const int lane = lane_id();
-    int64_t run = 0;
-    int idle = 0;
-    uint64_t w = lane < num_tiles ? ld_relaxed_gpu(words.count + lane) : 0;
-    for (int pos = 0;;) {
-        const unsigned missing = __ballot_sync(FULL_MASK, (w >> 62) == 0);
-        const int n = missing ? __ffs(missing) - 1 : 32;
-        const int next = pos + n;
-        const uint64_t w_next = next + lane < num_tiles ? ld_relaxed_gpu(words.count + next + lane) : 0;
-        if (n > 0) {
-            const int v = lane < n ? (int)(w & LB_VALUE_MASK) : 0;
-            const int incl = warp_incl_sum(v);
-            if (lane < n) st_relaxed_gpu(words.base + pos + lane, LB_PREFIX | (uint64_t)(run + incl - v));
-            run += __shfl_sync(FULL_MASK, incl, 31);
-            idle = 0;
-            if (next >= num_tiles) {
-                __syncwarp();  // the bases of all lanes lie before the fence of the one that publishes the length
-                return run;
-            }
-        } else if (++idle > poll_limit) {
-            if (lane == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = pos;
-            __threadfence();
-            for (int i = pos + lane; i < num_tiles; i += 32) st_relaxed_gpu(words.base + i, LB_FAILED);
-            return -1;
-        }
-        pos = next;
-        w = w_next;
-    }
-}
-
-// Output base of tile t, or -1 after a give-up. Called by all 32 lanes of one warp.
-__device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t, const int num_tiles, DeviceStatus *status, const int poll_limit) {
+// Output base of tile t, which has published `count`, or -1 after a give-up, here or in front of it. Called by all 32 lanes of one warp.
+__device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t, const int count, DeviceStatus *status, const int poll_limit) {
     if (t == 0) return 0;
-    auto record = [&]() {
-        if (lane_id() == 0 && atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
-        __syncwarp();
-        __threadfence();
-    };
-    uint64_t w = LB_AGGREGATE;  // lanes past the last predecessor add nothing
-    if (num_tiles <= DIRECT_TILES) {
-        int sum = 0;
-        for (int first = 0; first < t; first += 32) {
-            const int at = first + lane_id();
-            w = LB_AGGREGATE;
-            for (int polls = 0;; ++polls) {
-                if (at < t) w = ld_relaxed_gpu(words.count + at);
-                if (__all_sync(FULL_MASK, (w >> 62) != 0)) break;
-                if (polls >= poll_limit) {
-                    record();
-                    if (at < t) w = ld_relaxed_gpu(words.count + at);
-                    if (__all_sync(FULL_MASK, (w >> 62) != 0)) break;
-                    return -1;
-                }
+    const int lane = lane_id();
+    const uint32_t tag = (uint32_t)(words.tag >> 32);  // the upper word with no state in it
+    uint32_t sum = 0;                                  // two operands of up to 2^31 - 1 entries
+    bool failed = false;
+    int polls = 0;
+    for (int at = t - 1 - lane;;) {  // lane l looks at tile t - 1 - l, then 32 further back each time
+        uint64_t w = at >= 0 ? ld_relaxed_gpu(words.word + at) : words.tag | TW_SUM;  // before tile 0: an empty sum
+        uint32_t state = ((uint32_t)(w >> 32) ^ tag) >> 2;  // 1 to 3; anything else: unpublished
+        unsigned sums = __ballot_sync(FULL_MASK, state == 2u);
+        unsigned need = sums ? sums ^ (sums - 1u) : FULL_MASK;  // up to the nearest sum
+        const unsigned missing = __ballot_sync(FULL_MASK, state - 1u >= 3u) & need;
+        if (missing) {
+            if (++polls <= poll_limit) continue;
+            if ((missing >> lane) & 1u) {  // gives up on what is missing, unless it has come after all
+                const uint64_t now = atomicCAS(reinterpret_cast<unsigned long long *>(words.word + at), (unsigned long long)w, (unsigned long long)(words.tag | TW_FAILED));
+                w = now == w ? words.tag | TW_FAILED : now;
+                state = ((uint32_t)(w >> 32) ^ tag) >> 2;
             }
-            sum += (int)(w & LB_VALUE_MASK);
+            sums = __ballot_sync(FULL_MASK, state == 2u);
+            need = sums ? sums ^ (sums - 1u) : FULL_MASK;
         }
-        __syncwarp();  // every lane's look at the counts lies before the fence of the one that publishes the length
-        return __reduce_add_sync(FULL_MASK, sum);
+        failed = (__ballot_sync(FULL_MASK, state == 3u) & need) != 0u;
+        if ((need >> lane) & 1u) sum += (uint32_t)w;
+        if (sums || failed) break;
+        at -= 32;
     }
-    for (int polls = 0;; ++polls) {
-        if (lane_id() == 0) w = ld_relaxed_gpu(words.base + t);
-        w = __shfl_sync(FULL_MASK, w, 0);
-        if (w >> 62) break;
-        if (polls >= poll_limit) {
-            record();
-            if (lane_id() == 0) w = ld_relaxed_gpu(words.base + t);
-            w = __shfl_sync(FULL_MASK, w, 0);
-            break;
+    const int64_t base = failed ? -1 : (int64_t)__reduce_add_sync(FULL_MASK, sum);
+    if (lane == 0) {
+        if (failed) {
+            if (atomicCAS(&status->error, 0, ERR_LOOKBACK_TIMEOUT) == 0) status->detail = t;
+            publish_failure(words, t);
+        } else {
+            raise_word(words, t, TW_SUM | (uint64_t)(base + count));
         }
-        __nanosleep(64);
     }
-    return (w >> 62) == 2 ? (int64_t)(w & LB_VALUE_MASK) : -1;
+    return base;
 }
 
 // Exclusive prefix of the per-tile counts, in place, by one CTA; the grand total goes to

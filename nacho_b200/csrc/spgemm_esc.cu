@@ -1068,20 +1068,7 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
     __shared__ float s_val[SHORT_NT * SMALL_P];
     __shared__ int scan_tmp[40];
     __shared__ long long s_base;
-    auto finish = [&](long long total) {
-        __threadfence();
-        const bool bad = total < 0 || ld_relaxed_gpu_i32(&ctl->status.error) != 0;
-        publish_result_word(word, bad ? NB200_E_TIMEOUT : NB200_OK, bad ? 0 : total);
-    };
-    const bool scanned = num_tiles > DIRECT_TILES;
-    if (scanned && blockIdx.x == 0) {  // this CTA hands out the output bases and has no rows
-        if (threadIdx.x < 32) {
-            const int64_t total = scan_tile_counts(words, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
-            if (threadIdx.x == 0) finish(total);
-        }
-        return;
-    }
-    const int t = blockIdx.x - (scanned ? 1 : 0), tid = threadIdx.x, lane = lane_id();
+    const int t = blockIdx.x, tid = threadIdx.x, lane = lane_id();
     const int64_t i = (int64_t)t * SHORT_NT + tid;
     const int32_t lo = i < rows ? ld_nc(A.rp + i) : 0, hi = i < rows ? ld_nc(A.rp + i + 1) : 0;
     uint32_t pos[K], end[K];  // one past the last entry of 2^31 - 1 is still a position
@@ -1139,10 +1126,10 @@ __global__ void __launch_bounds__(SHORT_NT) k_esc_short(CsrView A, CsrView B, in
     const int rank = block_excl_sum<SHORT_NT>(count, scan_tmp, total);
     if (tid == 0) publish_count(words, t, total);
     if (warp_id() == 0) {
-        const int64_t b = tile_base(words, t, num_tiles, &ctl->status, LOOKBACK_POLL_LIMIT);
+        const int64_t b = tile_base(words, t, total, &ctl->status, LOOKBACK_POLL_LIMIT);
         if (lane == 0) {
             s_base = b;
-            if (t == num_tiles - 1 && !scanned) finish(b < 0 ? b : b + total);
+            if (t == num_tiles - 1) publish_result_word(word, b < 0 ? NB200_E_TIMEOUT : NB200_OK, b < 0 ? 0 : b + total);
         }
     }
     __syncthreads();
@@ -1617,11 +1604,11 @@ bool is_short(const EscPlan &plan) {
 int short_on(const EscPlan &plan, const nb200_csr *a, const nb200_csr *b, nb200_csr *c, cudaStream_t stream) {
     const CsrView A{a->row_ptr, a->col, a->val}, B{b->row_ptr, b->col, b->val};
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(plan.short_block);
-    const TileWords words = TileWords::at(plan.short_block + 4, plan.short_tiles);
+    const TileWords words = TileWords::at(plan.short_block + 4);
     auto kernel = plan.host.max_entries <= 4 ? k_esc_short<4> : plan.host.max_entries <= 6 ? k_esc_short<6> : k_esc_short<8>;
     {
         LaunchScope scope("esc_short", stream);
-        kernel<<<plan.short_tiles + (plan.short_tiles > DIRECT_TILES ? 1 : 0), SHORT_NT, 0, stream>>>(
+        kernel<<<plan.short_tiles, SHORT_NT, 0, stream>>>(
             A, B, a->rows, words, ctl, plan.short_tiles, c->row_ptr, c->col, c->val, plan.result + W_NNZ);
         NB200_CUDA(cudaGetLastError());
     }
