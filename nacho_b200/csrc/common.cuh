@@ -36,11 +36,26 @@ struct Workspace {
     size_t dev_bytes = 0;
     int64_t *host = nullptr;  // pinned, device-visible: 32 int64 slots for copies, then 32 result words that kernels write
     uint64_t generation = 0;  // bumped by every acquire: a holder can tell whether the block was handed out again
+    uint32_t tag = 0;         // acquire_tagged: the last tag or piece handed out, 0 while the block has to be cleared first
 };
 
 // `slot` selects one of several independent blocks per (device, stream): a driver that keeps an
 // intermediate alive across calls into other drivers takes slot 1 for it.
 int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int slot = 0);
+
+// Words that are written with a tag, 1 .. 2^28 - 1, which rises with every call: what an earlier call left there has a lower one, so nothing is
+// cleared between calls. The tag is part of a launch, so what is launched again without this call (a captured graph) must not use them. They
+// lie in a block of their own per (device, stream), which a later call may replace by a larger one. `mine`: eight zeroed words in a
+// block that stays, one of eight such pieces in turn; the launch has to clear `later`, which is handed out four calls on.
+struct Tagged {
+    uint64_t *words, *mine, *later;
+    uint32_t tag;
+};
+constexpr int TAGGED_SLOT = 6, RING_SLOT = 7;
+int acquire_tagged(cudaStream_t stream, size_t words, Tagged *out);
+// A launch that was given a piece did not run, or ended with an error: all pieces are cleared before one is used again. (wait_result_word
+// says so itself where it fails or the word reports an error.)
+void spoil_tagged(cudaStream_t stream);
 
 // Gives the device memory of one block back once the work queued on `stream` is done with it. Returns whether there was any.
 bool drop_workspace(cudaStream_t stream, int slot);
@@ -105,6 +120,9 @@ private:
     cudaEvent_t start_;
     bool timed_;
 };
+
+// Whether launches are being timed.
+bool profiling();
 
 // Launches `kernel` so that its CTAs may take their places while the kernel before it on the stream still
 // runs (programmatic dependent launch; that kernel says when, with trigger_dependents). A kernel that reads

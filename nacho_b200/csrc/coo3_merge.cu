@@ -67,9 +67,12 @@ struct WidePacking {
     }
 };
 
+// Tile cuts: positions in A and B. Without them the tiles find their cuts themselves, every `step` merged entries, with words of their own
+// (no step: a single tile).
 struct Cuts2 {
-    int32_t *a;
-    int32_t *b;
+    int32_t *a = nullptr, *b = nullptr;
+    int32_t step = 0;
+    OwnWords own;
 };
 
 template <typename PK>
@@ -85,6 +88,24 @@ __device__ __forceinline__ bool at_or_before(const Coo3In &A, int64_t m, const C
     const int32_t ja = ld_nc(A.j + m), jb = ld_nc(B.j + p);
     if (ja != jb) return ja < jb;
     return ld_nc(A.k + m) <= ld_nc(B.k + p);
+}
+
+// The cut at merged position d, equal coordinates on one side of it, between positions x_lo and x_hi of A, by G neighbouring lanes; all
+// lanes of a warp call this together. Returns the positions in A and B.
+template <int G>
+__device__ __forceinline__ int2 find_cut(const Coo3In &A, const Coo3In &B, const int64_t d, const int64_t x_lo, const int64_t x_hi, const bool mine) {
+    const int64_t x = group_count_true<G>((uint32_t)x_lo, (uint32_t)(mine ? x_hi : x_lo), [&](uint32_t m) { return at_or_before(A, m, B, d - 1 - m); });
+    int64_t y = d - x;
+    if (mine && x > 0 && y < B.nnz && ld_nc(A.i + x - 1) == ld_nc(B.i + y) && ld_nc(A.j + x - 1) == ld_nc(B.j + y) && ld_nc(A.k + x - 1) == ld_nc(B.k + y)) ++y;
+    return make_int2((int32_t)x, (int32_t)y);
+}
+
+// Cut t of a merge by a warp, over the whole range of A.
+__device__ __forceinline__ int2 tile_cut(const Coo3In &A, const Coo3In &B, const int32_t step, const int t, const int num_tiles) {
+    const int64_t total = (int64_t)A.nnz + B.nnz, d = min((int64_t)t * step, total);
+    const bool inner = t > 0 && t < num_tiles;
+    const int2 cut = find_cut<32>(A, B, d, max((int64_t)0, d - B.nnz), min(d, (int64_t)A.nnz), inner);
+    return inner ? cut : t == 0 ? make_int2(0, 0) : make_int2(A.nnz, B.nnz);
 }
 
 // Tile cuts, G lanes per cut. Cut t sits at merged position min(t * tile_step, total); equal coordinates stay on one
@@ -109,20 +130,11 @@ __global__ void __launch_bounds__(NT) k_coo3_partition(Coo3In A, Coo3In B, int64
         x_lo = max(x_lo, (int64_t)cuts.a[before]);
         x_hi = min(x_hi, (int64_t)cuts.a[min(before + between, num_tiles)]);
     }
-    const int64_t x = group_count_true<G>((uint32_t)x_lo, (uint32_t)(inner && mine ? x_hi : x_lo), [&](uint32_t m) { return at_or_before(A, m, B, d - 1 - m); });
-    int32_t pa = 0, pb = 0;
-    if (inner) {
-        int64_t y = d - x;
-        if (mine && x > 0 && y < B.nnz && ld_nc(A.i + x - 1) == ld_nc(B.i + y) && ld_nc(A.j + x - 1) == ld_nc(B.j + y) && ld_nc(A.k + x - 1) == ld_nc(B.k + y)) ++y;
-        pa = (int32_t)x;
-        pb = (int32_t)y;
-    } else if (t == num_tiles) {
-        pa = A.nnz;
-        pb = B.nnz;
-    }
+    int2 cut = find_cut<G>(A, B, d, x_lo, x_hi, inner && mine);
+    if (!inner) cut = t == 0 ? make_int2(0, 0) : make_int2(A.nnz, B.nnz);
     if ((threadIdx.x & (G - 1)) == 0 && mine) {
-        cuts.a[t] = pa;
-        cuts.b[t] = pb;
+        cuts.a[t] = cut.x;
+        cuts.b[t] = cut.y;
     }
 }
 
@@ -164,11 +176,12 @@ struct Coo3Plan {
 // A tile asks for the coordinates of one that starts a few microseconds later, so that they wait in L2. 100 M entries per
 // operand: 1238 us without, 1322, 1218, 1196 and 1197 with those 592, 296, 148 and 64 tiles ahead. Not for a tile that starts with
 // the first ones: 3 M entries per operand 77.1 -> 75.5 us.
-constexpr int TILES_AHEAD = 148, RESIDENT = 592;
+constexpr int TILES_AHEAD = 148;
 
 struct Coo3Shared {
     uint64_t mbar;
     long long base;  // output base of the tile
+    int2 cut[2];     // where it begins and ends, if it finds that out itself
     int wtotal[NT / 32];
     double partial[NT / 32];
 };
@@ -501,7 +514,17 @@ __global__ void __launch_bounds__(NT, 4) k_coo3_tile(const __grid_constant__ Coo
     const int t = blockIdx.x;
     int32_t a0 = 0, b0 = 0;
     int na = A.nnz, nb = B.nnz;
-    if (cuts.a) {
+    if (cuts.step) {
+        if (t == 0 && tid == 0) *cuts.own.clear = FusedCtl{};
+        const int w = tid >> 5;
+        if (w < 2) {
+            const int2 cut = tile_cut(A, B, cuts.step, t + w, num_tiles);
+            if ((tid & 31) == 0) sh.cut[w] = cut;
+        }
+        __syncthreads();
+        a0 = sh.cut[0].x, b0 = sh.cut[0].y;
+        na = sh.cut[1].x - a0, nb = sh.cut[1].y - b0;
+    } else if (cuts.a) {
         a0 = cuts.a[t], b0 = cuts.b[t];
         na = cuts.a[t + 1] - a0, nb = cuts.b[t + 1] - b0;
         if (tid == 96 && t + TILES_AHEAD >= RESIDENT && t + TILES_AHEAD < num_tiles) {
@@ -856,7 +879,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed((size_t)num_tiles) + 4);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4);
+    TileWords words = TileWords::at(fused_block + 4);
 
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     const Packing pk{bj, bk};
@@ -871,8 +894,13 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
             if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
         }
     }
-    if (num_tiles == 1 && fused && !wide) {
-        cuts = Cuts2{nullptr, nullptr};  // one tile: no cut to search, and the tile kernel clears the control block itself
+    const bool tagged = fused && !wide && num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    if (tagged) {
+        cuts = Cuts2{nullptr, nullptr, tile_step};
+        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return fail(st);
+        ctl = cuts.own.ctl, words = cuts.own.words;
+    } else if (num_tiles == 1 && fused && !wide) {
+        cuts = Cuts2{};  // one tile: no cut to search, and the tile kernel clears the control block itself
     } else {
         e = launch_coo3_partition(A, B, total, tile_step, num_tiles, cuts, fused_block, fused ? (int)TileWords::needed((size_t)num_tiles) + 4 : 4, stream);
     }
@@ -889,6 +917,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
     FusedCtl h;
     if (fused && !wide) {
         e = launch_coo3_tile<MODE_FUSED>(A, B, pk, cuts, nullptr, words, ctl, Z, num_tiles, v, stream);
+        if (e != cudaSuccess && tagged) spoil_tagged(stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "k_coo3_tile<fused>"));
         int64_t length;
         int device_status;
@@ -968,13 +997,19 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(block);
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     cudaError_t e = cudaSuccess;
-    if (num_tiles == 1) cuts = Cuts2{nullptr, nullptr};
+    const bool tagged = num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    if (tagged) {
+        cuts = Cuts2{nullptr, nullptr, tile_step};
+        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return st;
+        ctl = cuts.own.ctl;
+    } else if (num_tiles == 1) cuts = Cuts2{};
     else e = launch_coo3_partition(A, B, total, tile_step, num_tiles, cuts, block, 4, stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_partition");
     Coo3Out Z{};
     Z.host = result_word(ws, RW_COO3);
     Z.scalar = z;
     e = launch_coo3_tile<MODE_REDUCE>(A, B, Packing{bj, bk}, cuts, nullptr, TileWords{}, ctl, Z, num_tiles, v, stream);
+    if (e != cudaSuccess && tagged) spoil_tagged(stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_tile<reduce>");
     int64_t done;
     int device_status;

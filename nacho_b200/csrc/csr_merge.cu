@@ -31,9 +31,13 @@ namespace {
 
 constexpr int NT = CSR_NT;
 
-// Tile cuts: for cut t, {the row it falls in, the absolute positions in A and B, unused}. A null
-// pointer stands for the two cuts of a single tile, which need no search.
-using Cuts = int4 *;
+// Tile cuts: for cut t, {the row it falls in, the absolute positions in A and B, unused}. Without them the tiles find their cuts themselves, every
+// `step` merged entries, with words of their own (no step: a single tile, whose two cuts need no search).
+struct Cuts {
+    int4 *at = nullptr;
+    int32_t step = 0;
+    OwnWords own;
+};
 
 // One tile: rows i0 (where it begins) .. i1 (where the next one begins), its entries in A and B.
 struct TileRange {
@@ -79,27 +83,11 @@ __device__ __forceinline__ void finish_total(FusedCtl *ctl, const CsrOut &Z, lon
 
 // ------------------------------------------------------------------------- partition ----
 
-// G lanes per cut. Cut t sits at merged position min(t * tile_step, total).
+// Cut t, at merged position min(t * tile_step, total), by G neighbouring lanes; all lanes of a warp call this together.
 template <int G>
-__global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count,
-                                                       int32_t tile_step, int32_t num_tiles, Cuts cuts, long long *result,
-                                                       uint64_t *zero_block, int zero_words, const FusedCtl *earlier) {
-    wait_for_previous();   // the scratch that is cleared below may still be in use
-    trigger_dependents();  // the tile kernel may take its places; it waits for the cuts
-    const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
-    const int32_t rows = row_count.get();
-    // The merge in front of this one gave up: its offsets and columns are whatever the scratch held. No offset is
-    // followed, and every tile is empty; the tile kernel hands the status on.
-    const bool failed = gave_up(earlier);
+__device__ __forceinline__ int4 find_cut(const CsrIn &A, const CsrIn &B, const int32_t rows, const int32_t tile_step, const int t, const int num_tiles,
+                                         const bool failed) {
     const uint32_t total = (uint32_t)A.entries() + (uint32_t)B.entries();  // may be less than the tiles cover
-    if (result && gid == 0) {  // the tile kernel that follows fills in the rest
-        result[1] = NB200_OK;
-        result[2] = rows;
-    }
-    // the control block and the tile words of the kernel that follows start from zero (the grid has at
-    // least G >= 8 threads per tile word, so one word per thread covers them)
-    if (gid < zero_words) zero_block[gid] = 0;
-    const int t = (int)min(gid / G, (int64_t)num_tiles);  // spare groups repeat the last cut
     const int32_t a_base = row_offset(A, 0), b_base = row_offset(B, 0);
     const uint32_t d = (uint32_t)min((int64_t)t * tile_step, (int64_t)total);
     const bool inner = t > 0 && t < num_tiles && d < total && !failed;
@@ -118,15 +106,53 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
         return ld_late(A.col + a_lo + m) <= ld_late(B.col + b_lo + (dd - 1 - m));
     });
     int64_t y = dd - x;
-    if (inner) {
-        // Keep a column present in both operands on one side of the cut.
-        if (x > 0 && y < len_b && ld_late(A.col + a_lo + x - 1) == ld_late(B.col + b_lo + y)) ++y;
+    if (failed) return make_int4(0, 0, 0, 0);
+    if (!inner) return t == 0 ? make_int4(0, a_base, b_base, 0) : make_int4(rows, a_base + A.entries(), b_base + B.entries(), 0);
+    // Keep a column present in both operands on one side of the cut.
+    if (x > 0 && y < len_b && ld_late(A.col + a_lo + x - 1) == ld_late(B.col + b_lo + y)) ++y;
+    return make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0);
+}
+
+// The same by a warp, for a tile of its own accord.
+__device__ __forceinline__ int4 tile_cut(const CsrIn &A, const CsrIn &B, const RowCount &row_count, const int32_t tile_step, const int t, const int num_tiles,
+                                      const FusedCtl *earlier) {
+    return find_cut<32>(A, B, row_count.get(), tile_step, t, num_tiles, gave_up(earlier));
+}
+
+// A CTA in front of the tiles: eight lanes per cut, NT / 8 cuts a round.
+__device__ __forceinline__ void make_cuts(const CsrIn &A, const CsrIn &B, const RowCount &row_count, const Cuts &cuts, const int num_tiles, const FusedCtl *earlier) {
+    constexpr int G = 8;
+    const int32_t rows = row_count.get();
+    const bool failed = gave_up(earlier);
+    for (int first = cuts.own.first_cut() + blockIdx.x * (NT / G); first <= num_tiles; first += CUTTERS * (NT / G)) {
+        const int t = first + threadIdx.x / G;
+        const int4 cut = find_cut<G>(A, B, rows, cuts.step, min(t, num_tiles), num_tiles, failed);
+        if ((threadIdx.x & (G - 1)) == 0 && t <= num_tiles) store_cut(cuts.own, t, cut);
     }
-    if ((threadIdx.x & (G - 1)) == 0 && gid / G <= num_tiles) {
-        cuts[t] = failed ? make_int4(0, 0, 0, 0)
-                : inner ? make_int4(row, a_lo + (int32_t)x, b_lo + (int32_t)y, 0)
-                        : t == 0 ? make_int4(0, a_base, b_base, 0) : make_int4(rows, a_base + A.entries(), b_base + B.entries(), 0);
+}
+
+// G lanes per cut.
+template <int G>
+__global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCount row_count,
+                                                       int32_t tile_step, int32_t num_tiles, int4 *cuts, long long *result,
+                                                       uint64_t *zero_block, int zero_words, const FusedCtl *earlier) {
+    wait_for_previous();   // the scratch that is cleared below may still be in use
+    trigger_dependents();  // the tile kernel may take its places; it waits for the cuts
+    const int64_t gid = (int64_t)blockIdx.x * NT + threadIdx.x;
+    const int32_t rows = row_count.get();
+    // The merge in front of this one gave up: its offsets and columns are whatever the scratch held. No offset is
+    // followed, and every tile is empty; the tile kernel hands the status on.
+    const bool failed = gave_up(earlier);
+    if (result && gid == 0) {  // the tile kernel that follows fills in the rest
+        result[1] = NB200_OK;
+        result[2] = rows;
     }
+    // the control block and the tile words of the kernel that follows start from zero (the grid has at
+    // least G >= 8 threads per tile word, so one word per thread covers them)
+    if (gid < zero_words) zero_block[gid] = 0;
+    const int t = (int)min(gid / G, (int64_t)num_tiles);  // spare groups repeat the last cut
+    const int4 cut = find_cut<G>(A, B, rows, tile_step, t, num_tiles, failed);
+    if ((threadIdx.x & (G - 1)) == 0 && gid / G <= num_tiles) cuts[t] = cut;
 }
 
 // ------------------------------------------------------------------------ tile kernel ----
@@ -160,12 +186,18 @@ constexpr uint32_t ROW_FAR = 0xffffu;
 // they are read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns
 // ahead as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.) Not for a tile that starts with the
 // first ones, and at most as many offsets as a tile keeps: beyond those lie runs of empty rows, which could fill the L2.
-constexpr int TILES_AHEAD = 148, RESIDENT = 592;
+constexpr int TILES_AHEAD = 148;
+// Tiles up to which a call that waits for its length is one launch. Two operands of 24, 32, 40 and 50 M entries (6050, 8070, 10090 and 12610 tiles) take
+// 171.4, 217.4, 262.1 and 319.4 us with a launch for the cuts in front, 168.8, 216.3, 263.9 and 323.6 without: the places of the CTAs that make
+// the cuts are worth more than the time before the first tile then.
+constexpr int OWN_CUTS_UP_TO = 8192;
 
 // Fixed shared memory of a tile (one block for both key widths).
 struct TileShared {
     uint64_t mbar;
     long long base;                 // output base of the tile
+    int4 cut[2];                    // where it begins and ends, if it finds that out itself
+    int lost;                       // a cut did not come in time
     int trow[NT], wrow[NT / 32];    // the last row that starts at or before a thread's / between two warps' diagonals;
                                     // once every thread has its row, trow holds the threads' first results instead
     unsigned twin[NT];
@@ -194,7 +226,7 @@ struct TileShared {
 //   - an intersection keeps the gather: its results are few, and most values would be copied for nothing. What follows from a twin is done in a
 //     loop over a thread's twins, not as a test per step (16 M entries, half of them shared: 122 -> 114 us);
 //   - a tile needs 6 bytes of shared memory per entry instead of 16: 55 KB with 31 entries per thread, so four CTAs share an SM.
-template <int VT, int OP, int MODE, bool LEVELS, bool WIDE>
+template <int VT, int OP, int MODE, bool LEVELS, bool OWN, bool WIDE>
 __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const TileRange &tile, const int cbits, const int t,
                                           const int num_tiles, int32_t *tile_count, const TileWords &words, FusedCtl *ctl,
                                           const CsrOut &Z, const LevelOffsets &L, unsigned char *smem_raw, TileShared &sh,
@@ -479,7 +511,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
         if (lane == 0) {
             s_base = b;
             if (b < 0) publish_timeout(Z.result);
-            if (last) finish_total(ctl, Z, b < 0 ? b : b + total);
+            if (last) finish_total(ctl, Z, b < 0 || (OWN && sh.lost) ? -1 : b + total);
         }
     };
     if (last && wid == 0) ask_base();
@@ -704,15 +736,17 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     if (t == 0 && tid == 0) Z.rp[0] = 0;
 }
 
-template <int VT, int OP, int MODE, bool LEVELS>
+template <int VT, int OP, int MODE, bool LEVELS, bool OWN>
 __device__ __noinline__ void csr2_tile_wide(const CsrIn &A, const CsrIn &B, const TileRange tile, const int cbits, const int t,
                                             const int num_tiles, int32_t *tile_count, const TileWords &words, FusedCtl *ctl,
                                             const CsrOut &Z, const LevelOffsets &L, unsigned char *smem_raw, TileShared &sh,
                                           const int poll_limit) {
-    csr2_tile<VT, OP, MODE, LEVELS, true>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
+    csr2_tile<VT, OP, MODE, LEVELS, OWN, true>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
 }
 
-template <int V, int OP, int MODE, bool LEVELS>
+// OWN: without a launch in front of it. (A kernel of its own: with both in one the merges that have such a launch are 1.4 % slower, 67 M entries
+// per operand 394 -> 400 us.)
+template <int V, int OP, int MODE, bool LEVELS, bool OWN>
 __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ CsrIn A, const __grid_constant__ CsrIn B,
                                                                     const RowCount row_count, const Cuts cuts, int cbits,
                                                                     int32_t *tile_count, const __grid_constant__ TileWords words, FusedCtl *ctl,
@@ -723,6 +757,7 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     if (threadIdx.x == 0) {
         mbar_init(&sh.mbar, 1);
         mbar_fence_init();
+        if (OWN) sh.lost = 0;
     }
     __syncthreads();
     trigger_dependents();  // whatever follows on the stream that was launched for it may take its places, and waits
@@ -730,13 +765,45 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     // Tiles are numbered by CTA index: CTAs are dispatched in increasing index order, so a tile
     // only ever waits on CTAs that were dispatched before it (and every such wait is bounded).
     // first_tile is 0 except in the self-tests that leave tile 0 out; poll_limit is smaller in all self-tests.
-    const int t = blockIdx.x + first_tile;
+    const int t = OWN ? (int)blockIdx.x - cuts.own.cutters + first_tile : (int)blockIdx.x + first_tile;
     TileRange tile;
-    if (cuts) {
-        const int4 c0 = cuts[t], c1 = cuts[t + 1];
+    if (OWN) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *cuts.own.clear = FusedCtl{};
+        if (t < first_tile) {  // one of the CTAs in front of the tiles
+            make_cuts(A, B, row_count, cuts, num_tiles, Z.earlier);
+            return;
+        }
+        const int w = threadIdx.x >> 5;
+        const bool given = cuts.own.cutters && t >= cuts.own.first_cut();
+        if (w < 2) {
+            int4 cut = make_int4(0, 0, 0, 0);
+            const bool ok = !given || await_cut(cuts.own, t + w, poll_limit, &cut);
+            if (!given) cut = tile_cut(A, B, row_count, cuts.step, t + w, num_tiles, Z.earlier);
+            if (lane_id() == 0) {
+                sh.cut[w] = cut;
+                if (!ok) {  // reported, and the tile is empty
+                    sh.lost = 1;
+                    if (atomicCAS(&ctl->status.error, 0, ERR_LOOKBACK_TIMEOUT) == 0) ctl->status.detail = t;
+                    publish_failure(words, t);
+                }
+            }
+        }
+        __syncthreads();
+        const int4 c0 = sh.cut[0], c1 = sh.lost ? c0 : sh.cut[1];
+        tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
+        if (V != V_MOST && given && threadIdx.x == 96 && t + TILES_AHEAD < num_tiles) {
+            int4 from, to;
+            if (peek_cut(cuts.own, t + TILES_AHEAD, &from) && peek_cut(cuts.own, t + TILES_AHEAD + 1, &to)) {
+                const int32_t n = min(to.x - from.x, TilePlan<V, LEVELS>::ROWS) + 1;
+                if (A.rp) prefetch_l2(A.rp + from.x, n);
+                if (B.rp) prefetch_l2(B.rp + from.x, n);
+            }
+        }
+    } else if (cuts.at) {
+        const int4 c0 = cuts.at[t], c1 = cuts.at[t + 1];
         tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
         if (V != V_MOST && threadIdx.x == 96 && t + TILES_AHEAD >= RESIDENT && t + TILES_AHEAD < num_tiles) {
-            const int32_t r0 = cuts[t + TILES_AHEAD].x, n = min(cuts[t + TILES_AHEAD + 1].x - r0, TilePlan<V, LEVELS>::ROWS) + 1;
+            const int32_t r0 = cuts.at[t + TILES_AHEAD].x, n = min(cuts.at[t + TILES_AHEAD + 1].x - r0, TilePlan<V, LEVELS>::ROWS) + 1;
             if (A.rp) prefetch_l2(A.rp + r0, n);
             if (B.rp) prefetch_l2(B.rp + r0, n);
         }
@@ -755,9 +822,9 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     const uint64_t nr = (uint64_t)(tile.i1 - tile.i0) + 1;
     const bool narrow = cbits < 31 && (nr << cbits) <= 0x80000000ull;
     if (narrow) {
-        csr2_tile<V, OP, MODE, LEVELS, false>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
+        csr2_tile<V, OP, MODE, LEVELS, OWN, false>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
     } else {
-        csr2_tile_wide<V, OP, MODE, LEVELS>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
+        csr2_tile_wide<V, OP, MODE, LEVELS, OWN>(A, B, tile, cbits, t, num_tiles, tile_count, words, ctl, Z, L, smem_raw, sh, poll_limit);
     }
 }
 
@@ -775,13 +842,13 @@ constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_S
 constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between two tile cuts (a twin may add one)
 
 // Raises the tile kernel's dynamic shared-memory limit once per instantiation and device.
-template <int V, int OP, int MODE, bool LEVELS = false>
+template <int V, int OP, int MODE, bool LEVELS = false, bool OWN = false>
 cudaError_t configure_tile_kernel() {
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_csr2_tile<V, OP, MODE, LEVELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TilePlan<V, LEVELS>::BYTES);
+        cudaError_t e = cudaFuncSetAttribute(k_csr2_tile<V, OP, MODE, LEVELS, OWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TilePlan<V, LEVELS>::BYTES);
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
@@ -794,11 +861,18 @@ template <int V, int OP, int MODE, bool LEVELS = false>
 cudaError_t launch_tile_v(const CsrIn &A, const CsrIn &B, const RowCount &rows, const Cuts &cuts, int cbits, int32_t *tile_count,
                           TileWords words, FusedCtl *ctl, const CsrOut &Z, int num_tiles, cudaStream_t stream, const LaunchKnobs &knobs,
                           const LevelOffsets &levels = LevelOffsets()) {
+    constexpr size_t smem = TilePlan<V, LEVELS>::BYTES;
+    const dim3 grid(num_tiles - knobs.first_tile + cuts.own.cutters);
+    if (MODE == MODE_FUSED && cuts.step) {
+        constexpr bool OWN = MODE == MODE_FUSED;
+        cudaError_t e = configure_tile_kernel<V, OP, MODE, LEVELS, OWN>();
+        if (e != cudaSuccess) return e;
+        return launch_overlapped(k_csr2_tile<V, OP, MODE, LEVELS, OWN>, grid, dim3(NT), smem, stream, A, B, rows, cuts, cbits, tile_count, words, ctl, Z,
+                                 levels, num_tiles, knobs.first_tile, knobs.poll_limit);
+    }
     cudaError_t e = configure_tile_kernel<V, OP, MODE, LEVELS>();
     if (e != cudaSuccess) return e;
-    const dim3 grid(num_tiles - knobs.first_tile);
-    constexpr size_t smem = TilePlan<V, LEVELS>::BYTES;
-    return launch_overlapped(k_csr2_tile<V, OP, MODE, LEVELS>, grid, dim3(NT), smem, stream, A, B, rows, cuts, cbits, tile_count, words, ctl, Z,
+    return launch_overlapped(k_csr2_tile<V, OP, MODE, LEVELS, false>, grid, dim3(NT), smem, stream, A, B, rows, cuts, cbits, tile_count, words, ctl, Z,
                              levels, num_tiles, knobs.first_tile, knobs.poll_limit);
 }
 
@@ -816,7 +890,7 @@ cudaError_t launch_tile(const CsrIn &A, const CsrIn &B, const RowCount &rows, co
 
 // Eight lanes per cut once a full warp per cut would need more than one wave of the chip: the searches
 // then run a few dependent loads longer, but four times fewer warps issue them.
-cudaError_t launch_partition(const CsrIn &A, const CsrIn &B, const RowCount &rows, int num_tiles, int step, const Cuts &cuts,
+cudaError_t launch_partition(const CsrIn &A, const CsrIn &B, const RowCount &rows, int num_tiles, int step, int4 *cuts,
                              long long *result, uint64_t *zero_block, int zero_words, cudaStream_t stream, const FusedCtl *earlier = nullptr) {
     const int64_t lanes = num_tiles < 8192 ? 32 : 8;
     const int blocks = (int)(((int64_t)(num_tiles + 1) * lanes + NT - 1) / NT);
@@ -890,14 +964,15 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     Workspace *ws = nullptr;
     if ((st = acquire_workspace(stream, sizes.used(), &ws))) return fail(st);
     Carver carve(ws->dev);
-    Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
+    Cuts cuts;
+    cuts.at = carve.take<int4>((size_t)num_tiles + 1);
     int32_t *tile_count = carve.take<int32_t>((size_t)num_tiles + 1);
     // control block (status word, result length) and the tile words of the single-pass kernel, contiguous for the partition
     // kernel, which clears them; the two-pass route uses the control block alone
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     static_assert(sizeof(FusedCtl) <= 4 * sizeof(uint64_t), "control block must fit its slot");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4);
+    TileWords words = TileWords::at(fused_block + 4);
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};
     const int cbits = col_bits(a->cols);
@@ -915,11 +990,16 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
         if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&z->val), sizeof(float) * (size_t)bound, stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
     }
-    if (num_tiles == 1) {
-        cuts = nullptr;  // one tile: no cut to search, and the tile kernel clears the control block itself
+    const bool tagged = fused && !device_result && num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    if (tagged) {
+        cuts = Cuts{nullptr, step};
+        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return fail(st);
+        ctl = cuts.own.ctl, words = cuts.own.words;
+    } else if (num_tiles == 1) {
+        cuts.at = nullptr;  // one tile: no cut to search, and the tile kernel clears the control block itself
     } else {
         LaunchScope scope("csr2_partition", stream);
-        e = launch_partition(A, B, row_count, num_tiles, step, cuts, reinterpret_cast<long long *>(device_result), fused_block,
+        e = launch_partition(A, B, row_count, num_tiles, step, cuts.at, reinterpret_cast<long long *>(device_result), fused_block,
                              fused ? (int)TileWords::needed(num_tiles) + 4 : 4, stream);
     }
     if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_partition"));
@@ -939,6 +1019,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
         e = launch_tile<OP, MODE_FUSED>(A, B, row_count, cuts, cbits, nullptr, words, ctl,
                                         CsrOut{z->row_ptr, z->col, z->val, reinterpret_cast<long long *>(device_result), word}, num_tiles, v, stream,
                                         knobs);
+        if (e != cudaSuccess && tagged) spoil_tagged(stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "k_csr2_tile<fused>"));
         if (device_result) return NB200_OK;  // length, status and rows arrive in the caller's device words, written by the kernels
         int64_t length;
@@ -1049,7 +1130,8 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     if ((st = noalloc_scratch_address(&scratch))) return st;
     Carver carve(scratch);
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(NOALLOC_MAX_TILES) + 4);
-    Cuts cuts = carve.take<int4>((size_t)NOALLOC_MAX_TILES + 1);
+    Cuts cuts;
+    cuts.at = carve.take<int4>((size_t)NOALLOC_MAX_TILES + 1);
     static_assert(8 * (TileWords::needed(NOALLOC_MAX_TILES) + 4) + 16 * (NOALLOC_MAX_TILES + 1) + 512 <= NOALLOC_SCRATCH_BYTES,
                   "scratch layout must fit the fixed array");
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
@@ -1058,7 +1140,7 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     // must start at zero (the partition kernel clears them)
 
     const CsrIn A{a->row_ptr, a->col, a->val, a->nnz}, B{b->row_ptr, b->col, b->val, b->nnz};
-    NB200_CUDA(launch_partition(A, B, row_count, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream));
+    NB200_CUDA(launch_partition(A, B, row_count, num_tiles, step, cuts.at, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream));
     const CsrOut Z{z->row_ptr, z->col, z->val};
     NB200_CUDA((v == V_LARGE ? launch_tile_v<V_LARGE, OP_UNION, MODE_FUSED>(A, B, row_count, cuts, col_bits(a->cols), nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs())
                             : launch_tile_v<V_SMALL, OP_UNION, MODE_FUSED>(A, B, row_count, cuts, col_bits(a->cols), nullptr, words, ctl, Z, num_tiles, stream, LaunchKnobs())));
@@ -1090,17 +1172,24 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
     const int v = tile_v(total) == V_SMALL ? V_SMALL : levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE, step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
     Carver carve(scratch);
-    Cuts cuts = carve.take<int4>((size_t)num_tiles + 1);
+    Cuts cuts;
+    cuts.at = carve.take<int4>((size_t)num_tiles + 1);
     uint64_t *fused_block = carve.take<uint64_t>(TileWords::needed(num_tiles) + 4);
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(fused_block);
-    const TileWords words = TileWords::at(fused_block + 4);
+    TileWords words = TileWords::at(fused_block + 4);
     *ctl_out = ctl;
     cudaError_t e = cudaSuccess;
-    if (num_tiles == 1) {
-        cuts = nullptr;
+    const bool tagged = num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    if (tagged) {
+        cuts = Cuts{nullptr, step};
+        const int st = take_own_words(stream, num_tiles, &cuts.own);
+        if (st != NB200_OK) return st;
+        *ctl_out = ctl = cuts.own.ctl, words = cuts.own.words;
+    } else if (num_tiles == 1) {
+        cuts.at = nullptr;
     } else {
         LaunchScope scope("csr2_partition", stream);
-        e = launch_partition(A, B, rows, num_tiles, step, cuts, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream, Z.earlier);
+        e = launch_partition(A, B, rows, num_tiles, step, cuts.at, nullptr, fused_block, (int)TileWords::needed(num_tiles) + 4, stream, Z.earlier);
     }
     if (e != cudaSuccess) return note_cuda_error(e, "k_csr2_partition");
     const int cbits = col_bits(cols);
@@ -1116,6 +1205,7 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
     } else {
         e = launch_tile<OP_INTERSECT, MODE_FUSED>(A, B, rows, cuts, cbits, nullptr, words, ctl, Z, num_tiles, v, stream, knobs);
     }
+    if (e != cudaSuccess && tagged) spoil_tagged(stream);
     return e == cudaSuccess ? NB200_OK : note_cuda_error(e, "k_csr2_tile");
 }
 

@@ -109,6 +109,68 @@ __device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t
     return base;
 }
 
+// ------------------------------------------------------------------------- tile cuts ----
+//
+// A merge whose call waits for its length is one launch, where it does not have too many tiles: they find their cuts themselves, with words of their own
+// (acquire_tagged) in which nothing needs to be cleared but the control block of a later merge. The first tiles, those that are at work at once from
+// the start (four CTAs on each of 148 SMs), search for both of their cuts before anything else. For all others a few CTAs in front of
+// the tiles make the cuts, in order and faster than tiles end, and leave them in tagged words. A launch in front of the merge makes all cuts
+// before the first tile begins; the other routes keep it (asynchronous calls, whose launches may be captured and run again; counts before a
+// fill; a profiled call, which is to tell the searches from the merge). us a call, with that launch and without: sums of 10900 entries per operand
+// 15.6 and 14.9, 0.5 M 19.1 and 17.7, 3.3 M 44.2 and 40.4, 4.5 M in short rows 66.5 and 57.9; intersection of 16 M 88.5 and 83.5; three operands of 9 M 183 and
+// 176; trees of 100 K 45.8 and 41.8. Coordinate lists have such CTAs nowhere: their probes, of up to six loads far apart, cannot keep up
+// with the tiles (100 M entries per operand 1024 us with the launch, 1341 so), so they stay with RESIDENT tiles (inner product of 300 K entries 20.9 and 18.3).
+constexpr int RESIDENT = 592;  // tiles at work at once
+constexpr int CUTTERS = 32;    // CTAs that make cuts, where there are more tiles than that
+struct OwnWords {
+    FusedCtl *ctl = nullptr, *clear = nullptr;  // of this merge; of a later one
+    TileWords words{nullptr, 0};
+    uint64_t *cut = nullptr;  // four words a cut
+    int cutters = 0;          // leading CTAs that make the cuts from first_cut() on
+    __host__ __device__ int first_cut() const { return RESIDENT - CUTTERS; }
+};
+inline int take_own_words(cudaStream_t stream, int num_tiles, OwnWords *out) {
+    static_assert(sizeof(FusedCtl) <= 8 * sizeof(uint64_t), "a control block takes a piece");
+    const bool many = num_tiles > RESIDENT;
+    Tagged block;
+    const int st = acquire_tagged(stream, many ? 5 * (size_t)num_tiles + 4 : RESIDENT, &block);
+    if (st != NB200_OK) return st;
+    out->ctl = reinterpret_cast<FusedCtl *>(block.mine);
+    out->clear = reinterpret_cast<FusedCtl *>(block.later);
+    out->words = TileWords::at(block.words, block.tag);
+    out->cut = block.words + num_tiles;
+    out->cutters = many ? CUTTERS : 0;
+    return NB200_OK;
+}
+
+// One thread. What the reader of the cut goes on to read lies before it.
+__device__ __forceinline__ void store_cut(const OwnWords &own, const int t, const int4 cut) {
+    __threadfence();
+    uint64_t *w = own.cut + 4 * (size_t)t;
+    st_relaxed_gpu(w, own.words.tag | (uint32_t)cut.x);
+    st_relaxed_gpu(w + 1, own.words.tag | (uint32_t)cut.y);
+    st_relaxed_gpu(w + 2, own.words.tag | (uint32_t)cut.z);
+}
+// All lanes of a warp; every lane gets the cut. False after a give-up.
+__device__ __forceinline__ bool await_cut(const OwnWords &own, const int t, const int poll_limit, int4 *cut) {
+    const uint64_t *w = own.cut + 4 * (size_t)t + min(lane_id(), 2);
+    uint64_t v = 0;
+    for (int polls = 0;; ++polls) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+        if (__all_sync(FULL_MASK, (v ^ own.words.tag) >> TileWords::TAG_SHIFT == 0)) break;
+        if (polls >= poll_limit) return false;
+    }
+    *cut = make_int4(__shfl_sync(FULL_MASK, (int)v, 0), __shfl_sync(FULL_MASK, (int)v, 1), __shfl_sync(FULL_MASK, (int)v, 2), 0);
+    return true;
+}
+// One thread, without waiting: whether the cut is there.
+__device__ __forceinline__ bool peek_cut(const OwnWords &own, const int t, int4 *cut) {
+    const uint64_t *w = own.cut + 4 * (size_t)t;
+    const uint64_t x = ld_relaxed_gpu(w), y = ld_relaxed_gpu(w + 1), z = ld_relaxed_gpu(w + 2);
+    *cut = make_int4((int)x, (int)y, (int)z, 0);
+    return (((x ^ own.words.tag) | (y ^ own.words.tag) | (z ^ own.words.tag)) >> TileWords::TAG_SHIFT) == 0;
+}
+
 // Exclusive prefix of the per-tile counts, in place, by one CTA; the grand total goes to
 // *total_out (64-bit so that the host can detect int32 overflow).
 static __global__ void __launch_bounds__(1024) k_scan_tiles(int32_t *counts, int32_t n, int64_t *total_out) {

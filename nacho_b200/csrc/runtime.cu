@@ -88,6 +88,7 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
             NB200_CUDA(cudaFree(ws.dev));
             ws.dev = nullptr;
             ws.dev_bytes = 0;
+            ws.tag = 0;
         }
         size_t want = bytes + bytes / 4 + 4096;
         NB200_CUDA(cudaMalloc(&ws.dev, want));
@@ -95,6 +96,43 @@ int acquire_workspace(cudaStream_t stream, size_t bytes, Workspace **out, int sl
     }
     *out = &ws;
     return NB200_OK;
+}
+
+namespace {
+// A block that has to be cleared, which a capture would put off.
+int clear_block(Workspace *ws, cudaStream_t stream) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    NB200_CUDA(cudaStreamIsCapturing(stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return note_cuda_error(cudaErrorStreamCaptureUnsupported, "a call that waits for its result");
+    NB200_CUDA(cudaMemsetAsync(ws->dev, 0, ws->dev_bytes, stream));
+    return NB200_OK;
+}
+}  // namespace
+
+int acquire_tagged(cudaStream_t stream, size_t words, Tagged *out) {
+    Workspace *ring = nullptr, *block = nullptr;
+    int st;
+    if ((st = acquire_workspace(stream, 64 * sizeof(uint64_t), &ring, RING_SLOT))) return st;
+    if ((st = acquire_workspace(stream, words * sizeof(uint64_t), &block, TAGGED_SLOT))) return st;
+    if (ring->tag == 0 && (st = clear_block(ring, stream))) return st;
+    if (block->tag == 0 || block->tag + 1 >= 1u << 28) {
+        block->tag = 0;
+        if ((st = clear_block(block, stream))) return st;
+    }
+    if (++ring->tag == 0) ring->tag = 8;  // after 2^32 of them; the same piece
+    out->mine = static_cast<uint64_t *>(ring->dev) + 8 * (ring->tag % 8);
+    out->later = static_cast<uint64_t *>(ring->dev) + 8 * ((ring->tag + 4) % 8);
+    out->words = static_cast<uint64_t *>(block->dev);
+    out->tag = ++block->tag;
+    return NB200_OK;
+}
+
+void spoil_tagged(cudaStream_t stream) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> g(g_ws_mutex);
+    auto it = g_workspaces.find({{dev, RING_SLOT}, stream});
+    if (it != g_workspaces.end()) it->second.tag = 0;
 }
 
 bool drop_workspace(cudaStream_t stream, int slot) {
@@ -108,6 +146,7 @@ bool drop_workspace(cudaStream_t stream, int slot) {
     if (cudaStreamSynchronize(stream) != cudaSuccess || cudaFree(ws.dev) != cudaSuccess) return false;
     ws.dev = nullptr;
     ws.dev_bytes = 0;
+    ws.tag = 0;
     return true;
 }
 
@@ -121,11 +160,16 @@ int wait_result_word(const unsigned long long *word, cudaStream_t stream, int64_
         if (spins % 4096 != 0) continue;  // about every 100 us: has the stream failed, or ended without the word?
         const cudaError_t e = cudaStreamQuery(stream);
         if (e == cudaErrorNotReady) continue;
-        if (e != cudaSuccess) return note_cuda_error(e, "wait for a result length");
+        if (e != cudaSuccess) {
+            spoil_tagged(stream);
+            return note_cuda_error(e, "wait for a result length");
+        }
         if ((v = *w) & RW_VALID) break;
+        spoil_tagged(stream);
         return note_cuda_error(cudaErrorUnknown, "the kernels ended without a result length");
     }
     *device_status = (int)((v & ~RW_VALID) >> RW_STATUS_SHIFT);
+    if (*device_status != 0) spoil_tagged(stream);
     *value = (int64_t)(v & RW_VALUE_MASK);
     return NB200_OK;
 }
@@ -141,6 +185,8 @@ LaunchScope::LaunchScope(const char *name, cudaStream_t stream)
         cudaEventRecord(start_, stream_);
     }
 }
+
+bool profiling() { return g_profile_on.load(std::memory_order_relaxed) != 0; }
 
 LaunchScope::~LaunchScope() {
     if (!timed_) return;

@@ -89,6 +89,44 @@ def test_csr_values_off_alignment(nacho, oracle, total, shift):
     assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
 
 
+RESIDENT, OWN_CUTS_UP_TO = 592, 8192  # tiles that all find their cuts themselves; tiles beyond which a launch in front of the merge makes them
+LARGE_STEP = 256 * 31 - 1
+
+
+@pytest.mark.parametrize("total", [RESIDENT * SMALL_STEP, RESIDENT * SMALL_STEP + 1, 5_999_999, OWN_CUTS_UP_TO * LARGE_STEP, OWN_CUTS_UP_TO * LARGE_STEP + 1])
+def test_cuts_of_many_tiles(nacho, oracle, total):
+    """As many tiles as are at work at once and one more, and as many as have no launch in front of them and one more, on a stream of their
+    own each: what the calls there keep starts with the smallest, and has to grow inside the chain of a three-operand sum."""
+    import torch
+    rows, cols = total // 50 + 1, 1 << 16
+    rng = np.random.default_rng(total)
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+        if total < 6_000_000:
+            assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, ga)), oracle.csr_add_3(a, b, a, 8), "add_3")
+        assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+        assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+
+
+def test_pieces_of_many_calls(nacho):
+    """More reductions than control blocks are kept for, of one tile, of few and of many: each begins from nothing."""
+    import torch
+    rng = np.random.default_rng(3)
+    dims = (2000, 300, 200)
+
+    def tensor(n):
+        key = np.unique(rng.integers(0, dims[0] * dims[1] * dims[2], n))
+        c = np.stack([key // 60000, key // 200 % 300, key % 200], axis=1).astype(np.int32)
+        return nacho.to_coo3(c, np.ones(len(key), np.float32), dims, "cuda"), len(key)
+
+    operands = [tensor(n) for n in (500, 20_000, 400_000, 3_000_000)]
+    got = [nacho.gpu_inner_prod_coo_f32(t, t).values for _ in range(6) for t, _ in operands]
+    torch.cuda.synchronize()
+    assert [float(v.cpu()[0]) for v in got] == [float(n) for _ in range(6) for _, n in operands]  # sums of ones: exact in double, and below 2^24
+
+
 @pytest.mark.parametrize("gap", [3000, 1_200_000])
 def test_runs_of_empty_rows(nacho, oracle, gap):
     """More tiles than fit the chip at once, with more rows between two of them than a tile keeps offsets of, empty but for a few: what a tile
