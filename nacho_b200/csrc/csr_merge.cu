@@ -182,9 +182,9 @@ struct TilePlan {
 };
 constexpr uint32_t ROW_FAR = 0xffffu;
 
-// A tile asks for what one that starts a few microseconds later waits for first, so that it lies in L2 by then: the row offsets, which are read by plain loads, a
-// few dependent rounds of them (trees of 25 M entries per operand 384 -> 371 us), or in the large tile of a merge with a launch in front, the
-// longest ones, the columns (67 M entries 394 -> 386 us a call, product of 50 M 233 -> 230; merges of fewer tiles lose up to 0.5 %). Not for a tile that starts with the
+// A tile, other than the large one, asks for the row offsets of one that starts a few microseconds later, so that they wait in L2:
+// they are read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns
+// ahead as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.) Not for a tile that starts with the
 // first ones, and at most as many offsets as a tile keeps: beyond those lie runs of empty rows, which could fill the L2.
 constexpr int TILES_AHEAD = 148;
 // Tiles up to which a call that waits for its length is one launch. Two operands of 24, 32, 40 and 50 M entries (6050, 8070, 10090 and 12610 tiles) take
@@ -802,16 +802,10 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
     } else if (cuts.at) {
         const int4 c0 = cuts.at[t], c1 = cuts.at[t + 1];
         tile = TileRange{c0.x, c1.x, c0.y, c0.z, c1.y - c0.y, c1.z - c0.z};
-        if (threadIdx.x == 96 && t + TILES_AHEAD >= RESIDENT && t + TILES_AHEAD < num_tiles) {
-            const int4 from = cuts.at[t + TILES_AHEAD], to = cuts.at[t + TILES_AHEAD + 1];
-            if (V == V_MOST) {
-                prefetch_l2(A.col + from.y, to.y - from.y);
-                prefetch_l2(B.col + from.z, to.z - from.z);
-            } else {
-                const int32_t n = min(to.x - from.x, TilePlan<V, LEVELS>::ROWS) + 1;
-                if (A.rp) prefetch_l2(A.rp + from.x, n);
-                if (B.rp) prefetch_l2(B.rp + from.x, n);
-            }
+        if (V != V_MOST && threadIdx.x == 96 && t + TILES_AHEAD >= RESIDENT && t + TILES_AHEAD < num_tiles) {
+            const int32_t r0 = cuts.at[t + TILES_AHEAD].x, n = min(cuts.at[t + TILES_AHEAD + 1].x - r0, TilePlan<V, LEVELS>::ROWS) + 1;
+            if (A.rp) prefetch_l2(A.rp + r0, n);
+            if (B.rp) prefetch_l2(B.rp + r0, n);
         }
     } else {
         const int32_t rows = row_count.get();
