@@ -748,13 +748,15 @@ int bits_for(int32_t extent) {
     return b;
 }
 
-// Merged entries per worker thread: large tiles amortise the searches and the wait for the earlier counts, small
-// ones fill the chip when there are few entries. 100 M entries per operand, tile kernel: 1257 us with 13, 1195
-// with 17 (52 KB of shared memory: the most of which four CTAs fit an SM), 1331 with 19.
-constexpr int V_LARGE = 17, V_SMALL = 7;
-constexpr int64_t LARGE_FROM = 3000000;
-constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
 constexpr int tile_step_of(int v) { return NT * v - 1; }  // a twin may add one entry
+
+// Merged entries per worker thread: large tiles amortise the searches and the wait for the earlier counts, small
+// ones fill the chip when there are few entries, up to the number that can be at work at once (as in the CSR kernel). 100 M entries per operand, tile kernel: 1257 us with 13, 1195
+// with 17 (52 KB of shared memory: the most of which four CTAs fit an SM), 1331 with 19. Sums of 0.4, 0.6, 1, 1.3 M entries per
+// operand, whole call: 21.9, 32.2, 41.3, 48.2 us with 7, 21.3, 25.4, 39.7, 44.8 with 11, 32.4 and 42.4 the latter two with 17. A reduction has nothing
+// but the merge behind the staging: 0.1, 0.3, 0.6, 1 M 17.5, 18.6, 24.0, 31.5 with 7, 18.2, 18.9, 20.3, 29.1 with 11, 21.6 and 26.9 the latter two with 17.
+constexpr int V_LARGE = 17, V_SMALL = 11, V_REDUCE = 7;
+constexpr int tile_v(int64_t total, int small = V_SMALL) { return total > (int64_t)RESIDENT * tile_step_of(small) ? V_LARGE : small; }
 
 template <int VT, int MODE>
 cudaError_t launch_coo3_tile_v(const Coo3In &A, const Coo3In &B, const Packing &pk, const Cuts2 &cuts, int32_t *tile_count, const TileWords &words,
@@ -781,8 +783,9 @@ cudaError_t launch_coo3_tile(const Coo3In &A, const Coo3In &B, const Packing &pk
                              FusedCtl *ctl, const Coo3Out &Z, int num_tiles, int v, cudaStream_t stream) {
     static const char *const names[4] = {"coo3_add_count", "coo3_add_fill", "coo3_add_fused", "coo3_inner_prod"};
     LaunchScope scope(names[MODE], stream);
+    constexpr int SMALL = MODE == MODE_REDUCE ? V_REDUCE : V_SMALL;
     return v == V_LARGE ? launch_coo3_tile_v<V_LARGE, MODE>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles, stream)
-                        : launch_coo3_tile_v<V_SMALL, MODE>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles, stream);
+                        : launch_coo3_tile_v<SMALL, MODE>(A, B, pk, cuts, tile_count, words, ctl, Z, num_tiles, stream);
 }
 
 // Queues the cuts; `zero_words` words of control block and tile words are cleared on the way. Up to about a wave of
@@ -822,7 +825,7 @@ int check_coo3(const nb200_coo3 *t) {
 // coo3_add_scratch_bytes() bytes; result words and copies go to the pinned slots of `ws`); the CSF3 kernels use
 // this to keep their own temporaries and this function's in one pool block.
 // (Both sized for the smallest tile of the kernels here, an upper bound for the others.)
-static_assert(WCAP - 1 <= tile_step_of(V_SMALL), "scratch is sized for the smallest tile");
+static_assert(WCAP - 1 <= tile_step_of(V_REDUCE), "scratch is sized for the smallest tile");
 int64_t coo3_add_tiles(int64_t total_entries) { return (total_entries + (WCAP - 1) - 1) / (WCAP - 1); }
 
 size_t coo3_add_scratch_bytes(int64_t total_entries) {
@@ -977,7 +980,7 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
     if (bi + bj + bk > 63) return NB200_E_UNSUPPORTED;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    const int v = tile_v(total), tile_step = tile_step_of(v);
+    const int v = tile_v(total, V_REDUCE), tile_step = tile_step_of(v);
     const int64_t tiles64 = (total + tile_step - 1) / tile_step;
     if (tiles64 > INT32_MAX - 1) return NB200_E_OVERFLOW;
     const int num_tiles = (int)tiles64;

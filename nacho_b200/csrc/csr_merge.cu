@@ -830,16 +830,18 @@ __global__ void __launch_bounds__(NT, 4) k_csr2_tile(const __grid_constant__ Csr
 
 // ------------------------------------------------------------------------ host driver ----
 
-// Merged entries per worker thread. Large tiles amortise what a tile costs whatever its size (searches,
-// barriers, the wait for the earlier counts): 64 M entries per operand take 471 us with 31, 477 with 27, 526
-// with 15, 638 with 11. With fewer than about 750 large tiles the chip (592 resident ones) is better filled by
-// small ones: 2 M merged entries 22.8 us with 15 against 24.9, 0.8 M 15.8 against 18.9; at 6 M the two are even.
+constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between two tile cuts (a twin may add one)
+
+// Merged entries per worker thread. Large tiles amortise what a tile costs whatever its size (searches, barriers, the wait for the
+// earlier counts): 64 M entries per operand take 397 us with 31, 403 with 29, 407 with 27. Small ones fill the chip where there are few entries: 2 M
+// merged entries 20.9 us with 15, 25.0 with 11. They give way where they are more than can be at work at once: a second wave of
+// them costs more than places that stay empty in one of large tiles. Sums of 1.2, 1.5, 2, 2.6 M entries per operand 26.7, 30.7, 35.0, 41.1 us with
+// 15 and 23.0, 26.5, 31.2, 38.3 with 31, products of 1.3 and 2.3 M 25.0, 34.3 and 21.4, 27.9, trees of 1.5 M 66.4 and 60.9.
 // Both are odd: a thread's shares of A and B then start at odd word distances from its neighbour's where
 // rows alternate evenly, and the shared-memory banks are hit evenly (16 took twice the time of 18).
 constexpr int V_LARGE = V_MOST, V_SMALL = 15;
-constexpr int64_t LARGE_FROM = 6000000;
+constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1;
 constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
-constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between two tile cuts (a twin may add one)
 
 // Raises the tile kernel's dynamic shared-memory limit once per instantiation and device.
 template <int V, int OP, int MODE, bool LEVELS = false, bool OWN = false>

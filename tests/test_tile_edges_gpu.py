@@ -167,6 +167,12 @@ def test_coordinate_tiles(nacho, oracle, total, dims):
     assert abs(got - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30  # float32 products, 2^-24 each, summed wider
 
 
+@pytest.mark.parametrize("total", [592 * (256 * v - 1) + more for v in (7, 11, 17) for more in (0, 1)])
+def test_coordinate_tiles_of_one_wave(nacho, oracle, total):
+    """As many tiles of every size as are at work at once, and one entry more: there reductions, then sums, take larger ones, and then a launch for their cuts."""
+    test_coordinate_tiles(nacho, oracle, total, (1 << 9, 1 << 10, 1 << 11))
+
+
 @pytest.mark.parametrize("total", [9, COO_STEP - 2, 2 * COO_STEP + 5, 3_000_011])
 @pytest.mark.parametrize("shift", [(0, 1), (1, 0), (2, 3)])
 def test_coordinate_values_off_alignment(nacho, oracle, total, shift):
