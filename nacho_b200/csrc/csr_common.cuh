@@ -82,7 +82,7 @@ constexpr long long RW_HOLLOW = 1ll << 48;  // beside the length in a result wor
 
 // Test knobs of a launch: the first tile to run (a self-test of the bounded waits leaves tile 0
 // out, so that every other tile waits for a count that never comes) and the number of polls after
-// which a tile gives up on its output base; where tile 0 is left out, the CTA that hands out the bases too.
+// which a tile gives up on a cut or on its output base.
 struct LaunchKnobs {
     int first_tile = 0;
     int poll_limit = LOOKBACK_POLL_LIMIT;
@@ -91,7 +91,7 @@ constexpr int64_t SELFTEST_ENTRIES = 24000;  // three tiles, of whatever size: e
 
 // One single-pass merge as part of a longer call: the partition and the tile kernel are queued and nothing
 // is waited for. `scratch` holds csr2_scratch_bytes(entries) bytes; the control block (length, status) that
-// *ctl then points to lies in it. With `levels` the offsets mode runs (values are not read).
+// *ctl then points to lies in it, or in a block of the stream's that the next three merges there leave alone. With `levels` the offsets mode runs (values are not read).
 size_t csr2_scratch_bytes(int64_t entries);
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl, const LaunchKnobs &knobs = LaunchKnobs());
