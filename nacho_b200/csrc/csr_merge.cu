@@ -204,6 +204,19 @@ struct TileShared {
     int wtotal[NT / 32];            // survivors of each warp
 };
 
+// The last of rows from + 1 .. nr (relative to the tile) that starts at or before an entry, by bisection of the row offsets. A call,
+// because a merge with 64-bit keys has it twice in each of its steps, up to 62 times in a kernel: with the loop in every place such a
+// kernel waited for its instructions more than for anything else (9.8 of 18 stalled warps for each that issues, a third of the slots
+// used; beside the larger second half of a tile a sum of 33 M entries in columns beyond 2^30 went from 524 to 747 us a call; so 400).
+__device__ __noinline__ int far_row(const int32_t *rp, const int32_t entry, const int from, const int nr) {
+    int r = from + 1, top = nr;
+    while (r < top) {
+        const int mid = (r + top + 1) >> 1;
+        if (ld_late(rp + mid) <= entry) r = mid; else top = mid - 1;
+    }
+    return r;
+}
+
 // The tile body. Keys order entries by (row in tile, column):
 //   narrow  32 bits, (row << cbits) | column. A staged word is a column; the first entry of a row also
 //           carries, above the column bits, how many rows begin there, so that the key after key k of the
@@ -385,12 +398,7 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     auto marked_row = [&](const int at, const int pos, const int from, const int shift) -> int {
         const uint32_t mark = row_mark[at];
         if (mark != ROW_FAR) return (int)mark;
-        int r = from + 1, top = nr;
-        while (r < top) {  // the last row that starts at or before pos
-            const int mid = (r + top + 1) >> 1;
-            if ((int)((row_start(mid) >> shift) & 0xffffu) <= pos) r = mid; else top = mid - 1;
-        }
-        return r;
+        return shift ? far_row(B.rp + tile.i0, tile.b0 + pos, from, nr) : far_row(A.rp + tile.i0, tile.a0 + pos, from, nr);
     };
     {
         row = (int)warp_incl_max((unsigned)s_trow[tid]);

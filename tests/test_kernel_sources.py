@@ -15,6 +15,16 @@ def parameters(text, kernel):
     return re.search(re.escape(kernel) + r"\(([^{;]*)\)\s*\{", text).group(1)
 
 
+def test_steps_of_an_unrolled_merge_hold_no_loops():
+    """What a step of a tile's merge holds is in its kernel once for every entry of a thread, for both operands. With a search there the
+    kernels of 64-bit keys wait for their instructions: the search is a call."""
+    text = source("csr_merge.cu")
+    assert re.search(r"__noinline__\s+int\s+far_row\(", text)
+    body = text[text.index("auto marked_row = "):]
+    body = body[:body.index("};")]
+    assert "far_row(" in body and not re.search(r"\b(for|while|do)\b", body)
+
+
 def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():
     """A kernel that starts beside the one in front of it must not use read-only loads (ld.global.nc, or a const
     __restrict__ parameter that the compiler turns into one) for what that kernel writes: they may be issued before the
