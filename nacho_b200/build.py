@@ -9,6 +9,7 @@ from __future__ import annotations
 import concurrent.futures as cf
 import glob
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -52,6 +53,17 @@ def _read(path: str) -> str | None:
         return f.read()
 
 
+def _report(obj: str) -> str:
+    return obj[:-2] + ".ptxas.txt"
+
+
+def spills(name: str) -> dict[str, tuple[int, int]]:
+    """Bytes of spill stores and loads of every device function of ``csrc/<name>.cu``, by mangled name, as ptxas reported them."""
+    text = _read(_report(os.path.join(OBJ_DIR, name + ".o"))) or ""
+    found = re.findall(r"Function properties for (\S+)\n\s*\d+ bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads", text)
+    return {f: (int(stores), int(loads)) for f, stores, loads in found}
+
+
 def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -63,18 +75,19 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     for src in sources:
         obj = os.path.join(OBJ_DIR, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
-        if _stale(obj, [src] + headers):
-            cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", src, "-o", obj]
-            jobs.append(cmd)
+        if _stale(obj, [src] + headers) or not os.path.exists(_report(obj)):
+            jobs.append([nvcc] + NVCC_FLAGS + ["-Xptxas", "-v", "-c", src, "-o", obj])
 
     def run(cmd):
         r = subprocess.run(cmd, capture_output=True, text=True)
+        with open(_report(cmd[-1]), "w") as f:
+            f.write(r.stderr)
         return cmd, r
 
     with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         for cmd, r in ex.map(run, jobs):
             if verbose or ptxas_info or r.returncode != 0:
-                sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+                sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + (r.stderr if ptxas_info or r.returncode != 0 else ""))
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed for {cmd[-3]}")
     if jobs or _stale(LIB, objs):

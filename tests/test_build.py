@@ -1,5 +1,6 @@
-"""CPU suite: when the Python operators are built again, and what is built without a torch."""
+"""CPU suite: when the Python operators are built again, what is built without a torch, and what the compiler says of the kernels."""
 import os
+import re
 import subprocess
 import sys
 
@@ -43,3 +44,12 @@ def test_without_torch_the_library_is_built(commands, monkeypatch, capsys):
     monkeypatch.setitem(sys.modules, "torch", None)
     assert build.build_native(build._nvcc()) is None
     assert not commands and "torch is not installed" in capsys.readouterr().err
+
+
+def test_fills_of_large_tiles_stay_in_registers():
+    """Tiles that fill a room of the result's own length, four CTAs of 64 registers a thread to an SM, hold at most some words more: with
+    the columns of all results at once they spilled 80 bytes a thread (220 beside 64-bit keys) and lost what copying the values gains."""
+    build.build()
+    found = {name: bytes_ for name, bytes_ in build.spills("csr_merge").items() if re.search(r"csr2_tile(_wide)?ILi31ELi0ELi1ELb0E", name)}
+    assert len(found) == 2  # 32- and 64-bit keys
+    assert all(max(b) <= 64 for b in found.values()), found
