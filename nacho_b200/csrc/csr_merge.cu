@@ -860,8 +860,23 @@ constexpr int tile_step(int v) { return NT * v - 1; }  // merged entries between
 // Both are odd: a thread's shares of A and B then start at odd word distances from its neighbour's where
 // rows alternate evenly, and the shared-memory banks are hit evenly (16 took twice the time of 18).
 constexpr int V_LARGE = V_MOST, V_SMALL = 15;
-constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1;
-constexpr int tile_v(int64_t total) { return total >= LARGE_FROM ? V_LARGE : V_SMALL; }
+constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1, LARGE_ALWAYS_FROM = 6000000;
+// Up to LARGE_ALWAYS_FROM entries they stay small for two kinds of merge, whose large tiles take longer for an entry:
+//   - many rows. A large tile that more rows begin in than it keeps reads their offsets from L2 three times; a small one keeps more than
+//     twice as many. While all large tiles are at work at once that weighs less than the second wave of small ones, up to about twice
+//     the rows that are kept: sums of 2 M entries per operand in 1.4, 2, 4 and 8 M rows 41.1, 42.8, 56.1, 109 us with small tiles,
+//     40.5, 47.4, 74.8, 127 with large ones; of 2.7 M (two waves of large ones) in 1.1, 1.3, 2.7, 5.4 M rows 45.4, 46.0, 55.1, 74.3 and 44.4, 52.1, 70.7,
+//     111.7. Rows that are hardly ever filled, 80 M for 2 M entries: 1057 and 1170.
+//   - columns beyond 2^30, whose keys have 64 bits: a second wave of large tiles costs more than the waves of small ones. Sums of 2, 2.9 M
+//     entries per operand 38.1, 50.7 us with small tiles, 40.3, 75.1 with large ones, products 33.8, 42.5 and 31.0, 43.0.
+// `rows` is 0 where only the device knows it.
+inline int tile_v(int64_t total, int64_t rows, int32_t cols) {
+    if (total < LARGE_FROM) return V_SMALL;
+    if (total >= LARGE_ALWAYS_FROM) return V_LARGE;
+    const bool one_wave = total <= (int64_t)RESIDENT * tile_step(V_LARGE);
+    if (col_bits(cols) > 30 && !one_wave) return V_SMALL;
+    return rows * tile_step(V_LARGE) > (one_wave ? 2 : 1) * TilePlan<V_LARGE, false>::ROWS * total ? V_SMALL : V_LARGE;
+}
 
 // Raises the tile kernel's dynamic shared-memory limit once per instantiation and device.
 template <int V, int OP, int MODE, bool LEVELS = false, bool OWN = false>
@@ -941,7 +956,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
     const int32_t rows = a->rows;
     const RowCount row_count{rows};
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    const int v = tile_v(total), step = tile_step(v);
+    const int v = tile_v(total, rows, a->cols), step = tile_step(v);
     const int64_t tiles64 = (total + step - 1) / step;
     if (tiles64 > INT32_MAX - 1) return NB200_E_OVERFLOW;
     const int num_tiles = (int)tiles64;
@@ -1100,7 +1115,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
 // (so every GPU that loads the library holds these bytes until the process exits).
 constexpr int64_t NOALLOC_MAX_ENTRIES = 159350784;
 constexpr int NOALLOC_MAX_TILES = (int)(NOALLOC_MAX_ENTRIES / tile_step(V_LARGE)) + 1;
-static_assert(LARGE_FROM / tile_step(V_SMALL) + 1 <= NOALLOC_MAX_TILES, "small tiles must fit the scratch too");
+static_assert(LARGE_ALWAYS_FROM / tile_step(V_SMALL) + 1 <= NOALLOC_MAX_TILES, "small tiles must fit the scratch too");
 constexpr size_t NOALLOC_SCRATCH_BYTES = 1u << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
@@ -1135,7 +1150,7 @@ int csr_add_noalloc(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, int64_
     const int32_t rows = a->rows;
     const RowCount row_count{rows};
     const int64_t total = (int64_t)a->nnz + b->nnz;
-    const int v = tile_v(total), step = tile_step(v);
+    const int v = tile_v(total, rows, a->cols), step = tile_step(v);
     const int64_t tiles64 = (total + step - 1) / step;
     if (total > NOALLOC_MAX_ENTRIES) return NB200_E_UNSUPPORTED;
     if (capacity < total) return NB200_E_CAPACITY;  // this entry point has the single-pass route only
@@ -1191,7 +1206,8 @@ size_t csr2_scratch_bytes(int64_t entries) {
 int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows, int32_t cols, const CsrOut &Z, const LevelOffsets *levels,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl_out, const LaunchKnobs &knobs) {
     const int64_t total = (int64_t)A.nnz + B.nnz;
-    const int v = tile_v(total) == V_SMALL ? V_SMALL : levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE, step = tile_step(v);
+    const int large = levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE;
+    const int v = total < LARGE_FROM ? V_SMALL : large == V_LARGE ? tile_v(total, rows.dev ? 0 : rows.value, cols) : large, step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
     Carver carve(scratch);
     Cuts cuts;

@@ -110,6 +110,21 @@ def test_cuts_of_many_tiles(nacho, oracle, total):
         assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
 
 
+@pytest.mark.parametrize("total,rows,cols", [(t, (waves * 1856 * t) // LARGE_STEP + more, 1 << 13) for t, waves in ((RESIDENT * SMALL_STEP + 1, 2), (RESIDENT * LARGE_STEP, 2),
+                                                                                                                  (RESIDENT * LARGE_STEP + 1, 1)) for more in (0, 1)]
+                         + [(RESIDENT * LARGE_STEP + more, 1 << 12, (1 << 30) + wide) for more, wide in ((0, 1), (1, 0), (1, 1))])
+def test_rows_and_columns_that_keep_tiles_small(nacho, oracle, total, rows, cols):
+    """Merges on either side of the lines up to which many rows, and columns beyond 2^30, are merged in small tiles, more of them than are at
+    work at once."""
+    rng = np.random.default_rng(total + rows)
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, ga)), oracle.csr_add_3(a, b, a, 8), "add_3")
+
+
 def test_pieces_of_many_calls(nacho):
     """More reductions than control blocks are kept for, of one tile, of few and of many: each begins from nothing."""
     import torch
