@@ -897,11 +897,12 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
             if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
         }
     }
-    const bool tagged = fused && !wide && num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    bool tagged = fused && !wide && num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    OwnWords own;
+    if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return fail(st);
     if (tagged) {
-        cuts = Cuts2{nullptr, nullptr, tile_step};
-        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return fail(st);
-        ctl = cuts.own.ctl, words = cuts.own.words;
+        cuts = Cuts2{nullptr, nullptr, tile_step, own};
+        ctl = own.ctl, words = own.words;
     } else if (num_tiles == 1 && fused && !wide) {
         cuts = Cuts2{};  // one tile: no cut to search, and the tile kernel clears the control block itself
     } else {
@@ -1000,11 +1001,12 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(block);
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     cudaError_t e = cudaSuccess;
-    const bool tagged = num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    bool tagged = num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    OwnWords own;
+    if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return st;
     if (tagged) {
-        cuts = Cuts2{nullptr, nullptr, tile_step};
-        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return st;
-        ctl = cuts.own.ctl;
+        cuts = Cuts2{nullptr, nullptr, tile_step, own};
+        ctl = own.ctl;
     } else if (num_tiles == 1) cuts = Cuts2{};
     else e = launch_coo3_partition(A, B, total, tile_step, num_tiles, cuts, block, 4, stream);
     if (e != cudaSuccess) return note_cuda_error(e, "k_coo3_partition");

@@ -1027,11 +1027,12 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
         if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&z->val), sizeof(float) * (size_t)bound, stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
     }
-    const bool tagged = fused && !device_result && num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    bool tagged = fused && !device_result && num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    OwnWords own;
+    if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return fail(st);
     if (tagged) {
-        cuts = Cuts{nullptr, step};
-        if ((st = take_own_words(stream, num_tiles, &cuts.own))) return fail(st);
-        ctl = cuts.own.ctl, words = cuts.own.words;
+        cuts = Cuts{nullptr, step, own};
+        ctl = own.ctl, words = own.words;
     } else if (num_tiles == 1) {
         cuts.at = nullptr;  // one tile: no cut to search, and the tile kernel clears the control block itself
     } else {
@@ -1217,12 +1218,13 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
     TileWords words = TileWords::at(fused_block + 4);
     *ctl_out = ctl;
     cudaError_t e = cudaSuccess;
-    const bool tagged = num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    bool tagged = num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    OwnWords own;
+    const int st = take_own_words(stream, num_tiles, &tagged, &own);
+    if (st != NB200_OK) return st;
     if (tagged) {
-        cuts = Cuts{nullptr, step};
-        const int st = take_own_words(stream, num_tiles, &cuts.own);
-        if (st != NB200_OK) return st;
-        *ctl_out = ctl = cuts.own.ctl, words = cuts.own.words;
+        cuts = Cuts{nullptr, step, own};
+        *ctl_out = ctl = own.ctl, words = own.words;
     } else if (num_tiles == 1) {
         cuts.at = nullptr;
     } else {

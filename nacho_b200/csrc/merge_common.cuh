@@ -129,12 +129,16 @@ struct OwnWords {
     int cutters = 0;          // leading CTAs that make the cuts from first_cut() on
     __host__ __device__ int first_cut() const { return RESIDENT - CUTTERS; }
 };
-inline int take_own_words(cudaStream_t stream, int num_tiles, OwnWords *out) {
+// `wanted` is withdrawn where the device has no room for the words: the call then has the launch for its cuts, whose scratch it holds anyway
+// (and which asynchronous calls on the stream, that may be captured, find there).
+inline int take_own_words(cudaStream_t stream, int num_tiles, bool *wanted, OwnWords *out) {
     static_assert(sizeof(FusedCtl) <= 8 * sizeof(uint64_t), "a control block takes a piece");
+    if (!*wanted) return NB200_OK;
     const bool many = num_tiles > RESIDENT;
     Tagged block;
     const int st = acquire_tagged(stream, many ? 5 * (size_t)num_tiles + 4 : RESIDENT, &block);
-    if (st != NB200_OK) return st;
+    if (st == NB200_E_NOMEM) *wanted = false;
+    if (st != NB200_OK) return *wanted ? st : NB200_OK;
     out->ctl = reinterpret_cast<FusedCtl *>(block.mine);
     out->clear = reinterpret_cast<FusedCtl *>(block.later);
     out->words = TileWords::at(block.words, block.tag);

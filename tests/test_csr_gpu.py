@@ -437,3 +437,59 @@ def test_three_operand_add_by_each_route(nacho, oracle, n_a, n_b, n_c):
     assert_same(CSR(z.rows, z.cols, _d2h(z.row_ptr, z.rows + 1, np.int32), _d2h(z.col, z.nnz, np.int32), _d2h(z.val, z.nnz, np.float32)), want, "allocating")
     for p in (z.row_ptr, z.col, z.val):
         check(lib.nb200_free_async(p, None), "free")
+
+
+@pytest.mark.parametrize("before", ["a merge of a few tiles", "one of a single tile"])
+def test_lent_scratch_is_enough(nacho, before):
+    """A call with scratch of the caller's ends well on a device that has no room for anything more, whatever its stream has merged before."""
+    import torch
+    from nacho_b200 import _capi
+    from nacho_b200._capi import CsrStruct, check, lib
+    rows, cols, n = 60_000, 1 << 16, 3_000_000
+
+    def operand(n):
+        key = torch.unique(torch.randint(0, rows * cols, (n,), device="cuda"))
+        rp = torch.searchsorted(key // cols, torch.arange(rows + 1, device="cuda")).to(torch.int32)
+        return nacho.CSR_gpu(rp, (key % cols).to(torch.int32), torch.rand(key.numel(), device="cuda"), torch.tensor([rows, cols], dtype=torch.int32))
+
+    ops, few = [operand(n) for _ in range(3)], operand(6000 if before == "a merge of a few tiles" else 100)
+    want = nacho.gpu_csr_add_3_f32(*ops)
+    _capi.profile_enable(True)  # loads the kernels of the other route too
+    nacho.gpu_csr_add_3_f32(*ops)
+    _capi.profile_enable(False)
+    capacity = sum(m.values.numel() for m in ops)
+    rp, col = (torch.empty(k, dtype=torch.int32, device="cuda") for k in (rows + 1, capacity))
+    val = torch.empty(capacity, device="cuda")
+    z = CsrStruct(rows, cols, 0, rp.data_ptr(), col.data_ptr(), val.data_ptr())
+    structs = [m._struct() for m in ops]
+    scratch_bytes = lib.nb200_csr_add_3_f32_scratch(*(C.byref(s) for s in structs))
+    scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device="cuda")
+
+    def call(a, b, c):
+        return lib.nb200_csr_add_3_f32_lent(C.byref(a), C.byref(b), C.byref(c), C.byref(z), capacity, scratch.data_ptr(), scratch_bytes, None)
+
+    torch.cuda.synchronize()
+    check(lib.nb200_release_workspaces(), "release")
+    torch.cuda.empty_cache()
+    check(call(*[few._struct()] * 3), "few entries")  # takes what a call needs in host memory
+    torch.cuda.synchronize()
+    rt = C.CDLL("libcudart.so.12")
+    rt.cudaMalloc.argtypes, rt.cudaFree.argtypes = [C.POINTER(C.c_void_p), C.c_size_t], [C.c_void_p]
+    held = []
+    try:
+        for size in (1 << 30, 1 << 26, 1 << 21, 1 << 17, 1 << 14):  # less than the words of 700 tiles and more in one piece are left
+            p = C.c_void_p()
+            while rt.cudaMalloc(C.byref(p), size) == 0:
+                held.append(p.value)
+        rt.cudaGetLastError()
+        status = call(*structs)
+        torch.cuda.synchronize()
+    finally:
+        for p in held:
+            rt.cudaFree(p)
+    check(status, "lent")
+    assert z.nnz == want.values.numel() and torch.equal(rp, want.dim_j_offsets)
+    assert torch.equal(col[:z.nnz], want.dim_j_indices) and torch.equal(val[:z.nnz], want.values)
+    check(call(*structs), "lent, with room")
+    torch.cuda.synchronize()
+    assert z.nnz == want.values.numel() and torch.equal(val[:z.nnz], want.values)
