@@ -13,7 +13,8 @@ entries per operand, uniform rows). Rank 0 prints one JSON line:
              device copies of the operands and a device -> pinned host copy of the result are
              inside the timed region
   roofline   dominant kernel: algorithmic bytes per step / the time the step spends in that
-             kernel (CUDA events on the launching stream), against the measured HBM copy peak
+             kernel (CUDA events on the launching stream, around the launches that the timed steps
+             make too), against the measured HBM copy peak
   cpu_baseline  the reference's own CPU kernels (the C oracle port where the reference has
              none, i.e. SpGEMM) timed on the host cores on a bounded sample of the workload
   ref_gpu_baseline  at N = 1: the reference's own GPU kernels (emitted by its compiler, recompiled
@@ -612,7 +613,7 @@ def main():
     # ---- per-kernel timing, same workload, events on the launching stream
     prof_steps = max(3, min(args.steps, 10))
     _capi.profile_reset()
-    _capi.profile_enable(True)
+    _capi.profile_enable(True, as_called=True)
     for _ in range(prof_steps):
         step()
     finish()

@@ -132,7 +132,10 @@ uint64_t nb200_launch_count(void);
 /* Per-kernel device timing. While enabled, every kernel launch of the library is bracketed
  * by CUDA events on its stream. nb200_profile_read synchronises those events and reports,
  * for the kernel called `name`, the launches and their summed duration since the last
- * nb200_profile_reset; nb200_profile_names writes a comma-separated list of kernel names. */
+ * nb200_profile_reset; nb200_profile_names writes a comma-separated list of kernel names.
+ * `on`: 0 ends it. 2 times the launches that calls make anyway. 1 (or any other value) times merges
+ * that find their tile cuts themselves (calls that wait for their result, of up to about 65 million
+ * entries) as two launches, the search for the cuts and the merge proper: more than such a call takes. */
 int nb200_profile_enable(int on);
 int nb200_profile_reset(void);
 int nb200_profile_read(const char *name, int64_t *launches, double *total_ms);

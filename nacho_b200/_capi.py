@@ -142,8 +142,10 @@ def launch_count() -> int:
     return int(lib.nb200_launch_count())
 
 
-def profile_enable(on: bool) -> None:
-    check(lib.nb200_profile_enable(1 if on else 0), "nb200_profile_enable")
+def profile_enable(on: bool, as_called: bool = False) -> None:
+    """Times every launch from here on: those that calls make anyway (``as_called``), or with the searches for the tile cuts of a merge
+    in a launch of their own."""
+    check(lib.nb200_profile_enable((2 if as_called else 1) if on else 0), "nb200_profile_enable")
 
 
 def profile_reset() -> None:

@@ -121,8 +121,8 @@ private:
     bool timed_;
 };
 
-// Whether launches are being timed.
-bool profiling();
+// Whether launches are being timed in which the searches for the cuts are to show apart from the merge.
+bool profiling_apart();
 
 // Launches `kernel` so that its CTAs may take their places while the kernel before it on the stream still
 // runs (programmatic dependent launch; that kernel says when, with trigger_dependents). A kernel that reads

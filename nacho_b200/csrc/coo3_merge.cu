@@ -897,7 +897,7 @@ int coo3_add_run(const nb200_coo3 *a, const nb200_coo3 *b, nb200_coo3 *z, bool a
             if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
         }
     }
-    bool tagged = fused && !wide && num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    bool tagged = fused && !wide && num_tiles > 1 && num_tiles <= RESIDENT && !profiling_apart();
     OwnWords own;
     if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return fail(st);
     if (tagged) {
@@ -1001,7 +1001,7 @@ int coo3_inner_run(const nb200_coo3 *a, const nb200_coo3 *b, float *z, void *str
     FusedCtl *ctl = reinterpret_cast<FusedCtl *>(block);
     const Coo3In A{a->i, a->j, a->k, a->val, a->nnz}, B{b->i, b->j, b->k, b->val, b->nnz};
     cudaError_t e = cudaSuccess;
-    bool tagged = num_tiles > 1 && num_tiles <= RESIDENT && !profiling();
+    bool tagged = num_tiles > 1 && num_tiles <= RESIDENT && !profiling_apart();
     OwnWords own;
     if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return st;
     if (tagged) {

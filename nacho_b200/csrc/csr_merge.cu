@@ -1027,7 +1027,7 @@ int csr2_run(const nb200_csr *a, const nb200_csr *b, nb200_csr *z, bool alloc, i
         if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void **>(&z->val), sizeof(float) * (size_t)bound, stream);
         if (e != cudaSuccess) return fail(note_cuda_error(e, "cudaMallocAsync"));
     }
-    bool tagged = fused && !device_result && num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    bool tagged = fused && !device_result && num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling_apart();
     OwnWords own;
     if ((st = take_own_words(stream, num_tiles, &tagged, &own))) return fail(st);
     if (tagged) {
@@ -1218,7 +1218,7 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
     TileWords words = TileWords::at(fused_block + 4);
     *ctl_out = ctl;
     cudaError_t e = cudaSuccess;
-    bool tagged = num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling();
+    bool tagged = num_tiles > 1 && num_tiles <= OWN_CUTS_UP_TO && !profiling_apart();
     OwnWords own;
     const int st = take_own_words(stream, num_tiles, &tagged, &own);
     if (st != NB200_OK) return st;

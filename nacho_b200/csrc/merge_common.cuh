@@ -116,7 +116,7 @@ __device__ __forceinline__ int64_t tile_base(const TileWords &words, const int t
 // the start (four CTAs on each of 148 SMs), search for both of their cuts before anything else. For all others a few CTAs in front of
 // the tiles make the cuts, in order and faster than tiles end, and leave them in tagged words. A launch in front of the merge makes all cuts
 // before the first tile begins; the other routes keep it (asynchronous calls, whose launches may be captured and run again; counts before a
-// fill; a profiled call, which is to tell the searches from the merge). us a call, with that launch and without: sums of 10900 entries per operand
+// fill; a call profiled with 1, which is to tell the searches from the merge). us a call, with that launch and without: sums of 10900 entries per operand
 // 15.6 and 14.9, 0.5 M 19.1 and 17.7, 3.3 M 44.2 and 40.4, 4.5 M in short rows 66.5 and 57.9; intersection of 16 M 88.5 and 83.5; three operands of 9 M 183 and
 // 176; trees of 100 K 45.8 and 41.8. Coordinate lists have such CTAs nowhere: their probes, of up to six loads far apart, cannot keep up
 // with the tiles (100 M entries per operand 1024 us with the launch, 1341 so), so they stay with RESIDENT tiles (inner product of 300 K entries 20.9 and 18.3).

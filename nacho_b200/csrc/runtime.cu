@@ -186,7 +186,7 @@ LaunchScope::LaunchScope(const char *name, cudaStream_t stream)
     }
 }
 
-bool profiling() { return g_profile_on.load(std::memory_order_relaxed) != 0; }
+bool profiling_apart() { return g_profile_on.load(std::memory_order_relaxed) == 1; }
 
 LaunchScope::~LaunchScope() {
     if (!timed_) return;
@@ -247,7 +247,7 @@ int nb200_release_workspaces(void) {
 uint64_t nb200_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
 int nb200_profile_enable(int on) {
-    g_profile_on.store(on ? 1 : 0, std::memory_order_relaxed);
+    g_profile_on.store(on == 2 ? 2 : on ? 1 : 0, std::memory_order_relaxed);
     return NB200_OK;
 }
 

@@ -348,6 +348,39 @@ def test_launch_counter_and_profile(nacho, csr_golden):
     assert "csr2_partition" in _capi.profile_names()
 
 
+def test_profile_as_called(nacho):
+    """Timed as called, an operator makes the launches that it makes untimed, and every one of them shows."""
+    import torch
+    from nacho_b200 import _capi
+    rng = np.random.default_rng(2)
+    dims = (300, 200, 100)
+
+    def key(n):
+        return np.unique(rng.integers(0, dims[0] * dims[1] * dims[2], n))
+
+    def csr(k):
+        return csr_to_gpu(CSR(60_000, 100, np.searchsorted(k // 100, np.arange(60_001)).astype(np.int32), (k % 100).astype(np.int32), np.ones(len(k), np.float32)))
+
+    def coordinates(k):
+        return np.stack([k // 20_000, k // 100 % 200, k % 100], axis=1).astype(np.int32), np.ones(len(k), np.float32), dims, "cuda"
+
+    k = [key(30_000) for _ in range(3)]
+    m, t, f = [csr(x) for x in k], [nacho.to_coo3(*coordinates(x)) for x in k[:2]], [nacho.to_csf3(*coordinates(x)) for x in k[:2]]
+    for call in (lambda: nacho.gpu_csr_add_f32(*m[:2]), lambda: nacho.gpu_csr_mul_f32(*m[:2]), lambda: nacho.gpu_csr_add_3_f32(*m), lambda: nacho.gpu_coo3d_add_f32(*t),
+                 lambda: nacho.gpu_inner_prod_coo_f32(*t), lambda: nacho.gpu_csf_add_f32(*f)):
+        counts = []
+        for timed in (False, True):
+            before = _capi.launch_count()
+            _capi.profile_reset()
+            _capi.profile_enable(timed, as_called=True)
+            call()
+            torch.cuda.synchronize()
+            _capi.profile_enable(False)
+            counts.append(_capi.launch_count() - before)
+        assert counts[0] == counts[1] == sum(_capi.profile_read(name)[0] for name in _capi.profile_names())
+        assert all(_capi.profile_read(name)[0] == 0 for name in ("csr2_partition", "coo3_partition"))
+
+
 @pytest.mark.parametrize("op", ["add", "mul"])
 def test_host_streaming_entry_points(nacho, oracle, op):
     """Host-resident operands streamed through the GPU in row blocks (several blocks here)."""
