@@ -72,7 +72,7 @@ inline int check_csr(const nb200_csr *m, bool need_arrays) {
 
 // A row count that a call knows (`dev` null) or that an earlier launch on the stream leaves in device memory.
 struct RowCount {
-    int32_t value = 0;
+    int32_t value = 0;  // beside `dev`: the most there can be (0: unknown; chooses the tile, nothing else)
     const long long *dev = nullptr;
     bool short_rows = false;  // rows of a few dozen entries or less (chooses the tile, nothing else)
     __device__ __forceinline__ int32_t get() const { return dev ? (int32_t)*dev : value; }

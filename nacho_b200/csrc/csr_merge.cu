@@ -869,7 +869,8 @@ constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1, LARGE
 //     111.7. Rows that are hardly ever filled, 80 M for 2 M entries: 1057 and 1170.
 //   - columns beyond 2^30, whose keys have 64 bits: a second wave of large tiles costs more than the waves of small ones. Sums of 2, 2.9 M
 //     entries per operand 38.1, 50.7 us with small tiles, 40.3, 75.1 with large ones, products 33.8, 42.5 and 31.0, 43.0.
-// `rows` is 0 where only the device knows it.
+// `rows` is the most there can be where only the device knows how many (row lists; sums of 1.3, 1.9, 2.5, 2.95 M entries per operand in as many rows: 51, 60, 75, 85 us with
+// small tiles, 78, 91, 134, 145 with large ones), 0 if the call does not know that either.
 inline int tile_v(int64_t total, int64_t rows, int32_t cols) {
     if (total < LARGE_FROM) return V_SMALL;
     if (total >= LARGE_ALWAYS_FROM) return V_LARGE;
@@ -1208,7 +1209,7 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl_out, const LaunchKnobs &knobs) {
     const int64_t total = (int64_t)A.nnz + B.nnz;
     const int large = levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE;
-    const int v = total < LARGE_FROM ? V_SMALL : large == V_LARGE ? tile_v(total, rows.dev ? 0 : rows.value, cols) : large, step = tile_step(v);
+    const int v = total < LARGE_FROM ? V_SMALL : large == V_LARGE ? tile_v(total, rows.value, cols) : large, step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
     Carver carve(scratch);
     Cuts cuts;

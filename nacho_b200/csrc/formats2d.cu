@@ -240,7 +240,7 @@ int dcsr2_run(csr_into_fn op, bool is_union, const nb200_dcsr *a, const nb200_dc
     const bool one_pass = capacity >= (is_union ? total : std::min<int64_t>(a->nnz, b->nnz));
     bool hollow = false;
     if (one_pass) {
-        if ((st = csr2_enqueue(is_union ? OP_UNION : OP_INTERSECT, A, B, RowCount{0, &rows_ctl->total}, a->cols,
+        if ((st = csr2_enqueue(is_union ? OP_UNION : OP_INTERSECT, A, B, RowCount{(int32_t)std::min<int64_t>(stored, a->rows), &rows_ctl->total}, a->cols,
                                CsrOut{result_rp, z->j_idx, z->val, nullptr, length_word, rows_ctl}, nullptr, entry_scratch, stream, &ctl)))
             return st;
     }

@@ -25,6 +25,15 @@ def test_steps_of_an_unrolled_merge_hold_no_loops():
     assert "far_row(" in body and not re.search(r"\b(for|while|do)\b", body)
 
 
+def test_the_choice_of_tiles_knows_the_rows_of_row_lists():
+    """Only the device knows how many rows two row lists have together, the call knows the most there can be: large tiles lose to small ones
+    where rows hold an entry, so it has to say."""
+    merges = re.findall(r"csr2_enqueue\((.*?)\)\)\)?\s", source("formats2d.cu"), re.S)
+    of_entries = [m for m in merges if "&rows_ctl->total}" in m]
+    assert of_entries and all("RowCount{(int32_t)std::min<int64_t>(stored, a->rows), &rows_ctl->total}" in m for m in of_entries)
+    assert "tile_v(total, rows.value, cols)" in source("csr_merge.cu")
+
+
 def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():
     """A kernel that starts beside the one in front of it must not use read-only loads (ld.global.nc, or a const
     __restrict__ parameter that the compiler turns into one) for what that kernel writes: they may be issued before the

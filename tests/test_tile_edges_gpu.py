@@ -215,6 +215,20 @@ def test_coordinate_values_off_alignment(nacho, oracle, total, shift):
     assert abs(float(nacho.gpu_inner_prod_coo_f32(ga, gb).values.cpu()[0]) - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30
 
 
+@pytest.mark.parametrize("each", [1, 2, 5])
+@pytest.mark.parametrize("total", [RESIDENT * SMALL_STEP + more for more in (0, 1)] + [RESIDENT * LARGE_STEP + more for more in (0, 1)] + [5_999_999, 6_000_000])
+def test_row_lists_on_either_side_of_the_tiles_they_take(nacho, oracle, total, each):
+    """Rows of one entry, of two and of five, in lists whose entries are merged in small tiles and in large ones."""
+    from test_family_gpu import _dcsr_expected, csr_to_dcsr, dcsr_from_gpu, dcsr_to_gpu
+    rows, cols = 4 * total if each == 1 else total // (2 * each), 4000
+    rng = np.random.default_rng(total + each)
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    da, db = dcsr_to_gpu(nacho, csr_to_dcsr(a)), dcsr_to_gpu(nacho, csr_to_dcsr(b))
+    assert_same(dcsr_from_gpu(nacho.gpu_dcsr_add_f32(da, db)), _dcsr_expected(oracle.csr_add(a, b, 8), a, b, False), "dcsr add")
+    assert_same(dcsr_from_gpu(nacho.gpu_dcsr_mul_f32(da, db)), _dcsr_expected(oracle.csr_mul(a, b, 8), a, b, True), "dcsr mul")
+
+
 def test_stored_empty_rows_and_fibres(nacho, oracle):
     """Row lists that hold rows without entries, and trees that hold slices and fibres without any, come out without them."""
     from test_family_gpu import dcsr_from_gpu, dcsr_to_gpu
