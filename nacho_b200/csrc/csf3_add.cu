@@ -312,10 +312,10 @@ int csf_add_levels(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, cuda
     if ((st = csr2_enqueue(OP_UNION, CsrIn{nullptr, a->i_idx, nullptr, a->n_i}, CsrIn{nullptr, b->i_idx, nullptr, b->n_i}, RowCount{1}, a->dims[0],
                            CsrOut{nullptr, z->i_idx, nullptr, nullptr, word[0]}, &slices, scratch_i, stream, &ctl[0], first_knobs)))
         return st;
-    if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{0, &ctl[0]->total}, a->dims[1],
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ja, a->j_idx, nullptr, a->n_j}, CsrIn{jb, b->j_idx, nullptr, b->n_j}, RowCount{(int32_t)std::min<int64_t>(bound_i, a->dims[0]), &ctl[0]->total}, a->dims[1],
                            CsrOut{z->j_ptr, z->j_idx, nullptr, nullptr, word[1], ctl[0]}, &fibres, scratch_j, stream, &ctl[1])))
         return st;
-    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{0, &ctl[1]->total, total < SHORT_FIBRE * bound_j}, a->dims[2],
+    if ((st = csr2_enqueue(OP_UNION, CsrIn{ka, a->k_idx, a->val, a->n_k}, CsrIn{kb, b->k_idx, b->val, b->n_k}, RowCount{(int32_t)std::min<int64_t>(bound_j, (int64_t)a->dims[0] * a->dims[1]), &ctl[1]->total, total < SHORT_FIBRE * bound_j}, a->dims[2],
                            CsrOut{z->k_ptr, z->k_idx, z->val, nullptr, word[2], ctl[1]}, nullptr, scratch_k, stream, &ctl[2])))
         return st;
     int64_t length[3];

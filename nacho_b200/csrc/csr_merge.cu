@@ -867,16 +867,28 @@ constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1, LARGE
 //     the rows that are kept: sums of 2 M entries per operand in 1.4, 2, 4 and 8 M rows 41.1, 42.8, 56.1, 109 us with small tiles,
 //     40.5, 47.4, 74.8, 127 with large ones; of 2.7 M (two waves of large ones) in 1.1, 1.3, 2.7, 5.4 M rows 45.4, 46.0, 55.1, 74.3 and 44.4, 52.1, 70.7,
 //     111.7. Rows that are hardly ever filled, 80 M for 2 M entries: 1057 and 1170.
-//   - columns beyond 2^30, whose keys have 64 bits: a second wave of large tiles costs more than the waves of small ones. Sums of 2, 2.9 M
-//     entries per operand 38.1, 50.7 us with small tiles, 40.3, 75.1 with large ones, products 33.8, 42.5 and 31.0, 43.0.
+//   - keys of 64 bits, for columns beyond 2^30 or so many rows in a tile that their number and a column take more than 31 bits. Where a small
+//     tile gets by with 32 bits it is faster, and beyond one wave of large tiles always. Columns of 20, 22, 25 bits, sums of 1.25 M entries per operand in 0.75, 0.25,
+//     0.025 M rows 30.7, 28.5, 27.0 us with small tiles, 42.3, 35.5, 32.5 with large ones; of 2.95 M (two waves) in 0.6 M rows of 22, 25, 28 bits 43.6, 57.4, 57.6 and 76.6, 73.6, 77.5.
+//     One wave, 64 bits in either tile: up to the rows that a large tile keeps, sums of 2 M entries 38.1 and 40.3, products 33.8 and 31.0; beyond those small tiles (2 M in 1.2, 1.8 M
+//     rows of 25 bits 46.6, 50.9 and 50.4, 58.8). The tiles for short rows and for the levels of a tree give way to small ones of 32 bits alike: trees of 1.9, 2.5 M entries per
+//     operand in 0.9, 0.6 M fibres of 21, 22 bits 61.3, 67.4 and 77.8, 87.2 us; of 1.9 M fibres in 0.2 M slices of 23 bits 98.1 and 133.3.
 // `rows` is the most there can be where only the device knows how many (row lists; sums of 1.3, 1.9, 2.5, 2.95 M entries per operand in as many rows: 51, 60, 75, 85 us with
 // small tiles, 78, 91, 134, 145 with large ones), 0 if the call does not know that either.
-inline int tile_v(int64_t total, int64_t rows, int32_t cols) {
+inline int tile_v(int64_t total, int64_t rows, int32_t cols, int large = V_LARGE) {
     if (total < LARGE_FROM) return V_SMALL;
-    if (total >= LARGE_ALWAYS_FROM) return V_LARGE;
+    if (total >= LARGE_ALWAYS_FROM) return large;
     const bool one_wave = total <= (int64_t)RESIDENT * tile_step(V_LARGE);
-    if (col_bits(cols) > 30 && !one_wave) return V_SMALL;
-    return rows * tile_step(V_LARGE) > (one_wave ? 2 : 1) * TilePlan<V_LARGE, false>::ROWS * total ? V_SMALL : V_LARGE;
+    const int bits = col_bits(cols);
+    auto wide = [&](int v, int64_t more) {
+        const int64_t average = rows * tile_step(v) / total;
+        return bits > 30 || (average + 1 + more * (2 + average / 32)) << bits > int64_t(1) << 31;
+    };
+    const bool wide_keys = wide(large, 1);  // not the average tile alone
+    if (wide_keys && !wide(V_SMALL, 0)) return V_SMALL;
+    if (large != V_LARGE) return large;
+    if (wide_keys && !one_wave) return V_SMALL;
+    return rows * tile_step(V_LARGE) > (one_wave && !wide_keys ? 2 : 1) * TilePlan<V_LARGE, false>::ROWS * total ? V_SMALL : V_LARGE;
 }
 
 // Raises the tile kernel's dynamic shared-memory limit once per instantiation and device.
@@ -1209,7 +1221,7 @@ int csr2_enqueue(SetOp op, const CsrIn &A, const CsrIn &B, const RowCount &rows,
                  void *scratch, cudaStream_t stream, FusedCtl **ctl_out, const LaunchKnobs &knobs) {
     const int64_t total = (int64_t)A.nnz + B.nnz;
     const int large = levels ? V_LEVELS : rows.short_rows && op == OP_UNION ? V_FIBRES : V_LARGE;
-    const int v = total < LARGE_FROM ? V_SMALL : large == V_LARGE ? tile_v(total, rows.value, cols) : large, step = tile_step(v);
+    const int v = tile_v(total, rows.value, cols, large), step = tile_step(v);
     const int num_tiles = (int)std::max<int64_t>(1, (total + step - 1) / step);
     Carver carve(scratch);
     Cuts cuts;

@@ -1,6 +1,10 @@
 """CPU suite: rules that a compiled kernel cannot show and its source can."""
 import os
 import re
+import shutil
+import subprocess
+
+import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nacho_b200", "csrc")
 
@@ -31,7 +35,30 @@ def test_the_choice_of_tiles_knows_the_rows_of_row_lists():
     merges = re.findall(r"csr2_enqueue\((.*?)\)\)\)?\s", source("formats2d.cu"), re.S)
     of_entries = [m for m in merges if "&rows_ctl->total}" in m]
     assert of_entries and all("RowCount{(int32_t)std::min<int64_t>(stored, a->rows), &rows_ctl->total}" in m for m in of_entries)
-    assert "tile_v(total, rows.value, cols)" in source("csr_merge.cu")
+    assert re.search(r"tile_v\(total, rows\.value, cols\b", source("csr_merge.cu"))
+
+
+@pytest.mark.skipif(not shutil.which("g++"), reason="no host compiler")
+def test_keys_of_a_large_tile_are_no_wider_than_need_be(tmp_path):
+    """The choice of tiles by itself: a large one whose keys take 64 bits gives way to a small one that gets by with 32."""
+    text = source("csr_merge.cu")
+    rule = text[text.index("inline int tile_v("):]
+    rule = rule[:rule.index("\n}\n") + 3]
+    cases = [(2_500_000, 30_000, 20, 31), (2_500_000, 750_000, 20, 15), (2_500_000, 750_000, 14, 31), (2_500_000, 250_000, 22, 15), (2_500_000, 25_000, 25, 15),
+             (4_000_000, 1_200_000, 20, 15), (5_900_000, 60_000, 25, 15), (5_900_000, 590_000, 22, 15), (5_900_000, 590_000, 16, 31), (6_000_000, 750_000, 20, 31),
+             (2_272_688, 10, 10, 15), (2_272_689, 10, 10, 31), (4_000_000, 10, 31, 31), (4_900_000, 10, 31, 15)]
+    (tmp_path / "rule.cpp").write_text("""
+#include <cstdint>
+#include <cstdio>
+constexpr int RESIDENT = 592, V_SMALL = 15, V_LARGE = 31;
+constexpr int tile_step(int v) { return 256 * v - 1; }
+constexpr int64_t LARGE_FROM = (int64_t)RESIDENT * tile_step(V_SMALL) + 1, LARGE_ALWAYS_FROM = 6000000;
+template <int V, bool L> struct TilePlan { static constexpr int ROWS = 1856; };
+static int col_bits(int32_t cols) { int b = 1; while (b < 32 && (int64_t(1) << b) < cols) ++b; return b; }
+""" + rule + "int main() {" + "".join('printf("%%d ", tile_v(%d, %d, (int32_t)%dll));' % (total, rows, min(1 << bits, 2**31 - 1)) for total, rows, bits, _ in cases) + "}")
+    subprocess.run(["g++", "-std=c++17", "-o", str(tmp_path / "rule"), str(tmp_path / "rule.cpp")], check=True)
+    got = subprocess.run([str(tmp_path / "rule")], check=True, capture_output=True, text=True).stdout.split()
+    assert [int(v) for v in got] == [want for *_, want in cases]
 
 
 def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():

@@ -229,6 +229,20 @@ def test_row_lists_on_either_side_of_the_tiles_they_take(nacho, oracle, total, e
     assert_same(dcsr_from_gpu(nacho.gpu_dcsr_mul_f32(da, db)), _dcsr_expected(oracle.csr_mul(a, b, 8), a, b, True), "dcsr mul")
 
 
+@pytest.mark.parametrize("total", [RESIDENT * LARGE_STEP - 5, RESIDENT * LARGE_STEP + 5, 5_900_000])
+@pytest.mark.parametrize("per_row,bits", [(3.3, 20), (10, 22), (100, 25), (35, 25), (60, 28)])
+def test_tiles_on_either_side_of_wide_keys(nacho, oracle, total, per_row, bits):
+    """Rows and columns with which a large tile's keys take 64 bits and a small one's 32, and with which both take 64."""
+    rows, cols = int(total / per_row), 1 << bits
+    rng = np.random.default_rng(total + bits)
+    ka, kb = key_pair(total, rows * cols, 0.3, rng)
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb, rows, cols, rng)
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_3_f32(ga, gb, ga)), oracle.csr_add_3(a, b, a, 8), "add_3")
+
+
 def test_stored_empty_rows_and_fibres(nacho, oracle):
     """Row lists that hold rows without entries, and trees that hold slices and fibres without any, come out without them."""
     from test_family_gpu import dcsr_from_gpu, dcsr_to_gpu
