@@ -114,8 +114,8 @@ def test_levels_behind_one_that_gave_up(nacho, oracle):
 @pytest.mark.parametrize("total", [24_000, 400_000, 1_500_000, 6_100_000])
 def test_a_late_give_up_is_reported(nacho, oracle, total):
     """A first tile that takes a millisecond, for the two million empty rows it begins with, and others that wait for its
-    count for some polls only: a call either says that they gave up or its result is whole. Few tiles that add up the
-    counts themselves, many that are handed their base."""
+    count for some polls only: a call either says that they gave up or its result is whole. Few tiles, which all
+    find their cuts themselves, and many, whose cuts come from the CTAs in front of them."""
     import ctypes as C
     import torch
     from nacho_b200 import _capi

@@ -11,10 +11,10 @@ from oracle.cpu_oracle import COO3, CSF3, CSR, DCSR
 
 pytestmark = pytest.mark.gpu
 
-SMALL_STEP = 256 * 15 - 1  # entries of a CSR tile below LARGE_FROM entries
-LARGE_FROM = 6_000_000     # a tile holds 256 * 31 from here
-COO_STEP = 256 * 7 - 1     # entries of a coordinate tile below 3 M
-DIRECT_TILES = 128         # beyond it one CTA sums the tiles' lengths
+SMALL_STEP = 256 * 15 - 1  # entries of a small CSR tile
+LARGE_FROM = 6_000_000     # a tile holds 256 * 31 from here whatever its rows and columns (from SWITCH on where they allow it)
+COO_STEP = 256 * 7 - 1     # entries of a small coordinate tile of a reduction (of a sum: SUM_STEP)
+DIRECT_TILES = 128         # a few of the windows in which a tile reads the counts in front of it
 
 
 @pytest.fixture(scope="module")
@@ -213,6 +213,87 @@ def test_coordinate_values_off_alignment(nacho, oracle, total, shift):
     _, at_a, at_b = np.intersect1d(ka, kb, assume_unique=True, return_indices=True)
     terms = a.val[at_a].astype(np.float64) * b.val[at_b]
     assert abs(float(nacho.gpu_inner_prod_coo_f32(ga, gb).values.cpu()[0]) - terms.sum()) <= 1e-5 * np.abs(terms).sum() + 1e-30
+
+
+# Where tiles change size, and where a second tile begins: 31 entries per thread for matrices from more small tiles on than are at work at once,
+# 11 and 17 for sums of coordinates (7 and 17 for their reductions), 21 for the fibres of trees, 23 for the levels above.
+SWITCH = RESIDENT * SMALL_STEP + 1
+SUM_STEP, FIBRE_STEP, LEVEL_STEP = 256 * 11 - 1, 256 * 21 - 1, 256 * 23 - 1
+
+
+@pytest.mark.parametrize("shape", ["one row", "rows of an entry", "rows of ten", "wide rows", "equal operands"])
+@pytest.mark.parametrize("total", [SWITCH - 1, SWITCH, SWITCH + 1])
+def test_csr_tiles_where_they_grow(nacho, oracle, total, shape):
+    """The last small tiles and the first large ones, for every shape of a tile."""
+    test_csr_tiles(nacho, oracle, total, shape)
+
+
+@pytest.mark.parametrize("tiles", [31, 32, 33, 34, 64, 65, 66, 97])
+def test_windows_of_counts(nacho, oracle, tiles):
+    """A tile reads the counts in front of it 32 at a time: as many tiles as fill one window or two, one less and one more."""
+    test_csr_tiles(nacho, oracle, tiles * SMALL_STEP, "rows of ten")
+    test_coordinate_tiles(nacho, oracle, tiles * SUM_STEP, (1 << 9, 1 << 10, 1 << 11))
+
+
+@pytest.mark.parametrize("dims", [(3, 4, 1 << 28), (1 << 26, 9, 5), (1 << 20, 1 << 21, 1 << 22)])
+@pytest.mark.parametrize("total", [SUM_STEP - 1, SUM_STEP, SUM_STEP + 1, 2 * SUM_STEP, 2 * SUM_STEP + 1])
+def test_coordinate_tiles_of_a_sum(nacho, oracle, total, dims):
+    """One and two tiles of a sum, an entry more and less."""
+    test_coordinate_tiles(nacho, oracle, total, dims)
+
+
+@pytest.mark.parametrize("total", [SUM_STEP - 2, SUM_STEP + 1, 2 * SUM_STEP + 5, RESIDENT * SUM_STEP + 1])
+@pytest.mark.parametrize("shift", [(0, 1), (3, 2)])
+def test_coordinate_values_off_alignment_in_sums(nacho, oracle, total, shift):
+    test_coordinate_values_off_alignment(nacho, oracle, total, shift)
+
+
+@pytest.mark.parametrize("gap", [3000, 1_200_000])
+def test_runs_of_empty_rows_between_large_tiles(nacho, oracle, gap):
+    """More large tiles than are at work at once, so that the CTAs in front of them make the cuts, with runs of empty rows between."""
+    rng = np.random.default_rng(gap)
+    clusters, entries, cols = 16, 250_000, 5000
+    rows = clusters * (gap + 1000)
+    ka = np.concatenate([np.sort(rng.choice(1000 * cols, entries, replace=False)) + c * (gap + 1000) * cols for c in range(clusters)])
+    kb = np.unique(np.concatenate([ka[::3], ka[1::4] + 1]))
+    a, b = csr_of_keys(ka, rows, cols, rng), csr_of_keys(kb[kb < rows * cols], rows, cols, rng)
+    assert len(a.col) + len(b.col) > max(700 * LARGE_STEP, 6_000_000)  # from where tiles are large whatever the rows
+    ga, gb = csr_to_gpu(a), csr_to_gpu(b)
+    assert_same(csr_from_gpu(nacho.gpu_csr_add_f32(ga, gb)), oracle.csr_add(a, b, 8), "add")
+    assert_same(csr_from_gpu(nacho.gpu_csr_mul_f32(ga, gb)), oracle.csr_mul(a, b, 8), "mul")
+
+
+AHEAD = 148  # tiles in front of a tile whose row offsets it asks for
+
+
+@pytest.mark.parametrize("total", [9, 2 * SMALL_STEP + 5, SWITCH + 3, 5_200_000])
+@pytest.mark.parametrize("dims", [(4000, 3000, 500), (2000, 130, 2000)])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_trees_of_many_tiles(nacho, oracle, total, dims, shift):
+    """Trees of about an entry in a fibre, and of twenty, from one tile to more on both lower levels than are at work at once, so that some
+    find their cuts and the offsets they ask for ahead made by the CTAs in front of them; with values that lie on 16-byte
+    boundaries differently from their coordinates, too."""
+    import torch
+    from test_tensor3_gpu import csf3_from_gpu
+    rng = np.random.default_rng(total + dims[1])
+
+    def tree(key, by):
+        ij, k = np.divmod(key, dims[2])
+        new = np.flatnonzero(np.diff(ij, prepend=-1))
+        i, j = np.divmod(ij[new], dims[1])
+        first = np.flatnonzero(np.diff(i, prepend=-1))
+        t = CSF3(dims, i[first].astype(np.int32), np.append(first, len(new)).astype(np.int32), j.astype(np.int32), np.append(new, len(key)).astype(np.int32),
+                 k.astype(np.int32), rng.uniform(-1, 1, len(key)).astype(np.float32))
+        to = lambda x: torch.from_numpy(x).cuda()
+        val = torch.empty(len(key) + by, dtype=torch.float32, device="cuda")[by:].copy_(to(t.val))
+        return t, nacho.CSF3_gpu(to(t.i_idx), to(t.j_ptr), to(t.j_idx), to(t.k_ptr), to(t.k_idx), val, torch.tensor(dims, dtype=torch.int32))
+
+    ka, kb = key_pair(total, dims[0] * dims[1] * dims[2], 0.3, rng)
+    (a, ga), (b, gb) = tree(ka, shift), tree(kb, (4 - shift) % 4)
+    if total > 5_000_000:
+        assert total > (RESIDENT + AHEAD) * FIBRE_STEP
+        assert dims[1] != 3000 or len(a.j_idx) + len(b.j_idx) > (RESIDENT + AHEAD) * LEVEL_STEP
+    assert_same(csf3_from_gpu(nacho.gpu_csf_add_f32(ga, gb)), oracle.csf3_add(a, b), "csf3")
 
 
 @pytest.mark.parametrize("each", [1, 2, 5])
