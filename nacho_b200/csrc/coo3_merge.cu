@@ -194,8 +194,9 @@ __device__ __forceinline__ uint32_t shl32(uint32_t x, int s) {
 }
 
 // Brings the tile's values into shared memory, entry e of A to word oa + e of `to` and B's to ob + e: aligned interiors by bulk
-// copy on the second phase of the tile's mbarrier, ragged ends, and arrays whose alignment differs, by plain loads. Called by all threads after
-// a barrier behind the last use of the words.
+// copy on the second phase of the tile's mbarrier, ragged ends by plain loads, arrays whose alignment differs word by word, on their way during the
+// merge too (copies_landed; sums of 16 M and 60 M entries of that kind took 263 and 680 us a call with plain loads, which the merge waits for, 233 and 630 with values
+// gathered from L2 behind it, 219 and 581 so). Called by all threads after a barrier behind the last use of the words.
 __device__ __forceinline__ void coo3_stage_values(const float *a_val, const float *b_val, const int na, const int nb, const int oa, const int ob, uint32_t *to,
                                                   Coo3Shared &sh) {
     const int tid = threadIdx.x;
@@ -218,7 +219,7 @@ __device__ __forceinline__ void coo3_stage_values(const float *a_val, const floa
     for (int q = 0; q < 2; ++q) {
         // the ends of q: a warp each; nothing but ends where no vector is copied
         if (nv[q] == 0) {
-            for (int e = tid; e < count[q]; e += NT) to[at[q] + e] = __float_as_uint(__ldg(src[q] + e));
+            for (int e = tid; e < count[q]; e += NT) copy_word(to + at[q] + e, src[q] + e);
         } else if ((tid >> 5) == 1 + q && (tid & 31) < 6) {
             const int e = tid & 31, idx = e < 3 ? e : head[q] + 4 * nv[q] + (e - 3);
             if (e < 3 ? e < head[q] : idx < count[q]) to[at[q] + idx] = __float_as_uint(__ldg(src[q] + idx));
@@ -360,6 +361,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) *to++ = (uint16_t)src[i];
+        if (STAGED) copies_landed();
         const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
         if (!__syncthreads_and(landed)) {
             if (tid == 0) {
@@ -389,6 +391,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     // ---- rank the survivors inside the tile
     const int incl = warp_incl_sum(steps);
     if (lane == 31) sh.wtotal[wid] = incl;
+    if (STAGED) copies_landed();
     const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
     if (!__syncthreads_and(landed)) {  // the values did not land in time: report, touch nothing
         if (tid == 0) {

@@ -61,6 +61,13 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gmem_src, 
                  : "memory");
 }
 
+// One 4-byte word global -> shared, on its own: where no bulk copy can bring an array because its 16-byte boundaries lie elsewhere. The words
+// that a thread has started have landed for it, and behind a barrier for the others, once it has called copies_landed.
+__device__ __forceinline__ void copy_word(void *smem_dst, const void *gmem_src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Asks for the L2 lines of `count` 4-byte elements at `p` (the 16-byte-aligned part of the range), 64 MB at most: what lies
 // further on would be gone from L2 again before anything reads it.
 __device__ __forceinline__ void prefetch_l2(const void *p, int count) {

@@ -61,6 +61,18 @@ static int col_bits(int32_t cols) { int b = 1; while (b < 32 && (int64_t(1) << b
     assert [int(v) for v in got] == [want for *_, want in cases]
 
 
+def test_the_merge_does_not_wait_for_values_of_another_alignment():
+    """What brings a tile's values into shared memory stands in front of its merge: an array that no bulk copy can bring is not loaded by the
+    threads, which would wait for it there, but copied word by word, and landed before the values are used."""
+    text = source("coo3_merge.cu")
+    body = text[text.index("void coo3_stage_values("):text.index("void coo3_tile(")]
+    loop = body[body.index("for (int e = tid"):]
+    assert "copy_word(" in loop[:loop.index(";", loop.index(")"))] and "__ldg" not in loop[:loop.index("else if")]
+    tile = text[text.index("void coo3_tile("):]
+    waits = [m.start() for m in re.finditer(r"mbar_wait_bounded\(&sh\.mbar, 1, MBAR_POLL_LIMIT\);\n\s*if \(!__syncthreads_and", tile)]
+    assert len(waits) == 2 and all("copies_landed();" in tile[at - 150:at] for at in waits)
+
+
 def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():
     """A kernel that starts beside the one in front of it must not use read-only loads (ld.global.nc, or a const
     __restrict__ parameter that the compiler turns into one) for what that kernel writes: they may be issued before the
