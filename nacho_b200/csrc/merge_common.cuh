@@ -55,7 +55,7 @@ struct TileWords {
     // Words that are zero, or of lower tags, at the start.
     __host__ __device__ static TileWords at(uint64_t *p, uint32_t tag = 1) { return TileWords{p, (uint64_t)tag << TAG_SHIFT}; }
 };
-constexpr uint64_t TW_COUNT = 1ull << 34, TW_SUM = 2ull << 34, TW_FAILED = 3ull << 34, TW_VALUE_MASK = (1ull << 34) - 1;
+constexpr uint64_t TW_COUNT = 1ull << 34, TW_SUM = 2ull << 34, TW_FAILED = 3ull << 34;
 
 __device__ __forceinline__ void raise_word(const TileWords &words, const int t, const uint64_t state_and_value) {
     atomicMax(reinterpret_cast<unsigned long long *>(words.word + t), (unsigned long long)(words.tag | state_and_value));
@@ -147,9 +147,9 @@ inline int take_own_words(cudaStream_t stream, int num_tiles, bool *wanted, OwnW
     return NB200_OK;
 }
 
-// One thread. What the reader of the cut goes on to read lies before it.
+// One thread. A word carries its tag and its part of the cut together, and what a tile reads with them lies behind its own wait_for_previous:
+// nothing needs an order among these writes or beside others.
 __device__ __forceinline__ void store_cut(const OwnWords &own, const int t, const int4 cut) {
-    __threadfence();
     uint64_t *w = own.cut + 4 * (size_t)t;
     st_relaxed_gpu(w, own.words.tag | (uint32_t)cut.x);
     st_relaxed_gpu(w + 1, own.words.tag | (uint32_t)cut.y);
@@ -160,7 +160,7 @@ __device__ __forceinline__ bool await_cut(const OwnWords &own, const int t, cons
     const uint64_t *w = own.cut + 4 * (size_t)t + min(lane_id(), 2);
     uint64_t v = 0;
     for (int polls = 0;; ++polls) {
-        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
+        v = ld_relaxed_gpu(w);
         if (__all_sync(FULL_MASK, (v ^ own.words.tag) >> TileWords::TAG_SHIFT == 0)) break;
         if (polls >= poll_limit) return false;
     }
