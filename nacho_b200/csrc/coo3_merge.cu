@@ -174,7 +174,7 @@ struct Coo3Plan {
     static_assert(4 * SLOTS < 32768, "byte offsets of entries are kept in 15 bits");
 };
 // A tile asks for the coordinates of one that starts a few microseconds later, so that they wait in L2. 100 M entries per
-// operand: 1238 us without, 1322, 1218, 1196 and 1197 with those 592, 296, 148 and 64 tiles ahead. Not for a tile that starts with
+// operand: 1061 us without, 1184, 1042, 1031 and 1036 with those 592, 296, 148 and 64 tiles ahead. Not for a tile that starts with
 // the first ones: 3 M entries per operand 77.1 -> 75.5 us.
 constexpr int TILES_AHEAD = 148;
 
@@ -197,7 +197,8 @@ __device__ __forceinline__ uint32_t shl32(uint32_t x, int s) {
 // copy on the second phase of the tile's mbarrier, ragged ends by plain loads, arrays whose alignment differs word by word, on their way during the
 // merge too (copies_landed; sums of 16 M and 60 M entries of that kind took 263 and 680 us a call with plain loads, which the merge waits for, 233 and 630 with values
 // gathered from L2 behind it, 219 and 581 so). Called by all threads after a barrier behind the last use of the words.
-__device__ __forceinline__ void coo3_stage_values(const float *a_val, const float *b_val, const int na, const int nb, const int oa, const int ob, uint32_t *to,
+// Returns, to all of them, whether copies_landed has to be called; where it is not needed it is left out (100 M entries 1031 -> 1027).
+__device__ __forceinline__ bool coo3_stage_values(const float *a_val, const float *b_val, const int na, const int nb, const int oa, const int ob, uint32_t *to,
                                                   Coo3Shared &sh) {
     const int tid = threadIdx.x;
     const float *const src[2] = {a_val, b_val};
@@ -225,6 +226,7 @@ __device__ __forceinline__ void coo3_stage_values(const float *a_val, const floa
             if (e < 3 ? e < head[q] : idx < count[q]) to[at[q] + idx] = __float_as_uint(__ldg(src[q] + idx));
         }
     }
+    return nv[0] == 0 || nv[1] == 0;
 }
 
 // One tile. NARROW: the keys of the tile, counted from its smallest, fit 32 bits (true of nearly every tile of
@@ -286,7 +288,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     }
     __syncthreads();
     // ---- the values take the place of the k coordinates; they land during the merge
-    if (STAGED) coo3_stage_values(A.val + a0, B.val + b0, na, nb, oa, ob, raw + 2 * P::SLOTS, sh);
+    const bool word_by_word = STAGED && coo3_stage_values(A.val + a0, B.val + b0, na, nb, oa, ob, raw + 2 * P::SLOTS, sh);
 
     // ---- where this thread's share begins: merge-path diagonal tid * VT (ties take A first; a coordinate that
     // both operands hold stays on one side)
@@ -361,7 +363,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
 #pragma unroll
         for (int i = 0; i < VT; ++i)
             if ((twin >> i) & 1u) *to++ = (uint16_t)src[i];
-        if (STAGED) copies_landed();
+        if (word_by_word) copies_landed();
         const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
         if (!__syncthreads_and(landed)) {
             if (tid == 0) {
@@ -391,7 +393,7 @@ __device__ __forceinline__ void coo3_tile(const Coo3In &A, const Coo3In &B, cons
     // ---- rank the survivors inside the tile
     const int incl = warp_incl_sum(steps);
     if (lane == 31) sh.wtotal[wid] = incl;
-    if (STAGED) copies_landed();
+    if (word_by_word) copies_landed();
     const bool landed = !STAGED || wid > 0 || mbar_wait_bounded(&sh.mbar, 1, MBAR_POLL_LIMIT);
     if (!__syncthreads_and(landed)) {  // the values did not land in time: report, touch nothing
         if (tid == 0) {
@@ -754,8 +756,8 @@ int bits_for(int32_t extent) {
 constexpr int tile_step_of(int v) { return NT * v - 1; }  // a twin may add one entry
 
 // Merged entries per worker thread: large tiles amortise the searches and the wait for the earlier counts, small
-// ones fill the chip when there are few entries, up to the number that can be at work at once (as in the CSR kernel). 100 M entries per operand, tile kernel: 1257 us with 13, 1195
-// with 17 (52 KB of shared memory: the most of which four CTAs fit an SM), 1331 with 19. Sums of 0.4, 0.6, 1, 1.3 M entries per
+// ones fill the chip when there are few entries, up to the number that can be at work at once (as in the CSR kernel). 100 M entries per operand, whole call: 1122 us with 13, 1065
+// with 15, 1027 with 17 (52 KB of shared memory: the most of which four CTAs fit an SM), 1098 with 19. Sums of 0.4, 0.6, 1, 1.3 M entries per
 // operand, whole call: 21.9, 32.2, 41.3, 48.2 us with 7, 21.3, 25.4, 39.7, 44.8 with 11, 32.4 and 42.4 the latter two with 17. A reduction has nothing
 // but the merge behind the staging: 0.1, 0.3, 0.6, 1 M 17.5, 18.6, 24.0, 31.5 with 7, 18.2, 18.9, 20.3, 29.1 with 11, 21.6 and 26.9 the latter two with 17.
 constexpr int V_LARGE = 17, V_SMALL = 11, V_REDUCE = 7;

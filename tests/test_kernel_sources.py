@@ -65,12 +65,13 @@ def test_the_merge_does_not_wait_for_values_of_another_alignment():
     """What brings a tile's values into shared memory stands in front of its merge: an array that no bulk copy can bring is not loaded by the
     threads, which would wait for it there, but copied word by word, and landed before the values are used."""
     text = source("coo3_merge.cu")
-    body = text[text.index("void coo3_stage_values("):text.index("void coo3_tile(")]
+    body = text[text.index("bool coo3_stage_values("):text.index("void coo3_tile(")]
     loop = body[body.index("for (int e = tid"):]
     assert "copy_word(" in loop[:loop.index(";", loop.index(")"))] and "__ldg" not in loop[:loop.index("else if")]
     tile = text[text.index("void coo3_tile("):]
     waits = [m.start() for m in re.finditer(r"mbar_wait_bounded\(&sh\.mbar, 1, MBAR_POLL_LIMIT\);\n\s*if \(!__syncthreads_and", tile)]
-    assert len(waits) == 2 and all("copies_landed();" in tile[at - 150:at] for at in waits)
+    assert len(waits) == 2 and all("if (word_by_word) copies_landed();" in tile[at - 150:at] for at in waits)
+    assert re.search(r"return nv\[0\] == 0 \|\| nv\[1\] == 0;", body) and "word_by_word = STAGED && coo3_stage_values(" in tile
 
 
 def test_no_read_only_loads_of_what_an_overlapped_kernel_waits_for():
