@@ -272,17 +272,18 @@ int csf_add_expanded(const nb200_csf3 *a, const nb200_csf3 *b, nb200_csf3 *z, in
 //      CSR union writes Z's k_ptr, k_idx and val.
 // Steps 2 and 3 read their row count from device memory.
 
-// Measured against the expanded route: 25 M entries per operand in fibres of 7, 445 us against 821; 5 M in
-// fibres of 4, 230 against 258; 5000 in fibres of 1.1, 54 against 66. So it is taken wherever it applies.
+// Measured against the expanded route: 25 M entries per operand in fibres of 7, 262 us against 625; 5 M in
+// fibres of 4, 96 against 205; 5000 in fibres of 1, 39 against 63. So it is taken wherever it applies.
 bool levels_pay(const nb200_csf3 *a, const nb200_csf3 *b) {
     if (a->n_j == 0 || b->n_j == 0) return false;
     if (const char *e = std::getenv("NACHO_B200_CSF_TWO_LEVEL")) return e[0] != '0';  // read per call: tests take both routes
     return true;
 }
 
-// Up to this many entries per fibre of the operands, the tile for short rows takes the entries. 25 M entries per operand,
-// whole call, that tile against the large one: 365 us against 411 with 6 entries per fibre, 297 against 317 with 30, 291
-// against 294 with 50, 270 against 254 with 113; 5 M: 102 against 104 with 36.
+// Up to this many entries per fibre of the operands, the tile for short rows takes the entries. Whole call, that tile against the large one, with 1, 2, 4,
+// 12, 30 and 62 entries per fibre: 3 M entries per operand 94, 80, 70, 62, 60, 60 us and 111, 92, 72, 65, 60, 61; 8 M 174, 146, 124, 109, 105, 103 and 204, 160, 119, 104, 99, 98;
+// 25 M 440, 370, 292, 239, 220, 217 and 532, 409, 280, 228, 206, 203. The line was drawn when tiles gathered their values; since they copy them, the tile for
+// short rows earns its place up to some three entries per fibre, and beyond those among the smaller trees alone.
 constexpr int64_t SHORT_FIBRE = 64;
 
 // `done` tells whether the result is in place; it is not where an operand stores empty slices or fibres, which

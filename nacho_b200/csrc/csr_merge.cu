@@ -159,9 +159,9 @@ __global__ void __launch_bounds__(NT) k_csr2_partition(CsrIn A, CsrIn B, RowCoun
 
 
 // Large tile where the caller says that rows are short (the fibres of a tree): a tile of 31 with more rows than fit takes
-// twice the time of the others and holds up their output bases, and the twin mask by entries (below) pays. 25 M entries
-// per operand in 6 M fibres take 384 us with 17, 389 with 21, 426 with 23, 446 with 31; 50 M in 4 M fibres 513, 508,
-// 563, 548. The stored rows of a doubly compressed matrix are longer: 8 M entries per operand 123 us with 31, 127 with 21.
+// longer than the others and holds up their output bases, and the twin mask by entries (below) pays. Trees of 25 M entries per operand, whole call, with 1, 2, 4, 12
+// entries per fibre 440, 370, 292, 239 us with 21, 447, 373, 305, 250 with 17, 533, 358, 283, 232 with 23 and 532, 409, 280, 228 with 31; 8 M with 1 and 2 174 and 146 with
+// 21, 204 and 160 with 31.
 constexpr int V_FIBRES = 21, V_MOST = 31;  // V_MOST: the large tile otherwise
 
 // Shared-memory plan of the tile body. The column words of both operands lie in one array: A's entry e at
@@ -183,8 +183,8 @@ struct TilePlan {
 constexpr uint32_t ROW_FAR = 0xffffu;
 
 // A tile, other than the large one, asks for the row offsets of one that starts a few microseconds later, so that they wait in L2:
-// they are read by plain loads, a few dependent rounds of them. (Trees of 25 M entries per operand 384 -> 371 us. The columns
-// ahead as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead.) Not for a tile that starts with the
+// they are read by plain loads, a few dependent rounds of them. (Trees of 50 M entries per operand in fibres of 1, 6 and 30 entries 827, 498, 400 us without, 807, 495, 396
+// so; of 8 M no difference. The columns ahead as well cost the largest sums 1 to 4 %, whether 64, 148, 296 or 592 tiles ahead, when tiles gathered their values.) Not for a tile that starts with the
 // first ones, and at most as many offsets as a tile keeps: beyond those lie runs of empty rows, which could fill the L2.
 constexpr int TILES_AHEAD = 148;
 // Tiles up to which a call that waits for its length is one launch. Two operands of 24, 32, 40 and 50 M entries (6050, 8070, 10090 and 12610 tiles) take
@@ -227,8 +227,8 @@ __device__ __noinline__ int far_row(const int32_t *rp, const int32_t entry, cons
 // A row mark is 16 bits per staged word, in the place of the source indices that come later: the last row
 // that begins at the entry (ROW_FAR: beyond 16 bits, looked up in the row offsets).
 //
-// What bounds this kernel is instruction issue and, for a tile, latency: the wait for its columns and the
-// wait for the counts of all earlier tiles, together half of its lifetime. So
+// What bounds this kernel is instruction issue and, for a tile, latency: phases that barriers separate, with a wait for its columns in front (2.97 of
+// its 13 us; the wait for the counts of all earlier tiles is 0.15). So
 //   - the merge is sequential and moves columns only: one compare and at most two loads per result entry
 //     (a key-building pass, a register merge network and a per-entry value gather took four times the
 //     instructions), and it leaves a 16-bit source index per result entry;
@@ -249,8 +249,8 @@ __device__ __forceinline__ void csr2_tile(const CsrIn &A, const CsrIn &B, const 
     constexpr int W = NT / 32;
     constexpr Key END = WIDE ? (Key)~0ull : (Key)0x80000000u;  // after every key (narrow: keys are below 2^31), also with row bits added
     constexpr bool WRITES = MODE != MODE_COUNT;
-    // Rows of an entry or two: a mask by entries instead of steps spares every row offset a search of it (25 M entries per
-    // operand in 6 M rows: 391.5 -> 388.5 us). With fewer rows the mask costs more than the searches (67 M entries 458 -> 460.5).
+    // Rows of an entry or two: a mask by entries instead of steps spares every row offset a search of it (trees of 25 M entries per
+    // operand with 1 and 2 in a fibre: 461 -> 440, 378 -> 370 us). With fewer rows the mask costs more than the searches (12 in a fibre 235 -> 239).
     constexpr bool MANY_ROWS = VT == V_FIBRES;
     uint32_t *s_rows = reinterpret_cast<uint32_t *>(smem_raw + P::ROWS_AT);  // start of row r in the tile: A's in the lower half, B's in the upper
     int *s_trow = sh.trow, *s_wrow = sh.wrow, *s_rank = sh.trow, *s_wtotal = sh.wtotal;
